@@ -196,13 +196,16 @@ struct DevBuf {
 struct Slot {
     uint8_t *host = nullptr; // pinned
     size_t host_cap = 0;
-    DevBuf blob, clean, coef, planes, rgb, status, ckpt;
+    DevBuf blob, clean, segs, index, planes, rgb; // segs: per-segment scratch; index: per-block positions and DC values
     BatchHeader hdr{};
     ffcvb_plan plan{};
-    int n = 0, n_jpeg = 0, n_par = 0, n_seq = 0, max_pixels = 0, subseq_bits = 512, entropy_threads = 512;
+    int n = 0, n_jpeg = 0, n_segs = 0, n_multi = 0, n_restart = 0, max_tables = 0;
+    bool alike = false;
+    uint32_t max_raw = 0; // raw bytes of the largest segment
     int n_quad = 0, n_444 = 0, n_other = 0, max_w = 0, max_h = 0;
-    uint64_t jpeg_list_off = 0, par_list_off = 0, seq_list_off = 0, quad_tiles_off = 0;
-    int n_quad_tiles = 0;
+    uint64_t jpeg_list_off = 0, segs_off = 0, multi_off = 0, restart_off = 0, block_tiles_off = 0, quad_tiles_off = 0;
+    uint64_t status_off = 0; // status word and counter of finished segments of every sample
+    int n_block_tiles = 0, n_quad_tiles = 0;
     uint32_t total_blocks = 0;
     size_t clean_bytes = 0, plane_bytes = 0, rgb_bytes = 0, scan_bytes = 0, raw_bytes = 0, jpeg_bytes = 0;
     bool staged = false;
@@ -273,17 +276,15 @@ struct ffcvb_ctx {
     double share = 0.0;          // the adjusted share, 0..1
     int split_copy_threads = 4; // ... and how many of them copy at a time (more only crowd the gather out)
     // Tuning overrides, read from the environment once when the context is created (0 = none):
-    // FFCV_B200_COPY_THREADS, FFCV_B200_SUBSEQ_BITS, FFCV_B200_ENTROPY_THREADS, FFCV_B200_GATHER_CTAS,
-    // FFCV_B200_GATHER_IN_FLIGHT.
-    int tune_copy_threads = 0, tune_subseq_bits = 0, tune_entropy_threads = 0, gather_ctas = 0, gather_in_flight = 8;
+    // FFCV_B200_COPY_THREADS, FFCV_B200_SUBSEQ_BITS, FFCV_B200_GATHER_CTAS, FFCV_B200_GATHER_IN_FLIGHT.
+    int tune_copy_threads = 0, tune_subseq_bits = 0, gather_ctas = 0, gather_in_flight = 8;
     DevBuf one_src, one_dst; // single-image entry points
     // Decode index (ffcvb_set_decode_index): a pool of device memory that keeps, per JPEG stream seen,
     // the decoder states a finished decode left behind; entries are handed out in order and never
     // moved.  Keyed by the sample's offset in the file: the context then serves one file.
     struct IndexEntry {
         uint64_t off;
-        uint32_t cap;
-        uint32_t subseq_bits;
+        uint32_t segments;
         uint64_t created_seq;
     };
     // Header cache: what the marker segments of a JPEG sample said, kept per sample (key: its
@@ -299,7 +300,7 @@ struct ffcvb_ctx {
     };
     bool cache_headers = false; // ffcvb_set_header_cache: sample offsets identify samples (one file per context)
     std::unordered_map<uint64_t, CachedHeader> header_cache;
-    std::vector<std::unique_ptr<RawHuff>> huff_store;
+    std::vector<std::unique_ptr<HuffTable>> huff_store; // built tables
     std::vector<std::unique_ptr<std::array<uint16_t, 64>>> quant_store;
     std::vector<uint64_t> huff_store_hash, quant_store_hash;
     DevBuf index_pool, index_stats;
@@ -380,28 +381,6 @@ OpList make_oplist(const ffcvb_plan &p) {
     return o;
 }
 
-// CTA size and subsequence length of the speculative entropy decoder for a batch whose largest
-// scan has `max_scan_bytes`.  One pass of the CTA's threads should cover the largest image (the
-// decoder needs about 7 kbit to re-synchronise, so shorter subsequences only add repair rounds),
-// with subsequences of at most 1280 bits (a chunk of 512 of them must fit shared memory twice per
-// SM) and no more threads than that takes: small images decode faster with 128 or 256 threads per
-// CTA because more CTAs are resident (config 1: 0.98 ms with 512 threads, 0.79-0.84 with 256).
-// Multiples of 128 bits keep chunk starts 16-byte aligned.
-void pick_entropy_config(size_t max_scan_bytes, int *threads, int *subseq_bits) {
-    const size_t bits = max_scan_bytes * 8 + 1;
-    int nt = 512;
-    if (bits <= 128 * 1280) nt = 128;
-    else if (bits <= 256 * 1280) nt = 256;
-    size_t s = align_up(bits / nt + 1, 128);
-    if (s < 512) s = 512;
-    // Larger images: one chunk of long subsequences read from global memory (a chunk of 1280-bit
-    // subsequences per 655 kbit would serialise dozens of chunks per image); 65535 blocks per
-    // subsequence is the kernel's limit, a block has at least 6 bits
-    if (s > 256 * 1024) s = 256 * 1024;
-    *threads = nt;
-    *subseq_bits = (int)s;
-}
-
 } // namespace
 
 extern "C" {
@@ -428,11 +407,7 @@ int ffcvb_create(int device, int n_slots, int n_threads, ffcvb_ctx **out) {
         return v >= lo && v <= hi ? v : 0;
     };
     c->tune_copy_threads = env_int("FFCV_B200_COPY_THREADS", 1, 256);
-    c->tune_subseq_bits = (env_int("FFCV_B200_SUBSEQ_BITS", 128, 256 * 1024) + 127) / 128 * 128;
-    c->tune_entropy_threads = env_int("FFCV_B200_ENTROPY_THREADS", 128, 1024);
-    if (c->tune_entropy_threads != 128 && c->tune_entropy_threads != 256 && c->tune_entropy_threads != 512 &&
-        c->tune_entropy_threads != 1024)
-        c->tune_entropy_threads = 0; // only the CTA sizes the kernel is built for
+    c->tune_subseq_bits = env_int("FFCV_B200_SUBSEQ_BITS", 128, kMaxSubseqBits) / 32 * 32;
     c->gather_ctas = env_int("FFCV_B200_GATHER_CTAS", 1, 1024);
     if (env_int("FFCV_B200_GATHER_IN_FLIGHT", 4, 4)) c->gather_in_flight = 4;
     *out = c;
@@ -446,7 +421,7 @@ void ffcvb_destroy(ffcvb_ctx *ctx) {
     cudaDeviceSynchronize();
     for (auto &s : ctx->slots) {
         if (s.host) cudaFreeHost(s.host);
-        for (DevBuf *b : {&s.blob, &s.clean, &s.coef, &s.planes, &s.rgb, &s.status, &s.ckpt})
+        for (DevBuf *b : {&s.blob, &s.clean, &s.segs, &s.index, &s.planes, &s.rgb})
             if (b->p) cudaFree(b->p);
         for (auto &e : s.ev)
             if (e) cudaEventDestroy(e);
@@ -581,6 +556,7 @@ int stage_impl(ffcvb_ctx *ctx, int slot, const Source &source, const uint64_t *p
         size_t off = align_up(sizeof(BatchHeader), 16);
         off = align_up(off + sizeof(ImageDesc) * (size_t)n, 16);
         off = align_up(off + sizeof(int32_t) * (size_t)n * n_params_early, 16);
+        off = align_up(off + 2 * sizeof(int32_t) * (size_t)n, 16);
         for (const auto &r : s.pending_riders) off = align_up(off, 64) + r.item_bytes * (uint64_t)n;
         fd_payload_begin = off = align_up(off, A);
         spans.resize(n);
@@ -610,8 +586,11 @@ int stage_impl(ffcvb_ctx *ctx, int slot, const Source &source, const uint64_t *p
         fd_payload_end = off;
         // room behind the payloads for what is laid out after the parse: at most 255 tables of each kind
         size_t tail = 255 * (sizeof(HuffTable) + sizeof(MultTable)) + 3 * (sizeof(int32_t) * (size_t)n + 16) + 256;
-        for (int i = 0; i < n; i++) // and the colour kernel's tile table: at most the tiles of whole images
+        for (int i = 0; i < n; i++) { // and the tables of CTAs: at most those of whole images and of the shortest segments
             tail += sizeof(uint2) * (size_t)((((heights[i] + 1) / 2 + 7) / 8) * ((((widths[i] + 1) / 2 + 1) / 2 + 1 + 31) / 32));
+            tail += sizeof(uint2) * ((size_t)((heights[i] + 15) / 8) * ((widths[i] + 15) / 8) * 3 / kBlockTile + 4);
+            tail += sizeof(uint2) * (size_t)(sizes[i] / (64 * kSegSubs / 8) + 2);
+        }
         int grc;
         if ((grc = grow_host(ctx, s.host, s.host_cap, fd_payload_end + tail))) return grc;
     }
@@ -691,8 +670,8 @@ int stage_impl(ffcvb_ctx *ctx, int slot, const Source &source, const uint64_t *p
                     uint64_t *th = &s.table_hash[(size_t)i * 9 + 3 * c];
                     // (bits[17] and vals[256] lie next to each other in RawHuff)
                     static_assert(offsetof(RawHuff, vals) == 17, "RawHuff: vals must follow bits");
-                    th[0] = hash_bytes(h.dc[h.td[c]].bits, 17 + 256);
-                    th[1] = hash_bytes(h.ac[h.ta[c]].bits, 17 + 256);
+                    th[0] = hash_bytes(h.dc[h.td[c]].bits, 17 + 256) & ~1ull; // (the same code as a DC and as an AC table: two tables)
+                    th[1] = hash_bytes(h.ac[h.ta[c]].bits, 17 + 256) | 1ull;
                     th[2] = hash_bytes(h.quant[h.tq[c]], 128);
                 }
                 // scale of the decode (plan->dct_scale): only layouts whose planes end up at one resolution
@@ -791,10 +770,11 @@ int stage_impl(ffcvb_ctx *ctx, int slot, const Source &source, const uint64_t *p
             for (int k = 0; k < 2; k++) {
                 int found = -1;
                 for (int u = (int)ctx->huff_store.size() - 1; u >= 0 && found < 0; u--)
-                    if (ctx->huff_store_hash[u] == th[k] && memcmp(ctx->huff_store[u]->bits, tabs[k]->bits, 17) == 0) found = u;
+                    if (ctx->huff_store_hash[u] == th[k] && memcmp(ctx->huff_store[u]->vals, tabs[k]->vals, 256) == 0) found = u;
                 if (found < 0 && ctx->huff_store.size() < 60000) {
                     found = (int)ctx->huff_store.size();
-                    ctx->huff_store.emplace_back(new RawHuff(*tabs[k]));
+                    ctx->huff_store.emplace_back(new HuffTable());
+                    build_huff_table(*tabs[k], k == 0, ctx->huff_store.back().get());
                     ctx->huff_store_hash.push_back(th[k]);
                 }
                 room = room && found >= 0;
@@ -829,35 +809,57 @@ int stage_impl(ffcvb_ctx *ctx, int slot, const Source &source, const uint64_t *p
         }
     }
     // ---- serial: the batch's own table lists (indices into the store -> indices into the blob)
-    std::vector<const RawHuff *> huff_src;
+    std::vector<const HuffTable *> huff_src;
     std::vector<const uint16_t *> mult_src;
     std::vector<int> huff_of_store(ctx->huff_store.size(), -1), mult_of_store(ctx->quant_store.size(), -1);
-    std::vector<int32_t> jpeg_list, par_list, seq_list;
-    std::vector<uint2> quad_tiles; // (sample, tile x | tile y << 16) of the 4:2:0 colour kernel's CTAs
-    size_t clean_bytes = 0, plane_bytes = 0, rgb_bytes = 0, scan_bytes_par = 0;  // scan_bytes_par: largest scan
-    uint32_t total_blocks = 0;
-    int max_pixels = 0, max_w = 0, max_h = 0, n_quad = 0, n_444 = 0, n_other = 0;
+    std::vector<int32_t> jpeg_list, multi, restart;
+    std::vector<uint2> segs;        // (sample, segment) of the entropy decoder's CTAs
+    std::vector<uint2> blk_tiles;   // (sample, k) of the block decoder's CTAs
+    std::vector<uint2> quad_tiles;  // (sample, tile x | tile y << 16) of the 4:2:0 colour kernel's CTAs
+    size_t clean_bytes = 0, plane_bytes = 0, rgb_bytes = 0;
+    uint32_t total_blocks = 0, max_raw = 0;
+    int max_tables = 1, first_jpeg = -1;
+    bool alike = true; // all scans use the same tables in the same MCU layout
+    // Subsequence length: by the batch's bits, or, with a decode index, a function of the stream alone
+    // (1024 bits), so that the recorded states stay usable whatever batch the sample lands in.
+    uint32_t target_bits = 1024;
+    if (!ctx->index_pool.p) {
+        uint64_t bits = 0;
+        for (int i = 0; i < n; i++)
+            if (descs[i].mode == FFCVB_MODE_JPG && descs[i].host_status == 0) bits += (uint64_t)descs[i].scan_len * 8;
+        target_bits = subseq_target(bits);
+    }
+    if (ctx->tune_subseq_bits) target_bits = (uint32_t)ctx->tune_subseq_bits;
+    ctx->stage_seq++;
+    int max_w = 0, max_h = 0, n_quad = 0, n_444 = 0, n_other = 0;
     for (int i = 0; i < n; i++) {
         ImageDesc &d = descs[i];
         if (d.mode != FFCVB_MODE_JPG) continue;
         jpeg_list.push_back(i);
-        if (d.host_status != 0) {
-            par_list.push_back(i); // the kernel only records the status
+        if (d.host_status != 0) { // (no kernel touches it: its status word says so)
             d.block_base = total_blocks;
             continue;
         }
         const JpegHeader &h = s.headers[i];
         const uint16_t *ids = &s.table_id[(size_t)i * 9];
-        for (int c = 0; c < h.ncomp; c++) {
-            uint8_t *dst[2] = {&d.dc_tab[c], &d.ac_tab[c]};
-            for (int k = 0; k < 2; k++) {
+        d.fast_tables = 1;
+        for (int k = 0; k < 2; k++) { // the image's distinct tables: DC before AC
+            uint8_t *dst = k == 0 ? d.dc_tab : d.ac_tab;
+            for (int c = 0; c < h.ncomp; c++) {
                 int &slot_of = huff_of_store[ids[3 * c + k]];
                 if (slot_of < 0) {
                     slot_of = (int)huff_src.size();
                     huff_src.push_back(ctx->huff_store[ids[3 * c + k]].get());
                 }
-                *dst[k] = (uint8_t)slot_of;
+                int u = 0;
+                while (u < d.n_tab && d.tab_id[u] != (uint8_t)slot_of) u++;
+                if (u == d.n_tab) d.tab_id[d.n_tab++] = (uint8_t)slot_of;
+                dst[c] = (uint8_t)u;
+                if (!ctx->huff_store[ids[3 * c + k]]->fast_ok) d.fast_tables = 0;
             }
+            if (k == 0) d.n_dc_tab = d.n_tab;
+        }
+        for (int c = 0; c < h.ncomp; c++) {
             int &qslot = mult_of_store[ids[3 * c + 2]];
             if (qslot < 0) {
                 qslot = (int)mult_src.size();
@@ -869,12 +871,53 @@ int stage_impl(ffcvb_ctx *ctx, int slot, const Source &source, const uint64_t *p
             return fail(ctx, FFCVB_E_LIMIT, "more than 255 distinct Huffman or quantisation tables in a batch");
         d.block_base = total_blocks;
         total_blocks += d.nblocks;
+        if (2 * d.n_tab - d.n_dc_tab > max_tables) max_tables = 2 * d.n_tab - d.n_dc_tab;
+        if (first_jpeg < 0) first_jpeg = i;
+        const ImageDesc &f = descs[first_jpeg];
+        alike = alike && d.bpm == f.bpm && d.hs == f.hs && d.n_tab == f.n_tab && d.n_dc_tab == f.n_dc_tab &&
+                memcmp(d.tab_id, f.tab_id, sizeof(d.tab_id)) == 0 && memcmp(d.dc_tab, f.dc_tab, sizeof(d.dc_tab)) == 0 &&
+                memcmp(d.ac_tab, f.ac_tab, sizeof(d.ac_tab)) == 0;
         d.clean_off = clean_bytes;
-        clean_bytes += align_up((size_t)d.scan_len + 96, 16);
         if (d.restart_interval) { // table of interval starts behind the clean stream
+            clean_bytes += align_up((size_t)d.scan_len + 96, 16);
             d.rst_off = clean_bytes;
             const size_t mcus = (size_t)d.mcus_x * d.mcus_y;
             clean_bytes += align_up(4 * ((mcus + d.restart_interval - 1) / d.restart_interval + 2), 16);
+            restart.push_back(i);
+        } else {
+            const ScanLayout l = layout_scan(d.scan_len, target_bits);
+            d.subseq_bits = l.subseq_bits;
+            d.seg_raw = l.seg_raw;
+            d.seg_warm = l.seg_warm;
+            d.seg_stride = l.seg_stride;
+            d.seg_count = l.seg_count;
+            d.seg_first = (uint32_t)segs.size();
+            clean_bytes += (size_t)l.seg_count * l.seg_stride;
+            for (uint32_t k = 0; k < l.seg_count; k++) segs.push_back(make_uint2((uint32_t)i, k));
+            if (l.seg_count > 1) multi.push_back(i);
+            const uint32_t raw = kSegSubs * l.subseq_bits / 8 + kSegOverlap;
+            if (raw > max_raw) max_raw = raw;
+            if (ctx->index_pool.p) {
+                const uint64_t key = ptrs[i];
+                auto it = ctx->index_map.find(key);
+                if (it == ctx->index_map.end()) {
+                    const size_t bytes = decode_index_bytes(l.seg_count);
+                    if (ctx->index_used + bytes <= ctx->index_pool.cap) { // else this stream stays unindexed
+                        it = ctx->index_map.emplace(key, ffcvb_ctx::IndexEntry{ctx->index_used, l.seg_count, ctx->stage_seq}).first;
+                        ctx->index_used += bytes;
+                    }
+                } else if (ctx->stage_seq - it->second.created_seq < ctx->slots.size()) {
+                    it = ctx->index_map.end(); // recorded by a batch that may still run on another slot's stream: hands off
+                }
+                if (it != ctx->index_map.end() && it->second.segments == l.seg_count) {
+                    d.index_off = it->second.off;
+                    d.index_cap = it->second.segments;
+                }
+            }
+        }
+        {
+            const uint32_t tiles = block_tiles(d);
+            for (uint32_t k = 0; k < tiles; k++) blk_tiles.push_back(make_uint2((uint32_t)i, k));
         }
         for (int c = 0; c < h.ncomp; c++) {
             d.plane_off[c] = plane_bytes;
@@ -885,7 +928,6 @@ int stage_impl(ffcvb_ctx *ctx, int slot, const Source &source, const uint64_t *p
         d.rgb_off = rgb_bytes;
         d.rgb_pitch = (uint32_t)align_up((size_t)d.dec_width * 3, 16);
         rgb_bytes += (size_t)d.dec_height * d.rgb_pitch;
-        if ((int)d.dec_height * d.dec_width > max_pixels) max_pixels = (int)d.dec_height * d.dec_width;
         int bw = d.dec_width, bh = d.dec_height;
         {   // extent the colour kernels' grids must cover: the crop box (plus the odd edge of a
             // chroma cell) where the kernel converts only that, else the whole image
@@ -914,53 +956,6 @@ int stage_impl(ffcvb_ctx *ctx, int slot, const Source &source, const uint64_t *p
             n_444++;
         else
             n_other++;
-        if (d.restart_interval) {
-            seq_list.push_back(i);
-        } else {
-            par_list.push_back(i);
-            if (d.scan_len > scan_bytes_par) scan_bytes_par = d.scan_len;
-        }
-    }
-
-    // ---- entropy decode configuration: CTA size and longest subsequence by the batch's largest
-    // scan; with a decode index every image gets a subsequence length of its own and its entry
-    pick_entropy_config(scan_bytes_par, &s.entropy_threads, &s.subseq_bits);
-    if (ctx->tune_subseq_bits) s.subseq_bits = ctx->tune_subseq_bits;
-    if (ctx->tune_entropy_threads) s.entropy_threads = ctx->tune_entropy_threads;
-    ctx->stage_seq++;
-    for (int i : par_list) {
-        ImageDesc &d = descs[i];
-        d.subseq_bits = (uint32_t)s.subseq_bits;
-        d.index_cap = 0;
-        d.index_off = 0;
-        if (!ctx->index_pool.p || d.host_status != 0) continue;
-        // a function of the stream alone (the CTA size its own length would get), so that the
-        // recorded states stay usable whatever batch the sample lands in next time
-        int own_threads, own_bits;
-        pick_entropy_config(d.scan_len, &own_threads, &own_bits);
-        const size_t own = (size_t)own_bits;
-        d.subseq_bits = (uint32_t)own;
-        const uint64_t key = ptrs[i];
-        auto it = ctx->index_map.find(key);
-        if (it != ctx->index_map.end() && it->second.subseq_bits != d.subseq_bits) {
-            // the batch's CTA size changed the subsequence length: the old entry is of no use
-            // (its memory stays with the pool); a new one is recorded
-            ctx->index_map.erase(it);
-            it = ctx->index_map.end();
-        }
-        if (it == ctx->index_map.end()) {
-            const uint32_t cap = (uint32_t)(((size_t)d.scan_len * 8 + own - 1) / own + 2);
-            const size_t bytes = decode_index_bytes(cap);
-            if (ctx->index_used + bytes > ctx->index_pool.cap) continue; // pool full: this stream stays unindexed
-            ffcvb_ctx::IndexEntry e{ctx->index_used, cap, d.subseq_bits, ctx->stage_seq};
-            ctx->index_used += bytes;
-            it = ctx->index_map.emplace(key, e).first;
-        } else if (ctx->stage_seq - it->second.created_seq < ctx->slots.size()) {
-            // recorded by a batch that may still be running on another slot's stream: hands off
-            continue;
-        }
-        d.index_off = it->second.off;
-        d.index_cap = it->second.cap;
     }
 
     BatchHeader &hd = s.hdr;
@@ -981,16 +976,22 @@ int stage_impl(ffcvb_ctx *ctx, int slot, const Source &source, const uint64_t *p
     auto place_lists = [&] {
         s.jpeg_list_off = off;
         off = align_up(off + sizeof(int32_t) * jpeg_list.size(), 16);
-        s.par_list_off = off;
-        off = align_up(off + sizeof(int32_t) * par_list.size(), 16);
-        s.seq_list_off = off;
-        off = align_up(off + sizeof(int32_t) * seq_list.size(), 16);
+        s.multi_off = off;
+        off = align_up(off + sizeof(int32_t) * multi.size(), 16);
+        s.restart_off = off;
+        off = align_up(off + sizeof(int32_t) * restart.size(), 16);
+        s.segs_off = off;
+        off = align_up(off + sizeof(uint2) * segs.size(), 16);
+        s.block_tiles_off = off;
+        off = align_up(off + sizeof(uint2) * blk_tiles.size(), 16);
         s.quad_tiles_off = off;
         off = align_up(off + sizeof(uint2) * quad_tiles.size(), 16);
     };
     if (!from_fd) place_tables();
     hd.params_off = off;
     off = align_up(off + sizeof(int32_t) * (size_t)n * n_params, 16);
+    s.status_off = off;
+    off = align_up(off + 2 * sizeof(int32_t) * (size_t)n, 16);
     s.riders.swap(s.pending_riders);
     s.pending_riders.clear();
     for (auto &r : s.riders) {
@@ -1051,19 +1052,26 @@ int stage_impl(ffcvb_ctx *ctx, int slot, const Source &source, const uint64_t *p
         return fail(ctx, FFCVB_E_ARG, "ffcvb_stage_batch_fd: tables and lists do not fit behind the payloads");
     if ((rc = grow_host(ctx, s.host, s.host_cap, off + 64))) return rc;
     if ((rc = grow_dev(ctx, s.blob, off + 64))) return rc;
-    if ((rc = grow_dev(ctx, s.clean, clean_bytes + 64))) return rc;
-    if ((rc = grow_dev(ctx, s.coef, (size_t)total_blocks * 128 + 64))) return rc;
+    if ((rc = grow_dev(ctx, s.clean, clean_bytes + 512))) return rc;
+    if ((rc = grow_dev(ctx, s.segs, segs.size() * (sizeof(SegMeta) + 4 * kSegSubs + 16) + 64))) return rc;
+    if ((rc = grow_dev(ctx, s.index, (size_t)total_blocks * 6 + 64))) return rc;
     if ((rc = grow_dev(ctx, s.planes, plane_bytes + 64))) return rc;
     if ((rc = grow_dev(ctx, s.rgb, rgb_bytes + 64))) return rc;
-    if ((rc = grow_dev(ctx, s.status, sizeof(int32_t) * (size_t)n + 64))) return rc;
 
     memcpy(s.host, &hd, sizeof(hd));
     memcpy(s.host + hd.desc_off, descs.data(), sizeof(ImageDesc) * (size_t)n);
     for (size_t k = 0; k < huff_src.size(); k++)
-        build_huff_table(*huff_src[k], reinterpret_cast<HuffTable *>(s.host + hd.huff_off) + k);
+        memcpy(s.host + hd.huff_off + k * sizeof(HuffTable), huff_src[k], sizeof(HuffTable));
     for (size_t k = 0; k < mult_src.size(); k++)
         build_mult_table(mult_src[k], reinterpret_cast<MultTable *>(s.host + hd.mult_off) + k);
     memcpy(s.host + hd.params_off, params, sizeof(int32_t) * (size_t)n * n_params);
+    {
+        int32_t *st = reinterpret_cast<int32_t *>(s.host + s.status_off);
+        for (int i = 0; i < n; i++) {
+            st[i] = descs[i].mode == FFCVB_MODE_JPG ? descs[i].host_status : 0;
+            st[n + i] = 0;
+        }
+    }
     for (int i = 0; i < n; i++) {
         // a sample decoded at reduced scale: its crop box, for the kernels, is the box of the scaled
         // image that covers it
@@ -1103,10 +1111,19 @@ int stage_impl(ffcvb_ctx *ctx, int slot, const Source &source, const uint64_t *p
         }
     }
     if (!jpeg_list.empty()) memcpy(s.host + s.jpeg_list_off, jpeg_list.data(), 4 * jpeg_list.size());
-    if (!par_list.empty()) memcpy(s.host + s.par_list_off, par_list.data(), 4 * par_list.size());
-    if (!seq_list.empty()) memcpy(s.host + s.seq_list_off, seq_list.data(), 4 * seq_list.size());
+    if (!multi.empty()) memcpy(s.host + s.multi_off, multi.data(), 4 * multi.size());
+    if (!restart.empty()) memcpy(s.host + s.restart_off, restart.data(), 4 * restart.size());
+    if (!segs.empty()) memcpy(s.host + s.segs_off, segs.data(), sizeof(uint2) * segs.size());
+    if (!blk_tiles.empty()) memcpy(s.host + s.block_tiles_off, blk_tiles.data(), sizeof(uint2) * blk_tiles.size());
     if (!quad_tiles.empty()) memcpy(s.host + s.quad_tiles_off, quad_tiles.data(), sizeof(uint2) * quad_tiles.size());
     s.n_quad_tiles = (int)quad_tiles.size();
+    s.n_block_tiles = (int)blk_tiles.size();
+    s.n_segs = (int)segs.size();
+    s.n_multi = (int)multi.size();
+    s.n_restart = (int)restart.size();
+    s.max_raw = max_raw;
+    s.max_tables = max_tables;
+    s.alike = alike;
 
     const auto t2 = std::chrono::steady_clock::now();
     // ---- parallel: gather the payload bytes into pinned memory
@@ -1155,10 +1172,7 @@ int stage_impl(ffcvb_ctx *ctx, int slot, const Source &source, const uint64_t *p
     if (from_fd || s.staged_end <= hd.payload_off) s.stage_ms[2] = 0; // else: written when the copy completes
     s.stage_ms[3] = ms(t0, t3);
     s.n_jpeg = (int)jpeg_list.size();
-    s.n_par = (int)par_list.size();
-    s.n_seq = (int)seq_list.size();
     s.total_blocks = total_blocks;
-    s.max_pixels = max_pixels;
     s.max_w = max_w;
     s.max_h = max_h;
     s.n_quad = n_quad;
@@ -1167,10 +1181,6 @@ int stage_impl(ffcvb_ctx *ctx, int slot, const Source &source, const uint64_t *p
     s.clean_bytes = clean_bytes;
     s.plane_bytes = plane_bytes;
     s.rgb_bytes = rgb_bytes;
-    {
-        const size_t need = entropy_checkpoint_bytes((int)par_list.size(), s.entropy_threads, s.subseq_bits);
-        if (need && (rc = grow_dev(ctx, s.ckpt, need))) return rc;
-    }
     s.scan_bytes = s.raw_bytes = s.jpeg_bytes = 0;
     for (int i = 0; i < n; i++) {
         if (descs[i].mode == FFCVB_MODE_JPG) {
@@ -1276,19 +1286,24 @@ static int run_batch(ffcvb_ctx *ctx, Slot &s, cudaStream_t st, void *out_dev, bo
     const HuffTable *huff = reinterpret_cast<const HuffTable *>(blob + hd.huff_off);
     const MultTable *mult = reinterpret_cast<const MultTable *>(blob + hd.mult_off);
     const int32_t *params = reinterpret_cast<const int32_t *>(blob + hd.params_off);
-    int32_t *status = (int32_t *)s.status.p;
-    CU(cudaMemsetAsync(status, 0, sizeof(int32_t) * (size_t)s.n, st));
+    int32_t *status = reinterpret_cast<int32_t *>(blob + s.status_off);
     if (s.n_jpeg > 0) {
         const int32_t *jl = reinterpret_cast<const int32_t *>(blob + s.jpeg_list_off);
-        const int32_t *pl = reinterpret_cast<const int32_t *>(blob + s.par_list_off);
-        const int32_t *sl = reinterpret_cast<const int32_t *>(blob + s.seq_list_off);
-        launch_entropy_decode(descs, pl, s.n_par, sl, s.n_seq, blob, huff, (uint8_t *)s.clean.p,
-                              (int16_t *)s.coef.p, status, s.subseq_bits, s.entropy_threads,
-                              s.subseq_bits > kMaxStagedBits ? s.ckpt.p : nullptr, (uint8_t *)ctx->index_pool.p,
-                              (unsigned long long *)ctx->index_stats.p, st);
+        EntropyScratch scratch{};
+        scratch.clean = (uint8_t *)s.clean.p;
+        scratch.seg_dc = (int32_t *)s.segs.p;
+        scratch.sub_info = (uint32_t *)(scratch.seg_dc + 4 * (size_t)s.n_segs);
+        scratch.meta = (SegMeta *)(scratch.sub_info + kSegSubs * (size_t)s.n_segs);
+        scratch.done = (uint32_t *)(status + s.n);
+        scratch.pos = (uint32_t *)s.index.p;
+        scratch.dc = (int16_t *)(scratch.pos + s.total_blocks);
+        launch_entropy_decode(descs, reinterpret_cast<const uint2 *>(blob + s.segs_off), s.n_segs,
+                              reinterpret_cast<const int32_t *>(blob + s.multi_off), s.n_multi,
+                              reinterpret_cast<const int32_t *>(blob + s.restart_off), s.n_restart, blob, huff, scratch, status,
+                              s.max_raw, s.max_tables, s.alike, (uint8_t *)ctx->index_pool.p, (unsigned long long *)ctx->index_stats.p, st);
         if (prof) CU(cudaEventRecord(s.ev[2], st));
-        launch_idct(descs, jl, s.n_jpeg, s.total_blocks, mult, (const int16_t *)s.coef.p,
-                    (uint8_t *)s.planes.p, st);
+        launch_blocks(descs, reinterpret_cast<const uint2 *>(blob + s.block_tiles_off), s.n_block_tiles, huff, mult, scratch,
+                      (uint8_t *)s.planes.p, st);
         if (prof) CU(cudaEventRecord(s.ev[3], st));
         launch_color(descs, jl, s.n_jpeg, s.n_quad, s.n_444, s.n_other, s.max_w, s.max_h,
                      reinterpret_cast<const uint2 *>(blob + s.quad_tiles_off), s.n_quad_tiles, (const uint8_t *)s.planes.p,
@@ -1487,7 +1502,7 @@ int ffcvb_batch_launches(const ffcvb_ctx *ctx, int slot) {
     if (!ctx || slot < 0 || slot >= (int)ctx->slots.size() || !ctx->slots[slot].staged) return -1;
     const Slot &s = ctx->slots[slot];
     int k = 1 + (s.direct ? 1 : 0); // fused resize/augment/normalise (+ payload gather)
-    if (s.n_jpeg > 0) k += 1 + (s.n_quad > 0) + (s.n_444 > 0) + (s.n_other > 0) + (s.n_par > 0) + (s.n_seq > 0);
+    k += (s.n_quad > 0) + (s.n_444 > 0) + (s.n_other > 0) + (s.n_block_tiles > 0) + 2 * (s.n_segs > 0) + (s.n_multi > 0) + (s.n_restart > 0);
     return k;
 }
 
@@ -1498,7 +1513,7 @@ int ffcvb_batch_status(ffcvb_ctx *ctx, int slot, void *stream, int32_t *status, 
     Slot &s = ctx->slots[slot];
     if (!s.staged || n > s.n) return fail(ctx, FFCVB_E_ARG, "ffcvb_batch_status: nothing staged");
     CU(cudaSetDevice(ctx->device));
-    CU(cudaMemcpyAsync(status, s.status.p, sizeof(int32_t) * (size_t)n, cudaMemcpyDeviceToHost,
+    CU(cudaMemcpyAsync(status, (const uint8_t *)s.blob.p + s.status_off, sizeof(int32_t) * (size_t)n, cudaMemcpyDeviceToHost,
                        (cudaStream_t)stream));
     CU(cudaStreamSynchronize((cudaStream_t)stream));
     int bad = 0;

@@ -1,25 +1,55 @@
-// Batched baseline-JPEG entropy decode (ITU-T T.81 F.2) for sm_100a.
+// Batched baseline-JPEG entropy decode (ITU-T T.81 F.2) for sm_100a: from a scan to the place of
+// every 8x8 block in it.
 //
-// One CTA per image.  The scan has no restart markers in FFCV-written files
-// (ffcv/fields/rgb_image.py:26-34 passes only the quality to cv2.imencode), so parallelism inside
-// an image comes from the self-synchronising property of Huffman codes: the unstuffed bit stream
-// is cut into fixed-length subsequences, every thread decodes its subsequence from a guessed
-// state, and the guesses are repaired by re-decoding from the left neighbour's exit state until
-// no input changes (a Jacobi iteration on a chain whose first link is exact, so it converges in
-// a few rounds in practice -- about 7 kbit of stream, dominated by the block's slot inside the
-// MCU -- and in at most one round per subsequence in the worst case).  A prefix sum
-// of completed blocks then gives every thread its output position and a last pass writes the
-// coefficients.  DC differences are integrated per component by a block-wide scan.
+// The scan has no restart markers in FFCV-written files (ffcv/fields/rgb_image.py:26-34 passes only
+// the quality to cv2.imencode), so parallelism inside an image comes from the self-synchronising
+// property of Huffman codes.  What these kernels produce is not coefficients but an index: for every
+// block the bit position of its first AC symbol in the unstuffed stream, and its DC value.  With it
+// the inverse transform (idct.cu) decodes any block on its own, in parallel and only where the crop
+// needs it, and no coefficient ever travels through global memory.
 //
-// Integer / issue-bound work: tables live in shared memory, no tensor cores.
+//   scan_sync_kernel    one CTA per segment of a scan (about 128 subsequences): removes the byte
+//                       stuffing, decodes every subsequence from a guessed state and repairs the
+//                       guesses by re-decoding from the left neighbour's exit state until nothing
+//                       changes.  A decoder that starts mid-stream falls in step after 0.9 kbit on
+//                       average (4:2:0, quality 90; 99 % within 4 kbit), dominated by the block's
+//                       slot inside the MCU, so two passes and a few stragglers settle a segment.
+//                       Segments behind the first decode the last 8 kbit before them as a run-up.
+//   scan_stitch_kernel  scans of several segments: where a run-up was too short, walks
+//                       on from the exact state until it meets the recorded one.
+//   scan_index_kernel   every subsequence once more from its exact state: records the blocks; the
+//                       last CTA of an image integrates the DC differences.
+//
+// Integer work bound by instruction issue at large batches and by the chain look-up -> shift ->
+// look-up at small ones: about 25 instructions per symbol and lane, tables and stream in shared memory.
+#include "huffman.h"
 #include "kernels.h"
 
 namespace ffcvb {
 
+namespace {
 
-// Exclusive prefix sum over the block; `total` receives the block sum.  s_warp holds 33 ints.
-__device__ __forceinline__ int block_scan_exclusive(int v, int *s_warp, int &total) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
+constexpr int kThreads = kSegSubs;          // one thread per subsequence: a team of four warps per segment
+constexpr int kFastBytes = 2 * kHuffFast;   // a Huffman table in shared memory
+
+// The threads that work on one segment.  A CTA holds one team, or several that share the Huffman
+// tables in shared memory and meet at barriers of their own.
+template <int TEAMS>
+struct Team {
+    int index, tid;
+    __device__ __forceinline__ Team() : index(TEAMS == 1 ? 0 : threadIdx.x / kThreads), tid(TEAMS == 1 ? threadIdx.x : threadIdx.x % kThreads) {}
+    __device__ __forceinline__ void sync() const {
+        if (TEAMS == 1)
+            __syncthreads();
+        else
+            asm volatile("bar.sync %0, %1;" ::"r"(index + 1), "n"(kThreads) : "memory");
+    }
+};
+
+// Exclusive prefix sum over `warps` warps that meet at `sync`; `total` receives the sum.
+template <class Sync>
+__device__ __forceinline__ int scan_exclusive(int v, int tid, int warps, int *s_warp, int &total, Sync &&sync) {
+    const int lane = tid & 31, warp = tid >> 5;
     int inc = v;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
@@ -27,623 +57,629 @@ __device__ __forceinline__ int block_scan_exclusive(int v, int *s_warp, int &tot
         if (lane >= o) inc += t;
     }
     if (lane == 31) s_warp[warp] = inc;
-    __syncthreads();
-    if (warp == 0) {
-        int w = lane < nwarps ? s_warp[lane] : 0;
-        int winc = w;
+    sync();
+    int before = 0, all = 0;
 #pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            int t = __shfl_up_sync(0xffffffffu, winc, o);
-            if (lane >= o) winc += t;
-        }
-        s_warp[lane] = winc - w;
-        if (lane == 31) s_warp[32] = winc;
+    for (int k = 0; k < warps; k++) {
+        const int w = s_warp[k];
+        before += k < warp ? w : 0;
+        all += w;
     }
-    __syncthreads();
-    int r = inc - v + s_warp[warp];
-    total = s_warp[32];
-    __syncthreads();
-    return r;
+    sync();
+    total = all;
+    return before + inc - v;
+}
+template <int TEAMS>
+__device__ __forceinline__ int team_scan(const Team<TEAMS> &team, int v, int *s_warp, int &total) {
+    return scan_exclusive(v, team.tid, kThreads / 32, s_warp, total, [&] { team.sync(); });
 }
 
-// 32 bits of the bit stream starting at bit p.  The unstuffed stream is stored as 32-bit words
-// whose most significant bit comes first, so two word loads and one funnel shift do it.
-__device__ __forceinline__ uint32_t peek32(const uint32_t *__restrict__ words, uint32_t p) {
-    const uint32_t i = p >> 5;
-    return __funnelshift_l(words[i + 1], words[i], p);
+__device__ __forceinline__ uint32_t shared_address(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
+__device__ __forceinline__ uint32_t load_shared(uint32_t a) {
+    uint32_t v;
+    asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(a));
+    return v;
 }
 
-// A 96-bit window over the stream kept in registers: hi holds the word the current position lies
-// in, lo the next one, nx the one after.  Looking at the next 32 bits is one funnel shift, and the
-// stream is touched once per 32 bits consumed (a predicated load, issued a symbol or more before
-// its value is needed) instead of twice per symbol, which takes the stream's load latency out of
-// the chain symbol -> table look-up -> next symbol.  Lanes never diverge: advancing is a select.
-struct BitWindow {
-    const uint32_t *__restrict__ w;
-    uint32_t wi, r, hi, lo, nx;
-    __device__ __forceinline__ BitWindow(const uint32_t *__restrict__ words, uint32_t p) : w(words), wi(p >> 5), r(p & 31) {
-        hi = w[wi];
-        lo = w[wi + 1];
-        nx = w[wi + 2];
-    }
-    __device__ __forceinline__ uint32_t peek() const { return __funnelshift_l(lo, hi, r); }
-    // consume n < 32 bits
-    __device__ __forceinline__ void skip(uint32_t n) {
-        r += n;
-        const bool adv = r >= 32;
-        hi = adv ? lo : hi;
-        lo = adv ? nx : lo;
-        wi += adv ? 1u : 0u;
-        r &= 31;
-        if (adv) nx = w[wi + 2];
-    }
+// Global to shared memory without passing through registers; copies_wait: this thread's have landed.
+__device__ __forceinline__ void copy16_async(void *dst, const void *src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(shared_address(dst)), "l"(src) : "memory");
+}
+__device__ __forceinline__ void copies_wait() {
+    asm volatile("cp.async.commit_group;" ::: "memory");
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+}
+
+// Tables of an image in shared memory: for every block slot of an MCU where its Huffman tables are
+// and which slot follows, then HuffTable::fast of the image's distinct tables (DC, then AC), then
+// HuffTable::pair of the AC tables.
+struct Slot {
+    uint32_t tables; // shared-memory address of the DC table | of the AC table << 16
+    uint32_t next;   // shared-memory address of the slot that follows
 };
+struct Tables {
+    Slot slot[6];
+    uint32_t bpm, luma, pairs, pad; // blocks of an MCU, luma blocks among them; from an AC table to its pair table
+    uint16_t fast[8];               // (the first vector of the tables)
+};
+constexpr size_t kTablesHead = offsetof(Tables, fast);
+static_assert(kTablesHead % 16 == 0 && kFastBytes % 16 == 0 && offsetof(HuffTable, fast) % 16 == 0 && offsetof(HuffTable, pair) % 16 == 0,
+              "tables are copied in vectors");
+__host__ __device__ constexpr size_t tables_bytes(int n_tables) { return kTablesHead + (size_t)n_tables * kFastBytes; }
 
-// Entry (see HuffTable) of the Huffman code at the top of w: at most two dependent table reads.
-// An invalid code consumes 16 bits and acts as an end of block, so that speculative decoding
-// always makes progress.
-__device__ __forceinline__ uint32_t huff_lookup(const HuffTable &t, uint32_t w) {
-    uint32_t e = t.look[w >> 23];
-    if (e & 0x8000u) {
-        if (e != 0xFFFFu) {
-            e = t.sub[e & 0x7fffu][(w >> 16) & 127];
-        } else {
-            // more long-code prefixes than sub-tables (never with the tables encoders emit)
-            const int code = w >> 16;
-            e = 16u | (63u << 9); // no code at all: a 16-bit end of block
-#pragma unroll 1
-            for (int l = 10; l <= 16; l++) {
-                const int c = code >> (16 - l);
-                if (c <= t.maxcode[l]) {
-                    e = huff_entry(l, t.vals[(t.valoff[l] + c) & 255]);
-                    break;
-                }
-            }
+// Starts the copies of the tables; copies_wait and a barrier of the whole CTA complete them.
+__device__ __forceinline__ void load_tables(Tables *s, const ImageDesc &d, const HuffTable *__restrict__ huff) {
+    const int luma = d.hs * d.vs, n = d.n_tab, n_dc = d.n_dc_tab, tid = threadIdx.x;
+    const uint32_t fast = shared_address(s->fast);
+    if (d.fast_tables)
+        for (int u = 0; u < 2 * n - n_dc; u++) {
+            const HuffTable &t = huff[d.tab_id[u < n ? u : u - (n - n_dc)]];
+            const uint4 *src = reinterpret_cast<const uint4 *>(u < n ? t.fast : t.pair);
+            uint4 *dst = reinterpret_cast<uint4 *>(s->fast) + u * (kFastBytes / 16);
+            for (int i = tid; i < kFastBytes / 16; i += blockDim.x) copy16_async(dst + i, src + i);
         }
+    if (tid < d.bpm) {
+        const int comp = (d.ncomp == 1 || tid < luma) ? 0 : tid - luma + 1;
+        s->slot[tid].tables = (fast + d.dc_tab[comp] * (uint32_t)kFastBytes) | (fast + d.ac_tab[comp] * (uint32_t)kFastBytes) << 16;
+        s->slot[tid].next = shared_address(&s->slot[tid + 1 == d.bpm ? 0 : tid + 1]);
     }
-    return e;
+    if (tid == 0) {
+        s->bpm = d.bpm;
+        s->luma = d.ncomp == 1 ? 1 : luma;
+        s->pairs = (uint32_t)((n - n_dc) * kFastBytes);
+    }
 }
 
-__device__ __forceinline__ int extend(uint32_t bits, int s) {
-    // bits: the s-bit magnitude field (s >= 1)
-    return bits < (1u << (s - 1)) ? (int)bits - (1 << s) + 1 : (int)bits;
-}
-
+// Decoder state between two symbols: bit position, block slot inside the MCU, next zig-zag index
+// (0: DC expected).
 struct Cursor {
-    uint32_t p; // bit position in the unstuffed stream
-    int c;      // block slot inside the MCU
-    int z;      // next zigzag index, 0 = DC expected
+    uint32_t p;
+    int c, z;
 };
+// Packed into 16 bits relative to a position `from` that the cursor has reached by less than 32 bits.
+__device__ __forceinline__ uint32_t pack(const Cursor &s, uint32_t from) { return (s.p - from) | (uint32_t)s.c << 5 | (uint32_t)s.z << 8; }
+__device__ __forceinline__ Cursor unpack(uint32_t v, uint32_t from) { return Cursor{from + (v & 31), (int)((v >> 5) & 7), (int)((v >> 8) & 63)}; }
 
-__device__ __forceinline__ uint64_t pack(const Cursor &s) {
-    return ((uint64_t)s.p << 32) | ((uint32_t)s.c << 8) | (uint32_t)s.z;
-}
-__device__ __forceinline__ Cursor unpack(uint64_t v) {
-    Cursor s;
-    s.p = (uint32_t)(v >> 32);
-    s.c = (int)((v >> 8) & 0xffffff);
-    s.z = (int)(v & 0xff);
-    return s;
-}
-
-// Decodes symbols from `cur` until its position reaches `end`.  Returns the number of blocks
-// completed.  With WRITE, coefficients go to cf (image base) starting at block `blk`.
-// `words` holds the stream from bit `bit_base` on (the chunk's copy in shared memory).
-// The 32 lanes of a warp walk unrelated parts of the stream, so the step is written as straight
-// line code with selects (DC / AC / end-of-block / zero-run / block end all take the same path);
-// codes longer than the 9-bit first-level table cost one more table read.
-template <bool WRITE>
-__device__ __forceinline__ int decode_span(const uint32_t *__restrict__ words, uint32_t bit_base, Cursor &cur,
-                                           uint32_t end, int bpm, int luma, int ncomp,
-                                           const HuffTable *s_tab,
-                                           int16_t *__restrict__ cf, uint32_t blk,
-                                           uint32_t nblocks) {
-    int done = 0;
-    uint32_t p = cur.p;
-    int c = cur.c, z = cur.z;
-    int comp2 = (ncomp == 1 || c < luma) ? 0 : 2 * (c - luma + 1);
-    int16_t *out = cf + (size_t)blk * 64;
-    if (p >= end) return 0;
-    // Coefficients are stored in the order they are decoded (zig-zag order inside a block; the
-    // inverse transform undoes it when it loads the block), which lets a thread collect the four
-    // coefficients of an aligned group of zig-zag positions in a register and store them with one
-    // 8-byte store: a block's ~15 non-zero coefficients sit in ~5 such groups, and scattered stores
-    // are what the write pass is bound by.  Only a block this thread decodes from its first symbol
-    // is packed: a block shared with a neighbouring subsequence is written coefficient by
-    // coefficient, so that the two threads never touch the same bytes.
-    bool packing = z == 0;
-    int group = -1; // group of four positions held in `held`, -1: none
-    unsigned long long held = 0;
-    BitWindow win(words, p - bit_base);
-    while (p < end) {
-        const uint32_t w = win.peek();
-        const bool dc = z == 0;
-        const HuffTable &t = s_tab[comp2 + (dc ? 0 : 1)];
-        const uint32_t e = huff_lookup(t, w);
-        const int n = e & 31, s = (e >> 5) & 15;
-        const int zn = dc ? 1 : z + (int)(e >> 9); // DC: on to the first AC position
-        if (WRITE) {
-            // where this symbol's coefficient goes, if it has one
-            const int zpos = zn - 1;
-            if (s != 0 && zpos < 64 && blk < nblocks) {
-                const int v = extend((w << (n - s)) >> (32 - s), s);
-                if (packing) {
-                    const int g = zpos >> 2;
-                    if (g != group) {
-                        if (group >= 0) *reinterpret_cast<unsigned long long *>(out + 4 * group) = held;
-                        group = g;
-                        held = 0;
-                    }
-                    held |= (unsigned long long)(uint16_t)v << (16 * (zpos & 3));
-                } else {
-                    out[zpos] = (int16_t)v;
-                }
-            }
+// The walk below in plain code: for tables that are not fast_ok, and for the few walks on a stream in
+// global memory.  One symbol at a time, tables where they are.
+template <bool RECORD>
+__device__ __noinline__ uint32_t walk_plain(const uint32_t *words, Cursor &cur, uint32_t end, const ImageDesc &d,
+                                            const HuffTable *__restrict__ huff, uint32_t *pos, uint32_t blk, uint32_t limit) {
+    const int luma = d.ncomp == 1 ? 1 : d.hs * d.vs;
+    uint32_t done = 0;
+    while (cur.p < end) {
+        if (RECORD && cur.z == 0) {
+            if (blk < limit) pos[blk] = cur.p;
+            blk++;
         }
-        p += n;
-        win.skip(n);
-        const bool eob = zn >= 64;
-        z = eob ? 0 : zn;
-        done += eob ? 1 : 0;
-        if (WRITE) {
-            if (eob) {
-                if (group >= 0) *reinterpret_cast<unsigned long long *>(out + 4 * group) = held;
-                group = -1;
-                packing = true;
-            }
-            blk += eob ? 1 : 0;
-            out += eob ? 64 : 0;
-        }
-        c = eob ? ((c + 1 == bpm) ? 0 : c + 1) : c;
-        comp2 = (ncomp == 1 || c < luma) ? 0 : 2 * (c - luma + 1);
-    }
-    if (WRITE && group >= 0) {
-        // the subsequence ends inside a block: the next thread continues it, so only the
-        // coefficients themselves are written
-#pragma unroll
-        for (int k = 0; k < 4; k++) {
-            const uint32_t lane = (uint32_t)(held >> (16 * k)) & 0xffffu;
-            if (lane) out[4 * group + k] = (int16_t)lane;
+        const uint32_t w = __funnelshift_l(words[(cur.p >> 5) + 1], words[cur.p >> 5], cur.p);
+        const int comp = cur.c < luma ? 0 : cur.c - luma + 1;
+        const HuffTable *t = huff + d.tab_id[cur.z ? d.ac_tab[comp] : d.dc_tab[comp]];
+        uint32_t e = t->look[w >> (32 - kHuffBits)];
+        if (e & kHuffLong) e = huff_long(t, e, w);
+        cur.p += e & 31;
+        cur.z += (int)(e >> 9);
+        if (cur.z >= 64) {
+            cur.z = 0;
+            cur.c = cur.c + 1 == d.bpm ? 0 : cur.c + 1;
+            done++;
         }
     }
-    cur.p = p;
-    cur.c = c;
-    cur.z = z;
     return done;
 }
 
-// Counting walk for long subsequences (the variant that reads the stream from global memory).
-// A re-decode of a long subsequence from a corrected entry state soon runs exactly where the
-// previous decode ran: the two walks merge once position, slot and zig-zag index coincide.  Every
-// walk therefore leaves its state at check-points every `ck_bits` bits; a later walk that finds
-// the same state at a check-point stops there -- the exit state stands and the block count is its
-// own count so far plus what the previous walk counted from that check-point to the end.  The repair pass
-// of a multi-megabit image then costs the re-synchronisation distance, not the whole subsequence.
-struct CheckPoint {
-    unsigned long long state; // pack(position, slot, zig-zag index)
-    uint32_t rest;            // blocks the walk completed from here to the end of the subsequence
-    uint32_t pad;
-};
-
-template <bool COMPARE>
-__device__ __forceinline__ int count_span_checked(const uint32_t *__restrict__ words, Cursor &cur, uint32_t start,
-                                                  uint32_t end, int bpm, int luma, int ncomp,
-                                                  const HuffTable *s_tab, CheckPoint *__restrict__ ck, uint32_t ck_bits,
-                                                  bool &merged) {
-    int done = 0;
+// Decodes symbols from `cur` until its position reaches `end`; returns the number of blocks
+// completed.  `buf`: the segment's stream in shared memory (words most significant bit first).  With
+// RECORD every block that begins before `end` gets its position written to pos[blk], pos[blk + 1],
+// ... below pos[limit]; `blk` is the first of them.
+//
+// The 32 lanes of a warp walk unrelated places, so nothing in the loops branches: position (bits 0-17)
+// and zig-zag index (bits 24-30) share one word that an entry is simply added to; a 96-bit window over
+// the stream stays in registers (hi holds the word the position lies in, lo and nx the two behind it)
+// and is moved on by predicated instructions; so are the table switches and the slot at the end of a
+// block; codes too long for the first level are reached by the index's maximum.  As long as `end` is
+// more than kHuffBits away an entry may stand for two symbols (1.46 on average), so that the walk's
+// last position is the same whatever state it came from.
+constexpr uint32_t kPosMask = 0x3ffff;
+template <bool RECORD>
+__device__ __forceinline__ uint32_t walk(const unsigned char *buf, Cursor &cur, uint32_t end, const Tables *s, const ImageDesc &d,
+                                         const HuffTable *__restrict__ huff, uint32_t *pos = nullptr, uint32_t blk = 0, uint32_t limit = 0) {
+    if (cur.p >= end) return 0;
+    if (!d.fast_tables) return walk_plain<RECORD>(reinterpret_cast<const uint32_t *>(buf), cur, end, d, huff, pos, blk, limit);
+    const uint32_t pairs = s->pairs;
+    uint32_t st = cur.p | (uint32_t)cur.z << 24, done = 0;
+    const Slot here = s->slot[cur.c];
+    uint32_t ac = here.tables >> 16, tab = cur.z ? ac : here.tables & 0xffff;
+    uint32_t ahead = load_shared(here.next), after = load_shared(here.next + 4); // the slot that follows
+    uint32_t wa = shared_address(buf) + (cur.p >> 5) * 4;
+    uint32_t hi = load_shared(wa), lo = load_shared(wa + 4), nx = load_shared(wa + 8);
+    wa += 12;
+    if (RECORD && cur.z == 0) {
+        if (blk < limit) pos[blk] = cur.p;
+        blk++;
+    }
     uint32_t p = cur.p;
-    int c = cur.c, z = cur.z;
-    int comp2 = (ncomp == 1 || c < luma) ? 0 : 2 * (c - luma + 1);
-    const uint32_t k0 = (p - start) / ck_bits;
-    uint32_t k = k0;
-    uint32_t next_ck = start + (k + 1) * ck_bits;
-    int total = -1;
-    merged = false;
-    BitWindow win(words, p < end ? p : 0);
-    while (p < end) {
-        const uint32_t w = win.peek();
-        const bool dc = z == 0;
-        const HuffTable &t = s_tab[comp2 + (dc ? 0 : 1)];
-        const uint32_t e = huff_lookup(t, w);
-        const int zn = dc ? 1 : z + (int)(e >> 9);
-        p += e & 31;
-        win.skip(e & 31);
-        const bool eob = zn >= 64;
-        z = eob ? 0 : zn;
-        done += eob ? 1 : 0;
-        c = eob ? ((c + 1 == bpm) ? 0 : c + 1) : c;
-        comp2 = (ncomp == 1 || c < luma) ? 0 : 2 * (c - luma + 1);
-        if (p >= next_ck && p < end) {
-            Cursor here = {p, c, z};
-            const unsigned long long st = pack(here);
-            if (COMPARE && ck[k].state == st) {
-                merged = true; // from here on this walk is the previous one
-                total = done + (int)ck[k].rest;
-                break;
-            }
-            ck[k].state = st;
-            ck[k].rest = (uint32_t)done; // blocks so far; turned into blocks-to-the-end below
-            k++;
-            next_ck += ck_bits;
+    auto symbol = [&](bool live, bool paired) { // (not live: nothing moves)
+        const uint32_t w = __funnelshift_l(lo, hi, st);
+        const uint32_t index = (uint32_t)__viaddmax_s32((int)(w >> 16), kHuffFast - 65536, (int)(w >> 22));
+        uint32_t e = 0;
+        asm volatile("{\n\t"
+                     ".reg .pred q;\n\t"
+                     "setp.ne.u32 q, %2, 0;\n\t"
+                     "@q ld.shared.u16 %0, [%1];\n\t"
+                     "}"
+                     : "+r"(e)
+                     : "r"(tab + index * 2), "r"((uint32_t)live));
+        e = __byte_perm(e, 0, 0x1440); // bits consumed to bits 0-7, positions advanced to bits 24-31
+        const uint32_t before = st;
+        st += e;
+        asm volatile("{\n\t"
+                     ".reg .pred q;\n\t"
+                     ".reg .b32 t;\n\t"
+                     "xor.b32 t, %4, %5;\n\t"
+                     "and.b32 t, t, 32;\n\t"
+                     "setp.ne.u32 q, t, 0;\n\t"
+                     "@q mov.b32 %0, %1;\n\t"
+                     "@q mov.b32 %1, %2;\n\t"
+                     "@q ld.shared.u32 %2, [%3];\n\t"
+                     "@q add.u32 %3, %3, 4;\n\t"
+                     "}"
+                     : "+r"(hi), "+r"(lo), "+r"(nx), "+r"(wa)
+                     : "r"(before), "r"(st));
+        // (closer to the block's end a pair might reach beyond it with its first symbol)
+        const uint32_t to = ac + (paired && st < (uint32_t)(64 - kPairAdvance) << 24 ? pairs : 0);
+        tab = live ? to : tab;
+        const bool eob = st >= 0x40000000u;
+        asm volatile("{\n\t"
+                     ".reg .pred q;\n\t"
+                     "setp.ge.u32 q, %0, 0x40000000;\n\t"
+                     "@q and.b32 %0, %0, 0x3ffff;\n\t"
+                     "@q add.u32 %1, %1, 1;\n\t"
+                     "@q and.b32 %2, %4, 0xffff;\n\t"
+                     "@q shr.u32 %3, %4, 16;\n\t"
+                     "@q ld.shared.v2.u32 {%4, %5}, [%5];\n\t"
+                     "}"
+                     : "+r"(st), "+r"(done), "+r"(tab), "+r"(ac), "+r"(ahead), "+r"(after));
+        p = st & kPosMask;
+        if (RECORD) {
+            if (eob && p < end && blk < limit) pos[blk] = p;
+            blk += eob ? 1 : 0;
         }
+    };
+    const int pairs_end = (int)end - kHuffBits; // the first symbol of a pair that begins up to here ends before `end`
+    if ((int)p <= pairs_end) {
+        do {
+            symbol(true, true);
+            symbol((int)p <= pairs_end, true);
+        } while ((int)p <= pairs_end);
+        if (st >> 24) tab = ac; // (at 0 it is the DC table)
     }
-    if (!merged) {
-        total = done;
-        cur.p = p;
-        cur.c = c;
-        cur.z = z;
-    }
-    for (uint32_t j = k0; j < k; j++) ck[j].rest = (uint32_t)total - ck[j].rest;
-    return total;
+    while (p < end) symbol(true, false);
+    cur.p = p;
+    cur.z = (int)(st >> 24);
+    cur.c = (int)((cur.c + done) % s->bpm);
+    return done;
 }
 
-// kStaged: the chunk's bits are copied to shared memory first (subsequences of up to 1280 bits);
-// otherwise the threads read the unstuffed stream in global memory, which allows subsequences of
-// any length: a multi-megabit image is then one chunk of kEntropyThreads long subsequences that
-// re-synchronise in two or three (long, fully parallel) rounds instead of dozens of chunks that
-// wait for one another.
-template <int kEntropyThreads, bool kStaged>
-// (resident CTAs per SM: shared memory -- 27 KB of tables plus the stream -- allows 2 CTAs of 512
-// threads, 3 of 256 and 4 of 128 in the staged variants, so the register budget is set for those
-// counts rather than for full thread occupancy)
-__global__ void __launch_bounds__(kEntropyThreads, kEntropyThreads >= 1024 ? 1 : (kEntropyThreads == 512 ? 2 : (kEntropyThreads == 256 ? 4 : 6)))
-entropy_parallel_kernel(const ImageDesc *__restrict__ descs, const int32_t *__restrict__ list,
-                        const uint8_t *__restrict__ blob, const HuffTable *__restrict__ huff,
-                        uint8_t *__restrict__ clean, int16_t *__restrict__ coef,
-                        int32_t *__restrict__ status, int subseq_bits, CheckPoint *__restrict__ ckpt, int ck_bits,
-                        uint8_t *__restrict__ index_pool, unsigned long long *__restrict__ index_stats) {
-    extern __shared__ __align__(16) uint32_t s_stream[]; // this chunk of the unstuffed stream
-    __shared__ HuffTable s_tab[6];
-    __shared__ unsigned long long s_state[kEntropyThreads + 1];
-    __shared__ uint16_t s_blocks[kEntropyThreads]; // blocks completed inside each subsequence
-    __shared__ uint16_t s_list[kEntropyThreads];   // compacted indices of the dirty subsequences
-    __shared__ uint8_t s_dirty[kEntropyThreads + 1];
-    __shared__ int s_warp[33];
-    __shared__ uint32_t s_ix[2]; // decisions about the decode index, taken by one thread for the whole CTA
+// ---- byte stuffing -------------------------------------------------------------------------
+// Bytes of y (little-endian word x of the scan, prev: the byte before it) that are to be dropped: a
+// 00 behind an FF.  Bit 8k + 7 is set for byte k.
+__device__ __forceinline__ uint32_t stuffing_of(uint32_t x, uint32_t prev_word) {
+    const uint32_t y = x | ~__funnelshift_l(prev_word, x, 8); // a byte is 0 where x is 00 and its predecessor FF
+    return ~(((y & 0x7f7f7f7fu) + 0x7f7f7f7fu) | y | 0x7f7f7f7fu);
+}
+// The first k bytes of a word (as the flags above); k <= 0: none, k >= 4: all.
+__device__ __forceinline__ uint32_t first_bytes(int k) {
+    return k <= 0 ? 0u : (k >= 4 ? 0x80808080u : 0x80808080u >> (8 * (4 - k)));
+}
 
-    const int img = list[blockIdx.x];
-    const ImageDesc d = descs[img];
-    const int tid = threadIdx.x;
-    if (d.host_status != 0) {
-        if (tid == 0) status[img] = d.host_status;
-        return;
-    }
-    // ---- tables into shared memory
-    for (int c = 0; c < d.ncomp; c++) {
-        const uint32_t *sd = reinterpret_cast<const uint32_t *>(&huff[d.dc_tab[c]]);
-        const uint32_t *sa = reinterpret_cast<const uint32_t *>(&huff[d.ac_tab[c]]);
-        uint32_t *dd = reinterpret_cast<uint32_t *>(&s_tab[2 * c]);
-        uint32_t *da = reinterpret_cast<uint32_t *>(&s_tab[2 * c + 1]);
-        for (int i = tid; i < (int)(sizeof(HuffTable) / 4); i += kEntropyThreads) {
-            dd[i] = sd[i];
-            da[i] = sa[i];
-        }
-    }
-
-    // ---- remove byte stuffing (FF 00 -> FF) into the clean stream.  When the whole scan fits the
-    // shared-memory stream buffer (the usual case: the subsequence length is chosen so that the
-    // largest image of the batch is one chunk) the clean stream is built there and never touches
-    // global memory; otherwise it goes to the scratch buffer and is staged chunk by chunk.
-    const uint8_t *scan = blob + d.payload_off + d.scan_off;
-    const uint32_t stream_bytes = kStaged ? ((uint32_t)kEntropyThreads * (uint32_t)subseq_bits / 8 + 63) / 16 * 16 + 16 : 0;
-    const bool resident = kStaged && d.scan_len + 80 <= stream_bytes; // 64 zero bytes follow the stream
-    uint8_t *cl = resident ? reinterpret_cast<uint8_t *>(s_stream) : clean + d.clean_off;
-    uint32_t clean_len = 0, flush_base = 0;
-    // Every thread takes one aligned 16-byte word of the scan per pass (one load instead of sixteen);
-    // the byte before it, which decides whether a leading 00 is stuffing, comes from the lane below.
-    const uint32_t lead = (uint32_t)(reinterpret_cast<uintptr_t>(scan) & 15); // bytes of the first word before the scan
-    const uint4 *scan16 = reinterpret_cast<const uint4 *>(scan - lead);
-    for (uint32_t base = 0; base < d.scan_len + lead; base += kEntropyThreads * 16) {
-        const uint32_t chunk = base + tid * 16;         // offset of this thread's word from scan - lead
-        const int my = (int)chunk - (int)lead;           // scan offset of its first byte (negative in the first word)
-        uint4 v = make_uint4(0, 0, 0, 0);
-        if (chunk < d.scan_len + lead) v = scan16[chunk >> 4];
-        const uint32_t wv[4] = {v.x, v.y, v.z, v.w};
-        uint8_t b[16];
+// Unstuffs `len` raw bytes at `src` into `buf` (shared memory; room for len + 64 bytes and a word), most
+// significant byte of every word first, followed by 64 zero bytes.  `first`: nothing precedes the
+// bytes.  s_mark[k] receives how many kept bytes lie before raw offset at[k].  Returns the number of
+// bytes kept.  A thread takes 32 aligned bytes per pass; nearly all words lose nothing and leave as
+// one shifted word, single bytes are stored only where two threads' bytes share a word.
+template <int TEAMS>
+__device__ __forceinline__ uint32_t unstuff(const Team<TEAMS> &team, unsigned char *buf, const uint8_t *__restrict__ src, uint32_t len,
+                                            bool first, const uint32_t (&at)[2], int *s_warp, uint32_t *s_mark) {
+    constexpr int kWords = 8;
+    const int tid = team.tid;
+    const uint32_t lead = (uint32_t)(reinterpret_cast<uintptr_t>(src) & 15);
+    const uint8_t *aligned = src - lead;
+    const uint32_t nwords = ((lead + len + 15) >> 4) * 4;
+    uint32_t *words = reinterpret_cast<uint32_t *>(buf);
+    uint32_t kept = 0;
+    uint4 v[2];
+    auto fetch = [&](uint32_t w) {
 #pragma unroll
-        for (int i = 0; i < 16; i++) b[i] = (uint8_t)(wv[i >> 2] >> (8 * (i & 3)));
-        int prev = __shfl_up_sync(0xffffffffu, (int)b[15], 1);
-        if ((tid & 31) == 0) prev = (my > 0 && my <= (int)d.scan_len) ? scan[my - 1] : 0;
-        uint32_t keep = 0;
+        for (int k = 0; k < 2; k++) v[k] = w + 4 * k < nwords ? reinterpret_cast<const uint4 *>(aligned)[(w >> 2) + k] : make_uint4(0, 0, 0, 0);
+    };
+    fetch(tid * kWords);
+    for (uint32_t tile = 0; tile < nwords; tile += kThreads * kWords) {
+        const uint32_t w0 = tile + tid * kWords;
+        uint32_t x[kWords] = {v[0].x, v[0].y, v[0].z, v[0].w, v[1].x, v[1].y, v[1].z, v[1].w};
+        fetch(w0 + kThreads * kWords); // the next pass's bytes arrive during this one
+        const int off = (int)(w0 * 4) - (int)lead; // raw offset of the first of these bytes
+        const bool edge = off < 0 || off + kWords * 4 > (int)len;
+        if (first && off < 0) // what lies in front of the scan is no predecessor
 #pragma unroll
-        for (int i = 0; i < 16; i++) {
-            const int at = my + i;
-            const bool inside = at >= 0 && at < (int)d.scan_len;
-            if (inside && !(b[i] == 0 && prev == 0xFF)) keep |= 1u << i;
-            prev = inside ? b[i] : 0;
+            for (int k = 0; k < 4; k++) x[k] &= ~((first_bytes(-(off + 4 * k)) >> 7) * 255u);
+        uint32_t prev = __shfl_up_sync(0xffffffffu, x[kWords - 1], 1);
+        if ((tid & 31) == 0) prev = w0 < nwords && (w0 > 0 || (lead == 0 && !first)) ? (uint32_t)aligned[(int)(w0 * 4) - 1] << 24 : 0;
+        uint32_t keep[kWords];
+        int cnt = 0;
+#pragma unroll
+        for (int k = 0; k < kWords; k++) {
+            keep[k] = ~stuffing_of(x[k], k == 0 ? prev : x[k - 1]) & 0x80808080u;
+            if (edge) keep[k] &= ~first_bytes(-(off + 4 * k)) & first_bytes((int)len - (off + 4 * k));
+            cnt += __popc(keep[k]);
         }
         int total;
-        int off = block_scan_exclusive(__popc(keep), s_warp, total);
-        // byte k of the stream lives at address k ^ 3: every 32-bit word holds its bits MSB first
-        uint32_t o = clean_len + off;
-        if (kStaged) {
-            // into the stream buffer in shared memory (or, for the rare scan that does not fit it,
-            // byte by byte into the scratch buffer)
+        const uint32_t o = kept + (uint32_t)team_scan(team, cnt, s_warp, total);
 #pragma unroll
-            for (int i = 0; i < 16; i++)
-                if (keep & (1u << i)) cl[(o++) ^ 3u] = b[i];
-        } else {
-            // The variant for multi-megabit scans keeps the stream in global memory: it is collected
-            // in shared memory first and leaves as whole 16-byte vectors, one store per 16 bytes
-            // instead of one per byte.  flush_base (a multiple of 16) is the stream
-            // position of the buffer's first byte; fewer than 16 bytes stay behind per pass.
-            uint8_t *buf = reinterpret_cast<uint8_t *>(s_stream);
+        for (int m = 0; m < 2; m++) {
+            const int a = (int)at[m] - off;
+            if (a >= 0 && a < kWords * 4) { // raw offset at[m] is one of these bytes
+                uint32_t n = o;
 #pragma unroll
-            for (int i = 0; i < 16; i++)
-                if (keep & (1u << i)) buf[((o++) - flush_base) ^ 3u] = b[i];
-            __syncthreads();
-            const uint32_t have = clean_len + (uint32_t)total - flush_base, nvec = have >> 4;
-            uint4 *dst16 = reinterpret_cast<uint4 *>(cl + flush_base);
-            const uint4 *src16 = reinterpret_cast<const uint4 *>(buf);
-            for (uint32_t k = tid; k < nvec; k += kEntropyThreads) dst16[k] = src16[k];
-            uint4 rest = make_uint4(0, 0, 0, 0);
-            if (tid == 0) rest = src16[nvec];
-            __syncthreads();
-            if (tid == 0) reinterpret_cast<uint4 *>(buf)[0] = rest; // the incomplete vector moves to the front
-            flush_base += nvec << 4;
-            // (the next pass's block scan has barriers between this store and the first byte written)
+                for (int k = 0; k < kWords; k++) n += __popc(keep[k] & first_bytes(a - 4 * k));
+                s_mark[m] = n;
+            }
         }
-        clean_len += total;
+        // `acc` holds the bytes of word wi this thread has so far, ph bits of the word are taken (by it
+        // or by the thread before it)
+        uint32_t ph = (o & 3) * 8, acc = 0, wi = o >> 2, mine = o & 3; // bytes below `mine` are another thread's
+        auto store = [&](uint32_t upto) {
+            if (mine == 0 && upto == 4)
+                words[wi] = acc;
+            else
+                for (uint32_t q = mine; q < upto; q++) buf[(wi * 4 + q) ^ 3u] = (uint8_t)(acc >> (24 - 8 * q));
+            mine = 0;
+            wi++;
+        };
+#pragma unroll
+        for (int k = 0; k < kWords; k++) {
+            uint32_t b = __byte_perm(x[k], 0, 0x0123), bits = 32;
+            if (keep[k] != 0x80808080u) { // close the gaps, last byte first
+                bits = 8 * __popc(keep[k]);
+#pragma unroll 1
+                for (uint32_t gone = ~keep[k] & 0x80808080u; gone != 0; gone &= gone - 1) {
+                    // the dropped byte with the lowest address not yet dealt with is the one nearest the top
+                    const uint32_t q = (__ffs(gone) - 1) & ~7u, shift = q - (8 * __popc(~keep[k] & 0x80808080u & ((gone & (0u - gone)) - 1)));
+                    const uint32_t top = shift ? 0xffffffffu << (32 - shift) : 0;
+                    b = (b & top) | ((b << 8) & ~top);
+                }
+            }
+            acc |= b >> ph;
+            ph += bits;
+            if (ph >= 32) {
+                store(4);
+                ph -= 32;
+                acc = __funnelshift_lc(0u, b, bits - ph); // the ph bits that did not fit
+            }
+        }
+        store(ph / 8);
+        kept += (uint32_t)total;
     }
-    if (!kStaged) { // what is left in the buffer: fewer than 16 bytes
+    if (tid < 64) buf[(kept + tid) ^ 3u] = 0;
+    team.sync();
+    return kept;
+}
+
+// ---- kernels -------------------------------------------------------------------------------
+
+struct SyncShared {
+    uint16_t entry[kThreads + 2]; // state at the start of every subsequence, relative to it
+    uint16_t blocks[kThreads];    // blocks completed inside it
+    uint8_t list[2][kThreads];    // subsequences to decode (again)
+    int count[2];
+    int warp[kThreads / 32];
+    uint32_t mark[2];
+};
+// Shared memory of a team's stream: the aligned vectors that hold max_raw bytes, and the zero bytes behind.
+__host__ __device__ constexpr size_t stream_bytes(uint32_t max_raw) { return ((size_t)max_raw + 16 + 64 + 31) / 16 * 16; }
+
+__device__ __forceinline__ bool index_entry_valid(const DecodeIndexHeader *entry, const ImageDesc &d) {
+    const volatile DecodeIndexHeader *h = entry; // written by an earlier launch
+    return h->magic == kDecodeIndexMagic && h->scan_len == d.scan_len && h->subseq_bits == d.subseq_bits && h->segments == d.seg_count;
+}
+
+template <int TEAMS>
+__global__ void __launch_bounds__(kThreads * TEAMS)
+scan_sync_kernel(const ImageDesc *__restrict__ descs, const uint2 *__restrict__ segs, int n_segs, const uint8_t *__restrict__ blob,
+                 const HuffTable *__restrict__ huff, EntropyScratch scratch, const uint8_t *__restrict__ index_pool,
+                 unsigned long long *__restrict__ index_stats, int table_slots, uint32_t buf_bytes) {
+    extern __shared__ __align__(16) unsigned char s_dyn[];
+    __shared__ SyncShared s_teams[TEAMS];
+    const Team<TEAMS> team;
+    const int tid = team.tid;
+    SyncShared &sh = s_teams[team.index];
+    Tables *tables = reinterpret_cast<Tables *>(s_dyn);
+    unsigned char *buf = s_dyn + tables_bytes(table_slots) + team.index * buf_bytes;
+    const int mine = blockIdx.x * TEAMS + team.index;
+    const uint2 which = segs[min(mine, n_segs - 1)];
+    const uint32_t j = which.y;
+    const ImageDesc &d = descs[which.x];
+    const uint32_t S = d.subseq_bits, R = d.seg_raw, warm = j == 0 ? 0 : d.seg_warm;
+    load_tables(tables, d, huff); // (the same whichever team's sample they are taken from)
+    if (TEAMS > 1) {
+        copies_wait();
         __syncthreads();
-        if (tid < 16 && flush_base + tid < clean_len) cl[(flush_base + tid) ^ 3u] = reinterpret_cast<uint8_t *>(s_stream)[tid ^ 3u];
-        __syncthreads();
+        if (mine >= n_segs) return;
     }
-    if (tid < 64) cl[(clean_len + tid) ^ 3u] = 0;
-    __syncthreads();
 
-    const uint32_t *words = reinterpret_cast<const uint32_t *>(cl);
-    const uint32_t total_bits = clean_len * 8;
-    // this image's subsequence length; `subseq_bits` is the batch's longest, which sized the buffers
-    const uint32_t S = d.subseq_bits ? d.subseq_bits : (uint32_t)subseq_bits;
-    const int bpm = d.bpm, luma = d.hs * d.vs, ncomp = d.ncomp;
-    int16_t *cf = coef + (size_t)d.block_base * 64;
+    // ---- the segment's raw bytes: run-up, own part, and what follows it to the end of a block
+    const uint32_t scan_len = d.scan_len, own0 = j * R, own1 = min(own0 + R, scan_len);
+    const uint32_t raw0 = own0 - min(own0, warm * (S >> 3)), raw1 = min(own1 + kSegOverlap, scan_len);
+    const uint32_t at[2] = {own0 - raw0, own1 - raw0};
+    const uint32_t kept = unstuff(team, buf, blob + d.payload_off + d.scan_off + raw0, raw1 - raw0, raw0 == 0, at, sh.warp, sh.mark);
+    const uint32_t own_bit = at[0] == 0 ? 0 : sh.mark[0] * 8, own_end = own1 == raw1 ? kept * 8 : sh.mark[1] * 8;
+    {
+        uint4 *dst = reinterpret_cast<uint4 *>(scratch.clean + d.clean_off + (size_t)j * d.seg_stride);
+        const uint4 *src = reinterpret_cast<const uint4 *>(buf);
+        for (uint32_t k = tid; k < (kept + 64 + 15) / 16; k += kThreads) dst[k] = src[k];
+    }
+    const size_t seg = (size_t)d.seg_first + j;
+    const int n_own = (int)((own_end - own_bit + S - 1) / S), n_subs = (int)warm + n_own;
 
-    // ---- decode index: the states a finished decode of this very stream left behind
-    DecodeIndexHeader *ix_hdr = nullptr;
-    unsigned long long *ix_state = nullptr;
-    uint32_t *ix_blocks = nullptr;
-    bool indexed = false;
+    if (TEAMS == 1) copies_wait();
+
+    // ---- decode index: the states an earlier decode of this very stream left behind
     if (index_pool != nullptr && d.index_cap != 0) {
-        ix_hdr = reinterpret_cast<DecodeIndexHeader *>(index_pool + d.index_off);
-        ix_state = reinterpret_cast<unsigned long long *>(ix_hdr + 1);
-        ix_blocks = reinterpret_cast<uint32_t *>(ix_state + d.index_cap + 1);
+        const DecodeIndexHeader *h = reinterpret_cast<const DecodeIndexHeader *>(index_pool + d.index_off);
+        if (index_entry_valid(h, d)) { // (uniform: no launch that writes the entry runs now)
+            const uint32_t *src = reinterpret_cast<const uint32_t *>(h + 1) + (size_t)j * (kSegSubs + 2);
+            scratch.sub_info[seg * kSegSubs + tid] = __ldcg(src + tid);
+            if (tid == 0) {
+                scratch.meta[seg] = SegMeta{own_bit, own_end, kept, __ldcg(src + kSegSubs), __ldcg(src + kSegSubs + 1)};
+                if (j == 0 && index_stats) atomicAdd(index_stats, 1ull);
+            }
+            return;
+        }
+    }
+
+    // ---- guess and repair.  Subsequences t < warm lie in the run-up.
+    auto start_of = [&](int t) -> int { return (int)own_bit + (t - (int)warm) * (int)S; };
+    sh.entry[tid] = 0; // guess: a block, slot 0, begins here (exact for the scan's first subsequence)
+    sh.blocks[tid] = 0;
+    if (tid == 0) {
+        sh.entry[kThreads] = 0;
+        sh.count[0] = sh.count[1] = 0;
+    }
+    team.sync();
+    int n_list = n_subs;
+    for (int round = 0; round <= n_subs && n_list > 0; round++) {
+        int t = -1;
+        uint32_t in = 0;
+        if (tid < n_list) {
+            t = round == 0 ? (start_of(tid) >= 0 ? tid : -1) : sh.list[round & 1][tid];
+            if (t >= 0) in = sh.entry[t];
+        }
+        team.sync(); // every entry state is read before any exit state is written
+        if (tid == 0) sh.count[round & 1] = 0; // filled again from the next round's second half on
+        bool changed = false;
+        if (t >= 0) {
+            const uint32_t start = (uint32_t)start_of(t), end = min(start + S, own_end);
+            Cursor cur = unpack(in, start);
+            sh.blocks[t] = (uint16_t)walk<false>(buf, cur, end, tables, d, huff);
+            const uint32_t out = pack(cur, end);
+            changed = sh.entry[t + 1] != out;
+            if (changed) sh.entry[t + 1] = (uint16_t)out; // only this thread writes entry t + 1 in this round
+            changed = changed && t + 1 < n_subs;
+        }
+        __syncwarp();
+        const uint32_t who = __ballot_sync(0xffffffffu, changed);
+        if (who != 0) { // one place in the next list per warp, then per lane
+            int base = 0;
+            if ((tid & 31) == 0) base = atomicAdd(&sh.count[(round + 1) & 1], __popc(who));
+            base = __shfl_sync(0xffffffffu, base, 0);
+            if (changed) sh.list[(round + 1) & 1][base + __popc(who & ((1u << (tid & 31)) - 1))] = (uint8_t)(t + 1);
+        }
+        team.sync();
+        n_list = sh.count[(round + 1) & 1];
+    }
+
+    // ---- own subsequences: entry state and completed blocks
+    const uint32_t done = tid < n_own ? sh.blocks[tid + warm] : 0;
+    if (tid < n_own) scratch.sub_info[seg * kSegSubs + tid] = sh.entry[tid + warm] | done << 16;
+    int total;
+    team_scan(team, (int)done, sh.warp, total);
+    if (tid == 0) scratch.meta[seg] = SegMeta{own_bit, own_end, kept, sh.entry[n_subs], (uint32_t)total};
+}
+
+// Scans of several segments, one CTA each: the exit state of every segment has to be the entry state
+// the next one worked out from its run-up.  Where it is not, one thread walks on from the exact
+// state, subsequence by subsequence, until it meets the recorded ones; a walk that crosses a whole
+// segment makes the boundary behind it the next round's.
+__global__ void __launch_bounds__(kThreads)
+scan_stitch_kernel(const ImageDesc *__restrict__ descs, const int32_t *__restrict__ list, const HuffTable *__restrict__ huff,
+                   EntropyScratch scratch) {
+    const ImageDesc &d = descs[list[blockIdx.x]];
+    const int tid = threadIdx.x, n_seg = (int)d.seg_count;
+    const uint32_t S = d.subseq_bits;
+    SegMeta *meta = scratch.meta + d.seg_first;
+    uint32_t *info = scratch.sub_info + (size_t)d.seg_first * kSegSubs;
+    for (int round = 0; round < n_seg; round++) {
+        bool any = false;
+        for (int k0 = 1; k0 < n_seg; k0 += kThreads) { // (a round looks at all boundaries, kThreads at a time)
+            const int k = k0 + tid;
+            uint32_t exact = 0;
+            bool differs = false;
+            if (k < n_seg) {
+                exact = meta[k - 1].exit;
+                // an empty segment (its scan ended in stuffing) hands the state on
+                differs = meta[k].own_bit < meta[k].own_end ? exact != (info[(size_t)k * kSegSubs] & 0xffff) : exact != meta[k].exit;
+            }
+            if (!__syncthreads_or(differs)) continue;
+            any = true;
+            if (differs) {
+                const SegMeta m = meta[k];
+                const uint32_t *words = reinterpret_cast<const uint32_t *>(scratch.clean + d.clean_off + (size_t)k * d.seg_stride);
+                uint32_t *mine = info + (size_t)k * kSegSubs;
+                const int n_own = (int)((m.own_end - m.own_bit + S - 1) / S);
+                uint32_t state = exact, blocks = m.blocks;
+                int t = 0;
+                for (; t < n_own && (mine[t] & 0xffff) != state; t++) {
+                    const uint32_t start = m.own_bit + (uint32_t)t * S, end = min(start + S, m.own_end);
+                    Cursor cur = unpack(state, start);
+                    const uint32_t done = walk_plain<false>(words, cur, end, d, huff, nullptr, 0, 0);
+                    blocks += done - (mine[t] >> 16);
+                    mine[t] = state | done << 16;
+                    state = pack(cur, end);
+                }
+                meta[k].blocks = blocks;
+                if (t == n_own) meta[k].exit = state;
+            }
+            __syncthreads();
+        }
+        if (!any) break;
+    }
+}
+
+template <int TEAMS>
+__global__ void __launch_bounds__(kThreads * TEAMS)
+scan_index_kernel(const ImageDesc *__restrict__ descs, const uint2 *__restrict__ segs, int n_segs, const HuffTable *__restrict__ huff,
+                  EntropyScratch scratch, int32_t *__restrict__ status, uint8_t *__restrict__ index_pool,
+                  unsigned long long *__restrict__ index_stats, int table_slots, uint32_t buf_bytes) {
+    extern __shared__ __align__(16) unsigned char s_dyn[];
+    __shared__ int s_warps[TEAMS][kThreads / 32];
+    __shared__ uint32_t s_lasts[TEAMS];
+    const Team<TEAMS> team;
+    const int tid = team.tid;
+    int *s_warp = s_warps[team.index];
+    uint32_t &s_last = s_lasts[team.index];
+    Tables *tables = reinterpret_cast<Tables *>(s_dyn);
+    unsigned char *buf = s_dyn + tables_bytes(table_slots) + team.index * buf_bytes;
+    const int mine = blockIdx.x * TEAMS + team.index;
+    const uint2 which = segs[min(mine, n_segs - 1)];
+    const int img = (int)which.x;
+    const uint32_t j = which.y;
+    const ImageDesc &d = descs[img];
+    load_tables(tables, d, huff);
+    if (TEAMS > 1) {
+        copies_wait();
+        __syncthreads();
+        if (mine >= n_segs) return;
+    }
+    const size_t seg = (size_t)d.seg_first + j;
+    const SegMeta m = scratch.meta[seg];
+    const uint32_t S = d.subseq_bits, nblocks = d.nblocks;
+    uint32_t *pos = scratch.pos + d.block_base;
+    int16_t *dc = scratch.dc + d.block_base;
+
+    uint32_t base = 0; // blocks before this segment
+    if (j > 0) {
+        int before = 0, all;
+        for (uint32_t k = tid; k < j; k += kThreads) before += (int)scratch.meta[d.seg_first + k].blocks;
+        team_scan(team, before, s_warp, all);
+        base = (uint32_t)all;
+    }
+    const int n_own = (int)((m.own_end - m.own_bit + S - 1) / S);
+    const uint32_t info = tid < n_own ? scratch.sub_info[seg * kSegSubs + tid] : 0;
+    int sums[3] = {0, 0, 0};
+    if (base < nblocks) { // (uniform) otherwise the crop needs nothing of this segment
+        const uint32_t skip = m.own_bit >> 7; // vectors of the run-up
+        const uint4 *src = reinterpret_cast<const uint4 *>(scratch.clean + d.clean_off + (size_t)j * d.seg_stride);
+        for (uint32_t k = skip + tid; k < (m.bytes + 64 + 15) / 16; k += kThreads) copy16_async(buf + (size_t)(k - skip) * 16, src + k);
+        copies_wait();
+        int in_segment;
+        const uint32_t first = base + (uint32_t)team_scan(team, (int)(info >> 16), s_warp, in_segment); // (and a barrier for the copies)
+        const uint32_t bias = j * d.seg_stride * 8 + skip * 128; // stream position of the buffer's bit 0
+        const uint32_t start = m.own_bit - skip * 128 + (uint32_t)tid * S;
+        const uint32_t end = min(start + S, m.own_end - skip * 128);
+        Cursor cur = unpack(info & 0xffff, start);
+        const uint32_t b0 = first + (cur.z != 0 ? 1 : 0); // the block in progress belongs to the subsequence it began in
+        uint32_t b1 = b0;
+        int sum[3] = {0, 0, 0};
+        if (tid < n_own && first < nblocks && cur.p < end) {
+            const uint32_t stream = shared_address(buf), luma = tables->luma, bpm = tables->bpm;
+            const uint32_t done = walk<true>(buf, cur, end, tables, d, huff, pos, b0, nblocks);
+            b1 = min(first + done + (cur.z != 0 ? 1 : 0), nblocks);
+            // the DC symbols of the blocks found: positions move on to the first AC symbol, values count
+            // from the thread's first block
+            uint32_t slot = b0 % bpm, next_pos = b0 < b1 ? pos[b0] : 0;
+            for (uint32_t b = b0; b < b1; b++) {
+                const uint32_t p = next_pos, wa = stream + (p >> 5) * 4;
+                if (b + 1 < b1) next_pos = pos[b + 1];
+                const uint32_t w = __funnelshift_l(load_shared(wa + 4), load_shared(wa), p);
+                const int comp = slot < luma ? 0 : (int)(slot - luma) + 1;
+                const HuffTable *table = huff + d.tab_id[d.dc_tab[comp]];
+                uint32_t e = table->look[w >> (32 - kHuffBits)];
+                if (e & kHuffLong) e = huff_long(table, e, w);
+                const uint32_t n = e & 31, size = (e >> 5) & 15;
+                const int v = size ? huff_value(w, n, size) : 0;
+                sum[0] += comp == 0 ? v : 0;
+                sum[1] += comp == 1 ? v : 0;
+                sum[2] += comp == 2 ? v : 0;
+                pos[b] = bias + p + n;
+                dc[b] = (int16_t)(comp == 0 ? sum[0] : (comp == 1 ? sum[1] : sum[2]));
+                slot = slot + 1 == bpm ? 0 : slot + 1;
+            }
+        }
+        // what the segment holds before the thread's first block
+        int before[3];
+#pragma unroll
+        for (int c = 0; c < 3; c++) before[c] = c < d.ncomp ? team_scan(team, sum[c], s_warp, sums[c]) : 0;
+        uint32_t slot = b0 % tables->bpm;
+        for (uint32_t b = b0; b < b1; b++) {
+            dc[b] = (int16_t)(dc[b] + (slot < tables->luma ? before[0] : (slot == tables->luma ? before[1] : before[2])));
+            slot = slot + 1 == tables->bpm ? 0 : slot + 1;
+        }
+    }
+    if (tid == 0) {
+        int32_t *o = scratch.seg_dc + seg * 4;
+        o[0] = sums[0];
+        o[1] = sums[1];
+        o[2] = sums[2];
+    }
+    const bool record = index_pool != nullptr && d.index_cap != 0 &&
+                        !index_entry_valid(reinterpret_cast<const DecodeIndexHeader *>(index_pool + d.index_off), d);
+    if (record) {
+        uint32_t *dst = reinterpret_cast<uint32_t *>(index_pool + d.index_off + sizeof(DecodeIndexHeader)) + (size_t)j * (kSegSubs + 2);
+        dst[tid] = info;
         if (tid == 0) {
-            const volatile DecodeIndexHeader *h = ix_hdr; // entries are written by other launches: no caching
-            const uint32_t v = h->valid_subs;
-            const bool ok = h->magic == kDecodeIndexMagic && h->scan_len == d.scan_len && h->subseq_bits == S &&
-                            h->clean_len == clean_len && v <= d.index_cap && __ldcg(ix_blocks + v) >= d.nblocks;
-            s_ix[0] = ok ? 1u : 0u;
-            s_ix[1] = v;
-        }
-        __syncthreads();
-        indexed = s_ix[0] != 0;
-        const uint32_t valid = s_ix[1];
-        if (indexed) {
-            // Every subsequence starts from its recorded state and writes straight to its recorded
-            // place: one pass, no guessing.  (Uniform branch: all threads read the same header.)
-            {
-                uint4 *z16 = reinterpret_cast<uint4 *>(cf);
-                for (uint32_t k = tid; k < d.nblocks * 8; k += kEntropyThreads) z16[k] = make_uint4(0, 0, 0, 0);
-            }
-            __syncthreads();
-            for (uint32_t t = tid; t < valid; t += kEntropyThreads) {
-                const uint32_t b0 = __ldcg(ix_blocks + t);
-                if (b0 >= d.nblocks) break; // the crop needs nothing from here on
-                Cursor cur = unpack(__ldcg(ix_state + t));
-                uint32_t t_end = (t + 1) * S;
-                if (t_end > total_bits) t_end = total_bits;
-                decode_span<true>(words, 0, cur, t_end, bpm, luma, ncomp, s_tab, cf, b0, d.nblocks);
-            }
-            if (tid == 0) {
-                status[img] = 0;
-                if (index_stats) atomicAdd(index_stats, 1ull);
-            }
-            __syncthreads();
+            dst[kSegSubs] = m.exit;
+            dst[kSegSubs + 1] = m.blocks;
         }
     }
-
-    if (!indexed) {
-    Cursor zero = {0, 0, 0};
-    unsigned long long carry = pack(zero);
-    uint32_t blk_base = 0, zeroed_to = 0;
-    // every chunk moves the carry forward by at least one subsequence; the count is bounded all the
-    // same so that no input, however malformed, can keep the kernel running
-    const uint32_t max_chunks = total_bits / S + 2;
-    for (uint32_t chunk = 0; chunk < max_chunks; chunk++) {
-        const uint32_t carry_p = (uint32_t)(carry >> 32);
-        if (carry_p >= total_bits || blk_base >= d.nblocks) break;
-        const uint32_t first_sub = carry_p / S;
-        // subsequences of this chunk that hold data; threads beyond them stay out of the repair
-        uint32_t left = (total_bits - first_sub * S + S - 1) / S;
-        // When the crop needs only the upper part of the image, so does the decoder: the bits still
-        // to decode are estimated from the blocks still missing (at the rate seen so far, or the
-        // stream's average for the first chunk) with a quarter to spare; a short estimate only
-        // costs another chunk.
-        if (d.mcu_rows < d.mcus_y) {
-            const uint64_t all_blocks = (uint64_t)d.bpm * d.mcus_x * d.mcus_y;
-            const uint64_t missing = d.nblocks - blk_base;
-            const uint64_t bits = blk_base ? missing * (carry_p + 1) / blk_base : missing * total_bits / all_blocks;
-            const uint64_t want = (bits + bits / 4 + (carry_p - first_sub * S)) / S + 2;
-            if (want < left) left = (uint32_t)want;
+    // ---- the CTA that finishes an image last turns the segments' DC sums into sums before them
+    if (TEAMS == 1) copies_wait(); // (nothing may be under way when the CTA ends)
+    __threadfence();
+    team.sync();
+    if (tid == 0) s_last = atomicInc(&scratch.done[img], d.seg_count - 1) == d.seg_count - 1 ? 1 : 0; // wraps back to 0
+    team.sync();
+    if (!s_last) return;
+    __threadfence();
+    int carry[3] = {0, 0, 0}, blocks = 0;
+    for (uint32_t k0 = 0; k0 < d.seg_count; k0 += kThreads) {
+        const uint32_t k = k0 + tid;
+        int32_t *o = scratch.seg_dc + ((size_t)d.seg_first + k) * 4;
+        int n;
+        team_scan(team, k < d.seg_count ? (int)__ldcg(&scratch.meta[d.seg_first + k].blocks) : 0, s_warp, n);
+        blocks += n;
+#pragma unroll
+        for (int c = 0; c < 3; c++) {
+            int all;
+            const int e = team_scan(team, k < d.seg_count ? __ldcg(o + c) : 0, s_warp, all);
+            if (k < d.seg_count) o[c] = carry[c] + e;
+            carry[c] += all;
         }
-        const int nsub = left < (uint32_t)kEntropyThreads ? (int)left : kEntropyThreads;
-        const bool active = tid < nsub;
-        const uint32_t g = first_sub + tid;
-        const uint32_t sub_start = g * S;
-        uint32_t sub_end = sub_start + S;
-        if (sub_end > total_bits) sub_end = total_bits;
-        // The chunk's bits go to shared memory: every lane of a warp reads a different part of the
-        // stream for every symbol, which shared memory serves at a few cycles per warp while the
-        // same pattern on global memory saturates the L1 tag stage (one sector lookup per cycle).
-        const uint32_t bit_base = (kStaged && !resident) ? first_sub * S : 0; // S is a multiple of 128: 16-byte aligned in the stream
-        // the staged copy starts at bit_base: a pointer moved back by that many words takes absolute bit positions
-        const uint32_t *stream = (kStaged ? s_stream : words) - (bit_base >> 5);
-        if (kStaged && !resident) {
-            uint32_t n16 = ((uint32_t)nsub * S + 127) / 128 + 1; // one vector of overrun for the last symbol
-            const uint32_t have16 = (clean_len + 64 - (bit_base >> 3)) / 16; // zero padding included
-            if (n16 > have16) n16 = have16;
-            const uint4 *src16 = reinterpret_cast<const uint4 *>(words + (bit_base >> 5));
-            uint4 *dst16 = reinterpret_cast<uint4 *>(s_stream);
-            for (uint32_t k = tid; k < n16; k += kEntropyThreads) dst16[k] = src16[k];
-        }
-        Cursor guess = {sub_start, 0, 0};
-        s_state[tid] = tid == 0 ? carry : pack(guess);
-        s_dirty[tid] = 1;
-        s_blocks[tid] = 0;
-        __syncthreads();
-        // Repair rounds.  A subsequence is dirty when its entry state changed since it was last
-        // decoded.  Dirty subsequences are compacted each round so that the work fills
-        // whole warps (after the first rounds only a minority is dirty) and idle warps only meet
-        // at the barriers.
-        for (int iter = 0; iter <= nsub; iter++) {
-            const bool dirty = active && s_dirty[tid];
-            int n_dirty;
-            const int pos = block_scan_exclusive(dirty ? 1 : 0, s_warp, n_dirty);
-            if (n_dirty == 0) break;
-            if (dirty) s_list[pos] = (uint16_t)tid;
-            __syncthreads();
-            int t = -1;
-            unsigned long long in = 0;
-            if (tid < n_dirty) {
-                t = s_list[tid];
-                in = s_state[t];
-                s_dirty[t] = 0; // cleared before the barrier, set again (by the left neighbour) only after it
-            }
-            __syncthreads(); // every entry state is read before any exit state is written
-            if (t >= 0) {
-                Cursor cur = unpack(in);
-                const uint32_t t_start = (first_sub + (uint32_t)t) * S;
-                uint32_t t_end = t_start + S;
-                if (t_end > total_bits) t_end = total_bits;
-                bool merged = false;
-                if (!kStaged && ckpt != nullptr) {
-                    // long subsequences: stop where this walk rejoins the previous one
-                    const uint32_t per_sub = (uint32_t)subseq_bits / (uint32_t)ck_bits + 1; // stride: the batch's longest
-                    CheckPoint *ck = ckpt + ((size_t)blockIdx.x * kEntropyThreads + (size_t)t) * per_sub;
-                    int total;
-                    if (iter == 0)
-                        total = count_span_checked<false>(stream, cur, t_start, t_end, bpm, luma, ncomp, s_tab, ck,
-                                                          (uint32_t)ck_bits, merged);
-                    else
-                        total = count_span_checked<true>(stream, cur, t_start, t_end, bpm, luma, ncomp, s_tab, ck,
-                                                         (uint32_t)ck_bits, merged);
-                    s_blocks[t] = (uint16_t)total;
-                } else {
-                    s_blocks[t] = (uint16_t)decode_span<false>(stream, 0, cur, t_end, bpm, luma, ncomp, s_tab, nullptr, 0, 0);
-                }
-                if (!merged) {
-                    const unsigned long long out = pack(cur);
-                    if (s_state[t + 1] != out) { // only this thread writes entry t + 1 in this round
-                        s_state[t + 1] = out;
-                        s_dirty[t + 1] = 1;
-                    }
-                }
-            }
-            __syncthreads();
-        }
-        const int my_blocks = active ? s_blocks[tid] : 0;
-        int chunk_blocks;
-        const int first = block_scan_exclusive(my_blocks, s_warp, chunk_blocks);
-        if (ix_hdr != nullptr && chunk == 0 && first_sub == 0 && (uint32_t)nsub <= d.index_cap) {
-            // the entry states are final now: leave them, and the blocks before each, for the next
-            // decode of this stream (unless an entry that reaches at least as far is there already)
-            if (tid == 0) {
-                const volatile DecodeIndexHeader *h = ix_hdr;
-                const bool keep = h->magic == kDecodeIndexMagic && h->scan_len == d.scan_len && h->subseq_bits == S &&
-                                  h->clean_len == clean_len && h->valid_subs >= (uint32_t)nsub;
-                s_ix[0] = keep ? 1u : 0u;
-                if (!keep) ix_hdr->magic = 0;
-            }
-            __syncthreads();
-            if (s_ix[0] == 0) {
-                if (active) {
-                    ix_state[tid] = s_state[tid];
-                    ix_blocks[tid] = (uint32_t)first;
-                }
-                if (tid == 0) {
-                    ix_state[nsub] = s_state[nsub];
-                    ix_blocks[nsub] = (uint32_t)chunk_blocks;
-                }
-                __threadfence();
-                __syncthreads();
-                if (tid == 0) {
-                    ix_hdr->scan_len = d.scan_len;
-                    ix_hdr->subseq_bits = S;
-                    ix_hdr->clean_len = clean_len;
-                    ix_hdr->valid_subs = (uint32_t)nsub;
-                    __threadfence();
-                    ix_hdr->magic = kDecodeIndexMagic;
-                    if (index_stats) atomicAdd(index_stats + 1, 1ull);
-                }
-            }
-        }
-        // Only non-zero coefficients are stored, so the blocks this chunk writes to are cleared
-        // first: the ones it completes and the one left in progress at its end.  Done here rather
-        // than by a device-wide memset long before, the cleared lines are still in L2 when the
-        // coefficients arrive and reach DRAM once, as whole lines.
-        {
-            uint32_t target = blk_base + (uint32_t)chunk_blocks + 1;
-            if (target > d.nblocks) target = d.nblocks;
-            if (target > zeroed_to) {
-                uint4 *z16 = reinterpret_cast<uint4 *>(cf + (size_t)zeroed_to * 64);
-                const uint32_t nvec = (target - zeroed_to) * 8;
-                for (uint32_t k = tid; k < nvec; k += kEntropyThreads) z16[k] = make_uint4(0, 0, 0, 0);
-                zeroed_to = target;
-            }
-            __syncthreads();
-        }
-        if (active) {
-            Cursor cur = unpack(s_state[tid]);
-            decode_span<true>(stream, 0, cur, sub_end, bpm, luma, ncomp, s_tab, cf,
-                              blk_base + (uint32_t)first, d.nblocks);
-        }
-        carry = s_state[nsub];
-        blk_base += (uint32_t)chunk_blocks;
-        __syncthreads();
     }
-    if (tid == 0) status[img] = blk_base >= d.nblocks ? 0 : kErrData;
-    if (zeroed_to < d.nblocks) { // a stream that ended early: the blocks it never reached read as zero
-        uint4 *z16 = reinterpret_cast<uint4 *>(cf + (size_t)zeroed_to * 64);
-        const uint32_t nvec = (d.nblocks - zeroed_to) * 8;
-        for (uint32_t k = tid; k < nvec; k += kEntropyThreads) z16[k] = make_uint4(0, 0, 0, 0);
+    const bool complete = (uint32_t)blocks >= nblocks;
+    for (uint32_t b = (uint32_t)blocks + tid; b < nblocks; b += kThreads) { // a scan that ended early
+        pos[b] = kNoBlock;
+        dc[b] = 0;
     }
-    __syncthreads();
-    } // !indexed
-
-    // ---- integrate the DC differences of each component over the scan
-    const int nmcu = d.mcus_x * d.mcu_rows; // the MCUs that were decoded
-    int carry_y = 0, carry_cb = 0, carry_cr = 0;
-    for (int base = 0; base < nmcu; base += kEntropyThreads) {
-        const int m = base + tid;
-        int y[4] = {0, 0, 0, 0}, cb = 0, cr = 0;
-        if (m < nmcu) {
-            int acc = 0;
-            for (int k = 0; k < luma; k++) {
-                acc += cf[((size_t)m * bpm + k) * 64];
-                y[k] = acc;
-            }
-            if (ncomp == 3) {
-                cb = cf[((size_t)m * bpm + luma) * 64];
-                cr = cf[((size_t)m * bpm + luma + 1) * 64];
-            }
+    if (tid == 0) {
+        status[img] = complete ? 0 : kErrData;
+        if (record) {
+            DecodeIndexHeader *h = reinterpret_cast<DecodeIndexHeader *>(index_pool + d.index_off);
+            h->scan_len = d.scan_len;
+            h->subseq_bits = d.subseq_bits;
+            h->segments = d.seg_count;
+            __threadfence();
+            h->magic = kDecodeIndexMagic;
+            if (index_stats) atomicAdd(index_stats + 1, 1ull);
         }
-        int ty, tcb, tcr;
-        const int ey = block_scan_exclusive(y[luma - 1], s_warp, ty);
-        const int ecb = block_scan_exclusive(cb, s_warp, tcb);
-        const int ecr = block_scan_exclusive(cr, s_warp, tcr);
-        if (m < nmcu) {
-            for (int k = 0; k < luma; k++)
-                cf[((size_t)m * bpm + k) * 64] = (int16_t)(carry_y + ey + y[k]);
-            if (ncomp == 3) {
-                cf[((size_t)m * bpm + luma) * 64] = (int16_t)(carry_cb + ecb + cb);
-                cf[((size_t)m * bpm + luma + 1) * 64] = (int16_t)(carry_cr + ecr + cr);
-            }
-        }
-        carry_y += ty;
-        carry_cb += tcb;
-        carry_cr += tcr;
     }
 }
 
@@ -651,107 +687,49 @@ entropy_parallel_kernel(const ImageDesc *__restrict__ descs, const int32_t *__re
 // Streams with restart markers (DRI != 0): every restart interval is an independent piece of the
 // stream (byte aligned, DC predictors reset, T.81 F.2.1.3.1 / E.2.4), so no speculation is
 // needed: the unstuffing pass also removes the RSTn markers and records where each interval
-// starts, then one thread decodes one interval straight into its blocks' final positions, DC
-// prediction included.  One CTA per image.
-
-// Decodes `nblk` blocks starting at bit p (slot 0 of an MCU, predictors zero) into cf + blk * 64.
-// Returns the bit position reached, or 0xFFFFFFFF when the interval's bits ran out first.
-__device__ __forceinline__ uint32_t decode_interval(const uint32_t *__restrict__ words, uint32_t p, uint32_t limit,
-                                                    uint32_t nblk, int bpm, int luma, int ncomp,
-                                                    const HuffTable *s_tab,
-                                                    int16_t *__restrict__ cf, uint32_t blk) {
-    int pred[3] = {0, 0, 0};
-    int c = 0, z = 0;
-    int16_t *out = cf + (size_t)blk * 64;
-    uint32_t done = 0;
-    BitWindow win(words, p);
-    while (done < nblk) {
-        if (p >= limit) return 0xFFFFFFFFu;
-        const uint32_t w = win.peek();
-        const bool dc = z == 0;
-        const int comp = (ncomp == 1 || c < luma) ? 0 : c - luma + 1;
-        const HuffTable &t = s_tab[2 * comp + (dc ? 0 : 1)];
-        const uint32_t e = huff_lookup(t, w);
-        const int n = e & 31, s = (e >> 5) & 15;
-        const int zn = dc ? 1 : z + (int)(e >> 9);
-        const int zpos = zn - 1;
-        const int v = s ? extend((w << (n - s)) >> (32 - s), s) : 0;
-        if (dc) {
-            pred[comp] += v;
-            out[0] = (int16_t)pred[comp];
-        } else if (s != 0 && zpos < 64) {
-            out[zpos] = (int16_t)v; // zig-zag order, as everywhere
-        }
-        p += n;
-        win.skip(n);
-        if (zn >= 64) {
-            z = 0;
-            done++;
-            out += 64;
-            c = (c + 1 == bpm) ? 0 : c + 1;
-        } else {
-            z = zn;
-        }
-    }
-    return p;
-}
-
-template <int kThreads>
-__global__ void __launch_bounds__(kThreads)
-entropy_restart_kernel(const ImageDesc *__restrict__ descs, const int32_t *__restrict__ list,
-                       const uint8_t *__restrict__ blob, const HuffTable *__restrict__ huff,
-                       uint8_t *__restrict__ clean, int16_t *__restrict__ coef, int32_t *__restrict__ status) {
-    __shared__ HuffTable s_tab[6];
-    __shared__ int s_warp[33];
+// starts, then one thread walks one interval and records its blocks with their final DC values.
+// One CTA per image.
+constexpr int kRestartThreads = 256;
+__global__ void __launch_bounds__(kRestartThreads)
+scan_restart_kernel(const ImageDesc *__restrict__ descs, const int32_t *__restrict__ list, const uint8_t *__restrict__ blob,
+                    const HuffTable *__restrict__ huff, EntropyScratch scratch, int32_t *__restrict__ status) {
+    __shared__ int s_warp[kRestartThreads / 32];
     __shared__ int s_bad;
-
     const int img = list[blockIdx.x];
-    const ImageDesc d = descs[img];
-    const int tid = threadIdx.x;
-    if (d.host_status != 0) {
-        if (tid == 0) status[img] = d.host_status;
-        return;
-    }
-    for (int c = 0; c < d.ncomp; c++) {
-        const uint32_t *sd = reinterpret_cast<const uint32_t *>(&huff[d.dc_tab[c]]);
-        const uint32_t *sa = reinterpret_cast<const uint32_t *>(&huff[d.ac_tab[c]]);
-        uint32_t *dd = reinterpret_cast<uint32_t *>(&s_tab[2 * c]);
-        uint32_t *da = reinterpret_cast<uint32_t *>(&s_tab[2 * c + 1]);
-        for (int i = tid; i < (int)(sizeof(HuffTable) / 4); i += kThreads) {
-            dd[i] = sd[i];
-            da[i] = sa[i];
-        }
-    }
+    const ImageDesc &d = descs[img];
+    const int tid = threadIdx.x, bpm = d.bpm, luma = d.ncomp == 1 ? 1 : d.hs * d.vs;
     if (tid == 0) s_bad = 0;
 
     // ---- remove byte stuffing and restart markers; note where every interval starts
+    const uint32_t scan_len = d.scan_len;
     const uint8_t *scan = blob + d.payload_off + d.scan_off;
-    uint8_t *cl = clean + d.clean_off;
-    uint32_t *starts = reinterpret_cast<uint32_t *>(clean + d.rst_off); // byte offsets in the clean stream
+    uint8_t *cl = scratch.clean + d.clean_off;
+    uint32_t *starts = reinterpret_cast<uint32_t *>(scratch.clean + d.rst_off); // byte offsets in the clean stream
     const int nmcu_all = d.mcus_x * d.mcus_y, ri = d.restart_interval;
     const uint32_t cap = (uint32_t)((nmcu_all + ri - 1) / ri) + 1; // entries the table holds
     if (tid == 0) starts[0] = 0;
     uint32_t clean_len = 0, n_mark = 0;
-    for (uint32_t base = 0; base < d.scan_len; base += kThreads * 16) {
+    for (uint32_t base = 0; base < scan_len; base += kRestartThreads * 16) {
         const uint32_t my = base + tid * 16;
         uint8_t b[17];
         uint32_t keep = 0, marks = 0;
-        int prev = (my > 0 && my <= d.scan_len) ? scan[my - 1] : 0;
+        int prev = (my > 0 && my <= scan_len) ? scan[my - 1] : 0;
 #pragma unroll
-        for (int i = 0; i < 17; i++) b[i] = my + i < d.scan_len ? scan[my + i] : 0;
+        for (int i = 0; i < 17; i++) b[i] = my + i < scan_len ? scan[my + i] : 0;
 #pragma unroll
         for (int i = 0; i < 16; i++) {
             const uint32_t at = my + i;
             const bool rst_ff = b[i] == 0xFF && (b[i + 1] & 0xF8) == 0xD0;
             const bool rst_code = prev == 0xFF && (b[i] & 0xF8) == 0xD0;
             const bool stuffing = b[i] == 0 && prev == 0xFF;
-            if (at < d.scan_len && !rst_ff && !rst_code && !stuffing) keep |= 1u << i;
-            if (at < d.scan_len && rst_code) marks |= 1u << i;
+            if (at < scan_len && !rst_ff && !rst_code && !stuffing) keep |= 1u << i;
+            if (at < scan_len && rst_code) marks |= 1u << i;
             prev = b[i];
         }
         int total, mtotal;
-        const int off = block_scan_exclusive(__popc(keep), s_warp, total);
-        const int moff = block_scan_exclusive(__popc(marks), s_warp, mtotal);
+        auto sync = [] { __syncthreads(); };
+        const int off = scan_exclusive(__popc(keep), tid, kRestartThreads / 32, s_warp, total, sync);
+        const int moff = scan_exclusive(__popc(marks), tid, kRestartThreads / 32, s_warp, mtotal, sync);
         uint32_t o = clean_len + off, m = n_mark + moff;
 #pragma unroll
         for (int i = 0; i < 16; i++) {
@@ -765,69 +743,114 @@ entropy_restart_kernel(const ImageDesc *__restrict__ descs, const int32_t *__res
         n_mark += mtotal;
     }
     if (tid < 64) cl[(clean_len + tid) ^ 3u] = 0;
-    __syncthreads();
 
-    // ---- clear the image's blocks (only non-zero coefficients are stored), then one thread per
-    // restart interval
-    int16_t *cf = coef + (size_t)d.block_base * 64;
-    {
-        uint4 *z16 = reinterpret_cast<uint4 *>(cf);
-        for (uint32_t k = tid; k < d.nblocks * 8; k += kThreads) z16[k] = make_uint4(0, 0, 0, 0);
+    // ---- one thread per restart interval
+    uint32_t *pos = scratch.pos + d.block_base;
+    int16_t *dc = scratch.dc + d.block_base;
+    for (uint32_t k = tid; k < d.nblocks; k += kRestartThreads) {
+        pos[k] = kNoBlock;
+        dc[k] = 0;
     }
     __syncthreads();
     const uint32_t *words = reinterpret_cast<const uint32_t *>(cl);
-    const int bpm = d.bpm, luma = d.hs * d.vs, ncomp = d.ncomp;
     const int nmcu = d.mcus_x * d.mcu_rows; // the crop may need only the upper rows
     const uint32_t needed = (uint32_t)((nmcu + ri - 1) / ri);
     const uint32_t found = n_mark + 1 < cap ? n_mark + 1 : cap;
-    if (found < needed) {
-        if (tid == 0) s_bad = 1; // fewer intervals than the frame needs
-    }
-    for (uint32_t k = tid; k < needed && k < found; k += kThreads) {
-        const int first = (int)k * ri;
-        const int count = nmcu - first < ri ? nmcu - first : ri;
-        const uint32_t p0 = starts[k] * 8;
+    if (found < needed && tid == 0) s_bad = 1; // fewer intervals than the frame needs
+    for (uint32_t k = tid; k < needed && k < found; k += kRestartThreads) {
+        const int first = (int)k * ri, count = nmcu - first < ri ? nmcu - first : ri;
         const uint32_t limit = (k + 1 < found ? starts[k + 1] : clean_len) * 8;
-        const uint32_t p = decode_interval(words, p0, limit, (uint32_t)count * bpm, bpm, luma, ncomp, s_tab, cf,
-                                           (uint32_t)first * bpm);
-        if (p == 0xFFFFFFFFu) s_bad = 1;
+        uint32_t blk = (uint32_t)(first * bpm);
+        const uint32_t end_blk = blk + (uint32_t)(count * bpm);
+        int pred[3] = {0, 0, 0}, z = 0;
+        int c = 0;
+        uint32_t p = starts[k] * 8;
+        while (blk < end_blk) {
+            if (p >= limit) { // the interval's bits ran out
+                s_bad = 1;
+                break;
+            }
+            const uint32_t w = __funnelshift_l(words[(p >> 5) + 1], words[p >> 5], p);
+            const int comp = c < luma ? 0 : c - luma + 1;
+            const HuffTable *table = huff + d.tab_id[z ? d.ac_tab[comp] : d.dc_tab[comp]];
+            uint32_t e = table->look[w >> (32 - kHuffBits)];
+            if (e & kHuffLong) e = huff_long(table, e, w);
+            if (z == 0) {
+                const uint32_t n = e & 31, size = (e >> 5) & 15;
+                const int v = size ? huff_value(w, n, size) : 0;
+                pred[0] += comp == 0 ? v : 0;
+                pred[1] += comp == 1 ? v : 0;
+                pred[2] += comp == 2 ? v : 0;
+                pos[blk] = p + n;
+                dc[blk] = (int16_t)(comp == 0 ? pred[0] : (comp == 1 ? pred[1] : pred[2]));
+            }
+            p += e & 31;
+            z += (int)(e >> 9);
+            if (z >= 64) {
+                z = 0;
+                blk++;
+                c = c + 1 == bpm ? 0 : c + 1;
+            }
+        }
     }
     __syncthreads();
     if (tid == 0) status[img] = s_bad ? kErrData : 0;
 }
 
-void launch_entropy_decode(const ImageDesc *descs, const int32_t *list, int n_list,
-                           const int32_t *seq_list, int n_seq, const uint8_t *blob,
-                           const HuffTable *huff, uint8_t *clean, int16_t *coef, int32_t *status,
-                           int subseq_bits, int entropy_threads, void *checkpoints, uint8_t *index_pool,
-                           unsigned long long *index_stats, cudaStream_t stream) {
-    if (n_list > 0) {
-        const bool staged = subseq_bits <= kMaxStagedBits;
-        auto launch = [&](auto kernel, int threads) {
-            // (the non-staged variant uses the buffer only to collect the unstuffed stream: 16 bytes
-            // per thread and pass plus the incomplete vector carried over)
-            const size_t smem = staged ? ((size_t)threads * subseq_bits / 8 + 63) / 16 * 16 + 16 : (size_t)threads * 16 + 32;
-            cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-            kernel<<<n_list, threads, smem, stream>>>(descs, list, blob, huff, clean, coef, status, subseq_bits,
-                                                      static_cast<CheckPoint *>(checkpoints), kCheckPointBits,
-                                                      index_pool, index_stats);
-        };
-        switch (entropy_threads) {
-        case 128:
-            if (staged) launch(entropy_parallel_kernel<128, true>, 128); else launch(entropy_parallel_kernel<128, false>, 128);
-            break;
-        case 256:
-            if (staged) launch(entropy_parallel_kernel<256, true>, 256); else launch(entropy_parallel_kernel<256, false>, 256);
-            break;
-        case 1024:
-            if (staged) launch(entropy_parallel_kernel<1024, true>, 1024); else launch(entropy_parallel_kernel<1024, false>, 1024);
-            break;
-        default:
-            if (staged) launch(entropy_parallel_kernel<512, true>, 512); else launch(entropy_parallel_kernel<512, false>, 512);
-        }
+} // namespace
+
+uint32_t subseq_target(uint64_t total_bits) {
+    // About 1024 subsequences per SM: enough of them that the chain of look-ups is hidden, no more than
+    // that, because every one costs a re-synchronisation (0.9 kbit) on top of its own length.
+    const uint64_t t = total_bits / (148 * 1024);
+    return (uint32_t)(t < 256 ? 256 : (t > kMaxSubseqBits ? kMaxSubseqBits : (t + 31) / 32 * 32));
+}
+
+ScanLayout layout_scan(uint32_t scan_len, uint32_t target_bits) {
+    ScanLayout l{};
+    const uint64_t bits = (uint64_t)scan_len * 8;
+    const uint32_t warm = (8192 + target_bits - 1) / target_bits; // all but one in 10^4 run-ups are long enough
+    if (bits <= (uint64_t)kSegSubs * target_bits || (target_bits > 512 && bits <= (uint64_t)kSegSubs * kMaxSubseqBits)) {
+        l.seg_count = 1;
+        l.subseq_bits = (uint32_t)((bits + kSegSubs - 1) / kSegSubs + 31) / 32 * 32;
+        if (l.subseq_bits < 128) l.subseq_bits = 128;
+        l.seg_raw = kSegSubs * l.subseq_bits / 8;
+    } else {
+        const uint64_t own = kSegSubs - warm;
+        l.seg_count = (uint32_t)((bits + own * target_bits - 1) / (own * target_bits));
+        l.subseq_bits = (uint32_t)((bits + own * l.seg_count - 1) / (own * l.seg_count) + 31) / 32 * 32;
+        l.seg_warm = warm;
+        l.seg_raw = (uint32_t)own * l.subseq_bits / 8;
+        l.seg_count = (scan_len + l.seg_raw - 1) / l.seg_raw;
     }
-    if (n_seq > 0)
-        entropy_restart_kernel<256><<<n_seq, 256, 0, stream>>>(descs, seq_list, blob, huff, clean, coef, status);
+    l.seg_stride = (kSegSubs * l.subseq_bits / 8 + kSegOverlap + 64 + 31) / 16 * 16;
+    return l;
+}
+
+void launch_entropy_decode(const ImageDesc *descs, const uint2 *segs, int n_segs, const int32_t *multi, int n_multi,
+                           const int32_t *restart, int n_restart, const uint8_t *blob, const HuffTable *huff,
+                           const EntropyScratch &scratch, int32_t *status, uint32_t max_raw, int max_tables, bool alike,
+                           uint8_t *index_pool, unsigned long long *index_stats, cudaStream_t stream) {
+    if (n_segs > 0) {
+        const uint32_t buf = (uint32_t)stream_bytes(max_raw);
+        auto run = [&](auto sync_kernel, auto index_kernel, int teams) {
+            const size_t smem = tables_bytes(max_tables) + (size_t)teams * buf;
+            cudaFuncSetAttribute(sync_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+            cudaFuncSetAttribute(index_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+            const int grid = (n_segs + teams - 1) / teams;
+            sync_kernel<<<grid, kThreads * teams, smem, stream>>>(descs, segs, n_segs, blob, huff, scratch, index_pool, index_stats, max_tables, buf);
+            if (n_multi > 0) scan_stitch_kernel<<<n_multi, kThreads, 0, stream>>>(descs, multi, huff, scratch);
+            index_kernel<<<grid, kThreads * teams, smem, stream>>>(descs, segs, n_segs, huff, scratch, status, index_pool, index_stats, max_tables, buf);
+        };
+        // With enough segments to fill every SM four teams share a set of tables: eight segments of up to
+        // 22 KB fit an SM then, instead of five.
+        if (alike && n_segs >= 148 * 5)
+            run(scan_sync_kernel<4>, scan_index_kernel<4>, 4);
+        else
+            run(scan_sync_kernel<1>, scan_index_kernel<1>, 1);
+    }
+    if (n_restart > 0)
+        scan_restart_kernel<<<n_restart, kRestartThreads, 0, stream>>>(descs, restart, blob, huff, scratch, status);
 }
 
 } // namespace ffcvb

@@ -1,4 +1,5 @@
-// Dequantisation + fast integer inverse DCT + chroma upsampling + colour conversion (sm_100a).
+// AC symbol decode + dequantisation + fast integer inverse DCT + chroma upsampling + colour
+// conversion (sm_100a).
 //
 // The arithmetic is the variant TurboJPEG selects for the reference's call
 // (libffcv/libffcv.cpp:104-106, TJFLAG_FASTDCT without TJFLAG_FASTUPSAMPLE): the AAN fast integer
@@ -6,32 +7,19 @@
 // triangle ("fancy") chroma upsampler, and the 16.16 fixed-point YCbCr->RGB transform.  These are
 // integer butterflies in registers; they are not a dense contraction and must not be reordered,
 // so no tensor cores.
-#include <stdlib.h>
-
+#include "huffman.h"
 #include "kernels.h"
 
 namespace ffcvb {
 
-// The entropy decoder leaves a block's coefficients in zig-zag order (the order it decodes them
-// in); position in that order of the coefficient of row r, column c: kZigzagOf[r * 8 + c].  Used
-// with compile-time indices only (fully unrolled loops), so the permutation costs nothing.
+// Position in zig-zag order of the coefficient of row r, column c: zigzag_of(r * 8 + c).  Used with
+// compile-time indices only (fully unrolled loops), so the permutation costs nothing.
 __device__ __forceinline__ constexpr int zigzag_of(int n) {
     constexpr int t[64] = {0, 1, 5, 6, 14, 15, 27, 28, 2, 4, 7, 13, 16, 26, 29, 42, 3, 8, 12, 17, 25, 30, 41, 43, 9, 11, 18, 24, 31, 40, 44, 53, 10, 19, 23, 32, 39, 45, 52, 54, 20, 22, 33, 38, 46, 51, 55, 60, 21, 34, 37, 47, 50, 56, 59, 61, 35, 36, 48, 49, 57, 58, 62, 63};
     return t[n];
 }
 
-// Loads a block (64 int16 in zig-zag order, 16-byte aligned) into 32 registers of two.
-__device__ __forceinline__ void load_block(const int16_t *__restrict__ coef, int (&w)[32]) {
-#pragma unroll
-    for (int r = 0; r < 8; r++) {
-        const int4 v = reinterpret_cast<const int4 *>(coef)[r];
-        w[4 * r] = v.x;
-        w[4 * r + 1] = v.y;
-        w[4 * r + 2] = v.z;
-        w[4 * r + 3] = v.w;
-    }
-}
-// Coefficient of natural position n (row-major) out of the registers load_block filled.
+// Coefficient of natural position n (row-major) out of a block in zig-zag order, two per register.
 __device__ __forceinline__ int coef_at(const int (&w)[32], int n) {
     const int z = zigzag_of(n);
     return (z & 1) ? (w[z >> 1] >> 16) : (int)(short)(w[z >> 1] & 0xffff);
@@ -84,11 +72,10 @@ __device__ __forceinline__ int reduced_constant(int k, int m) {
 }
 
 template <int R>
-__device__ __forceinline__ void reduced_block(const int16_t *__restrict__ coef, const uint16_t *__restrict__ q,
+__device__ __forceinline__ void reduced_block(const int (&cw)[32], const uint16_t *__restrict__ q,
                                               uint8_t *__restrict__ dst, int pitch) {
     constexpr int N = 8 / R, L = R == 2 ? 1 : 2;
-    int a[8][8], cw[32];
-    load_block(coef, cw);
+    int a[8][8];
 #pragma unroll
     for (int r = 0; r < 8; r++) {
         const int4 qw = reinterpret_cast<const int4 *>(q)[r];
@@ -127,81 +114,118 @@ __device__ __forceinline__ void reduced_block(const int16_t *__restrict__ coef, 
     }
 }
 
-__device__ __forceinline__ int find_image(const ImageDesc *descs, const int32_t *list, int n_list,
-                                          uint32_t blk) {
-    // largest k with descs[list[k]].block_base <= blk (block_base ascends along the list)
-    int lo = 0, hi = n_list - 1;
-    while (lo < hi) {
-        int mid = (lo + hi + 1) >> 1;
-        if (descs[list[mid]].block_base <= blk)
-            lo = mid;
-        else
-            hi = mid - 1;
+// One thread per block: decodes the block's AC symbols from the place the entropy decoder recorded,
+// dequantising each value as it is stored (the block lies in shared memory, two coefficients per word,
+// one bank per lane), then transforms it in registers.  Only blocks inside the crop's reach run.
+// A warp takes blocks of one component that are neighbours in the plane: their symbol counts are
+// alike, their bits are near one another and their rows leave as one run.
+// Bound by instruction issue: about 30 per symbol and 1600 for the transform, per lane.
+__global__ void __launch_bounds__(kBlockTile)
+blocks_kernel(const ImageDesc *__restrict__ descs, const uint2 *__restrict__ tiles, const HuffTable *__restrict__ huff,
+              const MultTable *__restrict__ mult, EntropyScratch scratch, uint8_t *__restrict__ planes) {
+    constexpr int kLook = 1 << kHuffBits;
+    __shared__ __align__(16) uint32_t s_coef[32][kBlockTile];
+    __shared__ __align__(16) uint16_t s_look[2][kLook]; // AC tables of luma and of the first chroma component
+    __shared__ int16_t s_mult[3][64];
+    const uint2 tile = tiles[blockIdx.x];
+    const ImageDesc &d = descs[tile.x];
+    const int tid = threadIdx.x;
+    const int nx = d.idct_col1 - d.idct_col0, ny = d.mcu_rows - d.idct_row0, hs = d.hs, vs = d.vs;
+    const int mcus = nx * ny, luma = hs * vs, n_luma = mcus * luma, luma_pad = (n_luma + 31) & ~31, chroma_pad = (mcus + 31) & ~31;
+    const bool scaled = d.bs_luma != 8; // the coefficients stay as they are: the reduced transforms dequantise
+    {
+        const int first = (int)tile.y * kBlockTile; // which tables this tile needs
+        for (int t = 0; t < (d.ncomp == 3 ? 2 : 1); t++) {
+            if (t == 0 ? first >= luma_pad : first + kBlockTile <= luma_pad) continue;
+            const uint4 *src = reinterpret_cast<const uint4 *>(huff[d.tab_id[d.ac_tab[t]]].look);
+            for (int k = tid; k < kLook / 8; k += kBlockTile) reinterpret_cast<uint4 *>(s_look[t])[k] = src[k];
+        }
+        for (int k = tid; k < 64 * d.ncomp; k += kBlockTile)
+            s_mult[k >> 6][k & 63] = scaled && (k < 64 || d.bs_chroma != 8) ? (int16_t)1 : mult[d.q_tab[k >> 6]].m[k & 63];
     }
-    return list[lo];
-}
-
-__global__ void __launch_bounds__(128)
-idct_kernel(const ImageDesc *__restrict__ descs, const int32_t *__restrict__ list, int n_list,
-            uint32_t total_blocks, const MultTable *__restrict__ mult,
-            const int16_t *__restrict__ coef, uint8_t *__restrict__ planes) {
-    const uint32_t gb = blockIdx.x * blockDim.x + threadIdx.x;
-    if (gb >= total_blocks) return;
-    const ImageDesc &d = descs[find_image(descs, list, n_list, gb)];
-    if (d.host_status != 0) return;
-    const uint32_t b = gb - d.block_base;
-    if (b >= d.nblocks) return;
-    const int luma = d.hs * d.vs;
-    const uint32_t mcu = b / d.bpm;
-    const int slot = (int)(b - mcu * d.bpm);
-    const int my = mcu / d.mcus_x, mx = mcu - my * d.mcus_x;
-    if (my < d.idct_row0 || mx < d.idct_col0 || mx >= d.idct_col1) return; // outside the crop's reach
-    int comp, bx, by, plane_w, bs;
-    if (d.ncomp == 1 || slot < luma) {
-        comp = 0;
-        const int v = slot / d.hs, h = slot - v * d.hs;
-        bx = mx * d.hs + h;
-        by = my * d.vs + v;
+    __syncthreads();
+    int item = (int)tile.y * kBlockTile + tid, comp = 0, bx, by, plane_w, bs;
+    uint32_t blk;
+    if (item < luma_pad) {
+        if (item >= n_luma) return;
+        const int row = nx * hs;
+        by = item / row;
+        bx = item - by * row + d.idct_col0 * hs;
+        by += d.idct_row0 * vs;
+        const int my = by / vs, mx = bx / hs;
+        blk = (uint32_t)(my * d.mcus_x + mx) * d.bpm + (by - my * vs) * hs + (bx - mx * hs);
         bs = d.bs_luma;
-        plane_w = d.mcus_x * d.hs * bs;
+        plane_w = d.mcus_x * hs * bs;
     } else {
-        comp = slot - luma + 1;
-        bx = mx;
-        by = my;
+        item -= luma_pad;
+        comp = 1 + item / chroma_pad;
+        item -= (comp - 1) * chroma_pad;
+        if (d.ncomp != 3 || comp > 2 || item >= mcus) return;
+        by = item / nx;
+        bx = item - by * nx + d.idct_col0;
+        by += d.idct_row0;
+        blk = (uint32_t)(by * d.mcus_x + bx) * d.bpm + luma + comp - 1;
         bs = d.bs_chroma;
         plane_w = d.mcus_x * bs;
     }
+    // ---- the block's coefficients
+    const uint32_t p0 = scratch.pos[d.block_base + blk];
+    int dc = scratch.dc[d.block_base + blk];
+    if (d.seg_count > 1 && p0 != kNoBlock) dc += scratch.seg_dc[((size_t)d.seg_first + p0 / (d.seg_stride * 8)) * 4 + comp];
+    const int16_t *m = s_mult[comp];
+#pragma unroll
+    for (int k = 0; k < 32; k++) s_coef[k][tid] = 0;
+    reinterpret_cast<int16_t *>(&s_coef[0][tid])[0] = (int16_t)((int16_t)dc * m[0]);
+    if (p0 != kNoBlock) {
+        const int t = comp == 0 ? 0 : 1, table = d.ac_tab[comp];
+        const bool in_shared = comp < 2 || table == d.ac_tab[1]; // (a table of its own for Cr: read where it is)
+        const HuffTable *full = huff + d.tab_id[table];
+        const uint32_t *words = reinterpret_cast<const uint32_t *>(scratch.clean + d.clean_off);
+        uint32_t p = p0;
+        const uint32_t *w32 = words + (p >> 5);
+        uint32_t hi = w32[0], lo = w32[1], nx_ = w32[2], edge = (p & ~31u) + 32;
+        w32 += 3;
+        int z = 1;
+        do {
+            const uint32_t w = __funnelshift_l(lo, hi, p);
+            uint32_t e = in_shared ? s_look[t][w >> (32 - kHuffBits)] : full->look[w >> (32 - kHuffBits)];
+            if (e & kHuffLong) e = huff_long(full, e, w);
+            const uint32_t n = e & 31, size = (e >> 5) & 15;
+            p += n;
+            const bool next = p >= edge;
+            hi = next ? lo : hi;
+            lo = next ? nx_ : lo;
+            if (next) nx_ = *w32++;
+            edge += next ? 32 : 0;
+            z += (int)(e >> 9);
+            const int at = z - 1; // where the value goes
+            if (size != 0 && at < 64) reinterpret_cast<int16_t *>(&s_coef[at >> 1][tid])[at & 1] = (int16_t)(huff_value(w, n, size) * m[at]);
+        } while (z < 64);
+    }
+    int cw[32];
+#pragma unroll
+    for (int k = 0; k < 32; k++) cw[k] = (int)s_coef[k][tid];
+    uint8_t *dst = planes + d.plane_off[comp] + (size_t)(by * bs) * plane_w + bx * bs;
     if (bs != 8) { // scaled decode: this block becomes bs x bs samples
         const MultTable &mt = mult[d.q_tab[comp]];
-        const int16_t *cb = coef + (size_t)gb * 64;
-        uint8_t *dst = planes + d.plane_off[comp] + (size_t)(by * bs) * plane_w + bx * bs;
         if (bs == 4) {
-            reduced_block<2>(cb, mt.q, dst, plane_w);
+            reduced_block<2>(cw, mt.q, dst, plane_w);
         } else if (bs == 2) {
-            reduced_block<4>(cb, mt.q, dst, plane_w);
+            reduced_block<4>(cw, mt.q, dst, plane_w);
         } else {
-            const int a0 = (int)cb[0] * (int)mt.q[0];
+            const int a0 = coef_at(cw, 0) * (int)mt.q[0];
             dst[0] = (uint8_t)min(255, max(0, ((a0 + 4) >> 3) + 128));
         }
         return;
     }
-    const int16_t *q = mult[d.q_tab[comp]].m;
-    int v[8][8], cw[32];
-    load_block(coef + (size_t)gb * 64, cw);
+    int v[8][8];
 #pragma unroll
-    for (int r = 0; r < 8; r++) {
-        const int4 qw = reinterpret_cast<const int4 *>(q)[r];
-        const int qq[4] = {qw.x, qw.y, qw.z, qw.w};
+    for (int r = 0; r < 8; r++)
 #pragma unroll
-        for (int k = 0; k < 4; k++) {
-            v[r][2 * k] = w16(coef_at(cw, r * 8 + 2 * k) * (int)(short)(qq[k] & 0xffff));
-            v[r][2 * k + 1] = w16(coef_at(cw, r * 8 + 2 * k + 1) * (qq[k] >> 16));
-        }
-    }
+        for (int c = 0; c < 8; c++) v[r][c] = coef_at(cw, r * 8 + c);
 #pragma unroll
     for (int c = 0; c < 8; c++)
         idct8(v[0][c], v[1][c], v[2][c], v[3][c], v[4][c], v[5][c], v[6][c], v[7][c]);
-    uint8_t *dst = planes + d.plane_off[comp] + (size_t)(by * 8) * plane_w + bx * 8;
 #pragma unroll
     for (int r = 0; r < 8; r++) {
         idct8(v[r][0], v[r][1], v[r][2], v[r][3], v[r][4], v[r][5], v[r][6], v[r][7]);
@@ -217,6 +241,11 @@ idct_kernel(const ImageDesc *__restrict__ descs, const int32_t *__restrict__ lis
         }
         *reinterpret_cast<uint2 *>(dst + (size_t)r * plane_w) = make_uint2(lo, hi);
     }
+}
+
+void launch_blocks(const ImageDesc *descs, const uint2 *tiles, int n_tiles, const HuffTable *huff, const MultTable *mult,
+                   const EntropyScratch &scratch, uint8_t *planes, cudaStream_t stream) {
+    if (n_tiles > 0) blocks_kernel<<<n_tiles, kBlockTile, 0, stream>>>(descs, tiles, huff, mult, scratch, planes);
 }
 
 // ------------------------------------------------------------------------------------------
@@ -242,13 +271,6 @@ __device__ __forceinline__ int chroma_sample(const uint8_t *__restrict__ p, int 
     }
     if (cx == real_w - 1) return (cur * 4 + 7) >> 4;
     return (cur * 3 + 3 * row[cx + 1] + far[cx + 1] + 7) >> 4;
-}
-
-void launch_idct(const ImageDesc *descs, const int32_t *list, int n_list, uint32_t total_blocks,
-                 const MultTable *mult, const int16_t *coef, uint8_t *planes, cudaStream_t stream) {
-    if (total_blocks == 0) return;
-    idct_kernel<<<(total_blocks + 127) / 128, 128, 0, stream>>>(descs, list, n_list, total_blocks, mult,
-                                                               coef, planes);
 }
 
 // 16.16 fixed-point YCbCr -> RGB of libjpeg (jdcolor.c's tables written out), one pixel.

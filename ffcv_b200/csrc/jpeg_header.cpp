@@ -110,9 +110,11 @@ int parse_jpeg_header(const uint8_t *d, size_t n, JpegHeader *h) {
     return 0;
 }
 
-void build_huff_table(const RawHuff &raw, HuffTable *t) {
+void build_huff_table(const RawHuff &raw, bool is_dc, HuffTable *t) {
+    constexpr int B = kHuffBits;
     memset(t, 0, sizeof(*t));
     memcpy(t->vals, raw.vals, 256);
+    t->is_dc = is_dc;
     int code = 0, k = 0;
     for (int len = 1; len <= 16; len++) {
         t->valoff[len] = k - code;
@@ -125,21 +127,21 @@ void build_huff_table(const RawHuff &raw, HuffTable *t) {
     code = 0;
     k = 0;
     int n_sub = 0;
-    int sub_of_prefix[512];
-    for (int i = 0; i < 512; i++) sub_of_prefix[i] = -1;
+    int sub_of_prefix[1 << B];
+    for (int i = 0; i < 1 << B; i++) sub_of_prefix[i] = -1;
     for (int len = 1; len <= 16; len++) {
         for (int i = 0; i < raw.bits[len]; i++, k++, code++) {
             if (code >= (1 << len)) continue; // over-subscribed table: ignore the excess codes
-            const uint16_t entry = huff_entry(len, raw.vals[k]);
-            if (len <= 9) {
-                const int first = code << (9 - len);
-                for (int f = 0; f < (1 << (9 - len)); f++) t->look[first + f] = entry;
+            const uint16_t entry = huff_entry(len, raw.vals[k], is_dc);
+            if (len <= B) {
+                const int first = code << (B - len);
+                for (int f = 0; f < (1 << (B - len)); f++) t->look[first + f] = entry;
             } else {
-                const int prefix = code >> (len - 9);
+                const int prefix = code >> (len - B);
                 if (sub_of_prefix[prefix] < 0) {
                     if (n_sub < kHuffSubTables) {
                         sub_of_prefix[prefix] = n_sub;
-                        t->look[prefix] = (uint16_t)(0x8000 | n_sub);
+                        t->look[prefix] = (uint16_t)(kHuffLong | n_sub);
                         n_sub++;
                     } else {
                         sub_of_prefix[prefix] = kHuffSubTables; // no room: this prefix walks the code lengths
@@ -148,21 +150,38 @@ void build_huff_table(const RawHuff &raw, HuffTable *t) {
                 }
                 const int sub = sub_of_prefix[prefix];
                 if (sub < kHuffSubTables) {
-                    const int rest = (code << (16 - len)) & 127; // bits 10..16, left-aligned
+                    const int rest = (code << (16 - len)) & ((1 << (16 - B)) - 1); // the code's bits behind the prefix, left-aligned
                     for (int f = 0; f < (1 << (16 - len)); f++) t->sub[sub][rest + f] = entry;
                 }
             }
         }
         code <<= 1;
     }
-    // A bit pattern that is no code acts as a 16-bit end of block (the decoder must make progress
-    // on garbage too): written into the tables, so the look-up needs no special case.
-    const uint16_t invalid = (uint16_t)(16 | (63 << 9));
-    for (int i = 0; i < 512; i++)
-        if (t->look[i] == 0) t->look[i] = invalid;
-    for (int k = 0; k < n_sub; k++)
-        for (int i = 0; i < 128; i++)
-            if (t->sub[k][i] == 0) t->sub[k][i] = invalid;
+    // bit patterns that are no code: written into the tables, so the look-up needs no special case
+    for (int i = 0; i < 1 << B; i++)
+        if (t->look[i] == 0) t->look[i] = huff_invalid(is_dc);
+    for (int s = 0; s < n_sub; s++)
+        for (int i = 0; i < 1 << (16 - B); i++)
+            if (t->sub[s][i] == 0) t->sub[s][i] = huff_invalid(is_dc);
+    auto entry_of = [&](int v) -> uint16_t { // of the code at the top of the 16 bits v; 0: only the code-length walk knows
+        const uint16_t e = t->look[v >> (16 - B)];
+        return e == 0xFFFF ? 0 : ((e & kHuffLong) ? t->sub[e & (kHuffSubTables - 1)][v & ((1 << (16 - B)) - 1)] : e);
+    };
+    auto fast_of = [](uint16_t e) { return (uint16_t)((e & 31) | (e >> 9) << 8); };
+    t->fast_ok = 1;
+    for (int i = 0; i < kHuffFast; i++) {
+        const bool whole = i >= kHuffFast - kHuffExtra; // an entry for one value of 16 bits
+        const int v = whole ? 65536 - kHuffFast + i : i << (16 - B);
+        const uint16_t e = entry_of(v);
+        t->fast[i] = t->pair[i] = fast_of(e);
+        if (e == 0 || (!whole && (t->look[i] & kHuffLong))) t->fast_ok = 0;
+        // a second symbol, if the bits behind the first one hold all of it
+        const int n = e & 31, dz = e >> 9;
+        if (is_dc || whole || e == 0 || dz > kPairAdvance || n >= B) continue;
+        const uint16_t next = t->look[(i << n) & ((1 << B) - 1)];
+        if ((next & kHuffLong) || n + (next & 31) > B) continue;
+        t->pair[i] = (uint16_t)((n + (next & 31)) | (dz + (next >> 9)) << 8);
+    }
 }
 
 void build_mult_table(const uint16_t quant[64], MultTable *out) {
@@ -170,12 +189,12 @@ void build_mult_table(const uint16_t quant[64], MultTable *out) {
     double f[8];
     f[0] = 1.0;
     for (int k = 1; k < 8; k++) f[k] = sqrt(2.0) * cos(k * M_PI / 16.0);
-    for (int r = 0; r < 8; r++)
-        for (int c = 0; c < 8; c++) {
-            int32_t s = (int32_t)(f[r] * f[c] * 16384.0 + 0.5);
-            out->m[r * 8 + c] = (int16_t)(((int32_t)quant[r * 8 + c] * s + (1 << 11)) >> 12);
-            out->q[r * 8 + c] = quant[r * 8 + c];
-        }
+    for (int z = 0; z < 64; z++) {
+        const int r = kZigzag[z] >> 3, c = kZigzag[z] & 7;
+        const int32_t s = (int32_t)(f[r] * f[c] * 16384.0 + 0.5);
+        out->m[z] = (int16_t)(((int32_t)quant[kZigzag[z]] * s + (1 << 11)) >> 12);
+        out->q[kZigzag[z]] = quant[kZigzag[z]];
+    }
 }
 
 } // namespace ffcvb

@@ -28,7 +28,7 @@ struct JpegHeader {
 // a single interleaved scan, 1 or 3 components, luma 1x1 / 2x1 / 2x2 with 1x1 chroma.
 int parse_jpeg_header(const uint8_t *d, size_t n, JpegHeader *h);
 
-void build_huff_table(const RawHuff &raw, HuffTable *out);
+void build_huff_table(const RawHuff &raw, bool is_dc, HuffTable *out);
 void build_mult_table(const uint16_t quant[64], MultTable *out);
 
 } // namespace ffcvb

@@ -14,40 +14,51 @@ namespace ffcvb {
 constexpr int kGatherCtas = 16;
 void launch_gather_payloads(const ImageDesc *descs, int n, uint8_t *blob, int ctas, int in_flight, cudaStream_t stream);
 
-// Longest subsequence whose chunk the entropy decoder stages in shared memory.
-constexpr int kMaxStagedBits = 1280;
-// Longer subsequences leave check-points every kCheckPointBits bits (16 bytes each) so that a
-// repair pass can stop where it rejoins the previous pass: entropy_checkpoint_bytes() of scratch.
-constexpr int kCheckPointBits = 4096;
-inline size_t entropy_checkpoint_bytes(int n_images, int entropy_threads, int subseq_bits) {
-    if (subseq_bits <= kMaxStagedBits) return 0;
-    return (size_t)n_images * entropy_threads * (subseq_bits / kCheckPointBits + 1) * 16;
+// Scratch and results of the entropy decode of a batch (device memory, no initialisation needed
+// except `done`, which starts at zero once and is left at zero).
+struct EntropyScratch {
+    uint8_t *clean;      // unstuffed streams (ImageDesc::clean_off), 512 spare bytes behind them
+    SegMeta *meta;       // per segment
+    uint32_t *sub_info;  // per segment kSegSubs words: state at the start of a subsequence, blocks << 16
+    int32_t *seg_dc;     // per segment four words: DC value of each component before the segment
+    uint32_t *done;      // per sample
+    uint32_t *pos;       // per block: bit position of its first AC symbol from its image's clean_off
+    int16_t *dc;         // per block: DC value, relative to seg_dc of its segment
+};
+
+// Entropy decode: finds every block of the listed scans.  `segs` (device): one entry (sample, segment)
+// per segment of the samples without restart markers; `multi`: the samples with more than one
+// segment; `restart`: the samples with restart markers.  `max_raw` bounds a segment's raw bytes
+// with run-up and overlap, `max_tables` the tables of a sample in shared memory (its distinct DC tables
+// and twice its AC tables).  `alike`: all the samples in segs have the same tables and layout of an MCU.
+// status[sample] is set for every listed sample.  index_pool / index_stats: the decode index (see DecodeIndexHeader)
+// and two counters (images decoded from their entry, entries written); both may be nullptr.
+void launch_entropy_decode(const ImageDesc *descs, const uint2 *segs, int n_segs, const int32_t *multi, int n_multi,
+                           const int32_t *restart, int n_restart, const uint8_t *blob, const HuffTable *huff,
+                           const EntropyScratch &scratch, int32_t *status, uint32_t max_raw, int max_tables, bool alike,
+                           uint8_t *index_pool, unsigned long long *index_stats, cudaStream_t stream);
+
+// How a scan of scan_len bytes is cut into subsequences and segments.  `target_bits`: wished length of
+// a subsequence, see subseq_target.
+struct ScanLayout {
+    uint32_t subseq_bits, seg_raw, seg_warm, seg_stride, seg_count;
+};
+ScanLayout layout_scan(uint32_t scan_len, uint32_t target_bits);
+// Subsequence length for a batch with `total_bits` of scans: long ones re-synchronise fewer times,
+// short ones spread few scans over the GPU.
+uint32_t subseq_target(uint64_t total_bits);
+
+// Block decode: AC symbols, dequantisation and inverse transform of the blocks the crops need, into
+// the 8-bit component planes.  `tiles` (device): one entry (sample, k) per kBlockTile blocks of a
+// sample, block_tiles() of them per sample.
+constexpr int kBlockTile = 128;
+FFCVB_HD inline uint32_t block_tiles(const ImageDesc &d) {
+    const uint32_t mcus = (uint32_t)(d.idct_col1 - d.idct_col0) * (uint32_t)(d.mcu_rows - d.idct_row0);
+    const uint32_t luma = (mcus * d.hs * d.vs + 31) / 32 * 32, chroma = d.ncomp == 3 ? (mcus + 31) / 32 * 32 : 0;
+    return (luma + 2 * chroma + kBlockTile - 1) / kBlockTile;
 }
-
-// Entropy decode of every JPEG sample listed in `list` (indices into descs): unstuffs the scan
-// into `clean`, Huffman-decodes it into quantised coefficients (zig-zag order inside a block,
-// blocks in scan order, DC un-differenced) in `coef`, and records a per-sample status.
-// `subseq_bits` is the length of the subsequences decoded speculatively in parallel (multiple
-// of 32), `entropy_threads` (128, 256, 512 or 1024) the CTA size: one CTA decodes one image,
-// `entropy_threads` subsequences at a time.  Samples with restart markers are listed in `seq_list`
-// instead and take the restart-interval kernel (one thread per interval, no speculation; needs
-// descs[i].rst_off).  `coef` needs no initialisation: the kernels clear
-// every block they decode into.  `checkpoints`: entropy_checkpoint_bytes(n_list, ...) bytes of device
-// scratch when the subsequences are longer than kMaxStagedBits (may be nullptr: then every repair
-// pass walks its whole subsequence).
-// `subseq_bits` is the longest subsequence of the batch (an image's own length is
-// descs[i].subseq_bits <= subseq_bits).  `index_pool` / `index_stats`: the decode index (see
-// DecodeIndexHeader; descs[i].index_off / index_cap place an image's entry) and two counters
-// (images decoded from their index entry, entries written); both may be nullptr.
-void launch_entropy_decode(const ImageDesc *descs, const int32_t *list, int n_list,
-                           const int32_t *seq_list, int n_seq, const uint8_t *blob,
-                           const HuffTable *huff, uint8_t *clean, int16_t *coef, int32_t *status,
-                           int subseq_bits, int entropy_threads, void *checkpoints, uint8_t *index_pool,
-                           unsigned long long *index_stats, cudaStream_t stream);
-
-// Dequantise + fast integer IDCT of `total_blocks` blocks into the 8-bit component planes.
-void launch_idct(const ImageDesc *descs, const int32_t *list, int n_list, uint32_t total_blocks,
-                 const MultTable *mult, const int16_t *coef, uint8_t *planes, cudaStream_t stream);
+void launch_blocks(const ImageDesc *descs, const uint2 *tiles, int n_tiles, const HuffTable *huff, const MultTable *mult,
+                   const EntropyScratch &scratch, uint8_t *planes, cudaStream_t stream);
 
 // Chroma upsampling (triangle filter) + YCbCr->RGB into h*w*3 images in `rgb` (rows rgb_pitch
 // apart).  4:2:0 images (n_quad of them) go through the quad kernel and 4:4:4 images (n_444)

@@ -29,13 +29,20 @@ constexpr size_t kMaxStreamBytes = FFCVB_STATIC_MAX_STREAM_BYTES;    // compress
 constexpr size_t kMaxPaddedSamples = FFCVB_STATIC_MAX_PADDED_PIXELS; // per component, padded to MCUs
 
 // Scratch layout inside the static array (all offsets multiples of 256).
-constexpr size_t kMetaBytes = 48 * 1024;                             // descriptor, tables, list, status
-constexpr size_t kCleanBytes = kMaxStreamBytes + 512;                // unstuffed bit stream
-constexpr size_t kCoefBytes = 3 * kMaxPaddedSamples * sizeof(int16_t); // 64 coefficients per 64 samples
+constexpr uint32_t kSubseqTarget = 512;                              // one image: short subsequences spread it over the GPU
+constexpr size_t kMaxSegments = kMaxStreamBytes / ((kSegSubs / 2) * kSubseqTarget / 8) + 2;
+constexpr size_t kMaxBlocks = 3 * kMaxPaddedSamples / 64;
+constexpr size_t kMaxTiles = kMaxBlocks / kBlockTile + 4;
+constexpr size_t kMetaBytes = 96 * 1024;                             // descriptor, tables, lists, status
+// unstuffed bit stream: every segment with its run-up and overlap, at most half as much again
+constexpr size_t kCleanBytes = kMaxStreamBytes + kMaxStreamBytes / 2 + 4096;
+constexpr size_t kSegBytes = (kMaxSegments * (sizeof(SegMeta) + 4 * kSegSubs + 16) + 255) / 256 * 256;
+constexpr size_t kIndexBytes = (kMaxBlocks * 6 + 255) / 256 * 256;   // position and DC value of every block
 constexpr size_t kPlaneBytes = 3 * kMaxPaddedSamples + 1024;         // each plane rounded up to 256
 constexpr size_t kCleanOff = kMetaBytes;
-constexpr size_t kCoefOff = kCleanOff + kCleanBytes;
-constexpr size_t kPlaneOff = kCoefOff + kCoefBytes;
+constexpr size_t kSegOff = kCleanOff + kCleanBytes;
+constexpr size_t kIndexOff = kSegOff + kSegBytes;
+constexpr size_t kPlaneOff = kIndexOff + kIndexBytes;
 constexpr size_t kScratchBytes = kPlaneOff + kPlaneBytes;
 
 static __device__ __align__(256) unsigned char g_static_scratch[kScratchBytes];
@@ -49,8 +56,10 @@ std::mutex g_setup_mutex;
 struct Meta {
     ImageDesc desc;
     int32_t list[4];
-    int32_t status[4];
-    HuffTable huff[6];
+    int32_t status[4]; // [0] the image's status, [1] its counter of finished segments
+    uint2 segs[kMaxSegments];
+    uint2 tiles[kMaxTiles];
+    alignas(16) HuffTable huff[6]; // read with 16-byte loads
     alignas(16) MultTable mult[3]; // read with 16-byte loads
 };
 static_assert(sizeof(Meta) <= kMetaBytes, "metadata must fit its scratch region");
@@ -121,16 +130,47 @@ extern "C" int ffcvb_imdecode_static(const uint8_t *jpeg_host, uint64_t jpeg_siz
     if (luma_samples > kMaxPaddedSamples)
         return reject(FFCVB_E_LIMIT, "image larger than FFCVB_STATIC_MAX_PADDED_PIXELS");
     size_t plane = 0;
+    d.fast_tables = 1;
     for (int c = 0; c < h.ncomp; c++) {
-        build_huff_table(h.dc[h.td[c]], &m.huff[2 * c]);
-        build_huff_table(h.ac[h.ta[c]], &m.huff[2 * c + 1]);
+        // (chroma components nearly always share their tables)
+        const int t = c == 2 && h.td[2] == h.td[1] && h.ta[2] == h.ta[1] ? 1 : c;
+        if (t == c) {
+            build_huff_table(h.dc[h.td[c]], true, &m.huff[2 * c]);
+            build_huff_table(h.ac[h.ta[c]], false, &m.huff[2 * c + 1]);
+            d.n_dc_tab = (uint8_t)(c + 1);
+        }
+        d.dc_tab[c] = (uint8_t)t;
+        d.ac_tab[c] = (uint8_t)t; // + the number of DC tables, below
+        if (!m.huff[2 * t].fast_ok || !m.huff[2 * t + 1].fast_ok) d.fast_tables = 0;
         build_mult_table(h.quant[h.tq[c]], &m.mult[c]);
-        d.dc_tab[c] = (uint8_t)(2 * c);
-        d.ac_tab[c] = (uint8_t)(2 * c + 1);
         d.q_tab[c] = (uint8_t)c;
         d.plane_off[c] = plane;
         plane += ((size_t)d.mcus_x * (c == 0 ? d.hs : 1) * 8 * d.mcus_y * (c == 0 ? d.vs : 1) * 8 + 255) & ~(size_t)255;
     }
+
+    int n_segs = 0;
+    if (!d.restart_interval) {
+        const ScanLayout l = layout_scan(d.scan_len, kSubseqTarget);
+        d.subseq_bits = l.subseq_bits;
+        d.seg_raw = l.seg_raw;
+        d.seg_warm = l.seg_warm;
+        d.seg_stride = l.seg_stride;
+        d.seg_count = l.seg_count;
+        n_segs = (int)l.seg_count;
+        if (l.seg_count > kMaxSegments || (size_t)l.seg_count * l.seg_stride + 512 > kCleanBytes)
+            return reject(FFCVB_E_LIMIT, "JPEG stream too large for the static scratch");
+        for (uint32_t k = 0; k < l.seg_count; k++) m.segs[k] = make_uint2(0, k);
+    }
+    const uint32_t n_tiles = block_tiles(d);
+    if (n_tiles > kMaxTiles || d.nblocks > kMaxBlocks) return reject(FFCVB_E_LIMIT, "image larger than FFCVB_STATIC_MAX_PADDED_PIXELS");
+    for (uint32_t k = 0; k < n_tiles; k++) m.tiles[k] = make_uint2(0, k);
+
+    d.n_tab = (uint8_t)(2 * d.n_dc_tab);
+    for (int t = 0; t < d.n_dc_tab; t++) {
+        d.tab_id[t] = (uint8_t)(2 * t);
+        d.tab_id[d.n_dc_tab + t] = (uint8_t)(2 * t + 1);
+    }
+    for (int c = 0; c < h.ncomp; c++) d.ac_tab[c] = (uint8_t)(d.ac_tab[c] + d.n_dc_tab);
 
     // ---- queue the work; everything the kernels need beyond input and output lives in `scratch`
     cudaStream_t st = (cudaStream_t)stream;
@@ -141,15 +181,18 @@ extern "C" int ffcvb_imdecode_static(const uint8_t *jpeg_host, uint64_t jpeg_siz
         return reject(FFCVB_E_CUDA, "copy of the descriptor failed");
     const ImageDesc *desc_dev = &meta_dev->desc;
     const int32_t *list_dev = meta_dev->list; // {0}: the only image
-    const bool sequential = d.restart_interval != 0;
-    const size_t max_scan = d.scan_len;
-    size_t subseq = ((max_scan * 8 / 512 + 1) + 127) / 128 * 128;
-    subseq = subseq < 512 ? 512 : (subseq > 1280 ? 1280 : subseq);
-    launch_entropy_decode(desc_dev, list_dev, sequential ? 0 : 1, list_dev, sequential ? 1 : 0, jpeg_dev, meta_dev->huff,
-                          scratch + kCleanOff, reinterpret_cast<int16_t *>(scratch + kCoefOff), meta_dev->status,
-                          (int)subseq, 512, nullptr, nullptr, nullptr, st);
-    launch_idct(desc_dev, list_dev, 1, d.nblocks, meta_dev->mult, reinterpret_cast<const int16_t *>(scratch + kCoefOff),
-                scratch + kPlaneOff, st);
+    EntropyScratch es{};
+    es.clean = scratch + kCleanOff;
+    es.seg_dc = reinterpret_cast<int32_t *>(scratch + kSegOff);
+    es.sub_info = reinterpret_cast<uint32_t *>(es.seg_dc + 4 * kMaxSegments);
+    es.meta = reinterpret_cast<SegMeta *>(es.sub_info + kSegSubs * kMaxSegments);
+    es.done = reinterpret_cast<uint32_t *>(&meta_dev->status[1]);
+    es.pos = reinterpret_cast<uint32_t *>(scratch + kIndexOff);
+    es.dc = reinterpret_cast<int16_t *>(es.pos + kMaxBlocks);
+    launch_entropy_decode(desc_dev, meta_dev->segs, n_segs, list_dev, n_segs > 1 ? 1 : 0, list_dev, d.restart_interval ? 1 : 0,
+                          jpeg_dev, meta_dev->huff, es, meta_dev->status, kSegSubs * d.subseq_bits / 8 + kSegOverlap, 3 * d.n_dc_tab, false,
+                          nullptr, nullptr, st);
+    launch_blocks(desc_dev, meta_dev->tiles, (int)n_tiles, meta_dev->huff, meta_dev->mult, es, scratch + kPlaneOff, st);
     const bool quad = d.ncomp == 3 && d.hs == 2 && d.vs == 2 && (width + 1) / 2 >= 3;
     const bool full = d.ncomp == 3 && d.hs == 1 && d.vs == 1;
     launch_color(desc_dev, list_dev, 1, quad ? 1 : 0, full ? 1 : 0, (quad || full) ? 0 : 1, (int)width, (int)height,

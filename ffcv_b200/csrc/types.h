@@ -10,6 +10,13 @@ namespace ffcvb {
 constexpr int kMaxComponents = 3;
 constexpr int kPayloadAlign = 16;
 
+// A scan is entropy-decoded in segments of kSegSubs subsequences, one CTA each.  kSegOverlap raw
+// bytes behind a segment are unstuffed with it, so that a block that begins inside can be read to
+// its end (63 symbols of at most 26 bits = 205 bytes, twice that when every second byte is stuffing).
+constexpr int kSegSubs = 128;
+constexpr int kSegOverlap = 512;
+constexpr int kMaxSubseqBits = 1280; // longest subsequence: bounds a segment's shared memory
+
 // Per-sample work descriptor.
 struct ImageDesc {
     uint64_t payload_off;  // byte offset of the staged payload inside the blob (16-byte aligned)
@@ -30,8 +37,12 @@ struct ImageDesc {
     uint8_t ncomp, hs, vs, bpm; // luma sampling factors; blocks per MCU
     uint16_t mcus_x, mcus_y;
     uint16_t restart_interval;
-    uint8_t dc_tab[kMaxComponents], ac_tab[kMaxComponents]; // indices into the batch's HuffTable array
-    uint8_t q_tab[kMaxComponents];                          // indices into the batch's MultTable array
+    uint8_t fast_tables;             // every Huffman table is HuffTable::fast_ok
+    uint8_t n_tab, n_dc_tab;         // distinct Huffman tables of this image (the DC tables first):
+    uint8_t tab_id[6];               // their indices into the batch's HuffTable array,
+    uint8_t dc_tab[kMaxComponents];  // and which of them each component's
+    uint8_t ac_tab[kMaxComponents];  // DC and AC symbols use
+    uint8_t q_tab[kMaxComponents];   // indices into the batch's MultTable array
     uint8_t raw_skew;      // raw, gathered row by row: row r of the staged payload starts
                            // (src_addr + r * width * 3) & 15 bytes into its raw_pitch-wide slot
     // Decoding at reduced scale (1 / 2^scale_shift, JPEG only): every block of a component is
@@ -41,10 +52,12 @@ struct ImageDesc {
     // image have the same resolution.  dec_* equal height / width for unscaled and raw samples.
     uint8_t scale_shift, bs_luma, bs_chroma;
     uint16_t dec_height, dec_width;
-    // Speculative entropy decode: length in bits of this image's subsequences (multiple of 128), and
-    // its place in the decode index (index_cap == 0: none), see DecodeIndexHeader.
-    uint32_t subseq_bits;
-    uint32_t index_cap;    // subsequences the index entry has room for
+    // Entropy decode in segments (scans without restart markers): length in bits of the
+    // subsequences (multiple of 32); raw bytes of a segment; subsequences of run-up before every
+    // segment but the first; bytes of a segment's place in the unstuffed stream; and which of the
+    // batch's segments are this image's.
+    uint32_t subseq_bits, seg_raw, seg_warm, seg_stride, seg_first, seg_count;
+    uint32_t index_cap;    // place in the decode index (0: none), see DecodeIndexHeader
     uint64_t index_off;    // byte offset of the entry in the context's index pool
     // The crop box decides how much of the image is needed: the entropy decoder stops after
     // `mcu_rows` rows of MCUs and the inverse transform runs only on the MCUs of the box below
@@ -52,8 +65,8 @@ struct ImageDesc {
     uint16_t mcu_rows;                           // MCU rows to entropy-decode (<= mcus_y)
     uint16_t idct_row0, idct_col0, idct_col1;    // MCU box to transform: rows [idct_row0, mcu_rows), cols [idct_col0, idct_col1)
     uint32_t nblocks;      // 8x8 blocks to decode: bpm * mcus_x * mcu_rows
-    uint32_t block_base;   // first block of this image in the batch coefficient buffer
-    uint64_t clean_off;    // byte offset of the unstuffed scan in the bitstream scratch (4-aligned)
+    uint32_t block_base;   // first block of this image in the batch's block index
+    uint64_t clean_off;    // byte offset of the unstuffed scan in the bitstream scratch (16-aligned)
     uint64_t rst_off;      // streams with restart markers: byte offset, in the same scratch, of a table of
                            // ceil(MCUs / restart_interval) + 1 uint32 interval starts (4-aligned)
     uint64_t plane_off[kMaxComponents]; // byte offsets of the Y/Cb/Cr planes in the plane scratch
@@ -62,59 +75,89 @@ struct ImageDesc {
 };
 
 // Canonical Huffman code (ITU-T T.81 Annex C) prepared for table-driven decoding.
+constexpr int kHuffBits = 10;     // bits the first level resolves: 99 % of the symbols of photographs
 constexpr int kHuffSubTables = 8; // the standard tables need 5; others fall back to the code-length walk
+constexpr int kHuffExtra = 512;
+constexpr int kHuffFast = 65536 / 64 + kHuffExtra - kHuffExtra / 64;
+static_assert(kHuffBits == 10, "the fast tables count on it");
+constexpr int kPairAdvance = 4;
 struct HuffTable {
     // Table entries describe what a code does to the decoder rather than what it is (see
     // huff_entry): bits 0-4 the bits the symbol consumes (code + magnitude bits), bits 5-8 the
-    // number of magnitude bits, bits 9-14 the zig-zag positions an AC symbol advances (run + 1;
-    // 16 for a run of zeros; 63 for an end of block, which always reaches the block's end).
-    // First level, indexed by the next 9 bits: such an entry for codes of up to 9 bits;
-    // 0x8000 | k when the code is longer and continues in sub[k]; 0xFFFF when it is longer
+    // number of magnitude bits, bits 9-14 the zig-zag positions it advances (DC: 1; AC: run + 1,
+    // 16 for a run of zeros, 63 for an end of block, which always reaches the block's end).
+    // First level, indexed by the next kHuffBits bits: such an entry for codes that fit;
+    // kHuffLong | k when the code is longer and continues in sub[k]; all ones when it is longer
     // and no sub-table was left (walk maxcode/valoff instead).  A prefix that is no code holds
-    // the entry of a 16-bit end of block.
-    uint16_t look[512];
-    // Second level, indexed by bits 10..16 of the code: an entry as above.
-    uint16_t sub[kHuffSubTables][128];
+    // huff_invalid.
+    uint16_t look[1 << kHuffBits];
+    // Second level, indexed by the bits of the code behind those, up to the 16th: an entry as above.
+    uint16_t sub[kHuffSubTables][1 << (16 - kHuffBits)];
+    // For the entropy decoder's inner loop, which may not branch: the low byte of an entry is the number
+    // of bits consumed, the high byte the positions advanced.  With v the next 16 bits, the index is
+    // max(v / 64, v - 65536 + kHuffFast): the first kHuffBits bits, except for the last kHuffExtra values
+    // of v, which have an entry each.  Codes are assigned in order of their length, so the long ones
+    // are the last; whether all codes of more than kHuffBits bits lie there (those of the standard
+    // tables begin 320 before the end) is `fast_ok`.
+    uint16_t fast[kHuffFast];
+    // The same for AC symbols, but two at a time where the second one's bits are among the first
+    // kHuffBits as well and the first one advances at most kPairAdvance positions: with less than 64 -
+    // kPairAdvance positions behind it a block cannot end between the two.
+    uint16_t pair[kHuffFast];
     int32_t maxcode[18]; // largest code of each length, -1 if none
     int32_t valoff[17];  // index of the first symbol of each length minus its first code
+    int32_t is_dc, fast_ok, pad[3];
     uint8_t vals[256];
 };
+constexpr uint32_t kHuffLong = 0x8000u;
+static_assert(sizeof(HuffTable) % 16 == 0, "tables are copied in vectors");
 
-// Entry of a code of `len` bits for symbol `sym` (run << 4 | magnitude bits).  A symbol without
-// magnitude bits is a run of 16 zeros when its run field is 15 and ends the block otherwise.
 #if defined(__CUDACC__)
-__host__ __device__
+#define FFCVB_HD __host__ __device__
+#else
+#define FFCVB_HD
 #endif
-inline uint16_t huff_entry(int len, int sym) {
+// Entry of a code of `len` bits for symbol `sym` (run << 4 | magnitude bits).  An AC symbol without
+// magnitude bits is a run of 16 zeros when its run field is 15 and ends the block otherwise.
+FFCVB_HD inline uint16_t huff_entry(int len, int sym, bool dc) {
     const int s = sym & 15, r = sym >> 4;
-    const int dz = s != 0 ? r + 1 : (r == 15 ? 16 : 63);
+    const int dz = dc ? 1 : (s != 0 ? r + 1 : (r == 15 ? 16 : 63));
     return (uint16_t)((len + s) | (s << 5) | (dz << 9));
 }
+// A bit pattern that is no code: 16 bits without a value that end the block (an AC symbol), so that a
+// decoder on garbage makes progress.
+FFCVB_HD inline uint16_t huff_invalid(bool dc) { return (uint16_t)(16 | ((dc ? 1 : 63) << 9)); }
 
-// Dequantisation multipliers of the fast integer IDCT: quantiser step x AAN scale, 2 fraction bits;
-// and the plain quantiser steps, which the reduced-size transforms of a scaled decode use.
+// Dequantisation multipliers of the fast integer IDCT in zig-zag order: quantiser step x AAN scale, 2
+// fraction bits; and, in natural order, the plain quantiser steps, which the reduced-size transforms
+// of a scaled decode use.
 struct MultTable {
     int16_t m[64];
     uint16_t q[64];
 };
 
-// Decode index: what a finished speculative decode of a stream knows and the next decode of the
-// same stream can start from -- the exact decoder state at the start of every subsequence and the
-// number of blocks completed before it.  With it every subsequence is decoded once, straight into
-// its final place: no guessing, no repair rounds.  An entry lives in device memory:
-//   [DecodeIndexHeader][uint64 state x (cap + 1)][uint32 blocks_before x (cap + 1)]
-// and is valid when `magic` is set (written last) and scan_len / subseq_bits / clean_len match.
-struct DecodeIndexHeader {
-    uint32_t magic, scan_len, subseq_bits, valid_subs; // entries 0 .. valid_subs are final
-    uint32_t clean_len, reserved[3];
+// Segment of a scan as scan_sync_kernel leaves it.  Bits count from the start of the segment's
+// place in the unstuffed stream.
+struct SegMeta {
+    uint32_t own_bit, own_end; // the segment's own bits (behind its run-up, before its overlap)
+    uint32_t bytes;            // unstuffed bytes, overlap included
+    uint32_t exit;             // decoder state behind own_end (as in sub_info)
+    uint32_t blocks;           // blocks completed in the segment
 };
-constexpr uint32_t kDecodeIndexMagic = 0x58444946u;
-inline
-#if defined(__CUDACC__)
-__host__ __device__
-#endif
-size_t decode_index_bytes(uint32_t cap) {
-    return (sizeof(DecodeIndexHeader) + (size_t)(cap + 1) * 12 + 15) / 16 * 16;
+
+constexpr uint32_t kNoBlock = 0xFFFFFFFFu; // position of a block that the scan does not hold
+
+// Decode index: what a finished decode of a stream knows and the next decode of the same stream can
+// start from -- the exact decoder state at the start of every subsequence and the number of blocks
+// completed in it.  With it no guess has to be repaired.  An entry lives in device memory:
+//   [DecodeIndexHeader][per segment: uint32 sub_info x kSegSubs, uint32 exit, uint32 blocks]
+// and is valid when `magic` is set (written last) and the other fields match.
+struct DecodeIndexHeader {
+    uint32_t magic, scan_len, subseq_bits, segments;
+};
+constexpr uint32_t kDecodeIndexMagic = 0x58444947u;
+FFCVB_HD inline size_t decode_index_bytes(uint32_t segments) {
+    return (sizeof(DecodeIndexHeader) + (size_t)segments * (kSegSubs + 2) * 4 + 15) / 16 * 16;
 }
 
 struct BatchHeader {

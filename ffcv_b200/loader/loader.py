@@ -90,7 +90,7 @@ class Loader:
     decode_index_gb : float
         (not in the reference; off by default) GiB of GPU memory for a decode index: the first
         decode of every JPEG sample records the decoder's state at the start of each of its
-        subsequences (about 7 % of the stream's size); from the second epoch on the sample is
+        subsequences (about 3 % of the stream's size); from the second epoch on the sample is
         decoded in one pass from those states instead of being re-synchronised by guess and
         repair.  Same pixels; entropy decode 2-3x faster.  Samples that do not fit the pool any
         more stay unindexed.

@@ -161,7 +161,7 @@ int ffcvb_set_header_cache(ffcvb_ctx *ctx, int enabled);
  * after epoch, and what makes the decode of a stream without restart markers expensive on a GPU
  * -- finding the decoder's state at the start of every subsequence -- is the same every time.
  * With an index of `bytes` bytes of device memory (0 switches it off and frees it) the first decode
- * of a stream records those states (12 bytes per subsequence of 0.5-1.3 kbit: about 7 % of the
+ * of a stream records those states (4 bytes per subsequence of about 1 kbit: about 3 % of the
  * stream's size) and later decodes of the same stream start every subsequence from its recorded
  * state: one pass instead of the guess-and-repair rounds, same pixels.  Streams are told apart by
  * their offset in the file, so a context with an index must serve one file; entries of streams
@@ -290,7 +290,7 @@ int ffcvb_poison(ffcvb_ctx *ctx, void *stream, uint8_t *images_dev, int n, int64
  *   rgb_dev   : DEVICE output buffer of the caller
  * The work is queued on `stream` and the call returns; a corrupt entropy segment is not reported.
  * All scratch (unstuffed bit stream, coefficients, component planes, tables) lives in a fixed
- * array inside the library image, about 4.7 MB that every GPU loading the library holds until
+ * array inside the library image, about 3.1 MB that every GPU loading the library holds until
  * exit, which bounds one call to FFCVB_STATIC_MAX_STREAM_BYTES of JPEG data and
  * FFCVB_STATIC_MAX_PADDED_PIXELS luma samples after padding both sides up to whole MCUs (multiples
  * of 8 or 16); larger inputs are refused with FFCVB_E_LIMIT and a message on stderr.  The call

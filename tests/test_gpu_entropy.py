@@ -1,0 +1,126 @@
+"""The entropy decoder's branches at the sizes where they change: one or several segments per scan,
+one or four teams per CTA, the last CTA incomplete, Huffman tables its inner loop cannot use."""
+import cv2
+import numpy as np
+import pytest
+import torch as ch
+
+from parity import O
+
+pytestmark = pytest.mark.gpu
+
+
+def _jpeg(rng, h, w, quality=90, sampling=420):
+    from ffcv_b200.synthetic import synth_content
+    flags = [cv2.IMWRITE_JPEG_QUALITY, quality]
+    if sampling == 444:
+        flags += [cv2.IMWRITE_JPEG_SAMPLING_FACTOR, cv2.IMWRITE_JPEG_SAMPLING_FACTOR_444]
+    return cv2.imencode('.jpg', synth_content(rng, h, w)[..., ::-1], flags)[1].reshape(-1).copy()
+
+
+def _decode(buf, h, w):
+    from ffcv_b200.libffcv import imdecode
+    out = np.zeros((h, w, 3), np.uint8)
+    assert imdecode(buf, out, h, w) == 0
+    return out
+
+
+@pytest.mark.parametrize('sampling', [420, 444])
+def test_scans_around_the_segment_length(sampling):
+    # 128 subsequences of 256 bits are 4 KiB: scans of about one, two and three segments
+    rng = np.random.default_rng(sampling)
+    for h in range(60, 240, 9):
+        w = h + int(rng.integers(0, 20))
+        buf = _jpeg(rng, h, w, 90, sampling)
+        assert np.array_equal(_decode(buf, h, w), O.jpeg_decode(buf)), (h, w, buf.size)
+
+
+@pytest.mark.parametrize('n,mixed', [(739, False), (743, False), (743, True)], ids=['one_team', 'four_teams', 'tables_differ'])
+def test_batches_around_the_team_limit(n, mixed):
+    """740 segments are where four teams start to share a CTA (when all scans use the same tables)."""
+    from ffcv_b200 import libffcv as L
+    rng = np.random.default_rng(n + mixed)
+    h, w = 40, 56
+    bufs = [_jpeg(rng, h, w, int(rng.integers(60, 98)), 444 if mixed and k % 3 == 0 else 420) for k in range(n)]
+    sizes = np.array([b.size for b in bufs], np.uint64)
+    params = np.tile(np.array([0, 0, h, w], np.int32), (n, 1))
+    ctx = L.Context(0, 1, 4)
+    out = ch.zeros((n, h, w, 3), dtype=ch.uint8, device='cuda')
+    stream = ch.cuda.current_stream().cuda_stream
+    ctx.stage(0, np.concatenate(bufs), np.concatenate([[0], np.cumsum(sizes)[:-1]]).astype(np.uint64), sizes, np.zeros(n, np.uint8),
+              np.full(n, h, np.uint16), np.full(n, w, np.uint16), L.make_plan(h, w, 0, L.OUT_U8_NHWC), params)
+    ctx.submit(0, stream, out.data_ptr())
+    assert (ctx.status(0, stream, n) == 0).all()
+    got = out.cpu().numpy()
+    for k, b in enumerate(bufs):
+        assert np.array_equal(got[k], O.jpeg_decode(b)), k
+    ctx.close()
+
+
+def _grey_jpeg(rng, blocks_y, blocks_x, ac_lengths):
+    """A greyscale baseline stream of random sparse blocks with the AC code lengths given as {symbol: length}."""
+    def codes(lengths):
+        order = sorted(lengths, key=lambda s: (lengths[s], s))
+        out, code, prev = {}, 0, 0
+        for s in order:
+            code <<= lengths[s] - prev
+            prev = lengths[s]
+            out[s] = (code, prev)
+            code += 1
+        counts = [sum(1 for s in order if lengths[s] == n) for n in range(1, 17)]
+        return out, bytes(counts) + bytes(order)
+    dc, dc_seg = codes({s: 4 for s in range(12)})
+    ac, ac_seg = codes(ac_lengths)
+    bits = []
+
+    def put(value, n):
+        bits.extend((value >> k) & 1 for k in reversed(range(n)))
+
+    def put_value(v):
+        size = int(abs(v)).bit_length()
+        put(v if v > 0 else v + (1 << size) - 1, size)
+    dc_value = 0
+    for _ in range(blocks_y * blocks_x):
+        diff = int(rng.integers(-40, 41)) - dc_value
+        dc_value += diff
+        put(*dc[abs(diff).bit_length()])
+        put_value(diff)
+        z = 1
+        while z < 64 and rng.random() < 0.9:
+            run = int(rng.choice([0, 0, 0, 1, 2, 5, 20]))
+            v = int(rng.choice([-1, 1])) * int(rng.integers(1, 1 << int(rng.integers(1, 8))))
+            if z + run > 63:
+                break
+            while run > 15:
+                put(*ac[0xF0])
+                run -= 16
+                z += 16
+            put(*ac[run << 4 | abs(v).bit_length()])
+            put_value(v)
+            z += run + 1
+        if z < 64:
+            put(*ac[0])
+    bits += [1] * (-len(bits) % 8)
+    scan = np.packbits(np.array(bits, np.uint8)).tobytes().replace(b'\xff', b'\xff\x00')
+
+    def segment(marker, body):
+        return bytes([0xFF, marker]) + (len(body) + 2).to_bytes(2, 'big') + body
+    h, w = 8 * blocks_y, 8 * blocks_x
+    data = (b'\xff\xd8' + segment(0xDB, bytes([0]) + bytes(rng.integers(1, 20, 64).tolist())) +
+            segment(0xC0, bytes([8]) + h.to_bytes(2, 'big') + w.to_bytes(2, 'big') + bytes([1, 1, 0x11, 0])) +
+            segment(0xC4, bytes([0x00]) + dc_seg) + segment(0xC4, bytes([0x10]) + ac_seg) +
+            segment(0xDA, bytes([1, 1, 0x00, 0, 63, 0])) + scan + b'\xff\xd9')
+    return np.frombuffer(data, np.uint8).copy(), h, w
+
+
+@pytest.mark.parametrize('long_length', [12, 16], ids=['codes_of_12_bits', 'codes_of_16_bits'])
+@pytest.mark.parametrize('blocks', [(1, 1), (9, 7), (40, 33)])
+def test_tables_whose_long_codes_come_early(blocks, long_length):
+    """Three codes of 3 bits and all others of 12 or 16: long codes far from the end of the code space, more
+    of them than there are second-level tables for."""
+    lengths = {s: long_length for s in [0xF0] + [r << 4 | k for r in range(16) for k in range(1, 9)]}
+    lengths.update({0x00: 3, 0x01: 3, 0x02: 3})
+    buf, h, w = _grey_jpeg(np.random.default_rng(blocks[0] * 100 + long_length), *blocks, lengths)
+    want = O.jpeg_decode(buf)
+    assert np.abs(want.astype(int) - cv2.imdecode(buf, cv2.IMREAD_COLOR)).mean() < 6  # (cv2's accurate inverse transform)
+    assert np.array_equal(_decode(buf, h, w), want)
