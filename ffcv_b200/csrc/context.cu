@@ -188,6 +188,63 @@ void stream_copy(uint8_t *dst, const uint8_t *src, size_t n) {
     if (k < n) memcpy(dst + k, src + k, n - k);
 }
 
+// The distinct tables of a JPEG stream as indices into the context's stores: what all images of one
+// encoder share.
+struct TableSet {
+    uint8_t n_tab, n_dc_tab, fast, dc_tab[kMaxComponents], ac_tab[kMaxComponents]; // as in ImageDesc
+    uint16_t huff[6];                                                              // of the n_tab tables
+    uint16_t quant[kMaxComponents];
+};
+
+// What the marker segments of a JPEG stream said, as far as staging needs it.
+struct StreamHeader {
+    uint64_t size; // of the whole stream
+    uint32_t scan_off, scan_len, table_set;
+    uint16_t restart_interval, width, height;
+    int16_t status; // 0 or why the stream was rejected
+    uint8_t ncomp, hs, vs;
+};
+
+// StreamHeaders by the stream's offset in its file: open addressing, never shrinks.
+class HeaderCache {
+  public:
+    const StreamHeader *find(uint64_t key) const {
+        if (slots_.empty()) return nullptr;
+        for (size_t k = place(key);; k = (k + 1) & (slots_.size() - 1)) {
+            if (slots_[k].key == key) return &slots_[k].header;
+            if (slots_[k].key == kFree) return nullptr;
+        }
+    }
+    void insert(uint64_t key, const StreamHeader &h) {
+        if (2 * (count_ + 1) > slots_.size()) {
+            std::vector<Entry> old(slots_.empty() ? 1024 : slots_.size() * 2, Entry{kFree, {}});
+            old.swap(slots_);
+            count_ = 0;
+            for (const Entry &e : old)
+                if (e.key != kFree) insert(e.key, e.header);
+        }
+        size_t k = place(key);
+        while (slots_[k].key != kFree && slots_[k].key != key) k = (k + 1) & (slots_.size() - 1);
+        count_ += slots_[k].key == kFree;
+        slots_[k] = Entry{key, h};
+    }
+    size_t size() const { return count_; }
+    void clear() {
+        slots_.clear();
+        count_ = 0;
+    }
+
+  private:
+    static constexpr uint64_t kFree = ~0ull;
+    struct Entry {
+        uint64_t key;
+        StreamHeader header;
+    };
+    size_t place(uint64_t key) const { return (size_t)((key * 0x9E3779B97F4A7C15ull) >> 20) & (slots_.size() - 1); }
+    std::vector<Entry> slots_;
+    size_t count_ = 0;
+};
+
 struct DevBuf {
     void *p = nullptr;
     size_t cap = 0;
@@ -224,10 +281,15 @@ struct Slot {
     };
     std::vector<Rider> pending_riders, riders; // set for the next staging / staged with the current batch
     double stage_ms[4] = {0, 0, 0, 0}; // header parse, layout, payload copy, total
-    std::vector<JpegHeader> headers;
-    std::vector<uint64_t> table_hash; // per sample: hashes of its (DC, AC, quantisation) tables x 3 components
-    std::vector<uint16_t> table_id;   // per sample: the same nine tables as indices into the context's stores
-    std::vector<uint8_t> from_cache;  // per sample: its header came from the context's header cache
+    // working lists of the staging call, kept for their memory
+    std::vector<StreamHeader> headers;
+    std::vector<int> to_parse;
+    std::vector<JpegHeader> parsed;
+    std::vector<std::array<uint64_t, 9>> hashes; // of a parsed header's (DC, AC, quantisation) tables x 3 components
+    std::vector<int32_t> jpeg_list, multi, restart;
+    std::vector<uint2> seg_list;   // (sample, segment) of the entropy decoder's CTAs
+    std::vector<uint2> blk_tiles;  // (sample, k) of the block decoder's CTAs
+    std::vector<uint2> quad_tiles; // (sample, tile x | tile y << 16) of the 4:2:0 colour kernel's CTAs
     cudaEvent_t ev[6] = {nullptr, nullptr, nullptr, nullptr, nullptr, nullptr};
     // payload gather runs on its own high-priority stream so that its few CTAs are placed ahead of
     // the large grids other slots have queued, and the PCIe transfer overlaps their compute
@@ -241,6 +303,8 @@ struct Slot {
     bool gather_timed = false; // ev_gather_start .. ev_gathered bracket the last gather of this slot
     bool timed = false; // events of the last run are valid
 };
+
+constexpr double kMaxAdaptiveShare = 0.5; // of a pinned batch's bytes that the threads may be left to copy
 
 struct AuxBuf {
     DevBuf dev;
@@ -289,20 +353,13 @@ struct ffcvb_ctx {
     };
     // Header cache: what the marker segments of a JPEG sample said, kept per sample (key: its
     // offset in the file) so that from the second epoch on staging a sample is a table look-up
-    // instead of a parse; the few distinct Huffman and quantisation tables of a file live in a
-    // store of their own and the cache holds indices into it.
-    struct CachedHeader {
-        uint64_t size;
-        uint32_t scan_off, scan_len;
-        uint16_t restart_interval, width, height;
-        uint8_t ncomp, hs, vs;
-        uint16_t table[9]; // per component: DC, AC (huff_store), quantisation (quant_store)
-    };
+    // instead of a parse; the few distinct tables of a file live in stores of their own.
     bool cache_headers = false; // ffcvb_set_header_cache: sample offsets identify samples (one file per context)
-    std::unordered_map<uint64_t, CachedHeader> header_cache;
+    HeaderCache header_cache;
     std::vector<std::unique_ptr<HuffTable>> huff_store; // built tables
     std::vector<std::unique_ptr<std::array<uint16_t, 64>>> quant_store;
     std::vector<uint64_t> huff_store_hash, quant_store_hash;
+    std::vector<TableSet> table_sets;
     DevBuf index_pool, index_stats;
     size_t index_used = 0;
     std::unordered_map<uint64_t, IndexEntry> index_map;
@@ -485,6 +542,52 @@ size_t read_range(const Source &src, std::atomic<bool> &direct_broken, uint8_t *
     return done;
 }
 
+// Index of the table set of a parsed header (-1: the stores are full); `hash`: of its tables, three per
+// component.
+int intern_tables(ffcvb_ctx *ctx, const JpegHeader &h, const uint64_t *hash) {
+    TableSet ts;
+    memset(&ts, 0, sizeof(ts)); // compared bytewise
+    ts.fast = 1;
+    for (int k = 0; k < 2; k++) { // DC tables first
+        for (int c = 0; c < h.ncomp; c++) {
+            const RawHuff &raw = k == 0 ? h.dc[h.td[c]] : h.ac[h.ta[c]];
+            const uint64_t key = hash[3 * c + k];
+            int found = (int)ctx->huff_store.size() - 1;
+            while (found >= 0 && !(ctx->huff_store_hash[found] == key && memcmp(ctx->huff_store[found]->vals, raw.vals, 256) == 0)) found--;
+            if (found < 0) {
+                if (ctx->huff_store.size() >= 60000) return -1;
+                found = (int)ctx->huff_store.size();
+                ctx->huff_store.emplace_back(new HuffTable());
+                build_huff_table(raw, k == 0, ctx->huff_store.back().get());
+                ctx->huff_store_hash.push_back(key);
+            }
+            int u = k == 0 ? 0 : ts.n_dc_tab;
+            while (u < ts.n_tab && ts.huff[u] != (uint16_t)found) u++;
+            if (u == ts.n_tab) ts.huff[ts.n_tab++] = (uint16_t)found;
+            (k == 0 ? ts.dc_tab : ts.ac_tab)[c] = (uint8_t)u;
+            if (!ctx->huff_store[found]->fast_ok) ts.fast = 0;
+        }
+        if (k == 0) ts.n_dc_tab = ts.n_tab;
+    }
+    for (int c = 0; c < h.ncomp; c++) {
+        const uint16_t *q = h.quant[h.tq[c]];
+        int found = (int)ctx->quant_store.size() - 1;
+        while (found >= 0 && !(ctx->quant_store_hash[found] == hash[3 * c + 2] && memcmp(ctx->quant_store[found]->data(), q, 128) == 0)) found--;
+        if (found < 0) {
+            if (ctx->quant_store.size() >= 60000) return -1;
+            found = (int)ctx->quant_store.size();
+            ctx->quant_store.emplace_back(new std::array<uint16_t, 64>());
+            memcpy(ctx->quant_store.back()->data(), q, 128);
+            ctx->quant_store_hash.push_back(hash[3 * c + 2]);
+        }
+        ts.quant[c] = (uint16_t)found;
+    }
+    for (int k = (int)ctx->table_sets.size() - 1; k >= 0; k--)
+        if (memcmp(&ctx->table_sets[k], &ts, sizeof(ts)) == 0) return k;
+    ctx->table_sets.push_back(ts);
+    return (int)ctx->table_sets.size() - 1;
+}
+
 int stage_impl(ffcvb_ctx *ctx, int slot, const Source &source, const uint64_t *ptrs,
                const uint64_t *sizes, const uint8_t *modes, const uint16_t *heights,
                const uint16_t *widths, int n, const ffcvb_plan *plan, const int32_t *params) {
@@ -532,9 +635,6 @@ int stage_impl(ffcvb_ctx *ctx, int slot, const Source &source, const uint64_t *p
     descs.assign(n, ImageDesc{});
     s.src_ptrs.assign(ptrs, ptrs + n);
     s.headers.resize(n);
-    s.table_hash.assign((size_t)n * 9, 0);
-    s.table_id.assign((size_t)n * 9, 0);
-    s.from_cache.assign((size_t)n, 0);
 
     // ---- reading from file descriptors: every sample's bytes get their place in the pinned buffer
     // before anything is parsed (a JPEG header can only be parsed once it has been read), so the
@@ -549,6 +649,7 @@ int stage_impl(ffcvb_ctx *ctx, int slot, const Source &source, const uint64_t *p
         uint64_t want = 0; // bytes of the sample needed from lo + skip on
     };
     std::vector<Span> spans;
+    std::vector<uint8_t> short_read;
     const int n_params_early = 4 + 2 * plan->n_ops;
     size_t fd_payload_begin = 0, fd_payload_end = 0;
     if (from_fd) {
@@ -593,122 +694,142 @@ int stage_impl(ffcvb_ctx *ctx, int slot, const Source &source, const uint64_t *p
         }
         int grc;
         if ((grc = grow_host(ctx, s.host, s.host_cap, fd_payload_end + tail))) return grc;
+        short_read.assign(n, 0);
+        ctx->pool->parallel_for(n, 1, [&](int i) {
+            const Span &sp = spans[i];
+            if (sp.len && read_range(source, ctx->direct_broken, s.host + sp.dst, sp.lo, sp.len) < sp.skip + sp.want) short_read[i] = 1;
+        });
+    }
+    auto bytes_of = [&](int i) -> const uint8_t * { return from_fd ? s.host + spans[i].dst + spans[i].skip : file_base + ptrs[i]; };
+
+    // ---- headers: from the cache, or parsed (in parallel when there are many)
+    s.to_parse.clear();
+    for (int i = 0; i < n; i++) {
+        if (modes[i] != FFCVB_MODE_JPG) continue;
+        const StreamHeader *hit = ctx->cache_headers ? ctx->header_cache.find(ptrs[i]) : nullptr;
+        if (hit && hit->size == sizes[i] && !(from_fd && short_read[i]))
+            s.headers[i] = *hit;
+        else
+            s.to_parse.push_back(i);
+    }
+    if (!s.to_parse.empty()) {
+        const int m = (int)s.to_parse.size();
+        s.parsed.resize(m);
+        s.hashes.resize(m);
+        auto parse = [&](int k) {
+            const int i = s.to_parse[k];
+            JpegHeader &h = s.parsed[k];
+            StreamHeader &o = s.headers[i];
+            o = StreamHeader{};
+            o.size = sizes[i];
+            o.status = (int16_t)(from_fd && short_read[i] ? kErrData : parse_jpeg_header(bytes_of(i), (size_t)sizes[i], &h));
+            if (o.status != 0) return;
+            o.scan_off = (uint32_t)h.scan_off;
+            o.scan_len = (uint32_t)h.scan_len;
+            o.restart_interval = (uint16_t)h.restart_interval;
+            o.width = (uint16_t)h.width;
+            o.height = (uint16_t)h.height;
+            o.ncomp = (uint8_t)h.ncomp;
+            o.hs = (uint8_t)h.hs[0];
+            o.vs = (uint8_t)h.vs[0];
+            // (bits[17] and vals[256] lie next to each other in RawHuff)
+            static_assert(offsetof(RawHuff, vals) == 17, "RawHuff: vals must follow bits");
+            for (int c = 0; c < h.ncomp; c++) {
+                uint64_t *th = &s.hashes[k][3 * c];
+                if (c == 2 && h.td[2] == h.td[1] && h.ta[2] == h.ta[1] && h.tq[2] == h.tq[1]) {
+                    memcpy(th, th - 3, 3 * sizeof(uint64_t));
+                    continue;
+                }
+                th[0] = hash_bytes(h.dc[h.td[c]].bits, 17 + 256) & ~1ull; // (the same code as a DC and as an AC table: two tables)
+                th[1] = hash_bytes(h.ac[h.ta[c]].bits, 17 + 256) | 1ull;
+                th[2] = hash_bytes(h.quant[h.tq[c]], 128);
+            }
+        };
+        if (m < 12) // waking the staging threads takes longer
+            for (int k = 0; k < m; k++) parse(k);
+        else
+            ctx->pool->parallel_for(m, 8, parse);
+        for (int k = 0; k < m; k++) { // their tables enter the stores, the headers the cache
+            const int i = s.to_parse[k];
+            if (s.headers[i].status != 0) continue;
+            const int set = intern_tables(ctx, s.parsed[k], s.hashes[k].data());
+            if (set < 0) return fail(ctx, FFCVB_E_LIMIT, "more than 60000 distinct Huffman or quantisation tables in a file");
+            s.headers[i].table_set = (uint32_t)set;
+            if (ctx->cache_headers && ctx->header_cache.size() < (size_t)1 << 23) // ~0.9 GB of host memory at most
+                ctx->header_cache.insert(ptrs[i], s.headers[i]);
+        }
     }
 
-    // ---- per-sample: parse headers, decide what to stage
-    ctx->pool->parallel_for(n, from_fd ? 1 : 8, [&](int i) {
+    // ---- what is needed of every sample
+    for (int i = 0; i < n; i++) {
         ImageDesc &d = descs[i];
-        memset(&d, 0, sizeof(d));
         d.mode = modes[i];
         d.height = heights[i];
         d.width = widths[i];
-        bool short_read = false;
-        if (from_fd && spans[i].len) {
-            const Span &sp = spans[i];
-            const size_t got = read_range(source, ctx->direct_broken, s.host + sp.dst, sp.lo, sp.len);
-            short_read = got < sp.skip + sp.want;
-        }
-        const uint8_t *src = from_fd ? s.host + spans[i].dst + spans[i].skip : file_base + ptrs[i];
+        const int32_t *p = params + (size_t)i * n_params;
+        const bool box_ok = plan->resize && p[0] >= 0 && p[2] > 0 && p[0] + p[2] <= (int)d.height && p[1] >= 0 && p[3] > 0 &&
+                            p[1] + p[3] <= (int)d.width;
         if (modes[i] == FFCVB_MODE_JPG) {
-            JpegHeader &h = s.headers[i];
-            int rc;
-            const auto hit = (short_read || !ctx->cache_headers) ? ctx->header_cache.end() : ctx->header_cache.find(ptrs[i]);
-            if (hit != ctx->header_cache.end() && hit->second.size == sizes[i]) {
-                // seen before: only the fields the layout needs are restored (the tables are in the store)
-                const ffcvb_ctx::CachedHeader &ch = hit->second;
-                h.width = ch.width;
-                h.height = ch.height;
-                h.ncomp = ch.ncomp;
-                h.hs[0] = ch.hs;
-                h.vs[0] = ch.vs;
-                h.scan_off = ch.scan_off;
-                h.scan_len = ch.scan_len;
-                h.restart_interval = ch.restart_interval;
-                for (int k = 0; k < 9; k++) s.table_id[(size_t)i * 9 + k] = ch.table[k];
-                s.from_cache[i] = 1;
-                rc = 0;
-            } else {
-                rc = short_read ? kErrData : parse_jpeg_header(src, (size_t)sizes[i], &h);
-            }
-            if (rc == 0 && (h.width != d.width || h.height != d.height)) rc = kErrDims;
-            d.host_status = (int16_t)rc;
+            const StreamHeader &h = s.headers[i];
             d.payload_size = (uint32_t)sizes[i];
-            if (rc == 0) {
-                d.scan_off = (uint32_t)h.scan_off;
-                d.scan_len = (uint32_t)h.scan_len;
-                d.ncomp = (uint8_t)h.ncomp;
-                d.hs = (uint8_t)h.hs[0];
-                d.vs = (uint8_t)h.vs[0];
-                d.bpm = (uint8_t)(h.ncomp == 1 ? 1 : h.hs[0] * h.vs[0] + 2);
-                d.mcus_x = (uint16_t)((h.width + 8 * h.hs[0] - 1) / (8 * h.hs[0]));
-                d.mcus_y = (uint16_t)((h.height + 8 * h.vs[0] - 1) / (8 * h.vs[0]));
-                d.restart_interval = (uint16_t)h.restart_interval;
+            d.host_status = h.status == 0 && (h.width != d.width || h.height != d.height) ? (int16_t)kErrDims : h.status;
+            if (d.host_status == 0) {
+                d.scan_off = h.scan_off;
+                d.scan_len = h.scan_len;
+                d.ncomp = h.ncomp;
+                d.hs = h.hs;
+                d.vs = h.vs;
+                d.bpm = (uint8_t)(h.ncomp == 1 ? 1 : h.hs * h.vs + 2);
+                d.mcus_x = (uint16_t)((h.width + 8 * h.hs - 1) / (8 * h.hs));
+                d.mcus_y = (uint16_t)((h.height + 8 * h.vs - 1) / (8 * h.vs));
+                d.restart_interval = h.restart_interval;
                 d.mcu_rows = d.mcus_y;
                 d.idct_row0 = d.idct_col0 = 0;
                 d.idct_col1 = d.mcus_x;
+                const bool three = h.ncomp == 3, even = h.hs == 1 && h.vs == 1, quad = h.hs == 2 && h.vs == 2;
                 // With a crop box only part of the image is needed.  The colour kernels of 4:2:0
                 // and 4:4:4 images convert the box alone and reach at most one chroma sample
                 // (two pixels, three with an odd edge) beyond it; other layouts convert the whole image.
-                const bool boxed = h.ncomp == 3 && ((h.hs[0] == 2 && h.vs[0] == 2 && (h.width + 1) / 2 >= 3) ||
-                                                    (h.hs[0] == 1 && h.vs[0] == 1));
-                if (plan->resize && boxed) {
-                    const int32_t *p = params + (size_t)i * n_params;
-                    if (p[0] >= 0 && p[2] > 0 && p[0] + p[2] <= (int)d.height && p[1] >= 0 && p[3] > 0 &&
-                        p[1] + p[3] <= (int)d.width) {
-                        const int mh = 8 * d.vs, mw = 8 * d.hs;
-                        const int y0 = p[0] - 3 < 0 ? 0 : p[0] - 3, x0 = p[1] - 3 < 0 ? 0 : p[1] - 3;
-                        const int y1 = p[0] + p[2] + 3 > (int)d.height ? (int)d.height : p[0] + p[2] + 3;
-                        const int x1 = p[1] + p[3] + 3 > (int)d.width ? (int)d.width : p[1] + p[3] + 3;
-                        d.idct_row0 = (uint16_t)(y0 / mh);
-                        d.mcu_rows = (uint16_t)((y1 - 1) / mh + 1);
-                        d.idct_col0 = (uint16_t)(x0 / mw);
-                        d.idct_col1 = (uint16_t)((x1 - 1) / mw + 1);
-                    }
+                if (box_ok && three && ((quad && (h.width + 1) / 2 >= 3) || even)) {
+                    const int mh = 8 * d.vs, mw = 8 * d.hs;
+                    const int y0 = p[0] - 3 < 0 ? 0 : p[0] - 3, x0 = p[1] - 3 < 0 ? 0 : p[1] - 3;
+                    const int y1 = p[0] + p[2] + 3 > (int)d.height ? (int)d.height : p[0] + p[2] + 3;
+                    const int x1 = p[1] + p[3] + 3 > (int)d.width ? (int)d.width : p[1] + p[3] + 3;
+                    d.idct_row0 = (uint16_t)(y0 / mh);
+                    d.mcu_rows = (uint16_t)((y1 - 1) / mh + 1);
+                    d.idct_col0 = (uint16_t)(x0 / mw);
+                    d.idct_col1 = (uint16_t)((x1 - 1) / mw + 1);
                 }
                 d.nblocks = (uint32_t)d.bpm * d.mcus_x * d.mcu_rows;
-                for (int c = 0; c < h.ncomp && !s.from_cache[i]; c++) {
-                    uint64_t *th = &s.table_hash[(size_t)i * 9 + 3 * c];
-                    // (bits[17] and vals[256] lie next to each other in RawHuff)
-                    static_assert(offsetof(RawHuff, vals) == 17, "RawHuff: vals must follow bits");
-                    th[0] = hash_bytes(h.dc[h.td[c]].bits, 17 + 256) & ~1ull; // (the same code as a DC and as an AC table: two tables)
-                    th[1] = hash_bytes(h.ac[h.ta[c]].bits, 17 + 256) | 1ull;
-                    th[2] = hash_bytes(h.quant[h.tq[c]], 128);
-                }
                 // scale of the decode (plan->dct_scale): only layouts whose planes end up at one resolution
-                const bool scalable = h.ncomp == 3 && ((h.hs[0] == 1 && h.vs[0] == 1) || (h.hs[0] == 2 && h.vs[0] == 2));
+                const bool scalable = three && (even || quad);
                 int shift = 0;
                 if (plan->dct_scale > 0) {
                     shift = plan->dct_scale;
                     if (!scalable) d.host_status = (int16_t)kErrUnsupported;
-                } else if (plan->dct_scale < 0 && scalable) {
-                    const int32_t *p = params + (size_t)i * n_params;
-                    if (p[0] >= 0 && p[2] > 0 && p[0] + p[2] <= (int)d.height && p[1] >= 0 && p[3] > 0 &&
-                        p[1] + p[3] <= (int)d.width)
-                        while (shift < 3 && (p[2] >> (shift + 1)) >= plan->out_h && (p[3] >> (shift + 1)) >= plan->out_w) shift++;
+                } else if (plan->dct_scale < 0 && scalable && box_ok) {
+                    while (shift < 3 && (p[2] >> (shift + 1)) >= plan->out_h && (p[3] >> (shift + 1)) >= plan->out_w) shift++;
                 }
                 d.scale_shift = (uint8_t)shift;
                 d.bs_luma = (uint8_t)(8 >> shift);
-                d.bs_chroma = (uint8_t)((8 >> shift) * h.hs[0] > 8 ? 8 : (8 >> shift) * h.hs[0]);
+                d.bs_chroma = (uint8_t)((8 >> shift) * h.hs > 8 ? 8 : (8 >> shift) * h.hs);
             }
             d.dec_height = (uint16_t)((d.height + (1 << d.scale_shift) - 1) >> d.scale_shift);
             d.dec_width = (uint16_t)((d.width + (1 << d.scale_shift) - 1) >> d.scale_shift);
             if (d.bs_luma == 0) d.bs_luma = d.bs_chroma = 8; // rejected stream: fields stay consistent
+            if (direct) d.src_addr = src_dev_base + ptrs[i];
         } else {
             d.dec_height = d.height;
             d.dec_width = d.width;
             int r0 = 0, rows = d.height, c0 = 0, cols = d.width;
-            if (plan->resize) {
-                const int32_t *p = params + (size_t)i * n_params;
-                if (p[0] >= 0 && p[2] > 0 && p[0] + p[2] <= (int)d.height && p[1] >= 0 && p[3] > 0 &&
-                    p[1] + p[3] <= (int)d.width) {
-                    r0 = p[0];
-                    rows = p[2];
-                    c0 = p[1];
-                    cols = p[3];
-                }
+            if (box_ok) {
+                r0 = p[0];
+                rows = p[2];
+                c0 = p[1];
+                cols = p[3];
             }
             const uint64_t need = (uint64_t)d.height * d.width * 3;
-            if (sizes[i] < need || short_read) {
+            if (sizes[i] < need || (from_fd && short_read[i])) {
                 d.host_status = (int16_t)kErrData;
                 rows = 0;
             }
@@ -724,8 +845,7 @@ int stage_impl(ffcvb_ctx *ctx, int slot, const Source &source, const uint64_t *p
             d.payload_size = (uint32_t)((size_t)rows * d.raw_pitch);
             if (direct && rows > 0) d.src_addr = src_dev_base + ptrs[i] + ((uint64_t)r0 * d.width + c0) * 3;
         }
-        if (direct && modes[i] == FFCVB_MODE_JPG) d.src_addr = src_dev_base + ptrs[i];
-    });
+    }
 
     const auto t1 = std::chrono::steady_clock::now();
     // Split staging: with a pinned source the staging threads (and the copy engine) can carry part
@@ -740,7 +860,7 @@ int stage_impl(ffcvb_ctx *ctx, int slot, const Source &source, const uint64_t *p
             const double tc = s.staged_end > s.hdr.payload_off ? s.stage_ms[2] : 0.0;
             if (tg + tc > 0) ctx->share += 0.04 * ((double)tg - tc) / ((double)tg + tc);
             if (ctx->share < 0) ctx->share = 0;
-            if (ctx->share > 0.5) ctx->share = 0.5;
+            if (ctx->share > kMaxAdaptiveShare) ctx->share = kMaxAdaptiveShare;
         } else {
             cudaGetLastError(); // not run yet, or still running: keep the share
         }
@@ -757,65 +877,24 @@ int stage_impl(ffcvb_ctx *ctx, int slot, const Source &source, const uint64_t *p
             }
         }
     }
-    // ---- serial: headers parsed just now enter the cache, their tables the store
-    for (int i = 0; i < n; i++) {
-        const ImageDesc &d = descs[i];
-        if (d.mode != FFCVB_MODE_JPG || d.host_status != 0 || s.from_cache[i]) continue;
-        const JpegHeader &h = s.headers[i];
-        uint16_t *ids = &s.table_id[(size_t)i * 9];
-        bool room = true;
-        for (int c = 0; c < h.ncomp; c++) {
-            const uint64_t *th = &s.table_hash[(size_t)i * 9 + 3 * c];
-            const RawHuff *tabs[2] = {&h.dc[h.td[c]], &h.ac[h.ta[c]]};
-            for (int k = 0; k < 2; k++) {
-                int found = -1;
-                for (int u = (int)ctx->huff_store.size() - 1; u >= 0 && found < 0; u--)
-                    if (ctx->huff_store_hash[u] == th[k] && memcmp(ctx->huff_store[u]->vals, tabs[k]->vals, 256) == 0) found = u;
-                if (found < 0 && ctx->huff_store.size() < 60000) {
-                    found = (int)ctx->huff_store.size();
-                    ctx->huff_store.emplace_back(new HuffTable());
-                    build_huff_table(*tabs[k], k == 0, ctx->huff_store.back().get());
-                    ctx->huff_store_hash.push_back(th[k]);
-                }
-                room = room && found >= 0;
-                ids[3 * c + k] = (uint16_t)(found < 0 ? 0 : found);
-            }
-            int qfound = -1;
-            for (int u = (int)ctx->quant_store.size() - 1; u >= 0 && qfound < 0; u--)
-                if (ctx->quant_store_hash[u] == th[2] && (*ctx->quant_store[u])[0] == h.quant[h.tq[c]][0]) qfound = u;
-            if (qfound < 0 && ctx->quant_store.size() < 60000) {
-                qfound = (int)ctx->quant_store.size();
-                ctx->quant_store.emplace_back(new std::array<uint16_t, 64>());
-                memcpy(ctx->quant_store.back()->data(), h.quant[h.tq[c]], 128);
-                ctx->quant_store_hash.push_back(th[2]);
-            }
-            room = room && qfound >= 0;
-            ids[3 * c + 2] = (uint16_t)(qfound < 0 ? 0 : qfound);
-        }
-        if (!room) return fail(ctx, FFCVB_E_LIMIT, "more than 60000 distinct Huffman or quantisation tables in a file");
-        if (ctx->cache_headers && ctx->header_cache.size() < (size_t)1 << 23) { // ~0.5 GB of host memory at most
-            ffcvb_ctx::CachedHeader ch{};
-            ch.size = sizes[i];
-            ch.scan_off = (uint32_t)h.scan_off;
-            ch.scan_len = (uint32_t)h.scan_len;
-            ch.restart_interval = (uint16_t)h.restart_interval;
-            ch.width = (uint16_t)h.width;
-            ch.height = (uint16_t)h.height;
-            ch.ncomp = (uint8_t)h.ncomp;
-            ch.hs = (uint8_t)h.hs[0];
-            ch.vs = (uint8_t)h.vs[0];
-            memcpy(ch.table, ids, sizeof(ch.table));
-            ctx->header_cache[ptrs[i]] = ch;
-        }
-    }
-    // ---- serial: the batch's own table lists (indices into the store -> indices into the blob)
+    // ---- layout of the JPEG samples' work; the batch's own table lists (indices into the store ->
+    // indices into the blob), worked out once per table set
     std::vector<const HuffTable *> huff_src;
     std::vector<const uint16_t *> mult_src;
-    std::vector<int> huff_of_store(ctx->huff_store.size(), -1), mult_of_store(ctx->quant_store.size(), -1);
-    std::vector<int32_t> jpeg_list, multi, restart;
-    std::vector<uint2> segs;        // (sample, segment) of the entropy decoder's CTAs
-    std::vector<uint2> blk_tiles;   // (sample, k) of the block decoder's CTAs
-    std::vector<uint2> quad_tiles;  // (sample, tile x | tile y << 16) of the 4:2:0 colour kernel's CTAs
+    struct BatchSet {
+        uint32_t set;
+        uint8_t tab_id[6], q_tab[kMaxComponents];
+    };
+    std::vector<BatchSet> batch_sets;
+    int last_set = -1;
+    std::vector<int32_t> &jpeg_list = s.jpeg_list, &multi = s.multi, &restart = s.restart;
+    std::vector<uint2> &segs = s.seg_list, &blk_tiles = s.blk_tiles, &quad_tiles = s.quad_tiles;
+    jpeg_list.clear();
+    multi.clear();
+    restart.clear();
+    segs.clear();
+    blk_tiles.clear();
+    quad_tiles.clear();
     size_t clean_bytes = 0, plane_bytes = 0, rgb_bytes = 0;
     uint32_t total_blocks = 0, max_raw = 0;
     int max_tables = 1, first_jpeg = -1;
@@ -840,35 +919,40 @@ int stage_impl(ffcvb_ctx *ctx, int slot, const Source &source, const uint64_t *p
             d.block_base = total_blocks;
             continue;
         }
-        const JpegHeader &h = s.headers[i];
-        const uint16_t *ids = &s.table_id[(size_t)i * 9];
-        d.fast_tables = 1;
-        for (int k = 0; k < 2; k++) { // the image's distinct tables: DC before AC
-            uint8_t *dst = k == 0 ? d.dc_tab : d.ac_tab;
-            for (int c = 0; c < h.ncomp; c++) {
-                int &slot_of = huff_of_store[ids[3 * c + k]];
-                if (slot_of < 0) {
-                    slot_of = (int)huff_src.size();
-                    huff_src.push_back(ctx->huff_store[ids[3 * c + k]].get());
+        const uint32_t set_id = s.headers[i].table_set;
+        const TableSet &ts = ctx->table_sets[set_id];
+        if (last_set < 0 || batch_sets[last_set].set != set_id) {
+            for (last_set = (int)batch_sets.size() - 1; last_set >= 0 && batch_sets[last_set].set != set_id;) last_set--;
+            if (last_set < 0) {
+                BatchSet bs{};
+                bs.set = set_id;
+                for (int k = 0; k < ts.n_tab; k++) {
+                    const HuffTable *t = ctx->huff_store[ts.huff[k]].get();
+                    size_t u = 0;
+                    while (u < huff_src.size() && huff_src[u] != t) u++;
+                    if (u == huff_src.size()) huff_src.push_back(t);
+                    bs.tab_id[k] = (uint8_t)u;
                 }
-                int u = 0;
-                while (u < d.n_tab && d.tab_id[u] != (uint8_t)slot_of) u++;
-                if (u == d.n_tab) d.tab_id[d.n_tab++] = (uint8_t)slot_of;
-                dst[c] = (uint8_t)u;
-                if (!ctx->huff_store[ids[3 * c + k]]->fast_ok) d.fast_tables = 0;
+                for (int c = 0; c < d.ncomp; c++) {
+                    const uint16_t *q = ctx->quant_store[ts.quant[c]]->data();
+                    size_t u = 0;
+                    while (u < mult_src.size() && mult_src[u] != q) u++;
+                    if (u == mult_src.size()) mult_src.push_back(q);
+                    bs.q_tab[c] = (uint8_t)u;
+                }
+                if (huff_src.size() > 255 || mult_src.size() > 255)
+                    return fail(ctx, FFCVB_E_LIMIT, "more than 255 distinct Huffman or quantisation tables in a batch");
+                last_set = (int)batch_sets.size();
+                batch_sets.push_back(bs);
             }
-            if (k == 0) d.n_dc_tab = d.n_tab;
         }
-        for (int c = 0; c < h.ncomp; c++) {
-            int &qslot = mult_of_store[ids[3 * c + 2]];
-            if (qslot < 0) {
-                qslot = (int)mult_src.size();
-                mult_src.push_back(ctx->quant_store[ids[3 * c + 2]]->data());
-            }
-            d.q_tab[c] = (uint8_t)qslot;
-        }
-        if (huff_src.size() > 255 || mult_src.size() > 255)
-            return fail(ctx, FFCVB_E_LIMIT, "more than 255 distinct Huffman or quantisation tables in a batch");
+        d.fast_tables = ts.fast;
+        d.n_tab = ts.n_tab;
+        d.n_dc_tab = ts.n_dc_tab;
+        memcpy(d.tab_id, batch_sets[last_set].tab_id, sizeof(d.tab_id));
+        memcpy(d.dc_tab, ts.dc_tab, sizeof(d.dc_tab));
+        memcpy(d.ac_tab, ts.ac_tab, sizeof(d.ac_tab));
+        memcpy(d.q_tab, batch_sets[last_set].q_tab, sizeof(d.q_tab));
         d.block_base = total_blocks;
         total_blocks += d.nblocks;
         if (2 * d.n_tab - d.n_dc_tab > max_tables) max_tables = 2 * d.n_tab - d.n_dc_tab;
@@ -919,7 +1003,7 @@ int stage_impl(ffcvb_ctx *ctx, int slot, const Source &source, const uint64_t *p
             const uint32_t tiles = block_tiles(d);
             for (uint32_t k = 0; k < tiles; k++) blk_tiles.push_back(make_uint2((uint32_t)i, k));
         }
-        for (int c = 0; c < h.ncomp; c++) {
+        for (int c = 0; c < d.ncomp; c++) {
             d.plane_off[c] = plane_bytes;
             const size_t pw = (size_t)d.mcus_x * (c == 0 ? d.hs * d.bs_luma : d.bs_chroma);
             const size_t ph = (size_t)d.mcus_y * (c == 0 ? d.vs * d.bs_luma : d.bs_chroma);
@@ -1046,11 +1130,17 @@ int stage_impl(ffcvb_ctx *ctx, int slot, const Source &source, const uint64_t *p
     hd.total_bytes = off;
 
     int rc;
-    // The staging buffer is sized for the whole batch although a pinned source uses only part of
-    // it: the part varies from batch to batch, and regrowing page-locked memory stalls the device.
     if (from_fd && off + 64 > s.host_cap) // the payloads already sit in the buffer: it cannot be regrown now
         return fail(ctx, FFCVB_E_ARG, "ffcvb_stage_batch_fd: tables and lists do not fit behind the payloads");
-    if ((rc = grow_host(ctx, s.host, s.host_cap, off + 64))) return rc;
+    // A pinned source needs room for the part that is staged.  That part varies from batch to batch and
+    // regrowing page-locked memory stalls the device: room for the most that the split may stage.
+    size_t host_need = off;
+    if (direct) {
+        const double most = ctx->adaptive_split ? kMaxAdaptiveShare : ctx->cpu_share_permille / 1000.0;
+        host_need = hd.payload_off + (size_t)(most * (double)(off - hd.payload_off));
+        if (host_need < s.staged_end) host_need = s.staged_end;
+    }
+    if ((rc = grow_host(ctx, s.host, s.host_cap, host_need + 64))) return rc;
     if ((rc = grow_dev(ctx, s.blob, off + 64))) return rc;
     if ((rc = grow_dev(ctx, s.clean, clean_bytes + 512))) return rc;
     if ((rc = grow_dev(ctx, s.segs, segs.size() * (sizeof(SegMeta) + 4 * kSegSubs + 16) + 64))) return rc;
@@ -1269,7 +1359,14 @@ static int run_batch(ffcvb_ctx *ctx, Slot &s, cudaStream_t st, void *out_dev, bo
         CU(cudaMemcpyAsync(blob, s.host, hd.payload_off, cudaMemcpyHostToDevice, s.gather_stream));
         CU(cudaEventRecord(s.ev_gather_start, s.gather_stream)); // after the head's copy: that one queues behind other batches' transfers
         s.gather_timed = true;
-        launch_gather_payloads(reinterpret_cast<const ImageDesc *>(blob + hd.desc_off), s.n, blob, ctx->gather_ctas, ctx->gather_in_flight, s.gather_stream);
+        static_assert(FFCVB_MAX_RIDERS <= sizeof(SmallCopies::off) / sizeof(uint64_t), "a batch's riders fit one launch");
+        SmallCopies small{};
+        for (const auto &r : s.riders) {
+            small.off[small.n] = r.off;
+            small.bytes[small.n] = r.bytes;
+            small.dst[small.n++] = (uint8_t *)r.dst_dev;
+        }
+        launch_gather_payloads(reinterpret_cast<const ImageDesc *>(blob + hd.desc_off), s.n, blob, small, ctx->gather_ctas, ctx->gather_in_flight, s.gather_stream);
         CU(cudaEventRecord(s.ev_gathered, s.gather_stream));
         if (s.staged_end > hd.payload_off) { // the CPU-staged share rides the copy engine meanwhile
             if ((hrc = hold_for_copy(ctx, s, st))) return hrc;
@@ -1278,7 +1375,7 @@ static int run_batch(ffcvb_ctx *ctx, Slot &s, cudaStream_t st, void *out_dev, bo
         }
         CU(cudaStreamWaitEvent(st, s.ev_gathered, 0));
     }
-    if (copy)
+    if (copy && !s.direct)
         for (const auto &r : s.riders)
             if (r.bytes) CU(cudaMemcpyAsync(r.dst_dev, blob + r.off, r.bytes, cudaMemcpyDeviceToDevice, st));
     if (prof) CU(cudaEventRecord(s.ev[1], st));
@@ -1526,22 +1623,27 @@ int ffcvb_batch_status(ffcvb_ctx *ctx, int slot, void *stream, int32_t *status, 
     return bad;
 }
 
+} // extern "C"
+
 // Small per-call parameter arrays travel through a ring of sixteen pinned/device buffer pairs: copies
-// `bytes` from `host` into the next pair (plus `extra` bytes of uninitialised device scratch behind
-// them) on `st`.  The caller records a->ev on `st` once its kernels are queued.
-static int stage_aux(ffcvb_ctx *ctx, cudaStream_t st, const void *host, size_t bytes, size_t extra, AuxBuf **out) {
+// the `bytes` that `fill` writes to the next pair's device side on `st`.  The caller records a->ev on
+// `st` once its kernels are queued.
+template <class Fill>
+static int stage_aux(ffcvb_ctx *ctx, cudaStream_t st, size_t bytes, Fill &&fill, AuxBuf **out) {
     AuxBuf &a = ctx->aux[ctx->aux_next];
     ctx->aux_next = (ctx->aux_next + 1) % 16;
     if (!a.ev) CU(cudaEventCreateWithFlags(&a.ev, cudaEventDisableTiming));
     if (a.used) CU(cudaEventSynchronize(a.ev));
     int rc;
-    if ((rc = grow_dev(ctx, a.dev, bytes + extra))) return rc;
+    if ((rc = grow_dev(ctx, a.dev, bytes))) return rc;
     if ((rc = grow_host(ctx, a.host, a.host_cap, bytes))) return rc;
-    memcpy(a.host, host, bytes);
+    fill(a.host);
     CU(cudaMemcpyAsync(a.dev.p, a.host, bytes, cudaMemcpyHostToDevice, st));
     *out = &a;
     return FFCVB_OK;
 }
+
+extern "C" {
 
 int ffcvb_transform_device(ffcvb_ctx *ctx, void *stream, const uint8_t *src_dev, int n, int h, int w,
                            const ffcvb_plan *plan, const int32_t *params, void *out_dev) {
@@ -1554,7 +1656,7 @@ int ffcvb_transform_device(ffcvb_ctx *ctx, void *stream, const uint8_t *src_dev,
     const size_t bytes = sizeof(int32_t) * (size_t)n * n_params;
     AuxBuf *ap;
     int rc;
-    if ((rc = stage_aux(ctx, st, params, bytes, 0, &ap))) return rc;
+    if ((rc = stage_aux(ctx, st, bytes, [&](uint8_t *host) { memcpy(host, params, bytes); }, &ap))) return rc;
     AuxBuf &a = *ap;
     ResizeSource src{};
     src.uniform = src_dev;
@@ -1568,29 +1670,94 @@ int ffcvb_transform_device(ffcvb_ctx *ctx, void *stream, const uint8_t *src_dev,
     return FFCVB_OK;
 }
 
+// `values` per image; pixels unless it is no multiple of three (mixup alone)
+static int pixel_chain(ffcvb_ctx *ctx, void *stream, const uint8_t *src_dev, int n, int64_t values, int n_ops, const int32_t *kinds,
+                       const uint8_t *apply, const double *ratio, const double *lam, int out_size, const void *lut_dev, void *dst_dev) {
+    const int64_t pixels = values / 3;
+    const bool bytes_only = values % 3 != 0 && n_ops == 0 && lam && out_size == 1;
+    if (!src_dev || !dst_dev || n <= 0 || values <= 0 || (values % 3 != 0 && !bytes_only) || pixels > (int64_t)1 << 30 || n_ops < 0 || n_ops > kMaxChainOps ||
+        (n_ops > 0 && (!kinds || !apply || !ratio)) || (out_size != 1 && out_size != 2 && out_size != 4) || (out_size != 1 && !lut_dev) ||
+        (lam && src_dev == dst_dev) || (out_size != 1 && src_dev == dst_dev))
+        return fail(ctx, FFCVB_E_ARG, "ffcvb_pixel_chain: bad argument");
+    PixelChain chain{};
+    chain.n = n;
+    chain.n_ops = n_ops;
+    for (int k = 0; k < n_ops; k++) {
+        if (kinds[k] < FFCVB_JITTER_BRIGHTNESS || kinds[k] > FFCVB_JITTER_SATURATION)
+            return fail(ctx, FFCVB_E_ARG, "ffcvb_pixel_chain: unknown operation %d", kinds[k]);
+        chain.kind[k] = kinds[k];
+    }
+    for (int i = 0; lam && i < n; i++)
+        if (!(lam[i] >= 0.0 && lam[i] <= 1.0)) return fail(ctx, FFCVB_E_ARG, "ffcvb_pixel_chain: lam[%d] outside [0, 1]", i);
+    CU(cudaSetDevice(ctx->device));
+    cudaStream_t st = (cudaStream_t)stream;
+    // [ratio: doubles][lam: doubles][grey sums: zeroes][apply: bytes]
+    const size_t entries = (size_t)n_ops * n, lam_off = sizeof(double) * entries, sums_off = lam_off + (lam ? sizeof(double) * (size_t)n : 0);
+    const size_t apply_off = sums_off + sizeof(unsigned long long) * entries, bytes = apply_off + entries;
+    uint8_t *dev = nullptr;
+    AuxBuf *a = nullptr;
+    if (bytes > 0) {
+        int rc;
+        if ((rc = stage_aux(ctx, st, bytes, [&](uint8_t *host) {
+                 if (entries) memcpy(host, ratio, sizeof(double) * entries);
+                 if (lam) memcpy(host + lam_off, lam, sizeof(double) * (size_t)n);
+                 memset(host + sums_off, 0, sizeof(unsigned long long) * entries);
+                 if (entries) memcpy(host + apply_off, apply, entries);
+             }, &a)))
+            return rc;
+        dev = (uint8_t *)a->dev.p;
+        chain.ratio = (const double *)dev;
+        chain.lam = lam ? (const double *)(dev + lam_off) : nullptr;
+        chain.grey_sum = (unsigned long long *)(dev + sums_off);
+        chain.apply = dev + apply_off;
+    }
+    if (bytes_only)
+        launch_mixup_bytes(src_dev, (uint8_t *)dst_dev, (long long)values, chain, st);
+    else
+        launch_pixel_chain(src_dev, dst_dev, (int)pixels, chain, out_size, lut_dev, st);
+    CU(cudaGetLastError());
+    if (a) {
+        CU(cudaEventRecord(a->ev, st));
+        a->used = true;
+    }
+    return FFCVB_OK;
+}
+
+int ffcvb_pixel_chain(ffcvb_ctx *ctx, void *stream, const uint8_t *src_dev, int n, int64_t pixels, int n_ops, const int32_t *kinds,
+                      const uint8_t *apply, const double *ratio, const double *lam, int out_size, const void *lut_dev, void *dst_dev) {
+    if (!ctx) return FFCVB_E_ARG;
+    return pixel_chain(ctx, stream, src_dev, n, 3 * pixels, n_ops, kinds, apply, ratio, lam, out_size, lut_dev, dst_dev);
+}
+
+int ffcvb_onehot_mix(ffcvb_ctx *ctx, void *stream, int n, int classes, const int32_t *label, const float *lam, float *dst_dev) {
+    if (!ctx) return FFCVB_E_ARG;
+    if (n <= 0 || classes <= 0 || !label || !lam || !dst_dev) return fail(ctx, FFCVB_E_ARG, "ffcvb_onehot_mix: bad argument");
+    for (int i = 0; i < n; i++)
+        if (label[i] < 0 || label[i] >= classes) return fail(ctx, FFCVB_E_ARG, "ffcvb_onehot_mix: label[%d] = %d with %d classes", i, label[i], classes);
+    CU(cudaSetDevice(ctx->device));
+    cudaStream_t st = (cudaStream_t)stream;
+    AuxBuf *a;
+    int rc;
+    if ((rc = stage_aux(ctx, st, 8 * (size_t)n, [&](uint8_t *host) {
+             memcpy(host, label, 4 * (size_t)n);
+             memcpy(host + 4 * (size_t)n, lam, 4 * (size_t)n);
+         }, &a)))
+        return rc;
+    launch_onehot_mix(dst_dev, n, classes, (const int32_t *)a->dev.p, (const float *)a->dev.p + n, st);
+    CU(cudaGetLastError());
+    CU(cudaEventRecord(a->ev, st));
+    a->used = true;
+    return FFCVB_OK;
+}
+
 int ffcvb_color_jitter(ffcvb_ctx *ctx, void *stream, uint8_t *images_dev, int n, int h, int w, int kind,
                        const uint8_t *apply, const double *ratio) {
     if (!ctx) return FFCVB_E_ARG;
     if (!images_dev || n <= 0 || h <= 0 || w <= 0 || kind < 0 || kind > 2 || !apply || !ratio ||
         (int64_t)h * w > (int64_t)1 << 30)
         return fail(ctx, FFCVB_E_ARG, "ffcvb_color_jitter: bad argument");
-    CU(cudaSetDevice(ctx->device));
-    cudaStream_t st = (cudaStream_t)stream;
-    // [ratio: n doubles][apply: n bytes, padded][grey sums: n counters (device only)]
-    const size_t apply_off = sizeof(double) * (size_t)n, sums_off = align_up(apply_off + n, 8);
-    std::vector<uint8_t> pack(sums_off, 0);
-    memcpy(pack.data(), ratio, sizeof(double) * (size_t)n);
-    memcpy(pack.data() + apply_off, apply, (size_t)n);
-    AuxBuf *a;
-    int rc;
-    if ((rc = stage_aux(ctx, st, pack.data(), sums_off, sizeof(unsigned long long) * (size_t)n, &a))) return rc;
-    uint8_t *dev = (uint8_t *)a->dev.p;
-    launch_color_jitter(images_dev, n, h, w, kind, dev + apply_off, (const double *)dev,
-                        (unsigned long long *)(dev + sums_off), st);
-    CU(cudaGetLastError());
-    CU(cudaEventRecord(a->ev, st));
-    a->used = true;
-    return FFCVB_OK;
+    const int32_t kinds[1] = {kind};
+    return ffcvb_pixel_chain(ctx, stream, images_dev, n, (int64_t)h * w, 1, kinds, apply, ratio, nullptr, 1, nullptr, images_dev);
 }
 
 int ffcvb_mixup(ffcvb_ctx *ctx, void *stream, const uint8_t *src_dev, uint8_t *dst_dev, int n, int64_t count,
@@ -1598,18 +1765,7 @@ int ffcvb_mixup(ffcvb_ctx *ctx, void *stream, const uint8_t *src_dev, uint8_t *d
     if (!ctx) return FFCVB_E_ARG;
     if (!src_dev || !dst_dev || src_dev == dst_dev || n <= 0 || count <= 0 || !lam)
         return fail(ctx, FFCVB_E_ARG, "ffcvb_mixup: bad argument");
-    for (int i = 0; i < n; i++)
-        if (!(lam[i] >= 0.0 && lam[i] <= 1.0)) return fail(ctx, FFCVB_E_ARG, "ffcvb_mixup: lam[%d] outside [0, 1]", i);
-    CU(cudaSetDevice(ctx->device));
-    cudaStream_t st = (cudaStream_t)stream;
-    AuxBuf *a;
-    int rc;
-    if ((rc = stage_aux(ctx, st, lam, sizeof(double) * (size_t)n, 0, &a))) return rc;
-    launch_mixup(src_dev, dst_dev, n, (long long)count, (const double *)a->dev.p, st);
-    CU(cudaGetLastError());
-    CU(cudaEventRecord(a->ev, st));
-    a->used = true;
-    return FFCVB_OK;
+    return pixel_chain(ctx, stream, src_dev, n, count, 0, nullptr, nullptr, nullptr, lam, 1, nullptr, dst_dev);
 }
 
 int ffcvb_poison(ffcvb_ctx *ctx, void *stream, uint8_t *images_dev, int n, int64_t count, const uint8_t *apply,
@@ -1621,7 +1777,7 @@ int ffcvb_poison(ffcvb_ctx *ctx, void *stream, uint8_t *images_dev, int n, int64
     cudaStream_t st = (cudaStream_t)stream;
     AuxBuf *a;
     int rc;
-    if ((rc = stage_aux(ctx, st, apply, (size_t)n, 0, &a))) return rc;
+    if ((rc = stage_aux(ctx, st, (size_t)n, [&](uint8_t *host) { memcpy(host, apply, (size_t)n); }, &a))) return rc;
     launch_poison(images_dev, n, (long long)count, (const uint8_t *)a->dev.p, one_minus_alpha_dev, mask_dev,
                   (float)clamp_lo, (float)clamp_hi, st);
     CU(cudaGetLastError());

@@ -10,9 +10,14 @@ namespace ffcvb {
 // congest the memory system for the decode kernels running beside it.
 template <int kInFlight>
 __global__ void __launch_bounds__(256)
-gather_payloads_kernel(const ImageDesc *__restrict__ descs, int n, uint8_t *__restrict__ blob) {
+gather_payloads_kernel(const ImageDesc *__restrict__ descs, int n, uint8_t *__restrict__ blob, const __grid_constant__ SmallCopies small) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
-    for (int i = blockIdx.x; i < n; i += gridDim.x) {
+    if (blockIdx.x == gridDim.x - 1) { // one CTA of its own: values that arrived with the head of the blob
+        for (int k = 0; k < small.n; k++)
+            for (uint64_t b = threadIdx.x; b < small.bytes[k]; b += blockDim.x) small.dst[k][b] = blob[small.off[k] + b];
+        return;
+    }
+    for (int i = blockIdx.x; i < n; i += gridDim.x - 1) {
         const ImageDesc &d = descs[i];
         if (d.src_addr == 0 || d.payload_size == 0) continue;
         const uint8_t *src = reinterpret_cast<const uint8_t *>(d.src_addr);
@@ -81,14 +86,14 @@ gather_payloads_kernel(const ImageDesc *__restrict__ descs, int n, uint8_t *__re
     }
 }
 
-void launch_gather_payloads(const ImageDesc *descs, int n, uint8_t *blob, int ctas, int in_flight, cudaStream_t stream) {
+void launch_gather_payloads(const ImageDesc *descs, int n, uint8_t *blob, const SmallCopies &small, int ctas, int in_flight, cudaStream_t stream) {
     if (n <= 0) return;
     if (ctas < 1) ctas = kGatherCtas;
-    const int grid = n < ctas ? n : ctas;
+    const int grid = (n < ctas ? n : ctas) + 1;
     if (in_flight >= 8)
-        gather_payloads_kernel<8><<<grid, 256, 0, stream>>>(descs, n, blob);
+        gather_payloads_kernel<8><<<grid, 256, 0, stream>>>(descs, n, blob, small);
     else
-        gather_payloads_kernel<4><<<grid, 256, 0, stream>>>(descs, n, blob);
+        gather_payloads_kernel<4><<<grid, 256, 0, stream>>>(descs, n, blob, small);
 }
 
 } // namespace ffcvb

@@ -11,8 +11,14 @@ namespace ffcvb {
 // PCIe) into its place in the device blob.  Source and destination share their alignment mod 16.
 // `ctas`: CTAs of 256 threads that fetch (< 1: kGatherCtas); `in_flight`: 16-byte loads a thread
 // of a JPEG payload's copy has outstanding (4 or 8).
+// `small`: copies from the blob's head to other device buffers that ride along.
 constexpr int kGatherCtas = 16;
-void launch_gather_payloads(const ImageDesc *descs, int n, uint8_t *blob, int ctas, int in_flight, cudaStream_t stream);
+struct SmallCopies {
+    int n;
+    uint64_t off[8], bytes[8];
+    uint8_t *dst[8];
+};
+void launch_gather_payloads(const ImageDesc *descs, int n, uint8_t *blob, const SmallCopies &small, int ctas, int in_flight, cudaStream_t stream);
 
 // Scratch and results of the entropy decode of a batch (device memory, no initialisation needed
 // except `done`, which starts at zero once and is left at zero).
@@ -88,14 +94,28 @@ void launch_resize_augment(const ResizeSource &src, int n, const int32_t *params
 // Colour jitter kinds (ffcv/transforms/color_jitter.py).
 enum { kJitterBrightness = 0, kJitterContrast = 1, kJitterSaturation = 2 };
 
-// Brightness / contrast / saturation of the images of a uint8 [n, h, w, 3] batch whose apply[i]
-// is non-zero, in place, with factor ratio[i].  grey_sum: n scratch counters (contrast only).
-void launch_color_jitter(uint8_t *images, int n, int h, int w, int kind, const uint8_t *apply,
-                         const double *ratio, unsigned long long *grey_sum, cudaStream_t stream);
+// A chain of them on a uint8 batch of n images, optionally followed by mixup.  All pointers are device
+// pointers; apply and ratio hold n entries per operation, grey_sum too (zero at the start; used
+// by contrasts); lam: n mixup factors, or nullptr.
+constexpr int kMaxChainOps = 8;
+struct PixelChain {
+    int n, n_ops;
+    int kind[kMaxChainOps];
+    const uint8_t *apply;
+    const double *ratio;
+    unsigned long long *grey_sum;
+    const double *lam;
+};
+// src [n, pixels, 3] uint8 through the chain into dst [n, pixels, 3] of out_size bytes per value: 1
+// (dst may be src unless there is mixup), or 2 / 4 with the values of the 256 x 3 table `lut`.
+void launch_pixel_chain(const uint8_t *src, void *dst, int pixels, const PixelChain &chain, int out_size, const void *lut,
+                        cudaStream_t stream);
 
-// dst[i] = lam[i] * src[i] + (1 - lam[i]) * src[i - 1] over `count` uint8 values per image.
-void launch_mixup(const uint8_t *src, uint8_t *dst, int n, long long count, const double *lam,
-                  cudaStream_t stream);
+// The mixup alone on images of `count` values.
+void launch_mixup_bytes(const uint8_t *src, uint8_t *dst, long long count, const PixelChain &chain, cudaStream_t stream);
+
+// Soft one-hot rows [n, classes]: lam[i] at label[i], then 1 - lam[i] at label[i - 1].
+void launch_onehot_mix(float *dst, int n, int classes, const int32_t *label, const float *lam, cudaStream_t stream);
 
 // images[i] = clamp(images[i] * one_minus_alpha + mask) for the images with apply[i] != 0.
 void launch_poison(uint8_t *images, int n, long long count, const uint8_t *apply, const double *one_minus_alpha,

@@ -11,94 +11,184 @@
 //   brightness, contrast:  fma(t, v, (1 - t) * s)     (s = 0, or the mean of the grey image)
 //   saturation:            t * v + (1 - t) * grey      (not fused)
 //   mixup:                 fma(1 - t, partner, t * v)
-// HBM-bound byte work: each kernel reads and writes every byte of the selected images once.
+// Colour jitter, mixup and the normalisation behind them run as one chain: a thread takes four pixels
+// through every operation in registers, so a batch is read once (twice with mixup, and once more for
+// every contrast, which needs the mean of the image as the operations before it leave it) and written
+// once.  Bound by HBM for one operation and by the double-precision pipe for longer chains: bytes become
+// doubles, and doubles bytes, by an addition of 2^52 instead of the slow conversion instructions.
 #include "kernels.h"
 
 namespace ffcvb {
 
 namespace {
 
+// A byte as a double: 2^52 + v has v in its low word.
+__device__ __forceinline__ double to_double(uint32_t v) { return __dsub_rn(__hiloint2double(0x43300000, (int)v), 4503599627370496.0); }
+
+// A double truncated to a byte, clamped to 0 .. 255 (|v| < 2^31): the addition rounds down, and where
+// that differs from truncation the value is negative and becomes 0.
 __device__ __forceinline__ uint32_t clip_u8(double v) {
-    v = fmax(v, 0.0);
-    v = fmin(v, 255.0);
-    return __double2uint_rz(v);
+    const int i = __double2loint(__dadd_rd(v, 6755399441055744.0)); // 1.5 * 2^52
+    return (uint32_t)min(255, max(0, i));
 }
 
-__device__ __forceinline__ uint32_t grey_u8(uint32_t r, uint32_t g, uint32_t b) {
-    return __double2uint_rz(__fma_rn(0.114, (double)b, __fma_rn(0.587, (double)g, __dmul_rn(0.2989, (double)r))));
+__device__ __forceinline__ uint32_t grey_u8(const uint32_t (&v)[3]) {
+    return clip_u8(__fma_rn(0.114, to_double(v[2]), __fma_rn(0.587, to_double(v[1]), __dmul_rn(0.2989, to_double(v[0])))));
 }
 
 __device__ __forceinline__ uint32_t byte_of(const uint32_t (&w)[3], int k) { return (w[k >> 2] >> (8 * (k & 3))) & 255u; }
 
-// One thread per group of four pixels (12 bytes = three aligned words when `pixels` is a multiple
-// of four, which the launcher checks; otherwise one thread per pixel with byte accesses).
-template <int KIND, bool VEC>
-__global__ void __launch_bounds__(256)
-jitter_kernel(uint8_t *__restrict__ images, int pixels, const uint8_t *__restrict__ apply,
-              const double *__restrict__ ratio, const unsigned long long *__restrict__ grey_sum) {
-    const int img = blockIdx.y;
-    if (!apply[img]) return;
-    const double t = ratio[img], u = __dsub_rn(1.0, t);
-    double c = 0.0;
-    if (KIND == kJitterBrightness) c = __dmul_rn(u, 0.0);
-    if (KIND == kJitterContrast) c = __dmul_rn(u, __ddiv_rn((double)grey_sum[img], (double)pixels));
-    uint8_t *base = images + (size_t)img * pixels * 3;
-    const int per = VEC ? 4 : 1;
-    for (int p0 = (blockIdx.x * blockDim.x + threadIdx.x) * per; p0 < pixels; p0 += gridDim.x * blockDim.x * per) {
-        uint32_t w[3];
-        if (VEC) {
-            const uint32_t *src = reinterpret_cast<const uint32_t *>(base + (size_t)p0 * 3);
-            w[0] = src[0];
-            w[1] = src[1];
-            w[2] = src[2];
+struct ChainStep {
+    double t, u, c; // factor, 1 - factor, what brightness and contrast add
+    int kind;       // < 0: not applied to this image
+    bool wide;      // a factor so large (or not a number) that clip_u8 needs its argument clamped first
+};
+
+// The operations [0, n_ops) of image `img`, worked out by the first n_ops threads of the CTA.
+__device__ __forceinline__ void chain_steps(ChainStep *s, const PixelChain &chain, int n_ops, int img, int pixels, int k) {
+    if (k >= n_ops) return;
+    const size_t at = (size_t)k * chain.n + img;
+    ChainStep st{chain.ratio[at], 0.0, 0.0, chain.kind[k], false};
+    st.wide = !(fabs(st.t) < 1e6);
+    st.u = __dsub_rn(1.0, st.t);
+    if (st.kind == kJitterBrightness) st.c = __dmul_rn(st.u, 0.0);
+    if (st.kind == kJitterContrast) st.c = __dmul_rn(st.u, __ddiv_rn((double)chain.grey_sum[at], (double)pixels));
+    if (!chain.apply[at]) st.kind = -1;
+    s[k] = st;
+}
+
+__device__ __forceinline__ void apply_chain(const ChainStep *s, int n_ops, uint32_t (&v)[3]) {
+    for (int k = 0; k < n_ops; k++) {
+        const int kind = s[k].kind; // (uniform over the CTA)
+        if (kind < 0) continue;
+        const double t = s[k].t;
+        double x[3];
+        if (kind == kJitterSaturation) {
+            const double l = __dmul_rn(s[k].u, to_double(grey_u8(v)));
+#pragma unroll
+            for (int c = 0; c < 3; c++) x[c] = __dadd_rn(__dmul_rn(t, to_double(v[c])), l);
         } else {
-            const uint8_t *src = base + (size_t)p0 * 3;
-            w[0] = src[0] | (src[1] << 8) | (src[2] << 16);
-            w[1] = w[2] = 0;
+            const double add = s[k].c;
+#pragma unroll
+            for (int c = 0; c < 3; c++) x[c] = __fma_rn(t, to_double(v[c]), add);
         }
-        uint32_t o[3] = {0, 0, 0};
+        if (s[k].wide)
+            for (int c = 0; c < 3; c++) x[c] = fmin(fmax(x[c], -1.0), 256.0);
+#pragma unroll
+        for (int c = 0; c < 3; c++) v[c] = clip_u8(x[c]);
+    }
+}
+
+// Four pixels (12 bytes, three aligned words) at pixel p, or one by bytes.
+template <bool VEC>
+__device__ __forceinline__ void load_pixels(const uint8_t *base, int p, uint32_t (&w)[3]) {
+    const uint8_t *src = base + (size_t)p * 3;
+    if (VEC) {
+        const uint32_t *src4 = reinterpret_cast<const uint32_t *>(src);
+        w[0] = src4[0];
+        w[1] = src4[1];
+        w[2] = src4[2];
+    } else {
+        w[0] = src[0] | (src[1] << 8) | (src[2] << 16);
+        w[1] = w[2] = 0;
+    }
+}
+
+// One CTA column per image.  With MIX the image before it in the batch (the last one, for the first)
+// takes the same chain and is blended in.  OutT: bytes, or the bits of the table's floats.
+template <typename OutT, bool VEC, bool MIX>
+__global__ void __launch_bounds__(256)
+chain_kernel(const uint8_t *src, OutT *dst, int pixels, const __grid_constant__ PixelChain chain, const OutT *__restrict__ lut) {
+    constexpr int per = VEC ? 4 : 1;
+    __shared__ ChainStep s_steps[2][kMaxChainOps];
+    __shared__ OutT s_lut[sizeof(OutT) == 1 ? 1 : 768]; // per channel
+    const int img = blockIdx.y, partner = img == 0 ? chain.n - 1 : img - 1;
+    chain_steps(s_steps[0], chain, chain.n_ops, img, pixels, threadIdx.x);
+    if (MIX && threadIdx.x >= 32) chain_steps(s_steps[1], chain, chain.n_ops, partner, pixels, threadIdx.x - 32);
+    if constexpr (sizeof(OutT) > 1)
+        for (int k = threadIdx.x; k < 768; k += blockDim.x) s_lut[(k % 3) * 256 + k / 3] = lut[k];
+    __syncthreads();
+    const double lam = MIX ? chain.lam[img] : 1.0, rest = __dsub_rn(1.0, lam);
+    const uint8_t *a = src + (size_t)img * pixels * 3, *b = src + (size_t)partner * pixels * 3;
+    OutT *o = dst + (size_t)img * pixels * 3;
+    for (int p0 = (blockIdx.x * blockDim.x + threadIdx.x) * per; p0 < pixels; p0 += gridDim.x * blockDim.x * per) {
+        uint32_t w[3], x[3] = {0, 0, 0}, r[3] = {0, 0, 0};
+        load_pixels<VEC>(a, p0, w);
+        if (MIX) load_pixels<VEC>(b, p0, x);
+        OutT out[3 * per];
 #pragma unroll
         for (int q = 0; q < per; q++) {
-            const uint32_t r = byte_of(w, 3 * q), g = byte_of(w, 3 * q + 1), b = byte_of(w, 3 * q + 2);
-            const uint32_t v[3] = {r, g, b};
-            double l = 0.0;
-            if (KIND == kJitterSaturation) l = __dmul_rn(u, (double)grey_u8(r, g, b));
+            uint32_t v[3] = {byte_of(w, 3 * q), byte_of(w, 3 * q + 1), byte_of(w, 3 * q + 2)};
+            apply_chain(s_steps[0], chain.n_ops, v);
+            if (MIX) {
+                uint32_t y[3] = {byte_of(x, 3 * q), byte_of(x, 3 * q + 1), byte_of(x, 3 * q + 2)};
+                apply_chain(s_steps[1], chain.n_ops, y);
 #pragma unroll
-            for (int ch = 0; ch < 3; ch++) {
-                double x;
-                if (KIND == kJitterSaturation)
-                    x = __dadd_rn(__dmul_rn(t, (double)v[ch]), l);
+                for (int c = 0; c < 3; c++) v[c] = clip_u8(__fma_rn(rest, to_double(y[c]), __dmul_rn(lam, to_double(v[c]))));
+            }
+#pragma unroll
+            for (int c = 0; c < 3; c++) {
+                const int k = 3 * q + c;
+                if constexpr (sizeof(OutT) == 1)
+                    r[k >> 2] |= v[c] << (8 * (k & 3));
                 else
-                    x = __fma_rn(t, (double)v[ch], c);
-                const int k = 3 * q + ch;
-                o[k >> 2] |= clip_u8(x) << (8 * (k & 3));
+                    out[k] = s_lut[c * 256 + v[c]];
             }
         }
-        if (VEC) {
-            uint32_t *dst = reinterpret_cast<uint32_t *>(base + (size_t)p0 * 3);
-            dst[0] = o[0];
-            dst[1] = o[1];
-            dst[2] = o[2];
+        OutT *to = o + (size_t)p0 * 3;
+        if constexpr (sizeof(OutT) == 1) {
+            if (VEC) {
+                uint32_t *to4 = reinterpret_cast<uint32_t *>(to);
+                to4[0] = r[0];
+                to4[1] = r[1];
+                to4[2] = r[2];
+            } else {
+                to[0] = (uint8_t)r[0];
+                to[1] = (uint8_t)(r[0] >> 8);
+                to[2] = (uint8_t)(r[0] >> 16);
+            }
+        } else if (VEC) { // (12 values from a multiple of 12 on: 8-byte pieces are aligned)
+#pragma unroll
+            for (int k = 0; k < (int)(12 * sizeof(OutT) / 8); k++) {
+                uint2 piece;
+                if constexpr (sizeof(OutT) == 2)
+                    piece = make_uint2(out[4 * k] | (uint32_t)out[4 * k + 1] << 16, out[4 * k + 2] | (uint32_t)out[4 * k + 3] << 16);
+                else
+                    piece = make_uint2(out[2 * k], out[2 * k + 1]);
+                reinterpret_cast<uint2 *>(to)[k] = piece;
+            }
         } else {
-            uint8_t *dst = base + (size_t)p0 * 3;
-            dst[0] = (uint8_t)o[0];
-            dst[1] = (uint8_t)(o[0] >> 8);
-            dst[2] = (uint8_t)(o[0] >> 16);
+#pragma unroll
+            for (int k = 0; k < 3; k++) to[k] = out[k];
         }
     }
 }
 
-// Sum of the (truncated) grey values of every selected image, for the contrast mean.  Integer
-// sums, so the order of the additions does not matter.
+// Sum of the (truncated) grey values, as the operations before operation `upto` leave them, of every
+// image that operation (a contrast) applies to.  Integer sums, so the order of the additions does not
+// matter.
+template <bool VEC>
 __global__ void __launch_bounds__(256)
-grey_sum_kernel(const uint8_t *__restrict__ images, int pixels, const uint8_t *__restrict__ apply,
-                unsigned long long *__restrict__ grey_sum) {
+grey_sum_kernel(const uint8_t *__restrict__ images, int pixels, const __grid_constant__ PixelChain chain, int upto) {
+    constexpr int per = VEC ? 4 : 1;
+    __shared__ ChainStep s_steps[kMaxChainOps];
     const int img = blockIdx.y;
-    if (!apply[img]) return;
+    const size_t at = (size_t)upto * chain.n + img;
+    if (!chain.apply[at]) return;
+    chain_steps(s_steps, chain, upto, img, pixels, threadIdx.x);
+    __syncthreads();
     const uint8_t *base = images + (size_t)img * pixels * 3;
     unsigned int acc = 0; // at most 2^31 / 255 pixels per thread
-    for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < pixels; p += gridDim.x * blockDim.x)
-        acc += grey_u8(base[(size_t)p * 3], base[(size_t)p * 3 + 1], base[(size_t)p * 3 + 2]);
+    for (int p0 = (blockIdx.x * blockDim.x + threadIdx.x) * per; p0 < pixels; p0 += gridDim.x * blockDim.x * per) {
+        uint32_t w[3];
+        load_pixels<VEC>(base, p0, w);
+#pragma unroll
+        for (int q = 0; q < per; q++) {
+            uint32_t v[3] = {byte_of(w, 3 * q), byte_of(w, 3 * q + 1), byte_of(w, 3 * q + 2)};
+            apply_chain(s_steps, upto, v);
+            acc += grey_u8(v);
+        }
+    }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, o);
     __shared__ unsigned int s_part[8];
@@ -107,38 +197,27 @@ grey_sum_kernel(const uint8_t *__restrict__ images, int pixels, const uint8_t *_
     if (threadIdx.x == 0) {
         unsigned long long total = 0;
         for (int k = 0; k < (int)(blockDim.x >> 5); k++) total += s_part[k];
-        atomicAdd(&grey_sum[img], total);
+        atomicAdd(&chain.grey_sum[at], total);
     }
 }
 
-// dst[i] = lam[i] * src[i] + (1 - lam[i]) * src[i - 1] (image -1 = the last), truncated.
-template <bool VEC>
+// Mixup of images whose values do not group into pixels.
 __global__ void __launch_bounds__(256)
-mixup_kernel(const uint8_t *__restrict__ src, uint8_t *__restrict__ dst, int n, long long count,
-             const double *__restrict__ lam) {
-    const int img = blockIdx.y;
-    const double l = lam[img], u = __dsub_rn(1.0, l);
-    const uint8_t *a = src + (size_t)img * count;
-    const uint8_t *b = src + (size_t)(img == 0 ? n - 1 : img - 1) * count;
-    uint8_t *o = dst + (size_t)img * count;
-    const long long stride = (long long)gridDim.x * blockDim.x;
-    if (VEC) {
-        const uint32_t *a4 = reinterpret_cast<const uint32_t *>(a), *b4 = reinterpret_cast<const uint32_t *>(b);
-        uint32_t *o4 = reinterpret_cast<uint32_t *>(o);
-        for (long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x; k < count / 4; k += stride) {
-            const uint32_t x = a4[k], y = b4[k];
-            uint32_t r = 0;
-#pragma unroll
-            for (int q = 0; q < 4; q++) {
-                const double va = (double)((x >> (8 * q)) & 255u), vb = (double)((y >> (8 * q)) & 255u);
-                r |= (__double2uint_rz(__fma_rn(u, vb, __dmul_rn(l, va))) & 255u) << (8 * q);
-            }
-            o4[k] = r;
-        }
-    } else {
-        for (long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x; k < count; k += stride)
-            o[k] = (uint8_t)__double2uint_rz(__fma_rn(u, (double)b[k], __dmul_rn(l, (double)a[k])));
-    }
+mixup_bytes_kernel(const uint8_t *__restrict__ src, uint8_t *__restrict__ dst, long long count, const __grid_constant__ PixelChain chain) {
+    const int img = blockIdx.y, partner = img == 0 ? chain.n - 1 : img - 1;
+    const double lam = chain.lam[img], rest = __dsub_rn(1.0, lam);
+    const uint8_t *a = src + (size_t)img * count, *b = src + (size_t)partner * count;
+    for (long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x; k < count; k += (long long)gridDim.x * blockDim.x)
+        dst[(size_t)img * count + k] = (uint8_t)clip_u8(__fma_rn(rest, to_double(b[k]), __dmul_rn(lam, to_double(a[k]))));
+}
+
+// Soft labels of mixup: row i holds lam[i] at label i and 1 - lam[i] at the label of the sample before
+// it (which wins where the two are the same).
+__global__ void __launch_bounds__(256)
+onehot_mix_kernel(float *__restrict__ dst, int n, int classes, const int32_t *__restrict__ label, const float *__restrict__ lam) {
+    const int i = blockIdx.x, l0 = label[i], l1 = label[i == 0 ? n - 1 : i - 1];
+    const float a = lam[i], b = __fadd_rn(-a, 1.0f);
+    for (int c = threadIdx.x; c < classes; c += blockDim.x) dst[(size_t)i * classes + c] = c == l1 ? b : (c == l0 ? a : 0.0f);
 }
 
 // Poison: float32 scratch value per element, two statements that each round a float64 result to
@@ -169,38 +248,46 @@ int blocks_for(long long items, int per_block) {
 
 } // namespace
 
-void launch_color_jitter(uint8_t *images, int n, int h, int w, int kind, const uint8_t *apply,
-                         const double *ratio, unsigned long long *grey_sum, cudaStream_t stream) {
-    const int pixels = h * w;
-    const bool vec = pixels % 4 == 0 && (reinterpret_cast<uintptr_t>(images) & 3) == 0;
-    const dim3 grid(blocks_for(pixels / (vec ? 4 : 1), 256), n);
-    if (kind == kJitterContrast) {
-        cudaMemsetAsync(grey_sum, 0, sizeof(unsigned long long) * (size_t)n, stream);
-        grey_sum_kernel<<<dim3(blocks_for(pixels, 256 * 8), n), 256, 0, stream>>>(images, pixels, apply, grey_sum);
-    }
-#define FFCVB_JITTER(K)                                                                            \
-    if (vec)                                                                                       \
-        jitter_kernel<K, true><<<grid, 256, 0, stream>>>(images, pixels, apply, ratio, grey_sum);  \
-    else                                                                                           \
-        jitter_kernel<K, false><<<grid, 256, 0, stream>>>(images, pixels, apply, ratio, grey_sum);
-    if (kind == kJitterBrightness) {
-        FFCVB_JITTER(kJitterBrightness)
-    } else if (kind == kJitterContrast) {
-        FFCVB_JITTER(kJitterContrast)
-    } else {
-        FFCVB_JITTER(kJitterSaturation)
-    }
-#undef FFCVB_JITTER
+void launch_pixel_chain(const uint8_t *src, void *dst, int pixels, const PixelChain &chain, int out_size, const void *lut,
+                        cudaStream_t stream) {
+    const bool vec = pixels % 4 == 0 && ((reinterpret_cast<uintptr_t>(src) & 3) | (reinterpret_cast<uintptr_t>(dst) & (out_size == 1 ? 3 : 7))) == 0;
+    // a few passes per thread: what a CTA sets up serves more pixels
+    const dim3 grid(blocks_for(pixels / (vec ? 4 : 1), 256 * 2), chain.n);
+    for (int k = 0; k < chain.n_ops; k++)
+        if (chain.kind[k] == kJitterContrast) {
+            const dim3 sums(blocks_for(pixels / (vec ? 4 : 1), 256 * 4), chain.n);
+            if (vec)
+                grey_sum_kernel<true><<<sums, 256, 0, stream>>>(src, pixels, chain, k);
+            else
+                grey_sum_kernel<false><<<sums, 256, 0, stream>>>(src, pixels, chain, k);
+        }
+    auto run = [&](auto zero) {
+        using OutT = decltype(zero);
+        auto *out = static_cast<OutT *>(dst);
+        auto *table = static_cast<const OutT *>(lut);
+        if (vec && chain.lam)
+            chain_kernel<OutT, true, true><<<grid, 256, 0, stream>>>(src, out, pixels, chain, table);
+        else if (vec)
+            chain_kernel<OutT, true, false><<<grid, 256, 0, stream>>>(src, out, pixels, chain, table);
+        else if (chain.lam)
+            chain_kernel<OutT, false, true><<<grid, 256, 0, stream>>>(src, out, pixels, chain, table);
+        else
+            chain_kernel<OutT, false, false><<<grid, 256, 0, stream>>>(src, out, pixels, chain, table);
+    };
+    if (out_size == 1)
+        run(uint8_t{});
+    else if (out_size == 2)
+        run(uint16_t{});
+    else
+        run(uint32_t{});
 }
 
-void launch_mixup(const uint8_t *src, uint8_t *dst, int n, long long count, const double *lam,
-                  cudaStream_t stream) {
-    const bool vec = count % 4 == 0 && ((reinterpret_cast<uintptr_t>(src) | reinterpret_cast<uintptr_t>(dst)) & 3) == 0;
-    const dim3 grid(blocks_for(count / (vec ? 4 : 1), 256), n);
-    if (vec)
-        mixup_kernel<true><<<grid, 256, 0, stream>>>(src, dst, n, count, lam);
-    else
-        mixup_kernel<false><<<grid, 256, 0, stream>>>(src, dst, n, count, lam);
+void launch_mixup_bytes(const uint8_t *src, uint8_t *dst, long long count, const PixelChain &chain, cudaStream_t stream) {
+    mixup_bytes_kernel<<<dim3(blocks_for(count, 256), chain.n), 256, 0, stream>>>(src, dst, count, chain);
+}
+
+void launch_onehot_mix(float *dst, int n, int classes, const int32_t *label, const float *lam, cudaStream_t stream) {
+    onehot_mix_kernel<<<n, 256, 0, stream>>>(dst, n, classes, label, lam);
 }
 
 void launch_poison(uint8_t *images, int n, long long count, const uint8_t *apply, const double *one_minus_alpha,

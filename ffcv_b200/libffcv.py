@@ -73,6 +73,11 @@ lib.ffcvb_color_jitter.argtypes = [c_void_p, c_void_p, c_void_p, c_int, c_int, c
 lib.ffcvb_color_jitter.restype = c_int
 lib.ffcvb_mixup.argtypes = [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int64, c_void_p]
 lib.ffcvb_mixup.restype = c_int
+lib.ffcvb_pixel_chain.argtypes = [c_void_p, c_void_p, c_void_p, c_int, c_int64, c_int, c_void_p, c_void_p, c_void_p, c_void_p,
+                                  c_int, c_void_p, c_void_p]
+lib.ffcvb_pixel_chain.restype = c_int
+lib.ffcvb_onehot_mix.argtypes = [c_void_p, c_void_p, c_int, c_int, c_void_p, c_void_p, c_void_p]
+lib.ffcvb_onehot_mix.restype = c_int
 lib.ffcvb_poison.argtypes = [c_void_p, c_void_p, c_void_p, c_int, c_int64, c_void_p, c_void_p, c_void_p,
                              ctypes.c_double, ctypes.c_double]
 lib.ffcvb_poison.restype = c_int
@@ -146,6 +151,21 @@ def _as(a, dtype):
     return np.ascontiguousarray(a, dtype=dtype)
 
 
+class BatchArrays:
+    """The per-sample arrays of a staging call, checked once, for callers that refill the same arrays
+    batch after batch: data pointers, sizes, modes, heights, widths and the parameter table."""
+
+    def __init__(self, ptrs, sizes, modes, heights, widths, params):
+        arrays = (ptrs, sizes, modes, heights, widths, params)
+        for a, dtype in zip(arrays, (np.uint64, np.uint64, np.uint8, np.uint16, np.uint16, np.int32)):
+            if a.dtype != dtype or not a.flags.c_contiguous or len(a) != len(ptrs):
+                raise ValueError('staging arrays must be contiguous, of equal length and of the native types')
+        self.arrays = arrays
+        self.n = len(ptrs)
+        self.n_params = params.shape[1]
+        self.pointers = tuple(c_void_p(a.ctypes.data) for a in arrays)
+
+
 class FFCVBError(RuntimeError):
     pass
 
@@ -199,26 +219,37 @@ class Context:
                                    ctypes.byref(plan), params.ctypes.data)
         self._check(rc, 'ffcvb_stage_batch')
 
+    def stage_arrays(self, slot, file_base, batch, plan):
+        """:meth:`stage` of a :class:`BatchArrays`."""
+        assert batch.n_params == 4 + 2 * plan.n_ops
+        ptrs, sizes, modes, heights, widths, params = batch.pointers
+        if isinstance(file_base, tuple):
+            rc = lib.ffcvb_stage_batch_fd(self._h, slot, file_base[0], file_base[1], ptrs, sizes, modes, heights, widths,
+                                          batch.n, ctypes.byref(plan), params)
+        else:
+            rc = lib.ffcvb_stage_batch(self._h, slot, file_base, ptrs, sizes, modes, heights, widths, batch.n,
+                                       ctypes.byref(plan), params)
+        self._check(rc, 'ffcvb_stage_batch')
+
     def set_riders(self, slot, riders, n):
         """riders: sequence of (values, file_offsets, item_bytes, dst_ptr) -- exactly one of
         `values` (contiguous numpy array of n items) and `file_offsets` (uint64 array of n offsets
         from the file base given to stage) is not None.  Consumed by the next `stage` of the slot."""
         arr = (Rider * max(1, len(riders)))()
         keep = []
-        for k, (values, offsets, item_bytes, dst_ptr) in enumerate(riders):
+        for rider, (values, offsets, item_bytes, dst_ptr) in zip(arr, riders):
             if values is not None:
                 values = np.ascontiguousarray(values)
                 assert values.nbytes == n * item_bytes, (values.nbytes, n, item_bytes)
-                arr[k].host, arr[k].ptrs = values.ctypes.data, None
-                keep.append(values)
+                rider.host = values.ctypes.data
             else:
-                offsets = _as(offsets, np.uint64)
-                assert offsets.shape == (n,)
-                arr[k].host, arr[k].ptrs = None, offsets.ctypes.data
-                keep.append(offsets)
-            arr[k].item_bytes = int(item_bytes)
-            arr[k].dst_dev = int(dst_ptr)
-        self._check(lib.ffcvb_set_batch_riders(self._h, slot, arr, len(riders), int(n)), 'ffcvb_set_batch_riders')
+                values = _as(offsets, np.uint64)
+                assert values.shape == (n,)
+                rider.ptrs = values.ctypes.data
+            keep.append(values)
+            rider.item_bytes = item_bytes
+            rider.dst_dev = dst_ptr
+        self._check(lib.ffcvb_set_batch_riders(self._h, slot, arr, len(riders), n), 'ffcvb_set_batch_riders')
 
     def submit(self, slot, stream, out_ptr):
         self._check(lib.ffcvb_submit_batch(self._h, slot, stream or None, out_ptr), 'ffcvb_submit_batch')
@@ -240,6 +271,19 @@ class Context:
         lam = np.ascontiguousarray(lam, dtype=np.float64)
         assert lam.shape == (n,)
         self._check(lib.ffcvb_mixup(self._h, stream_ptr, src_ptr, dst_ptr, n, count, lam.ctypes.data), 'ffcvb_mixup')
+
+    def pixel_chain(self, stream_ptr, src_ptr, n, pixels, kinds, apply, ratio, lam, out_size, lut_ptr, dst_ptr):
+        """kinds: int32 [ops]; apply: uint8 [ops, n]; ratio: float64 [ops, n]; lam: float64 [n] or None."""
+        assert apply.shape == ratio.shape == (len(kinds), n) and (lam is None or lam.shape == (n,))
+        self._check(lib.ffcvb_pixel_chain(self._h, stream_ptr, src_ptr, n, pixels, len(kinds), kinds.ctypes.data,
+                                          apply.ctypes.data, ratio.ctypes.data, None if lam is None else lam.ctypes.data,
+                                          out_size, lut_ptr or None, dst_ptr), 'ffcvb_pixel_chain')
+
+    def onehot_mix(self, stream_ptr, n, classes, label, lam, dst_ptr):
+        """label: int32 [n]; lam: float32 [n]."""
+        assert label.shape == lam.shape == (n,)
+        self._check(lib.ffcvb_onehot_mix(self._h, stream_ptr, n, classes, label.ctypes.data, lam.ctypes.data, dst_ptr),
+                    'ffcvb_onehot_mix')
 
     def poison(self, stream_ptr, images_ptr, n, count, apply, one_minus_alpha_ptr, mask_ptr, lo, hi):
         apply = np.ascontiguousarray(apply, dtype=np.uint8)

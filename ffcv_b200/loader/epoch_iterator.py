@@ -28,7 +28,7 @@ class EpochIterator(Thread):
     def __init__(self, loader, order: Sequence[int], epoch: int):
         super().__init__(daemon=True)
         self.loader = loader
-        self.order = np.asarray(order)
+        self.order = np.ascontiguousarray(order, dtype=np.int64)
         self.epoch = epoch
         bs = loader.batch_size
         self.batches = [self.order[i:i + bs] for i in range(0, len(self.order), bs)]
@@ -60,6 +60,8 @@ class EpochIterator(Thread):
             start_event = ch.cuda.Event()
             start_event.record(self.current_stream)
         self.consumed = [start_event] * self.slots
+        self.consumed_events = [None] * self.slots  # one event per slot, recorded again and again
+        self.queues_work = loader.graph.queues_work()
         self.last_slot = None
         self.start()
 
@@ -92,25 +94,31 @@ class EpochIterator(Thread):
         if not self.is_cuda:
             return self.loader.graph.run_batch(batch_indices, slot, None, self.buffers, self.storage_state,
                                                self.epoch, b_ix)
-        # The slot's pinned staging buffer is about to be rewritten by the host: the copy and the
-        # kernels of the batch that used it last must have finished (a host-side wait; that batch
-        # was queued batches_ahead + 2 batches ago).
-        if self.slot_done[slot] is not None:
-            self.slot_done[slot].synchronize()
-        with ch.cuda.stream(stream):
-            if cuda_event is not None:
-                cuda_event.wait()
-            lookahead = self.batches[b_ix + 1] if b_ix + 1 < len(self.batches) else None
+        done = self.slot_done[slot]
+        if done is None:
+            done = self.slot_done[slot] = ch.cuda.Event()
+        elif self.queues_work:
+            # Host buffers of the slot are about to be rewritten: what read them must have finished (a
+            # host-side wait; that batch was queued batches_ahead + 2 batches ago).  The native context
+            # waits in the same way for its own staging buffer.
+            done.synchronize()
+        if cuda_event is not None:
+            cuda_event.wait(stream)
+        if self.queues_work:
+            with ch.cuda.stream(stream):
+                result = self.loader.graph.run_batch(batch_indices, slot, stream.cuda_stream, self.buffers,
+                                                     self.storage_state, self.epoch, b_ix)
+        else:
             result = self.loader.graph.run_batch(batch_indices, slot, stream.cuda_stream, self.buffers,
-                                                 self.storage_state, self.epoch, b_ix, lookahead=lookahead)
-            done = ch.cuda.Event()
-            done.record(stream)
-            self.slot_done[slot] = done
-            return result
+                                                 self.storage_state, self.epoch, b_ix)
+        done.record(stream)
+        return result
 
     def __next__(self):
         if self.is_cuda and self.last_slot is not None:
-            event = ch.cuda.Event()
+            event = self.consumed_events[self.last_slot]
+            if event is None:
+                event = self.consumed_events[self.last_slot] = ch.cuda.Event()
             event.record(self.current_stream)
             self.consumed[self.last_slot] = event
             self.last_slot = None
@@ -123,7 +131,7 @@ class EpochIterator(Thread):
             raise item.exc
         slot, result = item
         if self.is_cuda:
-            self.current_stream.wait_stream(self.cuda_streams[slot])
+            self.current_stream.wait_event(self.slot_done[slot])
             self.last_slot = slot
         return result
 

@@ -67,6 +67,7 @@ class OSCacheManager(MemoryManager):
         self.pin = bool(pin)
         self.pinned = False
         self._keepalive = None
+        self._base = None
         self.context = MemoryContext(self)
 
     def open(self):
@@ -163,7 +164,9 @@ class OSCacheManager(MemoryManager):
         return view
 
     def file_base(self):
-        return self.open().ctypes.data
+        if self._base is None:
+            self._base = self.open().ctypes.data
+        return self._base
 
     def schedule_epoch(self, batches):
         return self.context

@@ -7,13 +7,11 @@ operations that implement :meth:`Operation.fuse` becomes a :class:`FusedImagePla
 (or raw) sample bytes go to the GPU and one call of the native library produces the final tensor.
 Operations after the fused prefix run one by one through their ``generate_code`` closures.
 """
-from concurrent.futures import ThreadPoolExecutor
-
 import numpy as np
 import torch as ch
 
 from .. import libffcv as L
-from .sampling import batch_seed
+from .sampling import CROP_CENTER, CROP_RANDOM, CROP_WHOLE, batch_seed, gather_batch, prepare_batch
 
 
 class FusedImagePlan:
@@ -134,6 +132,32 @@ def sample_plan_params(plan, md, base_seed, epoch, batch_ix):
     return params
 
 
+def _native_sampling(plan):
+    """The arguments of :func:`prepare_batch` that draw a plan's parameters, or None when the plan
+    contains an operation that this module does not know (a subclass draws what it likes)."""
+    from ..fields.rgb_image import (CenterCropRGBImageDecoder, RandomResizedCropRGBImageDecoder, SimpleRGBImageDecoder)
+    from ..transforms.cutout import Cutout
+    from ..transforms.flip import RandomHorizontalFlip
+    from ..transforms.random_resized_crop import RandomResizedCrop
+    from ..transforms.translate import RandomTranslate
+    sampler = plan.crop_sampler or plan.decoder
+    scale = ratio = np.zeros(2)
+    if type(sampler) in (RandomResizedCropRGBImageDecoder, RandomResizedCrop):
+        crop, scale, ratio = CROP_RANDOM, np.array(sampler.scale, dtype=np.float64), np.array(sampler.ratio, dtype=np.float64)
+    elif type(sampler) is CenterCropRGBImageDecoder:
+        crop, ratio = CROP_CENTER, np.array([sampler.ratio, 0.0], dtype=np.float64)
+    elif type(sampler) is SimpleRGBImageDecoder:
+        crop = CROP_WHOLE
+    else:
+        return None
+    args = {RandomHorizontalFlip: lambda op: op.flip_prob, RandomTranslate: lambda op: op.padding, Cutout: lambda op: op.crop_size}
+    if any(type(op) not in args for (_, _, _, op) in plan.ops):
+        return None
+    types = np.array([t for (t, _, _, _) in plan.ops], dtype=np.int64)
+    values = np.array([float(args[type(op)](op)) for (_, _, _, op) in plan.ops], dtype=np.float64)
+    return crop, scale, ratio, types, values, int(plan.out_h), int(plan.out_w)
+
+
 class FusedImageExecutor:
     """Per-batch driver of a :class:`FusedImagePlan` on one native context."""
 
@@ -155,38 +179,52 @@ class FusedImageExecutor:
                                        self.table_dev.data_ptr() if self.table_dev is not None else 0,
                                        dct_scale=plan.dct_scale)
         self.n_params = 4 + 2 * len(ops)
+        # the sample table as columns, and the arrays a batch is prepared in (the native call has taken
+        # what it needs when it returns, so one set serves all batches)
+        self.columns = (np.ascontiguousarray(metadata['data_ptr'], dtype=np.uint64),
+                        np.ascontiguousarray(sample_sizes, dtype=np.uint64),
+                        np.ascontiguousarray(metadata['mode'], dtype=np.uint8),
+                        np.ascontiguousarray(metadata['height'], dtype=np.uint16),
+                        np.ascontiguousarray(metadata['width'], dtype=np.uint16))
+        self.sampling = _native_sampling(plan)
+        self._arrays = None
         self.last_params = None
-        self._prepared = None     # ((epoch, batch, n), arrays) drawn ahead for the next batch
         self.param_log = None     # set to a list to record (epoch, batch, indices, parameter table) per batch
-        self.h2d_bytes = 0
-        self.launches = 0
+        self._last_slot = None
         self.riders = []          # other fields' values for the next batch (see Graph.attach_riders)
-        self._helper = None       # one thread that draws the next batch's parameters (see __call__)
+
+    @property
+    def h2d_bytes(self):
+        """Bytes the last batch moved host->device."""
+        return 0 if self._last_slot is None else self.ctx.staged_bytes(self._last_slot)
+
+    @property
+    def launches(self):
+        """Kernels of this library the last batch launched."""
+        return 0 if self._last_slot is None else self.ctx.launches(self._last_slot)
 
     def allocate(self, batch_size, slots):
         p = self.plan
         return [ch.empty((batch_size,) + p.buffer_shape, dtype=p.torch_dtype, device=self.device) for _ in range(slots)]
 
-    def sample_params(self, batch_indices, epoch, batch_ix):
-        md = self.metadata[batch_indices]
-        params = sample_plan_params(self.plan, md, self.base_seed, epoch, batch_ix)
-        return md, np.ascontiguousarray(md['height']), np.ascontiguousarray(md['width']), params
-
     def prepare(self, batch_indices, epoch, batch_ix):
-        """Everything ffcvb_stage_batch needs for one batch, as contiguous arrays."""
-        md, heights, widths, params = self.sample_params(batch_indices, epoch, batch_ix)
-        return (np.ascontiguousarray(md['data_ptr'], dtype=np.uint64),
-                np.ascontiguousarray(self.sample_sizes[batch_indices], dtype=np.uint64),
-                np.ascontiguousarray(md['mode'], dtype=np.uint8), heights, widths, params)
-
-    def __call__(self, batch_indices, slot, stream_ptr, out, epoch, batch_ix, lookahead=None):
-        key = (epoch, batch_ix, len(batch_indices))
-        if self._prepared is not None and self._prepared[0] == key:
-            args = self._prepared[1]
+        """Everything ffcvb_stage_batch needs for one batch: the rows of the sample table and the
+        parameter table, in arrays that the next call overwrites."""
+        batch_indices = np.ascontiguousarray(batch_indices, dtype=np.int64)
+        n = len(batch_indices)
+        if self._arrays is None or len(self._arrays[1]) != n:
+            self._arrays = (tuple(np.empty(n, c.dtype) for c in self.columns), np.zeros((n, self.n_params), dtype=np.int32))
+            self._staging = L.BatchArrays(*self._arrays[0], self._arrays[1])
+        batch, params = self._arrays
+        if self.sampling is not None:
+            prepare_batch(batch_indices, self.columns, batch, self.base_seed, epoch, batch_ix, *self.sampling, params)
         else:
-            args = self.prepare(batch_indices, epoch, batch_ix)
-        self._prepared = None
-        params = args[5]
+            gather_batch(batch_indices, self.columns, batch)
+            params[:] = sample_plan_params(self.plan, self.metadata[batch_indices], self.base_seed, epoch, batch_ix)
+        return params
+
+    def __call__(self, batch_indices, slot, stream_ptr, out, epoch, batch_ix):
+        params = self.prepare(batch_indices, epoch, batch_ix)
         self.last_params = params
         if self.param_log is not None:
             self.param_log.append((epoch, batch_ix, np.array(batch_indices), params.copy()))
@@ -194,24 +232,11 @@ class FusedImageExecutor:
         if self.riders:
             self.ctx.set_riders(slot, self.riders, n)
             self.riders = []
-        # The next batch's parameters are drawn by a helper thread while this thread is inside the
-        # native calls (which release the interpreter lock): the loader thread's time per batch is
-        # what bounds the rate of the low-resolution configurations.
-        ahead = None
-        if lookahead is not None:
-            if self._helper is None:
-                self._helper = ThreadPoolExecutor(max_workers=1, thread_name_prefix='ffcv_b200_params')
-            ahead = self._helper.submit(self.prepare, lookahead, epoch, batch_ix + 1)
-        try:
-            # with asynchronous staging this returns while the staging threads still copy the payloads
-            self.ctx.stage(slot, self.file_base_fn(), *args[:5], self.native_plan, params)
-            dst = out[:n]
-            self.ctx.submit(slot, stream_ptr, dst.data_ptr())
-        finally:
-            if ahead is not None:
-                self._prepared = ((epoch, batch_ix + 1, len(lookahead)), ahead.result())
-        self.h2d_bytes = self.ctx.staged_bytes(slot)
-        self.launches = self.ctx.launches(slot)
+        # with asynchronous staging this returns while the staging threads still copy the payloads
+        self.ctx.stage_arrays(slot, self.file_base_fn(), self._staging, self.native_plan)
+        dst = out if len(out) == n else out[:n]
+        self.ctx.submit(slot, stream_ptr, dst.data_ptr())
+        self._last_slot = slot
         p = self.plan
         if p.torch_image:
             if p.needs_repack():

@@ -20,6 +20,8 @@ from .allocation_query import AllocationQuery, allocate_query
 from .fusion import FusedImageExecutor, FusedImagePlan
 from .pipeline_spec import PipelineSpec
 from .state import State
+from ..transforms.common import Squeeze
+from ..transforms.ops import View
 
 INITIAL_STATE = State(jit_mode=True, device=ch.device('cpu'), dtype=np.dtype('u1'), shape=None)
 
@@ -68,9 +70,12 @@ class _Pipeline:
         self.allocs = []
         self.executor = None  # FusedImageExecutor for the fused prefix
         self.n_fused = 0
-        self.codes = []
+        self.steps = []
+        self.first_step = 0
+        self.soft_labels = None  # the whole label pipeline of mixup as one call
         self.final_state = None
         self.rider_host = None  # index of the image pipeline whose staged bytes carry this field
+        self.column = None      # ... and the field's values or file offsets, contiguous
 
 
 class Graph:
@@ -94,6 +99,13 @@ class Graph:
             self.pipelines.append(_Pipeline(output_name, spec.source, fieldname_to_fix[spec.source],
                                             [spec.decoder] + list(spec.transforms)))
         self.collect_requirements()
+
+    def queues_work(self):
+        """Whether some operation behind the native calls may launch GPU work of its own (it then has
+        to run under the slot's stream)."""
+        return any(p.soft_labels is not None for p in self.pipelines) or \
+            any(chain is not None or type(p.ops[k]) not in (Squeeze, View) for p in self.pipelines for k, chain, _ in p.steps) or \
+            any(p.executor is not None and p.executor.plan.needs_repack() for p in self.pipelines)
 
     def collect_requirements(self):
         """Walks every pipeline root to leaf: ``accept_field``, ``accept_globals``,
@@ -124,8 +136,30 @@ class Graph:
                 p.executor = FusedImageExecutor(plan, self.context_factory(plan.device, pi), column,
                                                 mm.sizes_of(column['data_ptr']), mm.file_base, self.seed)
         self.attach_riders()
+        from .tail import PixelChain, SoftLabels
         for p in self.pipelines:
-            p.codes = [op.generate_code() for op in p.ops[p.n_fused:]]
+            # what is left of the pipeline, in steps: (position behind the step, chain or None, closure)
+            p.steps = []
+            p.soft_labels = None
+            k = p.n_fused
+            if p.executor is None and p.rider_host is None:
+                p.soft_labels = SoftLabels.match(p.ops)
+                if p.soft_labels is not None:
+                    p.column = np.ascontiguousarray(self.metadata[f'f{p.f_ix}'])
+                    k = SoftLabels.n_ops
+            p.first_step = k
+            while k < len(p.ops):
+                # a chain works on what the decoder's plan left: a uint8 batch in the plan's layout
+                plan = p.executor.plan if p.executor is not None else None
+                chain = None
+                if plan is not None and plan.table is None and not plan.torch_image:
+                    chain = PixelChain.match(p.ops, k, (plan.out_h, plan.out_w), p.executor.device)
+                if chain is not None and all(c is None or c.normalize is None for _, c, _ in p.steps):
+                    p.steps.append((k, chain, None))
+                    k = chain.end
+                else:
+                    p.steps.append((k, None, p.ops[k].generate_code()))
+                    k += 1
         return self.pipelines
 
     def attach_riders(self):
@@ -160,6 +194,7 @@ class Graph:
             if not cands:
                 continue
             p.rider_host = cands[0]
+            p.column = np.ascontiguousarray(self.metadata[f'f{p.f_ix}'])
             load[cands[0]] += 1
             p.n_fused = 3
 
@@ -170,8 +205,12 @@ class Graph:
                 buffers[(pi, 'fused')] = p.executor.allocate(batch_size, slots)
             if p.rider_host is not None:
                 buffers[(pi, 'rider')] = allocate_query(p.allocs[2], batch_size, slots)
-            for k in range(p.n_fused, len(p.ops)):
-                alloc = p.allocs[k]
+            owners = [(k, p.allocs[k]) for k, chain, _ in p.steps if chain is None]
+            owners += [(k, p.allocs[chain.buffer_op] if chain.buffer_op is not None else None) for k, chain, _ in p.steps
+                       if chain is not None]
+            if p.soft_labels is not None:
+                owners.append(('soft', p.allocs[p.first_step - 1]))
+            for k, alloc in owners:
                 if isinstance(alloc, AllocationQuery):
                     buffers[(pi, k)] = allocate_query(alloc, batch_size, slots)
                 elif isinstance(alloc, (tuple, list)):
@@ -188,38 +227,40 @@ class Graph:
             return tuple(Graph._select(b, slot, count) for b in buffer)
         return buffer[slot][:count]
 
-    def run_batch(self, batch_indices, slot, stream_ptr, buffers, storage_state, epoch, batch_ix, lookahead=None):
+    def run_batch(self, batch_indices, slot, stream_ptr, buffers, storage_state, epoch, batch_ix):
         """One batch through every pipeline; returns the outputs in declaration order."""
         n = len(batch_indices)
         results = []
         for pi, p in enumerate(self.pipelines):
             if p.rider_host is not None:  # queued before the image pipeline stages its batch
                 dst = buffers[(pi, 'rider')][slot][:n]
-                values = np.ascontiguousarray(self.metadata[f'f{p.f_ix}'][batch_indices])
+                values = p.column[batch_indices]
                 if isinstance(p.ops[0], NDArrayDecoder):
                     rider = (None, values.astype(np.uint64), int(p.ops[0].field.element_size), dst.data_ptr())
                 else:
                     rider = (values, None, values.dtype.itemsize, dst.data_ptr())
                 self.pipelines[p.rider_host].executor.riders.append(rider)
         for pi, p in enumerate(self.pipelines):
+            steps = p.steps
             if p.rider_host is not None:
                 value = buffers[(pi, 'rider')][slot][:n]
-                first = p.n_fused
             elif p.executor is not None:
-                value = p.executor(batch_indices, slot, stream_ptr, buffers[(pi, 'fused')][slot], epoch, batch_ix,
-                                   lookahead=lookahead)
-                first = p.n_fused
+                value = p.executor(batch_indices, slot, stream_ptr, buffers[(pi, 'fused')][slot], epoch, batch_ix)
+            elif p.soft_labels is not None:
+                value = p.soft_labels(p.column, buffers[(pi, 'soft')][slot][:n], batch_indices)
             else:
-                code = p.codes[0]
-                value = code(batch_indices, self._select(buffers[(pi, 0)], slot, n),
+                k, _, code = steps[0]
+                value = code(batch_indices, self._select(buffers[(pi, k)], slot, n),
                              self.metadata[f'f{p.f_ix}'], storage_state)
-                first = 1
-            for k in range(first, len(p.ops)):
+                steps = steps[1:]
+            for k, chain, code in steps:
+                mem = self._select(buffers[(pi, k)], slot, n)
+                if chain is not None:
+                    value = chain(value, mem, batch_indices, self.seed, epoch, batch_ix, pi)
+                    continue
                 begin = getattr(p.ops[k], 'begin_batch', None)
                 if begin is not None:  # operations that draw random numbers of their own
                     begin(self.seed, epoch, batch_ix, pi * 64 + k)
-                code = p.codes[k - p.n_fused]
-                mem = self._select(buffers[(pi, k)], slot, n)
                 if getattr(code, 'with_indices', False):
                     value = code(value, mem, batch_indices)
                 else:

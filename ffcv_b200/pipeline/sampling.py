@@ -109,6 +109,65 @@ def sample_cutouts(seed, n, height, width, crop_size, out):
 
 
 @njit(**_JIT)
+def _batch_seed(base_seed, epoch, batch_ix, op_ix):
+    # batch_seed in 64-bit arithmetic
+    x = (np.uint64(base_seed) * np.uint64(0x9E3779B97F4A7C15) + np.uint64(epoch) * np.uint64(0xBF58476D1CE4E5B9) +
+         np.uint64(batch_ix) * np.uint64(0x94D049BB133111EB) + np.uint64(op_ix) * np.uint64(0xD6E8FEB86659FD93))
+    x ^= x >> np.uint64(30)
+    x *= np.uint64(0xBF58476D1CE4E5B9)
+    x ^= x >> np.uint64(27)
+    x *= np.uint64(0x94D049BB133111EB)
+    x ^= x >> np.uint64(31)
+    return np.uint32(x & np.uint64(0xFFFFFFFF))
+
+
+CROP_WHOLE, CROP_RANDOM, CROP_CENTER = 0, 1, 2
+OP_FLIP, OP_TRANSLATE, OP_CUTOUT = 1, 2, 3  # ffcv_b200.libffcv's
+
+
+@njit(**_JIT)
+def gather_batch(indices, columns, batch):
+    # the batch's rows of the sample table: (data pointer, size, mode, height, width)
+    for k in range(indices.shape[0]):
+        i = indices[k]
+        batch[0][k] = columns[0][i]
+        batch[1][k] = columns[1][i]
+        batch[2][k] = columns[2][i]
+        batch[3][k] = columns[3][i]
+        batch[4][k] = columns[4][i]
+
+
+@njit(**_JIT)
+def prepare_batch(indices, columns, batch, base_seed, epoch, batch_ix, crop, scale, ratio, op_types, op_args,
+                  out_h, out_w, params):
+    # gather_batch and the whole parameter table of a batch in one call: the same draws, operation by
+    # operation, as the functions above
+    gather_batch(indices, columns, batch)
+    heights = batch[3]
+    widths = batch[4]
+    if crop == CROP_RANDOM:
+        sample_random_crops(_batch_seed(base_seed, epoch, batch_ix, 0), heights, widths, scale, ratio, params)
+    elif crop == CROP_CENTER:
+        sample_center_crops(heights, widths, ratio[0], params)
+    else:
+        for k in range(indices.shape[0]):
+            params[k, 0] = 0
+            params[k, 1] = 0
+            params[k, 2] = heights[k]
+            params[k, 3] = widths[k]
+    n = indices.shape[0]
+    for o in range(op_types.shape[0]):
+        seed = _batch_seed(base_seed, epoch, batch_ix, o + 1)
+        column = params[:, 4 + 2 * o:6 + 2 * o]
+        if op_types[o] == OP_FLIP:
+            sample_flips(seed, n, op_args[o], column)
+        elif op_types[o] == OP_TRANSLATE:
+            sample_translations(seed, n, int(op_args[o]), column)
+        else:
+            sample_cutouts(seed, n, out_h, out_w, int(op_args[o]), column)
+
+
+@njit(**_JIT)
 def sample_jitter(seed, n, p, low, high, apply, ratio):
     # the two vector draws of ffcv/transforms/color_jitter.py:44-45 (:86-87, :124-125), in that order
     np.random.seed(seed)

@@ -19,12 +19,15 @@ class _Jitter(DevicePixelOp):
         self.p = p
         self.magnitude = magnitude
 
+    def draw_into(self, apply, ratio):
+        sample_jitter(self.next_seed(), len(apply), float(self.p), float(max(0, 1 - self.magnitude)),
+                      float(1 + self.magnitude), apply, ratio)
+        self.last_draw = (apply, ratio)
+
     def draw(self, n):
         apply = np.zeros(n, dtype=np.uint8)
         ratio = np.zeros(n, dtype=np.float64)
-        sample_jitter(self.next_seed(), n, float(self.p), float(max(0, 1 - self.magnitude)),
-                      float(1 + self.magnitude), apply, ratio)
-        self.last_draw = (apply, ratio)
+        self.draw_into(apply, ratio)
         return apply, ratio
 
     def generate_code(self) -> Callable:

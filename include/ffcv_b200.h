@@ -272,6 +272,21 @@ int ffcvb_color_jitter(ffcvb_ctx *ctx, void *stream, uint8_t *images_dev, int n,
 int ffcvb_mixup(ffcvb_ctx *ctx, void *stream, const uint8_t *src_dev, uint8_t *dst_dev, int n, int64_t count,
                 const double *lam);
 
+/* A chain of the above in one call: the batch `src_dev` ([n, pixels, 3] uint8) goes through n_ops (at
+ * most 8) jitter operations in order, operation k being kinds[k] with apply[k * n + i] and
+ * ratio[k * n + i] for image i; then, when lam is not NULL, through ImageMixup; then, when out_size is 2
+ * or 4, through the 256 x 3 normalisation table `lut_dev` of that value size (normalize.py:58-109), into
+ * `dst_dev` ([n, pixels, 3] values of out_size bytes).  dst_dev may be src_dev only when out_size is 1
+ * and lam is NULL.  Same results as the single calls. */
+int ffcvb_pixel_chain(ffcvb_ctx *ctx, void *stream, const uint8_t *src_dev, int n, int64_t pixels, int n_ops,
+                      const int32_t *kinds, const uint8_t *apply, const double *ratio, const double *lam,
+                      int out_size, const void *lut_dev, void *dst_dev);
+
+/* MixupToOneHot of LabelMixup (mixup.py:66-121): row i of the float32 matrix dst_dev [n, classes] is zero
+ * except for lam[i] at label[i], then 1 - lam[i] at label[i - 1] (label -1 being label n - 1). */
+int ffcvb_onehot_mix(ffcvb_ctx *ctx, void *stream, int n, int classes, const int32_t *label, const float *lam,
+                     float *dst_dev);
+
 /* Poison (poisoning.py:45-60), in place on the images with apply[i] != 0:
  * clamp(image * one_minus_alpha + mask) evaluated through a float32 scratch value as the
  * reference does.  one_minus_alpha_dev and mask_dev are DEVICE arrays of `count` doubles (the
