@@ -266,6 +266,7 @@ struct Slot {
     uint32_t total_blocks = 0;
     size_t clean_bytes = 0, plane_bytes = 0, rgb_bytes = 0, scan_bytes = 0, raw_bytes = 0, jpeg_bytes = 0;
     bool staged = false;
+    bool packed = false; // single-image calls: the decoded rows are the result, without padding
     bool direct = false; // payloads are gathered by the GPU from pinned host memory
     size_t staged_end = 0; // blob bytes [0, staged_end) come from the pinned staging buffer
     bool copy_done = true; // the staging threads have finished this slot's payload copy (guarded by ctx->copy_m)
@@ -279,6 +280,11 @@ struct Slot {
         void *dst_dev = nullptr;
         uint64_t off = 0, bytes = 0;       // place in the blob (set by ffcvb_stage_batch)
     };
+    struct Copy { // a piece of a sample's payload that a staging thread copies
+        int sample;
+        size_t from, bytes;
+    };
+    std::vector<Copy> copies;
     std::vector<Rider> pending_riders, riders; // set for the next staging / staged with the current batch
     double stage_ms[4] = {0, 0, 0, 0}; // header parse, layout, payload copy, total
     // working lists of the staging call, kept for their memory
@@ -342,7 +348,12 @@ struct ffcvb_ctx {
     // Tuning overrides, read from the environment once when the context is created (0 = none):
     // FFCV_B200_COPY_THREADS, FFCV_B200_SUBSEQ_BITS, FFCV_B200_GATHER_CTAS, FFCV_B200_GATHER_IN_FLIGHT.
     int tune_copy_threads = 0, tune_subseq_bits = 0, gather_ctas = 0, gather_in_flight = 8;
-    DevBuf one_src, one_dst; // single-image entry points
+    // single-image entry points: their stream, device buffers, pinned result and events of its pieces
+    DevBuf one_src, one_dst;
+    uint8_t *one_host = nullptr, *one_in = nullptr;
+    size_t one_host_cap = 0, one_in_cap = 0;
+    cudaStream_t one_stream = nullptr;
+    cudaEvent_t one_ev[16] = {};
     // Decode index (ffcvb_set_decode_index): a pool of device memory that keeps, per JPEG stream seen,
     // the decoder states a finished decode left behind; entries are handed out in order and never
     // moved.  Keyed by the sample's offset in the file: the context then serves one file.
@@ -497,6 +508,11 @@ void ffcvb_destroy(ffcvb_ctx *ctx) {
     if (ctx->index_stats.p) cudaFree(ctx->index_stats.p);
     if (ctx->one_src.p) cudaFree(ctx->one_src.p);
     if (ctx->one_dst.p) cudaFree(ctx->one_dst.p);
+    if (ctx->one_host) cudaFreeHost(ctx->one_host);
+    if (ctx->one_in) cudaFreeHost(ctx->one_in);
+    if (ctx->one_stream) cudaStreamDestroy(ctx->one_stream);
+    for (auto &e : ctx->one_ev)
+        if (e) cudaEventDestroy(e);
     delete ctx->pool;
     delete ctx;
 }
@@ -1010,7 +1026,7 @@ int stage_impl(ffcvb_ctx *ctx, int slot, const Source &source, const uint64_t *p
             plane_bytes += align_up(pw * ph, 16);
         }
         d.rgb_off = rgb_bytes;
-        d.rgb_pitch = (uint32_t)align_up((size_t)d.dec_width * 3, 16);
+        d.rgb_pitch = s.packed ? (uint32_t)d.dec_width * 3 : (uint32_t)align_up((size_t)d.dec_width * 3, 16);
         rgb_bytes += (size_t)d.dec_height * d.rgb_pitch;
         int bw = d.dec_width, bh = d.dec_height;
         {   // extent the colour kernels' grids must cover: the crop box (plus the odd edge of a
@@ -1227,12 +1243,23 @@ int stage_impl(ffcvb_ctx *ctx, int slot, const Source &source, const uint64_t *p
             std::lock_guard<std::mutex> g(ctx->copy_m);
             s.copy_done = false;
         }
+        // a few large streams are shared out in pieces
+        const size_t piece = n < 4 * ctx->pool->size() ? 128 * 1024 : ~(size_t)0;
+        sp->copies.clear();
+        for (int i = 0; i < n; i++) {
+            const ImageDesc &d = descs[i];
+            if (d.payload_size == 0 || d.src_addr != 0) continue;
+            const bool rows = d.mode == FFCVB_MODE_RAW && d.cols != d.width;
+            const size_t step = rows ? d.payload_size : (piece < d.payload_size ? piece : d.payload_size);
+            for (size_t from = 0; from < d.payload_size; from += step)
+                sp->copies.push_back(Slot::Copy{i, from, d.payload_size - from < step ? d.payload_size - from : step});
+        }
         ctx->pool->post(
-            Pool::kAsync, n, 1,
-            [sp, host, file_base](int i) {
-                const ImageDesc &d = sp->descs[i];
-                if (d.payload_size == 0 || d.src_addr != 0) return;
-                const uint8_t *src = file_base + sp->src_ptrs[i];
+            Pool::kAsync, (int)sp->copies.size(), 1,
+            [sp, host, file_base](int k) {
+                const Slot::Copy &c = sp->copies[k];
+                const ImageDesc &d = sp->descs[c.sample];
+                const uint8_t *src = file_base + sp->src_ptrs[c.sample];
                 uint8_t *dst = host + d.payload_off;
                 if (d.mode == FFCVB_MODE_RAW && d.cols != d.width) {
                     // only the crop box travels: one run per row.  Plain copies: streaming stores on
@@ -1242,7 +1269,7 @@ int stage_impl(ffcvb_ctx *ctx, int slot, const Source &source, const uint64_t *p
                     for (int r = 0; r < d.rows; r++) memcpy(dst + r * (size_t)d.raw_pitch, src + r * pitch, run);
                 } else {
                     if (d.mode == FFCVB_MODE_RAW) src += (size_t)d.row0 * d.width * 3;
-                    stream_copy(dst, src, d.payload_size);
+                    stream_copy(dst + c.from, src + c.from, c.bytes);
                 }
                 _mm_sfence(); // streaming stores are weakly ordered: publish them before the copy is reported done
             },
@@ -1328,7 +1355,14 @@ static int hold_for_copy(ffcvb_ctx *ctx, Slot &s, cudaStream_t st) {
     return FFCVB_OK;
 }
 
-static int run_batch(ffcvb_ctx *ctx, Slot &s, cudaStream_t st, void *out_dev, bool copy) {
+// Where a single-image decode leaves its pixels (instead of the slot's scratch, and with no resize
+// behind it) and its status word: device or page-locked host memory.
+struct Single {
+    uint8_t *rgb;
+    int32_t *status;
+};
+
+static int run_batch(ffcvb_ctx *ctx, Slot &s, cudaStream_t st, void *out_dev, bool copy, const Single *single = nullptr) {
     if (ctx->copy_timeout.load())
         return fail(ctx, FFCVB_E_CUDA, "a payload copy did not finish within its time limit: the batch that waited for it is invalid");
     const BatchHeader &hd = s.hdr;
@@ -1383,7 +1417,8 @@ static int run_batch(ffcvb_ctx *ctx, Slot &s, cudaStream_t st, void *out_dev, bo
     const HuffTable *huff = reinterpret_cast<const HuffTable *>(blob + hd.huff_off);
     const MultTable *mult = reinterpret_cast<const MultTable *>(blob + hd.mult_off);
     const int32_t *params = reinterpret_cast<const int32_t *>(blob + hd.params_off);
-    int32_t *status = reinterpret_cast<int32_t *>(blob + s.status_off);
+    int32_t *status = single ? single->status : reinterpret_cast<int32_t *>(blob + s.status_off);
+    uint8_t *rgb = single ? single->rgb : (uint8_t *)s.rgb.p;
     if (s.n_jpeg > 0) {
         const int32_t *jl = reinterpret_cast<const int32_t *>(blob + s.jpeg_list_off);
         EntropyScratch scratch{};
@@ -1391,7 +1426,7 @@ static int run_batch(ffcvb_ctx *ctx, Slot &s, cudaStream_t st, void *out_dev, bo
         scratch.seg_dc = (int32_t *)s.segs.p;
         scratch.sub_info = (uint32_t *)(scratch.seg_dc + 4 * (size_t)s.n_segs);
         scratch.meta = (SegMeta *)(scratch.sub_info + kSegSubs * (size_t)s.n_segs);
-        scratch.done = (uint32_t *)(status + s.n);
+        scratch.done = (uint32_t *)(blob + s.status_off) + s.n;
         scratch.pos = (uint32_t *)s.index.p;
         scratch.dc = (int16_t *)(scratch.pos + s.total_blocks);
         launch_entropy_decode(descs, reinterpret_cast<const uint2 *>(blob + s.segs_off), s.n_segs,
@@ -1404,17 +1439,19 @@ static int run_batch(ffcvb_ctx *ctx, Slot &s, cudaStream_t st, void *out_dev, bo
         if (prof) CU(cudaEventRecord(s.ev[3], st));
         launch_color(descs, jl, s.n_jpeg, s.n_quad, s.n_444, s.n_other, s.max_w, s.max_h,
                      reinterpret_cast<const uint2 *>(blob + s.quad_tiles_off), s.n_quad_tiles, (const uint8_t *)s.planes.p,
-                     (uint8_t *)s.rgb.p, s.plan.resize ? params : nullptr, (int)hd.n_params, st);
+                     rgb, s.plan.resize ? params : nullptr, (int)hd.n_params, st);
         if (prof) CU(cudaEventRecord(s.ev[4], st));
     } else if (prof) {
         for (int k = 2; k <= 4; k++) CU(cudaEventRecord(s.ev[k], st));
     }
-    ResizeSource src{};
-    src.descs = descs;
-    src.blob = blob;
-    src.rgb = (const uint8_t *)s.rgb.p;
-    launch_resize_augment(src, s.n, params, (int)hd.n_params, make_oplist(s.plan), s.plan.resize,
-                          s.plan.out_h, s.plan.out_w, s.plan.out_kind, s.plan.lut_dev, out_dev, status, st);
+    if (!single) {
+        ResizeSource src{};
+        src.descs = descs;
+        src.blob = blob;
+        src.rgb = rgb;
+        launch_resize_augment(src, s.n, params, (int)hd.n_params, make_oplist(s.plan), s.plan.resize,
+                              s.plan.out_h, s.plan.out_w, s.plan.out_kind, s.plan.lut_dev, out_dev, status, st);
+    }
     CU(cudaGetLastError());
     if (prof) {
         CU(cudaEventRecord(s.ev[5], st));
@@ -1815,9 +1852,46 @@ static ffcvb_ctx *global_ctx() {
     if (!g_ctx) {
         int dev = 0;
         if (cudaGetDevice(&dev) != cudaSuccess) return nullptr;
-        if (ffcvb_create(dev, 1, 1, &g_ctx) != FFCVB_OK) return nullptr;
+        const long cores = sysconf(_SC_NPROCESSORS_ONLN);
+        if (ffcvb_create(dev, 1, cores >= 16 ? 8 : (cores >= 4 ? (int)cores / 2 : 1), &g_ctx) != FFCVB_OK) return nullptr;
+        if (cudaStreamCreateWithFlags(&g_ctx->one_stream, cudaStreamNonBlocking) != cudaSuccess) {
+            ffcvb_destroy(g_ctx);
+            g_ctx = nullptr;
+        }
     }
     return g_ctx;
+}
+
+// Results of up to kZeroCopyBytes are written by the kernels straight into page-locked memory, which
+// saves a copy's launch and latency; larger ones go through device memory, from where the copy engine
+// fetches them piece by piece while the staging threads move the pieces that have landed on to the
+// caller's pageable buffer (one thread alone moves about 10 GB/s, the link 55).
+static constexpr size_t kZeroCopyBytes = 512 * 1024, kResultHead = 64; // (the head holds the status word)
+
+// Queues the pieces of `bytes` from dev to the pinned result buffer, and copies them on into `out` when
+// `ok` says so (asked when the first piece has landed).  Returns false on a CUDA error.
+static bool fetch_result(ffcvb_ctx *ctx, const uint8_t *dev, uint8_t *out, size_t bytes, const std::function<bool()> &ok) {
+    cudaStream_t st = ctx->one_stream;
+    uint8_t *host = ctx->one_host + kResultHead;
+    constexpr size_t kUnit = 128 * 1024;
+    size_t piece = align_up((bytes + 15) / 16, kUnit);
+    if (piece < 4 * kUnit) piece = 4 * kUnit;
+    const int pieces = (int)((bytes + piece - 1) / piece);
+    for (int k = 0; k < pieces; k++) {
+        const size_t from = k * piece, len = bytes - from < piece ? bytes - from : piece;
+        if (!ctx->one_ev[k] && cudaEventCreateWithFlags(&ctx->one_ev[k], cudaEventDisableTiming) != cudaSuccess) return false;
+        if (cudaMemcpyAsync(host + from, dev + from, len, cudaMemcpyDeviceToHost, st) != cudaSuccess) return false;
+        if (cudaEventRecord(ctx->one_ev[k], st) != cudaSuccess) return false;
+    }
+    std::atomic<bool> good{true};
+    ctx->pool->parallel_for((int)((bytes + kUnit - 1) / kUnit), 1, [&](int i) {
+        const size_t from = i * kUnit, len = bytes - from < kUnit ? bytes - from : kUnit;
+        if (cudaEventSynchronize(ctx->one_ev[from / piece]) != cudaSuccess)
+            good.store(false);
+        else if (ok())
+            memcpy(out + from, host + from, len);
+    });
+    return good.load() && cudaStreamSynchronize(st) == cudaSuccess;
 }
 
 int imdecode(unsigned char *input_buffer, uint64_t input_size, uint32_t source_height,
@@ -1849,14 +1923,24 @@ int imdecode(unsigned char *input_buffer, uint64_t input_size, uint32_t source_h
     const uint8_t mode = FFCVB_MODE_JPG;
     const uint16_t hh = (uint16_t)crop_height, ww = (uint16_t)crop_width;
     const int32_t params[4] = {0, 0, (int32_t)crop_height, (int32_t)crop_width};
+    Slot &s = ctx->slots[0];
+    s.packed = true;
     if (ffcvb_stage_batch(ctx, 0, input_buffer, &ptr, &size, &mode, &hh, &ww, 1, &plan, params)) return -1;
+    if (s.descs[0].host_status != 0) return -1;
     const size_t out_bytes = (size_t)plan.out_h * plan.out_w * 3;
-    if (grow_dev(ctx, ctx->one_dst, out_bytes)) return -1;
-    if (ffcvb_submit_batch(ctx, 0, nullptr, ctx->one_dst.p)) return -1;
-    int32_t status = 0;
-    if (ffcvb_batch_status(ctx, 0, nullptr, &status, 1) != 0) return -1;
-    if (cudaMemcpy(output_buffer, ctx->one_dst.p, out_bytes, cudaMemcpyDeviceToHost) != cudaSuccess) return -1;
-    return 0;
+    const bool zero_copy = out_bytes <= kZeroCopyBytes;
+    if (grow_host(ctx, ctx->one_host, ctx->one_host_cap, kResultHead + out_bytes)) return -1;
+    if (!zero_copy && grow_dev(ctx, ctx->one_dst, out_bytes)) return -1;
+    volatile int32_t *status = (volatile int32_t *)ctx->one_host;
+    *status = 0;
+    const Single single{zero_copy ? ctx->one_host + kResultHead : (uint8_t *)ctx->one_dst.p, (int32_t *)ctx->one_host};
+    if (run_batch(ctx, s, ctx->one_stream, nullptr, true, &single)) return -1;
+    if (zero_copy) {
+        if (cudaStreamSynchronize(ctx->one_stream) != cudaSuccess || *status != 0) return -1;
+        memcpy(output_buffer, ctx->one_host + kResultHead, out_bytes);
+        return 0;
+    }
+    return fetch_result(ctx, (const uint8_t *)ctx->one_dst.p, output_buffer, out_bytes, [&] { return *status == 0; }) && *status == 0 ? 0 : -1;
 }
 
 void resize(int64_t cresizer, int64_t source_p, int64_t sx, int64_t sy, int64_t start_row,
@@ -1868,22 +1952,47 @@ void resize(int64_t cresizer, int64_t source_p, int64_t sx, int64_t sy, int64_t 
     if (start_row < 0 || start_col < 0 || end_row > sx || end_col > sy || end_row <= start_row ||
         end_col <= start_col)
         return;
-    // Only the rows of the region travel to the GPU.
-    const int rows = (int)(end_row - start_row);
-    const size_t src_bytes = (size_t)rows * sy * 3, dst_bytes = (size_t)tx * ty * 3;
-    if (grow_dev(ctx, ctx->one_src, src_bytes) || grow_dev(ctx, ctx->one_dst, dst_bytes)) return;
-    const uint8_t *src = (const uint8_t *)(intptr_t)source_p + (size_t)start_row * sy * 3;
-    if (cudaMemcpy(ctx->one_src.p, src, src_bytes, cudaMemcpyHostToDevice) != cudaSuccess) return;
-    ffcvb_plan plan{};
-    plan.out_h = (int32_t)tx;
-    plan.out_w = (int32_t)ty;
-    plan.resize = 1;
-    plan.out_kind = FFCVB_OUT_U8_NHWC;
-    const int32_t params[4] = {0, (int32_t)start_col, rows, (int32_t)(end_col - start_col)};
-    if (ffcvb_transform_device(ctx, nullptr, (const uint8_t *)ctx->one_src.p, 1, rows, (int)sy, &plan, params,
-                               ctx->one_dst.p))
+    // Only the region travels to the GPU, behind its parameters.
+    const int rows = (int)(end_row - start_row), cols = (int)(end_col - start_col);
+    const size_t pitch = (size_t)cols * 3, src_bytes = kResultHead + (size_t)rows * pitch, dst_bytes = (size_t)tx * ty * 3;
+    const bool zero_copy = dst_bytes <= kZeroCopyBytes;
+    if (cudaSetDevice(ctx->device) != cudaSuccess) return;
+    if (grow_dev(ctx, ctx->one_src, src_bytes + 64) || grow_host(ctx, ctx->one_in, ctx->one_in_cap, src_bytes) ||
+        grow_host(ctx, ctx->one_host, ctx->one_host_cap, kResultHead + dst_bytes) || (!zero_copy && grow_dev(ctx, ctx->one_dst, dst_bytes)))
         return;
-    cudaMemcpy((void *)(intptr_t)dest_p, ctx->one_dst.p, dst_bytes, cudaMemcpyDeviceToHost);
+    const int32_t params[4] = {0, 0, rows, cols};
+    memcpy(ctx->one_in, params, sizeof(params));
+    const uint8_t *src = (const uint8_t *)(intptr_t)source_p + ((size_t)start_row * sy + start_col) * 3;
+    uint8_t *in = ctx->one_in + kResultHead;
+    auto copy_rows = [&](int lo, int hi) {
+        if (cols == sy)
+            memcpy(in + lo * pitch, src + lo * pitch, (hi - lo) * pitch);
+        else
+            for (int r = lo; r < hi; r++) memcpy(in + r * pitch, src + (size_t)r * sy * 3, pitch);
+    };
+    cudaStream_t st = ctx->one_stream;
+    // in parts of about 256 KB, each under way while the next one is copied (many of them: by all threads)
+    const int part = (int)(256 * 1024 / pitch) + 1, parts = (rows + part - 1) / part;
+    const bool together = parts > 8;
+    if (together) ctx->pool->parallel_for(parts, 1, [&](int k) { copy_rows(k * part, (k + 1) * part < rows ? (k + 1) * part : rows); });
+    for (int k = 0; k < (together ? 1 : parts); k++) {
+        const int lo = k * part, hi = together || lo + part > rows ? rows : lo + part;
+        if (!together) copy_rows(lo, hi);
+        const size_t from = k == 0 ? 0 : kResultHead + lo * pitch, to = kResultHead + hi * pitch;
+        if (cudaMemcpyAsync((uint8_t *)ctx->one_src.p + from, ctx->one_in + from, to - from, cudaMemcpyHostToDevice, st) != cudaSuccess) return;
+    }
+    ResizeSource rs{};
+    rs.uniform = (const uint8_t *)ctx->one_src.p + kResultHead;
+    rs.uniform_h = rows;
+    rs.uniform_w = cols;
+    uint8_t *out = zero_copy ? ctx->one_host + kResultHead : (uint8_t *)ctx->one_dst.p;
+    launch_resize_augment(rs, 1, (const int32_t *)ctx->one_src.p, 4, OpList{}, 1, (int)tx, (int)ty, FFCVB_OUT_U8_NHWC, nullptr, out, nullptr, st);
+    if (cudaGetLastError() != cudaSuccess) return;
+    if (zero_copy) {
+        if (cudaStreamSynchronize(st) == cudaSuccess) memcpy((void *)(intptr_t)dest_p, out, dst_bytes);
+    } else {
+        fetch_result(ctx, out, (uint8_t *)(intptr_t)dest_p, dst_bytes, [] { return true; });
+    }
 }
 
 void my_memcpy(void *source, void *dst, uint64_t size) { memcpy(dst, source, size); }
