@@ -268,6 +268,8 @@ struct Slot {
     bool staged = false;
     bool packed = false; // single-image calls: the decoded rows are the result, without padding
     bool direct = false; // payloads are gathered by the GPU from pinned host memory
+    const uint8_t *range_src = nullptr; // the payloads lie in one piece of pinned memory: copied as such
+    size_t range_len = 0;
     size_t staged_end = 0; // blob bytes [0, staged_end) come from the pinned staging buffer
     bool copy_done = true; // the staging threads have finished this slot's payload copy (guarded by ctx->copy_m)
     std::vector<ImageDesc> descs;
@@ -297,15 +299,14 @@ struct Slot {
     std::vector<uint2> blk_tiles;  // (sample, k) of the block decoder's CTAs
     std::vector<uint2> quad_tiles; // (sample, tile x | tile y << 16) of the 4:2:0 colour kernel's CTAs
     cudaEvent_t ev[6] = {nullptr, nullptr, nullptr, nullptr, nullptr, nullptr};
-    // payload gather runs on its own high-priority stream so that its few CTAs are placed ahead of
-    // the large grids other slots have queued, and the PCIe transfer overlaps their compute
-    cudaStream_t gather_stream = nullptr;
     cudaEvent_t ev_begin = nullptr, ev_gather_start = nullptr, ev_gathered = nullptr;
-    // recorded behind the last work queued on the slot: staging the slot again waits for it, so a
-    // caller that forgets to fence the ring gets a stall instead of a batch whose descriptors are
-    // overwritten under its kernels
-    cudaEvent_t ev_done = nullptr;
+    // recorded behind the copies of the slot's last batch: staging the slot again waits for it, so a
+    // caller that forgets to fence the ring gets a stall instead of a batch that is overwritten under
+    // its copies (on the device the slot's stream keeps its batches in order)
+    cudaEvent_t ev_copied = nullptr;
     bool in_flight = false;
+    cudaStream_t last_stream = nullptr; // the stream that batch was queued on
+    cudaEvent_t ev_done = nullptr;      // behind all of its work
     bool gather_timed = false; // ev_gather_start .. ev_gathered bracket the last gather of this slot
     bool timed = false; // events of the last run are valid
 };
@@ -346,8 +347,14 @@ struct ffcvb_ctx {
     double share = 0.0;          // the adjusted share, 0..1
     int split_copy_threads = 4; // ... and how many of them copy at a time (more only crowd the gather out)
     // Tuning overrides, read from the environment once when the context is created (0 = none):
-    // FFCV_B200_COPY_THREADS, FFCV_B200_SUBSEQ_BITS, FFCV_B200_GATHER_CTAS, FFCV_B200_GATHER_IN_FLIGHT.
-    int tune_copy_threads = 0, tune_subseq_bits = 0, gather_ctas = 0, gather_in_flight = 8;
+    // FFCV_B200_COPY_THREADS, FFCV_B200_SUBSEQ_BITS, FFCV_B200_GATHER_CTAS.
+    int tune_copy_threads = 0, tune_subseq_bits = 0, gather_ctas = 0;
+    // Transfers of a page-locked source run on one stream of their own, in the order of the batches: two
+    // batches that share the link would both arrive late, and the first one's kernels would have nothing
+    // to overlap with.  High priority, so that a gather's few CTAs are placed ahead of the large grids
+    // that are queued.
+    cudaStream_t copy_stream = nullptr;
+    int32_t *gather_failed = nullptr; // page-locked: set by a gather whose wait for the link ran out
     // single-image entry points: their stream, device buffers, pinned result and events of its pieces
     DevBuf one_src, one_dst;
     uint8_t *one_host = nullptr, *one_in = nullptr;
@@ -477,7 +484,6 @@ int ffcvb_create(int device, int n_slots, int n_threads, ffcvb_ctx **out) {
     c->tune_copy_threads = env_int("FFCV_B200_COPY_THREADS", 1, 256);
     c->tune_subseq_bits = env_int("FFCV_B200_SUBSEQ_BITS", 128, kMaxSubseqBits) / 32 * 32;
     c->gather_ctas = env_int("FFCV_B200_GATHER_CTAS", 1, 1024);
-    if (env_int("FFCV_B200_GATHER_IN_FLIGHT", 4, 4)) c->gather_in_flight = 4;
     *out = c;
     return FFCVB_OK;
 }
@@ -493,9 +499,9 @@ void ffcvb_destroy(ffcvb_ctx *ctx) {
             if (b->p) cudaFree(b->p);
         for (auto &e : s.ev)
             if (e) cudaEventDestroy(e);
-        if (s.gather_stream) cudaStreamDestroy(s.gather_stream);
         if (s.ev_begin) cudaEventDestroy(s.ev_begin);
         if (s.ev_done) cudaEventDestroy(s.ev_done);
+        if (s.ev_copied) cudaEventDestroy(s.ev_copied);
         if (s.ev_gathered) cudaEventDestroy(s.ev_gathered);
         if (s.ev_gather_start) cudaEventDestroy(s.ev_gather_start);
     }
@@ -506,6 +512,8 @@ void ffcvb_destroy(ffcvb_ctx *ctx) {
     }
     if (ctx->index_pool.p) cudaFree(ctx->index_pool.p);
     if (ctx->index_stats.p) cudaFree(ctx->index_stats.p);
+    if (ctx->gather_failed) cudaFreeHost(ctx->gather_failed);
+    if (ctx->copy_stream) cudaStreamDestroy(ctx->copy_stream);
     if (ctx->one_src.p) cudaFree(ctx->one_src.p);
     if (ctx->one_dst.p) cudaFree(ctx->one_dst.p);
     if (ctx->one_host) cudaFreeHost(ctx->one_host);
@@ -617,7 +625,7 @@ int stage_impl(ffcvb_ctx *ctx, int slot, const Source &source, const uint64_t *p
     CU(cudaSetDevice(ctx->device));
     Slot &s = ctx->slots[slot];
     if (s.in_flight) { // normally complete long ago (the caller fences the ring): returns at once
-        CU(cudaEventSynchronize(s.ev_done));
+        CU(cudaEventSynchronize(s.ev_copied));
         s.in_flight = false;
     }
     s.staged = false;
@@ -867,7 +875,28 @@ int stage_impl(ffcvb_ctx *ctx, int slot, const Source &source, const uint64_t *p
     // Split staging: with a pinned source the staging threads (and the copy engine) can carry part
     // of the bytes while the GPU gathers the rest, so that neither path alone has to fill the link.
     // Samples are dealt to the CPU side greedily so that its share of the running byte count holds.
-    if (direct && ctx->adaptive_split) {
+    // Samples that follow one another in the file (a sequential pass) need no gather: the copy engine
+    // takes the whole piece, at the link's full rate and beside the kernels.  Worth it as long as little
+    // else lies between them.
+    s.range_len = 0;
+    if (direct) {
+        uint64_t lo = ~0ull, hi = 0, sum = 0;
+        bool whole = true;
+        for (int i = 0; i < n && whole; i++) {
+            const ImageDesc &d = descs[i];
+            if (d.src_addr == 0 || d.payload_size == 0) continue;
+            whole = d.mode == FFCVB_MODE_JPG || d.cols == d.width;
+            lo = d.src_addr < lo ? d.src_addr : lo;
+            hi = d.src_addr + d.payload_size > hi ? d.src_addr + d.payload_size : hi;
+            sum += d.payload_size;
+        }
+        if (whole && sum > 0 && hi - lo <= sum + sum / 16 + 4096) {
+            lo &= ~15ull;
+            s.range_src = file_base + (lo - src_dev_base);
+            s.range_len = (size_t)(hi - lo);
+        }
+    }
+    if (direct && ctx->adaptive_split && s.range_len == 0) {
         // The slot's previous batch tells how long its two halves took: the staging threads' copy
         // (host clock) and the GPU's gather (events).  Move the share towards equal times; the
         // step is small because the measurement is several batches old.
@@ -883,7 +912,7 @@ int stage_impl(ffcvb_ctx *ctx, int slot, const Source &source, const uint64_t *p
         s.gather_timed = false;
         ctx->cpu_share_permille = (int)(ctx->share * 1000 + 0.5);
     }
-    if (direct && ctx->cpu_share_permille > 0) {
+    if (direct && ctx->cpu_share_permille > 0 && s.range_len == 0) {
         uint64_t total = 0, cpu = 0;
         for (int i = 0; i < n; i++) {
             total += descs[i].payload_size;
@@ -1124,7 +1153,13 @@ int stage_impl(ffcvb_ctx *ctx, int slot, const Source &source, const uint64_t *p
             off = align_up(off + descs[i].payload_size, kPayloadAlign);
         }
         s.staged_end = off;
-        for (int i = 0; i < n; i++) {
+        if (s.range_len) {
+            const uint64_t lo = src_dev_base + (uint64_t)(s.range_src - file_base);
+            for (int i = 0; i < n; i++)
+                if (descs[i].src_addr != 0) descs[i].payload_off = off + (descs[i].src_addr - lo);
+            off = align_up(off + s.range_len, kPayloadAlign);
+        }
+        for (int i = 0; i < n && s.range_len == 0; i++) {
             ImageDesc &d = descs[i];
             if (d.src_addr == 0) continue;
             // Gathered payloads keep their source alignment mod 16 so that both sides move in whole
@@ -1151,7 +1186,9 @@ int stage_impl(ffcvb_ctx *ctx, int slot, const Source &source, const uint64_t *p
     // A pinned source needs room for the part that is staged.  That part varies from batch to batch and
     // regrowing page-locked memory stalls the device: room for the most that the split may stage.
     size_t host_need = off;
-    if (direct) {
+    if (s.range_len) {
+        host_need = s.staged_end;
+    } else if (direct) {
         const double most = ctx->adaptive_split ? kMaxAdaptiveShare : ctx->cpu_share_permille / 1000.0;
         host_need = hd.payload_off + (size_t)(most * (double)(off - hd.payload_off));
         if (host_need < s.staged_end) host_need = s.staged_end;
@@ -1362,7 +1399,10 @@ struct Single {
     int32_t *status;
 };
 
-static int run_batch(ffcvb_ctx *ctx, Slot &s, cudaStream_t st, void *out_dev, bool copy, const Single *single = nullptr) {
+// `outputs_free`: an event the work that writes to the caller's buffers (out_dev, the riders'
+// destinations) has to wait for; all before it only touches memory of the slot.
+static int run_batch(ffcvb_ctx *ctx, Slot &s, cudaStream_t st, void *out_dev, bool copy, const Single *single = nullptr,
+                     cudaEvent_t outputs_free = nullptr) {
     if (ctx->copy_timeout.load())
         return fail(ctx, FFCVB_E_CUDA, "a payload copy did not finish within its time limit: the batch that waited for it is invalid");
     const BatchHeader &hd = s.hdr;
@@ -1374,44 +1414,53 @@ static int run_batch(ffcvb_ctx *ctx, Slot &s, cudaStream_t st, void *out_dev, bo
             if (!e) CU(cudaEventCreate(&e));
         CU(cudaEventRecord(s.ev[0], st));
     }
+    if (!s.ev_copied) {
+        CU(cudaEventCreateWithFlags(&s.ev_copied, cudaEventDisableTiming));
+        CU(cudaEventCreateWithFlags(&s.ev_done, cudaEventDisableTiming));
+    }
+    if (s.last_stream != st && s.last_stream != nullptr) CU(cudaStreamWaitEvent(st, s.ev_done, 0)); // (the slot changed streams)
+    s.last_stream = st;
     int hrc;
     if (copy && !s.direct) {
         if ((hrc = hold_for_copy(ctx, s, st))) return hrc;
         CU(cudaMemcpyAsync(blob, s.host, hd.total_bytes, cudaMemcpyHostToDevice, st));
     } else if (copy) {
-        if (!s.gather_stream) {
+        if (!ctx->copy_stream) {
+            CU(cudaHostAlloc((void **)&ctx->gather_failed, 64, cudaHostAllocDefault));
+            *ctx->gather_failed = 0;
             int lo = 0, hi = 0;
             CU(cudaDeviceGetStreamPriorityRange(&lo, &hi));
-            CU(cudaStreamCreateWithPriority(&s.gather_stream, cudaStreamNonBlocking, hi));
+            CU(cudaStreamCreateWithPriority(&ctx->copy_stream, cudaStreamNonBlocking, hi));
+        }
+        if (!s.ev_begin) {
             CU(cudaEventCreateWithFlags(&s.ev_begin, cudaEventDisableTiming));
             CU(cudaEventCreate(&s.ev_gather_start));
             CU(cudaEventCreate(&s.ev_gathered));
         }
-        CU(cudaEventRecord(s.ev_begin, st)); // everything the caller ordered before this batch
-        CU(cudaStreamWaitEvent(s.gather_stream, s.ev_begin, 0));
-
-        CU(cudaMemcpyAsync(blob, s.host, hd.payload_off, cudaMemcpyHostToDevice, s.gather_stream));
-        CU(cudaEventRecord(s.ev_gather_start, s.gather_stream)); // after the head's copy: that one queues behind other batches' transfers
-        s.gather_timed = true;
-        static_assert(FFCVB_MAX_RIDERS <= sizeof(SmallCopies::off) / sizeof(uint64_t), "a batch's riders fit one launch");
-        SmallCopies small{};
-        for (const auto &r : s.riders) {
-            small.off[small.n] = r.off;
-            small.bytes[small.n] = r.bytes;
-            small.dst[small.n++] = (uint8_t *)r.dst_dev;
+        if (*(volatile int32_t *)ctx->gather_failed) return fail(ctx, FFCVB_E_CUDA, "a payload gather gave up waiting for the link");
+        CU(cudaEventRecord(s.ev_begin, st)); // the slot's previous batch
+        CU(cudaStreamWaitEvent(ctx->copy_stream, s.ev_begin, 0));
+        CU(cudaMemcpyAsync(blob, s.host, hd.payload_off, cudaMemcpyHostToDevice, ctx->copy_stream));
+        s.gather_timed = s.range_len == 0;
+        if (s.gather_timed) {
+            CU(cudaEventRecord(s.ev_gather_start, ctx->copy_stream));
+            launch_gather_payloads(reinterpret_cast<const ImageDesc *>(blob + hd.desc_off), s.n, blob, ctx->gather_ctas, ctx->gather_failed,
+                                   ctx->copy_stream);
+        } else {
+            CU(cudaMemcpyAsync(blob + hd.payload_off, s.range_src, s.range_len, cudaMemcpyHostToDevice, ctx->copy_stream));
         }
-        launch_gather_payloads(reinterpret_cast<const ImageDesc *>(blob + hd.desc_off), s.n, blob, small, ctx->gather_ctas, ctx->gather_in_flight, s.gather_stream);
-        CU(cudaEventRecord(s.ev_gathered, s.gather_stream));
-        if (s.staged_end > hd.payload_off) { // the CPU-staged share rides the copy engine meanwhile
+        CU(cudaEventRecord(s.ev_gathered, ctx->copy_stream));
+        if (s.range_len == 0 && s.staged_end > hd.payload_off) { // the CPU-staged share rides the copy engine meanwhile
             if ((hrc = hold_for_copy(ctx, s, st))) return hrc;
             CU(cudaMemcpyAsync(blob + hd.payload_off, s.host + hd.payload_off, s.staged_end - hd.payload_off,
                                cudaMemcpyHostToDevice, st));
         }
         CU(cudaStreamWaitEvent(st, s.ev_gathered, 0));
     }
-    if (copy && !s.direct)
-        for (const auto &r : s.riders)
-            if (r.bytes) CU(cudaMemcpyAsync(r.dst_dev, blob + r.off, r.bytes, cudaMemcpyDeviceToDevice, st));
+    if (copy) {
+        CU(cudaEventRecord(s.ev_copied, st));
+        s.in_flight = true;
+    }
     if (prof) CU(cudaEventRecord(s.ev[1], st));
     const ImageDesc *descs = reinterpret_cast<const ImageDesc *>(blob + hd.desc_off);
     const HuffTable *huff = reinterpret_cast<const HuffTable *>(blob + hd.huff_off);
@@ -1444,22 +1493,29 @@ static int run_batch(ffcvb_ctx *ctx, Slot &s, cudaStream_t st, void *out_dev, bo
     } else if (prof) {
         for (int k = 2; k <= 4; k++) CU(cudaEventRecord(s.ev[k], st));
     }
+    if (outputs_free) CU(cudaStreamWaitEvent(st, outputs_free, 0));
     if (!single) {
+        static_assert(FFCVB_MAX_RIDERS <= sizeof(SmallCopies::src) / sizeof(uint8_t *), "a batch's riders fit one launch");
+        SmallCopies small{};
+        for (const auto &r : s.riders) {
+            if (!copy) break;
+            small.src[small.n] = blob + r.off;
+            small.bytes[small.n] = r.bytes;
+            small.dst[small.n++] = (uint8_t *)r.dst_dev;
+        }
         ResizeSource src{};
         src.descs = descs;
         src.blob = blob;
         src.rgb = rgb;
         launch_resize_augment(src, s.n, params, (int)hd.n_params, make_oplist(s.plan), s.plan.resize,
-                              s.plan.out_h, s.plan.out_w, s.plan.out_kind, s.plan.lut_dev, out_dev, status, st);
+                              s.plan.out_h, s.plan.out_w, s.plan.out_kind, s.plan.lut_dev, out_dev, status, small, st);
     }
     CU(cudaGetLastError());
     if (prof) {
         CU(cudaEventRecord(s.ev[5], st));
         s.timed = true;
     }
-    if (!s.ev_done) CU(cudaEventCreateWithFlags(&s.ev_done, cudaEventDisableTiming));
     CU(cudaEventRecord(s.ev_done, st));
-    s.in_flight = true;
     return FFCVB_OK;
 }
 
@@ -1572,13 +1628,17 @@ int ffcvb_batch_times(ffcvb_ctx *ctx, int slot, float *ms) {
 }
 
 int ffcvb_submit_batch(ffcvb_ctx *ctx, int slot, void *stream, void *out_dev) {
+    return ffcvb_submit_batch_after(ctx, slot, stream, out_dev, nullptr);
+}
+
+int ffcvb_submit_batch_after(ffcvb_ctx *ctx, int slot, void *stream, void *out_dev, void *outputs_free) {
     if (!ctx) return FFCVB_E_ARG;
     if (slot < 0 || slot >= (int)ctx->slots.size() || !out_dev)
         return fail(ctx, FFCVB_E_ARG, "ffcvb_submit_batch: bad argument");
     Slot &s = ctx->slots[slot];
     if (!s.staged) return fail(ctx, FFCVB_E_ARG, "ffcvb_submit_batch: slot %d has no staged batch", slot);
     CU(cudaSetDevice(ctx->device));
-    return run_batch(ctx, s, (cudaStream_t)stream, out_dev, true);
+    return run_batch(ctx, s, (cudaStream_t)stream, out_dev, true, nullptr, (cudaEvent_t)outputs_free);
 }
 
 /* Re-runs the kernels of a batch whose bytes a previous ffcvb_submit_batch already put in HBM
@@ -1635,7 +1695,7 @@ int ffcvb_batch_info(const ffcvb_ctx *ctx, int slot, int64_t *info) {
 int ffcvb_batch_launches(const ffcvb_ctx *ctx, int slot) {
     if (!ctx || slot < 0 || slot >= (int)ctx->slots.size() || !ctx->slots[slot].staged) return -1;
     const Slot &s = ctx->slots[slot];
-    int k = 1 + (s.direct ? 1 : 0); // fused resize/augment/normalise (+ payload gather)
+    int k = 1 + (s.direct && s.range_len == 0 ? 1 : 0); // fused resize/augment/normalise (+ payload gather)
     k += (s.n_quad > 0) + (s.n_444 > 0) + (s.n_other > 0) + (s.n_block_tiles > 0) + 2 * (s.n_segs > 0) + (s.n_multi > 0) + (s.n_restart > 0);
     return k;
 }
@@ -1700,7 +1760,7 @@ int ffcvb_transform_device(ffcvb_ctx *ctx, void *stream, const uint8_t *src_dev,
     src.uniform_h = h;
     src.uniform_w = w;
     launch_resize_augment(src, n, (const int32_t *)a.dev.p, n_params, make_oplist(*plan), plan->resize,
-                          plan->out_h, plan->out_w, plan->out_kind, plan->lut_dev, out_dev, nullptr, st);
+                          plan->out_h, plan->out_w, plan->out_kind, plan->lut_dev, out_dev, nullptr, SmallCopies{}, st);
     CU(cudaGetLastError());
     CU(cudaEventRecord(a.ev, st));
     a.used = true;
@@ -1986,7 +2046,7 @@ void resize(int64_t cresizer, int64_t source_p, int64_t sx, int64_t sy, int64_t 
     rs.uniform_h = rows;
     rs.uniform_w = cols;
     uint8_t *out = zero_copy ? ctx->one_host + kResultHead : (uint8_t *)ctx->one_dst.p;
-    launch_resize_augment(rs, 1, (const int32_t *)ctx->one_src.p, 4, OpList{}, 1, (int)tx, (int)ty, FFCVB_OUT_U8_NHWC, nullptr, out, nullptr, st);
+    launch_resize_augment(rs, 1, (const int32_t *)ctx->one_src.p, 4, OpList{}, 1, (int)tx, (int)ty, FFCVB_OUT_U8_NHWC, nullptr, out, nullptr, SmallCopies{}, st);
     if (cudaGetLastError() != cudaSuccess) return;
     if (zero_copy) {
         if (cudaStreamSynchronize(st) == cudaSuccess) memcpy((void *)(intptr_t)dest_p, out, dst_bytes);

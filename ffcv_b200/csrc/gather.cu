@@ -1,99 +1,148 @@
-// Payload gather from pinned host memory over PCIe (sm_100a): the SMs read the sample bytes of a
+// Payload gather from pinned host memory over PCIe (sm_100a): the GPU reads the sample bytes of a
 // batch straight out of the page-locked dataset file, so no host core touches them.
 #include "kernels.h"
 
 namespace ffcvb {
 
-// 16 CTAs of 256 threads with eight 16-byte loads in flight each (512 KB outstanding) move 43-44
-// GB/s inside the loader's pipeline (four in flight: 43.0, eight: 44.0; a single pinned DMA copy:
-// 55); more CTAs are slower (32: 38.9 GB/s, 8: 42.3): more outstanding system-memory reads only
-// congest the memory system for the decode kernels running beside it.
-template <int kInFlight>
-__global__ void __launch_bounds__(256)
-gather_payloads_kernel(const ImageDesc *__restrict__ descs, int n, uint8_t *__restrict__ blob, const __grid_constant__ SmallCopies small) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
-    if (blockIdx.x == gridDim.x - 1) { // one CTA of its own: values that arrived with the head of the blob
-        for (int k = 0; k < small.n; k++)
-            for (uint64_t b = threadIdx.x; b < small.bytes[k]; b += blockDim.x) small.dst[k][b] = blob[small.off[k] + b];
-        return;
-    }
-    for (int i = blockIdx.x; i < n; i += gridDim.x - 1) {
-        const ImageDesc &d = descs[i];
-        if (d.src_addr == 0 || d.payload_size == 0) continue;
-        const uint8_t *src = reinterpret_cast<const uint8_t *>(d.src_addr);
-        uint8_t *dst = blob + d.payload_off;
-        if (d.mode == 1 && d.raw_skew) {
-            // Raw sample, crop box only.  A row is fetched as the aligned 16-byte words of host
-            // memory that contain it and stored as such into its 16-byte aligned slot, so the
-            // pixels keep their source alignment inside the slot and no byte is shuffled.  (A
-            // word that holds one byte of the row lies in the same page as that byte: the reads
-            // stay inside the pinned allocation.)  Two rows per warp and pass, all loads of a
-            // pass issued before its stores: up to 8 x 512 bytes in flight per warp.
-            const uint32_t run = (uint32_t)d.cols * 3, pitch = (uint32_t)d.width * 3;
-            for (int r0 = 2 * warp; r0 < d.rows; r0 += 2 * nwarps) {
-                const uint4 *s16[2];
-                uint4 *d16[2];
-                uint32_t nchunk[2];
-#pragma unroll
-                for (int q = 0; q < 2; q++) {
-                    const int r = r0 + q;
-                    const uint8_t *s = src + (size_t)r * pitch;
-                    const uint32_t a = (uint32_t)(reinterpret_cast<uintptr_t>(s) & 15);
-                    s16[q] = reinterpret_cast<const uint4 *>(s - a);
-                    d16[q] = reinterpret_cast<uint4 *>(dst + (size_t)r * d.raw_pitch);
-                    nchunk[q] = r < d.rows ? (a + run + 15) >> 4 : 0;
-                }
-                const uint32_t most = nchunk[0] > nchunk[1] ? nchunk[0] : nchunk[1];
-#pragma unroll 1
-                for (uint32_t c0 = 0; c0 < most; c0 += 128) {
-                    uint4 v[2][4];
-#pragma unroll
-                    for (int q = 0; q < 2; q++)
-#pragma unroll
-                        for (int u = 0; u < 4; u++) {
-                            const uint32_t c = c0 + u * 32 + lane;
-                            if (c < nchunk[q]) v[q][u] = s16[q][c];
-                        }
-#pragma unroll
-                    for (int q = 0; q < 2; q++)
-#pragma unroll
-                        for (int u = 0; u < 4; u++) {
-                            const uint32_t c = c0 + u * 32 + lane;
-                            if (c < nchunk[q]) d16[q][c] = v[q][u];
-                        }
-                }
-            }
-            continue;
-        }
-        const uint32_t size = d.payload_size;
-        uint32_t head = (uint32_t)((16 - (d.src_addr & 15)) & 15);
-        if (head > size) head = size;
-        if ((reinterpret_cast<uintptr_t>(dst) & 15) != (d.src_addr & 15)) head = size; // never: bytes only
-        for (uint32_t k = threadIdx.x; k < head; k += blockDim.x) dst[k] = src[k];
-        const uint32_t nvec = (size - head) >> 4;
-        const uint4 *s16 = reinterpret_cast<const uint4 *>(src + head);
-        uint4 *d16 = reinterpret_cast<uint4 *>(dst + head);
-        uint32_t k = threadIdx.x;
-        for (; k + (kInFlight - 1) * blockDim.x < nvec; k += kInFlight * blockDim.x) {
-            uint4 v[kInFlight]; // all loads of a pass are issued before its stores
-#pragma unroll
-            for (int u = 0; u < kInFlight; u++) v[u] = s16[k + u * blockDim.x];
-#pragma unroll
-            for (int u = 0; u < kInFlight; u++) d16[k + u * blockDim.x] = v[u];
-        }
-        for (; k < nvec; k += blockDim.x) d16[k] = s16[k];
-        for (uint32_t t = head + (nvec << 4) + threadIdx.x; t < size; t += blockDim.x) dst[t] = src[t];
+namespace {
+
+// The bytes go through shared memory as bulk copies (host -> shared, shared -> device) that one thread
+// per CTA issues: a ring of kStages pieces per CTA, half of them on their way in while the others leave.
+// What bounds it is the link: 64 CTAs x 8 KB keep 512 KB outstanding and move 48.6 GB/s of JPEG streams
+// and 46 GB/s of 0.7 KB crop rows (a plain DMA copy: 55.6), against 36-45 and 30-41 GB/s of a kernel of
+// 16 x 256 threads with eight 16-byte loads each.  As important is what it leaves to the decode kernels
+// beside it: no issue slots, 32 threads and 8 KB of shared memory on 64 SMs.
+constexpr int kStages = 8, kPiece = 1024, kAhead = 5; // kAhead: pieces on their way in
+
+__device__ __forceinline__ uint32_t shared_address(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
+
+struct Ring {
+    uint64_t dst[kStages];
+    uint32_t len[kStages];
+    uint32_t issued, stored;
+    bool failed;
+};
+
+// Waits for the piece in stage `st`, two seconds at most; false: it did not arrive.
+__device__ __forceinline__ bool arrived(uint64_t *bars, uint32_t st, uint32_t parity) {
+    uint64_t begin = 0;
+    for (;;) {
+        uint32_t ok;
+        asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+                     : "=r"(ok)
+                     : "r"(shared_address(&bars[st])), "r"(parity)
+                     : "memory");
+        if (ok) return true;
+        uint64_t now;
+        asm volatile("mov.u64 %0, %globaltimer;" : "=l"(now));
+        if (begin == 0) begin = now;
+        if (now - begin > 2000000000ull) return false;
     }
 }
 
-void launch_gather_payloads(const ImageDesc *descs, int n, uint8_t *blob, const SmallCopies &small, int ctas, int in_flight, cudaStream_t stream) {
+// Sends the oldest piece on its way in out again.
+__device__ __forceinline__ void store_oldest(Ring &r, uint8_t *buf, uint64_t *bars, uint8_t *blob) {
+    const uint32_t st = r.stored % kStages;
+    if (!arrived(bars, st, (r.stored / kStages) & 1)) {
+        r.failed = true;
+        return;
+    }
+    asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(blob + r.dst[st]), "r"(shared_address(buf + st * kPiece)),
+                 "r"(r.len[st])
+                 : "memory");
+    asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+    r.stored++;
+}
+
+// Sends `len` bytes (a multiple of 16, as both addresses) through the ring.
+__device__ __forceinline__ void send(Ring &r, uint8_t *buf, uint64_t *bars, uint8_t *blob, uint64_t src, uint64_t dst, uint32_t len) {
+    for (uint32_t off = 0; off < len && !r.failed; off += kPiece) {
+        if (r.issued - r.stored >= kAhead) store_oldest(r, buf, bars, blob);
+        if (r.failed) return;
+        const uint32_t st = r.issued % kStages, take = min(len - off, (uint32_t)kPiece);
+        // the piece that used this stage last has been read out: at most kStages - kAhead stores are younger
+        if (r.issued >= kStages) asm volatile("cp.async.bulk.wait_group.read %0;" ::"n"(kStages - kAhead) : "memory");
+        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(shared_address(&bars[st])), "r"(take) : "memory");
+        asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(shared_address(buf + st * kPiece)),
+                     "l"(src + off), "r"(take), "r"(shared_address(&bars[st]))
+                     : "memory");
+        r.dst[st] = dst + off;
+        r.len[st] = take;
+        r.issued++;
+    }
+}
+
+// The CTAs take the samples in turn, each split into `parts` when there are few.
+__global__ void __launch_bounds__(32)
+gather_payloads_kernel(const ImageDesc *__restrict__ descs, int n, int parts, uint8_t *__restrict__ blob, int32_t *__restrict__ failed) {
+    __shared__ __align__(128) uint8_t s_buf[kStages * kPiece];
+    __shared__ __align__(8) uint64_t s_bars[kStages];
+    const int lane = threadIdx.x;
+    if (lane < kStages) asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(shared_address(&s_bars[lane])) : "memory");
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    __syncwarp();
+    const int items = n * parts, step = gridDim.x;
+    Ring ring{};
+    for (int first = blockIdx.x; first < items; first += 32 * step) {
+        // the descriptors of this CTA's next 32 items, one per lane
+        const int item = first + lane * step;
+        uint64_t src = 0, dst = 0;
+        uint32_t run = 0, rows = 0, src_pitch = 0, dst_pitch = 0;
+        if (item < items) {
+            const ImageDesc &d = descs[item / parts];
+            const uint32_t part = item % parts;
+            if (d.src_addr != 0 && d.payload_size != 0) {
+                if (d.mode == 1 && d.raw_skew) { // a crop box: rows, each as the aligned 16-byte words that hold it
+                    const uint32_t per = ((uint32_t)d.rows + parts - 1) / parts, r0 = part * per, r1 = min(r0 + per, (uint32_t)d.rows);
+                    src_pitch = (uint32_t)d.width * 3;
+                    dst_pitch = d.raw_pitch;
+                    run = (uint32_t)d.cols * 3;
+                    rows = r1 > r0 ? r1 - r0 : 0;
+                    src = d.src_addr + (uint64_t)r0 * src_pitch;
+                    dst = d.payload_off + (uint64_t)r0 * dst_pitch;
+                } else { // one run; source and destination have the same alignment
+                    const uint32_t lead = (uint32_t)(d.src_addr & 15), all = lead + d.payload_size;
+                    const uint32_t per = ((all + parts - 1) / parts + 15) & ~15u, b0 = part * per, b1 = min(b0 + per, all);
+                    rows = b1 > b0 ? 1 : 0;
+                    run = b1 - b0;
+                    src = d.src_addr - lead + b0;
+                    dst = d.payload_off - lead + b0;
+                }
+            }
+        }
+        for (int k = 0; k < 32 && first + k * step < items; k++) {
+            const uint64_t s = __shfl_sync(0xffffffffu, src, k), t = __shfl_sync(0xffffffffu, dst, k);
+            const uint32_t len = __shfl_sync(0xffffffffu, run, k), m = __shfl_sync(0xffffffffu, rows, k);
+            const uint32_t sp = __shfl_sync(0xffffffffu, src_pitch, k), dp = __shfl_sync(0xffffffffu, dst_pitch, k);
+            if (lane == 0)
+                for (uint32_t r = 0; r < m && !ring.failed; r++) {
+                    // (a word that holds one byte of the run lies in the same page as that byte: the reads stay
+                    // inside the pinned allocation)
+                    const uint64_t from = s + (uint64_t)r * sp;
+                    const uint32_t lead = (uint32_t)(from & 15);
+                    send(ring, s_buf, s_bars, blob, from - lead, t + (uint64_t)r * dp, (lead + len + 15) & ~15u);
+                }
+            __syncwarp();
+        }
+    }
+    if (lane == 0) {
+        while (ring.stored != ring.issued && !ring.failed) store_oldest(ring, s_buf, s_bars, blob);
+        asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
+        if (ring.failed) {
+            *failed = 1;
+            for (; ring.stored != ring.issued; ring.stored++) arrived(s_bars, ring.stored % kStages, (ring.stored / kStages) & 1);
+        }
+    }
+}
+
+} // namespace
+
+void launch_gather_payloads(const ImageDesc *descs, int n, uint8_t *blob, int ctas, int32_t *failed, cudaStream_t stream) {
     if (n <= 0) return;
     if (ctas < 1) ctas = kGatherCtas;
-    const int grid = (n < ctas ? n : ctas) + 1;
-    if (in_flight >= 8)
-        gather_payloads_kernel<8><<<grid, 256, 0, stream>>>(descs, n, blob, small);
-    else
-        gather_payloads_kernel<4><<<grid, 256, 0, stream>>>(descs, n, blob, small);
+    const int parts = n >= 4 * ctas ? 1 : (4 * ctas + n - 1) / n;
+    gather_payloads_kernel<<<ctas, 32, 0, stream>>>(descs, n, parts, blob, failed);
 }
 
 } // namespace ffcvb

@@ -8,17 +8,11 @@
 namespace ffcvb {
 
 // Pulls every sample's payload from pinned host memory (descs[i].src_addr, read by the SMs over
-// PCIe) into its place in the device blob.  Source and destination share their alignment mod 16.
-// `ctas`: CTAs of 256 threads that fetch (< 1: kGatherCtas); `in_flight`: 16-byte loads a thread
-// of a JPEG payload's copy has outstanding (4 or 8).
-// `small`: copies from the blob's head to other device buffers that ride along.
-constexpr int kGatherCtas = 16;
-struct SmallCopies {
-    int n;
-    uint64_t off[8], bytes[8];
-    uint8_t *dst[8];
-};
-void launch_gather_payloads(const ImageDesc *descs, int n, uint8_t *blob, const SmallCopies &small, int ctas, int in_flight, cudaStream_t stream);
+// PCIe) into its place in the device blob.  Source and destination share their alignment mod 16, and the
+// bytes up to the next 16-byte boundaries around a payload's place are overwritten too.  `ctas`: CTAs
+// that fetch (< 1: kGatherCtas).  `failed` (device-visible) is set when a wait for the link ran out.
+constexpr int kGatherCtas = 64;
+void launch_gather_payloads(const ImageDesc *descs, int n, uint8_t *blob, int ctas, int32_t *failed, cudaStream_t stream);
 
 // Scratch and results of the entropy decode of a batch (device memory, no initialisation needed
 // except `done`, which starts at zero once and is left at zero).
@@ -86,10 +80,18 @@ struct ResizeSource {
     int uniform_h, uniform_w;
 };
 
+// Copies of a few kilobytes from one place in device memory to another that ride along.
+struct SmallCopies {
+    int n;
+    uint64_t bytes[8];
+    const uint8_t *src[8];
+    uint8_t *dst[8];
+};
+
 // Fused crop + INTER_AREA resize + flip/translate/cutout + lookup-table normalise.
 void launch_resize_augment(const ResizeSource &src, int n, const int32_t *params, int n_params,
                            const OpList &ops, int resize, int out_h, int out_w, int out_kind,
-                           const void *lut, void *out, const int32_t *status, cudaStream_t stream);
+                           const void *lut, void *out, const int32_t *status, const SmallCopies &small, cudaStream_t stream);
 
 // Colour jitter kinds (ffcv/transforms/color_jitter.py).
 enum { kJitterBrightness = 0, kJitterContrast = 1, kJitterSaturation = 2 };

@@ -155,7 +155,7 @@ resize_augment_kernel(const __grid_constant__ ResizeSource src, const int32_t *_
                       const __grid_constant__ OpList ops,
                       int resize, int out_h, int out_w, int band_rows, int groups, int planar, int win_bytes,
                       const OutT *__restrict__ lut, OutT *__restrict__ out,
-                      const int32_t *__restrict__ status) {
+                      const int32_t *__restrict__ status, const __grid_constant__ SmallCopies small) {
     extern __shared__ __align__(16) unsigned char s_raw[];
     constexpr bool kU8 = sizeof(OutT) == 1;
     // shared layout: [out tile][lut][x taps (5 arrays of out_w)][y taps (5 arrays of out_h)]
@@ -178,6 +178,9 @@ resize_augment_kernel(const __grid_constant__ ResizeSource src, const int32_t *_
         s_raw + ((off + sizeof(int) * (5 * ((size_t)out_w + out_h) + kMaxWindowRows) + 15) & ~(size_t)15);
 
     const int i = blockIdx.y;
+    if (blockIdx.x == 0 && i == 0)
+        for (int k = 0; k < small.n; k++)
+            for (uint64_t b = threadIdx.x; b < small.bytes[k]; b += blockDim.x) small.dst[k][b] = small.src[k][b];
     if (!kU8)
         for (int k = threadIdx.x; k < 768; k += blockDim.x) s_lut[(k % 3) * 256 + k / 3] = lut[k]; // per channel
 
@@ -568,7 +571,7 @@ resize_augment_kernel(const __grid_constant__ ResizeSource src, const int32_t *_
 template <typename OutT>
 static void launch_typed(const ResizeSource &src, int n, const int32_t *params, int n_params, const OpList &ops,
                          int resize, int out_h, int out_w, int planar, const void *lut, void *out,
-                         const int32_t *status, cudaStream_t stream) {
+                         const int32_t *status, const SmallCopies &small, cudaStream_t stream) {
     int band = (2048 + out_w - 1) / out_w;
     if (band < 1) band = 1;
     if (band > out_h) band = out_h;
@@ -607,20 +610,20 @@ static void launch_typed(const ResizeSource &src, int n, const int32_t *params, 
         }
     }
     kern<<<grid, 256, smem, stream>>>(src, params, n_params, ops, resize, out_h, out_w, band, groups, planar,
-                                      (int)win, (const OutT *)lut, (OutT *)out, status);
+                                      (int)win, (const OutT *)lut, (OutT *)out, status, small);
 }
 
 void launch_resize_augment(const ResizeSource &src, int n, const int32_t *params, int n_params,
                            const OpList &ops, int resize, int out_h, int out_w, int out_kind,
-                           const void *lut, void *out, const int32_t *status, cudaStream_t stream) {
+                           const void *lut, void *out, const int32_t *status, const SmallCopies &small, cudaStream_t stream) {
     if (n <= 0) return;
     const int planar = out_kind == kOutF16Nchw || out_kind == kOutF32Nchw;
     if (out_kind == kOutU8)
-        launch_typed<uint8_t>(src, n, params, n_params, ops, resize, out_h, out_w, 0, nullptr, out, status, stream);
+        launch_typed<uint8_t>(src, n, params, n_params, ops, resize, out_h, out_w, 0, nullptr, out, status, small, stream);
     else if (out_kind == kOutF16Nhwc || out_kind == kOutF16Nchw)
-        launch_typed<uint16_t>(src, n, params, n_params, ops, resize, out_h, out_w, planar, lut, out, status, stream);
+        launch_typed<uint16_t>(src, n, params, n_params, ops, resize, out_h, out_w, planar, lut, out, status, small, stream);
     else
-        launch_typed<uint32_t>(src, n, params, n_params, ops, resize, out_h, out_w, planar, lut, out, status, stream);
+        launch_typed<uint32_t>(src, n, params, n_params, ops, resize, out_h, out_w, planar, lut, out, status, small, stream);
 }
 
 } // namespace ffcvb

@@ -59,6 +59,8 @@ lib.ffcvb_stage_batch_fd.argtypes = [c_void_p, c_int, c_int, c_int, c_void_p, c_
 lib.ffcvb_stage_batch_fd.restype = c_int
 lib.ffcvb_submit_batch.argtypes = [c_void_p, c_int, c_void_p, c_void_p]
 lib.ffcvb_submit_batch.restype = c_int
+lib.ffcvb_submit_batch_after.argtypes = [c_void_p, c_int, c_void_p, c_void_p, c_void_p]
+lib.ffcvb_submit_batch_after.restype = c_int
 lib.ffcvb_rerun_batch.argtypes = [c_void_p, c_int, c_void_p, c_void_p]
 lib.ffcvb_rerun_batch.restype = c_int
 lib.ffcvb_set_header_cache.argtypes = [c_void_p, c_int]
@@ -251,8 +253,9 @@ class Context:
             rider.dst_dev = dst_ptr
         self._check(lib.ffcvb_set_batch_riders(self._h, slot, arr, len(riders), n), 'ffcvb_set_batch_riders')
 
-    def submit(self, slot, stream, out_ptr):
-        self._check(lib.ffcvb_submit_batch(self._h, slot, stream or None, out_ptr), 'ffcvb_submit_batch')
+    def submit(self, slot, stream, out_ptr, outputs_free=None):
+        """outputs_free: handle of an event that writing to the outputs has to wait for."""
+        self._check(lib.ffcvb_submit_batch_after(self._h, slot, stream or None, out_ptr, outputs_free), 'ffcvb_submit_batch')
 
     def rerun(self, slot, stream, out_ptr):
         self._check(lib.ffcvb_rerun_batch(self._h, slot, stream or None, out_ptr), 'ffcvb_rerun_batch')

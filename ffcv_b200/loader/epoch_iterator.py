@@ -62,6 +62,7 @@ class EpochIterator(Thread):
         self.consumed = [start_event] * self.slots
         self.consumed_events = [None] * self.slots  # one event per slot, recorded again and again
         self.queues_work = loader.graph.queues_work()
+        self.fused_only = self.is_cuda and loader.graph.first_work_is_fused()
         self.last_slot = None
         self.start()
 
@@ -102,15 +103,21 @@ class EpochIterator(Thread):
             # host-side wait; that batch was queued batches_ahead + 2 batches ago).  The native context
             # waits in the same way for its own staging buffer.
             done.synchronize()
+        # Only the work that writes to buffers the consumer sees waits for it: a single image pipeline hands
+        # the event down, so that transfer and decode of this batch run beside whatever is queued.
+        handle = None
         if cuda_event is not None:
-            cuda_event.wait(stream)
+            if self.fused_only:
+                handle = cuda_event.cuda_event
+            else:
+                cuda_event.wait(stream)
         if self.queues_work:
             with ch.cuda.stream(stream):
                 result = self.loader.graph.run_batch(batch_indices, slot, stream.cuda_stream, self.buffers,
-                                                     self.storage_state, self.epoch, b_ix)
+                                                     self.storage_state, self.epoch, b_ix, handle)
         else:
             result = self.loader.graph.run_batch(batch_indices, slot, stream.cuda_stream, self.buffers,
-                                                 self.storage_state, self.epoch, b_ix)
+                                                 self.storage_state, self.epoch, b_ix, handle)
         done.record(stream)
         return result
 

@@ -223,7 +223,7 @@ class FusedImageExecutor:
             params[:] = sample_plan_params(self.plan, self.metadata[batch_indices], self.base_seed, epoch, batch_ix)
         return params
 
-    def __call__(self, batch_indices, slot, stream_ptr, out, epoch, batch_ix):
+    def __call__(self, batch_indices, slot, stream_ptr, out, epoch, batch_ix, outputs_free=None):
         params = self.prepare(batch_indices, epoch, batch_ix)
         self.last_params = params
         if self.param_log is not None:
@@ -235,7 +235,7 @@ class FusedImageExecutor:
         # with asynchronous staging this returns while the staging threads still copy the payloads
         self.ctx.stage_arrays(slot, self.file_base_fn(), self._staging, self.native_plan)
         dst = out if len(out) == n else out[:n]
-        self.ctx.submit(slot, stream_ptr, dst.data_ptr())
+        self.ctx.submit(slot, stream_ptr, dst.data_ptr(), outputs_free)
         self._last_slot = slot
         p = self.plan
         if p.torch_image:

@@ -100,6 +100,13 @@ class Graph:
                                             [spec.decoder] + list(spec.transforms)))
         self.collect_requirements()
 
+    def first_work_is_fused(self):
+        """Whether the first GPU work a batch queues is the native call of an image pipeline (labels and
+        arrays that are not part of it come later): then that call alone has to know what to wait for."""
+        with_work = [p for p in self.pipelines if p.rider_host is None]
+        return bool(with_work) and with_work[0].executor is not None and \
+            sum(p.executor is not None for p in self.pipelines) == 1
+
     def queues_work(self):
         """Whether some operation behind the native calls may launch GPU work of its own (it then has
         to run under the slot's stream)."""
@@ -227,8 +234,9 @@ class Graph:
             return tuple(Graph._select(b, slot, count) for b in buffer)
         return buffer[slot][:count]
 
-    def run_batch(self, batch_indices, slot, stream_ptr, buffers, storage_state, epoch, batch_ix):
-        """One batch through every pipeline; returns the outputs in declaration order."""
+    def run_batch(self, batch_indices, slot, stream_ptr, buffers, storage_state, epoch, batch_ix, outputs_free=None):
+        """One batch through every pipeline; returns the outputs in declaration order.  `outputs_free`:
+        handle of an event that the work writing to the slot's buffers has to wait for."""
         n = len(batch_indices)
         results = []
         for pi, p in enumerate(self.pipelines):
@@ -245,7 +253,8 @@ class Graph:
             if p.rider_host is not None:
                 value = buffers[(pi, 'rider')][slot][:n]
             elif p.executor is not None:
-                value = p.executor(batch_indices, slot, stream_ptr, buffers[(pi, 'fused')][slot], epoch, batch_ix)
+                value = p.executor(batch_indices, slot, stream_ptr, buffers[(pi, 'fused')][slot], epoch, batch_ix,
+                                   outputs_free)
             elif p.soft_labels is not None:
                 value = p.soft_labels(p.column, buffers[(pi, 'soft')][slot][:n], batch_indices)
             else:

@@ -212,6 +212,11 @@ int ffcvb_staging_split(const ffcvb_ctx *ctx);
  * closures after it.  Returns after queueing. */
 int ffcvb_submit_batch(ffcvb_ctx *ctx, int slot, void *stream, void *out_dev);
 
+/* The same, for a caller that still has work queued on its own stream which uses `out_dev` or the
+ * riders' destinations: only what writes to those waits for the event `outputs_free` (a cudaEvent_t
+ * handle, NULL = none), while the transfer and the decode into the slot's own memory start at once. */
+int ffcvb_submit_batch_after(ffcvb_ctx *ctx, int slot, void *stream, void *out_dev, void *outputs_free);
+
 /* Re-runs the kernels of a batch whose staged bytes an earlier ffcvb_submit_batch on this slot
  * already copied to the GPU: same work, no host->device copy.  For measuring the rate with inputs
  * resident in HBM; no counterpart in the reference. */
