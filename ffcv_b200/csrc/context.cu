@@ -79,10 +79,13 @@ class Pool {
             j.limit = max_threads > 0 ? max_threads : 1 << 30;
             j.active = true;
         }
+        const int chunks = (n + (grain < 1 ? 1 : grain) - 1) / (grain < 1 ? 1 : grain);
         if (workers_.empty())
             wait(lane); // nobody else would run it
-        else
+        else if (chunks >= (int)workers_.size())
             cv_.notify_all();
+        else
+            for (int k = 0; k < chunks; k++) cv_.notify_one();
     }
     // Lends the calling thread to the lane's job, then waits until the job is complete.
     void wait(Lane lane) {
@@ -345,6 +348,8 @@ struct ffcvb_ctx {
     int cpu_share_permille = 0; // pinned source: share of the payload bytes the staging threads copy
     bool adaptive_split = false; // ... adjusted from batch to batch so that both sides take equally long
     double share = 0.0;          // the adjusted share, 0..1
+    double batch_interval = 0.0; // ms between two staging calls, smoothed
+    std::chrono::steady_clock::time_point last_staged;
     int split_copy_threads = 4; // ... and how many of them copy at a time (more only crowd the gather out)
     // Tuning overrides, read from the environment once when the context is created (0 = none):
     // FFCV_B200_COPY_THREADS, FFCV_B200_SUBSEQ_BITS, FFCV_B200_GATHER_CTAS.
@@ -898,12 +903,21 @@ int stage_impl(ffcvb_ctx *ctx, int slot, const Source &source, const uint64_t *p
     }
     if (direct && ctx->adaptive_split && s.range_len == 0) {
         // The slot's previous batch tells how long its two halves took: the staging threads' copy
-        // (host clock) and the GPU's gather (events).  Move the share towards equal times; the
-        // step is small because the measurement is several batches old.
+        // (host clock) and the GPU's gather (events).  While the gather takes most of the time between two
+        // batches the link is what they wait for: move the share towards equal times, in small steps
+        // because the measurement is several batches old.  Otherwise the threads' help is not needed.
+        const auto now = std::chrono::steady_clock::now();
+        const double since = ctx->last_staged.time_since_epoch().count()
+                                 ? std::chrono::duration<double, std::milli>(now - ctx->last_staged).count() : 0.0;
+        ctx->last_staged = now;
+        if (since > 0 && since < 100) ctx->batch_interval = ctx->batch_interval > 0 ? 0.75 * ctx->batch_interval + 0.25 * since : since;
         float tg = 0;
         if (s.gather_timed && cudaEventElapsedTime(&tg, s.ev_gather_start, s.ev_gathered) == cudaSuccess) {
             const double tc = s.staged_end > s.hdr.payload_off ? s.stage_ms[2] : 0.0;
-            if (tg + tc > 0) ctx->share += 0.04 * ((double)tg - tc) / ((double)tg + tc);
+            if (tg < 0.7 * ctx->batch_interval && tc < 0.7 * ctx->batch_interval)
+                ctx->share = ctx->share < 0.02 ? 0 : 0.8 * ctx->share;
+            else if (tg + tc > 0)
+                ctx->share += 0.04 * ((double)tg - tc) / ((double)tg + tc);
             if (ctx->share < 0) ctx->share = 0;
             if (ctx->share > kMaxAdaptiveShare) ctx->share = kMaxAdaptiveShare;
         } else {

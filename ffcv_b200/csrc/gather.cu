@@ -8,10 +8,11 @@ namespace {
 
 // The bytes go through shared memory as bulk copies (host -> shared, shared -> device) that one thread
 // per CTA issues: a ring of kStages pieces per CTA, half of them on their way in while the others leave.
-// What bounds it is the link: 64 CTAs x 8 KB keep 512 KB outstanding and move 48.6 GB/s of JPEG streams
-// and 46 GB/s of 0.7 KB crop rows (a plain DMA copy: 55.6), against 36-45 and 30-41 GB/s of a kernel of
-// 16 x 256 threads with eight 16-byte loads each.  As important is what it leaves to the decode kernels
-// beside it: no issue slots, 32 threads and 8 KB of shared memory on 64 SMs.
+// What bounds it is the link: one CTA per SM with 8 KB moves 46-48 GB/s of JPEG streams and 39-42 GB/s of
+// 0.7 KB crop rows inside the loader's pipeline (a plain DMA copy: 54.5; 64 CTAs: 33 GB/s of rows; two per SM:
+// 3 % more rows, but the decode kernels beside it slow down by as much), against 36-45 and 26-39 GB/s of a
+// kernel of 16 x 256 threads with eight 16-byte loads each.  As important is what it leaves to the decode
+// kernels: no issue slots, and 8 KB of shared memory per SM, which two CTAs of the entropy decoder do not need.
 constexpr int kStages = 8, kPiece = 1024, kAhead = 5; // kAhead: pieces on their way in
 
 __device__ __forceinline__ uint32_t shared_address(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }

@@ -11,7 +11,7 @@ namespace ffcvb {
 // PCIe) into its place in the device blob.  Source and destination share their alignment mod 16, and the
 // bytes up to the next 16-byte boundaries around a payload's place are overwritten too.  `ctas`: CTAs
 // that fetch (< 1: kGatherCtas).  `failed` (device-visible) is set when a wait for the link ran out.
-constexpr int kGatherCtas = 64;
+constexpr int kGatherCtas = 148;
 void launch_gather_payloads(const ImageDesc *descs, int n, uint8_t *blob, int ctas, int32_t *failed, cudaStream_t stream);
 
 // Scratch and results of the entropy decode of a batch (device memory, no initialisation needed
