@@ -256,14 +256,13 @@ struct DevBuf {
 struct Slot {
     uint8_t *host = nullptr; // pinned
     size_t host_cap = 0;
-    DevBuf blob, clean, segs, index, planes, rgb; // segs: per-segment scratch; index: per-block positions and DC values
+    DevBuf blob, clean, segs, slot_tables, index, planes, rgb; // segs: per-segment scratch; index: per-block positions and DC values
     BatchHeader hdr{};
     ffcvb_plan plan{};
-    int n = 0, n_jpeg = 0, n_segs = 0, n_multi = 0, n_restart = 0, max_tables = 0;
-    bool alike = false;
-    uint32_t max_raw = 0; // raw bytes of the largest segment
+    int n = 0, n_jpeg = 0;
+    EntropyWork work{}; // (the lists' addresses are filled in when the batch runs)
     int n_quad = 0, n_444 = 0, n_other = 0, max_w = 0, max_h = 0;
-    uint64_t jpeg_list_off = 0, segs_off = 0, multi_off = 0, restart_off = 0, block_tiles_off = 0, quad_tiles_off = 0;
+    uint64_t jpeg_list_off = 0, segs_off = 0, multi_off = 0, slot_images_off = 0, restart_off = 0, block_tiles_off = 0, quad_tiles_off = 0;
     uint64_t status_off = 0; // status word and counter of finished segments of every sample
     int n_block_tiles = 0, n_quad_tiles = 0;
     uint32_t total_blocks = 0;
@@ -297,7 +296,8 @@ struct Slot {
     std::vector<int> to_parse;
     std::vector<JpegHeader> parsed;
     std::vector<std::array<uint64_t, 9>> hashes; // of a parsed header's (DC, AC, quantisation) tables x 3 components
-    std::vector<int32_t> jpeg_list, multi, restart;
+    std::vector<int32_t> jpeg_list, multi, slot_images, restart;
+    std::vector<uint2> slot_segs;  // those of slot_images, behind
     std::vector<uint2> seg_list;   // (sample, segment) of the entropy decoder's CTAs
     std::vector<uint2> blk_tiles;  // (sample, k) of the block decoder's CTAs
     std::vector<uint2> quad_tiles; // (sample, tile x | tile y << 16) of the 4:2:0 colour kernel's CTAs
@@ -500,7 +500,7 @@ void ffcvb_destroy(ffcvb_ctx *ctx) {
     cudaDeviceSynchronize();
     for (auto &s : ctx->slots) {
         if (s.host) cudaFreeHost(s.host);
-        for (DevBuf *b : {&s.blob, &s.clean, &s.segs, &s.index, &s.planes, &s.rgb})
+        for (DevBuf *b : {&s.blob, &s.clean, &s.segs, &s.slot_tables, &s.index, &s.planes, &s.rgb})
             if (b->p) cudaFree(b->p);
         for (auto &e : s.ev)
             if (e) cudaEventDestroy(e);
@@ -715,7 +715,7 @@ int stage_impl(ffcvb_ctx *ctx, int slot, const Source &source, const uint64_t *p
         }
         fd_payload_end = off;
         // room behind the payloads for what is laid out after the parse: at most 255 tables of each kind
-        size_t tail = 255 * (sizeof(HuffTable) + sizeof(MultTable)) + 3 * (sizeof(int32_t) * (size_t)n + 16) + 256;
+        size_t tail = 255 * (sizeof(HuffTable) + sizeof(MultTable)) + 4 * (sizeof(int32_t) * (size_t)n + 16) + 256;
         for (int i = 0; i < n; i++) { // and the tables of CTAs: at most those of whole images and of the shortest segments
             tail += sizeof(uint2) * (size_t)((((heights[i] + 1) / 2 + 7) / 8) * ((((widths[i] + 1) / 2 + 1) / 2 + 1 + 31) / 32));
             tail += sizeof(uint2) * ((size_t)((heights[i] + 15) / 8) * ((widths[i] + 15) / 8) * 3 / kBlockTile + 4);
@@ -946,26 +946,33 @@ int stage_impl(ffcvb_ctx *ctx, int slot, const Source &source, const uint64_t *p
     };
     std::vector<BatchSet> batch_sets;
     int last_set = -1;
-    std::vector<int32_t> &jpeg_list = s.jpeg_list, &multi = s.multi, &restart = s.restart;
+    std::vector<int32_t> &jpeg_list = s.jpeg_list, &multi = s.multi, &slot_images = s.slot_images, &restart = s.restart;
     std::vector<uint2> &segs = s.seg_list, &blk_tiles = s.blk_tiles, &quad_tiles = s.quad_tiles;
     jpeg_list.clear();
     multi.clear();
+    slot_images.clear();
+    s.slot_segs.clear();
     restart.clear();
     segs.clear();
     blk_tiles.clear();
     quad_tiles.clear();
     size_t clean_bytes = 0, plane_bytes = 0, rgb_bytes = 0;
-    uint32_t total_blocks = 0, max_raw = 0;
-    int max_tables = 1, first_jpeg = -1;
-    bool alike = true; // all scans use the same tables in the same MCU layout
+    uint32_t total_blocks = 0;
+    EntropyWork &work = s.work;
+    work = EntropyWork{};
+    work.max_tables = 1;
+    work.alike = true;
+    int first_jpeg = -1;
     // Subsequence length: by the batch's bits, or, with a decode index, a function of the stream alone
     // (1024 bits), so that the recorded states stay usable whatever batch the sample lands in.
-    uint32_t target_bits = 1024;
+    uint32_t target_bits = 1024, seg_total = 0;
+    bool few = false; // few enough bits to decode from every slot at once
     if (!ctx->index_pool.p) {
         uint64_t bits = 0;
         for (int i = 0; i < n; i++)
             if (descs[i].mode == FFCVB_MODE_JPG && descs[i].host_status == 0) bits += (uint64_t)descs[i].scan_len * 8;
         target_bits = subseq_target(bits);
+        few = bits <= kSlotModeBits && !ctx->tune_subseq_bits;
     }
     if (ctx->tune_subseq_bits) target_bits = (uint32_t)ctx->tune_subseq_bits;
     ctx->stage_seq++;
@@ -1014,10 +1021,10 @@ int stage_impl(ffcvb_ctx *ctx, int slot, const Source &source, const uint64_t *p
         memcpy(d.q_tab, batch_sets[last_set].q_tab, sizeof(d.q_tab));
         d.block_base = total_blocks;
         total_blocks += d.nblocks;
-        if (2 * d.n_tab - d.n_dc_tab > max_tables) max_tables = 2 * d.n_tab - d.n_dc_tab;
+        if (2 * d.n_tab - d.n_dc_tab > work.max_tables) work.max_tables = 2 * d.n_tab - d.n_dc_tab;
         if (first_jpeg < 0) first_jpeg = i;
         const ImageDesc &f = descs[first_jpeg];
-        alike = alike && d.bpm == f.bpm && d.hs == f.hs && d.n_tab == f.n_tab && d.n_dc_tab == f.n_dc_tab &&
+        work.alike = work.alike && d.bpm == f.bpm && d.hs == f.hs && d.n_tab == f.n_tab && d.n_dc_tab == f.n_dc_tab &&
                 memcmp(d.tab_id, f.tab_id, sizeof(d.tab_id)) == 0 && memcmp(d.dc_tab, f.dc_tab, sizeof(d.dc_tab)) == 0 &&
                 memcmp(d.ac_tab, f.ac_tab, sizeof(d.ac_tab)) == 0;
         d.clean_off = clean_bytes;
@@ -1028,18 +1035,26 @@ int stage_impl(ffcvb_ctx *ctx, int slot, const Source &source, const uint64_t *p
             clean_bytes += align_up(4 * ((mcus + d.restart_interval - 1) / d.restart_interval + 2), 16);
             restart.push_back(i);
         } else {
-            const ScanLayout l = layout_scan(d.scan_len, target_bits);
+            const bool slots = few && d.bpm > 3; // (a guess among three slots falls in step within 1.4 kbit)
+            const ScanLayout l = slots ? layout_scan_slots(d.scan_len) : layout_scan(d.scan_len, target_bits);
             d.subseq_bits = l.subseq_bits;
             d.seg_raw = l.seg_raw;
             d.seg_warm = l.seg_warm;
             d.seg_stride = l.seg_stride;
             d.seg_count = l.seg_count;
-            d.seg_first = (uint32_t)segs.size();
+            d.seg_first = seg_total;
+            seg_total += l.seg_count;
             clean_bytes += (size_t)l.seg_count * l.seg_stride;
-            for (uint32_t k = 0; k < l.seg_count; k++) segs.push_back(make_uint2((uint32_t)i, k));
-            if (l.seg_count > 1) multi.push_back(i);
-            const uint32_t raw = kSegSubs * l.subseq_bits / 8 + kSegOverlap;
-            if (raw > max_raw) max_raw = raw;
+            if (slots) {
+                d.slots = 1 + (uint32_t)s.slot_segs.size();
+                slot_images.push_back(i);
+                if ((int)l.seg_count > work.max_slot_segs) work.max_slot_segs = (int)l.seg_count;
+            } else if (l.seg_count > 1) {
+                multi.push_back(i);
+            }
+            for (uint32_t k = 0; k < l.seg_count; k++) (slots ? s.slot_segs : segs).push_back(make_uint2((uint32_t)i, k));
+            const uint32_t raw = l.seg_stride - 64 - 16; // (at least run-up, own bytes and overlap)
+            if (raw > work.max_raw) work.max_raw = raw;
             if (ctx->index_pool.p) {
                 const uint64_t key = ptrs[i];
                 auto it = ctx->index_map.find(key);
@@ -1121,10 +1136,12 @@ int stage_impl(ffcvb_ctx *ctx, int slot, const Source &source, const uint64_t *p
         off = align_up(off + sizeof(int32_t) * jpeg_list.size(), 16);
         s.multi_off = off;
         off = align_up(off + sizeof(int32_t) * multi.size(), 16);
+        s.slot_images_off = off;
+        off = align_up(off + sizeof(int32_t) * slot_images.size(), 16);
         s.restart_off = off;
         off = align_up(off + sizeof(int32_t) * restart.size(), 16);
         s.segs_off = off;
-        off = align_up(off + sizeof(uint2) * segs.size(), 16);
+        off = align_up(off + sizeof(uint2) * (segs.size() + s.slot_segs.size()), 16);
         s.block_tiles_off = off;
         off = align_up(off + sizeof(uint2) * blk_tiles.size(), 16);
         s.quad_tiles_off = off;
@@ -1210,7 +1227,8 @@ int stage_impl(ffcvb_ctx *ctx, int slot, const Source &source, const uint64_t *p
     if ((rc = grow_host(ctx, s.host, s.host_cap, host_need + 64))) return rc;
     if ((rc = grow_dev(ctx, s.blob, off + 64))) return rc;
     if ((rc = grow_dev(ctx, s.clean, clean_bytes + 512))) return rc;
-    if ((rc = grow_dev(ctx, s.segs, segs.size() * (sizeof(SegMeta) + 4 * kSegSubs + 16) + 64))) return rc;
+    if ((rc = grow_dev(ctx, s.segs, seg_total * (sizeof(SegMeta) + 4 * kSegSubs + 16) + 64))) return rc;
+    if (!s.slot_segs.empty() && (rc = grow_dev(ctx, s.slot_tables, s.slot_segs.size() * sizeof(SlotTables)))) return rc;
     if ((rc = grow_dev(ctx, s.index, (size_t)total_blocks * 6 + 64))) return rc;
     if ((rc = grow_dev(ctx, s.planes, plane_bytes + 64))) return rc;
     if ((rc = grow_dev(ctx, s.rgb, rgb_bytes + 64))) return rc;
@@ -1269,18 +1287,19 @@ int stage_impl(ffcvb_ctx *ctx, int slot, const Source &source, const uint64_t *p
     }
     if (!jpeg_list.empty()) memcpy(s.host + s.jpeg_list_off, jpeg_list.data(), 4 * jpeg_list.size());
     if (!multi.empty()) memcpy(s.host + s.multi_off, multi.data(), 4 * multi.size());
+    if (!slot_images.empty()) memcpy(s.host + s.slot_images_off, slot_images.data(), 4 * slot_images.size());
     if (!restart.empty()) memcpy(s.host + s.restart_off, restart.data(), 4 * restart.size());
     if (!segs.empty()) memcpy(s.host + s.segs_off, segs.data(), sizeof(uint2) * segs.size());
+    if (!s.slot_segs.empty()) memcpy(s.host + s.segs_off + sizeof(uint2) * segs.size(), s.slot_segs.data(), sizeof(uint2) * s.slot_segs.size());
     if (!blk_tiles.empty()) memcpy(s.host + s.block_tiles_off, blk_tiles.data(), sizeof(uint2) * blk_tiles.size());
     if (!quad_tiles.empty()) memcpy(s.host + s.quad_tiles_off, quad_tiles.data(), sizeof(uint2) * quad_tiles.size());
     s.n_quad_tiles = (int)quad_tiles.size();
     s.n_block_tiles = (int)blk_tiles.size();
-    s.n_segs = (int)segs.size();
-    s.n_multi = (int)multi.size();
-    s.n_restart = (int)restart.size();
-    s.max_raw = max_raw;
-    s.max_tables = max_tables;
-    s.alike = alike;
+    work.n_guess = (int)segs.size();
+    work.n_slots = (int)s.slot_segs.size();
+    work.n_multi = (int)multi.size();
+    work.n_slot_images = (int)slot_images.size();
+    work.n_restart = (int)restart.size();
 
     const auto t2 = std::chrono::steady_clock::now();
     // ---- parallel: gather the payload bytes into pinned memory
@@ -1486,16 +1505,21 @@ static int run_batch(ffcvb_ctx *ctx, Slot &s, cudaStream_t st, void *out_dev, bo
         const int32_t *jl = reinterpret_cast<const int32_t *>(blob + s.jpeg_list_off);
         EntropyScratch scratch{};
         scratch.clean = (uint8_t *)s.clean.p;
+        EntropyWork work = s.work;
+        work.segs = reinterpret_cast<const uint2 *>(blob + s.segs_off);
+        work.multi = reinterpret_cast<const int32_t *>(blob + s.multi_off);
+        work.slot_images = reinterpret_cast<const int32_t *>(blob + s.slot_images_off);
+        work.restart = reinterpret_cast<const int32_t *>(blob + s.restart_off);
+        const size_t n_segs = (size_t)work.n_guess + work.n_slots;
         scratch.seg_dc = (int32_t *)s.segs.p;
-        scratch.sub_info = (uint32_t *)(scratch.seg_dc + 4 * (size_t)s.n_segs);
-        scratch.meta = (SegMeta *)(scratch.sub_info + kSegSubs * (size_t)s.n_segs);
+        scratch.sub_info = (uint32_t *)(scratch.seg_dc + 4 * n_segs);
+        scratch.meta = (SegMeta *)(scratch.sub_info + kSegSubs * n_segs);
+        scratch.slots = (SlotTables *)s.slot_tables.p;
         scratch.done = (uint32_t *)(blob + s.status_off) + s.n;
         scratch.pos = (uint32_t *)s.index.p;
         scratch.dc = (int16_t *)(scratch.pos + s.total_blocks);
-        launch_entropy_decode(descs, reinterpret_cast<const uint2 *>(blob + s.segs_off), s.n_segs,
-                              reinterpret_cast<const int32_t *>(blob + s.multi_off), s.n_multi,
-                              reinterpret_cast<const int32_t *>(blob + s.restart_off), s.n_restart, blob, huff, scratch, status,
-                              s.max_raw, s.max_tables, s.alike, (uint8_t *)ctx->index_pool.p, (unsigned long long *)ctx->index_stats.p, st);
+        launch_entropy_decode(descs, work, blob, huff, scratch, status, (uint8_t *)ctx->index_pool.p,
+                              (unsigned long long *)ctx->index_stats.p, st);
         if (prof) CU(cudaEventRecord(s.ev[2], st));
         launch_blocks(descs, reinterpret_cast<const uint2 *>(blob + s.block_tiles_off), s.n_block_tiles, huff, mult, scratch,
                       (uint8_t *)s.planes.p, st);
@@ -1710,7 +1734,8 @@ int ffcvb_batch_launches(const ffcvb_ctx *ctx, int slot) {
     if (!ctx || slot < 0 || slot >= (int)ctx->slots.size() || !ctx->slots[slot].staged) return -1;
     const Slot &s = ctx->slots[slot];
     int k = 1 + (s.direct && s.range_len == 0 ? 1 : 0); // fused resize/augment/normalise (+ payload gather)
-    k += (s.n_quad > 0) + (s.n_444 > 0) + (s.n_other > 0) + (s.n_block_tiles > 0) + 2 * (s.n_segs > 0) + (s.n_multi > 0) + (s.n_restart > 0);
+    k += (s.n_quad > 0) + (s.n_444 > 0) + (s.n_other > 0) + (s.n_block_tiles > 0) + (s.work.n_guess > 0) + (s.work.n_multi > 0) +
+         2 * (s.work.n_slots > 0) + (s.work.n_guess + s.work.n_slots > 0) + (s.work.n_restart > 0);
     return k;
 }
 

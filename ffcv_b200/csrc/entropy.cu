@@ -17,6 +17,8 @@
 //                       Segments behind the first decode the last 8 kbit before them as a run-up.
 //   scan_stitch_kernel  scans of several segments: where a run-up was too short, walks
 //                       on from the exact state until it meets the recorded one.
+//   scan_slots_kernel, scan_chain_kernel   instead of the two above while a batch's scans leave most of the
+//                       GPU idle: every subsequence from all block slots at once, see there.
 //   scan_index_kernel   every subsequence once more from its exact state: records the blocks; the
 //                       last CTA of an image integrates the DC differences.
 //
@@ -34,15 +36,16 @@ constexpr int kFastBytes = 2 * kHuffFast;   // a Huffman table in shared memory
 
 // The threads that work on one segment.  A CTA holds one team, or several that share the Huffman
 // tables in shared memory and meet at barriers of their own.
-template <int TEAMS>
+template <int TEAMS, int SIZE = kThreads>
 struct Team {
+    static constexpr int size = SIZE;
     int index, tid;
-    __device__ __forceinline__ Team() : index(TEAMS == 1 ? 0 : threadIdx.x / kThreads), tid(TEAMS == 1 ? threadIdx.x : threadIdx.x % kThreads) {}
+    __device__ __forceinline__ Team() : index(TEAMS == 1 ? 0 : threadIdx.x / SIZE), tid(TEAMS == 1 ? threadIdx.x : threadIdx.x % SIZE) {}
     __device__ __forceinline__ void sync() const {
         if (TEAMS == 1)
             __syncthreads();
         else
-            asm volatile("bar.sync %0, %1;" ::"r"(index + 1), "n"(kThreads) : "memory");
+            asm volatile("bar.sync %0, %1;" ::"r"(index + 1), "n"(SIZE) : "memory");
     }
 };
 
@@ -69,9 +72,9 @@ __device__ __forceinline__ int scan_exclusive(int v, int tid, int warps, int *s_
     total = all;
     return before + inc - v;
 }
-template <int TEAMS>
-__device__ __forceinline__ int team_scan(const Team<TEAMS> &team, int v, int *s_warp, int &total) {
-    return scan_exclusive(v, team.tid, kThreads / 32, s_warp, total, [&] { team.sync(); });
+template <class AnyTeam>
+__device__ __forceinline__ int team_scan(const AnyTeam &team, int v, int *s_warp, int &total) {
+    return scan_exclusive(v, team.tid, AnyTeam::size / 32, s_warp, total, [&] { team.sync(); });
 }
 
 __device__ __forceinline__ uint32_t shared_address(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -278,8 +281,8 @@ __device__ __forceinline__ uint32_t first_bytes(int k) {
 // bytes.  s_mark[k] receives how many kept bytes lie before raw offset at[k].  Returns the number of
 // bytes kept.  A thread takes 32 aligned bytes per pass; nearly all words lose nothing and leave as
 // one shifted word, single bytes are stored only where two threads' bytes share a word.
-template <int TEAMS>
-__device__ __forceinline__ uint32_t unstuff(const Team<TEAMS> &team, unsigned char *buf, const uint8_t *__restrict__ src, uint32_t len,
+template <class AnyTeam>
+__device__ __forceinline__ uint32_t unstuff(const AnyTeam &team, unsigned char *buf, const uint8_t *__restrict__ src, uint32_t len,
                                             bool first, const uint32_t (&at)[2], int *s_warp, uint32_t *s_mark) {
     constexpr int kWords = 8;
     const int tid = team.tid;
@@ -294,10 +297,10 @@ __device__ __forceinline__ uint32_t unstuff(const Team<TEAMS> &team, unsigned ch
         for (int k = 0; k < 2; k++) v[k] = w + 4 * k < nwords ? reinterpret_cast<const uint4 *>(aligned)[(w >> 2) + k] : make_uint4(0, 0, 0, 0);
     };
     fetch(tid * kWords);
-    for (uint32_t tile = 0; tile < nwords; tile += kThreads * kWords) {
+    for (uint32_t tile = 0; tile < nwords; tile += AnyTeam::size * kWords) {
         const uint32_t w0 = tile + tid * kWords;
         uint32_t x[kWords] = {v[0].x, v[0].y, v[0].z, v[0].w, v[1].x, v[1].y, v[1].z, v[1].w};
-        fetch(w0 + kThreads * kWords); // the next pass's bytes arrive during this one
+        fetch(w0 + AnyTeam::size * kWords); // the next pass's bytes arrive during this one
         const int off = (int)(w0 * 4) - (int)lead; // raw offset of the first of these bytes
         const bool edge = off < 0 || off + kWords * 4 > (int)len;
         if (first && off < 0) // what lies in front of the scan is no predecessor
@@ -430,7 +433,7 @@ scan_sync_kernel(const ImageDesc *__restrict__ descs, const uint2 *__restrict__ 
             const uint32_t *src = reinterpret_cast<const uint32_t *>(h + 1) + (size_t)j * (kSegSubs + 2);
             scratch.sub_info[seg * kSegSubs + tid] = __ldcg(src + tid);
             if (tid == 0) {
-                scratch.meta[seg] = SegMeta{own_bit, own_end, kept, __ldcg(src + kSegSubs), __ldcg(src + kSegSubs + 1)};
+                scratch.meta[seg] = SegMeta{own_bit, own_end, kept, __ldcg(src + kSegSubs), __ldcg(src + kSegSubs + 1), 0};
                 if (j == 0 && index_stats) atomicAdd(index_stats, 1ull);
             }
             return;
@@ -483,7 +486,7 @@ scan_sync_kernel(const ImageDesc *__restrict__ descs, const uint2 *__restrict__ 
     if (tid < n_own) scratch.sub_info[seg * kSegSubs + tid] = sh.entry[tid + warm] | done << 16;
     int total;
     team_scan(team, (int)done, sh.warp, total);
-    if (tid == 0) scratch.meta[seg] = SegMeta{own_bit, own_end, kept, sh.entry[n_subs], (uint32_t)total};
+    if (tid == 0) scratch.meta[seg] = SegMeta{own_bit, own_end, kept, sh.entry[n_subs], (uint32_t)total, 0};
 }
 
 // Scans of several segments, one CTA each: the exit state of every segment has to be the entry state
@@ -535,6 +538,293 @@ scan_stitch_kernel(const ImageDesc *__restrict__ descs, const int32_t *__restric
     }
 }
 
+// ---- few scans: every slot at once --------------------------------------------------------
+// What keeps a decoder that starts mid-stream out of step is the block's slot inside the MCU.  With the GPU
+// mostly idle every subsequence is therefore decoded from all slots in parallel, then from the exit states of
+// the subsequence before it that were not among those, and so on for kSlotRounds rounds; the real state is
+// among the known ones by then.  Three times the work of one guess, but a chain of 4 x 512 bits instead of the
+// 6 to 10 kbit that the slowest of a few hundred guesses takes to fall in step: a 224x256 photograph's
+// scan takes 33 + 7 us instead of 61 + 5, one of 1213x1617 pixels 36 + 15 instead of 105 + 15.
+constexpr int kSlotRunUp = kSlotRounds, kSlotThreads = ((kSlotSubs + kSlotRunUp) * 6 + 31) / 32 * 32;
+
+struct SlotShared {
+    uint16_t state[kSlotSubs + kSlotRunUp + 1][kSlotStates]; // entry states, relative to the subsequence's start
+    uint16_t exit[kSlotSubs + kSlotRunUp][kSlotStates];      // ... and what they lead to
+    uint16_t blocks[kSlotSubs + kSlotRunUp][kSlotStates];
+    uint8_t next[kSlotSubs + kSlotRunUp][kSlotStates];       // place of `exit` among the next subsequence's states, or kSlotMiss
+    int count[kSlotSubs + kSlotRunUp + 1];
+    uint16_t list[kSlotThreads]; // (subsequence << 4 | state) to decode
+    int n_list;
+    int warp[kSlotThreads / 32];
+    uint32_t mark[2];
+};
+
+// Place of state e among the first n of `states` (two per word), or kSlotMiss.
+__device__ __forceinline__ uint32_t find_state(const uint16_t *states, int n, uint32_t e) {
+    const uint32_t *pairs = reinterpret_cast<const uint32_t *>(states);
+    uint32_t found = kSlotMiss;
+#pragma unroll
+    for (int k = kSlotStates / 2 - 1; k >= 0; k--) {
+        const uint32_t p = pairs[k];
+        if ((p >> 16) == e && 2 * k + 1 < n) found = 2 * k + 1;
+        if ((p & 0xffff) == e && 2 * k < n) found = 2 * k;
+    }
+    return found;
+}
+
+// One CTA per segment, at first one thread per (subsequence, slot).  Bound by the chain of look-ups, at one or
+// two CTAs per SM.
+__global__ void __launch_bounds__(kSlotThreads)
+scan_slots_kernel(const ImageDesc *__restrict__ descs, const uint2 *__restrict__ segs, const uint8_t *__restrict__ blob,
+                  const HuffTable *__restrict__ huff, EntropyScratch scratch, int table_slots) {
+    extern __shared__ __align__(16) unsigned char s_dyn[];
+    __shared__ __align__(16) SlotShared sh;
+    const Team<1, kSlotThreads> team;
+    const int tid = team.tid;
+    Tables *tables = reinterpret_cast<Tables *>(s_dyn);
+    unsigned char *buf = s_dyn + tables_bytes(table_slots);
+    const uint2 which = segs[blockIdx.x];
+    const uint32_t j = which.y;
+    const ImageDesc &d = descs[which.x];
+    const uint32_t S = d.subseq_bits, R = d.seg_raw, warm = j == 0 ? 0 : d.seg_warm;
+    const int bpm = d.bpm;
+    load_tables(tables, d, huff);
+    const uint32_t scan_len = d.scan_len, own0 = j * R, own1 = min(own0 + R, scan_len);
+    const uint32_t raw0 = own0 - min(own0, warm * (S >> 3)), raw1 = min(own1 + kSegOverlap, scan_len);
+    const uint32_t at[2] = {own0 - raw0, own1 - raw0};
+    const uint32_t kept = unstuff(team, buf, blob + d.payload_off + d.scan_off + raw0, raw1 - raw0, raw0 == 0, at, sh.warp, sh.mark);
+    const uint32_t own_bit = at[0] == 0 ? 0 : sh.mark[0] * 8, own_end = own1 == raw1 ? kept * 8 : sh.mark[1] * 8;
+    {
+        uint4 *dst = reinterpret_cast<uint4 *>(scratch.clean + d.clean_off + (size_t)j * d.seg_stride);
+        for (uint32_t k = tid; k < (kept + 64 + 15) / 16; k += kSlotThreads) dst[k] = reinterpret_cast<const uint4 *>(buf)[k];
+    }
+    const size_t seg = (size_t)d.seg_first + j;
+    const int n_own = (int)((own_end - own_bit + S - 1) / S), n_subs = (int)warm + n_own;
+    auto start_of = [&](int t) -> int { return (int)own_bit + (t - (int)warm) * (int)S; };
+    // ---- the guesses: every slot (the scan itself begins with slot 0)
+    for (int k = tid; k < (n_subs + 1) * kSlotStates; k += kSlotThreads) {
+        const int c = k % kSlotStates;
+        sh.state[k / kSlotStates][c] = (uint16_t)pack(Cursor{0, c < bpm ? c : 0, 0}, 0);
+        if (k / kSlotStates < n_subs) sh.next[k / kSlotStates][c] = kSlotMiss;
+    }
+    for (int t = tid; t <= n_subs; t += kSlotThreads) sh.count[t] = j == 0 && t == 0 ? 1 : (t == n_subs ? 0 : bpm);
+    copies_wait();
+    __syncthreads();
+    auto decode = [&](int t, int i) {
+        // (the run-up lacks the bytes that its stuffing took: its first subsequence is shorter)
+        const uint32_t start = (uint32_t)max(start_of(t), 0), end = (uint32_t)max(min(start_of(t + 1), (int)own_end), 0);
+        Cursor cur = unpack(sh.state[t][i], start);
+        sh.blocks[t][i] = (uint16_t)walk<false>(buf, cur, end, tables, d, huff);
+        sh.exit[t][i] = (uint16_t)pack(cur, end);
+    };
+    int lo = 0; // states of this thread's subsequence that were decoded in the last round: [lo, hi)
+    for (int round = 0; round < kSlotRounds; round++) {
+        int sub = tid / bpm, which_state = tid - sub * bpm;
+        bool live = sub < n_subs && which_state < sh.count[min(sub, n_subs)];
+        if (round > 0) {
+            live = tid < sh.n_list;
+            sub = live ? sh.list[tid] >> 4 : 0;
+            which_state = live ? sh.list[tid] & (kSlotStates - 1) : 0;
+        }
+        if (live) decode(sub, which_state);
+        __syncthreads();
+        if (tid == 0) sh.n_list = 0;
+        __syncthreads();
+        // thread t looks its subsequence's new exits up among the next one's states; the unknown ones join them
+        const int t = tid;
+        int first_new = 0, n_new = 0;
+        if (t < n_subs) {
+            const int hi = sh.count[t];
+            // (count[t] may grow below, by the thread before this one: a barrier lies between)
+            int n = sh.count[t + 1];
+            first_new = n;
+            for (int i = lo; i < hi; i++) {
+                const uint32_t e = sh.exit[t][i];
+                uint32_t at_ = find_state(sh.state[t + 1], n, e);
+                if (at_ == kSlotMiss && n < kSlotStates - 1 && round + 1 < kSlotRounds && t + 1 < n_subs) {
+                    at_ = n;
+                    sh.state[t + 1][n++] = (uint16_t)e;
+                }
+                sh.next[t][i] = (uint8_t)at_;
+            }
+            lo = hi;
+            n_new = n - first_new;
+        }
+        __syncthreads();
+        if (n_new > 0) {
+            sh.count[t + 1] = first_new + n_new;
+            const int base = atomicAdd(&sh.n_list, n_new); // (at most one per state decoded in this round, hence per thread)
+            for (int k = 0; k < n_new; k++) sh.list[base + k] = (uint16_t)((t + 1) << 4 | (first_new + k));
+        }
+        __syncthreads();
+        if (sh.n_list == 0) break;
+    }
+    // ---- what the segment makes of every state its first own subsequence may begin in
+    SlotTables *out = scratch.slots + (d.slots - 1) + j;
+    if (tid < 32) {
+        SlotMap map{kNoState, 0};
+        const bool wanted = n_own > 0 && tid < min(sh.count[warm], kSlotStates);
+        auto follow = [&](int i, bool repair) {
+            const int entry = i;
+            uint32_t total = 0;
+            int t = (int)warm;
+            for (; t + 1 < n_subs; t++) {
+                total += sh.blocks[t][i];
+                int to = sh.next[t][i];
+                if (to == kSlotMiss && repair && sh.count[t + 1] < kSlotStates - 1) {
+                    to = sh.count[t + 1]++;
+                    sh.state[t + 1][to] = sh.exit[t][i];
+                    decode(t + 1, to);
+                    sh.next[t + 1][to] = t + 2 < n_subs ? (uint8_t)find_state(sh.state[t + 2], sh.count[t + 2], sh.exit[t + 1][to]) : (uint8_t)kSlotMiss;
+                    sh.next[t][i] = (uint8_t)to;
+                }
+                if (to == kSlotMiss) return;
+                i = to;
+            }
+            map = SlotMap{sh.state[warm][entry], sh.exit[t][i] | (total + sh.blocks[t][i]) << 16};
+        };
+        if (wanted) follow(tid, false);
+        // Which of them the run-up's guesses lead to: the real one is nearly always among these few, so where
+        // one of these meets an unknown state a thread decodes on until it is in step.
+        int i = tid;
+        bool reached = tid < sh.count[0];
+        for (int t = 0; t < (int)warm && reached; t++) {
+            i = sh.next[t][i];
+            reached = i != kSlotMiss;
+        }
+        const uint32_t unresolved = __ballot_sync(0xffffffffu, wanted && map.from == kNoState);
+        for (uint32_t left = unresolved & __reduce_or_sync(0xffffffffu, reached ? 1u << i : 0u); left; left &= left - 1) {
+            if (tid == __ffs(left) - 1) follow(tid, true);
+            __syncwarp();
+        }
+        if (tid < kSlotStates) out->map[tid] = map;
+    }
+    __syncthreads();
+    for (int k = tid; k < n_own * kSlotStates; k += kSlotThreads) {
+        const int t = k / kSlotStates, i = k % kSlotStates;
+        out->info[t][i] = i < sh.count[t + warm] ? sh.state[t + warm][i] | (uint32_t)sh.blocks[t + warm][i] << 16 : kNoState;
+        out->next[t][i] = sh.next[t + warm][i];
+    }
+    if (tid == 0) scratch.meta[seg] = SegMeta{own_bit, own_end, kept, 0, 0, 0};
+}
+
+// One CTA per image: follows the real state from segment to segment through their maps.  Many segments are
+// shared out: every warp composes the maps of a run of them for all 16 states, the first warp chains
+// the runs, then every warp follows the real state through its own run.  Where the real state is not
+// among a segment's (one in several thousand), one thread decodes that segment.
+constexpr int kChainThreads = 1024;
+__global__ void __launch_bounds__(kChainThreads)
+scan_chain_kernel(const ImageDesc *__restrict__ descs, const int32_t *__restrict__ list, const HuffTable *__restrict__ huff,
+                  EntropyScratch scratch, int map_slots) {
+    extern __shared__ __align__(16) SlotMap s_maps[]; // [segment][state]
+    __shared__ uint32_t s_entry[kChainThreads / 32 + 1];
+    __shared__ SlotMap s_run[kChainThreads / 32][kSlotStates]; // (state, or kNoState; state behind the run)
+    __shared__ uint8_t s_done[kChainThreads / 32];
+    const ImageDesc &d = descs[list[blockIdx.x]];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, n_seg = (int)d.seg_count;
+    SlotTables *tabs = scratch.slots + (d.slots - 1);
+    SegMeta *meta = scratch.meta + d.seg_first;
+    const uint32_t S = d.subseq_bits;
+    const bool staged = n_seg <= map_slots;
+    if (staged)
+        for (int k = tid; k < n_seg * kSlotStates; k += blockDim.x) s_maps[k] = tabs[k / kSlotStates].map[k % kSlotStates];
+    __syncthreads();
+    auto map_of = [&](int k, int i) -> SlotMap { return staged ? s_maps[k * kSlotStates + i] : tabs[k].map[i]; };
+    // The real state `state` through segment k, by a whole warp: which of its states it is, and what is behind it.
+    auto follow = [&](int k, uint32_t state) -> uint32_t {
+        const SlotMap m = map_of(k, lane & (kSlotStates - 1));
+        const uint32_t who = __ballot_sync(0xffffffffu, m.from == state) & ((1u << kSlotStates) - 1);
+        uint32_t behind;
+        if (who != 0) {
+            const int src = __ffs(who) - 1;
+            behind = __shfl_sync(0xffffffffu, m.to, src);
+            if (lane == 0) {
+                meta[k].entry = src;
+                meta[k].exit = behind & 0xffff;
+                meta[k].blocks = behind >> 16;
+            }
+        } else {
+            if (lane == 0) { // subsequence by subsequence; those with an unknown state are decoded here, into the last place
+                const SegMeta sm = meta[k];
+                SlotTables &tab = tabs[k];
+                const uint32_t *words = reinterpret_cast<const uint32_t *>(scratch.clean + d.clean_off + (size_t)k * d.seg_stride);
+                const int n_own = (int)((sm.own_end - sm.own_bit + S - 1) / S);
+                uint32_t at = state, blocks = 0, from = kSlotMiss;
+                uint32_t i = kSlotMiss; // place of `at` among the states of subsequence t
+                for (int t = 0; t < n_own; t++) {
+                    const uint32_t start = sm.own_bit + (uint32_t)t * S, end = min(start + S, sm.own_end);
+                    if (i == kSlotMiss)
+                        for (uint32_t c = 0; c < kSlotStates - 1 && i == kSlotMiss; c++)
+                            if ((tab.info[t][c] & 0xffff) == at) i = c;
+                    const bool known = i != kSlotMiss;
+                    if (!known) i = kSlotStates - 1;
+                    if (t == 0) meta[k].entry = i;
+                    else tab.next[t - 1][from] = (uint8_t)i;
+                    uint32_t to = known && t + 1 < n_own ? tab.next[t][i] : kSlotMiss;
+                    if (to == kSlotMiss) {
+                        Cursor cur = unpack(at, start);
+                        const uint32_t done = walk_plain<false>(words, cur, end, d, huff, nullptr, 0, 0);
+                        tab.info[t][i] = at | done << 16;
+                        at = pack(cur, end);
+                        blocks += done;
+                    } else {
+                        blocks += tab.info[t][i] >> 16;
+                        at = tab.info[t + 1][to] & 0xffff;
+                    }
+                    from = i;
+                    i = to;
+                }
+                if (n_own == 0) meta[k].entry = 0;
+                meta[k].exit = at;
+                meta[k].blocks = blocks;
+                behind = at;
+            }
+            behind = __shfl_sync(0xffffffffu, behind, 0);
+        }
+        return behind & 0xffff;
+    };
+    const int warps = blockDim.x / 32, run = (n_seg + warps - 1) / warps, first = warp * run, last = min(first + run, n_seg);
+    if (warps == 1) {
+        uint32_t state = 0;
+        for (int k = 0; k < n_seg; k++) state = follow(k, state);
+        return;
+    }
+    if (first < last && lane < kSlotStates) {
+        const SlotMap m = map_of(first, lane);
+        uint32_t at = m.from == kNoState ? kNoState : m.to & 0xffff;
+        for (int k = first + 1; k < last; k++) {
+            uint32_t to = kNoState;
+            for (int i = 0; i < kSlotStates; i++) {
+                const SlotMap o = map_of(k, i);
+                if (o.from == at && at != kNoState) to = o.to & 0xffff;
+            }
+            at = to;
+        }
+        s_run[warp][lane] = SlotMap{at == kNoState ? kNoState : m.from, at};
+    }
+    if (lane == 0) s_done[warp] = 0;
+    __syncthreads();
+    if (warp == 0) {
+        uint32_t state = 0;
+        for (int w = 0; w < warps && w * run < n_seg; w++) {
+            if (lane == 0) s_entry[w] = state;
+            const SlotMap m = s_run[w][lane & (kSlotStates - 1)];
+            const uint32_t who = __ballot_sync(0xffffffffu, m.from == state) & ((1u << kSlotStates) - 1);
+            if (who != 0) {
+                state = __shfl_sync(0xffffffffu, m.to, __ffs(who) - 1);
+            } else { // the run cannot be skipped
+                for (int k = w * run; k < min((w + 1) * run, n_seg); k++) state = follow(k, state);
+                if (lane == 0) s_done[w] = 1;
+            }
+        }
+    }
+    __syncthreads();
+    if (first < last && !s_done[warp]) {
+        uint32_t state = s_entry[warp];
+        for (int k = first; k < last; k++) state = follow(k, state);
+    }
+}
+
 template <int TEAMS>
 __global__ void __launch_bounds__(kThreads * TEAMS)
 scan_index_kernel(const ImageDesc *__restrict__ descs, const uint2 *__restrict__ segs, int n_segs, const HuffTable *__restrict__ huff,
@@ -574,7 +864,23 @@ scan_index_kernel(const ImageDesc *__restrict__ descs, const uint2 *__restrict__
         base = (uint32_t)all;
     }
     const int n_own = (int)((m.own_end - m.own_bit + S - 1) / S);
-    const uint32_t info = tid < n_own ? scratch.sub_info[seg * kSegSubs + tid] : 0;
+    uint32_t info = 0;
+    if (d.slots == 0) {
+        if (tid < n_own) info = scratch.sub_info[seg * kSegSubs + tid];
+    } else { // one thread follows the real state from subsequence to subsequence
+        const SlotTables *t = scratch.slots + (d.slots - 1) + j;
+        uint8_t *next = buf, *path = buf + sizeof(t->next); // (the buffer is free until the stream arrives)
+        for (int k = tid; k < (int)(sizeof(t->next) / 16); k += kThreads) reinterpret_cast<uint4 *>(next)[k] = reinterpret_cast<const uint4 *>(t->next)[k];
+        team.sync();
+        if (tid == 0)
+            for (int k = 0, i = (int)m.entry; k < n_own; k++) {
+                path[k] = (uint8_t)i;
+                i = next[k * kSlotStates + i] & (kSlotStates - 1);
+            }
+        team.sync();
+        if (tid < n_own) info = t->info[tid][path[tid]];
+        team.sync();
+    }
     int sums[3] = {0, 0, 0};
     if (base < nblocks) { // (uniform) otherwise the crop needs nothing of this segment
         const uint32_t skip = m.own_bit >> 7; // vectors of the run-up
@@ -827,30 +1133,64 @@ ScanLayout layout_scan(uint32_t scan_len, uint32_t target_bits) {
     return l;
 }
 
-void launch_entropy_decode(const ImageDesc *descs, const uint2 *segs, int n_segs, const int32_t *multi, int n_multi,
-                           const int32_t *restart, int n_restart, const uint8_t *blob, const HuffTable *huff,
-                           const EntropyScratch &scratch, int32_t *status, uint32_t max_raw, int max_tables, bool alike,
-                           uint8_t *index_pool, unsigned long long *index_stats, cudaStream_t stream) {
+ScanLayout layout_scan_slots(uint32_t scan_len) {
+    ScanLayout l{};
+    const uint64_t bits = (uint64_t)scan_len * 8, own = (uint64_t)kSlotSubs * kSlotBits;
+    l.seg_count = (uint32_t)((bits + own - 1) / own);
+    if (l.seg_count < 1) l.seg_count = 1;
+    l.subseq_bits = (uint32_t)((bits + kSlotSubs * l.seg_count - 1) / (kSlotSubs * l.seg_count) + 31) / 32 * 32;
+    if (l.subseq_bits < 256) l.subseq_bits = 256;
+    l.seg_warm = kSlotRunUp;
+    l.seg_raw = kSlotSubs * l.subseq_bits / 8;
+    l.seg_count = scan_len ? (scan_len + l.seg_raw - 1) / l.seg_raw : 1;
+    l.seg_stride = ((kSlotSubs + kSlotRunUp) * l.subseq_bits / 8 + kSegOverlap + 64 + 31) / 16 * 16;
+    return l;
+}
+
+void launch_entropy_decode(const ImageDesc *descs, const EntropyWork &work, const uint8_t *blob, const HuffTable *huff,
+                           const EntropyScratch &scratch, int32_t *status, uint8_t *index_pool, unsigned long long *index_stats,
+                           cudaStream_t stream) {
+    const int n_segs = work.n_guess + work.n_slots;
     if (n_segs > 0) {
-        const uint32_t buf = (uint32_t)stream_bytes(max_raw);
-        auto run = [&](auto sync_kernel, auto index_kernel, int teams) {
-            const size_t smem = tables_bytes(max_tables) + (size_t)teams * buf;
-            cudaFuncSetAttribute(sync_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-            cudaFuncSetAttribute(index_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-            const int grid = (n_segs + teams - 1) / teams;
-            sync_kernel<<<grid, kThreads * teams, smem, stream>>>(descs, segs, n_segs, blob, huff, scratch, index_pool, index_stats, max_tables, buf);
-            if (n_multi > 0) scan_stitch_kernel<<<n_multi, kThreads, 0, stream>>>(descs, multi, huff, scratch);
-            index_kernel<<<grid, kThreads * teams, smem, stream>>>(descs, segs, n_segs, huff, scratch, status, index_pool, index_stats, max_tables, buf);
-        };
+        const uint32_t buf = (uint32_t)stream_bytes(work.max_raw);
+        const int tables = work.max_tables;
+        auto allow = [](auto kernel, size_t smem) { cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); };
         // With enough segments to fill every SM four teams share a set of tables: eight segments of up to
         // 22 KB fit an SM then, instead of five.
-        if (alike && n_segs >= 148 * 5)
-            run(scan_sync_kernel<4>, scan_index_kernel<4>, 4);
-        else
-            run(scan_sync_kernel<1>, scan_index_kernel<1>, 1);
+        const int teams = work.alike && n_segs >= 148 * 5 ? 4 : 1;
+        const size_t smem = tables_bytes(tables) + (size_t)teams * buf;
+        if (work.n_guess > 0) {
+            const int grid = (work.n_guess + teams - 1) / teams;
+            auto run = [&](auto kernel) {
+                allow(kernel, smem);
+                kernel<<<grid, kThreads * teams, smem, stream>>>(descs, work.segs, work.n_guess, blob, huff, scratch, index_pool, index_stats, tables, buf);
+            };
+            if (teams == 4) run(scan_sync_kernel<4>); else run(scan_sync_kernel<1>);
+            if (work.n_multi > 0) scan_stitch_kernel<<<work.n_multi, kThreads, 0, stream>>>(descs, work.multi, huff, scratch);
+        }
+        if (work.n_slots > 0) {
+            const size_t one = tables_bytes(tables) + buf;
+            allow(scan_slots_kernel, one);
+            scan_slots_kernel<<<work.n_slots, kSlotThreads, one, stream>>>(descs, work.segs + work.n_guess, blob, huff, scratch, tables);
+            // As many runs as segments in each: both are followed one after the other.  The maps fit
+            // shared memory up to 1500 segments (6 MB of scan).
+            int warps = 1;
+            if (work.max_slot_segs > 12)
+                while (warps * warps < work.max_slot_segs && warps < kChainThreads / 32) warps++;
+            const int slots = work.max_slot_segs < 1500 ? work.max_slot_segs : 1500;
+            const size_t maps = (size_t)slots * kSlotStates * sizeof(SlotMap);
+            allow(scan_chain_kernel, maps);
+            scan_chain_kernel<<<work.n_slot_images, warps * 32, maps, stream>>>(descs, work.slot_images, huff, scratch, slots);
+        }
+        auto run = [&](auto kernel) {
+            allow(kernel, smem);
+            kernel<<<(n_segs + teams - 1) / teams, kThreads * teams, smem, stream>>>(descs, work.segs, n_segs, huff, scratch, status, index_pool,
+                                                                                  index_stats, tables, buf);
+        };
+        if (teams == 4) run(scan_index_kernel<4>); else run(scan_index_kernel<1>);
     }
-    if (n_restart > 0)
-        scan_restart_kernel<<<n_restart, kRestartThreads, 0, stream>>>(descs, restart, blob, huff, scratch, status);
+    if (work.n_restart > 0)
+        scan_restart_kernel<<<work.n_restart, kRestartThreads, 0, stream>>>(descs, work.restart, blob, huff, scratch, status);
 }
 
 } // namespace ffcvb

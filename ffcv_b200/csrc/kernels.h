@@ -20,23 +20,35 @@ struct EntropyScratch {
     uint8_t *clean;      // unstuffed streams (ImageDesc::clean_off), 512 spare bytes behind them
     SegMeta *meta;       // per segment
     uint32_t *sub_info;  // per segment kSegSubs words: state at the start of a subsequence, blocks << 16
+    SlotTables *slots;   // per segment of the samples with ImageDesc::slots
     int32_t *seg_dc;     // per segment four words: DC value of each component before the segment
     uint32_t *done;      // per sample
     uint32_t *pos;       // per block: bit position of its first AC symbol from its image's clean_off
     int16_t *dc;         // per block: DC value, relative to seg_dc of its segment
 };
 
-// Entropy decode: finds every block of the listed scans.  `segs` (device): one entry (sample, segment)
-// per segment of the samples without restart markers; `multi`: the samples with more than one
-// segment; `restart`: the samples with restart markers.  `max_raw` bounds a segment's raw bytes
-// with run-up and overlap, `max_tables` the tables of a sample in shared memory (its distinct DC tables
-// and twice its AC tables).  `alike`: all the samples in segs have the same tables and layout of an MCU.
-// status[sample] is set for every listed sample.  index_pool / index_stats: the decode index (see DecodeIndexHeader)
-// and two counters (images decoded from their entry, entries written); both may be nullptr.
-void launch_entropy_decode(const ImageDesc *descs, const uint2 *segs, int n_segs, const int32_t *multi, int n_multi,
-                           const int32_t *restart, int n_restart, const uint8_t *blob, const HuffTable *huff,
-                           const EntropyScratch &scratch, int32_t *status, uint32_t max_raw, int max_tables, bool alike,
-                           uint8_t *index_pool, unsigned long long *index_stats, cudaStream_t stream);
+// What an entropy decode works on (device lists).
+struct EntropyWork {
+    const uint2 *segs;     // (sample, segment) of every segment of the samples without restart markers:
+    int n_guess, n_slots;  // first the n_guess of samples decoded from one guess per subsequence, then those with ImageDesc::slots
+    const int32_t *multi;  // samples of the first kind with more than one segment
+    int n_multi;
+    const int32_t *slot_images; // samples of the second kind
+    int n_slot_images;
+    const int32_t *restart; // samples with restart markers
+    int n_restart;
+    uint32_t max_raw;      // bounds a segment's raw bytes with run-up and overlap
+    int max_tables;        // bounds the tables of a sample in shared memory (its distinct DC tables and twice its AC tables)
+    int max_slot_segs;     // most segments of one of slot_images
+    bool alike;            // all samples in segs have the same tables and layout of an MCU
+};
+
+// Entropy decode: finds every block of the listed scans.  status[sample] is set for every listed
+// sample.  index_pool / index_stats: the decode index (see DecodeIndexHeader) and two counters (images
+// decoded from their entry, entries written); both may be nullptr.
+void launch_entropy_decode(const ImageDesc *descs, const EntropyWork &work, const uint8_t *blob, const HuffTable *huff,
+                           const EntropyScratch &scratch, int32_t *status, uint8_t *index_pool, unsigned long long *index_stats,
+                           cudaStream_t stream);
 
 // How a scan of scan_len bytes is cut into subsequences and segments.  `target_bits`: wished length of
 // a subsequence, see subseq_target.
@@ -44,6 +56,12 @@ struct ScanLayout {
     uint32_t subseq_bits, seg_raw, seg_warm, seg_stride, seg_count;
 };
 ScanLayout layout_scan(uint32_t scan_len, uint32_t target_bits);
+// The same for a scan decoded from every slot at once, which is done while a batch's scans leave most of
+// the GPU idle otherwise: three times the work, but a chain of 4 x 512 bits instead of 6 to 10 kbit.  Measured on
+// batches of 224x256 to 400x500 photographs: 193 -> 137 us at 1 image, 399 -> 355 at 15 Mbit, 771 -> 754 at
+// 45 Mbit, even at 60.
+ScanLayout layout_scan_slots(uint32_t scan_len);
+constexpr uint64_t kSlotModeBits = 40u << 20; // of a batch, at most
 // Subsequence length for a batch with `total_bits` of scans: long ones re-synchronise fewer times,
 // short ones spread few scans over the GPU.
 uint32_t subseq_target(uint64_t total_bits);

@@ -189,9 +189,15 @@ extern "C" int ffcvb_imdecode_static(const uint8_t *jpeg_host, uint64_t jpeg_siz
     es.done = reinterpret_cast<uint32_t *>(&meta_dev->status[1]);
     es.pos = reinterpret_cast<uint32_t *>(scratch + kIndexOff);
     es.dc = reinterpret_cast<int16_t *>(es.pos + kMaxBlocks);
-    launch_entropy_decode(desc_dev, meta_dev->segs, n_segs, list_dev, n_segs > 1 ? 1 : 0, list_dev, d.restart_interval ? 1 : 0,
-                          jpeg_dev, meta_dev->huff, es, meta_dev->status, kSegSubs * d.subseq_bits / 8 + kSegOverlap, 3 * d.n_dc_tab, false,
-                          nullptr, nullptr, st);
+    EntropyWork work{};
+    work.segs = meta_dev->segs;
+    work.n_guess = n_segs;
+    work.multi = work.restart = list_dev;
+    work.n_multi = n_segs > 1 ? 1 : 0;
+    work.n_restart = d.restart_interval ? 1 : 0;
+    work.max_raw = kSegSubs * d.subseq_bits / 8 + kSegOverlap;
+    work.max_tables = 3 * d.n_dc_tab;
+    launch_entropy_decode(desc_dev, work, jpeg_dev, meta_dev->huff, es, meta_dev->status, nullptr, nullptr, st);
     launch_blocks(desc_dev, meta_dev->tiles, (int)n_tiles, meta_dev->huff, meta_dev->mult, es, scratch + kPlaneOff, st);
     const bool quad = d.ncomp == 3 && d.hs == 2 && d.vs == 2 && (width + 1) / 2 >= 3;
     const bool full = d.ncomp == 3 && d.hs == 1 && d.vs == 1;

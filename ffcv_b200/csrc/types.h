@@ -16,6 +16,21 @@ constexpr int kPayloadAlign = 16;
 constexpr int kSegSubs = 128;
 constexpr int kSegOverlap = 512;
 constexpr int kMaxSubseqBits = 1280; // longest subsequence: bounds a segment's shared memory
+// Few scans are decoded from every possible block slot at once (scan_slots_kernel): segments of up to
+// kSlotSubs subsequences of kSlotBits bits, each with up to kSlotStates entry states; the last place is kept
+// for a state that was not found in time.
+constexpr int kSlotSubs = 64, kSlotBits = 512, kSlotStates = 16, kSlotRounds = 4;
+constexpr uint32_t kSlotMiss = 255;
+
+struct alignas(8) SlotMap {
+    uint32_t from, to; // state before (kNoState: none), state behind | blocks << 16
+};
+struct SlotTables {                         // of one segment
+    uint32_t info[kSlotSubs][kSlotStates];  // entry state of a subsequence | blocks completed in it << 16
+    uint8_t next[kSlotSubs][kSlotStates];   // which state of the next subsequence it leads to
+    SlotMap map[kSlotStates];               // per state of the first subsequence
+};
+constexpr uint32_t kNoState = 0xFFFFFFFFu;
 
 // Per-sample work descriptor.
 struct ImageDesc {
@@ -57,6 +72,7 @@ struct ImageDesc {
     // segment but the first; bytes of a segment's place in the unstuffed stream; and which of the
     // batch's segments are this image's.
     uint32_t subseq_bits, seg_raw, seg_warm, seg_stride, seg_first, seg_count;
+    uint32_t slots;        // decoded from every slot at once: 1 + the first of the image's SlotTables (0: not)
     uint32_t index_cap;    // place in the decode index (0: none), see DecodeIndexHeader
     uint64_t index_off;    // byte offset of the entry in the context's index pool
     // The crop box decides how much of the image is needed: the entropy decoder stops after
@@ -143,6 +159,7 @@ struct SegMeta {
     uint32_t bytes;            // unstuffed bytes, overlap included
     uint32_t exit;             // decoder state behind own_end (as in sub_info)
     uint32_t blocks;           // blocks completed in the segment
+    uint32_t entry;            // SlotTables: which state of the first subsequence is the real one
 };
 
 constexpr uint32_t kNoBlock = 0xFFFFFFFFu; // position of a block that the scan does not hold

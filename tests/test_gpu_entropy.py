@@ -124,3 +124,29 @@ def test_tables_whose_long_codes_come_early(blocks, long_length):
     want = O.jpeg_decode(buf)
     assert np.abs(want.astype(int) - cv2.imdecode(buf, cv2.IMREAD_COLOR)).mean() < 6  # (cv2's accurate inverse transform)
     assert np.array_equal(_decode(buf, h, w), want)
+
+
+@pytest.mark.parametrize('quality', [75, 98])
+@pytest.mark.parametrize('h,w', [(33, 47), (256, 250), (531, 707), (1300, 1100)], ids=lambda v: str(v))
+@pytest.mark.parametrize('subseq_bits', ['', '512'], ids=['from_every_slot', 'from_one_guess'])
+def test_few_large_scans(h, w, quality, subseq_bits, monkeypatch):
+    """Batches of few scans: one, several and (for the run that follows the real state) very many segments,
+    photographs and pure noise, whose blocks are longer than a subsequence."""
+    from ffcv_b200 import libffcv as L
+    monkeypatch.setenv('FFCV_B200_SUBSEQ_BITS', subseq_bits)
+    rng = np.random.default_rng(h + quality)
+    bufs = [_jpeg(rng, h, w, quality), cv2.imencode('.jpg', rng.integers(0, 256, (h, w, 3), np.uint8), [cv2.IMWRITE_JPEG_QUALITY, quality])[1].reshape(-1)]
+    n = len(bufs)
+    sizes = np.array([b.size for b in bufs], np.uint64)
+    ctx = L.Context(0, 1, 2)
+    out = ch.zeros((n, h, w, 3), dtype=ch.uint8, device='cuda')
+    stream = ch.cuda.current_stream().cuda_stream
+    ctx.stage(0, np.concatenate(bufs), np.concatenate([[0], np.cumsum(sizes)[:-1]]).astype(np.uint64), sizes, np.zeros(n, np.uint8),
+              np.full(n, h, np.uint16), np.full(n, w, np.uint16), L.make_plan(h, w, 0, L.OUT_U8_NHWC),
+              np.tile(np.array([0, 0, h, w], np.int32), (n, 1)))
+    ctx.submit(0, stream, out.data_ptr())
+    assert (ctx.status(0, stream, n) == 0).all()
+    got = out.cpu().numpy()
+    for k, b in enumerate(bufs):
+        assert np.array_equal(got[k], O.jpeg_decode(b)), k
+    ctx.close()
