@@ -450,6 +450,18 @@ bool valid_plan(const ffcvb_plan *p) {
     return true;
 }
 
+// The box of a sample decoded at reduced scale that covers its crop box.
+void scaled_box(const ImageDesc &d, int32_t *p) {
+    const int sh = d.scale_shift, r0 = p[0] >> sh, c0 = p[1] >> sh;
+    int r1 = (p[0] + p[2] + (1 << sh) - 1) >> sh, c1 = (p[1] + p[3] + (1 << sh) - 1) >> sh;
+    if (r1 > (int)d.dec_height) r1 = d.dec_height;
+    if (c1 > (int)d.dec_width) c1 = d.dec_width;
+    p[0] = r0;
+    p[1] = c0;
+    p[2] = r1 - r0;
+    p[3] = c1 - c0;
+}
+
 OpList make_oplist(const ffcvb_plan &p) {
     OpList o{};
     o.n_ops = p.n_ops;
@@ -717,7 +729,7 @@ int stage_impl(ffcvb_ctx *ctx, int slot, const Source &source, const uint64_t *p
         // room behind the payloads for what is laid out after the parse: at most 255 tables of each kind
         size_t tail = 255 * (sizeof(HuffTable) + sizeof(MultTable)) + 4 * (sizeof(int32_t) * (size_t)n + 16) + 256;
         for (int i = 0; i < n; i++) { // and the tables of CTAs: at most those of whole images and of the shortest segments
-            tail += sizeof(uint2) * (size_t)((((heights[i] + 1) / 2 + 7) / 8) * ((((widths[i] + 1) / 2 + 1) / 2 + 1 + 31) / 32));
+            tail += sizeof(uint2) * (size_t)quad_tiles_x(widths[i]) * quad_tiles_y(heights[i]);
             tail += sizeof(uint2) * ((size_t)((heights[i] + 15) / 8) * ((widths[i] + 15) / 8) * 3 / kBlockTile + 4);
             tail += sizeof(uint2) * (size_t)(sizes[i] / (64 * kSegSubs / 8) + 2);
         }
@@ -977,6 +989,8 @@ int stage_impl(ffcvb_ctx *ctx, int slot, const Source &source, const uint64_t *p
     if (ctx->tune_subseq_bits) target_bits = (uint32_t)ctx->tune_subseq_bits;
     ctx->stage_seq++;
     int max_w = 0, max_h = 0, n_quad = 0, n_444 = 0, n_other = 0;
+    const bool can_fuse = plan->resize && !s.packed;
+    const ResizeShape shape = can_fuse ? resize_shape(plan->out_h, plan->out_w, plan->out_kind) : ResizeShape{};
     for (int i = 0; i < n; i++) {
         ImageDesc &d = descs[i];
         if (d.mode != FFCVB_MODE_JPG) continue;
@@ -1083,8 +1097,23 @@ int stage_impl(ffcvb_ctx *ctx, int slot, const Source &source, const uint64_t *p
             const size_t ph = (size_t)d.mcus_y * (c == 0 ? d.vs * d.bs_luma : d.bs_chroma);
             plane_bytes += align_up(pw * ph, 16);
         }
+        if (can_fuse && d.host_status == 0) {
+            // The resize kernel converts the planes of a 4:2:0 or equal-resolution image itself, into its window
+            // of source pixels, if the regime is one that works from a window and enough rows fit.
+            int32_t box[4];
+            memcpy(box, params + (size_t)i * n_params, sizeof(box));
+            const bool quad = d.ncomp == 3 && d.scale_shift == 0 && d.hs == 2 && d.vs == 2 && (d.width + 1) / 2 >= 3;
+            const bool plain = d.ncomp == 3 && (d.scale_shift != 0 || (d.hs == 1 && d.vs == 1));
+            if ((quad || plain) && box[0] >= 0 && box[1] >= 0 && box[2] > 0 && box[3] > 0 && box[0] + box[2] <= (int)d.height &&
+                box[1] + box[3] <= (int)d.width) {
+                scaled_box(d, box);
+                const Scaling sc = scaling_of(box[2], box[3], plan->out_h, plan->out_w);
+                if (sc.regime == kArea || sc.regime == kLinear) d.fuse_rows = (uint16_t)window_band(box[3], sc.sc_y, shape.band, shape.win);
+            }
+        }
         d.rgb_off = rgb_bytes;
         d.rgb_pitch = s.packed ? (uint32_t)d.dec_width * 3 : (uint32_t)align_up((size_t)d.dec_width * 3, 16);
+        if (d.fuse_rows) continue;
         rgb_bytes += (size_t)d.dec_height * d.rgb_pitch;
         int bw = d.dec_width, bh = d.dec_height;
         {   // extent the colour kernels' grids must cover: the crop box (plus the odd edge of a
@@ -1107,7 +1136,7 @@ int stage_impl(ffcvb_ctx *ctx, int slot, const Source &source, const uint64_t *p
         else if (d.ncomp == 3 && d.hs == 2 && d.vs == 2 && (d.width + 1) / 2 >= 3) {
             n_quad++;
             // the tiles of 64 x 8 chroma samples (one CTA each) that cover this image's box
-            const uint32_t tiles_x = (uint32_t)((((bw + 1) / 2 + 1) / 2 + 1 + 31) / 32), tiles_y = (uint32_t)(((bh + 1) / 2 + 7) / 8);
+            const uint32_t tiles_x = quad_tiles_x(bw), tiles_y = quad_tiles_y(bh);
             for (uint32_t ty = 0; ty < tiles_y; ty++)
                 for (uint32_t tx = 0; tx < tiles_x; tx++) quad_tiles.push_back(make_uint2((uint32_t)i, tx | ty << 16));
         } else if (d.ncomp == 3 && d.hs == 1 && d.vs == 1)
@@ -1250,17 +1279,8 @@ int stage_impl(ffcvb_ctx *ctx, int slot, const Source &source, const uint64_t *p
     for (int i = 0; i < n; i++) {
         // a sample decoded at reduced scale: its crop box, for the kernels, is the box of the scaled
         // image that covers it
-        const int sh = descs[i].scale_shift;
-        if (sh == 0 || !plan->resize) continue;
-        int32_t *p = reinterpret_cast<int32_t *>(s.host + hd.params_off) + (size_t)i * n_params;
-        const int r0 = p[0] >> sh, c0 = p[1] >> sh;
-        int r1 = (p[0] + p[2] + (1 << sh) - 1) >> sh, c1 = (p[1] + p[3] + (1 << sh) - 1) >> sh;
-        if (r1 > (int)descs[i].dec_height) r1 = descs[i].dec_height;
-        if (c1 > (int)descs[i].dec_width) c1 = descs[i].dec_width;
-        p[0] = r0;
-        p[1] = c0;
-        p[2] = r1 - r0;
-        p[3] = c1 - c0;
+        if (descs[i].scale_shift == 0 || !plan->resize) continue;
+        scaled_box(descs[i], reinterpret_cast<int32_t *>(s.host + hd.params_off) + (size_t)i * n_params);
     }
     for (const auto &r : s.riders) {
         if (!r.inline_bytes.empty()) {
@@ -1545,6 +1565,7 @@ static int run_batch(ffcvb_ctx *ctx, Slot &s, cudaStream_t st, void *out_dev, bo
         src.descs = descs;
         src.blob = blob;
         src.rgb = rgb;
+        src.planes = (const uint8_t *)s.planes.p;
         launch_resize_augment(src, s.n, params, (int)hd.n_params, make_oplist(s.plan), s.plan.resize,
                               s.plan.out_h, s.plan.out_w, s.plan.out_kind, s.plan.lut_dev, out_dev, status, small, st);
     }

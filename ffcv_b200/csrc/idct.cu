@@ -7,6 +7,7 @@
 // triangle ("fancy") chroma upsampler, and the 16.16 fixed-point YCbCr->RGB transform.  These are
 // integer butterflies in registers; they are not a dense contraction and must not be reordered,
 // so no tensor cores.
+#include "color.h"
 #include "huffman.h"
 #include "kernels.h"
 
@@ -273,26 +274,18 @@ __device__ __forceinline__ int chroma_sample(const uint8_t *__restrict__ p, int 
     return (cur * 3 + 3 * row[cx + 1] + far[cx + 1] + 7) >> 4;
 }
 
-// 16.16 fixed-point YCbCr -> RGB of libjpeg (jdcolor.c's tables written out), one pixel.
-__device__ __forceinline__ uint32_t ycc_to_rgb(int lum, int cb, int cr) {
-    cb -= 128;
-    cr -= 128;
-    const int r = lum + ((91881 * cr + 32768) >> 16);
-    const int g = lum + ((-22554 * cb - 46802 * cr + 32768) >> 16);
-    const int b = lum + ((116130 * cb + 32768) >> 16);
-    return (uint32_t)min(255, max(0, r)) | (uint32_t)min(255, max(0, g)) << 8 | (uint32_t)min(255, max(0, b)) << 16;
-}
-
 // Stores four RGB pixels (12 bytes, the fourth byte of each word of `px` unused) at `o`: three
 // words when the address allows and all four pixels exist, else the first `count` pixels by bytes.
 __device__ __forceinline__ void store_rgb4(uint8_t *o, const uint32_t *px, int count, bool words) {
     if (words && count == 4) {
         uint32_t *w = reinterpret_cast<uint32_t *>(o);
-        w[0] = px[0] | px[1] << 24;
-        w[1] = px[1] >> 8 | px[2] << 16;
-        w[2] = px[2] >> 16 | px[3] << 8;
+        w[0] = pick(px[0], px[1], 0x4210);
+        w[1] = pick(px[1], px[2], 0x5421);
+        w[2] = pick(px[2], px[3], 0x6542);
     } else {
-        for (int k = 0; k < count; k++) {
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            if (k >= count) break;
             o[3 * k] = (uint8_t)px[k];
             o[3 * k + 1] = (uint8_t)(px[k] >> 8);
             o[3 * k + 2] = (uint8_t)(px[k] >> 16);
@@ -315,13 +308,10 @@ __device__ __forceinline__ void convert_box(const int32_t *params, int n_params,
     }
 }
 
-// 4:2:0 images: one thread per pair of chroma samples = 4 x 2 output pixels.  The triangle filter
-// of the eight pixels reads a 3 x 4 chroma neighbourhood (image edges replicate, which is what the
-// filter's edge formulas amount to): its vertical blends are computed once per column, the luma
-// samples arrive as one word per row and the pixels leave as three words per row (the rows of the
-// RGB scratch start on 16-byte boundaries and a thread's first pixel is a multiple of four).
-// Only the chroma cells the crop box touches are converted.
-__global__ void __launch_bounds__(256)
+// 4:2:0 images: one thread per four chroma samples of a row = 8 x 2 output pixels (quad_pixels); they leave as
+// three words per four pixels (the rows of the RGB scratch start on 16-byte boundaries and a thread's
+// first pixel is a multiple of eight).  Only the chroma cells the crop box touches are converted.
+__global__ void __launch_bounds__(128)
 color_quad_kernel(const ImageDesc *__restrict__ descs, const int32_t *__restrict__ list,
                   const uint2 *__restrict__ tiles, const uint8_t *__restrict__ planes, uint8_t *__restrict__ rgb,
                   const int32_t *__restrict__ params, int n_params) {
@@ -339,65 +329,27 @@ color_quad_kernel(const ImageDesc *__restrict__ descs, const int32_t *__restrict
         tile_y = blockIdx.y;
     }
     const ImageDesc &d = descs[img];
-    if (d.host_status != 0 || d.ncomp != 3 || d.hs != 2 || d.vs != 2 || d.scale_shift != 0) return;
+    if (d.host_status != 0 || d.ncomp != 3 || d.hs != 2 || d.vs != 2 || d.scale_shift != 0 || d.fuse_rows) return;
     const int W = d.width, H = d.height;
-    const int real_w = (W + 1) >> 1, real_h = (H + 1) >> 1;
-    if (real_w < 3) return; // too narrow for the filter: the per-pixel kernel replicates
+    const QuadPlanes p{planes + d.plane_off[0], planes + d.plane_off[1], planes + d.plane_off[2], d.mcus_x * 16, d.mcus_x * 8, (W + 1) >> 1, (H + 1) >> 1};
+    if (p.real_w < 3) return; // too narrow for the filter: the per-pixel kernel replicates
     int x0, y0, x1, y1;
     convert_box(params, n_params, img, W, H, x0, y0, x1, y1);
-    const int cx = ((x0 >> 1) & ~1) + 2 * (tile_x * 32 + threadIdx.x); // even: pixel 2 * cx is a multiple of 4
+    const int cx = ((x0 >> 1) & ~3) + 4 * (tile_x * 16 + threadIdx.x);
     const int cy = (y0 >> 1) + tile_y * 8 + threadIdx.y;
     if (cx > ((x1 - 1) >> 1) || cy > ((y1 - 1) >> 1)) return;
-    const int yw = d.mcus_x * 16, cw = d.mcus_x * 8;
-    const int xl = max(cx - 1, 0), xr = min(cx + 2, real_w - 1);
-    const bool second = cx + 1 <= real_w - 1; // the pair's second column exists
-    const int yu = max(cy - 1, 0), yd = min(cy + 1, real_h - 1);
-    // chroma of the 4 x 2 pixels: [Cb, Cr][row][pixel]
-    int cval[2][2][4];
-#pragma unroll
-    for (int k = 0; k < 2; k++) {
-        const uint8_t *P = planes + d.plane_off[1 + k];
-        const uint8_t *ru = P + (size_t)yu * cw, *rc = P + (size_t)cy * cw, *rd = P + (size_t)yd * cw;
-        int up[4], dn[4]; // columns cx - 1 .. cx + 2 blended towards the row above / below
-        {
-            const int c = rc[xl];
-            up[0] = 3 * c + ru[xl];
-            dn[0] = 3 * c + rd[xl];
-        }
-        {
-            const uint32_t u = *reinterpret_cast<const uint16_t *>(ru + cx), c = *reinterpret_cast<const uint16_t *>(rc + cx),
-                           w = *reinterpret_cast<const uint16_t *>(rd + cx);
-            up[1] = 3 * (int)(c & 255) + (int)(u & 255);
-            dn[1] = 3 * (int)(c & 255) + (int)(w & 255);
-            up[2] = second ? 3 * (int)(c >> 8) + (int)(u >> 8) : up[1];
-            dn[2] = second ? 3 * (int)(c >> 8) + (int)(w >> 8) : dn[1];
-        }
-        {
-            const int c = rc[xr];
-            up[3] = second ? 3 * c + ru[xr] : up[1];
-            dn[3] = second ? 3 * c + rd[xr] : dn[1];
-        }
-#pragma unroll
-        for (int j = 0; j < 2; j++) { // the pair's columns
-            cval[k][0][2 * j] = (3 * up[1 + j] + up[j] + 8) >> 4;
-            cval[k][0][2 * j + 1] = (3 * up[1 + j] + up[2 + j] + 7) >> 4;
-            cval[k][1][2 * j] = (3 * dn[1 + j] + dn[j] + 8) >> 4;
-            cval[k][1][2 * j + 1] = (3 * dn[1 + j] + dn[2 + j] + 7) >> 4;
-        }
-    }
-    const uint8_t *Y = planes + d.plane_off[0];
+    uint32_t px[2][8];
+    quad_pixels(p, cx, cy, px);
     uint8_t *out = rgb + d.rgb_off;
-    const int x = 2 * cx, count = min(4, W - x);
+    const int x = 2 * cx;
     const bool words = ((reinterpret_cast<uintptr_t>(out) | d.rgb_pitch) & 3) == 0;
 #pragma unroll
     for (int r = 0; r < 2; r++) {
         const int y = 2 * cy + r;
         if (y >= H) continue;
-        const uint32_t lum = *reinterpret_cast<const uint32_t *>(Y + (size_t)y * yw + x);
-        uint32_t px[4];
-#pragma unroll
-        for (int q = 0; q < 4; q++) px[q] = ycc_to_rgb((lum >> (8 * q)) & 255, cval[0][r][q], cval[1][r][q]);
-        store_rgb4(out + (size_t)y * d.rgb_pitch + (size_t)x * 3, px, count, words);
+        uint8_t *o = out + (size_t)y * d.rgb_pitch + (size_t)x * 3;
+        store_rgb4(o, px[r], min(4, W - x), words);
+        store_rgb4(o + 12, px[r] + 4, min(4, W - x - 4), words);
     }
 }
 
@@ -411,7 +363,7 @@ color_444_kernel(const ImageDesc *__restrict__ descs, const int32_t *__restrict_
                  const int32_t *__restrict__ params, int n_params) {
     const int img = list[blockIdx.z];
     const ImageDesc &d = descs[img];
-    if (d.host_status != 0 || d.ncomp != 3 || !(d.scale_shift != 0 || (d.hs == 1 && d.vs == 1))) return;
+    if (d.host_status != 0 || d.ncomp != 3 || !(d.scale_shift != 0 || (d.hs == 1 && d.vs == 1)) || d.fuse_rows) return;
     const int W = d.dec_width, H = d.dec_height;
     int x0, y0, x1, y1;
     convert_box(params, n_params, img, W, H, x0, y0, x1, y1);
@@ -425,23 +377,8 @@ color_444_kernel(const ImageDesc *__restrict__ descs, const int32_t *__restrict_
     const bool words_in = ((pw | (int)(d.plane_off[0] | d.plane_off[1] | d.plane_off[2])) & 3) == 0;
     const bool words_out = ((reinterpret_cast<uintptr_t>(out) | d.rgb_pitch) & 3) == 0;
     for (int y = y0 + blockIdx.y * 8 + threadIdx.y; y < y1; y += gridDim.y * 8) {
-        const size_t s = (size_t)y * pw + x;
-        uint32_t lum = 0, cb = 0, cr = 0;
-        if (words_in) {
-            lum = *reinterpret_cast<const uint32_t *>(Y + s);
-            cb = *reinterpret_cast<const uint32_t *>(Cb + s);
-            cr = *reinterpret_cast<const uint32_t *>(Cr + s);
-        } else {
-            for (int q = 0; q < count; q++) {
-                lum |= (uint32_t)Y[s + q] << (8 * q);
-                cb |= (uint32_t)Cb[s + q] << (8 * q);
-                cr |= (uint32_t)Cr[s + q] << (8 * q);
-            }
-        }
         uint32_t px[4];
-#pragma unroll
-        for (int q = 0; q < 4; q++)
-            px[q] = ycc_to_rgb((lum >> (8 * q)) & 255, (cb >> (8 * q)) & 255, (cr >> (8 * q)) & 255);
+        plain_pixels(Y, Cb, Cr, (size_t)y * pw + x, count, words_in, px);
         store_rgb4(out + (size_t)y * d.rgb_pitch + (size_t)x * 3, px, count, words_out);
     }
 }
@@ -494,11 +431,10 @@ void launch_color(const ImageDesc *descs, const int32_t *list, int n_list, int n
     }
     if (n_quad > 0 && quad_tiles != nullptr) {
         if (n_quad_tiles > 0)
-            color_quad_kernel<<<n_quad_tiles, dim3(32, 8), 0, stream>>>(descs, list, quad_tiles, planes, rgb, crop_params,
+            color_quad_kernel<<<n_quad_tiles, dim3(16, 8), 0, stream>>>(descs, list, quad_tiles, planes, rgb, crop_params,
                                                                         n_params);
     } else if (n_quad > 0) {
-        dim3 grid((((max_w + 1) / 2 + 1) / 2 + 1 + 31) / 32, ((max_h + 1) / 2 + 7) / 8, n_list); // pairs of chroma columns
-        color_quad_kernel<<<grid, dim3(32, 8), 0, stream>>>(descs, list, nullptr, planes, rgb, crop_params, n_params);
+        color_quad_kernel<<<dim3(quad_tiles_x(max_w), quad_tiles_y(max_h), n_list), dim3(16, 8), 0, stream>>>(descs, list, nullptr, planes, rgb, crop_params, n_params);
     }
     if (n_other > 0) {
         int bx = (max_w * max_h + 256 * 4 - 1) / (256 * 4);

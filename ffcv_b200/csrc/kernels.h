@@ -1,5 +1,7 @@
 // Launch wrappers of the CUDA kernels (sm_100a).  All pointers are device pointers unless noted.
 #pragma once
+#include <float.h>
+#include <math.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -80,7 +82,7 @@ void launch_blocks(const ImageDesc *descs, const uint2 *tiles, int n_tiles, cons
 
 // Chroma upsampling (triangle filter) + YCbCr->RGB into h*w*3 images in `rgb` (rows rgb_pitch
 // apart).  4:2:0 images (n_quad of them) go through the quad kernel and 4:4:4 images (n_444)
-// through a 2-D kernel, both converting only the crop box given by `crop_params` (row, col, h, w
+// through a 2-D kernel (neither counts those with ImageDesc::fuse_rows), both converting only the crop box given by `crop_params` (row, col, h, w
 // per sample; nullptr = whole image); the other n_other images go through the generic kernel.
 // max_w / max_h bound the boxes in the list.  quad_tiles (device; may be nullptr): one entry
 // (sample, tile x | tile y << 16) per tile of 64 x 8 chroma samples the quad kernel has to
@@ -89,11 +91,60 @@ void launch_color(const ImageDesc *descs, const int32_t *list, int n_list, int n
                   int max_w, int max_h, const uint2 *quad_tiles, int n_quad_tiles, const uint8_t *planes,
                   uint8_t *rgb, const int32_t *crop_params, int n_params, cudaStream_t stream);
 
+// Tiles of 64 x 8 chroma samples that cover a box of bw x bh pixels wherever it begins (a thread converts four
+// samples of a row, beginning at a multiple of four).
+inline uint32_t quad_tiles_x(int bw) { return (uint32_t)(((bw + 1) / 2 + 6) / 4 + 15) / 16; }
+inline uint32_t quad_tiles_y(int bh) { return (uint32_t)((bh + 1) / 2 + 7) / 8; }
+
+// Scaling regime of a crop of ch x cw pixels resized to out_h x out_w, as OpenCV decides it.
+enum { kCopy = 0, kInteger = 1, kArea = 2, kLinear = 3 };
+struct Scaling {
+    int regime, isx, isy;
+    double inv_x, inv_y, sc_x, sc_y;
+};
+FFCVB_HD inline Scaling scaling_of(int ch, int cw, int out_h, int out_w) {
+    Scaling s{kCopy, 1, 1, 1, 1, 1, 1};
+    if (ch != out_h || cw != out_w) {
+        s.inv_x = (double)out_w / cw;
+        s.inv_y = (double)out_h / ch;
+        s.sc_x = 1.0 / s.inv_x;
+        s.sc_y = 1.0 / s.inv_y;
+        if (s.sc_x >= 1 && s.sc_y >= 1) {
+            s.isx = (int)rint(s.sc_x);
+            s.isy = (int)rint(s.sc_y);
+            s.regime = (fabs(s.sc_x - s.isx) < DBL_EPSILON && fabs(s.sc_y - s.isy) < DBL_EPSILON) ? kInteger : kArea;
+        } else {
+            s.regime = kLinear;
+        }
+    }
+    return s;
+}
+
+// How the resize kernel works on an output: rows per band, runs of rows per column, bytes of the window of
+// source pixels, and of shared memory.
+struct ResizeShape {
+    int band, groups;
+    size_t win, smem;
+};
+ResizeShape resize_shape(int out_h, int out_w, int out_kind);
+// Pixels (words) of a row of the window, and the output rows whose source rows fit in it: `band` of them or
+// fewer, 0 when so few fit that windows do not pay.  (b output rows span at most b * sc_y + 3 source rows.)
+FFCVB_HD inline int window_pitch(int cw) { return (cw + 14) & ~7; }
+FFCVB_HD inline int window_band(int cw, double sc_y, int band, size_t win) {
+    const int cap = (int)(win / (4 * (size_t)window_pitch(cw)));
+    if (cap < 4) return 0;
+    const double fit = (cap - 3) / sc_y;
+    if (fit >= band) return band;
+    const int b = (int)fit & ~1; // (even: most bands then begin on 16 bytes)
+    return b >= 4 ? b : 0;
+}
+
 // Source of the fused kernel.
 struct ResizeSource {
     const ImageDesc *descs; // per-sample descriptors, or nullptr for a uniform device batch
     const uint8_t *blob;    // raw payloads live here (descs != nullptr)
     const uint8_t *rgb;     // decoded JPEG samples live here (descs != nullptr)
+    const uint8_t *planes;  // ... or here, those with ImageDesc::fuse_rows
     const uint8_t *uniform; // [n, h, w, 3] uint8 (descs == nullptr)
     int uniform_h, uniform_w;
 };

@@ -6,32 +6,29 @@
 //   RandomTranslate                       ffcv/transforms/translate.py:35-44
 //   Cutout                                ffcv/transforms/cutout.py:36-46
 //   NormalizeImage (256x3 table gather)   ffcv/transforms/normalize.py:58-109
-// Every output pixel is traced backwards through the augmentations to either a fill colour or a
+// Every output pixel traces backwards through the augmentations to either a fill colour or a
 // pixel of the resized crop, whose value is computed with OpenCV's INTER_AREA arithmetic:
 //   equal size -> copy; integer factors -> box sum ((s+2)>>2 for 2x2, else
 //   round-half-even(float(s) * float(1/area))); both factors >= 1 -> separable fractional
 //   coverage accumulated in fp32 in source order (no FMA contraction); any factor < 1 -> 2-tap
 //   interpolation on both axes with 11-bit fixed-point weights.
-// Byte work bound by instruction issue: a few CTAs per sample, each producing every k-th band of
-// output rows; tap positions and weights are computed once per CTA into shared memory and serve all
-// its bands; the source rows a band reads are staged in shared memory by asynchronous 16-byte
-// copies when they fit (taps straight from global memory otherwise); every band's normalised tile
-// is assembled in shared memory and leaves with coalesced 16-byte stores.  In the fractional
-// shrinking and the enlarging regime a thread owns an output column for a run of rows, so that
-// what a source row contributes (its horizontal sums, its interpolated values) is shared by the
-// output rows that touch it.
-#include <float.h>
-
-#include <type_traits>
-
+// Byte work bound by instruction issue: a few CTAs per sample, each producing every k-th band of output rows;
+// tap positions and weights are computed once per CTA into shared memory and serve all its bands.  The
+// source pixels a band reads are gathered in a window in shared memory first, one word per pixel, so
+// that a tap is one load for three channels.  For JPEG samples the window is filled from the decoded
+// planes: chroma upsampling and colour conversion happen there and no RGB image travels through global
+// memory (taps come from global memory byte by byte when too few rows fit).  Every band's normalised tile is
+// assembled in shared memory and leaves with coalesced 16-byte stores.  In the fractional shrinking and the
+// enlarging regime a thread owns an output column for a run of rows, so that what a source row contributes
+// (its horizontal sums, its interpolated values) is shared by the output rows that touch it; what a
+// translation or a cutout fills is painted over the band afterwards.
+#include "color.h"
 #include "kernels.h"
 
 namespace ffcvb {
 
 enum { kOpFlip = 1, kOpTranslate = 2, kOpCutout = 3 };
 enum { kOutU8 = 0, kOutF16Nhwc = 1, kOutF16Nchw = 2, kOutF32Nhwc = 3, kOutF32Nchw = 4 };
-enum { kCopy = 0, kInteger = 1, kArea = 2, kLinear = 3 };
-constexpr int kMaxWindowRows = 96; // source rows of a band that can be staged in shared memory
 
 struct AreaTaps {
     int first, n;
@@ -79,103 +76,132 @@ __device__ __forceinline__ void linear_taps(int d, int ssize, double inv, double
     }
     w0 = min(32767, __float2int_rn(__fmul_rn(__fsub_rn(1.f, f), 2048.f)));
     w1 = min(32767, __float2int_rn(__fmul_rn(f, 2048.f)));
+    if (clamp_last && s + 1 >= ssize) {
+        w0 = 2048;
+        w1 = 0;
+    }
 }
 
 __device__ __forceinline__ int sat_round(float v) { return min(255, max(0, __float2int_rn(v))); }
 
-// uint8 -> float without the conversion pipe: 2^23 + v is representable; the 2^23 is taken off again
-// inside the multiplication, fma(2^23 + v, w, -2^23 * w)
-__device__ __forceinline__ float u8biased(uint32_t v) { return __uint_as_float(0x4B000000u | v); }
-
-// 16 bytes from global to shared memory without passing through registers (L2 only: each source
-// byte is staged once); copies_wait() returns when this thread's copies have landed.
-__device__ __forceinline__ void copy16_async(uint32_t dst_shared, const void *src) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst_shared), "l"(src) : "memory");
+// Byte k of a pixel -> float without the conversion pipe: 2^23 + v is representable; the 2^23 is taken off
+// again inside the multiplication, fma(2^23 + v, w, -2^23 * w)
+template <int k>
+__device__ __forceinline__ float biased(uint32_t px) {
+    return __uint_as_float(pick(px, 0x4B000000u, 0x7440u | k));
 }
-__device__ __forceinline__ void copies_wait() {
-    asm volatile("cp.async.commit_group;" ::: "memory");
-    asm volatile("cp.async.wait_group 0;" ::: "memory");
+// sat_round of a value that is not negative
+__device__ __forceinline__ int round_byte(float v) { return (int)(__float_as_uint(__fadd_rn(fminf(v, 255.f), 8388608.f)) & 0xff); }
+
+// A pixel of a row: of the window's words, or of packed bytes.
+__device__ __forceinline__ uint32_t pixel(const uint32_t *row, int x) { return row[x]; }
+__device__ __forceinline__ uint32_t pixel(const uint8_t *row, int x) {
+    return (uint32_t)row[3 * x] | (uint32_t)row[3 * x + 1] << 8 | (uint32_t)row[3 * x + 2] << 16;
 }
 
-// Per-axis tap tables in shared memory, computed once per CTA (double-precision position
-// arithmetic as OpenCV does it, then only fp32 / integer work per pixel).
-struct TapTables {
-    int *first;  // first source index (area) / source index (linear)
-    int *count;  // area: taps | has_l << 16 | has_r << 17; linear: w0 << 16 | w1
-    float *wl, *wm, *wr;
+// Taps of an output column or row, computed once per CTA (double-precision position arithmetic as
+// OpenCV does it, then only fp32 / integer work per pixel).  Area: first and number of the source indices, weights
+// of the first, the middle and the last tap (0 if there is only one).
+__device__ __forceinline__ uint4 make_area_taps(int d, int ssize, double scale) {
+    const AreaTaps a = area_taps(d, ssize, scale);
+    const float last = a.has_r ? a.wr : a.wm, first = a.has_l ? a.wl : (a.n == 1 ? last : a.wm);
+    return make_uint4((uint32_t)a.first | (uint32_t)a.n << 16, __float_as_uint(first), __float_as_uint(a.wm),
+                      __float_as_uint(a.n == 1 ? 0.f : last));
+}
+// Linear: the two source indices and their weights.
+__device__ __forceinline__ uint4 make_linear_taps(int d, int ssize, double inv, double scale, bool clamp_last) {
+    int s, w0, w1;
+    linear_taps(d, ssize, inv, scale, clamp_last, s, w0, w1);
+    return make_uint4((uint32_t)min(s, ssize - 1), (uint32_t)min(s + 1, ssize - 1), __float_as_uint((float)w0), __float_as_uint((float)w1));
+}
+
+// A column's horizontal sums: first tap, the whole cells between, last tap, rounded after every operation.
+// fma(2^23 + v, w, -2^23 * w) is the correctly rounded v * w, exactly what the multiplication of the
+// converted value gives (2^23 * w is exact).
+struct AreaColumn {
+    int first, last;
+    float w_first, w_mid, w_last;
+    __device__ __forceinline__ explicit AreaColumn(uint4 t) {
+        first = (int)(t.x & 0xffff);
+        last = first + (int)(t.x >> 16) - 1;
+        w_first = __uint_as_float(t.y);
+        w_mid = __uint_as_float(t.z);
+        w_last = __uint_as_float(t.w);
+    }
+    template <class Row>
+    __device__ __forceinline__ void across(Row row, float (&p)[3]) const {
+        uint32_t px = pixel(row, first);
+        float c = -8388608.0f * w_first;
+        p[0] = __fmaf_rn(biased<0>(px), w_first, c);
+        p[1] = __fmaf_rn(biased<1>(px), w_first, c);
+        p[2] = __fmaf_rn(biased<2>(px), w_first, c);
+        c = -8388608.0f * w_mid;
+        for (int k = first + 1; k < last; k++) {
+            px = pixel(row, k);
+            p[0] = __fadd_rn(p[0], __fmaf_rn(biased<0>(px), w_mid, c));
+            p[1] = __fadd_rn(p[1], __fmaf_rn(biased<1>(px), w_mid, c));
+            p[2] = __fadd_rn(p[2], __fmaf_rn(biased<2>(px), w_mid, c));
+        }
+        px = pixel(row, last);
+        c = -8388608.0f * w_last;
+        p[0] = __fadd_rn(p[0], __fmaf_rn(biased<0>(px), w_last, c));
+        p[1] = __fadd_rn(p[1], __fmaf_rn(biased<1>(px), w_last, c));
+        p[2] = __fadd_rn(p[2], __fmaf_rn(biased<2>(px), w_last, c));
+    }
 };
 
-__device__ __forceinline__ void fill_taps(const TapTables &t, int k, int d, int regime, int ssize, double inv,
-                                          double scale, bool clamp_last) {
-    if (regime == kArea) {
-        const AreaTaps a = area_taps(d, ssize, scale);
-        t.first[k] = a.first;
-        t.count[k] = a.n | (a.has_l ? 1 << 16 : 0) | (a.has_r ? 1 << 17 : 0);
-        t.wl[k] = a.wl;
-        t.wm[k] = a.wm;
-        t.wr[k] = a.wr;
-    } else if (regime == kLinear) {
-        int s, w0, w1;
-        linear_taps(d, ssize, inv, scale, clamp_last, s, w0, w1);
-        if (clamp_last && s + 1 >= ssize) {
-            w0 = 2048;
-            w1 = 0;
-        }
-        t.first[k] = s;
-        t.count[k] = (w0 << 16) | w1;
+// OpenCV's fixed-point bilinear, in floating point whose roundings do what the shifts do: with S the two taps'
+// weighted sum (an exact integer below 2^20), 2^27 + S rounded down is 2^27 + 16 * (S >> 4), and
+// fma(b, that, 2^43 - 2^27 * b) rounded down is 2^43 + 2^20 * (b * (S >> 4) >> 16), the product of the integers
+// in the low bits of its mantissa.
+struct LinearColumn {
+    int x0, x1;
+    float w0, w1;
+    __device__ __forceinline__ explicit LinearColumn(uint4 t) {
+        x0 = (int)t.x;
+        x1 = (int)t.y;
+        w0 = __uint_as_float(t.z);
+        w1 = __uint_as_float(t.w);
     }
+    template <class Row>
+    __device__ __forceinline__ void across(Row row, float (&h)[3]) const {
+        const uint32_t p = pixel(row, x0), q = pixel(row, x1);
+        const float c0 = -8388608.0f * w0, c1 = -8388608.0f * w1;
+        auto one = [&](float a, float b) { return __fadd_rd(__fadd_rn(__fmaf_rn(a, w0, c0), __fmaf_rn(b, w1, c1)), 134217728.f); };
+        h[0] = one(biased<0>(p), biased<0>(q));
+        h[1] = one(biased<1>(p), biased<1>(q));
+        h[2] = one(biased<2>(p), biased<2>(q));
+    }
+};
+// (The weights' sum is at most 2049, so 255 is not exceeded.)
+__device__ __forceinline__ int blend_rows(float ha, float hb, float b0, float k0, float b1, float k1) {
+    const uint32_t u = __float_as_uint(__fmaf_rd(b0, ha, k0)), v = __float_as_uint(__fmaf_rd(b1, hb, k1));
+    return (int)((u + v + 2u - 2u * (170u << 23)) >> 2);
 }
 
-// Scaling regime of a crop of ch x cw pixels resized to out_h x out_w, as OpenCV decides it.
-struct Scaling {
-    int regime, isx, isy;
-    double inv_x, inv_y, sc_x, sc_y;
-};
-__device__ __forceinline__ Scaling scaling_of(int ch, int cw, int out_h, int out_w) {
-    Scaling s{kCopy, 1, 1, 1, 1, 1, 1};
-    if (ch != out_h || cw != out_w) {
-        s.inv_x = (double)out_w / cw;
-        s.inv_y = (double)out_h / ch;
-        s.sc_x = 1.0 / s.inv_x;
-        s.sc_y = 1.0 / s.inv_y;
-        if (s.sc_x >= 1 && s.sc_y >= 1) {
-            s.isx = __double2int_rn(s.sc_x);
-            s.isy = __double2int_rn(s.sc_y);
-            s.regime = (fabs(s.sc_x - s.isx) < DBL_EPSILON && fabs(s.sc_y - s.isy) < DBL_EPSILON) ? kInteger : kArea;
-        } else {
-            s.regime = kLinear;
-        }
-    }
-    return s;
-}
+// a / n for a, n < 2^16, inv_n = ceil(2^32 / n)
+__device__ __forceinline__ int divided(uint32_t a, uint32_t inv_n, int n) { return n == 1 ? (int)a : (int)__umulhi(a, inv_n); }
+__device__ __forceinline__ uint32_t inverse(int n) { return (uint32_t)((0x100000000ull + n - 1) / n); }
 
 template <typename OutT>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(256, 4)
 resize_augment_kernel(const __grid_constant__ ResizeSource src, const int32_t *__restrict__ params, int n_params,
                       const __grid_constant__ OpList ops,
-                      int resize, int out_h, int out_w, int band_rows, int groups, int planar, int win_bytes,
+                      int resize, int out_h, int out_w, const __grid_constant__ ResizeShape shape, int planar,
                       const OutT *__restrict__ lut, OutT *__restrict__ out,
                       const int32_t *__restrict__ status, const __grid_constant__ SmallCopies small) {
     extern __shared__ __align__(16) unsigned char s_raw[];
     constexpr bool kU8 = sizeof(OutT) == 1;
-    // shared layout: [out tile][lut][x taps (5 arrays of out_w)][y taps (5 arrays of out_h)]
-    //                [start of each window row][window of source rows (win_bytes)]
+    // shared layout: [out tile][lut][x taps][y taps][window of source pixels]; y taps are indexed by the row of
+    // the resized crop (a translation can move a band anywhere)
     int band0 = 0, rows = 0; // the band of output rows being produced (see the loop below)
-    const int tile_elems = band_rows * out_w * 3;
+    const int groups = shape.groups;
     OutT *s_out = reinterpret_cast<OutT *>(s_raw);
-    size_t off = ((size_t)tile_elems * sizeof(OutT) + 15) & ~(size_t)15;
+    size_t off = ((size_t)shape.band * out_w * 3 * sizeof(OutT) + 15) & ~(size_t)15;
     OutT *s_lut = reinterpret_cast<OutT *>(s_raw + off);
     off += (768 * sizeof(OutT) + 15) & ~(size_t)15;
-    // y taps are indexed by the row of the resized crop (a translation can move a band anywhere)
-    int *ibase = reinterpret_cast<int *>(s_raw + off);
-    TapTables tx{ibase, ibase + out_w, reinterpret_cast<float *>(ibase + 2 * out_w),
-                 reinterpret_cast<float *>(ibase + 3 * out_w), reinterpret_cast<float *>(ibase + 4 * out_w)};
-    int *jbase = ibase + 5 * out_w;
-    TapTables ty{jbase, jbase + out_h, reinterpret_cast<float *>(jbase + 2 * out_h),
-                 reinterpret_cast<float *>(jbase + 3 * out_h), reinterpret_cast<float *>(jbase + 4 * out_h)};
-    int *s_rowoff = jbase + 5 * out_h;
-    unsigned char *s_win =
-        s_raw + ((off + sizeof(int) * (5 * ((size_t)out_w + out_h) + kMaxWindowRows) + 15) & ~(size_t)15);
+    uint4 *tx = reinterpret_cast<uint4 *>(s_raw + off), *ty = tx + out_w;
+    uint32_t *s_win = reinterpret_cast<uint32_t *>(ty + out_h);
 
     const int i = blockIdx.y;
     if (blockIdx.x == 0 && i == 0)
@@ -191,6 +217,7 @@ resize_augment_kernel(const __grid_constant__ ResizeSource src, const int32_t *_
     uint32_t skew_base = 0, skew_pitch = 0;
     bool skew = false;
     bool ok = true;
+    int fuse = 0; // output rows per band of a sample whose planes are converted here
     if (src.descs) {
         const ImageDesc &d = src.descs[i];
         img_h = d.dec_height; // the decoded size: smaller than the stored one after a scaled decode
@@ -209,6 +236,7 @@ resize_augment_kernel(const __grid_constant__ ResizeSource src, const int32_t *_
             }
         } else {
             base = src.rgb + d.rgb_off;
+            fuse = d.fuse_rows;
             ok = d.host_status == 0 && (status == nullptr || status[i] == 0);
         }
     } else {
@@ -228,37 +256,56 @@ resize_augment_kernel(const __grid_constant__ ResizeSource src, const int32_t *_
     } else {
         ok = ok && img_h == out_h && img_w == out_w;
     }
-    // With flips only (or no augmentation) nothing is ever filled and the column an output column
-    // comes from does not depend on the row: the trace is done once per column.
-    bool flips_only = true;
-    for (int k = 0; k < ops.n_ops; k++) flips_only = flips_only && ops.type[k] == kOpFlip;
-    bool rows_in_place = true; // no translation: output row y comes from row y of the resized crop
-    for (int k = 0; k < ops.n_ops; k++) rows_in_place = rows_in_place && ops.type[k] != kOpTranslate;
+    // What is not filled maps to the crop's rows and columns with an offset and a direction.
+    bool flips_only = true; // nothing is ever filled
+    int dy = 0, dx = 0, step_x = 1;
+    for (int k = ops.n_ops - 1; k >= 0; k--) {
+        flips_only = flips_only && ops.type[k] == kOpFlip;
+        if (ops.type[k] == kOpTranslate) {
+            dy += prm[4 + 2 * k] - ops.arg[k];
+            dx += prm[5 + 2 * k] - ops.arg[k];
+        } else if (ops.type[k] == kOpFlip && prm[4 + 2 * k]) {
+            dx = out_w - 1 - dx;
+            step_x = -step_x;
+        }
+    }
 
-    // The scale factors (four double-precision divisions) are worked out by one thread.
+    // The scale factors (four double-precision divisions) are worked out by one thread, and so are the
+    // conversion units of a window row and the number of output rows whose source rows fit the window.
     __shared__ Scaling s_scaling;
-    if (threadIdx.x == 0 && ok) s_scaling = scaling_of(ch, cw, out_h, out_w);
+    __shared__ int s_window, s_units, s_lead;
+    __shared__ uint32_t s_inv_units;
+    if (threadIdx.x == 0 && ok) {
+        s_scaling = scaling_of(ch, cw, out_h, out_w);
+        const bool fits = s_scaling.regime == kArea || s_scaling.regime == kLinear;
+        s_window = fuse ? fuse : (fits ? window_band(cw, s_scaling.sc_y, shape.band, shape.win) : 0);
+        const bool quad = fuse && src.descs[i].scale_shift == 0 && src.descs[i].hs == 2;
+        s_lead = fuse ? (quad ? cj & 7 : cj & 3) : 0; // a unit begins at a multiple of its width
+        s_units = quad ? (s_lead + cw + 7) / 8 : (s_lead + cw + 3) / 4;
+        s_inv_units = inverse(s_units);
+    }
     __syncthreads();
     int regime = kCopy, isx = 1, isy = 1;
+    const int window = ok ? s_window : 0, band_rows = window ? window : shape.band;
+    const int lead = ok ? s_lead : 0, wpitch = window_pitch(cw);
     const int nbands = (out_h + band_rows - 1) / band_rows;
+    if ((int)blockIdx.x >= nbands) return;
     if (ok) {
         const Scaling &sc = s_scaling;
         regime = sc.regime;
         isx = sc.isx;
         isy = sc.isy;
         if (regime == kArea || regime == kLinear) {
-            // x taps of every column; y taps of the rows this CTA produces (of all rows when a
-            // translation can move a band anywhere)
-            const int my_bands = rows_in_place ? (nbands - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x : nbands;
-            const int band_step = rows_in_place ? (int)gridDim.x : 1, band_first = rows_in_place ? (int)blockIdx.x : 0;
+            // x taps of every column, y taps of the rows of the crop that this CTA needs
+            const int my_bands = (nbands - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x;
             for (int e = threadIdx.x; e < out_w + my_bands * band_rows; e += blockDim.x) {
-                if (e < out_w) {
-                    fill_taps(tx, e, e, regime, cw, sc.inv_x, sc.sc_x, true);
-                } else {
-                    const int k = e - out_w, b = k / band_rows;
-                    const int y = (band_first + b * band_step) * band_rows + (k - b * band_rows);
-                    if (y < out_h) fill_taps(ty, y, y, regime, ch, sc.inv_y, sc.sc_y, false);
-                }
+                const bool column = e < out_w;
+                const int k = e - out_w, b = column ? 0 : k / band_rows;
+                const int at = column ? e : ((int)blockIdx.x + b * (int)gridDim.x) * band_rows + (k - b * band_rows) + dy;
+                if (at < 0 || at >= (column ? out_w : out_h)) continue;
+                const int ssize = column ? cw : ch;
+                const double inv = column ? sc.inv_x : sc.inv_y, scale = column ? sc.sc_x : sc.sc_y;
+                (column ? tx : ty)[at] = regime == kArea ? make_area_taps(at, ssize, scale) : make_linear_taps(at, ssize, inv, scale, column);
             }
         }
     }
@@ -272,7 +319,7 @@ resize_augment_kernel(const __grid_constant__ ResizeSource src, const int32_t *_
         return p;
     };
     int npix = 0;
-    const uint32_t inv_w = (uint32_t)((0x100000000ull + out_w - 1) / out_w); // pix / out_w for pix < 2^16
+    const uint32_t inv_w = inverse(out_w);
     // Traces an output pixel back through the augmentations: either a fill colour, or the position
     // (y, x) of a pixel of the resized crop.
     auto trace = [&](int oy, int ox, int &y, int &x, int *val) -> bool {
@@ -302,19 +349,17 @@ resize_augment_kernel(const __grid_constant__ ResizeSource src, const int32_t *_
     // normalise (table gather, one 256-entry table per channel) into the shared tile, in final
     // memory order: element = pix * pix_step + c * chan_step
     int pix_step = 3, chan_step = 1;
-    auto emit = [&](int pix, const int *val) {
-        OutT *o = s_out + pix * pix_step;
-#pragma unroll
-        for (int c = 0; c < 3; c++) {
-            if constexpr (kU8)
-                o[c * chan_step] = (OutT)val[c];
-            else
-                o[c * chan_step] = s_lut[c * 256 + val[c]];
+    auto emit = [&](OutT *o, int v0, int v1, int v2) {
+        if constexpr (kU8) {
+            o[0] = (OutT)v0;
+            o[chan_step] = (OutT)v1;
+            o[2 * chan_step] = (OutT)v2;
+        } else {
+            o[0] = s_lut[v0];
+            o[chan_step] = s_lut[256 + v1];
+            o[2 * chan_step] = s_lut[512 + v2];
         }
     };
-    bool mirrored = false;
-    if (flips_only)
-        for (int k = 0; k < ops.n_ops; k++) mirrored ^= prm[4 + 2 * k] != 0;
     // A CTA produces every gridDim.x-th band of its image: what was set up above (descriptor, tap
     // tables, lookup table) serves all of them.
     for (int band = blockIdx.x; band < nbands; band += gridDim.x) {
@@ -323,198 +368,146 @@ resize_augment_kernel(const __grid_constant__ ResizeSource src, const int32_t *_
     npix = rows * out_w;
     pix_step = planar ? 1 : 3;
     chan_step = planar ? npix : 1;
-    // The source rows this band reads are staged in shared memory first, when they fit: whole
-    // 16-byte words, many in flight per thread, instead of byte loads that each wait for a first
-    // touch of their sector in L2 or HBM (asynchronous copies, no registers in between).  The
-    // window keeps every row at its 16-byte phase.
-    bool staged = false;
+    // The source pixels this band reads, in the window: rows win_lo .. of the crop, `wpitch` words apart, the crop's
+    // first column at `lead`.
     int win_lo = 0;
-    if (win_bytes > 0 && rows_in_place && ok && (regime == kArea || regime == kLinear)) {
-        const int yb = band0 + rows - 1;
-        int hi;
-        if (regime == kArea) {
-            win_lo = ty.first[band0];
-            hi = ty.first[yb] + (ty.count[yb] & 0xffff) - 1;
-        } else {
-            win_lo = min(ty.first[band0], ch - 1);
-            hi = min(ty.first[yb] + 1, ch - 1);
-        }
-        const int nrows = hi - win_lo + 1, pitch = ((cw * 3 + 15) & ~15) + 16;
-        if (nrows <= kMaxWindowRows && nrows * pitch <= win_bytes) {
-            staged = true;
-            const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-            for (int row = warp; row < nrows; row += blockDim.x >> 5) {
-                const uint8_t *p = row_ptr(win_lo + row);
-                const uint32_t phase = (uint32_t)(reinterpret_cast<uintptr_t>(p) & 15);
-                const uint4 *g = reinterpret_cast<const uint4 *>(p - phase);
-                const uint32_t d = (uint32_t)__cvta_generic_to_shared(s_win + row * pitch);
-                const int chunks = (int)(phase + cw * 3 + 15) >> 4;
-                for (int k = lane; k < chunks; k += 32) copy16_async(d + 16u * k, g + k);
-                if (lane == 0) s_rowoff[row] = row * pitch + (int)phase;
+    const int y_lo = max(0, band0 + dy), y_hi = min(out_h, band0 + rows + dy); // rows of the crop in this band
+    if (window && y_lo < y_hi) {
+        const uint4 top = ty[y_lo], bottom = ty[y_hi - 1];
+        win_lo = (int)(regime == kArea ? top.x & 0xffff : top.x);
+        const int hi = (int)(regime == kArea ? (bottom.x & 0xffff) + (bottom.x >> 16) - 1 : bottom.y);
+        const int units = s_units;
+        const uint32_t inv_units = s_inv_units;
+        if (fuse) {
+            const ImageDesc &d = src.descs[i];
+            const uint8_t *py = src.planes + d.plane_off[0], *pb = src.planes + d.plane_off[1], *pr = src.planes + d.plane_off[2];
+            const int r0 = ci + win_lo, r1 = ci + hi; // rows of the image
+            if (d.scale_shift == 0 && d.hs == 2) {
+                const QuadPlanes p{py, pb, pr, d.mcus_x * 16, d.mcus_x * 8, (d.width + 1) >> 1, (d.height + 1) >> 1};
+                const int n_items = units * ((r1 >> 1) - (r0 >> 1) + 1);
+                for (int e = threadIdx.x; e < n_items; e += blockDim.x) {
+                    const int v = divided(e, inv_units, units), u = e - v * units, cy = (r0 >> 1) + v;
+                    uint32_t px[2][8];
+                    quad_pixels(p, ((cj - lead) >> 1) + 4 * u, cy, px);
+#pragma unroll
+                    for (int r = 0; r < 2; r++) {
+                        const int y = 2 * cy + r;
+                        if (y < r0 || y > r1) continue;
+                        uint4 *w = reinterpret_cast<uint4 *>(s_win + (y - r0) * wpitch + 8 * u);
+                        w[0] = make_uint4(px[r][0], px[r][1], px[r][2], px[r][3]);
+                        w[1] = make_uint4(px[r][4], px[r][5], px[r][6], px[r][7]);
+                    }
+                }
+            } else {
+                const int pw = d.mcus_x * d.hs * d.bs_luma;
+                const bool words = (pw & 3) == 0; // (planes begin at multiples of 16)
+                const int n_items = units * (r1 - r0 + 1);
+                for (int e = threadIdx.x; e < n_items; e += blockDim.x) {
+                    const int v = divided(e, inv_units, units), x = cj - lead + 4 * (e - v * units);
+                    uint32_t px[4];
+                    plain_pixels(py, pb, pr, (size_t)(r0 + v) * pw + x, min(4, img_w - x), words, px);
+                    *reinterpret_cast<uint4 *>(s_win + v * wpitch + (x - cj + lead)) = make_uint4(px[0], px[1], px[2], px[3]);
+                }
             }
-            copies_wait();
-            __syncthreads();
+        } else { // packed pixels: four at a time out of the aligned words that hold them
+            const int n_items = units * (hi - win_lo + 1);
+            for (int e = threadIdx.x; e < n_items; e += blockDim.x) {
+                const int v = divided(e, inv_units, units), u = e - v * units;
+                const uint8_t *p = row_ptr(win_lo + v) + 12 * u;
+                const uint32_t phase = (uint32_t)(reinterpret_cast<uintptr_t>(p) & 3), bytes = phase + 3 * min(4, cw - 4 * u);
+                const uint32_t *g = reinterpret_cast<const uint32_t *>(p - phase);
+                uint32_t w[4];
+#pragma unroll
+                for (int k = 0; k < 4; k++) w[k] = 4 * k < bytes ? g[k] : 0;
+#pragma unroll
+                for (int k = 0; k < 3; k++) w[k] = __funnelshift_r(w[k], w[k + 1], 8 * phase);
+                *reinterpret_cast<uint4 *>(s_win + v * wpitch + 4 * u) =
+                    make_uint4(w[0], pick(w[0], w[1], 0x0543), pick(w[1], w[2], 0x0432), w[2] >> 8);
+            }
         }
+        __syncthreads();
     }
-    if (regime == kArea && ok) {
-        // Shrinking by fractional factors is separable: OpenCV first sums every source row
-        // horizontally with the x weights, then combines those row sums with the y weights.  A
-        // thread therefore owns one output column for a run of consecutive output rows: the x taps
-        // and weights of its column live in registers for the whole run, and the horizontal sum of
-        // a source row that two neighbouring output rows share (the row their boundary cuts) is
-        // computed once.  Same operations in the same order as the per-pixel form, so the same bits.
+    auto window_row = [&](int y) -> const uint32_t * { return s_win + (y - win_lo) * wpitch + lead; };
+    if (regime == kArea || regime == kLinear) { // (and ok)
+        // OpenCV first sums every source row horizontally with the x weights, then combines those row sums with
+        // the y weights; likewise for its two-tap interpolation.  A thread therefore owns one output column for
+        // a run of consecutive output rows: the taps and weights of its column live in registers for the whole
+        // run, and what a source row contributes is computed once for neighbouring output rows that share it.
+        // Same operations in the same order as the per-pixel form, so the same bits.
         const int run = (rows + groups - 1) / groups;
-        auto area_columns = [&](auto from_window) {
-        for (int t = threadIdx.x; t < groups * out_w; t += blockDim.x) {
-            const int g = (int)__umulhi((uint32_t)t, inv_w), ox = t - g * out_w;
-            const int r_end = min(rows, (g + 1) * run);
-            int cx = -1, xoff = 0, xmid = 0, xlast = 0; // column whose taps are loaded
-            bool two = false;
-            float w_first = 0.f, w_mid = 0.f, w_last = 0.f, c_first = 0.f, c_mid = 0.f, c_last = 0.f;
-            int pj = -1;                       // source row whose horizontal sums are held
-            float p0 = 0.f, p1 = 0.f, p2 = 0.f;
-            const int x_plain = mirrored ? out_w - 1 - ox : ox;
-            // horizontal sums of one source row: first tap, the whole cells between, last tap.
-            // fma(2^23 + v, w, -2^23 * w) is the correctly rounded v * w, exactly what the
-            // multiplication of the converted value gives (2^23 * w is exact).
-            auto across = [&](int row) {
-                const uint8_t *p;
-                if constexpr (decltype(from_window)::value)
-                    p = s_win + s_rowoff[row - win_lo] + xoff;
-                else
-                    p = row_ptr(row) + xoff;
-                p0 = __fmaf_rn(u8biased(p[0]), w_first, c_first);
-                p1 = __fmaf_rn(u8biased(p[1]), w_first, c_first);
-                p2 = __fmaf_rn(u8biased(p[2]), w_first, c_first);
-                const uint8_t *q = p + 3;
-                for (int k = 0; k < xmid; k++, q += 3) {
-                    p0 = __fadd_rn(p0, __fmaf_rn(u8biased(q[0]), w_mid, c_mid));
-                    p1 = __fadd_rn(p1, __fmaf_rn(u8biased(q[1]), w_mid, c_mid));
-                    p2 = __fadd_rn(p2, __fmaf_rn(u8biased(q[2]), w_mid, c_mid));
-                }
-                if (two) {
-                    p0 = __fadd_rn(p0, __fmaf_rn(u8biased(p[xlast]), w_last, c_last));
-                    p1 = __fadd_rn(p1, __fmaf_rn(u8biased(p[xlast + 1]), w_last, c_last));
-                    p2 = __fadd_rn(p2, __fmaf_rn(u8biased(p[xlast + 2]), w_last, c_last));
-                }
-            };
-            for (int r = g * run; r < r_end; r++) {
-                int y = band0 + r, x = x_plain, val[3] = {0, 0, 0};
-                if (flips_only || !trace(band0 + r, ox, y, x, val)) {
-                    if (x != cx) {
-                        cx = x;
-                        pj = -1;
-                        const int xc = tx.count[x], xn = xc & 0xffff;
-                        const bool xl = xc & (1 << 16), xr = xc & (1 << 17);
-                        xoff = tx.first[x] * 3;
-                        w_mid = tx.wm[x];
-                        w_last = xr ? tx.wr[x] : w_mid;
-                        w_first = xl ? tx.wl[x] : (xn == 1 ? w_last : w_mid);
-                        two = xn >= 2;
-                        xmid = max(xn - 2, 0);
-                        xlast = (xn - 1) * 3;
-                        c_first = -8388608.0f * w_first;
-                        c_mid = -8388608.0f * w_mid;
-                        c_last = -8388608.0f * w_last;
+        // row_of: a row of the crop, in the window or in global memory
+        auto columns = [&](auto row_of) {
+            for (int t = threadIdx.x; t < groups * out_w; t += blockDim.x) {
+                const int g = divided(t, inv_w, out_w), ox = t - g * out_w;
+                const int begin = max(y_lo, band0 + g * run + dy), end = min(y_hi, band0 + (g + 1) * run + dy);
+                const uint4 taps = tx[min(max(step_x * ox + dx, 0), out_w - 1)];
+                OutT *o = s_out + ((begin - dy - band0) * out_w + ox) * pix_step;
+                const int row_step = out_w * pix_step;
+                if (regime == kArea) {
+                    const AreaColumn column(taps);
+                    int pj = -1; // source row whose horizontal sums are held
+                    float p[3] = {0.f, 0.f, 0.f};
+                    for (int y = begin; y < end; y++, o += row_step) {
+                        const uint4 c = ty[y];
+                        const int yf = (int)(c.x & 0xffff), ye = yf + (int)(c.x >> 16) - 1;
+                        // only the first source row can be the one the previous output row ended with
+                        if (yf != pj) column.across(row_of(yf), p);
+                        float beta = __uint_as_float(c.y);
+                        float a0 = __fmul_rn(beta, p[0]), a1 = __fmul_rn(beta, p[1]), a2 = __fmul_rn(beta, p[2]);
+                        for (int j = yf + 1; j <= ye; j++) {
+                            column.across(row_of(j), p);
+                            beta = __uint_as_float(j == ye ? c.w : c.z);
+                            a0 = __fadd_rn(a0, __fmul_rn(beta, p[0]));
+                            a1 = __fadd_rn(a1, __fmul_rn(beta, p[1]));
+                            a2 = __fadd_rn(a2, __fmul_rn(beta, p[2]));
+                        }
+                        pj = ye;
+                        emit(o, round_byte(a0), round_byte(a1), round_byte(a2));
                     }
-                    const int yf = ty.first[y], yc = ty.count[y], yn = yc & 0xffff;
-                    const float ywm = ty.wm[y];
-                    const float y_last = (yc & (1 << 17)) ? ty.wr[y] : ywm;
-                    const float y_first = (yc & (1 << 16)) ? ty.wl[y] : (yn == 1 ? y_last : ywm);
-                    // only the first source row can be the one the previous output row ended with
-                    if (yf != pj) across(yf);
-                    float a0 = __fmul_rn(y_first, p0), a1 = __fmul_rn(y_first, p1), a2 = __fmul_rn(y_first, p2);
-                    for (int j = 1; j < yn; j++) {
-                        across(yf + j);
-                        const float beta = j == yn - 1 ? y_last : ywm;
-                        a0 = __fadd_rn(a0, __fmul_rn(beta, p0));
-                        a1 = __fadd_rn(a1, __fmul_rn(beta, p1));
-                        a2 = __fadd_rn(a2, __fmul_rn(beta, p2));
+                } else {
+                    const LinearColumn column(taps);
+                    int ra = -1, rb = -1; // source rows whose interpolated values ha / hb hold
+                    float ha[3] = {0.f, 0.f, 0.f}, hb[3] = {0.f, 0.f, 0.f};
+                    for (int y = begin; y < end; y++, o += row_step) {
+                        const uint4 c = ty[y];
+                        const int r0 = (int)c.x, r1 = (int)c.y;
+                        // rows only move forward: the upper row is the former upper or lower one, or both are new
+                        if (r0 != ra) {
+                            if (r0 == rb) {
+#pragma unroll
+                                for (int k = 0; k < 3; k++) ha[k] = hb[k];
+                            } else {
+                                column.across(row_of(r0), ha);
+                            }
+                            ra = r0;
+                        }
+                        if (r1 != rb) {
+                            column.across(row_of(r1), hb);
+                            rb = r1;
+                        }
+                        const float b0 = __uint_as_float(c.z), b1 = __uint_as_float(c.w);
+                        const float k0 = __fmaf_rn(b0, -134217728.f, 8796093022208.f), k1 = __fmaf_rn(b1, -134217728.f, 8796093022208.f);
+                        emit(o, blend_rows(ha[0], hb[0], b0, k0, b1, k1), blend_rows(ha[1], hb[1], b0, k0, b1, k1),
+                             blend_rows(ha[2], hb[2], b0, k0, b1, k1));
                     }
-                    pj = yf + yn - 1;
-                    val[0] = sat_round(a0);
-                    val[1] = sat_round(a1);
-                    val[2] = sat_round(a2);
                 }
-                emit(r * out_w + ox, val);
+            }
+        };
+        if (window)
+            columns(window_row);
+        else
+            columns(row_ptr);
+        if (!flips_only) { // what is filled, over it
+            __syncthreads();
+            for (int pix = threadIdx.x; pix < npix; pix += blockDim.x) {
+                const int r = divided(pix, inv_w, out_w), ox = pix - r * out_w;
+                int y, x, val[3];
+                if (trace(band0 + r, ox, y, x, val)) emit(s_out + pix * pix_step, val[0], val[1], val[2]);
             }
         }
-        };
-        if (staged)
-            area_columns(std::true_type{});
-        else
-            area_columns(std::false_type{});
-    } else if (regime == kLinear && ok) {
-        // Enlarging (OpenCV's fixed-point bilinear) with the same ownership: the two taps of the
-        // column stay in registers, and of the two source rows an output row blends, the next
-        // output row nearly always shares one or both, whose horizontally interpolated values
-        // are kept instead of being fetched and interpolated again.
-        const int run = (rows + groups - 1) / groups;
-        auto linear_columns = [&](auto from_window) {
-        for (int t = threadIdx.x; t < groups * out_w; t += blockDim.x) {
-            const int g = (int)__umulhi((uint32_t)t, inv_w), ox = t - g * out_w;
-            const int r_end = min(rows, (g + 1) * run);
-            int cx = -1, o0 = 0, o1 = 0, xa0 = 0, xa1 = 0;
-            int ra = -1, rb = -1; // source rows whose interpolated values ha / hb hold
-            int ha[3] = {0, 0, 0}, hb[3] = {0, 0, 0};
-            const int x_plain = mirrored ? out_w - 1 - ox : ox;
-            for (int r = g * run; r < r_end; r++) {
-                int y = band0 + r, x = x_plain, val[3] = {0, 0, 0};
-                if (flips_only || !trace(band0 + r, ox, y, x, val)) {
-                    if (x != cx) {
-                        cx = x;
-                        ra = rb = -1;
-                        const int sx = tx.first[x], xw = tx.count[x];
-                        xa0 = xw >> 16;
-                        xa1 = xw & 0xffff;
-                        o0 = 3 * sx;
-                        o1 = 3 * min(sx + 1, cw - 1);
-                    }
-                    const int sy = ty.first[y], yw = ty.count[y], b0 = yw >> 16, b1 = yw & 0xffff;
-                    const int ry0 = min(sy, ch - 1), ry1 = min(sy + 1, ch - 1);
-                    auto across = [&](int row, int *h) {
-                        const uint8_t *S;
-                        if constexpr (decltype(from_window)::value)
-                            S = s_win + s_rowoff[row - win_lo];
-                        else
-                            S = row_ptr(row);
-#pragma unroll
-                        for (int c = 0; c < 3; c++) h[c] = (S[o0 + c] * xa0 + S[o1 + c] * xa1) >> 4;
-                    };
-                    // rows only move forward: the upper row is the former upper or lower one
-                    // (selects, no branch), or both rows are new
-                    if (ry0 == rb) {
-#pragma unroll
-                        for (int c = 0; c < 3; c++) ha[c] = hb[c];
-                    } else if (ry0 != ra) {
-                        across(ry0, ha);
-                    }
-                    if (ry1 == ry0) {
-#pragma unroll
-                        for (int c = 0; c < 3; c++) hb[c] = ha[c];
-                    } else if (ry1 != rb) {
-                        across(ry1, hb);
-                    }
-                    ra = ry0;
-                    rb = ry1;
-#pragma unroll
-                    for (int c = 0; c < 3; c++) {
-                        // non-negative terms: only the upper bound can be exceeded (by rounding of the weights)
-                        const int v = (((b0 * ha[c]) >> 16) + ((b1 * hb[c]) >> 16) + 2) >> 2;
-                        val[c] = min(255, v);
-                    }
-                }
-                emit(r * out_w + ox, val);
-            }
-        }
-        };
-        if (staged)
-            linear_columns(std::true_type{});
-        else
-            linear_columns(std::false_type{});
     } else {
         for (int pix = threadIdx.x; pix < npix; pix += blockDim.x) {
-            const int r = (int)__umulhi((uint32_t)pix, inv_w), ox = pix - r * out_w;
+            const int r = divided(pix, inv_w, out_w), ox = pix - r * out_w;
             int y, x, val[3] = {0, 0, 0};
             if (!trace(band0 + r, ox, y, x, val) && ok) {
                 if (regime == kCopy) {
@@ -544,7 +537,7 @@ resize_augment_kernel(const __grid_constant__ ResizeSource src, const int32_t *_
                     }
                 }
             }
-            emit(pix, val);
+            emit(s_out + pix * pix_step, val[0], val[1], val[2]);
         }
     }
     __syncthreads();
@@ -568,49 +561,55 @@ resize_augment_kernel(const __grid_constant__ ResizeSource src, const int32_t *_
     }
 }
 
-template <typename OutT>
-static void launch_typed(const ResizeSource &src, int n, const int32_t *params, int n_params, const OpList &ops,
-                         int resize, int out_h, int out_w, int planar, const void *lut, void *out,
-                         const int32_t *status, const SmallCopies &small, cudaStream_t stream) {
+ResizeShape resize_shape(int out_h, int out_w, int out_kind) {
+    const size_t elem = out_kind == kOutU8 ? 1 : (out_kind == kOutF16Nhwc || out_kind == kOutF16Nchw ? 2 : 4);
+    ResizeShape s{};
     int band = (2048 + out_w - 1) / out_w;
     if (band < 1) band = 1;
     if (band > out_h) band = out_h;
     auto smem_for = [&](int b) {
-        size_t tile = (((size_t)b * out_w * 3 * sizeof(OutT)) + 15) & ~(size_t)15;
-        size_t lutb = (768 * sizeof(OutT) + 15) & ~(size_t)15;
-        return ((tile + lutb + sizeof(int) * (5 * ((size_t)out_w + out_h) + kMaxWindowRows)) + 15) & ~(size_t)15;
+        return (((size_t)b * out_w * 3 * elem + 15) & ~(size_t)15) + ((768 * elem + 15) & ~(size_t)15) + sizeof(uint4) * ((size_t)out_w + out_h);
     };
     while (band > 1 && smem_for(band) > 200 * 1024) band /= 2;
-    // window of source rows: what is left of a quarter of the SM's shared memory (four resident
-    // CTAs of 256 threads is what the registers allow), at most 32 KiB
+    // window of source pixels: what is left of a quarter of the SM's shared memory (four resident
+    // CTAs of 256 threads is what the registers allow), at most 40 KiB
     const size_t quarter = (227 * 1024) / 4 - 1024;
     size_t win = smem_for(band) + 4096 <= quarter ? quarter - smem_for(band) : 0;
-    if (win > 32 * 1024) win = 32 * 1024;
-    win &= ~(size_t)15;
-    const size_t smem = smem_for(band) + win;
-    auto kern = resize_augment_kernel<OutT>;
-    if (smem > 48 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    // CTAs per image: enough of them for about eight waves of the GPU (148 SMs x 4 resident CTAs;
-    // fewer waves measured slower, more cost the set-up its amortisation), at most one per band
-    const int nbands = (out_h + band - 1) / band;
-    int per_image = (8 * 148 * 4 + n - 1) / n;
-    if (per_image > nbands) per_image = nbands;
-    if (per_image < 1) per_image = 1;
-    dim3 grid(per_image, n);
-    // column path of the area regime: the band's rows are dealt to `groups` runs per column so that
+    if (win > 40 * 1024) win = 40 * 1024;
+    s.win = win & ~(size_t)15;
+    s.smem = smem_for(band) + s.win;
+    s.band = band;
+    // column paths: the band's rows are dealt to `groups` runs per column so that
     // the (column, run) items fill the CTA's 256 threads evenly, with runs of at least 3 rows
-    int groups = 1;
+    s.groups = 1;
     double best = 0;
     for (int g = 1; g <= 4 && (band + g - 1) / g >= 3; g++) {
         const int items = g * out_w;
         const double use = (double)items / (((items + 255) / 256) * 256);
         if (use > best + 1e-9) {
             best = use;
-            groups = g;
+            s.groups = g;
         }
     }
-    kern<<<grid, 256, smem, stream>>>(src, params, n_params, ops, resize, out_h, out_w, band, groups, planar,
-                                      (int)win, (const OutT *)lut, (OutT *)out, status, small);
+    return s;
+}
+
+template <typename OutT>
+static void launch_typed(const ResizeSource &src, int n, const int32_t *params, int n_params, const OpList &ops,
+                         int resize, int out_h, int out_w, int planar, const ResizeShape &shape, const void *lut, void *out,
+                         const int32_t *status, const SmallCopies &small, cudaStream_t stream) {
+    auto kern = resize_augment_kernel<OutT>;
+    if (shape.smem > 48 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shape.smem);
+    // CTAs per image: enough of them for about eight waves of the GPU (148 SMs x 4 resident CTAs;
+    // fewer waves measured slower, more cost the set-up its amortisation), at most one per band (a sample
+    // whose window holds fewer rows has more of them, of at least four rows)
+    const int least = shape.band > 4 ? 4 : shape.band, nbands = (out_h + least - 1) / least;
+    int per_image = (8 * 148 * 4 + n - 1) / n;
+    if (per_image > nbands) per_image = nbands;
+    if (per_image < 1) per_image = 1;
+    dim3 grid(per_image, n);
+    kern<<<grid, 256, shape.smem, stream>>>(src, params, n_params, ops, resize, out_h, out_w, shape, planar,
+                                            (const OutT *)lut, (OutT *)out, status, small);
 }
 
 void launch_resize_augment(const ResizeSource &src, int n, const int32_t *params, int n_params,
@@ -618,12 +617,13 @@ void launch_resize_augment(const ResizeSource &src, int n, const int32_t *params
                            const void *lut, void *out, const int32_t *status, const SmallCopies &small, cudaStream_t stream) {
     if (n <= 0) return;
     const int planar = out_kind == kOutF16Nchw || out_kind == kOutF32Nchw;
+    const ResizeShape shape = resize_shape(out_h, out_w, out_kind);
     if (out_kind == kOutU8)
-        launch_typed<uint8_t>(src, n, params, n_params, ops, resize, out_h, out_w, 0, nullptr, out, status, small, stream);
+        launch_typed<uint8_t>(src, n, params, n_params, ops, resize, out_h, out_w, 0, shape, nullptr, out, status, small, stream);
     else if (out_kind == kOutF16Nhwc || out_kind == kOutF16Nchw)
-        launch_typed<uint16_t>(src, n, params, n_params, ops, resize, out_h, out_w, planar, lut, out, status, small, stream);
+        launch_typed<uint16_t>(src, n, params, n_params, ops, resize, out_h, out_w, planar, shape, lut, out, status, small, stream);
     else
-        launch_typed<uint32_t>(src, n, params, n_params, ops, resize, out_h, out_w, planar, lut, out, status, small, stream);
+        launch_typed<uint32_t>(src, n, params, n_params, ops, resize, out_h, out_w, planar, shape, lut, out, status, small, stream);
 }
 
 } // namespace ffcvb

@@ -87,6 +87,8 @@ struct ImageDesc {
                            // ceil(MCUs / restart_interval) + 1 uint32 interval starts (4-aligned)
     uint64_t plane_off[kMaxComponents]; // byte offsets of the Y/Cb/Cr planes in the plane scratch
     uint64_t rgb_off;      // byte offset of the decoded h*w*3 image in the RGB scratch
+    uint16_t fuse_rows;    // the resize kernel converts the planes itself, for this many output rows at a time (0: the
+                           // colour kernels leave an image in the RGB scratch)
     uint64_t src_addr;     // device-visible address of the payload in pinned host memory (0: staged copy)
 };
 
