@@ -990,7 +990,8 @@ int stage_impl(ffcvb_ctx *ctx, int slot, const Source &source, const uint64_t *p
     ctx->stage_seq++;
     int max_w = 0, max_h = 0, n_quad = 0, n_444 = 0, n_other = 0;
     const bool can_fuse = plan->resize && !s.packed;
-    const ResizeShape shape = can_fuse ? resize_shape(plan->out_h, plan->out_w, plan->out_kind) : ResizeShape{};
+    const ResizeShape shape = can_fuse ? resize_shape(n, plan->out_h, plan->out_w, plan->out_kind) : ResizeShape{};
+    const size_t tile_row = (size_t)plan->out_w * 3 * (plan->out_kind == FFCVB_OUT_U8_NHWC ? 1 : (plan->out_kind == FFCVB_OUT_F16_NHWC || plan->out_kind == FFCVB_OUT_F16_NCHW ? 2 : 4));
     for (int i = 0; i < n; i++) {
         ImageDesc &d = descs[i];
         if (d.mode != FFCVB_MODE_JPG) continue;
@@ -1108,7 +1109,7 @@ int stage_impl(ffcvb_ctx *ctx, int slot, const Source &source, const uint64_t *p
                 box[1] + box[3] <= (int)d.width) {
                 scaled_box(d, box);
                 const Scaling sc = scaling_of(box[2], box[3], plan->out_h, plan->out_w);
-                if (sc.regime == kArea || sc.regime == kLinear) d.fuse_rows = (uint16_t)window_band(box[3], sc.sc_y, shape.band, shape.win);
+                if (sc.regime == kArea || sc.regime == kLinear) d.fuse_rows = (uint16_t)window_band(box[3], sc.sc_y, tile_row, shape);
             }
         }
         d.rgb_off = rgb_bytes;

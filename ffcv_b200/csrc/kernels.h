@@ -120,21 +120,22 @@ FFCVB_HD inline Scaling scaling_of(int ch, int cw, int out_h, int out_w) {
     return s;
 }
 
-// How the resize kernel works on an output: rows per band, runs of rows per column, bytes of the window of
-// source pixels, and of shared memory.
+// How the resize kernel works on an output: rows per band without and (at most) with a window of source
+// pixels; bytes of shared memory for the output tile and the window, and of all.
 struct ResizeShape {
-    int band, groups;
-    size_t win, smem;
+    int band, max_band;
+    size_t room, smem;
 };
-ResizeShape resize_shape(int out_h, int out_w, int out_kind);
-// Pixels (words) of a row of the window, and the output rows whose source rows fit in it: `band` of them or
-// fewer, 0 when so few fit that windows do not pay.  (b output rows span at most b * sc_y + 3 source rows.)
+ResizeShape resize_shape(int n, int out_h, int out_w, int out_kind);
+// Pixels (words) of a row of the window, and the output rows per band whose tile (rows of tile_row bytes) and source
+// rows fit in the room; 0 when so few fit that a window does not pay.  b output rows span at most
+// b * sc_y + 3 source rows, of which those that two bands share are fetched twice, so more is better.
 FFCVB_HD inline int window_pitch(int cw) { return (cw + 14) & ~7; }
-FFCVB_HD inline int window_band(int cw, double sc_y, int band, size_t win) {
-    const int cap = (int)(win / (4 * (size_t)window_pitch(cw)));
-    if (cap < 4) return 0;
-    const double fit = (cap - 3) / sc_y;
-    if (fit >= band) return band;
+FFCVB_HD inline int window_band(int cw, double sc_y, size_t tile_row, const ResizeShape &shape) {
+    const double pitch = 4.0 * window_pitch(cw), left = (double)shape.room - 16 - 3 * pitch;
+    if (left <= 0) return 0;
+    const double fit = left / ((double)tile_row + sc_y * pitch);
+    if (fit >= shape.max_band) return shape.max_band;
     const int b = (int)fit & ~1; // (even: most bands then begin on 16 bytes)
     return b >= 4 ? b : 0;
 }

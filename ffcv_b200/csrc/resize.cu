@@ -115,9 +115,40 @@ __device__ __forceinline__ uint4 make_linear_taps(int d, int ssize, double inv, 
     return make_uint4((uint32_t)min(s, ssize - 1), (uint32_t)min(s + 1, ssize - 1), __float_as_uint((float)w0), __float_as_uint((float)w1));
 }
 
+// Two floats per register pair, and two operations per instruction.
+struct Two {
+    unsigned long long v;
+    __device__ __forceinline__ Two() {}
+    __device__ __forceinline__ Two(float lo, float hi) { asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "f"(lo), "f"(hi)); }
+    __device__ __forceinline__ float lo() const { return half(0); }
+    __device__ __forceinline__ float hi() const { return half(1); }
+    __device__ __forceinline__ float half(int k) const {
+        float a, b;
+        asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
+        return k ? b : a;
+    }
+};
+__device__ __forceinline__ Two fma_rn(Two a, Two b, Two c) {
+    Two r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v));
+    return r;
+}
+__device__ __forceinline__ Two fma_rd(Two a, Two b, Two c) {
+    Two r;
+    asm("fma.rm.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v));
+    return r;
+}
+__device__ __forceinline__ Two add_rn(Two a, Two b) {
+    Two r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+    return r;
+}
+// (as a sum with zero: a product that is added next may be contracted into one rounding, which must not happen)
+__device__ __forceinline__ Two mul_rn(Two a, Two b) { return fma_rn(a, b, Two(0.f, 0.f)); }
+
 // A column's horizontal sums: first tap, the whole cells between, last tap, rounded after every operation.
 // fma(2^23 + v, w, -2^23 * w) is the correctly rounded v * w, exactly what the multiplication of the
-// converted value gives (2^23 * w is exact).
+// converted value gives (2^23 * w is exact).  Red and green share their instructions.
 struct AreaColumn {
     int first, last;
     float w_first, w_mid, w_last;
@@ -128,55 +159,70 @@ struct AreaColumn {
         w_mid = __uint_as_float(t.z);
         w_last = __uint_as_float(t.w);
     }
+    static __device__ __forceinline__ void tap(uint32_t px, float w, Two &rg, float &b) {
+        const float c = -8388608.0f * w;
+        rg = fma_rn(Two(biased<0>(px), biased<1>(px)), Two(w, w), Two(c, c));
+        b = __fmaf_rn(biased<2>(px), w, c);
+    }
     template <class Row>
-    __device__ __forceinline__ void across(Row row, float (&p)[3]) const {
-        uint32_t px = pixel(row, first);
-        float c = -8388608.0f * w_first;
-        p[0] = __fmaf_rn(biased<0>(px), w_first, c);
-        p[1] = __fmaf_rn(biased<1>(px), w_first, c);
-        p[2] = __fmaf_rn(biased<2>(px), w_first, c);
-        c = -8388608.0f * w_mid;
+    __device__ __forceinline__ void across(Row row, Two &rg, float &b) const {
+        Two rg2;
+        float b2;
+        tap(pixel(row, first), w_first, rg, b);
         for (int k = first + 1; k < last; k++) {
-            px = pixel(row, k);
-            p[0] = __fadd_rn(p[0], __fmaf_rn(biased<0>(px), w_mid, c));
-            p[1] = __fadd_rn(p[1], __fmaf_rn(biased<1>(px), w_mid, c));
-            p[2] = __fadd_rn(p[2], __fmaf_rn(biased<2>(px), w_mid, c));
+            tap(pixel(row, k), w_mid, rg2, b2);
+            rg = add_rn(rg, rg2);
+            b = __fadd_rn(b, b2);
         }
-        px = pixel(row, last);
-        c = -8388608.0f * w_last;
-        p[0] = __fadd_rn(p[0], __fmaf_rn(biased<0>(px), w_last, c));
-        p[1] = __fadd_rn(p[1], __fmaf_rn(biased<1>(px), w_last, c));
-        p[2] = __fadd_rn(p[2], __fmaf_rn(biased<2>(px), w_last, c));
+        tap(pixel(row, last), w_last, rg2, b2);
+        rg = add_rn(rg, rg2);
+        b = __fadd_rn(b, b2);
     }
 };
 
 // OpenCV's fixed-point bilinear, in floating point whose roundings do what the shifts do: with S the two taps'
 // weighted sum (an exact integer below 2^20), 2^27 + S rounded down is 2^27 + 16 * (S >> 4), and
 // fma(b, that, 2^43 - 2^27 * b) rounded down is 2^43 + 2^20 * (b * (S >> 4) >> 16), the product of the integers
-// in the low bits of its mantissa.
+// in the low bits of its mantissa.  The two taps of a channel share their instruction, and so do the two rows.
 struct LinearColumn {
     int x0, x1;
-    float w0, w1;
+    Two w, c;
     __device__ __forceinline__ explicit LinearColumn(uint4 t) {
         x0 = (int)t.x;
         x1 = (int)t.y;
-        w0 = __uint_as_float(t.z);
-        w1 = __uint_as_float(t.w);
+        w = Two(__uint_as_float(t.z), __uint_as_float(t.w));
+        c = mul_rn(w, Two(-8388608.0f, -8388608.0f));
     }
     template <class Row>
     __device__ __forceinline__ void across(Row row, float (&h)[3]) const {
         const uint32_t p = pixel(row, x0), q = pixel(row, x1);
-        const float c0 = -8388608.0f * w0, c1 = -8388608.0f * w1;
-        auto one = [&](float a, float b) { return __fadd_rd(__fadd_rn(__fmaf_rn(a, w0, c0), __fmaf_rn(b, w1, c1)), 134217728.f); };
+        auto one = [&](float a, float b) {
+            const Two s = fma_rn(Two(a, b), w, c);
+            return __fadd_rd(__fadd_rn(s.lo(), s.hi()), 134217728.f);
+        };
         h[0] = one(biased<0>(p), biased<0>(q));
         h[1] = one(biased<1>(p), biased<1>(q));
         h[2] = one(biased<2>(p), biased<2>(q));
     }
 };
 // (The weights' sum is at most 2049, so 255 is not exceeded.)
-__device__ __forceinline__ int blend_rows(float ha, float hb, float b0, float k0, float b1, float k1) {
-    const uint32_t u = __float_as_uint(__fmaf_rd(b0, ha, k0)), v = __float_as_uint(__fmaf_rd(b1, hb, k1));
-    return (int)((u + v + 2u - 2u * (170u << 23)) >> 2);
+__device__ __forceinline__ int blend_rows(float upper, float lower, Two b, Two k) {
+    const Two u = fma_rd(b, Two(upper, lower), k);
+    return (int)((__float_as_uint(u.lo()) + __float_as_uint(u.hi()) + 2u - 2u * (170u << 23)) >> 2);
+}
+
+// The column paths deal a band's rows to this many runs per column, so that the (column, run) items fill the
+// CTA's 256 threads evenly, with runs of at least 3 rows.
+__device__ __forceinline__ int row_groups(int out_w, int band) {
+    int groups = 1, best = 0;
+    for (int g = 1; g <= 4 && (band + g - 1) / g >= 3; g++) {
+        const int items = g * out_w, use = items * 256 / ((items + 255) / 256 * 256);
+        if (use > best) {
+            best = use;
+            groups = g;
+        }
+    }
+    return groups;
 }
 
 // a / n for a, n < 2^16, inv_n = ceil(2^32 / n)
@@ -192,16 +238,13 @@ resize_augment_kernel(const __grid_constant__ ResizeSource src, const int32_t *_
                       const int32_t *__restrict__ status, const __grid_constant__ SmallCopies small) {
     extern __shared__ __align__(16) unsigned char s_raw[];
     constexpr bool kU8 = sizeof(OutT) == 1;
-    // shared layout: [out tile][lut][x taps][y taps][window of source pixels]; y taps are indexed by the row of
+    // shared layout: [lut][x taps][y taps][out tile][window of source pixels]; y taps are indexed by the row of
     // the resized crop (a translation can move a band anywhere)
     int band0 = 0, rows = 0; // the band of output rows being produced (see the loop below)
-    const int groups = shape.groups;
-    OutT *s_out = reinterpret_cast<OutT *>(s_raw);
-    size_t off = ((size_t)shape.band * out_w * 3 * sizeof(OutT) + 15) & ~(size_t)15;
-    OutT *s_lut = reinterpret_cast<OutT *>(s_raw + off);
-    off += (768 * sizeof(OutT) + 15) & ~(size_t)15;
-    uint4 *tx = reinterpret_cast<uint4 *>(s_raw + off), *ty = tx + out_w;
-    uint32_t *s_win = reinterpret_cast<uint32_t *>(ty + out_h);
+    OutT *s_lut = reinterpret_cast<OutT *>(s_raw);
+    uint4 *tx = reinterpret_cast<uint4 *>(s_raw + 768 * sizeof(OutT)), *ty = tx + out_w;
+    OutT *s_out = reinterpret_cast<OutT *>(ty + out_h);
+    const size_t tile_row = (size_t)out_w * 3 * sizeof(OutT);
 
     const int i = blockIdx.y;
     if (blockIdx.x == 0 && i == 0)
@@ -273,21 +316,23 @@ resize_augment_kernel(const __grid_constant__ ResizeSource src, const int32_t *_
     // The scale factors (four double-precision divisions) are worked out by one thread, and so are the
     // conversion units of a window row and the number of output rows whose source rows fit the window.
     __shared__ Scaling s_scaling;
-    __shared__ int s_window, s_units, s_lead;
+    __shared__ int s_window, s_units, s_lead, s_groups;
     __shared__ uint32_t s_inv_units;
     if (threadIdx.x == 0 && ok) {
         s_scaling = scaling_of(ch, cw, out_h, out_w);
         const bool fits = s_scaling.regime == kArea || s_scaling.regime == kLinear;
-        s_window = fuse ? fuse : (fits ? window_band(cw, s_scaling.sc_y, shape.band, shape.win) : 0);
+        s_window = fuse ? fuse : (fits ? window_band(cw, s_scaling.sc_y, tile_row, shape) : 0);
         const bool quad = fuse && src.descs[i].scale_shift == 0 && src.descs[i].hs == 2;
         s_lead = fuse ? (quad ? cj & 7 : cj & 3) : 0; // a unit begins at a multiple of its width
         s_units = quad ? (s_lead + cw + 7) / 8 : (s_lead + cw + 3) / 4;
         s_inv_units = inverse(s_units);
+        s_groups = row_groups(out_w, s_window ? s_window : shape.band);
     }
     __syncthreads();
     int regime = kCopy, isx = 1, isy = 1;
     const int window = ok ? s_window : 0, band_rows = window ? window : shape.band;
-    const int lead = ok ? s_lead : 0, wpitch = window_pitch(cw);
+    const int lead = ok ? s_lead : 0, wpitch = window_pitch(cw), groups = ok ? s_groups : 1;
+    uint32_t *s_win = reinterpret_cast<uint32_t *>(reinterpret_cast<unsigned char *>(s_out) + (((size_t)band_rows * tile_row + 15) & ~(size_t)15));
     const int nbands = (out_h + band_rows - 1) / band_rows;
     if ((int)blockIdx.x >= nbands) return;
     if (ok) {
@@ -446,23 +491,24 @@ resize_augment_kernel(const __grid_constant__ ResizeSource src, const int32_t *_
                 if (regime == kArea) {
                     const AreaColumn column(taps);
                     int pj = -1; // source row whose horizontal sums are held
-                    float p[3] = {0.f, 0.f, 0.f};
+                    Two rg(0.f, 0.f);
+                    float b = 0.f;
                     for (int y = begin; y < end; y++, o += row_step) {
                         const uint4 c = ty[y];
                         const int yf = (int)(c.x & 0xffff), ye = yf + (int)(c.x >> 16) - 1;
                         // only the first source row can be the one the previous output row ended with
-                        if (yf != pj) column.across(row_of(yf), p);
+                        if (yf != pj) column.across(row_of(yf), rg, b);
                         float beta = __uint_as_float(c.y);
-                        float a0 = __fmul_rn(beta, p[0]), a1 = __fmul_rn(beta, p[1]), a2 = __fmul_rn(beta, p[2]);
+                        Two sum_rg = mul_rn(Two(beta, beta), rg);
+                        float sum_b = __fmul_rn(beta, b);
                         for (int j = yf + 1; j <= ye; j++) {
-                            column.across(row_of(j), p);
+                            column.across(row_of(j), rg, b);
                             beta = __uint_as_float(j == ye ? c.w : c.z);
-                            a0 = __fadd_rn(a0, __fmul_rn(beta, p[0]));
-                            a1 = __fadd_rn(a1, __fmul_rn(beta, p[1]));
-                            a2 = __fadd_rn(a2, __fmul_rn(beta, p[2]));
+                            sum_rg = add_rn(sum_rg, mul_rn(Two(beta, beta), rg));
+                            sum_b = __fadd_rn(sum_b, __fmul_rn(beta, b));
                         }
                         pj = ye;
-                        emit(o, round_byte(a0), round_byte(a1), round_byte(a2));
+                        emit(o, round_byte(sum_rg.lo()), round_byte(sum_rg.hi()), round_byte(sum_b));
                     }
                 } else {
                     const LinearColumn column(taps);
@@ -485,10 +531,9 @@ resize_augment_kernel(const __grid_constant__ ResizeSource src, const int32_t *_
                             column.across(row_of(r1), hb);
                             rb = r1;
                         }
-                        const float b0 = __uint_as_float(c.z), b1 = __uint_as_float(c.w);
-                        const float k0 = __fmaf_rn(b0, -134217728.f, 8796093022208.f), k1 = __fmaf_rn(b1, -134217728.f, 8796093022208.f);
-                        emit(o, blend_rows(ha[0], hb[0], b0, k0, b1, k1), blend_rows(ha[1], hb[1], b0, k0, b1, k1),
-                             blend_rows(ha[2], hb[2], b0, k0, b1, k1));
+                        const Two b(__uint_as_float(c.z), __uint_as_float(c.w));
+                        const Two k = fma_rn(b, Two(-134217728.f, -134217728.f), Two(8796093022208.f, 8796093022208.f));
+                        emit(o, blend_rows(ha[0], hb[0], b, k), blend_rows(ha[1], hb[1], b, k), blend_rows(ha[2], hb[2], b, k));
                     }
                 }
             }
@@ -561,36 +606,25 @@ resize_augment_kernel(const __grid_constant__ ResizeSource src, const int32_t *_
     }
 }
 
-ResizeShape resize_shape(int out_h, int out_w, int out_kind) {
+ResizeShape resize_shape(int n, int out_h, int out_w, int out_kind) {
     const size_t elem = out_kind == kOutU8 ? 1 : (out_kind == kOutF16Nhwc || out_kind == kOutF16Nchw ? 2 : 4);
     ResizeShape s{};
+    const size_t fixed = 768 * elem + sizeof(uint4) * ((size_t)out_w + out_h), row = (size_t)out_w * 3 * elem;
+    // without a window: about 2048 pixels per band
     int band = (2048 + out_w - 1) / out_w;
-    if (band < 1) band = 1;
     if (band > out_h) band = out_h;
-    auto smem_for = [&](int b) {
-        return (((size_t)b * out_w * 3 * elem + 15) & ~(size_t)15) + ((768 * elem + 15) & ~(size_t)15) + sizeof(uint4) * ((size_t)out_w + out_h);
-    };
-    while (band > 1 && smem_for(band) > 200 * 1024) band /= 2;
-    // window of source pixels: what is left of a quarter of the SM's shared memory (four resident
-    // CTAs of 256 threads is what the registers allow), at most 40 KiB
-    const size_t quarter = (227 * 1024) / 4 - 1024;
-    size_t win = smem_for(band) + 4096 <= quarter ? quarter - smem_for(band) : 0;
-    if (win > 40 * 1024) win = 40 * 1024;
-    s.win = win & ~(size_t)15;
-    s.smem = smem_for(band) + s.win;
+    while (band > 1 && fixed + band * row > 200 * 1024) band /= 2;
     s.band = band;
-    // column paths: the band's rows are dealt to `groups` runs per column so that
-    // the (column, run) items fill the CTA's 256 threads evenly, with runs of at least 3 rows
-    s.groups = 1;
-    double best = 0;
-    for (int g = 1; g <= 4 && (band + g - 1) / g >= 3; g++) {
-        const int items = g * out_w;
-        const double use = (double)items / (((items + 255) / 256) * 256);
-        if (use > best + 1e-9) {
-            best = use;
-            s.groups = g;
-        }
-    }
+    // With one: as many rows (up to 5120 pixels) as fit, with their window, in a quarter of the SM's shared memory; four
+    // resident CTAs of 256 threads is what the registers allow.  Small batches get bands enough for all SMs.
+    s.max_band = (5120 + out_w - 1) / out_w;
+    const int64_t spread = (int64_t)out_h * n / (148 * 4);
+    if (spread < s.max_band) s.max_band = spread < 4 ? 4 : (int)spread;
+    if (s.max_band > out_h) s.max_band = out_h;
+    const size_t quarter = (227 * 1024) / 4 - 1024;
+    s.room = quarter > fixed ? (quarter - fixed) & ~(size_t)15 : 0;
+    const size_t tile = (band * row + 15) & ~(size_t)15;
+    s.smem = fixed + (s.room > tile ? s.room : tile);
     return s;
 }
 
@@ -603,7 +637,7 @@ static void launch_typed(const ResizeSource &src, int n, const int32_t *params, 
     // CTAs per image: enough of them for about eight waves of the GPU (148 SMs x 4 resident CTAs;
     // fewer waves measured slower, more cost the set-up its amortisation), at most one per band (a sample
     // whose window holds fewer rows has more of them, of at least four rows)
-    const int least = shape.band > 4 ? 4 : shape.band, nbands = (out_h + least - 1) / least;
+    const int least = shape.room && shape.band > 4 ? 4 : shape.band, nbands = (out_h + least - 1) / least;
     int per_image = (8 * 148 * 4 + n - 1) / n;
     if (per_image > nbands) per_image = nbands;
     if (per_image < 1) per_image = 1;
@@ -617,7 +651,7 @@ void launch_resize_augment(const ResizeSource &src, int n, const int32_t *params
                            const void *lut, void *out, const int32_t *status, const SmallCopies &small, cudaStream_t stream) {
     if (n <= 0) return;
     const int planar = out_kind == kOutF16Nchw || out_kind == kOutF32Nchw;
-    const ResizeShape shape = resize_shape(out_h, out_w, out_kind);
+    const ResizeShape shape = resize_shape(n, out_h, out_w, out_kind);
     if (out_kind == kOutU8)
         launch_typed<uint8_t>(src, n, params, n_params, ops, resize, out_h, out_w, 0, shape, nullptr, out, status, small, stream);
     else if (out_kind == kOutF16Nhwc || out_kind == kOutF16Nchw)
