@@ -1106,9 +1106,12 @@ scan_restart_kernel(const ImageDesc *__restrict__ descs, const int32_t *__restri
 } // namespace
 
 uint32_t subseq_target(uint64_t total_bits) {
-    // About 1024 subsequences per SM: enough of them that the chain of look-ups is hidden, no more than
-    // that, because every one costs a re-synchronisation (0.9 kbit) on top of its own length.
-    const uint64_t t = total_bits / (148 * 1024);
+    // A subsequence costs a re-synchronisation (0.9 kbit, 0.35 without subsampling) on top of its own length, so
+    // long ones are less work; short ones are a shorter chain, which decides while few bits leave the GPU
+    // mostly idle.  256 subsequences per SM are enough of them: batches of 80 Mbit, alone / four in flight, take
+    // 473 / 335 us at 512 bits, 424 / 274 at 1024, 388 / 255 at 1280; a 4:4:4 scan of 24 Mbit 554 us at 256 bits,
+    // 505 at 512, 499 at 768, 509 at 1024.
+    const uint64_t t = total_bits / (148 * 256);
     return (uint32_t)(t < 256 ? 256 : (t > kMaxSubseqBits ? kMaxSubseqBits : (t + 31) / 32 * 32));
 }
 

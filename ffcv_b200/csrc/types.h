@@ -16,6 +16,7 @@ constexpr int kPayloadAlign = 16;
 constexpr int kSegSubs = 128;
 constexpr int kSegOverlap = 512;
 constexpr int kMaxSubseqBits = 1280; // longest subsequence: bounds a segment's shared memory
+static_assert(kSegSubs * kMaxSubseqBits + 8 * kSegOverlap < 1 << 18, "a position inside a segment has 18 bits");
 // Few scans are decoded from every possible block slot at once (scan_slots_kernel): segments of up to
 // kSlotSubs subsequences of kSlotBits bits, each with up to kSlotStates entry states; the last place is kept
 // for a state that was not found in time.
