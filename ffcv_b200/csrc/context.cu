@@ -1522,6 +1522,7 @@ static int run_batch(ffcvb_ctx *ctx, Slot &s, cudaStream_t st, void *out_dev, bo
     const int32_t *params = reinterpret_cast<const int32_t *>(blob + hd.params_off);
     int32_t *status = single ? single->status : reinterpret_cast<int32_t *>(blob + s.status_off);
     uint8_t *rgb = single ? single->rgb : (uint8_t *)s.rgb.p;
+    bool early = false;
     if (s.n_jpeg > 0) {
         const int32_t *jl = reinterpret_cast<const int32_t *>(blob + s.jpeg_list_off);
         EntropyScratch scratch{};
@@ -1539,15 +1540,16 @@ static int run_batch(ffcvb_ctx *ctx, Slot &s, cudaStream_t st, void *out_dev, bo
         scratch.done = (uint32_t *)(blob + s.status_off) + s.n;
         scratch.pos = (uint32_t *)s.index.p;
         scratch.dc = (int16_t *)(scratch.pos + s.total_blocks);
+        early = work.early() && !prof;
         launch_entropy_decode(descs, work, blob, huff, scratch, status, (uint8_t *)ctx->index_pool.p,
                               (unsigned long long *)ctx->index_stats.p, st);
         if (prof) CU(cudaEventRecord(s.ev[2], st));
         launch_blocks(descs, reinterpret_cast<const uint2 *>(blob + s.block_tiles_off), s.n_block_tiles, huff, mult, scratch,
-                      (uint8_t *)s.planes.p, st);
+                      (uint8_t *)s.planes.p, early, st);
         if (prof) CU(cudaEventRecord(s.ev[3], st));
         launch_color(descs, jl, s.n_jpeg, s.n_quad, s.n_444, s.n_other, s.max_w, s.max_h,
                      reinterpret_cast<const uint2 *>(blob + s.quad_tiles_off), s.n_quad_tiles, (const uint8_t *)s.planes.p,
-                     rgb, s.plan.resize ? params : nullptr, (int)hd.n_params, st);
+                     rgb, s.plan.resize ? params : nullptr, (int)hd.n_params, early, st);
         if (prof) CU(cudaEventRecord(s.ev[4], st));
     } else if (prof) {
         for (int k = 2; k <= 4; k++) CU(cudaEventRecord(s.ev[k], st));
@@ -1568,7 +1570,8 @@ static int run_batch(ffcvb_ctx *ctx, Slot &s, cudaStream_t st, void *out_dev, bo
         src.rgb = rgb;
         src.planes = (const uint8_t *)s.planes.p;
         launch_resize_augment(src, s.n, params, (int)hd.n_params, make_oplist(s.plan), s.plan.resize,
-                              s.plan.out_h, s.plan.out_w, s.plan.out_kind, s.plan.lut_dev, out_dev, status, small, st);
+                              s.plan.out_h, s.plan.out_w, s.plan.out_kind, s.plan.lut_dev, out_dev, status, small,
+                              early && !outputs_free, st);
     }
     CU(cudaGetLastError());
     if (prof) {
@@ -1821,7 +1824,7 @@ int ffcvb_transform_device(ffcvb_ctx *ctx, void *stream, const uint8_t *src_dev,
     src.uniform_h = h;
     src.uniform_w = w;
     launch_resize_augment(src, n, (const int32_t *)a.dev.p, n_params, make_oplist(*plan), plan->resize,
-                          plan->out_h, plan->out_w, plan->out_kind, plan->lut_dev, out_dev, nullptr, SmallCopies{}, st);
+                          plan->out_h, plan->out_w, plan->out_kind, plan->lut_dev, out_dev, nullptr, SmallCopies{}, false, st);
     CU(cudaGetLastError());
     CU(cudaEventRecord(a.ev, st));
     a.used = true;
@@ -2107,7 +2110,7 @@ void resize(int64_t cresizer, int64_t source_p, int64_t sx, int64_t sy, int64_t 
     rs.uniform_h = rows;
     rs.uniform_w = cols;
     uint8_t *out = zero_copy ? ctx->one_host + kResultHead : (uint8_t *)ctx->one_dst.p;
-    launch_resize_augment(rs, 1, (const int32_t *)ctx->one_src.p, 4, OpList{}, 1, (int)tx, (int)ty, FFCVB_OUT_U8_NHWC, nullptr, out, nullptr, SmallCopies{}, st);
+    launch_resize_augment(rs, 1, (const int32_t *)ctx->one_src.p, 4, OpList{}, 1, (int)tx, (int)ty, FFCVB_OUT_U8_NHWC, nullptr, out, nullptr, SmallCopies{}, false, st);
     if (cudaGetLastError() != cudaSuccess) return;
     if (zero_copy) {
         if (cudaStreamSynchronize(st) == cudaSuccess) memcpy((void *)(intptr_t)dest_p, out, dst_bytes);

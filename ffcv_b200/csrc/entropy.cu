@@ -393,6 +393,7 @@ scan_sync_kernel(const ImageDesc *__restrict__ descs, const uint2 *__restrict__ 
                  unsigned long long *__restrict__ index_stats, int table_slots, uint32_t buf_bytes) {
     extern __shared__ __align__(16) unsigned char s_dyn[];
     __shared__ SyncShared s_teams[TEAMS];
+    next_may_begin();
     const Team<TEAMS> team;
     const int tid = team.tid;
     SyncShared &sh = s_teams[team.index];
@@ -496,6 +497,8 @@ scan_sync_kernel(const ImageDesc *__restrict__ descs, const uint2 *__restrict__ 
 __global__ void __launch_bounds__(kThreads)
 scan_stitch_kernel(const ImageDesc *__restrict__ descs, const int32_t *__restrict__ list, const HuffTable *__restrict__ huff,
                    EntropyScratch scratch) {
+    next_may_begin();
+    await_previous();
     const ImageDesc &d = descs[list[blockIdx.x]];
     const int tid = threadIdx.x, n_seg = (int)d.seg_count;
     const uint32_t S = d.subseq_bits;
@@ -579,6 +582,8 @@ scan_slots_kernel(const ImageDesc *__restrict__ descs, const uint2 *__restrict__
                   const HuffTable *__restrict__ huff, EntropyScratch scratch, int table_slots) {
     extern __shared__ __align__(16) unsigned char s_dyn[];
     __shared__ __align__(16) SlotShared sh;
+    next_may_begin();
+    await_previous();
     const Team<1, kSlotThreads> team;
     const int tid = team.tid;
     Tables *tables = reinterpret_cast<Tables *>(s_dyn);
@@ -720,6 +725,8 @@ scan_chain_kernel(const ImageDesc *__restrict__ descs, const int32_t *__restrict
     __shared__ uint32_t s_entry[kChainThreads / 32 + 1];
     __shared__ SlotMap s_run[kChainThreads / 32][kSlotStates]; // (state, or kNoState; state behind the run)
     __shared__ uint8_t s_done[kChainThreads / 32];
+    next_may_begin();
+    await_previous();
     const ImageDesc &d = descs[list[blockIdx.x]];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, n_seg = (int)d.seg_count;
     SlotTables *tabs = scratch.slots + (d.slots - 1);
@@ -833,6 +840,7 @@ scan_index_kernel(const ImageDesc *__restrict__ descs, const uint2 *__restrict__
     extern __shared__ __align__(16) unsigned char s_dyn[];
     __shared__ int s_warps[TEAMS][kThreads / 32];
     __shared__ uint32_t s_lasts[TEAMS];
+    next_may_begin();
     const Team<TEAMS> team;
     const int tid = team.tid;
     int *s_warp = s_warps[team.index];
@@ -845,6 +853,7 @@ scan_index_kernel(const ImageDesc *__restrict__ descs, const uint2 *__restrict__
     const uint32_t j = which.y;
     const ImageDesc &d = descs[img];
     load_tables(tables, d, huff);
+    await_previous();
     if (TEAMS > 1) {
         copies_wait();
         __syncthreads();
@@ -1157,6 +1166,7 @@ void launch_entropy_decode(const ImageDesc *descs, const EntropyWork &work, cons
     if (n_segs > 0) {
         const uint32_t buf = (uint32_t)stream_bytes(work.max_raw);
         const int tables = work.max_tables;
+        const bool early = work.early();
         auto allow = [](auto kernel, size_t smem) { cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); };
         // With enough segments to fill every SM four teams share a set of tables: eight segments of up to
         // 22 KB fit an SM then, instead of five.
@@ -1169,12 +1179,12 @@ void launch_entropy_decode(const ImageDesc *descs, const EntropyWork &work, cons
                 kernel<<<grid, kThreads * teams, smem, stream>>>(descs, work.segs, work.n_guess, blob, huff, scratch, index_pool, index_stats, tables, buf);
             };
             if (teams == 4) run(scan_sync_kernel<4>); else run(scan_sync_kernel<1>);
-            if (work.n_multi > 0) scan_stitch_kernel<<<work.n_multi, kThreads, 0, stream>>>(descs, work.multi, huff, scratch);
+            if (work.n_multi > 0) launch(early, work.n_multi, kThreads, 0, stream, scan_stitch_kernel, descs, work.multi, huff, scratch);
         }
         if (work.n_slots > 0) {
             const size_t one = tables_bytes(tables) + buf;
             allow(scan_slots_kernel, one);
-            scan_slots_kernel<<<work.n_slots, kSlotThreads, one, stream>>>(descs, work.segs + work.n_guess, blob, huff, scratch, tables);
+            launch(early && work.n_guess > 0, work.n_slots, kSlotThreads, one, stream, scan_slots_kernel, descs, work.segs + work.n_guess, blob, huff, scratch, tables);
             // As many runs as segments in each: both are followed one after the other.  The maps fit
             // shared memory up to 1500 segments (6 MB of scan).
             int warps = 1;
@@ -1183,12 +1193,12 @@ void launch_entropy_decode(const ImageDesc *descs, const EntropyWork &work, cons
             const int slots = work.max_slot_segs < 1500 ? work.max_slot_segs : 1500;
             const size_t maps = (size_t)slots * kSlotStates * sizeof(SlotMap);
             allow(scan_chain_kernel, maps);
-            scan_chain_kernel<<<work.n_slot_images, warps * 32, maps, stream>>>(descs, work.slot_images, huff, scratch, slots);
+            launch(early, work.n_slot_images, warps * 32, maps, stream, scan_chain_kernel, descs, work.slot_images, huff, scratch, slots);
         }
         auto run = [&](auto kernel) {
             allow(kernel, smem);
-            kernel<<<(n_segs + teams - 1) / teams, kThreads * teams, smem, stream>>>(descs, work.segs, n_segs, huff, scratch, status, index_pool,
-                                                                                  index_stats, tables, buf);
+            launch(early, (n_segs + teams - 1) / teams, kThreads * teams, smem, stream, kernel, descs, work.segs, n_segs, huff, scratch, status, index_pool,
+                   index_stats, tables, buf);
         };
         if (teams == 4) run(scan_index_kernel<4>); else run(scan_index_kernel<1>);
     }

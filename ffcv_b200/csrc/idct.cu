@@ -128,6 +128,7 @@ blocks_kernel(const ImageDesc *__restrict__ descs, const uint2 *__restrict__ til
     __shared__ __align__(16) uint32_t s_coef[32][kBlockTile];
     __shared__ __align__(16) uint16_t s_look[2][kLook]; // AC tables of luma and of the first chroma component
     __shared__ int16_t s_mult[3][64];
+    next_may_begin();
     const uint2 tile = tiles[blockIdx.x];
     const ImageDesc &d = descs[tile.x];
     const int tid = threadIdx.x;
@@ -144,6 +145,7 @@ blocks_kernel(const ImageDesc *__restrict__ descs, const uint2 *__restrict__ til
         for (int k = tid; k < 64 * d.ncomp; k += kBlockTile)
             s_mult[k >> 6][k & 63] = scaled && (k < 64 || d.bs_chroma != 8) ? (int16_t)1 : mult[d.q_tab[k >> 6]].m[k & 63];
     }
+    await_previous();
     __syncthreads();
     int item = (int)tile.y * kBlockTile + tid, comp = 0, bx, by, plane_w, bs;
     uint32_t blk;
@@ -245,8 +247,8 @@ blocks_kernel(const ImageDesc *__restrict__ descs, const uint2 *__restrict__ til
 }
 
 void launch_blocks(const ImageDesc *descs, const uint2 *tiles, int n_tiles, const HuffTable *huff, const MultTable *mult,
-                   const EntropyScratch &scratch, uint8_t *planes, cudaStream_t stream) {
-    if (n_tiles > 0) blocks_kernel<<<n_tiles, kBlockTile, 0, stream>>>(descs, tiles, huff, mult, scratch, planes);
+                   const EntropyScratch &scratch, uint8_t *planes, bool early, cudaStream_t stream) {
+    if (n_tiles > 0) launch(early, n_tiles, kBlockTile, 0, stream, blocks_kernel, descs, tiles, huff, mult, scratch, planes);
 }
 
 // ------------------------------------------------------------------------------------------
@@ -335,6 +337,8 @@ __global__ void __launch_bounds__(128)
 color_quad_kernel(const ImageDesc *__restrict__ descs, const int32_t *__restrict__ list,
                   const uint2 *__restrict__ tiles, const uint8_t *__restrict__ planes, uint8_t *__restrict__ rgb,
                   const int32_t *__restrict__ params, int n_params) {
+    next_may_begin();
+    await_previous();
     // which sample and which tile of 64 x 8 chroma samples of its box: from the batch's tile table
     // (one CTA per tile that exists), or, without a table, from a grid that covers the largest box
     int img, tile_x, tile_y;
@@ -383,6 +387,8 @@ __global__ void __launch_bounds__(256)
 color_444_kernel(const ImageDesc *__restrict__ descs, const int32_t *__restrict__ list,
                  const uint8_t *__restrict__ planes, uint8_t *__restrict__ rgb,
                  const int32_t *__restrict__ params, int n_params) {
+    next_may_begin();
+    await_previous();
     const int img = list[blockIdx.z];
     const ImageDesc &d = descs[img];
     if (d.host_status != 0 || d.ncomp != 3 || !(d.scale_shift != 0 || (d.hs == 1 && d.vs == 1)) || d.fuse_rows) return;
@@ -410,6 +416,8 @@ color_444_kernel(const ImageDesc *__restrict__ descs, const int32_t *__restrict_
 __global__ void __launch_bounds__(256)
 color_other_kernel(const ImageDesc *__restrict__ descs, const int32_t *__restrict__ list,
                    const uint8_t *__restrict__ planes, uint8_t *__restrict__ rgb) {
+    next_may_begin();
+    await_previous();
     const ImageDesc &d = descs[list[blockIdx.y]];
     if (d.host_status != 0) return;
     const int W = d.width, H = d.height;
@@ -443,25 +451,25 @@ color_other_kernel(const ImageDesc *__restrict__ descs, const int32_t *__restric
 
 void launch_color(const ImageDesc *descs, const int32_t *list, int n_list, int n_quad, int n_444, int n_other,
                   int max_w, int max_h, const uint2 *quad_tiles, int n_quad_tiles, const uint8_t *planes, uint8_t *rgb, const int32_t *crop_params,
-                  int n_params, cudaStream_t stream) {
+                  int n_params, bool early, cudaStream_t stream) {
     if (n_list == 0) return;
     if (n_444 > 0) {
         int gy = (max_h + 7) / 8;
         if (gy > 64) gy = 64;
         dim3 grid(((max_w + 3) / 4 + 1 + 31) / 32, gy, n_list); // + 1: a box starts up to 3 pixels into its first group
-        color_444_kernel<<<grid, dim3(32, 8), 0, stream>>>(descs, list, planes, rgb, crop_params, n_params);
+        launch(early, grid, dim3(32, 8), 0, stream, color_444_kernel, descs, list, planes, rgb, crop_params, n_params);
     }
     if (n_quad > 0 && quad_tiles != nullptr) {
         if (n_quad_tiles > 0)
-            color_quad_kernel<<<n_quad_tiles, dim3(16, 8), 0, stream>>>(descs, list, quad_tiles, planes, rgb, crop_params,
-                                                                        n_params);
+            launch(early, n_quad_tiles, dim3(16, 8), 0, stream, color_quad_kernel, descs, list, quad_tiles, planes, rgb, crop_params, n_params);
     } else if (n_quad > 0) {
-        color_quad_kernel<<<dim3(quad_tiles_x(max_w), quad_tiles_y(max_h), n_list), dim3(16, 8), 0, stream>>>(descs, list, nullptr, planes, rgb, crop_params, n_params);
+        launch(early, dim3(quad_tiles_x(max_w), quad_tiles_y(max_h), n_list), dim3(16, 8), 0, stream, color_quad_kernel, descs, list, nullptr, planes, rgb,
+               crop_params, n_params);
     }
     if (n_other > 0) {
         int bx = (max_w * max_h + 256 * 4 - 1) / (256 * 4);
         bx = bx < 1 ? 1 : (bx > 1024 ? 1024 : bx);
-        color_other_kernel<<<dim3(bx, n_list), 256, 0, stream>>>(descs, list, planes, rgb);
+        launch(early, dim3(bx, n_list), 256, 0, stream, color_other_kernel, descs, list, planes, rgb);
     }
 }
 

@@ -16,6 +16,32 @@ namespace ffcvb {
 constexpr int kGatherCtas = 148;
 void launch_gather_payloads(const ImageDesc *descs, int n, uint8_t *blob, int ctas, int32_t *failed, cudaStream_t stream);
 
+// The kernels of a small batch follow one another early: each is launched as soon as all CTAs of the one before
+// have begun (next_may_begin, first thing), fetches its tables and then waits in hardware for the one before to
+// end (await_previous, by every CTA before it reads or writes anything of the batch's, so that the end of the last
+// kernel means the end of all).  Only where the batch leaves SMs free: waiting CTAs hold shared memory and
+// registers that a large batch's neighbours on other streams need.  Per call: one
+// image of 100x133 pixels 103 -> 90 us, 224x256 116 -> 105, 900x1200 286 -> 275; 16 requests 144.4 -> 141.4.
+constexpr int kEarlySegments = 2 * 148;
+#if defined(__CUDACC__)
+__device__ __forceinline__ void next_may_begin() { asm volatile("griddepcontrol.launch_dependents;"); }
+__device__ __forceinline__ void await_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+template <class... P, class... A>
+void launch(bool early, dim3 grid, dim3 block, size_t smem, cudaStream_t stream, void (*kernel)(P...), A... args) {
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t config{};
+    config.gridDim = grid;
+    config.blockDim = block;
+    config.dynamicSmemBytes = smem;
+    config.stream = stream;
+    config.attrs = &attr;
+    config.numAttrs = early ? 1 : 0;
+    cudaLaunchKernelEx(&config, kernel, P(args)...);
+}
+#endif
+
 // Scratch and results of the entropy decode of a batch (device memory, no initialisation needed
 // except `done`, which starts at zero once and is left at zero).
 struct EntropyScratch {
@@ -43,6 +69,7 @@ struct EntropyWork {
     int max_tables;        // bounds the tables of a sample in shared memory (its distinct DC tables and twice its AC tables)
     int max_slot_segs;     // most segments of one of slot_images
     bool alike;            // all samples in segs have the same tables and layout of an MCU
+    bool early() const { return n_restart == 0 && n_guess + n_slots > 0 && n_guess + n_slots <= kEarlySegments; } // see kEarlySegments
 };
 
 // Entropy decode: finds every block of the listed scans.  status[sample] is set for every listed
@@ -78,7 +105,7 @@ FFCVB_HD inline uint32_t block_tiles(const ImageDesc &d) {
     return (luma + 2 * chroma + kBlockTile - 1) / kBlockTile;
 }
 void launch_blocks(const ImageDesc *descs, const uint2 *tiles, int n_tiles, const HuffTable *huff, const MultTable *mult,
-                   const EntropyScratch &scratch, uint8_t *planes, cudaStream_t stream);
+                   const EntropyScratch &scratch, uint8_t *planes, bool early, cudaStream_t stream);
 
 // Chroma upsampling (triangle filter) + YCbCr->RGB into h*w*3 images in `rgb` (rows rgb_pitch
 // apart).  4:2:0 images (n_quad of them) go through the quad kernel and 4:4:4 images (n_444)
@@ -89,7 +116,7 @@ void launch_blocks(const ImageDesc *descs, const uint2 *tiles, int n_tiles, cons
 // convert, so that it launches exactly those CTAs instead of a grid over the largest box.
 void launch_color(const ImageDesc *descs, const int32_t *list, int n_list, int n_quad, int n_444, int n_other,
                   int max_w, int max_h, const uint2 *quad_tiles, int n_quad_tiles, const uint8_t *planes,
-                  uint8_t *rgb, const int32_t *crop_params, int n_params, cudaStream_t stream);
+                  uint8_t *rgb, const int32_t *crop_params, int n_params, bool early, cudaStream_t stream);
 
 // Tiles of 64 x 8 chroma samples that cover a box of bw x bh pixels wherever it begins (a thread converts four
 // samples of a row, beginning at a multiple of four).
@@ -161,7 +188,7 @@ struct SmallCopies {
 // Fused crop + INTER_AREA resize + flip/translate/cutout + lookup-table normalise.
 void launch_resize_augment(const ResizeSource &src, int n, const int32_t *params, int n_params,
                            const OpList &ops, int resize, int out_h, int out_w, int out_kind,
-                           const void *lut, void *out, const int32_t *status, const SmallCopies &small, cudaStream_t stream);
+                           const void *lut, void *out, const int32_t *status, const SmallCopies &small, bool early, cudaStream_t stream);
 
 // Colour jitter kinds (ffcv/transforms/color_jitter.py).
 enum { kJitterBrightness = 0, kJitterContrast = 1, kJitterSaturation = 2 };

@@ -237,6 +237,7 @@ resize_augment_kernel(const __grid_constant__ ResizeSource src, const int32_t *_
                       const OutT *__restrict__ lut, OutT *__restrict__ out,
                       const int32_t *__restrict__ status, const __grid_constant__ SmallCopies small) {
     extern __shared__ __align__(16) unsigned char s_raw[];
+    await_previous();
     constexpr bool kU8 = sizeof(OutT) == 1;
     // shared layout: [lut][x taps][y taps][out tile][window of source pixels]; y taps are indexed by the row of
     // the resized crop (a translation can move a band anywhere)
@@ -631,7 +632,7 @@ ResizeShape resize_shape(int n, int out_h, int out_w, int out_kind) {
 template <typename OutT>
 static void launch_typed(const ResizeSource &src, int n, const int32_t *params, int n_params, const OpList &ops,
                          int resize, int out_h, int out_w, int planar, const ResizeShape &shape, const void *lut, void *out,
-                         const int32_t *status, const SmallCopies &small, cudaStream_t stream) {
+                         const int32_t *status, const SmallCopies &small, bool early, cudaStream_t stream) {
     auto kern = resize_augment_kernel<OutT>;
     if (shape.smem > 48 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shape.smem);
     // CTAs per image: enough of them for about eight waves of the GPU (148 SMs x 4 resident CTAs;
@@ -642,22 +643,22 @@ static void launch_typed(const ResizeSource &src, int n, const int32_t *params, 
     if (per_image > nbands) per_image = nbands;
     if (per_image < 1) per_image = 1;
     dim3 grid(per_image, n);
-    kern<<<grid, 256, shape.smem, stream>>>(src, params, n_params, ops, resize, out_h, out_w, shape, planar,
-                                            (const OutT *)lut, (OutT *)out, status, small);
+    launch(early, grid, 256, shape.smem, stream, kern, src, params, n_params, ops, resize, out_h, out_w, shape, planar, (const OutT *)lut, (OutT *)out,
+           status, small);
 }
 
 void launch_resize_augment(const ResizeSource &src, int n, const int32_t *params, int n_params,
                            const OpList &ops, int resize, int out_h, int out_w, int out_kind,
-                           const void *lut, void *out, const int32_t *status, const SmallCopies &small, cudaStream_t stream) {
+                           const void *lut, void *out, const int32_t *status, const SmallCopies &small, bool early, cudaStream_t stream) {
     if (n <= 0) return;
     const int planar = out_kind == kOutF16Nchw || out_kind == kOutF32Nchw;
     const ResizeShape shape = resize_shape(n, out_h, out_w, out_kind);
     if (out_kind == kOutU8)
-        launch_typed<uint8_t>(src, n, params, n_params, ops, resize, out_h, out_w, 0, shape, nullptr, out, status, small, stream);
+        launch_typed<uint8_t>(src, n, params, n_params, ops, resize, out_h, out_w, 0, shape, nullptr, out, status, small, early, stream);
     else if (out_kind == kOutF16Nhwc || out_kind == kOutF16Nchw)
-        launch_typed<uint16_t>(src, n, params, n_params, ops, resize, out_h, out_w, planar, shape, lut, out, status, small, stream);
+        launch_typed<uint16_t>(src, n, params, n_params, ops, resize, out_h, out_w, planar, shape, lut, out, status, small, early, stream);
     else
-        launch_typed<uint32_t>(src, n, params, n_params, ops, resize, out_h, out_w, planar, shape, lut, out, status, small, stream);
+        launch_typed<uint32_t>(src, n, params, n_params, ops, resize, out_h, out_w, planar, shape, lut, out, status, small, early, stream);
 }
 
 } // namespace ffcvb

@@ -198,11 +198,11 @@ extern "C" int ffcvb_imdecode_static(const uint8_t *jpeg_host, uint64_t jpeg_siz
     work.max_raw = kSegSubs * d.subseq_bits / 8 + kSegOverlap;
     work.max_tables = 3 * d.n_dc_tab;
     launch_entropy_decode(desc_dev, work, jpeg_dev, meta_dev->huff, es, meta_dev->status, nullptr, nullptr, st);
-    launch_blocks(desc_dev, meta_dev->tiles, (int)n_tiles, meta_dev->huff, meta_dev->mult, es, scratch + kPlaneOff, st);
+    launch_blocks(desc_dev, meta_dev->tiles, (int)n_tiles, meta_dev->huff, meta_dev->mult, es, scratch + kPlaneOff, work.early(), st);
     const bool quad = d.ncomp == 3 && d.hs == 2 && d.vs == 2 && (width + 1) / 2 >= 3;
     const bool full = d.ncomp == 3 && d.hs == 1 && d.vs == 1;
     launch_color(desc_dev, list_dev, 1, quad ? 1 : 0, full ? 1 : 0, (quad || full) ? 0 : 1, (int)width, (int)height,
-                 nullptr, 0, scratch + kPlaneOff, rgb_dev, nullptr, 0, st);
+                 nullptr, 0, scratch + kPlaneOff, rgb_dev, nullptr, 0, work.early(), st);
     if (cudaGetLastError() != cudaSuccess) return reject(FFCVB_E_CUDA, "kernel launch failed");
     return FFCVB_OK;
 }

@@ -150,3 +150,28 @@ def test_few_large_scans(h, w, quality, subseq_bits, monkeypatch):
     for k, b in enumerate(bufs):
         assert np.array_equal(got[k], O.jpeg_decode(b)), k
     ctx.close()
+
+
+@pytest.mark.parametrize('n', [1, 2, 296, 297])
+def test_batches_whose_kernels_begin_early(n):
+    """Up to 296 segments every kernel is launched while the one before runs.  Both ways of decoding in a batch,
+    and batches behind one another in the same slot and buffers."""
+    from ffcv_b200 import libffcv as L
+    rng = np.random.default_rng(n)
+    h, w = 40, 56
+    ctx = L.Context(0, 1, 2)
+    stream = ch.cuda.current_stream().cuda_stream
+    outs, wants = [], []
+    for b in range(4):
+        bufs = [_jpeg(rng, h, w, int(rng.integers(60, 98)), 444 if k % 3 == 1 else 420) for k in range(n)]
+        sizes = np.array([b.size for b in bufs], np.uint64)
+        outs.append(ch.zeros((n, h, w, 3), dtype=ch.uint8, device='cuda'))
+        ctx.stage(0, np.concatenate(bufs), np.concatenate([[0], np.cumsum(sizes)[:-1]]).astype(np.uint64), sizes, np.zeros(n, np.uint8),
+                  np.full(n, h, np.uint16), np.full(n, w, np.uint16), L.make_plan(h, w, 0, L.OUT_U8_NHWC),
+                  np.tile(np.array([0, 0, h, w], np.int32), (n, 1)))
+        ctx.submit(0, stream, outs[-1].data_ptr())
+        wants.append(np.stack([O.jpeg_decode(b) for b in bufs]))
+    assert (ctx.status(0, stream, n) == 0).all()
+    for got, want in zip(outs, wants):
+        assert np.array_equal(got.cpu().numpy(), want)
+    ctx.close()
