@@ -1736,8 +1736,14 @@ int ffcvb_gather_time(ffcvb_ctx *ctx, int slot, float *ms) {
     *ms = -1.0f;
     if (!s.gather_timed) return FFCVB_OK; // this slot's last batch was not gathered by the GPU
     CU(cudaSetDevice(ctx->device));
-    CU(cudaEventSynchronize(s.ev_gathered));
-    CU(cudaEventElapsedTime(ms, s.ev_gather_start, s.ev_gathered));
+    // (a loader's worker may submit the slot's next batch between the wait and the reading: wait for that one then)
+    cudaError_t e = cudaErrorNotReady;
+    for (int k = 0; k < 100 && e == cudaErrorNotReady; k++) {
+        CU(cudaEventSynchronize(s.ev_gathered));
+        e = cudaEventElapsedTime(ms, s.ev_gather_start, s.ev_gathered);
+    }
+    if (e == cudaErrorNotReady) cudaGetLastError();
+    CU(e);
     return FFCVB_OK;
 }
 
