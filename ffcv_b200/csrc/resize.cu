@@ -637,8 +637,9 @@ static void launch_typed(const ResizeSource &src, int n, const int32_t *params, 
     if (shape.smem > 48 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shape.smem);
     // CTAs per image: enough of them for about eight waves of the GPU (148 SMs x 4 resident CTAs;
     // fewer waves measured slower, more cost the set-up its amortisation), at most one per band (a sample
-    // whose window holds fewer rows has more of them, of at least four rows)
-    const int least = shape.room && shape.band > 4 ? 4 : shape.band, nbands = (out_h + least - 1) / least;
+    // whose window holds fewer rows has more of them, of at least four rows; without scaling there is no window:
+    // 512 images of 32x32 pixels take 15 us in one CTA each, 31 with seven idle ones beside it)
+    const int least = resize && shape.room && shape.band > 4 ? 4 : shape.band, nbands = (out_h + least - 1) / least;
     int per_image = (8 * 148 * 4 + n - 1) / n;
     if (per_image > nbands) per_image = nbands;
     if (per_image < 1) per_image = 1;
