@@ -1558,8 +1558,17 @@ static int run_batch(ffcvb_ctx *ctx, Slot &s, cudaStream_t st, void *out_dev, bo
     if (!single) {
         static_assert(FFCVB_MAX_RIDERS <= sizeof(SmallCopies::src) / sizeof(uint8_t *), "a batch's riders fit one launch");
         SmallCopies small{};
+        const Slot::Rider *large[FFCVB_MAX_RIDERS];
+        int n_large = 0;
+        uint64_t words = 0;
         for (const auto &r : s.riders) {
             if (!copy) break;
+            const uint64_t mine = small_copy_words(r.bytes, blob + r.off, r.dst_dev);
+            if (words + mine > kSmallCopyWords) {
+                large[n_large++] = &r;
+                continue;
+            }
+            words += mine;
             small.src[small.n] = blob + r.off;
             small.bytes[small.n] = r.bytes;
             small.dst[small.n++] = (uint8_t *)r.dst_dev;
@@ -1572,6 +1581,8 @@ static int run_batch(ffcvb_ctx *ctx, Slot &s, cudaStream_t st, void *out_dev, bo
         launch_resize_augment(src, s.n, params, (int)hd.n_params, make_oplist(s.plan), s.plan.resize,
                               s.plan.out_h, s.plan.out_w, s.plan.out_kind, s.plan.lut_dev, out_dev, status, small,
                               early && !outputs_free, st);
+        for (int k = 0; k < n_large; k++) // (behind the kernel, which may have been launched early)
+            CU(cudaMemcpyAsync(large[k]->dst_dev, blob + large[k]->off, large[k]->bytes, cudaMemcpyDeviceToDevice, st));
     }
     CU(cudaGetLastError());
     if (prof) {

@@ -229,6 +229,33 @@ __device__ __forceinline__ int row_groups(int out_w, int band) {
 __device__ __forceinline__ int divided(uint32_t a, uint32_t inv_n, int n) { return n == 1 ? (int)a : (int)__umulhi(a, inv_n); }
 __device__ __forceinline__ uint32_t inverse(int n) { return (uint32_t)((0x100000000ull + n - 1) / n); }
 
+// One of SmallCopies, by a CTA of 256 threads: every thread has its words (at most kSmallCopyWords / 256) under way
+// at once.
+template <typename Word>
+__device__ __forceinline__ void copy_words(const uint8_t *__restrict__ src, uint8_t *__restrict__ dst, uint32_t bytes) {
+    constexpr int kEach = kSmallCopyWords / 256;
+    const uint32_t n = bytes / sizeof(Word);
+    const Word *from = reinterpret_cast<const Word *>(src);
+    Word *to = reinterpret_cast<Word *>(dst), v[kEach];
+#pragma unroll
+    for (int k = 0; k < kEach; k++)
+        if (threadIdx.x + 256 * k < n) v[k] = from[threadIdx.x + 256 * k];
+#pragma unroll
+    for (int k = 0; k < kEach; k++)
+        if (threadIdx.x + 256 * k < n) to[threadIdx.x + 256 * k] = v[k];
+    const uint32_t done = n * (uint32_t)sizeof(Word);
+    if (threadIdx.x < bytes - done) dst[done + threadIdx.x] = src[done + threadIdx.x];
+}
+__device__ __noinline__ void copy_small(const uint8_t *src, uint8_t *dst, uint32_t bytes) {
+    const uint32_t word = copy_word(src, dst);
+    if (word == 16)
+        copy_words<uint4>(src, dst, bytes);
+    else if (word == 4)
+        copy_words<uint32_t>(src, dst, bytes);
+    else
+        copy_words<uint8_t>(src, dst, bytes);
+}
+
 template <typename OutT>
 __global__ void __launch_bounds__(256, 4)
 resize_augment_kernel(const __grid_constant__ ResizeSource src, const int32_t *__restrict__ params, int n_params,
@@ -249,8 +276,7 @@ resize_augment_kernel(const __grid_constant__ ResizeSource src, const int32_t *_
 
     const int i = blockIdx.y;
     if (blockIdx.x == 0 && i == 0)
-        for (int k = 0; k < small.n; k++)
-            for (uint64_t b = threadIdx.x; b < small.bytes[k]; b += blockDim.x) small.dst[k][b] = small.src[k][b];
+        for (int k = 0; k < small.n; k++) copy_small(small.src[k], small.dst[k], (uint32_t)small.bytes[k]);
     if (!kU8)
         for (int k = threadIdx.x; k < 768; k += blockDim.x) s_lut[(k % 3) * 256 + k / 3] = lut[k]; // per channel
 
