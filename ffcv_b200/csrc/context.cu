@@ -24,6 +24,7 @@
 #include <vector>
 
 #include "../../include/ffcv_b200.h"
+#include "decode_index.h"
 #include "jpeg_header.h"
 #include "kernels.h"
 #include "types.h"
@@ -366,14 +367,6 @@ struct ffcvb_ctx {
     size_t one_host_cap = 0, one_in_cap = 0;
     cudaStream_t one_stream = nullptr;
     cudaEvent_t one_ev[16] = {};
-    // Decode index (ffcvb_set_decode_index): a pool of device memory that keeps, per JPEG stream seen,
-    // the decoder states a finished decode left behind; entries are handed out in order and never
-    // moved.  Keyed by the sample's offset in the file: the context then serves one file.
-    struct IndexEntry {
-        uint64_t off;
-        uint32_t segments;
-        uint64_t created_seq;
-    };
     // Header cache: what the marker segments of a JPEG sample said, kept per sample (key: its
     // offset in the file) so that from the second epoch on staging a sample is a table look-up
     // instead of a parse; the few distinct tables of a file live in stores of their own.
@@ -383,10 +376,11 @@ struct ffcvb_ctx {
     std::vector<std::unique_ptr<std::array<uint16_t, 64>>> quant_store;
     std::vector<uint64_t> huff_store_hash, quant_store_hash;
     std::vector<TableSet> table_sets;
+    // Decode index (ffcvb_set_decode_index): a pool of device memory that keeps, per JPEG stream seen,
+    // the decoder states a finished decode left behind; entries are handed out in order and never
+    // moved.  Keyed by the sample's offset in the file: the context then serves one file.
     DevBuf index_pool, index_stats;
-    size_t index_used = 0;
-    std::unordered_map<uint64_t, IndexEntry> index_map;
-    uint64_t stage_seq = 0;
+    DecodeIndex index;
 };
 
 namespace {
@@ -987,7 +981,16 @@ int stage_impl(ffcvb_ctx *ctx, int slot, const Source &source, const uint64_t *p
         few = bits <= kSlotModeBits && !ctx->tune_subseq_bits;
     }
     if (ctx->tune_subseq_bits) target_bits = (uint32_t)ctx->tune_subseq_bits;
-    ctx->stage_seq++;
+    if (ctx->index_pool.p) {
+        for (size_t k = 0; k < ctx->slots.size(); k++) { // whose writers have ended
+            if (!ctx->index.unsettled((int)k)) continue;
+            if (cudaEventQuery(ctx->slots[k].ev_done) == cudaSuccess)
+                ctx->index.ended((int)k);
+            else
+                cudaGetLastError(); // still running
+        }
+        ctx->index.staged(slot);
+    }
     int max_w = 0, max_h = 0, n_quad = 0, n_444 = 0, n_other = 0;
     const bool can_fuse = plan->resize && !s.packed;
     const ResizeShape shape = can_fuse ? resize_shape(n, plan->out_h, plan->out_w, plan->out_kind) : ResizeShape{};
@@ -1071,21 +1074,9 @@ int stage_impl(ffcvb_ctx *ctx, int slot, const Source &source, const uint64_t *p
             const uint32_t raw = l.seg_stride - 64 - 16; // (at least run-up, own bytes and overlap)
             if (raw > work.max_raw) work.max_raw = raw;
             if (ctx->index_pool.p) {
-                const uint64_t key = ptrs[i];
-                auto it = ctx->index_map.find(key);
-                if (it == ctx->index_map.end()) {
-                    const size_t bytes = decode_index_bytes(l.seg_count);
-                    if (ctx->index_used + bytes <= ctx->index_pool.cap) { // else this stream stays unindexed
-                        it = ctx->index_map.emplace(key, ffcvb_ctx::IndexEntry{ctx->index_used, l.seg_count, ctx->stage_seq}).first;
-                        ctx->index_used += bytes;
-                    }
-                } else if (ctx->stage_seq - it->second.created_seq < ctx->slots.size()) {
-                    it = ctx->index_map.end(); // recorded by a batch that may still run on another slot's stream: hands off
-                }
-                if (it != ctx->index_map.end() && it->second.segments == l.seg_count) {
-                    d.index_off = it->second.off;
-                    d.index_cap = it->second.segments;
-                }
+                const DecodeIndex::Place place = ctx->index.take(ptrs[i], l.seg_count, decode_index_bytes(l.seg_count), slot);
+                d.index_off = place.off;
+                d.index_use = place.use;
             }
         }
         {
@@ -1459,6 +1450,7 @@ static int run_batch(ffcvb_ctx *ctx, Slot &s, cudaStream_t st, void *out_dev, bo
                      cudaEvent_t outputs_free = nullptr) {
     if (ctx->copy_timeout.load())
         return fail(ctx, FFCVB_E_CUDA, "a payload copy did not finish within its time limit: the batch that waited for it is invalid");
+    const int slot = (int)(&s - ctx->slots.data());
     const BatchHeader &hd = s.hdr;
     uint8_t *blob = (uint8_t *)s.blob.p;
     const bool prof = ctx->profile;
@@ -1514,6 +1506,7 @@ static int run_batch(ffcvb_ctx *ctx, Slot &s, cudaStream_t st, void *out_dev, bo
     if (copy) {
         CU(cudaEventRecord(s.ev_copied, st));
         s.in_flight = true;
+        if (ctx->index_pool.p) ctx->index.submitted(slot);
     }
     if (prof) CU(cudaEventRecord(s.ev[1], st));
     const ImageDesc *descs = reinterpret_cast<const ImageDesc *>(blob + hd.desc_off);
@@ -1590,6 +1583,7 @@ static int run_batch(ffcvb_ctx *ctx, Slot &s, cudaStream_t st, void *out_dev, bo
         s.timed = true;
     }
     CU(cudaEventRecord(s.ev_done, st));
+    if (ctx->index_pool.p) ctx->index.marked(slot);
     return FFCVB_OK;
 }
 
@@ -1638,12 +1632,12 @@ int ffcvb_set_decode_index(ffcvb_ctx *ctx, uint64_t bytes) {
         CU(cudaFree(ctx->index_pool.p));
         ctx->index_pool = DevBuf{};
     }
-    ctx->index_map.clear();
-    ctx->index_used = 0;
+    ctx->index.reset(0, (int)ctx->slots.size());
     if (bytes == 0) return FFCVB_OK;
     bytes = align_up((size_t)bytes, 1 << 20);
     CU(cudaMalloc(&ctx->index_pool.p, (size_t)bytes));
     ctx->index_pool.cap = (size_t)bytes;
+    ctx->index.reset((size_t)bytes, (int)ctx->slots.size());
     CU(cudaMemset(ctx->index_pool.p, 0, (size_t)bytes)); // no entry is valid yet
     if (!ctx->index_stats.p) {
         CU(cudaMalloc(&ctx->index_stats.p, 64));
@@ -1656,8 +1650,8 @@ int ffcvb_set_decode_index(ffcvb_ctx *ctx, uint64_t bytes) {
 int ffcvb_decode_index_stats(ffcvb_ctx *ctx, uint64_t *out) {
     if (!ctx || !out) return FFCVB_E_ARG;
     out[0] = out[1] = 0;
-    out[2] = ctx->index_map.size();
-    out[3] = ctx->index_used;
+    out[2] = ctx->index.entries();
+    out[3] = ctx->index.used();
     if (!ctx->index_stats.p) return FFCVB_OK;
     CU(cudaSetDevice(ctx->device));
     CU(cudaMemcpy(out, ctx->index_stats.p, 16, cudaMemcpyDeviceToHost));

@@ -427,10 +427,11 @@ scan_sync_kernel(const ImageDesc *__restrict__ descs, const uint2 *__restrict__ 
 
     if (TEAMS == 1) copies_wait();
 
-    // ---- decode index: the states an earlier decode of this very stream left behind
-    if (index_pool != nullptr && d.index_cap != 0) {
+    // ---- decode index: the states an earlier decode of this very stream left behind (the answer is uniform: a
+    // batch is only given an entry that no launch beside it writes)
+    if (index_pool != nullptr && d.index_use != 0) {
         const DecodeIndexHeader *h = reinterpret_cast<const DecodeIndexHeader *>(index_pool + d.index_off);
-        if (index_entry_valid(h, d)) { // (uniform: no launch that writes the entry runs now)
+        if (index_entry_valid(h, d)) {
             const uint32_t *src = reinterpret_cast<const uint32_t *>(h + 1) + (size_t)j * (kSegSubs + 2);
             scratch.sub_info[seg * kSegSubs + tid] = __ldcg(src + tid);
             if (tid == 0) {
@@ -946,7 +947,7 @@ scan_index_kernel(const ImageDesc *__restrict__ descs, const uint2 *__restrict__
         o[1] = sums[1];
         o[2] = sums[2];
     }
-    const bool record = index_pool != nullptr && d.index_cap != 0 &&
+    const bool record = index_pool != nullptr && (d.index_use & 2) != 0 &&
                         !index_entry_valid(reinterpret_cast<const DecodeIndexHeader *>(index_pool + d.index_off), d);
     if (record) {
         uint32_t *dst = reinterpret_cast<uint32_t *>(index_pool + d.index_off + sizeof(DecodeIndexHeader)) + (size_t)j * (kSegSubs + 2);

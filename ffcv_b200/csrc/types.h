@@ -74,7 +74,7 @@ struct ImageDesc {
     // batch's segments are this image's.
     uint32_t subseq_bits, seg_raw, seg_warm, seg_stride, seg_first, seg_count;
     uint32_t slots;        // decoded from every slot at once: 1 + the first of the image's SlotTables (0: not)
-    uint32_t index_cap;    // place in the decode index (0: none), see DecodeIndexHeader
+    uint32_t index_use;    // place in the decode index: 0 none, bit 0 the entry may be read, bit 1 and is written
     uint64_t index_off;    // byte offset of the entry in the context's index pool
     // The crop box decides how much of the image is needed: the entropy decoder stops after
     // `mcu_rows` rows of MCUs and the inverse transform runs only on the MCUs of the box below
@@ -171,7 +171,8 @@ constexpr uint32_t kNoBlock = 0xFFFFFFFFu; // position of a block that the scan 
 // start from -- the exact decoder state at the start of every subsequence and the number of blocks
 // completed in it.  With it no guess has to be repaired.  An entry lives in device memory:
 //   [DecodeIndexHeader][per segment: uint32 sub_info x kSegSubs, uint32 exit, uint32 blocks]
-// and is valid when `magic` is set (written last) and the other fields match.
+// and is valid when `magic` is set (written last) and the other fields match.  Which batch writes it and which
+// may read it is settled on the host (DecodeIndex).
 struct DecodeIndexHeader {
     uint32_t magic, scan_len, subseq_bits, segments;
 };

@@ -1,0 +1,60 @@
+"""The decode index with batches of several slots under way at once."""
+import cv2
+import numpy as np
+import pytest
+import torch as ch
+
+from ffcv_b200 import libffcv as L
+from ffcv_b200.synthetic import synth_content
+from parity import O
+
+pytestmark = pytest.mark.gpu
+
+
+class _Job:
+    def __init__(self, n, h, w):
+        rng = np.random.default_rng(n)
+        bufs = [cv2.imencode('.jpg', synth_content(rng, h, w), [cv2.IMWRITE_JPEG_QUALITY, 90])[1].reshape(-1) for _ in range(n)]
+        self.want = np.stack([O.jpeg_decode(b) for b in bufs])
+        sizes = np.array([b.size for b in bufs], np.uint64)
+        self.args = (np.concatenate(bufs), np.concatenate([[0], np.cumsum(sizes)[:-1]]).astype(np.uint64), sizes, np.zeros(n, np.uint8),
+                     np.full(n, h, np.uint16), np.full(n, w, np.uint16), L.make_plan(h, w, 0, L.OUT_U8_NHWC),
+                     np.tile(np.array([0, 0, h, w], np.int32), (n, 1)))
+
+    def queue(self, ctx, slot, stream):
+        out = ch.zeros(self.want.shape, dtype=ch.uint8, device='cuda')
+        ch.cuda.current_stream().synchronize()
+        ctx.stage(slot, *self.args)
+        ctx.submit(slot, stream.cuda_stream, out.data_ptr())
+        return out
+
+
+def test_entries_are_handed_out_when_their_writer_has_ended():
+    """Slot 0's batch, which writes the entries, waits behind other work of its stream; the batches that slot 1
+    decodes meanwhile neither read nor write them."""
+    job, n = _Job(6, 120, 144), 6
+    ctx = L.Context(0, 2, 2)
+    ctx.set_decode_index(1 << 20)
+    held, free = ch.cuda.Stream(), ch.cuda.Stream()
+    job.queue(ctx, 1, free)  # scratch of both slots is there: nothing below allocates and waits for the device
+    job.queue(ctx, 0, free)
+    ch.cuda.synchronize()
+    ctx.set_decode_index(1 << 20)  # empty again
+    with ch.cuda.stream(held):
+        ch.cuda._sleep(1 << 30)  # about half a second
+    first = job.queue(ctx, 0, held)
+    for _ in range(4):
+        out = job.queue(ctx, 1, free)
+        free.synchronize()
+        assert np.array_equal(out.cpu().numpy(), job.want)
+        stats = ctx.decode_index_stats()
+        assert not held.query(), 'the held batch ran too early for this test'
+        assert (stats['used'], stats['recorded'], stats['entries']) == (0, 0, n)
+    held.synchronize()
+    assert np.array_equal(first.cpu().numpy(), job.want)
+    assert ctx.decode_index_stats()['recorded'] == n
+    out = job.queue(ctx, 1, free)
+    free.synchronize()
+    assert np.array_equal(out.cpu().numpy(), job.want)
+    assert ctx.decode_index_stats()['used'] == n
+    ctx.close()
