@@ -313,6 +313,7 @@ struct Slot {
     cudaEvent_t ev_done = nullptr;      // behind all of its work
     bool gather_timed = false; // ev_gather_start .. ev_gathered bracket the last gather of this slot
     bool timed = false; // events of the last run are valid
+    uint64_t index_life = 0; // of the decode index that the staged batch has places in
 };
 
 constexpr double kMaxAdaptiveShare = 0.5; // of a pinned batch's bytes that the threads may be left to copy
@@ -381,6 +382,7 @@ struct ffcvb_ctx {
     // moved.  Keyed by the sample's offset in the file: the context then serves one file.
     DevBuf index_pool, index_stats;
     DecodeIndex index;
+    uint64_t index_life = 0; // counts the calls that set the index up: places of an earlier one mean nothing
 };
 
 namespace {
@@ -991,6 +993,7 @@ int stage_impl(ffcvb_ctx *ctx, int slot, const Source &source, const uint64_t *p
         }
         ctx->index.staged(slot);
     }
+    s.index_life = ctx->index_life;
     int max_w = 0, max_h = 0, n_quad = 0, n_444 = 0, n_other = 0;
     const bool can_fuse = plan->resize && !s.packed;
     const ResizeShape shape = can_fuse ? resize_shape(n, plan->out_h, plan->out_w, plan->out_kind) : ResizeShape{};
@@ -1451,6 +1454,7 @@ static int run_batch(ffcvb_ctx *ctx, Slot &s, cudaStream_t st, void *out_dev, bo
     if (ctx->copy_timeout.load())
         return fail(ctx, FFCVB_E_CUDA, "a payload copy did not finish within its time limit: the batch that waited for it is invalid");
     const int slot = (int)(&s - ctx->slots.data());
+    const bool indexed = ctx->index_pool.p && s.index_life == ctx->index_life;
     const BatchHeader &hd = s.hdr;
     uint8_t *blob = (uint8_t *)s.blob.p;
     const bool prof = ctx->profile;
@@ -1506,7 +1510,7 @@ static int run_batch(ffcvb_ctx *ctx, Slot &s, cudaStream_t st, void *out_dev, bo
     if (copy) {
         CU(cudaEventRecord(s.ev_copied, st));
         s.in_flight = true;
-        if (ctx->index_pool.p) ctx->index.submitted(slot);
+        if (indexed) ctx->index.submitted(slot);
     }
     if (prof) CU(cudaEventRecord(s.ev[1], st));
     const ImageDesc *descs = reinterpret_cast<const ImageDesc *>(blob + hd.desc_off);
@@ -1534,7 +1538,7 @@ static int run_batch(ffcvb_ctx *ctx, Slot &s, cudaStream_t st, void *out_dev, bo
         scratch.pos = (uint32_t *)s.index.p;
         scratch.dc = (int16_t *)(scratch.pos + s.total_blocks);
         early = work.early() && !prof;
-        launch_entropy_decode(descs, work, blob, huff, scratch, status, (uint8_t *)ctx->index_pool.p,
+        launch_entropy_decode(descs, work, blob, huff, scratch, status, indexed ? (uint8_t *)ctx->index_pool.p : nullptr,
                               (unsigned long long *)ctx->index_stats.p, st);
         if (prof) CU(cudaEventRecord(s.ev[2], st));
         launch_blocks(descs, reinterpret_cast<const uint2 *>(blob + s.block_tiles_off), s.n_block_tiles, huff, mult, scratch,
@@ -1583,7 +1587,7 @@ static int run_batch(ffcvb_ctx *ctx, Slot &s, cudaStream_t st, void *out_dev, bo
         s.timed = true;
     }
     CU(cudaEventRecord(s.ev_done, st));
-    if (ctx->index_pool.p) ctx->index.marked(slot);
+    if (indexed) ctx->index.marked(slot);
     return FFCVB_OK;
 }
 
@@ -1633,6 +1637,7 @@ int ffcvb_set_decode_index(ffcvb_ctx *ctx, uint64_t bytes) {
         ctx->index_pool = DevBuf{};
     }
     ctx->index.reset(0, (int)ctx->slots.size());
+    ctx->index_life++;
     if (bytes == 0) return FFCVB_OK;
     bytes = align_up((size_t)bytes, 1 << 20);
     CU(cudaMalloc(&ctx->index_pool.p, (size_t)bytes));

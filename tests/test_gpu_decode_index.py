@@ -58,3 +58,26 @@ def test_entries_are_handed_out_when_their_writer_has_ended():
     assert np.array_equal(out.cpu().numpy(), job.want)
     assert ctx.decode_index_stats()['used'] == n
     ctx.close()
+
+
+def test_a_batch_staged_before_the_index_was_set_up_again_leaves_it_alone():
+    job, n = _Job(3, 64, 80), 3
+    ctx = L.Context(0, 1, 2)
+    ctx.set_decode_index(1 << 20)
+    stream = ch.cuda.Stream()
+    for again in (1 << 20, 0):
+        out = ch.zeros(job.want.shape, dtype=ch.uint8, device='cuda')
+        ch.cuda.synchronize()
+        ctx.stage(0, *job.args)
+        ctx.set_decode_index(again)
+        ctx.submit(0, stream.cuda_stream, out.data_ptr())
+        ch.cuda.synchronize()
+        assert np.array_equal(out.cpu().numpy(), job.want)
+        assert ctx.decode_index_stats()['recorded'] == 0
+    ctx.set_decode_index(1 << 20)
+    for use in (0, n):
+        out = job.queue(ctx, 0, stream)
+        ch.cuda.synchronize()
+        assert np.array_equal(out.cpu().numpy(), job.want)
+        assert ctx.decode_index_stats()['used'] == use
+    ctx.close()
