@@ -362,6 +362,7 @@ struct ffcvb_ctx {
     // that are queued.
     cudaStream_t copy_stream = nullptr;
     int32_t *gather_failed = nullptr; // page-locked: set by a gather whose wait for the link ran out
+    uint64_t gather_limit_ns = 2000000000ull; // of such a wait (FFCV_B200_GATHER_LIMIT_MS)
     // single-image entry points: their stream, device buffers, pinned result and events of its pieces
     DevBuf one_src, one_dst;
     uint8_t *one_host = nullptr, *one_in = nullptr;
@@ -497,6 +498,8 @@ int ffcvb_create(int device, int n_slots, int n_threads, ffcvb_ctx **out) {
     c->tune_copy_threads = env_int("FFCV_B200_COPY_THREADS", 1, 256);
     c->tune_subseq_bits = env_int("FFCV_B200_SUBSEQ_BITS", 128, kMaxSubseqBits) / 32 * 32;
     c->gather_ctas = env_int("FFCV_B200_GATHER_CTAS", 1, 1024);
+    if (const char *e = getenv("FFCV_B200_GATHER_LIMIT_MS"))
+        if (*e >= '0' && *e <= '9') c->gather_limit_ns = (uint64_t)env_int("FFCV_B200_GATHER_LIMIT_MS", 0, 600000) * 1000000;
     *out = c;
     return FFCVB_OK;
 }
@@ -1440,6 +1443,14 @@ static int hold_for_copy(ffcvb_ctx *ctx, Slot &s, cudaStream_t st) {
     return FFCVB_OK;
 }
 
+// An error, once, when a gather of an earlier batch has given up since the last call.
+static int report_gather(ffcvb_ctx *ctx) {
+    volatile int32_t *failed = ctx->gather_failed;
+    if (!failed || !*failed) return FFCVB_OK;
+    *failed = 0;
+    return fail(ctx, FFCVB_E_CUDA, "the payloads of an earlier batch did not arrive in time: ffcvb_batch_status flags its samples");
+}
+
 // Where a single-image decode leaves its pixels (instead of the slot's scratch, and with no resize
 // behind it) and its status word: device or page-locked host memory.
 struct Single {
@@ -1453,6 +1464,11 @@ static int run_batch(ffcvb_ctx *ctx, Slot &s, cudaStream_t st, void *out_dev, bo
                      cudaEvent_t outputs_free = nullptr) {
     if (ctx->copy_timeout.load())
         return fail(ctx, FFCVB_E_CUDA, "a payload copy did not finish within its time limit: the batch that waited for it is invalid");
+    int hrc;
+    if (single && ctx->gather_failed)
+        *ctx->gather_failed = 0; // (its call has returned the image's status)
+    else if ((hrc = report_gather(ctx)))
+        return hrc;
     const int slot = (int)(&s - ctx->slots.data());
     const bool indexed = ctx->index_pool.p && s.index_life == ctx->index_life;
     const BatchHeader &hd = s.hdr;
@@ -1470,7 +1486,6 @@ static int run_batch(ffcvb_ctx *ctx, Slot &s, cudaStream_t st, void *out_dev, bo
     }
     if (s.last_stream != st && s.last_stream != nullptr) CU(cudaStreamWaitEvent(st, s.ev_done, 0)); // (the slot changed streams)
     s.last_stream = st;
-    int hrc;
     if (copy && !s.direct) {
         if ((hrc = hold_for_copy(ctx, s, st))) return hrc;
         CU(cudaMemcpyAsync(blob, s.host, hd.total_bytes, cudaMemcpyHostToDevice, st));
@@ -1487,15 +1502,14 @@ static int run_batch(ffcvb_ctx *ctx, Slot &s, cudaStream_t st, void *out_dev, bo
             CU(cudaEventCreate(&s.ev_gather_start));
             CU(cudaEventCreate(&s.ev_gathered));
         }
-        if (*(volatile int32_t *)ctx->gather_failed) return fail(ctx, FFCVB_E_CUDA, "a payload gather gave up waiting for the link");
         CU(cudaEventRecord(s.ev_begin, st)); // the slot's previous batch
         CU(cudaStreamWaitEvent(ctx->copy_stream, s.ev_begin, 0));
         CU(cudaMemcpyAsync(blob, s.host, hd.payload_off, cudaMemcpyHostToDevice, ctx->copy_stream));
         s.gather_timed = s.range_len == 0;
         if (s.gather_timed) {
             CU(cudaEventRecord(s.ev_gather_start, ctx->copy_stream));
-            launch_gather_payloads(reinterpret_cast<const ImageDesc *>(blob + hd.desc_off), s.n, blob, ctx->gather_ctas, ctx->gather_failed,
-                                   ctx->copy_stream);
+            launch_gather_payloads(reinterpret_cast<ImageDesc *>(blob + hd.desc_off), s.n, blob, ctx->gather_ctas,
+                                   reinterpret_cast<int32_t *>(blob + s.status_off), ctx->gather_limit_ns, ctx->gather_failed, ctx->copy_stream);
         } else {
             CU(cudaMemcpyAsync(blob + hd.payload_off, s.range_src, s.range_len, cudaMemcpyHostToDevice, ctx->copy_stream));
         }
@@ -1779,6 +1793,8 @@ int ffcvb_batch_launches(const ffcvb_ctx *ctx, int slot) {
          2 * (s.work.n_slots > 0) + (s.work.n_guess + s.work.n_slots > 0) + (s.work.n_restart > 0);
     return k;
 }
+
+int ffcvb_check(ffcvb_ctx *ctx) { return ctx ? report_gather(ctx) : FFCVB_E_ARG; }
 
 int ffcvb_batch_status(ffcvb_ctx *ctx, int slot, void *stream, int32_t *status, int n) {
     if (!ctx) return FFCVB_E_ARG;

@@ -947,7 +947,7 @@ scan_index_kernel(const ImageDesc *__restrict__ descs, const uint2 *__restrict__
         o[1] = sums[1];
         o[2] = sums[2];
     }
-    const bool record = index_pool != nullptr && (d.index_use & 2) != 0 &&
+    const bool record = index_pool != nullptr && (d.index_use & 2) != 0 && d.host_status == 0 &&
                         !index_entry_valid(reinterpret_cast<const DecodeIndexHeader *>(index_pool + d.index_off), d);
     if (record) {
         uint32_t *dst = reinterpret_cast<uint32_t *>(index_pool + d.index_off + sizeof(DecodeIndexHeader)) + (size_t)j * (kSegSubs + 2);
@@ -986,7 +986,7 @@ scan_index_kernel(const ImageDesc *__restrict__ descs, const uint2 *__restrict__
         dc[b] = 0;
     }
     if (tid == 0) {
-        status[img] = complete ? 0 : kErrData;
+        status[img] = d.host_status != 0 ? (int)d.host_status : (complete ? 0 : (int)kErrData);
         if (record) {
             DecodeIndexHeader *h = reinterpret_cast<DecodeIndexHeader *>(index_pool + d.index_off);
             h->scan_len = d.scan_len;
@@ -1110,7 +1110,7 @@ scan_restart_kernel(const ImageDesc *__restrict__ descs, const int32_t *__restri
         }
     }
     __syncthreads();
-    if (tid == 0) status[img] = s_bad ? kErrData : 0;
+    if (tid == 0) status[img] = d.host_status != 0 ? (int)d.host_status : (s_bad ? (int)kErrData : 0);
 }
 
 } // namespace

@@ -21,14 +21,22 @@ struct Ring {
     uint64_t dst[kStages];
     uint32_t len[kStages];
     uint32_t issued, stored;
+    uint64_t limit; // of a wait, in nanoseconds
     bool failed;
 };
 
-// Waits for the piece in stage `st`, two seconds at most; false: it did not arrive.
-__device__ __forceinline__ bool arrived(uint64_t *bars, uint32_t st, uint32_t parity) {
+// Waits for the piece in stage `st`, `limit` nanoseconds at most (0: looks once); false: it did not arrive.
+__device__ __forceinline__ bool arrived(uint64_t *bars, uint32_t st, uint32_t parity, uint64_t limit) {
     uint64_t begin = 0;
     for (;;) {
         uint32_t ok;
+        if (limit == 0) {
+            asm volatile("{\n\t.reg .pred p;\n\tmbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+                         : "=r"(ok)
+                         : "r"(shared_address(&bars[st])), "r"(parity)
+                         : "memory");
+            return ok != 0;
+        }
         asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
                      : "=r"(ok)
                      : "r"(shared_address(&bars[st])), "r"(parity)
@@ -37,14 +45,14 @@ __device__ __forceinline__ bool arrived(uint64_t *bars, uint32_t st, uint32_t pa
         uint64_t now;
         asm volatile("mov.u64 %0, %globaltimer;" : "=l"(now));
         if (begin == 0) begin = now;
-        if (now - begin > 2000000000ull) return false;
+        if (now - begin > limit) return false;
     }
 }
 
 // Sends the oldest piece on its way in out again.
 __device__ __forceinline__ void store_oldest(Ring &r, uint8_t *buf, uint64_t *bars, uint8_t *blob) {
     const uint32_t st = r.stored % kStages;
-    if (!arrived(bars, st, (r.stored / kStages) & 1)) {
+    if (!arrived(bars, st, (r.stored / kStages) & 1, r.limit)) {
         r.failed = true;
         return;
     }
@@ -73,9 +81,11 @@ __device__ __forceinline__ void send(Ring &r, uint8_t *buf, uint64_t *bars, uint
     }
 }
 
-// The CTAs take the samples in turn, each split into `parts` when there are few.
+// The CTAs take the samples in turn, each split into `parts` when there are few.  One that gives up marks all of its
+// samples as failed, for the kernels that follow and in `status`.
 __global__ void __launch_bounds__(32)
-gather_payloads_kernel(const ImageDesc *__restrict__ descs, int n, int parts, uint8_t *__restrict__ blob, int32_t *__restrict__ failed) {
+gather_payloads_kernel(ImageDesc *descs, int n, int parts, uint8_t *__restrict__ blob, int32_t *status, uint64_t limit,
+                       int32_t *failed) {
     __shared__ __align__(128) uint8_t s_buf[kStages * kPiece];
     __shared__ __align__(8) uint64_t s_bars[kStages];
     const int lane = threadIdx.x;
@@ -85,6 +95,7 @@ gather_payloads_kernel(const ImageDesc *__restrict__ descs, int n, int parts, ui
     __syncwarp();
     const int items = n * parts, step = gridDim.x;
     Ring ring{};
+    ring.limit = limit;
     for (int first = blockIdx.x; first < items; first += 32 * step) {
         // the descriptors of this CTA's next 32 items, one per lane
         const int item = first + lane * step;
@@ -131,19 +142,27 @@ gather_payloads_kernel(const ImageDesc *__restrict__ descs, int n, int parts, ui
         while (ring.stored != ring.issued && !ring.failed) store_oldest(ring, s_buf, s_bars, blob);
         asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
         if (ring.failed) {
+            for (int item = blockIdx.x; item < items; item += step) {
+                ImageDesc &d = descs[item / parts];
+                if (d.src_addr == 0 || d.payload_size == 0) continue;
+                d.host_status = (int16_t)kErrData;
+                status[item / parts] = kErrData;
+            }
             *failed = 1;
-            for (; ring.stored != ring.issued; ring.stored++) arrived(s_bars, ring.stored % kStages, (ring.stored / kStages) & 1);
+            const uint64_t drain = max(limit, (uint64_t)2000000000ull); // (shared memory must outlive the copies into it)
+            for (; ring.stored != ring.issued; ring.stored++) arrived(s_bars, ring.stored % kStages, (ring.stored / kStages) & 1, drain);
         }
     }
 }
 
 } // namespace
 
-void launch_gather_payloads(const ImageDesc *descs, int n, uint8_t *blob, int ctas, int32_t *failed, cudaStream_t stream) {
+void launch_gather_payloads(ImageDesc *descs, int n, uint8_t *blob, int ctas, int32_t *status, uint64_t limit_ns, int32_t *failed,
+                            cudaStream_t stream) {
     if (n <= 0) return;
     if (ctas < 1) ctas = kGatherCtas;
     const int parts = n >= 4 * ctas ? 1 : (4 * ctas + n - 1) / n;
-    gather_payloads_kernel<<<ctas, 32, 0, stream>>>(descs, n, parts, blob, failed);
+    gather_payloads_kernel<<<ctas, 32, 0, stream>>>(descs, n, parts, blob, status, limit_ns, failed);
 }
 
 } // namespace ffcvb

@@ -12,9 +12,11 @@ namespace ffcvb {
 // Pulls every sample's payload from pinned host memory (descs[i].src_addr, read by the SMs over
 // PCIe) into its place in the device blob.  Source and destination share their alignment mod 16, and the
 // bytes up to the next 16-byte boundaries around a payload's place are overwritten too.  `ctas`: CTAs
-// that fetch (< 1: kGatherCtas).  `failed` (device-visible) is set when a wait for the link ran out.
+// that fetch (< 1: kGatherCtas).  Where a piece has not arrived after limit_ns the samples of its CTA get
+// host_status and their word in `status` set to kErrData, and `failed` (device-visible) is set.
 constexpr int kGatherCtas = 148;
-void launch_gather_payloads(const ImageDesc *descs, int n, uint8_t *blob, int ctas, int32_t *failed, cudaStream_t stream);
+void launch_gather_payloads(ImageDesc *descs, int n, uint8_t *blob, int ctas, int32_t *status, uint64_t limit_ns, int32_t *failed,
+                            cudaStream_t stream);
 
 // The kernels of a small batch follow one another early: each is launched as soon as all CTAs of the one before
 // have begun (next_may_begin, first thing), fetches its tables and then waits in hardware for the one before to

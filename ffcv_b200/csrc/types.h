@@ -38,7 +38,7 @@ struct ImageDesc {
     uint64_t payload_off;  // byte offset of the staged payload inside the blob (16-byte aligned)
     uint32_t payload_size; // staged bytes
     uint16_t mode;         // 0 jpg, 1 raw (ffcv/fields/rgb_image.py:21-23)
-    int16_t host_status;   // 0, or a negative code when the host parser rejected the stream
+    int16_t host_status;   // 0, or a negative code: the host parser rejected the stream, or its bytes did not arrive
     uint16_t height, width;
     uint16_t row0, rows;   // raw: first image row present in the staged payload, number of rows
     uint16_t col0, cols;   // raw: first image column present, number of columns

@@ -107,6 +107,8 @@ lib.ffcvb_batch_launches.argtypes = [c_void_p, c_int]
 lib.ffcvb_batch_launches.restype = c_int
 lib.ffcvb_batch_status.argtypes = [c_void_p, c_int, c_void_p, c_void_p, c_int]
 lib.ffcvb_batch_status.restype = c_int
+lib.ffcvb_check.argtypes = [c_void_p]
+lib.ffcvb_check.restype = c_int
 lib.ffcvb_transform_device.argtypes = [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int,
                                        POINTER(Plan), c_void_p, c_void_p]
 lib.ffcvb_transform_device.restype = c_int
@@ -352,6 +354,10 @@ class Context:
         if bad < 0:
             self._check(bad, 'ffcvb_batch_status')
         return st
+
+    def check(self):
+        """Raises when payloads of an earlier batch did not arrive (see ffcvb_check)."""
+        self._check(lib.ffcvb_check(self._h), 'ffcvb_check')
 
     def transform_device(self, stream, src_ptr, n, h, w, plan, params, out_ptr):
         params = np.ascontiguousarray(params, dtype=np.int32)

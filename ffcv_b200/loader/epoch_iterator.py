@@ -132,6 +132,7 @@ class EpochIterator(Thread):
         item = self.output_queue.get()
         if item is None:
             self.close()
+            self.loader.check()
             raise StopIteration()
         if isinstance(item, _Failure):
             self.close()

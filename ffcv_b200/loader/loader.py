@@ -245,6 +245,12 @@ class Loader:
                 self._contexts[index].set_decode_index(int(self.decode_index_gb * (1 << 30)))
         return self._contexts[index]
 
+    def check(self):
+        """Raises when the bytes of a batch that has run did not reach the GPU; waits for nothing.  Called
+        at the end of every epoch."""
+        for context in self._contexts.values():
+            context.check()
+
     def slot_streams(self):
         if self._streams is None:
             self._streams = [ch.cuda.Stream(self.device) for _ in range(self.batches_ahead + 2)]

@@ -250,6 +250,13 @@ int ffcvb_gather_time(ffcvb_ctx *ctx, int slot, float *ms);
  * The reference drops imdecode's return code (rgb_image.py:131,196); this keeps it. */
 int ffcvb_batch_status(ffcvb_ctx *ctx, int slot, void *stream, int32_t *status, int n);
 
+/* When the GPU fetches payloads from page-locked memory it waits two seconds for a piece of them
+ * (FFCV_B200_GATHER_LIMIT_MS in the environment of ffcvb_create: other limits).  The samples of a batch
+ * whose pieces do not arrive are flagged (ffcvb_batch_status) and blank, and the next call of
+ * ffcvb_submit_batch or ffcvb_check returns FFCVB_E_CUDA, once.  ffcvb_check waits for nothing: it
+ * tells of the batches that have run. */
+int ffcvb_check(ffcvb_ctx *ctx);
+
 /* Augment + normalise a batch that already sits on the device as uint8 [n, h, w, 3]
  * (`src_dev`), e.g. the output of an earlier call; params as above (host pointer, crop box
  * honoured when plan.resize == 1).  Used when a pipeline cannot be fused into one call. */
