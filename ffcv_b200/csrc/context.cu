@@ -1456,6 +1456,7 @@ static int report_gather(ffcvb_ctx *ctx) {
 struct Single {
     uint8_t *rgb;
     int32_t *status;
+    bool whole_rows; // see launch_color
 };
 
 // `outputs_free`: an event the work that writes to the caller's buffers (out_dev, the riders'
@@ -1560,7 +1561,7 @@ static int run_batch(ffcvb_ctx *ctx, Slot &s, cudaStream_t st, void *out_dev, bo
         if (prof) CU(cudaEventRecord(s.ev[3], st));
         launch_color(descs, jl, s.n_jpeg, s.n_quad, s.n_444, s.n_other, s.max_w, s.max_h,
                      reinterpret_cast<const uint2 *>(blob + s.quad_tiles_off), s.n_quad_tiles, (const uint8_t *)s.planes.p,
-                     rgb, s.plan.resize ? params : nullptr, (int)hd.n_params, early, st);
+                     rgb, s.plan.resize ? params : nullptr, (int)hd.n_params, single && single->whole_rows, early, st);
         if (prof) CU(cudaEventRecord(s.ev[4], st));
     } else if (prof) {
         for (int k = 2; k <= 4; k++) CU(cudaEventRecord(s.ev[k], st));
@@ -2089,7 +2090,8 @@ int imdecode(unsigned char *input_buffer, uint64_t input_size, uint32_t source_h
     if (!zero_copy && grow_dev(ctx, ctx->one_dst, out_bytes)) return -1;
     volatile int32_t *status = (volatile int32_t *)ctx->one_host;
     *status = 0;
-    const Single single{zero_copy ? ctx->one_host + kResultHead : (uint8_t *)ctx->one_dst.p, (int32_t *)ctx->one_host};
+    const Single single{zero_copy ? ctx->one_host + kResultHead : (uint8_t *)ctx->one_dst.p, (int32_t *)ctx->one_host,
+                        zero_copy || plan.out_w % 4 != 0};
     if (run_batch(ctx, s, ctx->one_stream, nullptr, true, &single)) return -1;
     if (zero_copy) {
         if (cudaStreamSynchronize(ctx->one_stream) != cudaSuccess || *status != 0) return -1;

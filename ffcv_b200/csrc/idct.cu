@@ -302,8 +302,9 @@ __device__ __forceinline__ void store_rgb4(uint8_t *o, const uint32_t *px, int c
 // A warp stores `bytes` bytes of a row at `row` (shared memory, whole words; a word behind them may be read) to dst:
 // consecutive words whatever dst's alignment, because the rows of a caller's image begin anywhere and may
 // lie in host memory, where every partial sector is a transaction of its own.  With the six words of each
-// thread stored one by one the kernel below took 37 us for a 224x256 image in host memory (now 14) and 20 for one of
-// 1213x1617 pixels on the GPU (now 11).
+// thread stored one by one the kernel for 4:2:0 took 37 us for a 224x256 image in host memory (now 14) and 20 for one of
+// 1213x1617 pixels on the GPU (now 11); calls with 4:4:4 images of 224x253 and 401x419 pixels took 283 and 565 us
+// with single bytes (now 94 and 117).
 constexpr int kRowPixels = 128, kRowWords = kRowPixels * 3 / 4 + 4;
 __device__ __forceinline__ void store_row(uint8_t *dst, const uint32_t *row, int bytes, int lane) {
     const int head = min((int)(-reinterpret_cast<uintptr_t>(dst) & 3), bytes), words = (bytes - head) >> 2;
@@ -382,7 +383,10 @@ color_quad_kernel(const ImageDesc *__restrict__ descs, const int32_t *__restrict
 // 4:4:4 images, and images decoded at reduced scale (whose chroma blocks were inverted to the luma
 // resolution): no upsampling, one thread per four pixels of a row of the crop box (one word of each
 // plane in, three words out), every thread walking a column strip so that the grid stays small
-// for very large images.
+// for very large images.  kRows: rows leave whole (store_row), for results whose rows do not begin on words or that
+// lie in host memory; on the GPU the three words of each thread are better (64 images of 1200x1400: 190 us, 231
+// with whole rows).
+template <bool kRows>
 __global__ void __launch_bounds__(256)
 color_444_kernel(const ImageDesc *__restrict__ descs, const int32_t *__restrict__ list,
                  const uint8_t *__restrict__ planes, uint8_t *__restrict__ rgb,
@@ -398,21 +402,35 @@ color_444_kernel(const ImageDesc *__restrict__ descs, const int32_t *__restrict_
     const int pw = d.mcus_x * d.hs * d.bs_luma; // = the chroma planes' pitch: all planes have one resolution here
     const uint8_t *Y = planes + d.plane_off[0], *Cb = planes + d.plane_off[1], *Cr = planes + d.plane_off[2];
     uint8_t *out = rgb + d.rgb_off;
-    const int x = (x0 & ~3) + 4 * (blockIdx.x * 32 + threadIdx.x);
-    if (x >= x1) return;
+    __shared__ __align__(16) uint32_t s_rows[kRows ? 8 : 1][kRowWords];
+    const int first = (x0 & ~3) + kRowPixels * blockIdx.x, x = first + 4 * threadIdx.x;
+    if (kRows ? first >= x1 : x >= x1) return;
     const int count = min(4, W - x);
     // a plane's pitch is a multiple of 8 only at full scale; reduced planes may be narrower
     const bool words_in = ((pw | (int)(d.plane_off[0] | d.plane_off[1] | d.plane_off[2])) & 3) == 0;
     const bool words_out = ((reinterpret_cast<uintptr_t>(out) | d.rgb_pitch) & 3) == 0;
     for (int y = y0 + blockIdx.y * 8 + threadIdx.y; y < y1; y += gridDim.y * 8) {
         uint32_t px[4];
-        plain_pixels(Y, Cb, Cr, (size_t)y * pw + x, count, words_in, px);
-        store_rgb4(out + (size_t)y * d.rgb_pitch + (size_t)x * 3, px, count, words_out);
+        if (!kRows) {
+            plain_pixels(Y, Cb, Cr, (size_t)y * pw + x, count, words_in, px);
+            store_rgb4(out + (size_t)y * d.rgb_pitch + (size_t)x * 3, px, count, words_out);
+            continue;
+        }
+        if (x < x1) {
+            plain_pixels(Y, Cb, Cr, (size_t)y * pw + x, count, words_in, px);
+            pack_rgb4(&s_rows[threadIdx.y][3 * threadIdx.x], px);
+        }
+        __syncwarp();
+        store_row(out + (size_t)y * d.rgb_pitch + (size_t)first * 3, s_rows[threadIdx.y], 3 * min(kRowPixels, x1 - first), threadIdx.x);
+        __syncwarp();
     }
 }
 
 // Per-pixel kernel for everything the kernels above leave out (4:2:2, greyscale, 4:2:0 images
-// narrower than the triangle filter).
+// narrower than the triangle filter).  kRows: where rows follow one another without a gap, as those of a single
+// image do, a warp's 32 pixels leave as 24 words (a choice at run time costs batches a third: 211 -> 277 us for 256
+// 4:2:2 images of 300x400).
+template <bool kRows>
 __global__ void __launch_bounds__(256)
 color_other_kernel(const ImageDesc *__restrict__ descs, const int32_t *__restrict__ list,
                    const uint8_t *__restrict__ planes, uint8_t *__restrict__ rgb) {
@@ -431,6 +449,9 @@ color_other_kernel(const ImageDesc *__restrict__ descs, const int32_t *__restric
     const uint8_t *Cb = planes + d.plane_off[1];
     const uint8_t *Cr = planes + d.plane_off[2];
     uint8_t *out = rgb + d.rgb_off;
+    __shared__ __align__(16) uint8_t s_pixels[kRows ? 256 / 32 : 1][32 * 3];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const bool gapless = kRows && d.rgb_pitch == (uint32_t)W * 3 && (reinterpret_cast<uintptr_t>(out) & 3) == 0;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < npix; i += gridDim.x * blockDim.x) {
         const int y = i / W, x = i - y * W;
         const int lum = Y[(size_t)y * yw + x];
@@ -442,22 +463,28 @@ color_other_kernel(const ImageDesc *__restrict__ descs, const int32_t *__restric
             g = lum + ((-22554 * cb - 46802 * cr + 32768) >> 16);
             b = lum + ((116130 * cb + 32768) >> 16);
         }
-        uint8_t *o = out + (size_t)y * d.rgb_pitch + (size_t)x * 3;
+        const bool whole = gapless && i - lane + 32 <= npix; // (uniform in the warp)
+        uint8_t *o = whole ? &s_pixels[warp][3 * lane] : out + (size_t)y * d.rgb_pitch + (size_t)x * 3;
         o[0] = (uint8_t)min(255, max(0, r));
         o[1] = (uint8_t)min(255, max(0, g));
         o[2] = (uint8_t)min(255, max(0, b));
+        if (whole) {
+            __syncwarp();
+            if (lane < 24) reinterpret_cast<uint32_t *>(out + 3 * (size_t)(i - lane))[lane] = reinterpret_cast<const uint32_t *>(s_pixels[warp])[lane];
+            __syncwarp();
+        }
     }
 }
 
 void launch_color(const ImageDesc *descs, const int32_t *list, int n_list, int n_quad, int n_444, int n_other,
                   int max_w, int max_h, const uint2 *quad_tiles, int n_quad_tiles, const uint8_t *planes, uint8_t *rgb, const int32_t *crop_params,
-                  int n_params, bool early, cudaStream_t stream) {
+                  int n_params, bool whole_rows, bool early, cudaStream_t stream) {
     if (n_list == 0) return;
     if (n_444 > 0) {
         int gy = (max_h + 7) / 8;
         if (gy > 64) gy = 64;
         dim3 grid(((max_w + 3) / 4 + 1 + 31) / 32, gy, n_list); // + 1: a box starts up to 3 pixels into its first group
-        launch(early, grid, dim3(32, 8), 0, stream, color_444_kernel, descs, list, planes, rgb, crop_params, n_params);
+        launch(early, grid, dim3(32, 8), 0, stream, whole_rows ? color_444_kernel<true> : color_444_kernel<false>, descs, list, planes, rgb, crop_params, n_params);
     }
     if (n_quad > 0 && quad_tiles != nullptr) {
         if (n_quad_tiles > 0)
@@ -469,7 +496,7 @@ void launch_color(const ImageDesc *descs, const int32_t *list, int n_list, int n
     if (n_other > 0) {
         int bx = (max_w * max_h + 256 * 4 - 1) / (256 * 4);
         bx = bx < 1 ? 1 : (bx > 1024 ? 1024 : bx);
-        launch(early, dim3(bx, n_list), 256, 0, stream, color_other_kernel, descs, list, planes, rgb);
+        launch(early, dim3(bx, n_list), 256, 0, stream, whole_rows ? color_other_kernel<true> : color_other_kernel<false>, descs, list, planes, rgb);
     }
 }
 

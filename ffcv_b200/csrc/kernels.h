@@ -115,10 +115,11 @@ void launch_blocks(const ImageDesc *descs, const uint2 *tiles, int n_tiles, cons
 // per sample; nullptr = whole image); the other n_other images go through the generic kernel.
 // max_w / max_h bound the boxes in the list.  quad_tiles (device; may be nullptr): one entry
 // (sample, tile x | tile y << 16) per tile of 64 x 8 chroma samples the quad kernel has to
-// convert, so that it launches exactly those CTAs instead of a grid over the largest box.
+// convert, so that it launches exactly those CTAs instead of a grid over the largest box.  whole_rows: the
+// images lie in host memory or their rows do not begin on words.
 void launch_color(const ImageDesc *descs, const int32_t *list, int n_list, int n_quad, int n_444, int n_other,
                   int max_w, int max_h, const uint2 *quad_tiles, int n_quad_tiles, const uint8_t *planes,
-                  uint8_t *rgb, const int32_t *crop_params, int n_params, bool early, cudaStream_t stream);
+                  uint8_t *rgb, const int32_t *crop_params, int n_params, bool whole_rows, bool early, cudaStream_t stream);
 
 // Tiles of 64 x 8 chroma samples that cover a box of bw x bh pixels wherever it begins (a thread converts four
 // samples of a row, beginning at a multiple of four).
