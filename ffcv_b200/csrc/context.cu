@@ -27,6 +27,7 @@
 #include "decode_index.h"
 #include "jpeg_header.h"
 #include "kernels.h"
+#include "table_store.h"
 #include "types.h"
 
 using namespace ffcvb;
@@ -191,14 +192,6 @@ void stream_copy(uint8_t *dst, const uint8_t *src, size_t n) {
     }
     if (k < n) memcpy(dst + k, src + k, n - k);
 }
-
-// The distinct tables of a JPEG stream as indices into the context's stores: what all images of one
-// encoder share.
-struct TableSet {
-    uint8_t n_tab, n_dc_tab, fast, dc_tab[kMaxComponents], ac_tab[kMaxComponents]; // as in ImageDesc
-    uint16_t huff[6];                                                              // of the n_tab tables
-    uint16_t quant[kMaxComponents];
-};
 
 // What the marker segments of a JPEG stream said, as far as staging needs it.
 struct StreamHeader {
@@ -371,13 +364,10 @@ struct ffcvb_ctx {
     cudaEvent_t one_ev[16] = {};
     // Header cache: what the marker segments of a JPEG sample said, kept per sample (key: its
     // offset in the file) so that from the second epoch on staging a sample is a table look-up
-    // instead of a parse; the few distinct tables of a file live in stores of their own.
+    // instead of a parse; the few distinct tables of a file live in a store of their own.
     bool cache_headers = false; // ffcvb_set_header_cache: sample offsets identify samples (one file per context)
     HeaderCache header_cache;
-    std::vector<std::unique_ptr<HuffTable>> huff_store; // built tables
-    std::vector<std::unique_ptr<std::array<uint16_t, 64>>> quant_store;
-    std::vector<uint64_t> huff_store_hash, quant_store_hash;
-    std::vector<TableSet> table_sets;
+    TableStore tables;
     // Decode index (ffcvb_set_decode_index): a pool of device memory that keeps, per JPEG stream seen,
     // the decoder states a finished decode left behind; entries are handed out in order and never
     // moved.  Keyed by the sample's offset in the file: the context then serves one file.
@@ -582,52 +572,6 @@ size_t read_range(const Source &src, std::atomic<bool> &direct_broken, uint8_t *
     return done;
 }
 
-// Index of the table set of a parsed header (-1: the stores are full); `hash`: of its tables, three per
-// component.
-int intern_tables(ffcvb_ctx *ctx, const JpegHeader &h, const uint64_t *hash) {
-    TableSet ts;
-    memset(&ts, 0, sizeof(ts)); // compared bytewise
-    ts.fast = 1;
-    for (int k = 0; k < 2; k++) { // DC tables first
-        for (int c = 0; c < h.ncomp; c++) {
-            const RawHuff &raw = k == 0 ? h.dc[h.td[c]] : h.ac[h.ta[c]];
-            const uint64_t key = hash[3 * c + k];
-            int found = (int)ctx->huff_store.size() - 1;
-            while (found >= 0 && !(ctx->huff_store_hash[found] == key && memcmp(ctx->huff_store[found]->vals, raw.vals, 256) == 0)) found--;
-            if (found < 0) {
-                if (ctx->huff_store.size() >= 60000) return -1;
-                found = (int)ctx->huff_store.size();
-                ctx->huff_store.emplace_back(new HuffTable());
-                build_huff_table(raw, k == 0, ctx->huff_store.back().get());
-                ctx->huff_store_hash.push_back(key);
-            }
-            int u = k == 0 ? 0 : ts.n_dc_tab;
-            while (u < ts.n_tab && ts.huff[u] != (uint16_t)found) u++;
-            if (u == ts.n_tab) ts.huff[ts.n_tab++] = (uint16_t)found;
-            (k == 0 ? ts.dc_tab : ts.ac_tab)[c] = (uint8_t)u;
-            if (!ctx->huff_store[found]->fast_ok) ts.fast = 0;
-        }
-        if (k == 0) ts.n_dc_tab = ts.n_tab;
-    }
-    for (int c = 0; c < h.ncomp; c++) {
-        const uint16_t *q = h.quant[h.tq[c]];
-        int found = (int)ctx->quant_store.size() - 1;
-        while (found >= 0 && !(ctx->quant_store_hash[found] == hash[3 * c + 2] && memcmp(ctx->quant_store[found]->data(), q, 128) == 0)) found--;
-        if (found < 0) {
-            if (ctx->quant_store.size() >= 60000) return -1;
-            found = (int)ctx->quant_store.size();
-            ctx->quant_store.emplace_back(new std::array<uint16_t, 64>());
-            memcpy(ctx->quant_store.back()->data(), q, 128);
-            ctx->quant_store_hash.push_back(hash[3 * c + 2]);
-        }
-        ts.quant[c] = (uint16_t)found;
-    }
-    for (int k = (int)ctx->table_sets.size() - 1; k >= 0; k--)
-        if (memcmp(&ctx->table_sets[k], &ts, sizeof(ts)) == 0) return k;
-    ctx->table_sets.push_back(ts);
-    return (int)ctx->table_sets.size() - 1;
-}
-
 int stage_impl(ffcvb_ctx *ctx, int slot, const Source &source, const uint64_t *ptrs,
                const uint64_t *sizes, const uint8_t *modes, const uint16_t *heights,
                const uint16_t *widths, int n, const ffcvb_plan *plan, const int32_t *params) {
@@ -743,6 +687,10 @@ int stage_impl(ffcvb_ctx *ctx, int slot, const Source &source, const uint64_t *p
     auto bytes_of = [&](int i) -> const uint8_t * { return from_fd ? s.host + spans[i].dst + spans[i].skip : file_base + ptrs[i]; };
 
     // ---- headers: from the cache, or parsed (in parallel when there are many)
+    if (ctx->tables.full()) {
+        ctx->tables.clear();
+        ctx->header_cache.clear();
+    }
     s.to_parse.clear();
     for (int i = 0; i < n; i++) {
         if (modes[i] != FFCVB_MODE_JPG) continue;
@@ -792,9 +740,7 @@ int stage_impl(ffcvb_ctx *ctx, int slot, const Source &source, const uint64_t *p
         for (int k = 0; k < m; k++) { // their tables enter the stores, the headers the cache
             const int i = s.to_parse[k];
             if (s.headers[i].status != 0) continue;
-            const int set = intern_tables(ctx, s.parsed[k], s.hashes[k].data());
-            if (set < 0) return fail(ctx, FFCVB_E_LIMIT, "more than 60000 distinct Huffman or quantisation tables in a file");
-            s.headers[i].table_set = (uint32_t)set;
+            s.headers[i].table_set = ctx->tables.add(s.parsed[k], s.hashes[k].data());
             if (ctx->cache_headers && ctx->header_cache.size() < (size_t)1 << 23) // ~0.9 GB of host memory at most
                 ctx->header_cache.insert(ptrs[i], s.headers[i]);
         }
@@ -949,8 +895,7 @@ int stage_impl(ffcvb_ctx *ctx, int slot, const Source &source, const uint64_t *p
     }
     // ---- layout of the JPEG samples' work; the batch's own table lists (indices into the store ->
     // indices into the blob), worked out once per table set
-    std::vector<const HuffTable *> huff_src;
-    std::vector<const uint16_t *> mult_src;
+    std::vector<uint32_t> huff_src, mult_src;
     struct BatchSet {
         uint32_t set;
         uint8_t tab_id[6], q_tab[kMaxComponents];
@@ -1010,24 +955,22 @@ int stage_impl(ffcvb_ctx *ctx, int slot, const Source &source, const uint64_t *p
             continue;
         }
         const uint32_t set_id = s.headers[i].table_set;
-        const TableSet &ts = ctx->table_sets[set_id];
+        const TableSet &ts = ctx->tables.set(set_id);
         if (last_set < 0 || batch_sets[last_set].set != set_id) {
             for (last_set = (int)batch_sets.size() - 1; last_set >= 0 && batch_sets[last_set].set != set_id;) last_set--;
             if (last_set < 0) {
                 BatchSet bs{};
                 bs.set = set_id;
                 for (int k = 0; k < ts.n_tab; k++) {
-                    const HuffTable *t = ctx->huff_store[ts.huff[k]].get();
                     size_t u = 0;
-                    while (u < huff_src.size() && huff_src[u] != t) u++;
-                    if (u == huff_src.size()) huff_src.push_back(t);
+                    while (u < huff_src.size() && huff_src[u] != ts.huff[k]) u++;
+                    if (u == huff_src.size()) huff_src.push_back(ts.huff[k]);
                     bs.tab_id[k] = (uint8_t)u;
                 }
                 for (int c = 0; c < d.ncomp; c++) {
-                    const uint16_t *q = ctx->quant_store[ts.quant[c]]->data();
                     size_t u = 0;
-                    while (u < mult_src.size() && mult_src[u] != q) u++;
-                    if (u == mult_src.size()) mult_src.push_back(q);
+                    while (u < mult_src.size() && mult_src[u] != ts.quant[c]) u++;
+                    if (u == mult_src.size()) mult_src.push_back(ts.quant[c]);
                     bs.q_tab[c] = (uint8_t)u;
                 }
                 if (huff_src.size() > 255 || mult_src.size() > 255)
@@ -1263,9 +1206,9 @@ int stage_impl(ffcvb_ctx *ctx, int slot, const Source &source, const uint64_t *p
     memcpy(s.host, &hd, sizeof(hd));
     memcpy(s.host + hd.desc_off, descs.data(), sizeof(ImageDesc) * (size_t)n);
     for (size_t k = 0; k < huff_src.size(); k++)
-        memcpy(s.host + hd.huff_off + k * sizeof(HuffTable), huff_src[k], sizeof(HuffTable));
+        memcpy(s.host + hd.huff_off + k * sizeof(HuffTable), &ctx->tables.built(huff_src[k]), sizeof(HuffTable));
     for (size_t k = 0; k < mult_src.size(); k++)
-        build_mult_table(mult_src[k], reinterpret_cast<MultTable *>(s.host + hd.mult_off) + k);
+        build_mult_table(ctx->tables.quant(mult_src[k]), reinterpret_cast<MultTable *>(s.host + hd.mult_off) + k);
     memcpy(s.host + hd.params_off, params, sizeof(int32_t) * (size_t)n * n_params);
     {
         int32_t *st = reinterpret_cast<int32_t *>(s.host + s.status_off);

@@ -200,3 +200,18 @@ def test_imdecode_scaled_refuses_what_it_cannot_scale():
     assert imdecode(_encode(img, 90, 422), got, 64, 80, 64, 80, 0, 0, 1, 2) == -1   # 4:2:2
     assert imdecode(_encode(img, 90), got, 64, 80, 64, 80, 0, 0, 1, 3) == -1         # 1/3 is not offered
     assert imdecode(_encode(img, 90), got, 64, 80, 64, 80, 0, 0, 1, 2) == 0
+
+
+def test_streams_that_each_bring_tables_of_their_own():
+    """60 200 distinct quantisation tables, one a call, through the process-wide context: it keeps a bounded
+    number of them and goes on."""
+    from ffcv_b200.libffcv import imdecode
+    rng = np.random.default_rng(5)
+    buf = cv2.imencode('.jpg', rng.integers(0, 256, (8, 8), np.uint8), [cv2.IMWRITE_JPEG_QUALITY, 50])[1].reshape(-1).copy()
+    at = bytes(buf).index(b'\xff\xdb') + 5  # behind marker, length and destination
+    out = np.zeros((8, 8, 3), np.uint8)
+    for k in range(60200):
+        buf[at:at + 4] = 1 + k % 200, 1 + k // 200 % 200, 1 + k // 40000, 17
+        assert imdecode(buf, out, 8, 8) == 0, k
+        if k % 6000 == 0 or k > 60190:
+            assert np.array_equal(out, O.jpeg_decode(buf)), k
