@@ -424,6 +424,23 @@ int grow_host(ffcvb_ctx *ctx, uint8_t *&p, size_t &cap_io, size_t need) {
     return 0;
 }
 
+// The same for a buffer whose first `used` bytes have to stay.
+int grow_host_keeping(ffcvb_ctx *ctx, uint8_t *&p, size_t &cap_io, size_t need, size_t used) {
+    if (need <= cap_io) return 0;
+    uint8_t *larger = nullptr;
+    size_t cap = 0;
+    const int rc = grow_host(ctx, larger, cap, need);
+    if (rc) return rc;
+    if (p) {
+        memcpy(larger, p, used);
+        CU(cudaDeviceSynchronize());
+        CU(cudaFreeHost(p));
+    }
+    p = larger;
+    cap_io = cap;
+    return 0;
+}
+
 bool valid_plan(const ffcvb_plan *p) {
     if (!p || p->out_h <= 0 || p->out_w <= 0 || p->n_ops < 0 || p->n_ops > FFCVB_MAX_OPS) return false;
     if (p->out_kind < FFCVB_OUT_U8_NHWC || p->out_kind > FFCVB_OUT_F32_NCHW) return false;
@@ -669,8 +686,9 @@ int stage_impl(ffcvb_ctx *ctx, int slot, const Source &source, const uint64_t *p
             off += sp.len;
         }
         fd_payload_end = off;
-        // room behind the payloads for what is laid out after the parse: at most 255 tables of each kind
-        size_t tail = 255 * (sizeof(HuffTable) + sizeof(MultTable)) + 4 * (sizeof(int32_t) * (size_t)n + 16) + 256;
+        // room behind the payloads for what is laid out after the parse: more tables of each kind than the images of
+        // a few encoders have (with more of them the buffer grows below)
+        size_t tail = 16 * (sizeof(HuffTable) + sizeof(MultTable)) + 4 * (sizeof(int32_t) * (size_t)n + 16) + 256;
         for (int i = 0; i < n; i++) { // and the tables of CTAs: at most those of whole images and of the shortest segments
             tail += sizeof(uint2) * (size_t)quad_tiles_x(widths[i]) * quad_tiles_y(heights[i]);
             tail += sizeof(uint2) * ((size_t)((heights[i] + 15) / 8) * ((widths[i] + 15) / 8) * 3 / kBlockTile + 4);
@@ -1182,8 +1200,6 @@ int stage_impl(ffcvb_ctx *ctx, int slot, const Source &source, const uint64_t *p
     hd.total_bytes = off;
 
     int rc;
-    if (from_fd && off + 64 > s.host_cap) // the payloads already sit in the buffer: it cannot be regrown now
-        return fail(ctx, FFCVB_E_ARG, "ffcvb_stage_batch_fd: tables and lists do not fit behind the payloads");
     // A pinned source needs room for the part that is staged.  That part varies from batch to batch and
     // regrowing page-locked memory stalls the device: room for the most that the split may stage.
     size_t host_need = off;
@@ -1194,7 +1210,11 @@ int stage_impl(ffcvb_ctx *ctx, int slot, const Source &source, const uint64_t *p
         host_need = hd.payload_off + (size_t)(most * (double)(off - hd.payload_off));
         if (host_need < s.staged_end) host_need = s.staged_end;
     }
-    if ((rc = grow_host(ctx, s.host, s.host_cap, host_need + 64))) return rc;
+    if (from_fd) // (the payloads lie in the buffer already)
+        rc = grow_host_keeping(ctx, s.host, s.host_cap, host_need + 64, fd_payload_end);
+    else
+        rc = grow_host(ctx, s.host, s.host_cap, host_need + 64);
+    if (rc) return rc;
     if ((rc = grow_dev(ctx, s.blob, off + 64))) return rc;
     if ((rc = grow_dev(ctx, s.clean, clean_bytes + 512))) return rc;
     if ((rc = grow_dev(ctx, s.segs, seg_total * (sizeof(SegMeta) + 4 * kSegSubs + 16) + 64))) return rc;

@@ -494,3 +494,34 @@ def test_decode_index_gives_the_same_pixels(datasets, cfg, res, batch, epochs):
     assert seen[-1]['used'] > seen[0]['used'] and seen[-1]['used'] >= n_jpeg // 2, seen
     status = ctx.status(0, ch.cuda.current_stream().cuda_stream, 1)
     assert (status == 0).all()
+
+
+@pytest.mark.parametrize('n', [3, 40], ids=['few_tables', 'more_tables_than_expected'])
+def test_direct_read_of_streams_with_tables_of_their_own(tmp_path, n):
+    """Samples read from a file descriptor lie in the pinned buffer before their tables are known: with more tables
+    than there is room for behind them the buffer grows around the samples."""
+    import cv2
+    from ffcv_b200 import libffcv as L
+    from ffcv_b200.synthetic import synth_content
+    from parity import O
+    rng = np.random.default_rng(n)
+    bufs, h, w = [], 48, 64
+    for k in range(n):
+        flags = [cv2.IMWRITE_JPEG_QUALITY, 50 + k, cv2.IMWRITE_JPEG_OPTIMIZE, 1]
+        bufs.append(cv2.imencode('.jpg', synth_content(rng, h, w), flags)[1].reshape(-1).copy())
+    path = str(tmp_path / 'streams')
+    np.concatenate(bufs).tofile(path)
+    sizes = np.array([b.size for b in bufs], np.uint64)
+    ptrs = np.concatenate([[0], np.cumsum(sizes)[:-1]]).astype(np.uint64)
+    ctx = L.Context(0, 1, 4)
+    out = ch.zeros((n, h, w, 3), dtype=ch.uint8, device='cuda')
+    stream = ch.cuda.current_stream().cuda_stream
+    fd = os.open(path, os.O_RDONLY)
+    for _ in range(2):
+        ctx.stage(0, (fd, -1), ptrs, sizes, np.zeros(n, np.uint8), np.full(n, h, np.uint16), np.full(n, w, np.uint16),
+                  L.make_plan(h, w, 0, L.OUT_U8_NHWC), np.tile(np.array([0, 0, h, w], np.int32), (n, 1)))
+        ctx.submit(0, stream, out.data_ptr())
+        assert (ctx.status(0, stream, n) == 0).all()
+        assert np.array_equal(out.cpu().numpy(), np.stack([O.jpeg_decode(b) for b in bufs]))
+    os.close(fd)
+    ctx.close()
