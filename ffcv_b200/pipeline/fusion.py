@@ -188,7 +188,7 @@ class FusedImageExecutor:
                         np.ascontiguousarray(metadata['width'], dtype=np.uint16))
         self.sampling = _native_sampling(plan)
         self._arrays = None
-        self.last_params = None
+        self.last_params = None   # parameter table of the last batch, an array of its own
         self.param_log = None     # set to a list to record (epoch, batch, indices, parameter table) per batch
         self._last_slot = None
         self.riders = []          # other fields' values for the next batch (see Graph.attach_riders)
@@ -225,9 +225,9 @@ class FusedImageExecutor:
 
     def __call__(self, batch_indices, slot, stream_ptr, out, epoch, batch_ix, outputs_free=None):
         params = self.prepare(batch_indices, epoch, batch_ix)
-        self.last_params = params
+        self.last_params = params.copy()
         if self.param_log is not None:
-            self.param_log.append((epoch, batch_ix, np.array(batch_indices), params.copy()))
+            self.param_log.append((epoch, batch_ix, np.array(batch_indices), self.last_params))
         n = len(batch_indices)
         if self.riders:
             self.ctx.set_riders(slot, self.riders, n)

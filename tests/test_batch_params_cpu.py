@@ -38,3 +38,40 @@ def test_prepare_batch_equals_the_single_draws(n, crop):
             column = np.zeros((n, 2), np.int32)
             draw(S.batch_seed(seed, epoch, batch_ix, k + 1), column)
             assert np.array_equal(params[:, 4 + 2 * k:6 + 2 * k], column)
+
+
+def test_last_params_of_a_batch_outlive_it():
+    """The parameter table a caller took from the executor is not the array the next batch is prepared in."""
+    import torch as ch
+    from ffcv_b200.fields.decoders import RandomResizedCropRGBImageDecoder
+    from ffcv_b200.pipeline.fusion import FusedImageExecutor, FusedImagePlan
+    from ffcv_b200.transforms import RandomHorizontalFlip
+
+    class Recorder:  # in place of the native context
+        def __init__(self):
+            self.staged = []
+
+        def stage_arrays(self, slot, base, arrays, plan):
+            self.staged.append(arrays.arrays[5].copy())
+
+        def submit(self, *args):
+            pass
+
+    n = 40
+    md = np.zeros(n, dtype=[('mode', 'u1'), ('width', '<u2'), ('height', '<u2'), ('data_ptr', '<u8')])
+    md['width'], md['height'] = 300, 200
+    plan = FusedImagePlan()
+    for op in (RandomResizedCropRGBImageDecoder((32, 32)), RandomHorizontalFlip()):
+        assert op.fuse(plan)
+    plan.device = ch.device('cpu')
+    ctx = Recorder()
+    exe = FusedImageExecutor(plan, ctx, md, np.full(n, 1000, np.uint64), lambda: 0, 7)
+    exe.param_log = []
+    out = exe.allocate(16, 1)[0]
+    taken = []
+    for b in range(3):
+        exe(np.arange(16), 0, 0, out, 0, b)
+        taken.append(exe.last_params)
+    assert all(np.array_equal(t, s) for t, s in zip(taken, ctx.staged))
+    assert all(np.array_equal(t, s) for (_, _, _, t), s in zip(exe.param_log, ctx.staged))
+    assert not np.array_equal(taken[0], taken[1]) and not np.array_equal(taken[1], taken[2])
