@@ -338,6 +338,7 @@ struct ffcvb_ctx {
     std::string err;
     AuxBuf aux[16];
     int aux_next = 0;
+    std::mutex aux_m; // held from stage_aux to the recording of the buffer's event: several threads may share a context
     bool profile = false;
     bool async_staging = false;
     int cpu_share_permille = 0; // pinned source: share of the payload bytes the staging threads copy
@@ -1783,8 +1784,8 @@ int ffcvb_batch_status(ffcvb_ctx *ctx, int slot, void *stream, int32_t *status, 
 } // extern "C"
 
 // Small per-call parameter arrays travel through a ring of sixteen pinned/device buffer pairs: copies
-// the `bytes` that `fill` writes to the next pair's device side on `st`.  The caller records a->ev on
-// `st` once its kernels are queued.
+// the `bytes` that `fill` writes to the next pair's device side on `st`.  The caller holds aux_m and records
+// a->ev on `st` once its kernels are queued.
 template <class Fill>
 static int stage_aux(ffcvb_ctx *ctx, cudaStream_t st, size_t bytes, Fill &&fill, AuxBuf **out) {
     AuxBuf &a = ctx->aux[ctx->aux_next];
@@ -1811,6 +1812,7 @@ int ffcvb_transform_device(ffcvb_ctx *ctx, void *stream, const uint8_t *src_dev,
     cudaStream_t st = (cudaStream_t)stream;
     const int n_params = 4 + 2 * plan->n_ops;
     const size_t bytes = sizeof(int32_t) * (size_t)n * n_params;
+    std::lock_guard<std::mutex> guard(ctx->aux_m);
     AuxBuf *ap;
     int rc;
     if ((rc = stage_aux(ctx, st, bytes, [&](uint8_t *host) { memcpy(host, params, bytes); }, &ap))) return rc;
@@ -1852,6 +1854,7 @@ static int pixel_chain(ffcvb_ctx *ctx, void *stream, const uint8_t *src_dev, int
     const size_t entries = (size_t)n_ops * n, lam_off = sizeof(double) * entries, sums_off = lam_off + (lam ? sizeof(double) * (size_t)n : 0);
     const size_t apply_off = sums_off + sizeof(unsigned long long) * entries, bytes = apply_off + entries;
     uint8_t *dev = nullptr;
+    std::lock_guard<std::mutex> guard(ctx->aux_m);
     AuxBuf *a = nullptr;
     if (bytes > 0) {
         int rc;
@@ -1893,6 +1896,7 @@ int ffcvb_onehot_mix(ffcvb_ctx *ctx, void *stream, int n, int classes, const int
         if (label[i] < 0 || label[i] >= classes) return fail(ctx, FFCVB_E_ARG, "ffcvb_onehot_mix: label[%d] = %d with %d classes", i, label[i], classes);
     CU(cudaSetDevice(ctx->device));
     cudaStream_t st = (cudaStream_t)stream;
+    std::lock_guard<std::mutex> guard(ctx->aux_m);
     AuxBuf *a;
     int rc;
     if ((rc = stage_aux(ctx, st, 8 * (size_t)n, [&](uint8_t *host) {
@@ -1932,6 +1936,7 @@ int ffcvb_poison(ffcvb_ctx *ctx, void *stream, uint8_t *images_dev, int n, int64
         return fail(ctx, FFCVB_E_ARG, "ffcvb_poison: bad argument");
     CU(cudaSetDevice(ctx->device));
     cudaStream_t st = (cudaStream_t)stream;
+    std::lock_guard<std::mutex> guard(ctx->aux_m);
     AuxBuf *a;
     int rc;
     if ((rc = stage_aux(ctx, st, (size_t)n, [&](uint8_t *host) { memcpy(host, apply, (size_t)n); }, &a))) return rc;

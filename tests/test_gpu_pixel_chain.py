@@ -51,3 +51,35 @@ def test_mixup_of_values_that_are_no_pixels(n, count):
     ctx.mixup(ch.cuda.current_stream().cuda_stream, src.data_ptr(), dst.data_ptr(), n, count, lam)
     assert np.array_equal(dst.cpu().numpy(), O.mixup(imgs.reshape(n, 1, count, 1), lam).reshape(n, count))
     ctx.close()
+
+
+def test_threads_share_a_context():
+    """Two loaders' threads call the process-wide context at once, each on a stream of its own."""
+    import threading
+    from ffcv_b200 import libffcv as L
+    ctx = L.Context(0, 1, 1)
+    wrong = []
+
+    def work(seed):
+        rng = np.random.default_rng(seed)
+        stream = ch.cuda.Stream()
+        for round_ in range(60):
+            n, h, w = int(rng.integers(1, 200)), 4, 5
+            imgs = rng.integers(0, 256, (n, h, w, 3), dtype=np.uint8)
+            lam, apply, ratio = rng.random(n), (rng.random((1, n)) < 0.5).astype(np.uint8), rng.uniform(0.5, 1.5, (1, n))
+            with ch.cuda.stream(stream):
+                src = ch.from_numpy(imgs).cuda()
+                outs = [ch.empty_like(src) for _ in range(20)]
+                for out in outs:
+                    ctx.pixel_chain(stream.cuda_stream, src.data_ptr(), n, h * w, np.zeros(1, np.int32), apply, ratio, lam, 1, 0, out.data_ptr())
+                stream.synchronize()
+            want = O.mixup(O.color_jitter(imgs, 0, apply[0].astype(bool), ratio[0]), lam)
+            if not all(np.array_equal(out.cpu().numpy(), want) for out in outs):
+                wrong.append((seed, round_))
+    threads = [threading.Thread(target=work, args=(seed,)) for seed in range(4)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not wrong
+    ctx.close()
