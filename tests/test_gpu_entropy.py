@@ -36,9 +36,12 @@ def test_scans_around_the_segment_length(sampling):
 
 
 @pytest.mark.parametrize('n,mixed', [(739, False), (743, False), (743, True)], ids=['one_team', 'four_teams', 'tables_differ'])
-def test_batches_around_the_team_limit(n, mixed):
-    """740 segments are where four teams start to share a CTA (when all scans use the same tables)."""
+@pytest.mark.parametrize('subseq_bits', ['', '512'], ids=['from_every_slot', 'from_one_guess'])
+def test_batches_around_the_team_limit(n, mixed, subseq_bits, monkeypatch):
+    """740 segments are where four teams start to share a CTA (when all scans use the same tables): of the index
+    kernel, and, as these small batches only do when asked to, of the guess-and-repair kernel."""
     from ffcv_b200 import libffcv as L
+    monkeypatch.setenv('FFCV_B200_SUBSEQ_BITS', subseq_bits)
     rng = np.random.default_rng(n + mixed)
     h, w = 40, 56
     bufs = [_jpeg(rng, h, w, int(rng.integers(60, 98)), 444 if mixed and k % 3 == 0 else 420) for k in range(n)]
