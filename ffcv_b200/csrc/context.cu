@@ -277,7 +277,7 @@ struct Slot {
     int n_quad = 0, n_444 = 0, n_other = 0, max_w = 0, max_h = 0;
     uint64_t jpeg_list_off = 0, segs_off = 0, multi_off = 0, slot_images_off = 0, restart_off = 0, block_tiles_off = 0, quad_tiles_off = 0;
     uint64_t status_off = 0; // status word and counter of finished segments of every sample
-    int n_block_tiles = 0, n_quad_tiles = 0;
+    int n_block_tiles = 0, n_quad_tiles = 0, bands = 1;
     uint32_t total_blocks = 0;
     size_t clean_bytes = 0, plane_bytes = 0, rgb_bytes = 0, scan_bytes = 0, raw_bytes = 0, jpeg_bytes = 0;
     bool staged = false;
@@ -1263,6 +1263,7 @@ int stage_impl(ffcvb_ctx *ctx, int slot, const Source &source, const uint64_t *p
         if (descs[i].scale_shift == 0 || !plan->resize) continue;
         scaled_box(descs[i], reinterpret_cast<int32_t *>(s.host + hd.params_off) + (size_t)i * n_params);
     }
+    s.bands = resize_bands(reinterpret_cast<const int32_t *>(s.host + hd.params_off), n, n_params, plan->resize, plan->out_h, plan->out_w, plan->out_kind);
     for (const auto &r : s.riders) {
         if (!r.inline_bytes.empty()) {
             memcpy(s.host + r.off, r.inline_bytes.data(), r.bytes);
@@ -1574,7 +1575,7 @@ static int run_batch(ffcvb_ctx *ctx, Slot &s, cudaStream_t st, void *out_dev, bo
         src.rgb = rgb;
         src.planes = (const uint8_t *)s.planes.p;
         launch_resize_augment(src, s.n, params, (int)hd.n_params, make_oplist(s.plan), s.plan.resize,
-                              s.plan.out_h, s.plan.out_w, s.plan.out_kind, s.plan.lut_dev, out_dev, status, small,
+                              s.plan.out_h, s.plan.out_w, s.plan.out_kind, s.bands, s.plan.lut_dev, out_dev, status, small,
                               early && !outputs_free, st);
         for (int k = 0; k < n_large; k++) // (behind the kernel, which may have been launched early)
             CU(cudaMemcpyAsync(large[k]->dst_dev, blob + large[k]->off, large[k]->bytes, cudaMemcpyDeviceToDevice, st));
@@ -1841,7 +1842,8 @@ int ffcvb_transform_device(ffcvb_ctx *ctx, void *stream, const uint8_t *src_dev,
     src.uniform_h = h;
     src.uniform_w = w;
     launch_resize_augment(src, n, (const int32_t *)a.dev.p, n_params, make_oplist(*plan), plan->resize,
-                          plan->out_h, plan->out_w, plan->out_kind, plan->lut_dev, out_dev, nullptr, SmallCopies{}, false, st);
+                          plan->out_h, plan->out_w, plan->out_kind,
+                          resize_bands(params, n, n_params, plan->resize, plan->out_h, plan->out_w, plan->out_kind), plan->lut_dev, out_dev, nullptr, SmallCopies{}, false, st);
     CU(cudaGetLastError());
     CU(cudaEventRecord(a.ev, st));
     a.used = true;
@@ -2136,7 +2138,8 @@ void resize(int64_t cresizer, int64_t source_p, int64_t sx, int64_t sy, int64_t 
     rs.uniform_h = rows;
     rs.uniform_w = cols;
     uint8_t *out = zero_copy ? ctx->one_host + kResultHead : (uint8_t *)ctx->one_dst.p;
-    launch_resize_augment(rs, 1, (const int32_t *)ctx->one_src.p, 4, OpList{}, 1, (int)tx, (int)ty, FFCVB_OUT_U8_NHWC, nullptr, out, nullptr, SmallCopies{}, false, st);
+    launch_resize_augment(rs, 1, (const int32_t *)ctx->one_src.p, 4, OpList{}, 1, (int)tx, (int)ty, FFCVB_OUT_U8_NHWC,
+                          resize_bands(params, 1, 4, 1, (int)tx, (int)ty, FFCVB_OUT_U8_NHWC), nullptr, out, nullptr, SmallCopies{}, false, st);
     if (cudaGetLastError() != cudaSuccess) return;
     if (zero_copy) {
         if (cudaStreamSynchronize(st) == cudaSuccess) memcpy((void *)(intptr_t)dest_p, out, dst_bytes);

@@ -200,9 +200,15 @@ FFCVB_HD inline uint64_t small_copy_words(uint64_t bytes, const void *src, const
     return bytes / word + (bytes % word != 0);
 }
 
+// CTAs per image of the kernel below: as many as the image with the most bands has, at most enough of them for
+// about eight waves of the GPU (148 SMs x 4 resident CTAs; fewer waves measured slower, more cost the set-up its
+// amortisation).  `params` is in host memory.  Worth a look at every box: a CTA without a band costs as much set-up as
+// one with (512 images of 32x32 pixels to 24x24: 21 us, 36 with a CTA for every four rows; 256 of 192x192 to 96x96: 39 and 60).
+int resize_bands(const int32_t *params, int n, int n_params, int resize, int out_h, int out_w, int out_kind);
+
 // Fused crop + INTER_AREA resize + flip/translate/cutout + lookup-table normalise.
 void launch_resize_augment(const ResizeSource &src, int n, const int32_t *params, int n_params,
-                           const OpList &ops, int resize, int out_h, int out_w, int out_kind,
+                           const OpList &ops, int resize, int out_h, int out_w, int out_kind, int bands,
                            const void *lut, void *out, const int32_t *status, const SmallCopies &small, bool early, cudaStream_t stream);
 
 // Colour jitter kinds (ffcv/transforms/color_jitter.py).

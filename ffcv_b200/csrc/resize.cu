@@ -655,37 +655,48 @@ ResizeShape resize_shape(int n, int out_h, int out_w, int out_kind) {
     return s;
 }
 
+int resize_bands(const int32_t *params, int n, int n_params, int resize, int out_h, int out_w, int out_kind) {
+    const ResizeShape shape = resize_shape(n, out_h, out_w, out_kind);
+    const size_t elem = out_kind == kOutU8 ? 1 : (out_kind == kOutF16Nhwc || out_kind == kOutF16Nchw ? 2 : 4), tile_row = (size_t)out_w * 3 * elem;
+    const int plain = (out_h + shape.band - 1) / shape.band, most = (8 * 148 * 4 + n - 1) / n;
+    int bands = 1;
+    for (int i = 0; i < n && bands < most; i++) {
+        const int32_t *box = params + (size_t)i * n_params;
+        int mine = plain;
+        if (resize && box[2] > 0 && box[3] > 0) {
+            const Scaling sc = scaling_of(box[2], box[3], out_h, out_w);
+            const int window = sc.regime == kArea || sc.regime == kLinear ? window_band(box[3], sc.sc_y, tile_row, shape) : 0;
+            if (window) mine = (out_h + window - 1) / window;
+        }
+        if (mine > bands) bands = mine;
+        if (!resize) break; // (all alike)
+    }
+    return bands < most ? bands : most;
+}
+
 template <typename OutT>
 static void launch_typed(const ResizeSource &src, int n, const int32_t *params, int n_params, const OpList &ops,
-                         int resize, int out_h, int out_w, int planar, const ResizeShape &shape, const void *lut, void *out,
+                         int resize, int out_h, int out_w, int planar, const ResizeShape &shape, int bands, const void *lut, void *out,
                          const int32_t *status, const SmallCopies &small, bool early, cudaStream_t stream) {
     auto kern = resize_augment_kernel<OutT>;
     if (shape.smem > 48 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shape.smem);
-    // CTAs per image: enough of them for about eight waves of the GPU (148 SMs x 4 resident CTAs;
-    // fewer waves measured slower, more cost the set-up its amortisation), at most one per band (a sample
-    // whose window holds fewer rows has more of them, of at least four rows; without scaling there is no window:
-    // 512 images of 32x32 pixels take 15 us in one CTA each, 31 with seven idle ones beside it)
-    const int least = resize && shape.room && shape.band > 4 ? 4 : shape.band, nbands = (out_h + least - 1) / least;
-    int per_image = (8 * 148 * 4 + n - 1) / n;
-    if (per_image > nbands) per_image = nbands;
-    if (per_image < 1) per_image = 1;
-    dim3 grid(per_image, n);
+    dim3 grid(bands, n);
     launch(early, grid, 256, shape.smem, stream, kern, src, params, n_params, ops, resize, out_h, out_w, shape, planar, (const OutT *)lut, (OutT *)out,
            status, small);
 }
 
 void launch_resize_augment(const ResizeSource &src, int n, const int32_t *params, int n_params,
-                           const OpList &ops, int resize, int out_h, int out_w, int out_kind,
+                           const OpList &ops, int resize, int out_h, int out_w, int out_kind, int bands,
                            const void *lut, void *out, const int32_t *status, const SmallCopies &small, bool early, cudaStream_t stream) {
     if (n <= 0) return;
     const int planar = out_kind == kOutF16Nchw || out_kind == kOutF32Nchw;
     const ResizeShape shape = resize_shape(n, out_h, out_w, out_kind);
     if (out_kind == kOutU8)
-        launch_typed<uint8_t>(src, n, params, n_params, ops, resize, out_h, out_w, 0, shape, nullptr, out, status, small, early, stream);
+        launch_typed<uint8_t>(src, n, params, n_params, ops, resize, out_h, out_w, 0, shape, bands, nullptr, out, status, small, early, stream);
     else if (out_kind == kOutF16Nhwc || out_kind == kOutF16Nchw)
-        launch_typed<uint16_t>(src, n, params, n_params, ops, resize, out_h, out_w, planar, shape, lut, out, status, small, early, stream);
+        launch_typed<uint16_t>(src, n, params, n_params, ops, resize, out_h, out_w, planar, shape, bands, lut, out, status, small, early, stream);
     else
-        launch_typed<uint32_t>(src, n, params, n_params, ops, resize, out_h, out_w, planar, shape, lut, out, status, small, early, stream);
+        launch_typed<uint32_t>(src, n, params, n_params, ops, resize, out_h, out_w, planar, shape, bands, lut, out, status, small, early, stream);
 }
 
 } // namespace ffcvb
