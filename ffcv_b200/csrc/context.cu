@@ -1862,18 +1862,21 @@ static int pixel_chain(ffcvb_ctx *ctx, void *stream, const uint8_t *src_dev, int
     PixelChain chain{};
     chain.n = n;
     chain.n_ops = n_ops;
+    bool contrast = false;
     for (int k = 0; k < n_ops; k++) {
         if (kinds[k] < FFCVB_JITTER_BRIGHTNESS || kinds[k] > FFCVB_JITTER_SATURATION)
             return fail(ctx, FFCVB_E_ARG, "ffcvb_pixel_chain: unknown operation %d", kinds[k]);
         chain.kind[k] = kinds[k];
+        contrast = contrast || kinds[k] == FFCVB_JITTER_CONTRAST;
     }
     for (int i = 0; lam && i < n; i++)
         if (!(lam[i] >= 0.0 && lam[i] <= 1.0)) return fail(ctx, FFCVB_E_ARG, "ffcvb_pixel_chain: lam[%d] outside [0, 1]", i);
     CU(cudaSetDevice(ctx->device));
     cudaStream_t st = (cudaStream_t)stream;
-    // [ratio: doubles][lam: doubles][grey sums: zeroes][apply: bytes]
+    // [ratio: doubles][lam: doubles][grey sums: zeroes, if there is a contrast][apply: bytes].  (A copy of up to one
+    // kilobyte arrives 4 us sooner than a larger one.)
     const size_t entries = (size_t)n_ops * n, lam_off = sizeof(double) * entries, sums_off = lam_off + (lam ? sizeof(double) * (size_t)n : 0);
-    const size_t apply_off = sums_off + sizeof(unsigned long long) * entries, bytes = apply_off + entries;
+    const size_t sums = contrast ? sizeof(unsigned long long) * entries : 0, apply_off = sums_off + sums, bytes = apply_off + entries;
     uint8_t *dev = nullptr;
     std::lock_guard<std::mutex> guard(ctx->aux_m);
     AuxBuf *a = nullptr;
@@ -1882,7 +1885,7 @@ static int pixel_chain(ffcvb_ctx *ctx, void *stream, const uint8_t *src_dev, int
         if ((rc = stage_aux(ctx, st, bytes, [&](uint8_t *host) {
                  if (entries) memcpy(host, ratio, sizeof(double) * entries);
                  if (lam) memcpy(host + lam_off, lam, sizeof(double) * (size_t)n);
-                 memset(host + sums_off, 0, sizeof(unsigned long long) * entries);
+                 memset(host + sums_off, 0, sums);
                  if (entries) memcpy(host + apply_off, apply, entries);
              }, &a)))
             return rc;

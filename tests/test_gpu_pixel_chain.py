@@ -83,3 +83,23 @@ def test_threads_share_a_context():
         t.join()
     assert not wrong
     ctx.close()
+
+
+@pytest.mark.parametrize('kind', [0, 1, 2])
+@pytest.mark.parametrize('shape', [(1, 1, 1), (5, 3, 7), (3, 16, 20), (130, 8, 8)], ids=str)
+def test_one_operation_in_place(shape, kind):
+    """A jitter alone has a kernel of its own: words and single pixels, factors far outside a byte's range, images that
+    are left alone."""
+    from ffcv_b200 import libffcv as L
+    n, h, w = shape
+    rng = np.random.default_rng(n + kind)
+    imgs = rng.integers(0, 256, (n, h, w, 3), dtype=np.uint8)
+    apply, ratio = (rng.random(n) < 0.6).astype(np.uint8), rng.uniform(0.0, 2.5, n)
+    apply[0], ratio[0] = 1, 3e7
+    if n > 1:
+        apply[1], ratio[1] = 1, -4.0
+    ctx = L.Context(0, 1, 1)
+    dev = ch.from_numpy(imgs).cuda()
+    ctx.color_jitter(ch.cuda.current_stream().cuda_stream, dev.data_ptr(), n, h, w, kind, apply, ratio)
+    assert np.array_equal(dev.cpu().numpy(), O.color_jitter(imgs, kind, apply.astype(bool), ratio))
+    ctx.close()
