@@ -88,11 +88,12 @@ struct ScanLayout {
 };
 ScanLayout layout_scan(uint32_t scan_len, uint32_t target_bits);
 // The same for a scan decoded from every slot at once, which is done while a batch's scans leave most of
-// the GPU idle otherwise: three times the work, but a chain of 4 x 512 bits instead of 6 to 10 kbit.  Measured on
-// batches of 224x256 to 400x500 photographs: 193 -> 137 us at 1 image, 399 -> 355 at 15 Mbit, 771 -> 754 at
-// 45 Mbit, even at 60.
+// the GPU idle otherwise: three times the work, but a chain of 4 x 512 bits instead of 6 to 10 kbit.  Kernels of a
+// batch of 4:2:0 photographs, alone / as one of four in flight, from every slot and from one guess: 0.2 Mbit 77 / 23
+// and 96 / 27 us, 2.3 Mbit 95 / 43 and 135 / 61, 9.5 Mbit 153 / 76 and 164 / 74, 16 Mbit 195 / 125 and 200 / 98, 25 Mbit
+// 274 / 203 and 240 / 140, 38 Mbit 362 / 289 and 279 / 190.
 ScanLayout layout_scan_slots(uint32_t scan_len);
-constexpr uint64_t kSlotModeBits = 40u << 20; // of a batch, at most
+constexpr uint64_t kSlotModeBits = 16u << 20; // of a batch, at most
 // Subsequence length for a batch with `total_bits` of scans: long ones re-synchronise fewer times,
 // short ones spread few scans over the GPU.
 uint32_t subseq_target(uint64_t total_bits);
