@@ -770,6 +770,7 @@ int stage_impl(ffcvb_ctx *ctx, int slot, const Source &source, const uint64_t *p
                 th[1] = hash_bytes(h.ac[h.ta[c]].bits, 17 + 256) | 1ull;
                 th[2] = hash_bytes(h.quant[h.tq[c]], 128);
             }
+            o.table_set = ctx->tables.find(h, s.hashes[k].data()); // (here, where the tables are in this thread's cache)
         };
         if (m < 12) // waking the staging threads takes longer
             for (int k = 0; k < m; k++) parse(k);
@@ -778,7 +779,7 @@ int stage_impl(ffcvb_ctx *ctx, int slot, const Source &source, const uint64_t *p
         for (int k = 0; k < m; k++) { // their tables enter the stores, the headers the cache
             const int i = s.to_parse[k];
             if (s.headers[i].status != 0) continue;
-            s.headers[i].table_set = ctx->tables.add(s.parsed[k], s.hashes[k].data());
+            if (s.headers[i].table_set == TableStore::kNone) s.headers[i].table_set = ctx->tables.add(s.parsed[k], s.hashes[k].data());
             if (ctx->cache_headers && ctx->header_cache.size() < (size_t)1 << 23) // ~0.9 GB of host memory at most
                 ctx->header_cache.insert(ptrs[i], s.headers[i]);
         }

@@ -17,7 +17,7 @@ namespace ffcvb {
 
 // The distinct tables of a JPEG stream: what all images of one encoder share.
 struct TableSet {
-    uint8_t n_tab, n_dc_tab, fast, dc_tab[kMaxComponents], ac_tab[kMaxComponents]; // as in ImageDesc
+    uint8_t ncomp, n_tab, n_dc_tab, fast, dc_tab[kMaxComponents], ac_tab[kMaxComponents]; // as in ImageDesc
     uint32_t huff[6];                                                              // of the n_tab tables
     uint32_t quant[kMaxComponents];
 };
@@ -36,10 +36,22 @@ class TableStore {
         for (Built &b : built_) b.index = kNone;
     }
 
-    // Index of the table set of a parsed header; `hash`: of its tables, three per component (DC, AC, quantisation).
+    static constexpr uint32_t kNone = 0xFFFFFFFFu;
+    // Index of the table set of a parsed header, kNone if it is not there; `hash`: of its tables, three per component
+    // (DC, AC, quantisation).  Several threads may look at once.
+    uint32_t find(const JpegHeader &h, const uint64_t *hash) const {
+        const auto range = set_by_hash_.equal_range(key_of(h, hash));
+        for (auto it = range.first; it != range.second; ++it)
+            if (is(sets_[it->second], h)) return it->second;
+        return kNone;
+    }
+    // The same, put there if it is not.
     uint32_t add(const JpegHeader &h, const uint64_t *hash) {
+        const uint32_t known = find(h, hash);
+        if (known != kNone) return known;
         TableSet ts;
-        memset(&ts, 0, sizeof(ts)); // compared bytewise
+        memset(&ts, 0, sizeof(ts));
+        ts.ncomp = (uint8_t)h.ncomp;
         ts.fast = 1;
         for (int k = 0; k < 2; k++) { // DC tables first
             for (int c = 0; c < h.ncomp; c++) {
@@ -52,13 +64,8 @@ class TableStore {
             }
             if (k == 0) ts.n_dc_tab = ts.n_tab;
         }
-        uint64_t key = 0;
         for (int c = 0; c < h.ncomp; c++) ts.quant[c] = add_quant(h.quant[h.tq[c]], hash[3 * c + 2]);
-        for (int c = 0; c < 3 * h.ncomp; c++) key = (key ^ hash[c]) * 0xFF51AFD7ED558CCDull, key ^= key >> 29;
-        const auto range = set_by_hash_.equal_range(key);
-        for (auto it = range.first; it != range.second; ++it)
-            if (memcmp(&sets_[it->second], &ts, sizeof(ts)) == 0) return it->second;
-        set_by_hash_.emplace(key, (uint32_t)sets_.size());
+        set_by_hash_.emplace(key_of(h, hash), (uint32_t)sets_.size());
         sets_.push_back(ts);
         return (uint32_t)sets_.size() - 1;
     }
@@ -66,7 +73,7 @@ class TableStore {
         const auto range = huff_by_hash_.equal_range(hash);
         for (auto it = range.first; it != range.second; ++it) {
             const Huff &t = huff_[it->second];
-            if (t.dc == dc && memcmp(t.raw.bits, raw.bits, 17) == 0 && memcmp(t.raw.vals, raw.vals, 256) == 0) return it->second;
+            if (t.dc == dc && same(t.raw, raw)) return it->second;
         }
         const uint32_t index = (uint32_t)huff_.size();
         huff_by_hash_.emplace(hash, index);
@@ -99,7 +106,7 @@ class TableStore {
     }
 
   private:
-    static constexpr uint32_t kNone = 0xFFFFFFFFu, kBuilt = 256; // (a batch has at most 255)
+    static constexpr uint32_t kBuilt = 256; // (a batch has at most 255)
     struct Huff {
         RawHuff raw;
         bool dc, fast;
@@ -108,6 +115,27 @@ class TableStore {
         uint32_t index = kNone;
         std::unique_ptr<HuffTable> table;
     };
+    static bool same(const RawHuff &a, const RawHuff &b) { return memcmp(a.bits, b.bits, 17) == 0 && memcmp(a.vals, b.vals, 256) == 0; }
+    static uint64_t key_of(const JpegHeader &h, const uint64_t *hash) {
+        uint64_t key = (uint64_t)h.ncomp;
+        for (int c = 0; c < 3 * h.ncomp; c++) {
+            key = (key ^ hash[c]) * 0xFF51AFD7ED558CCDull;
+            key ^= key >> 29;
+        }
+        return key;
+    }
+    // Whether `ts` holds the tables of this header, each where its components look for it.
+    bool is(const TableSet &ts, const JpegHeader &h) const {
+        if (ts.ncomp != h.ncomp) return false;
+        for (int c = 0; c < h.ncomp; c++) {
+            if (c == 2 && h.td[2] == h.td[1] && h.ta[2] == h.ta[1] && h.tq[2] == h.tq[1])
+                return ts.dc_tab[2] == ts.dc_tab[1] && ts.ac_tab[2] == ts.ac_tab[1] && ts.quant[2] == ts.quant[1];
+            if (!same(huff_[ts.huff[ts.dc_tab[c]]].raw, h.dc[h.td[c]]) || !same(huff_[ts.huff[ts.ac_tab[c]]].raw, h.ac[h.ta[c]]) ||
+                memcmp(quant_[ts.quant[c]].data(), h.quant[h.tq[c]], 128) != 0)
+                return false;
+        }
+        return true;
+    }
     std::vector<Huff> huff_;
     std::vector<std::array<uint16_t, 64>> quant_;
     std::vector<TableSet> sets_;

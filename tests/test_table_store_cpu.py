@@ -54,15 +54,27 @@ int main() {
     CHECK(iq != ir && store.add_quant(q, 9) == iq && store.quant(ir)[63] == 1);
     store.clear();
 
+    // headers whose hashes are all alike, in more or fewer components
+    uint64_t none[9] = {};
+    JpegHeader heads[5] = {header(1), header(2), header(1), header(1), header(1)};
+    heads[2].ta[2] = 0;
+    heads[3].tq[1] = 0;
+    heads[4].ncomp = 1;
+    for (int k = 0; k < 5; k++) CHECK(store.find(heads[k], none) == TableStore::kNone && store.add(heads[k], none) == (uint32_t)k);
+    for (int k = 0; k < 5; k++) CHECK(store.find(heads[k], none) == (uint32_t)k);
+    CHECK(store.set(2).ac_tab[2] == store.set(2).ac_tab[0] && store.set(3).quant[1] == store.set(3).quant[0]);
+    store.clear();
+
     // as many distinct tables as are kept, four a header
     const size_t before = mallinfo2().uordblks + mallinfo2().hblkhd;
     unsigned n = 0;
-    uint64_t hash[9];
+    uint64_t hash[9] = {};
     for (; !store.full(); n++) {
         const JpegHeader h = header(n);
         for (int k = 0; k < 9; k++) hash[k] = (uint64_t)n * 16 + (k < 3 ? k : 3 + k % 3);
+        CHECK(n % 1000 != 0 || store.find(h, hash) == TableStore::kNone);
         const uint32_t set = store.add(h, hash);
-        CHECK(set == n && store.add(h, hash) == set);
+        CHECK(set == n && store.add(h, hash) == set && store.find(h, hash) == set);
         const TableSet &ts = store.set(set);
         CHECK(ts.n_tab == 4 && ts.n_dc_tab == 2 && ts.dc_tab[0] == 0 && ts.dc_tab[1] == 1 && ts.dc_tab[2] == 1 && ts.ac_tab[0] == 2 && ts.ac_tab[2] == 3);
     }
