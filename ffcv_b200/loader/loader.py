@@ -85,8 +85,8 @@ class Loader:
         most ``FFCV_B200_PIN_LIMIT_GB`` (default 64) GiB and the copies of all ranks of the host
         (``LOCAL_WORLD_SIZE``) fit half of the memory available now; else the staged path is used.
         Measured on config 2: 1 GPU + 16 threads
-        255-270 k img/s staged, 250-270 k gathered, 300-330 k split (below); 8 GPUs + 32 cores
-        326 k staged, 1.15 M gathered.  ``FFCV_B200_PIN_FILE`` = 0 / 1 overrides.
+        258 k img/s staged, 282-293 k gathered, 280-312 k split (below); 8 GPUs + 32 cores, with
+        former kernels, 326 k staged, 1.15 M gathered.  ``FFCV_B200_PIN_FILE`` = 0 / 1 overrides.
     decode_index_gb : float
         (not in the reference; off by default) GiB of GPU memory for a decode index: the first
         decode of every JPEG sample records the decoder's state at the start of each of its
