@@ -8,12 +8,15 @@ namespace {
 
 // The bytes go through shared memory as bulk copies (host -> shared, shared -> device) that one thread
 // per CTA issues: a ring of kStages pieces per CTA, half of them on their way in while the others leave.
-// What bounds it is the link: one CTA per SM with 8 KB moves 46-48 GB/s of JPEG streams and 39-42 GB/s of
-// 0.7 KB crop rows inside the loader's pipeline (a plain DMA copy: 54.5; 64 CTAs: 33 GB/s of rows; two per SM:
-// 3 % more rows, but the decode kernels beside it slow down by as much), against 36-45 and 26-39 GB/s of a
-// kernel of 16 x 256 threads with eight 16-byte loads each.  As important is what it leaves to the decode
+// What bounds it is the link, and there the number of read requests: about 400 million a second, one for every
+// line of 128 bytes that a piece touches.  Pieces therefore end at multiples of kLine of the source, so that no
+// line is asked for twice: alone, one CTA per SM with 8 KB moves 49.5 / 50.3 / 50.9 GB/s of JPEG streams of 16 KB,
+// 60 KB and 1.7 MB (46.7 / 47.3 / 48.0 with pieces cut from the stream's first word on) and 44.7 GB/s of 0.7 KB crop
+// rows (44.1); pieces of 512 bytes and of 2 KB: the same.  A plain DMA copy: 54.5; 64 CTAs: 33 GB/s of rows; two per SM:
+// 3 % more rows, but the decode kernels beside it slow down by as much.  As important is what it leaves to the decode
 // kernels: no issue slots, and 8 KB of shared memory per SM, which two CTAs of the entropy decoder do not need.
 constexpr int kStages = 8, kPiece = 1024, kAhead = 5; // kAhead: pieces on their way in
+constexpr uint32_t kLine = 128;
 
 __device__ __forceinline__ uint32_t shared_address(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
@@ -65,10 +68,12 @@ __device__ __forceinline__ void store_oldest(Ring &r, uint8_t *buf, uint64_t *ba
 
 // Sends `len` bytes (a multiple of 16, as both addresses) through the ring.
 __device__ __forceinline__ void send(Ring &r, uint8_t *buf, uint64_t *bars, uint8_t *blob, uint64_t src, uint64_t dst, uint32_t len) {
-    for (uint32_t off = 0; off < len && !r.failed; off += kPiece) {
+    uint32_t take;
+    for (uint32_t off = 0; off < len && !r.failed; off += take) {
         if (r.issued - r.stored >= kAhead) store_oldest(r, buf, bars, blob);
         if (r.failed) return;
-        const uint32_t st = r.issued % kStages, take = min(len - off, (uint32_t)kPiece);
+        const uint32_t st = r.issued % kStages;
+        take = min(len - off, (uint32_t)kPiece - ((uint32_t)(src + off) & (kLine - 1)));
         // the piece that used this stage last has been read out: at most kStages - kAhead stores are younger
         if (r.issued >= kStages) asm volatile("cp.async.bulk.wait_group.read %0;" ::"n"(kStages - kAhead) : "memory");
         asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(shared_address(&bars[st])), "r"(take) : "memory");
