@@ -277,6 +277,7 @@ struct Slot {
     int n_quad = 0, n_444 = 0, n_other = 0, max_w = 0, max_h = 0;
     uint64_t jpeg_list_off = 0, segs_off = 0, multi_off = 0, slot_images_off = 0, restart_off = 0, block_tiles_off = 0, quad_tiles_off = 0;
     uint64_t status_off = 0; // status word and counter of finished segments of every sample
+    uint64_t items_off = 0;  // ResizeItem of every sample
     int n_block_tiles = 0, n_quad_tiles = 0, bands = 1;
     uint32_t total_blocks = 0;
     size_t clean_bytes = 0, plane_bytes = 0, rgb_bytes = 0, scan_bytes = 0, raw_bytes = 0, jpeg_bytes = 0;
@@ -309,6 +310,7 @@ struct Slot {
     std::vector<int> to_parse;
     std::vector<JpegHeader> parsed;
     std::vector<std::array<uint64_t, 9>> hashes; // of a parsed header's (DC, AC, quantisation) tables x 3 components
+    std::vector<ResizeItem> items;
     std::vector<int32_t> jpeg_list, multi, slot_images, restart;
     std::vector<uint2> slot_segs;  // those of slot_images, behind
     std::vector<uint2> seg_list;   // (sample, segment) of the entropy decoder's CTAs
@@ -679,6 +681,7 @@ int stage_impl(ffcvb_ctx *ctx, int slot, const Source &source, const uint64_t *p
         off = align_up(off + sizeof(ImageDesc) * (size_t)n, 16);
         off = align_up(off + sizeof(int32_t) * (size_t)n * n_params_early, 16);
         off = align_up(off + 2 * sizeof(int32_t) * (size_t)n, 16);
+        if (plan->resize) off += sizeof(ResizeItem) * (size_t)n;
         for (const auto &r : s.pending_riders) off = align_up(off, 64) + r.item_bytes * (uint64_t)n;
         fd_payload_begin = off = align_up(off, A);
         spans.resize(n);
@@ -983,10 +986,26 @@ int stage_impl(ffcvb_ctx *ctx, int slot, const Source &source, const uint64_t *p
     s.index_life = ctx->index_life;
     int max_w = 0, max_h = 0, n_quad = 0, n_444 = 0, n_other = 0;
     const bool can_fuse = plan->resize && !s.packed;
-    const ResizeShape shape = can_fuse ? resize_shape(n, plan->out_h, plan->out_w, plan->out_kind) : ResizeShape{};
-    const size_t tile_row = (size_t)plan->out_w * 3 * (plan->out_kind == FFCVB_OUT_U8_NHWC ? 1 : (plan->out_kind == FFCVB_OUT_F16_NHWC || plan->out_kind == FFCVB_OUT_F16_NCHW ? 2 : 4));
+    ResizeItems items(n, plan->out_h, plan->out_w, plan->out_kind);
+    s.items.resize(plan->resize ? n : 0);
     for (int i = 0; i < n; i++) {
         ImageDesc &d = descs[i];
+        if (plan->resize) {
+            // The resize kernel converts the planes of a 4:2:0 or equal-resolution image itself, into its window
+            // of source pixels, if the regime is one that works from a window and enough rows fit.
+            int32_t box[4];
+            memcpy(box, params + (size_t)i * n_params, sizeof(box));
+            if (d.scale_shift) scaled_box(d, box);
+            ResizeItems::Fuse fuse = ResizeItems::kPacked;
+            if (can_fuse && d.mode == FFCVB_MODE_JPG && d.host_status == 0 && d.ncomp == 3) {
+                if (d.scale_shift != 0 || (d.hs == 1 && d.vs == 1))
+                    fuse = ResizeItems::kFusePlain;
+                else if (d.hs == 2 && d.vs == 2 && (d.width + 1) / 2 >= 3)
+                    fuse = ResizeItems::kFuseQuad;
+            }
+            s.items[i] = items.make(box, d.dec_height, d.dec_width, fuse);
+            if (fuse != ResizeItems::kPacked) d.fuse_rows = (uint16_t)s.items[i].window;
+        }
         if (d.mode != FFCVB_MODE_JPG) continue;
         jpeg_list.push_back(i);
         if (d.host_status != 0) { // (no kernel touches it: its status word says so)
@@ -1077,20 +1096,6 @@ int stage_impl(ffcvb_ctx *ctx, int slot, const Source &source, const uint64_t *p
             const size_t ph = (size_t)d.mcus_y * (c == 0 ? d.vs * d.bs_luma : d.bs_chroma);
             plane_bytes += align_up(pw * ph, 16);
         }
-        if (can_fuse && d.host_status == 0) {
-            // The resize kernel converts the planes of a 4:2:0 or equal-resolution image itself, into its window
-            // of source pixels, if the regime is one that works from a window and enough rows fit.
-            int32_t box[4];
-            memcpy(box, params + (size_t)i * n_params, sizeof(box));
-            const bool quad = d.ncomp == 3 && d.scale_shift == 0 && d.hs == 2 && d.vs == 2 && (d.width + 1) / 2 >= 3;
-            const bool plain = d.ncomp == 3 && (d.scale_shift != 0 || (d.hs == 1 && d.vs == 1));
-            if ((quad || plain) && box[0] >= 0 && box[1] >= 0 && box[2] > 0 && box[3] > 0 && box[0] + box[2] <= (int)d.height &&
-                box[1] + box[3] <= (int)d.width) {
-                scaled_box(d, box);
-                const Scaling sc = scaling_of(box[2], box[3], plan->out_h, plan->out_w);
-                if (sc.regime == kArea || sc.regime == kLinear) d.fuse_rows = (uint16_t)window_band(box[3], sc.sc_y, tile_row, shape);
-            }
-        }
         d.rgb_off = rgb_bytes;
         d.rgb_pitch = s.packed ? (uint32_t)d.dec_width * 3 : (uint32_t)align_up((size_t)d.dec_width * 3, 16);
         if (d.fuse_rows) continue;
@@ -1161,6 +1166,8 @@ int stage_impl(ffcvb_ctx *ctx, int slot, const Source &source, const uint64_t *p
     off = align_up(off + sizeof(int32_t) * (size_t)n * n_params, 16);
     s.status_off = off;
     off = align_up(off + 2 * sizeof(int32_t) * (size_t)n, 16);
+    s.items_off = off;
+    off += sizeof(ResizeItem) * s.items.size();
     s.riders.swap(s.pending_riders);
     s.pending_riders.clear();
     for (auto &r : s.riders) {
@@ -1264,7 +1271,8 @@ int stage_impl(ffcvb_ctx *ctx, int slot, const Source &source, const uint64_t *p
         if (descs[i].scale_shift == 0 || !plan->resize) continue;
         scaled_box(descs[i], reinterpret_cast<int32_t *>(s.host + hd.params_off) + (size_t)i * n_params);
     }
-    s.bands = resize_bands(reinterpret_cast<const int32_t *>(s.host + hd.params_off), n, n_params, plan->resize, plan->out_h, plan->out_w, plan->out_kind);
+    if (!s.items.empty()) memcpy(s.host + s.items_off, s.items.data(), sizeof(ResizeItem) * s.items.size());
+    s.bands = items.bands();
     for (const auto &r : s.riders) {
         if (!r.inline_bytes.empty()) {
             memcpy(s.host + r.off, r.inline_bytes.data(), r.bytes);
@@ -1575,7 +1583,7 @@ static int run_batch(ffcvb_ctx *ctx, Slot &s, cudaStream_t st, void *out_dev, bo
         src.blob = blob;
         src.rgb = rgb;
         src.planes = (const uint8_t *)s.planes.p;
-        launch_resize_augment(src, s.n, params, (int)hd.n_params, make_oplist(s.plan), s.plan.resize,
+        launch_resize_augment(src, s.n, params, (int)hd.n_params, reinterpret_cast<const ResizeItem *>(blob + s.items_off), make_oplist(s.plan), s.plan.resize,
                               s.plan.out_h, s.plan.out_w, s.plan.out_kind, s.bands, s.plan.lut_dev, out_dev, status, small,
                               early && !outputs_free, st);
         for (int k = 0; k < n_large; k++) // (behind the kernel, which may have been launched early)
@@ -1832,19 +1840,24 @@ int ffcvb_transform_device(ffcvb_ctx *ctx, void *stream, const uint8_t *src_dev,
     CU(cudaSetDevice(ctx->device));
     cudaStream_t st = (cudaStream_t)stream;
     const int n_params = 4 + 2 * plan->n_ops;
-    const size_t bytes = sizeof(int32_t) * (size_t)n * n_params;
+    const size_t items_off = plan->resize ? sizeof(ResizeItem) * (size_t)n : 0, bytes = items_off + sizeof(int32_t) * (size_t)n * n_params; // (the items lie first)
+    ResizeItems items(n, plan->out_h, plan->out_w, plan->out_kind);
     std::lock_guard<std::mutex> guard(ctx->aux_m);
     AuxBuf *ap;
     int rc;
-    if ((rc = stage_aux(ctx, st, bytes, [&](uint8_t *host) { memcpy(host, params, bytes); }, &ap))) return rc;
+    if ((rc = stage_aux(ctx, st, bytes, [&](uint8_t *host) {
+             for (int i = 0; i < n && plan->resize; i++)
+                 reinterpret_cast<ResizeItem *>(host)[i] = items.make(params + (size_t)i * n_params, h, w, ResizeItems::kPacked);
+             memcpy(host + items_off, params, bytes - items_off);
+         }, &ap)))
+        return rc;
     AuxBuf &a = *ap;
     ResizeSource src{};
     src.uniform = src_dev;
     src.uniform_h = h;
     src.uniform_w = w;
-    launch_resize_augment(src, n, (const int32_t *)a.dev.p, n_params, make_oplist(*plan), plan->resize,
-                          plan->out_h, plan->out_w, plan->out_kind,
-                          resize_bands(params, n, n_params, plan->resize, plan->out_h, plan->out_w, plan->out_kind), plan->lut_dev, out_dev, nullptr, SmallCopies{}, false, st);
+    launch_resize_augment(src, n, (const int32_t *)((const uint8_t *)a.dev.p + items_off), n_params, (const ResizeItem *)a.dev.p, make_oplist(*plan), plan->resize,
+                          plan->out_h, plan->out_w, plan->out_kind, items.bands(), plan->lut_dev, out_dev, nullptr, SmallCopies{}, false, st);
     CU(cudaGetLastError());
     CU(cudaEventRecord(a.ev, st));
     a.used = true;
@@ -2017,6 +2030,7 @@ static ffcvb_ctx *global_ctx() {
 // fetches them piece by piece while the staging threads move the pieces that have landed on to the
 // caller's pageable buffer (one thread alone moves about 10 GB/s, the link 55).
 static constexpr size_t kZeroCopyBytes = 512 * 1024, kResultHead = 64; // (the head holds the status word)
+static constexpr size_t kInputHead = 128;                              // parameters and ResizeItem of a resize call
 
 // Queues the pieces of `bytes` from dev to the pinned result buffer, and copies them on into `out` when
 // `ok` says so (asked when the first piece has landed).  Returns false on a CUDA error.
@@ -2105,16 +2119,19 @@ void resize(int64_t cresizer, int64_t source_p, int64_t sx, int64_t sy, int64_t 
         return;
     // Only the region travels to the GPU, behind its parameters.
     const int rows = (int)(end_row - start_row), cols = (int)(end_col - start_col);
-    const size_t pitch = (size_t)cols * 3, src_bytes = kResultHead + (size_t)rows * pitch, dst_bytes = (size_t)tx * ty * 3;
+    const size_t pitch = (size_t)cols * 3, src_bytes = kInputHead + (size_t)rows * pitch, dst_bytes = (size_t)tx * ty * 3;
     const bool zero_copy = dst_bytes <= kZeroCopyBytes;
     if (cudaSetDevice(ctx->device) != cudaSuccess) return;
     if (grow_dev(ctx, ctx->one_src, src_bytes + 64) || grow_host(ctx, ctx->one_in, ctx->one_in_cap, src_bytes) ||
         grow_host(ctx, ctx->one_host, ctx->one_host_cap, kResultHead + dst_bytes) || (!zero_copy && grow_dev(ctx, ctx->one_dst, dst_bytes)))
         return;
     const int32_t params[4] = {0, 0, rows, cols};
+    ResizeItems items(1, (int)tx, (int)ty, FFCVB_OUT_U8_NHWC);
+    const ResizeItem item = items.make(params, rows, cols, ResizeItems::kPacked);
     memcpy(ctx->one_in, params, sizeof(params));
+    memcpy(ctx->one_in + 64, &item, sizeof(item));
     const uint8_t *src = (const uint8_t *)(intptr_t)source_p + ((size_t)start_row * sy + start_col) * 3;
-    uint8_t *in = ctx->one_in + kResultHead;
+    uint8_t *in = ctx->one_in + kInputHead;
     auto copy_rows = [&](int lo, int hi, auto copy) {
         if (cols == sy)
             copy(in + lo * pitch, src + lo * pitch, (hi - lo) * pitch);
@@ -2134,16 +2151,16 @@ void resize(int64_t cresizer, int64_t source_p, int64_t sx, int64_t sy, int64_t 
     for (int k = 0; k < (together ? 1 : parts); k++) {
         const int lo = k * part, hi = together || lo + part > rows ? rows : lo + part;
         if (!together) copy_rows(lo, hi, memcpy);
-        const size_t from = k == 0 ? 0 : kResultHead + lo * pitch, to = kResultHead + hi * pitch;
+        const size_t from = k == 0 ? 0 : kInputHead + lo * pitch, to = kInputHead + hi * pitch;
         if (cudaMemcpyAsync((uint8_t *)ctx->one_src.p + from, ctx->one_in + from, to - from, cudaMemcpyHostToDevice, st) != cudaSuccess) return;
     }
     ResizeSource rs{};
-    rs.uniform = (const uint8_t *)ctx->one_src.p + kResultHead;
+    rs.uniform = (const uint8_t *)ctx->one_src.p + kInputHead;
     rs.uniform_h = rows;
     rs.uniform_w = cols;
     uint8_t *out = zero_copy ? ctx->one_host + kResultHead : (uint8_t *)ctx->one_dst.p;
-    launch_resize_augment(rs, 1, (const int32_t *)ctx->one_src.p, 4, OpList{}, 1, (int)tx, (int)ty, FFCVB_OUT_U8_NHWC,
-                          resize_bands(params, 1, 4, 1, (int)tx, (int)ty, FFCVB_OUT_U8_NHWC), nullptr, out, nullptr, SmallCopies{}, false, st);
+    launch_resize_augment(rs, 1, (const int32_t *)ctx->one_src.p, 4, (const ResizeItem *)((const uint8_t *)ctx->one_src.p + 64), OpList{}, 1, (int)tx, (int)ty,
+                          FFCVB_OUT_U8_NHWC, items.bands(), nullptr, out, nullptr, SmallCopies{}, false, st);
     if (cudaGetLastError() != cudaSuccess) return;
     if (zero_copy) {
         if (cudaStreamSynchronize(st) == cudaSuccess) memcpy((void *)(intptr_t)dest_p, out, dst_bytes);

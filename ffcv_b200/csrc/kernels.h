@@ -5,6 +5,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <vector>
+
 #include "types.h"
 
 namespace ffcvb {
@@ -201,14 +203,45 @@ FFCVB_HD inline uint64_t small_copy_words(uint64_t bytes, const void *src, const
     return bytes / word + (bytes % word != 0);
 }
 
-// CTAs per image of the kernel below: as many as the image with the most bands has, at most enough of them for
-// about eight waves of the GPU (148 SMs x 4 resident CTAs; fewer waves measured slower, more cost the set-up its
-// amortisation).  `params` is in host memory.  Worth a look at every box: a CTA without a band costs as much set-up as
+// What the resize kernel's CTAs have to know about an image, worked out on the host: four double-precision divisions,
+// and integer ones, that took one thread of every CTA 11 000 cycles while the others waited (a quarter of the
+// kernel: 1024 images to 160x160 pixels 212 us, 168 this way).
+struct alignas(16) ResizeItem {
+    double inv_x, inv_y, sc_x, sc_y; // as in Scaling
+    int32_t regime, isx, isy;
+    int32_t window;      // output rows per band with a window of source pixels (0: without one)
+    int32_t units;       // conversion units of a window row, and ceil(2^32 / units)
+    uint32_t inv_units;
+    int32_t lead;        // place of the crop's first pixel in its unit
+    int32_t groups;      // runs of rows that a band is dealt out in
+};
+// Makes them, and the CTAs per image of the kernel below: as many as the image with the most bands has, at most enough of
+// them for about eight waves of the GPU (148 SMs x 4 resident CTAs; fewer waves measured slower, more cost the set-up
+// its amortisation).  Worth a look at every box: a CTA without a band costs as much set-up as
 // one with (512 images of 32x32 pixels to 24x24: 21 us, 36 with a CTA for every four rows; 256 of 192x192 to 96x96: 39 and 60).
-int resize_bands(const int32_t *params, int n, int n_params, int resize, int out_h, int out_w, int out_kind);
+class ResizeItems {
+  public:
+    ResizeItems(int n, int out_h, int out_w, int out_kind);
+    // The image's crop box, inside the image (else: an empty item).  Packed pixels are read as such; fuse: from
+    // planes (kFuseQuad: 4:2:0, kFusePlain: of one resolution) if a window of them pays, as item.window then says.
+    enum Fuse { kPacked, kFuseQuad, kFusePlain };
+    ResizeItem make(const int32_t *box, int img_h, int img_w, Fuse fuse);
+    int bands() const { // (none made: without a window)
+        const int bands = bands_ ? bands_ : (out_h_ + shape_.band - 1) / shape_.band;
+        return bands < most_ ? bands : most_;
+    }
 
-// Fused crop + INTER_AREA resize + flip/translate/cutout + lookup-table normalise.
-void launch_resize_augment(const ResizeSource &src, int n, const int32_t *params, int n_params,
+  private:
+    int groups(int band);
+    int out_h_, out_w_, bands_ = 0, most_;
+    size_t tile_row_;
+    ResizeShape shape_;
+    std::vector<uint8_t> groups_; // by rows of a band, 0: not worked out
+};
+
+// Fused crop + INTER_AREA resize + flip/translate/cutout + lookup-table normalise.  items (device): one per image
+// (may be nullptr without `resize`).
+void launch_resize_augment(const ResizeSource &src, int n, const int32_t *params, int n_params, const ResizeItem *items,
                            const OpList &ops, int resize, int out_h, int out_w, int out_kind, int bands,
                            const void *lut, void *out, const int32_t *status, const SmallCopies &small, bool early, cudaStream_t stream);
 

@@ -86,17 +86,21 @@ __device__ __forceinline__ int sat_round(float v) { return min(255, max(0, __flo
 
 // Byte k of a pixel -> float without the conversion pipe: 2^23 + v is representable; the 2^23 is taken off
 // again inside the multiplication, fma(2^23 + v, w, -2^23 * w)
+constexpr uint32_t kBias = 0x4B000000u; // the bits of 2^23
 template <int k>
 __device__ __forceinline__ float biased(uint32_t px) {
-    return __uint_as_float(pick(px, 0x4B000000u, 0x7440u | k));
+    return __uint_as_float(pick(px, kBias, 0x7440u | k));
 }
-// sat_round of a value that is not negative
-__device__ __forceinline__ int round_byte(float v) { return (int)(__float_as_uint(__fadd_rn(fminf(v, 255.f), 8388608.f)) & 0xff); }
 
-// A pixel of a row: of the window's words, or of packed bytes.
+// A pixel of a row: of the window's words, or of packed bytes, of which the first `width` pixels may be read.
+struct PackedRow {
+    const uint8_t *bytes;
+    int width;
+};
 __device__ __forceinline__ uint32_t pixel(const uint32_t *row, int x) { return row[x]; }
-__device__ __forceinline__ uint32_t pixel(const uint8_t *row, int x) {
-    return (uint32_t)row[3 * x] | (uint32_t)row[3 * x + 1] << 8 | (uint32_t)row[3 * x + 2] << 16;
+__device__ __forceinline__ uint32_t pixel(const PackedRow &row, int x) {
+    const uint8_t *p = row.bytes + 3 * min(x, row.width - 1);
+    return (uint32_t)p[0] | (uint32_t)p[1] << 8 | (uint32_t)p[2] << 16;
 }
 
 // Taps of an output column or row, computed once per CTA (double-precision position arithmetic as
@@ -143,91 +147,93 @@ __device__ __forceinline__ Two add_rn(Two a, Two b) {
     asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
     return r;
 }
+__device__ __forceinline__ Two add_rd(Two a, Two b) {
+    Two r;
+    asm("add.rm.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+    return r;
+}
 // (as a sum with zero: a product that is added next may be contracted into one rounding, which must not happen)
 __device__ __forceinline__ Two mul_rn(Two a, Two b) { return fma_rn(a, b, Two(0.f, 0.f)); }
 
-// A column's horizontal sums: first tap, the whole cells between, last tap, rounded after every operation.
-// fma(2^23 + v, w, -2^23 * w) is the correctly rounded v * w, exactly what the multiplication of the
-// converted value gives (2^23 * w is exact).  Red and green share their instructions.
-struct AreaColumn {
-    int first, last;
-    float w_first, w_mid, w_last;
-    __device__ __forceinline__ explicit AreaColumn(uint4 t) {
-        first = (int)(t.x & 0xffff);
-        last = first + (int)(t.x >> 16) - 1;
-        w_first = __uint_as_float(t.y);
-        w_mid = __uint_as_float(t.z);
-        w_last = __uint_as_float(t.w);
+// Two neighbouring columns' horizontal sums: first tap, the whole cells between, last tap, rounded after every
+// operation.  fma(2^23 + v, w, -2^23 * w) is the correctly rounded v * w, exactly what the multiplication of the
+// converted value gives (2^23 * w is exact).  The columns share their instructions, one channel at a time.  A cell of
+// `scale` pixels has scale - 0.002 <= n < scale + 1.998 taps (area_taps), so the columns have equally many or one has
+// one more; the other's pixel there may be the one behind the crop's last, and its weight is zero, which changes no sum.
+struct AreaPair {
+    int first[2], mids, taps; // tap `mids` + 1 is the first that is the last one of either column
+    Two w_first, w_mid, w_tail[2];
+    __device__ __forceinline__ AreaPair(uint4 a, uint4 b) {
+        const int na = (int)(a.x >> 16), nb = (int)(b.x >> 16);
+        first[0] = (int)(a.x & 0xffff);
+        first[1] = (int)(b.x & 0xffff);
+        taps = max(na, nb);
+        mids = max(min(na, nb) - 2, 0);
+        w_first = Two(__uint_as_float(a.y), __uint_as_float(b.y));
+        w_mid = Two(__uint_as_float(a.z), __uint_as_float(b.z));
+#pragma unroll
+        for (int k = 0; k < 2; k++) w_tail[k] = Two(weight(a, mids + 1 + k), weight(b, mids + 1 + k));
     }
-    static __device__ __forceinline__ void tap(uint32_t px, float w, Two &rg, float &b) {
-        const float c = -8388608.0f * w;
-        rg = fma_rn(Two(biased<0>(px), biased<1>(px)), Two(w, w), Two(c, c));
-        b = __fmaf_rn(biased<2>(px), w, c);
+    // of tap k >= 1
+    static __device__ __forceinline__ float weight(uint4 t, int k) {
+        const int last = (int)(t.x >> 16) - 1;
+        return k < last ? __uint_as_float(t.z) : (k == last ? __uint_as_float(t.w) : 0.f);
+    }
+    static __device__ __forceinline__ void tap(uint32_t p, uint32_t q, Two w, Two (&v)[3]) {
+        const Two c = fma_rn(w, Two(-8388608.0f, -8388608.0f), Two(0.f, 0.f));
+        v[0] = fma_rn(Two(biased<0>(p), biased<0>(q)), w, c);
+        v[1] = fma_rn(Two(biased<1>(p), biased<1>(q)), w, c);
+        v[2] = fma_rn(Two(biased<2>(p), biased<2>(q)), w, c);
     }
     template <class Row>
-    __device__ __forceinline__ void across(Row row, Two &rg, float &b) const {
-        Two rg2;
-        float b2;
-        tap(pixel(row, first), w_first, rg, b);
-        for (int k = first + 1; k < last; k++) {
-            tap(pixel(row, k), w_mid, rg2, b2);
-            rg = add_rn(rg, rg2);
-            b = __fadd_rn(b, b2);
-        }
-        tap(pixel(row, last), w_last, rg2, b2);
-        rg = add_rn(rg, rg2);
-        b = __fadd_rn(b, b2);
+    __device__ __forceinline__ void more(Row row, int k, Two w, Two (&sum)[3]) const {
+        Two v[3];
+        tap(pixel(row, first[0] + k), pixel(row, first[1] + k), w, v);
+#pragma unroll
+        for (int c = 0; c < 3; c++) sum[c] = add_rn(sum[c], v[c]);
+    }
+    template <class Row>
+    __device__ __forceinline__ void across(Row row, Two (&sum)[3]) const {
+        tap(pixel(row, first[0]), pixel(row, first[1]), w_first, sum);
+        for (int k = 1; k <= mids; k++) more(row, k, w_mid, sum);
+        if (taps > mids + 1) more(row, mids + 1, w_tail[0], sum);
+        if (taps > mids + 2) more(row, mids + 2, w_tail[1], sum);
     }
 };
 
 // OpenCV's fixed-point bilinear, in floating point whose roundings do what the shifts do: with S the two taps'
 // weighted sum (an exact integer below 2^20), 2^27 + S rounded down is 2^27 + 16 * (S >> 4), and
 // fma(b, that, 2^43 - 2^27 * b) rounded down is 2^43 + 2^20 * (b * (S >> 4) >> 16), the product of the integers
-// in the low bits of its mantissa.  The two taps of a channel share their instruction, and so do the two rows.
-struct LinearColumn {
-    int x0, x1;
-    Two w, c;
-    __device__ __forceinline__ explicit LinearColumn(uint4 t) {
-        x0 = (int)t.x;
-        x1 = (int)t.y;
-        w = Two(__uint_as_float(t.z), __uint_as_float(t.w));
-        c = mul_rn(w, Two(-8388608.0f, -8388608.0f));
+// in the low bits of its mantissa.  Two neighbouring columns share their instructions.
+struct LinearPair {
+    int x0[2], x1[2];
+    Two w0, w1, c0, c1;
+    __device__ __forceinline__ LinearPair(uint4 a, uint4 b) {
+        x0[0] = (int)a.x, x1[0] = (int)a.y;
+        x0[1] = (int)b.x, x1[1] = (int)b.y;
+        w0 = Two(__uint_as_float(a.z), __uint_as_float(b.z));
+        w1 = Two(__uint_as_float(a.w), __uint_as_float(b.w));
+        c0 = mul_rn(w0, Two(-8388608.0f, -8388608.0f));
+        c1 = mul_rn(w1, Two(-8388608.0f, -8388608.0f));
     }
     template <class Row>
-    __device__ __forceinline__ void across(Row row, float (&h)[3]) const {
-        const uint32_t p = pixel(row, x0), q = pixel(row, x1);
-        auto one = [&](float a, float b) {
-            const Two s = fma_rn(Two(a, b), w, c);
-            return __fadd_rd(__fadd_rn(s.lo(), s.hi()), 134217728.f);
+    __device__ __forceinline__ void across(Row row, Two (&h)[3]) const {
+        const uint32_t p0 = pixel(row, x0[0]), q0 = pixel(row, x0[1]), p1 = pixel(row, x1[0]), q1 = pixel(row, x1[1]);
+        auto one = [&](float a0, float b0, float a1, float b1) {
+            const Two s = add_rn(fma_rn(Two(a0, b0), w0, c0), fma_rn(Two(a1, b1), w1, c1));
+            return add_rd(s, Two(134217728.f, 134217728.f));
         };
-        h[0] = one(biased<0>(p), biased<0>(q));
-        h[1] = one(biased<1>(p), biased<1>(q));
-        h[2] = one(biased<2>(p), biased<2>(q));
+        h[0] = one(biased<0>(p0), biased<0>(q0), biased<0>(p1), biased<0>(q1));
+        h[1] = one(biased<1>(p0), biased<1>(q0), biased<1>(p1), biased<1>(q1));
+        h[2] = one(biased<2>(p0), biased<2>(q0), biased<2>(p1), biased<2>(q1));
     }
 };
-// (The weights' sum is at most 2049, so 255 is not exceeded.)
-__device__ __forceinline__ int blend_rows(float upper, float lower, Two b, Two k) {
-    const Two u = fma_rd(b, Two(upper, lower), k);
-    return (int)((__float_as_uint(u.lo()) + __float_as_uint(u.hi()) + 2u - 2u * (170u << 23)) >> 2);
-}
-
-// The column paths deal a band's rows to this many runs per column, so that the (column, run) items fill the
-// CTA's 256 threads evenly, with runs of at least 3 rows.
-__device__ __forceinline__ int row_groups(int out_w, int band) {
-    int groups = 1, best = 0;
-    for (int g = 1; g <= 4 && (band + g - 1) / g >= 3; g++) {
-        const int items = g * out_w, use = items * 256 / ((items + 255) / 256 * 256);
-        if (use > best) {
-            best = use;
-            groups = g;
-        }
-    }
-    return groups;
-}
+// A column's value out of the two rows' products.  (The weights' sum is at most 2049, so 255 is not exceeded.)
+__device__ __forceinline__ uint32_t blended(float upper, float lower) { return (__float_as_uint(upper) + __float_as_uint(lower) + 2u - 2u * (170u << 23)) >> 2; }
 
 // a / n for a, n < 2^16, inv_n = ceil(2^32 / n)
 __device__ __forceinline__ int divided(uint32_t a, uint32_t inv_n, int n) { return n == 1 ? (int)a : (int)__umulhi(a, inv_n); }
-__device__ __forceinline__ uint32_t inverse(int n) { return (uint32_t)((0x100000000ull + n - 1) / n); }
+__host__ __device__ __forceinline__ uint32_t inverse(int n) { return (uint32_t)((0x100000000ull + n - 1) / n); }
 
 // One of SmallCopies, by a CTA of 256 threads: every thread has its words (at most kSmallCopyWords / 256) under way
 // at once.
@@ -259,6 +265,7 @@ __device__ __noinline__ void copy_small(const uint8_t *src, uint8_t *dst, uint32
 template <typename OutT>
 __global__ void __launch_bounds__(256, 4)
 resize_augment_kernel(const __grid_constant__ ResizeSource src, const int32_t *__restrict__ params, int n_params,
+                      const ResizeItem *__restrict__ items,
                       const __grid_constant__ OpList ops,
                       int resize, int out_h, int out_w, const __grid_constant__ ResizeShape shape, int planar,
                       const OutT *__restrict__ lut, OutT *__restrict__ out,
@@ -277,8 +284,8 @@ resize_augment_kernel(const __grid_constant__ ResizeSource src, const int32_t *_
     const int i = blockIdx.y;
     if (blockIdx.x == 0 && i == 0)
         for (int k = 0; k < small.n; k++) copy_small(small.src[k], small.dst[k], (uint32_t)small.bytes[k]);
-    if (!kU8)
-        for (int k = threadIdx.x; k < 768; k += blockDim.x) s_lut[(k % 3) * 256 + k / 3] = lut[k]; // per channel
+    ResizeItem item{};
+    if (resize) item = items[i];
 
     // ---- where the sample's pixels are
     const uint8_t *base;
@@ -287,7 +294,7 @@ resize_augment_kernel(const __grid_constant__ ResizeSource src, const int32_t *_
     uint32_t skew_base = 0, skew_pitch = 0;
     bool skew = false;
     bool ok = true;
-    int fuse = 0; // output rows per band of a sample whose planes are converted here
+    bool fuse = false; // a sample whose planes are converted here
     if (src.descs) {
         const ImageDesc &d = src.descs[i];
         img_h = d.dec_height; // the decoded size: smaller than the stored one after a scaled decode
@@ -306,7 +313,7 @@ resize_augment_kernel(const __grid_constant__ ResizeSource src, const int32_t *_
             }
         } else {
             base = src.rgb + d.rgb_off;
-            fuse = d.fuse_rows;
+            fuse = d.fuse_rows != 0;
             ok = d.host_status == 0 && (status == nullptr || status[i] == 0);
         }
     } else {
@@ -340,45 +347,25 @@ resize_augment_kernel(const __grid_constant__ ResizeSource src, const int32_t *_
         }
     }
 
-    // The scale factors (four double-precision divisions) are worked out by one thread, and so are the
-    // conversion units of a window row and the number of output rows whose source rows fit the window.
-    __shared__ Scaling s_scaling;
-    __shared__ int s_window, s_units, s_lead, s_groups;
-    __shared__ uint32_t s_inv_units;
-    if (threadIdx.x == 0 && ok) {
-        s_scaling = scaling_of(ch, cw, out_h, out_w);
-        const bool fits = s_scaling.regime == kArea || s_scaling.regime == kLinear;
-        s_window = fuse ? fuse : (fits ? window_band(cw, s_scaling.sc_y, tile_row, shape) : 0);
-        const bool quad = fuse && src.descs[i].scale_shift == 0 && src.descs[i].hs == 2;
-        s_lead = fuse ? (quad ? cj & 7 : cj & 3) : 0; // a unit begins at a multiple of its width
-        s_units = quad ? (s_lead + cw + 7) / 8 : (s_lead + cw + 3) / 4;
-        s_inv_units = inverse(s_units);
-        s_groups = row_groups(out_w, s_window ? s_window : shape.band);
-    }
-    __syncthreads();
-    int regime = kCopy, isx = 1, isy = 1;
-    const int window = ok ? s_window : 0, band_rows = window ? window : shape.band;
-    const int lead = ok ? s_lead : 0, wpitch = window_pitch(cw), groups = ok ? s_groups : 1;
+    const int window = ok ? item.window : 0, band_rows = window ? window : shape.band;
+    const int lead = item.lead, wpitch = window_pitch(cw), groups = item.groups;
     uint32_t *s_win = reinterpret_cast<uint32_t *>(reinterpret_cast<unsigned char *>(s_out) + (((size_t)band_rows * tile_row + 15) & ~(size_t)15));
     const int nbands = (out_h + band_rows - 1) / band_rows;
     if ((int)blockIdx.x >= nbands) return;
-    if (ok) {
-        const Scaling &sc = s_scaling;
-        regime = sc.regime;
-        isx = sc.isx;
-        isy = sc.isy;
-        if (regime == kArea || regime == kLinear) {
-            // x taps of every column, y taps of the rows of the crop that this CTA needs
-            const int my_bands = (nbands - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x;
-            for (int e = threadIdx.x; e < out_w + my_bands * band_rows; e += blockDim.x) {
-                const bool column = e < out_w;
-                const int k = e - out_w, b = column ? 0 : k / band_rows;
-                const int at = column ? e : ((int)blockIdx.x + b * (int)gridDim.x) * band_rows + (k - b * band_rows) + dy;
-                if (at < 0 || at >= (column ? out_w : out_h)) continue;
-                const int ssize = column ? cw : ch;
-                const double inv = column ? sc.inv_x : sc.inv_y, scale = column ? sc.sc_x : sc.sc_y;
-                (column ? tx : ty)[at] = regime == kArea ? make_area_taps(at, ssize, scale) : make_linear_taps(at, ssize, inv, scale, column);
-            }
+    if (!kU8)
+        for (int k = threadIdx.x; k < 768; k += blockDim.x) s_lut[(k % 3) * 256 + k / 3] = lut[k]; // per channel
+    const int regime = ok ? item.regime : kCopy, isx = item.isx, isy = item.isy;
+    if (regime == kArea || regime == kLinear) {
+        // x taps of every column, y taps of the rows of the crop that this CTA needs
+        const int my_bands = (nbands - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x;
+        for (int e = threadIdx.x; e < out_w + my_bands * band_rows; e += blockDim.x) {
+            const bool column = e < out_w;
+            const int k = e - out_w, b = column ? 0 : k / band_rows;
+            const int at = column ? e : ((int)blockIdx.x + b * (int)gridDim.x) * band_rows + (k - b * band_rows) + dy;
+            if (at < 0 || at >= (column ? out_w : out_h)) continue;
+            const int ssize = column ? cw : ch;
+            const double inv = column ? item.inv_x : item.inv_y, scale = column ? item.sc_x : item.sc_y;
+            (column ? tx : ty)[at] = regime == kArea ? make_area_taps(at, ssize, scale) : make_linear_taps(at, ssize, inv, scale, column);
         }
     }
     __syncthreads();
@@ -391,7 +378,7 @@ resize_augment_kernel(const __grid_constant__ ResizeSource src, const int32_t *_
         return p;
     };
     int npix = 0;
-    const uint32_t inv_w = inverse(out_w);
+    const uint32_t inv_w = inverse(out_w), inv_pairs = inverse((out_w + 1) >> 1);
     // Traces an output pixel back through the augmentations: either a fill colour, or the position
     // (y, x) of a pixel of the resized crop.
     auto trace = [&](int oy, int ox, int &y, int &x, int *val) -> bool {
@@ -432,6 +419,59 @@ resize_augment_kernel(const __grid_constant__ ResizeSource src, const int32_t *_
             o[2 * chan_step] = s_lut[512 + v2];
         }
     };
+    // The same for two neighbouring pixels of a row, the first of an even column; `bias` is on top of every value.
+    // They leave as whole words (bytes: half-words) where rows have an even number of pixels.
+    const bool even = (out_w & 1) == 0;
+    const uint32_t lut_address = (uint32_t)__cvta_generic_to_shared(s_lut);
+    auto emit_pair = [&](OutT *o, const uint32_t (&v)[2][3], uint32_t bias, bool both) {
+        uint32_t e[2][3];
+#pragma unroll
+        for (int p = 0; p < 2; p++)
+#pragma unroll
+            for (int c = 0; c < 3; c++) {
+                // (the bias goes out of the address, which has 32 bits like the product)
+                const uint32_t at = lut_address - bias * (uint32_t)sizeof(OutT) + v[p][c] * (uint32_t)sizeof(OutT);
+                if constexpr (kU8)
+                    e[p][c] = v[p][c];
+                else if constexpr (sizeof(OutT) == 2)
+                    asm("{\n\t.reg .u16 h;\n\tld.shared.u16 h, [%1];\n\tcvt.u32.u16 %0, h;\n\t}" : "=r"(e[p][c]) : "r"(at + 256 * 2 * c));
+                else
+                    asm("ld.shared.u32 %0, [%1];" : "=r"(e[p][c]) : "r"(at + 256 * 4 * c));
+            }
+        if (!even) {
+#pragma unroll
+            for (int p = 0; p < 2; p++) {
+                if (p == 1 && !both) break;
+#pragma unroll
+                for (int c = 0; c < 3; c++) o[p * pix_step + c * chan_step] = (OutT)e[p][c];
+            }
+        } else if constexpr (kU8) {
+            uint16_t *w = reinterpret_cast<uint16_t *>(o);
+            w[0] = (uint16_t)pick(e[0][0], e[0][1], 0x0040);
+            w[1] = (uint16_t)pick(e[0][2], e[1][0], 0x0040);
+            w[2] = (uint16_t)pick(e[1][1], e[1][2], 0x0040);
+        } else if constexpr (sizeof(OutT) == 2) {
+            if (planar) {
+#pragma unroll
+                for (int c = 0; c < 3; c++) *reinterpret_cast<uint32_t *>(o + c * chan_step) = pick(e[0][c], e[1][c], 0x5410);
+            } else {
+                uint32_t *w = reinterpret_cast<uint32_t *>(o);
+                w[0] = pick(e[0][0], e[0][1], 0x5410);
+                w[1] = pick(e[0][2], e[1][0], 0x5410);
+                w[2] = pick(e[1][1], e[1][2], 0x5410);
+            }
+        } else {
+            if (planar) {
+#pragma unroll
+                for (int c = 0; c < 3; c++) *reinterpret_cast<uint2 *>(o + c * chan_step) = make_uint2(e[0][c], e[1][c]);
+            } else {
+                uint2 *w = reinterpret_cast<uint2 *>(o);
+                w[0] = make_uint2(e[0][0], e[0][1]);
+                w[1] = make_uint2(e[0][2], e[1][0]);
+                w[2] = make_uint2(e[1][1], e[1][2]);
+            }
+        }
+    };
     // A CTA produces every gridDim.x-th band of its image: what was set up above (descriptor, tap
     // tables, lookup table) serves all of them.
     for (int band = blockIdx.x; band < nbands; band += gridDim.x) {
@@ -448,8 +488,8 @@ resize_augment_kernel(const __grid_constant__ ResizeSource src, const int32_t *_
         const uint4 top = ty[y_lo], bottom = ty[y_hi - 1];
         win_lo = (int)(regime == kArea ? top.x & 0xffff : top.x);
         const int hi = (int)(regime == kArea ? (bottom.x & 0xffff) + (bottom.x >> 16) - 1 : bottom.y);
-        const int units = s_units;
-        const uint32_t inv_units = s_inv_units;
+        const int units = item.units;
+        const uint32_t inv_units = item.inv_units;
         if (fuse) {
             const ImageDesc &d = src.descs[i];
             const uint8_t *py = src.planes + d.plane_off[0], *pb = src.planes + d.plane_off[1], *pr = src.planes + d.plane_off[2];
@@ -502,45 +542,58 @@ resize_augment_kernel(const __grid_constant__ ResizeSource src, const int32_t *_
     auto window_row = [&](int y) -> const uint32_t * { return s_win + (y - win_lo) * wpitch + lead; };
     if (regime == kArea || regime == kLinear) { // (and ok)
         // OpenCV first sums every source row horizontally with the x weights, then combines those row sums with
-        // the y weights; likewise for its two-tap interpolation.  A thread therefore owns one output column for
-        // a run of consecutive output rows: the taps and weights of its column live in registers for the whole
-        // run, and what a source row contributes is computed once for neighbouring output rows that share it.
+        // the y weights; likewise for its two-tap interpolation.  A thread therefore owns two neighbouring output
+        // columns for a run of consecutive output rows: the taps and weights of its columns live in registers for the
+        // whole run, what a source row contributes is computed once for neighbouring output rows that share
+        // it, and the columns share instructions and the loop around them.
         // Same operations in the same order as the per-pixel form, so the same bits.
-        const int run = (rows + groups - 1) / groups;
+        const int run = (rows + groups - 1) / groups, pairs = (out_w + 1) >> 1;
         // row_of: a row of the crop, in the window or in global memory
         auto columns = [&](auto row_of) {
-            for (int t = threadIdx.x; t < groups * out_w; t += blockDim.x) {
-                const int g = divided(t, inv_w, out_w), ox = t - g * out_w;
+            for (int t = threadIdx.x; t < groups * pairs; t += blockDim.x) {
+                const int g = divided(t, inv_pairs, pairs), ox = 2 * (t - g * pairs);
+                const bool both = ox + 1 < out_w;
                 const int begin = max(y_lo, band0 + g * run + dy), end = min(y_hi, band0 + (g + 1) * run + dy);
-                const uint4 taps = tx[min(max(step_x * ox + dx, 0), out_w - 1)];
+                auto taps_of = [&](int x) { return tx[min(max(step_x * x + dx, 0), out_w - 1)]; };
+                const uint4 taps = taps_of(ox), beside = taps_of(both ? ox + 1 : ox);
                 OutT *o = s_out + ((begin - dy - band0) * out_w + ox) * pix_step;
                 const int row_step = out_w * pix_step;
                 if (regime == kArea) {
-                    const AreaColumn column(taps);
+                    const AreaPair pair(taps, beside);
                     int pj = -1; // source row whose horizontal sums are held
-                    Two rg(0.f, 0.f);
-                    float b = 0.f;
+                    Two row[3];
+                    row[0] = row[1] = row[2] = Two(0.f, 0.f);
                     for (int y = begin; y < end; y++, o += row_step) {
                         const uint4 c = ty[y];
                         const int yf = (int)(c.x & 0xffff), ye = yf + (int)(c.x >> 16) - 1;
                         // only the first source row can be the one the previous output row ended with
-                        if (yf != pj) column.across(row_of(yf), rg, b);
+                        if (yf != pj) pair.across(row_of(yf), row);
                         float beta = __uint_as_float(c.y);
-                        Two sum_rg = mul_rn(Two(beta, beta), rg);
-                        float sum_b = __fmul_rn(beta, b);
+                        Two sum[3];
+#pragma unroll
+                        for (int k = 0; k < 3; k++) sum[k] = mul_rn(Two(beta, beta), row[k]);
                         for (int j = yf + 1; j <= ye; j++) {
-                            column.across(row_of(j), rg, b);
+                            pair.across(row_of(j), row);
                             beta = __uint_as_float(j == ye ? c.w : c.z);
-                            sum_rg = add_rn(sum_rg, mul_rn(Two(beta, beta), rg));
-                            sum_b = __fadd_rn(sum_b, __fmul_rn(beta, b));
+#pragma unroll
+                            for (int k = 0; k < 3; k++) sum[k] = add_rn(sum[k], mul_rn(Two(beta, beta), row[k]));
                         }
                         pj = ye;
-                        emit(o, round_byte(sum_rg.lo()), round_byte(sum_rg.hi()), round_byte(sum_b));
+                        // 2^23 + the rounded value.  (The weights of an axis sum up to 1 but for rounding, so 255 is not exceeded.)
+                        uint32_t v[2][3];
+#pragma unroll
+                        for (int k = 0; k < 3; k++) {
+                            const Two r = add_rn(sum[k], Two(8388608.f, 8388608.f));
+                            v[0][k] = __float_as_uint(r.lo());
+                            v[1][k] = __float_as_uint(r.hi());
+                        }
+                        emit_pair(o, v, kBias, both);
                     }
                 } else {
-                    const LinearColumn column(taps);
+                    const LinearPair pair(taps, beside);
                     int ra = -1, rb = -1; // source rows whose interpolated values ha / hb hold
-                    float ha[3] = {0.f, 0.f, 0.f}, hb[3] = {0.f, 0.f, 0.f};
+                    Two ha[3], hb[3];
+                    ha[0] = ha[1] = ha[2] = hb[0] = hb[1] = hb[2] = Two(0.f, 0.f);
                     for (int y = begin; y < end; y++, o += row_step) {
                         const uint4 c = ty[y];
                         const int r0 = (int)c.x, r1 = (int)c.y;
@@ -550,17 +603,25 @@ resize_augment_kernel(const __grid_constant__ ResizeSource src, const int32_t *_
 #pragma unroll
                                 for (int k = 0; k < 3; k++) ha[k] = hb[k];
                             } else {
-                                column.across(row_of(r0), ha);
+                                pair.across(row_of(r0), ha);
                             }
                             ra = r0;
                         }
                         if (r1 != rb) {
-                            column.across(row_of(r1), hb);
+                            pair.across(row_of(r1), hb);
                             rb = r1;
                         }
-                        const Two b(__uint_as_float(c.z), __uint_as_float(c.w));
-                        const Two k = fma_rn(b, Two(-134217728.f, -134217728.f), Two(8796093022208.f, 8796093022208.f));
-                        emit(o, blend_rows(ha[0], hb[0], b, k), blend_rows(ha[1], hb[1], b, k), blend_rows(ha[2], hb[2], b, k));
+                        const Two b0(__uint_as_float(c.z), __uint_as_float(c.z)), b1(__uint_as_float(c.w), __uint_as_float(c.w));
+                        const Two k0 = fma_rn(b0, Two(-134217728.f, -134217728.f), Two(8796093022208.f, 8796093022208.f));
+                        const Two k1 = fma_rn(b1, Two(-134217728.f, -134217728.f), Two(8796093022208.f, 8796093022208.f));
+                        uint32_t v[2][3];
+#pragma unroll
+                        for (int k = 0; k < 3; k++) {
+                            const Two upper = fma_rd(b0, ha[k], k0), lower = fma_rd(b1, hb[k], k1);
+                            v[0][k] = blended(upper.lo(), lower.lo());
+                            v[1][k] = blended(upper.hi(), lower.hi());
+                        }
+                        emit_pair(o, v, 0, both);
                     }
                 }
             }
@@ -568,7 +629,7 @@ resize_augment_kernel(const __grid_constant__ ResizeSource src, const int32_t *_
         if (window)
             columns(window_row);
         else
-            columns(row_ptr);
+            columns([&](int y) { return PackedRow{row_ptr(y), cw}; });
         if (!flips_only) { // what is filled, over it
             __syncthreads();
             for (int pix = threadIdx.x; pix < npix; pix += blockDim.x) {
@@ -633,12 +694,14 @@ resize_augment_kernel(const __grid_constant__ ResizeSource src, const int32_t *_
     }
 }
 
+static size_t value_size(int out_kind) { return out_kind == kOutU8 ? 1 : (out_kind == kOutF16Nhwc || out_kind == kOutF16Nchw ? 2 : 4); }
+
 ResizeShape resize_shape(int n, int out_h, int out_w, int out_kind) {
-    const size_t elem = out_kind == kOutU8 ? 1 : (out_kind == kOutF16Nhwc || out_kind == kOutF16Nchw ? 2 : 4);
+    const size_t elem = value_size(out_kind);
     ResizeShape s{};
     const size_t fixed = 768 * elem + sizeof(uint4) * ((size_t)out_w + out_h), row = (size_t)out_w * 3 * elem;
-    // without a window: about 2048 pixels per band
-    int band = (2048 + out_w - 1) / out_w;
+    // without a window: about 3072 pixels per band
+    int band = (3072 + out_w - 1) / out_w;
     if (band > out_h) band = out_h;
     while (band > 1 && fixed + band * row > 200 * 1024) band /= 2;
     s.band = band;
@@ -651,52 +714,76 @@ ResizeShape resize_shape(int n, int out_h, int out_w, int out_kind) {
     const size_t quarter = (227 * 1024) / 4 - 1024;
     s.room = quarter > fixed ? (quarter - fixed) & ~(size_t)15 : 0;
     const size_t tile = (band * row + 15) & ~(size_t)15;
-    s.smem = fixed + (s.room > tile ? s.room : tile);
+    s.smem = fixed + (s.room > tile ? s.room : tile) + 16; // (a zero weight's pixel lies up to one behind the window)
     return s;
 }
 
-int resize_bands(const int32_t *params, int n, int n_params, int resize, int out_h, int out_w, int out_kind) {
-    const ResizeShape shape = resize_shape(n, out_h, out_w, out_kind);
-    const size_t elem = out_kind == kOutU8 ? 1 : (out_kind == kOutF16Nhwc || out_kind == kOutF16Nchw ? 2 : 4), tile_row = (size_t)out_w * 3 * elem;
-    const int plain = (out_h + shape.band - 1) / shape.band, most = (8 * 148 * 4 + n - 1) / n;
-    int bands = 1;
-    for (int i = 0; i < n && bands < most; i++) {
-        const int32_t *box = params + (size_t)i * n_params;
-        int mine = plain;
-        if (resize && box[2] > 0 && box[3] > 0) {
-            const Scaling sc = scaling_of(box[2], box[3], out_h, out_w);
-            const int window = sc.regime == kArea || sc.regime == kLinear ? window_band(box[3], sc.sc_y, tile_row, shape) : 0;
-            if (window) mine = (out_h + window - 1) / window;
+ResizeItems::ResizeItems(int n, int out_h, int out_w, int out_kind)
+    : out_h_(out_h), out_w_(out_w), most_((8 * 148 * 4 + n - 1) / n), tile_row_((size_t)out_w * 3 * value_size(out_kind)),
+      shape_(resize_shape(n, out_h, out_w, out_kind)), groups_((shape_.band > shape_.max_band ? shape_.band : shape_.max_band) + 1, 0) {}
+
+// The column paths deal a band's rows to this many runs per pair of columns, so that the (pair, run) items fill the
+// CTA's 256 threads evenly, with runs of at least 2 rows.
+int ResizeItems::groups(int band) {
+    if (groups_[band]) return groups_[band];
+    const int pairs = (out_w_ + 1) / 2;
+    int groups = 1, best = 0;
+    for (int g = 1; g <= 8 && (band + g - 1) / g >= 2; g++) {
+        const int items = g * pairs, use = items * 256 / ((items + 255) / 256 * 256);
+        if (use > best) {
+            best = use;
+            groups = g;
         }
-        if (mine > bands) bands = mine;
-        if (!resize) break; // (all alike)
     }
-    return bands < most ? bands : most;
+    groups_[band] = (uint8_t)groups;
+    return groups;
+}
+
+ResizeItem ResizeItems::make(const int32_t *box, int img_h, int img_w, Fuse fuse) {
+    ResizeItem item{};
+    const int ch = box[2], cw = box[3];
+    if (!(ch > 0 && cw > 0 && box[0] >= 0 && box[1] >= 0 && box[0] + ch <= img_h && box[1] + cw <= img_w)) return item;
+    const Scaling sc = scaling_of(ch, cw, out_h_, out_w_);
+    item.inv_x = sc.inv_x;
+    item.inv_y = sc.inv_y;
+    item.sc_x = sc.sc_x;
+    item.sc_y = sc.sc_y;
+    item.regime = sc.regime;
+    item.isx = sc.isx;
+    item.isy = sc.isy;
+    if (sc.regime == kArea || sc.regime == kLinear) item.window = window_band(cw, sc.sc_y, tile_row_, shape_);
+    if (item.window && fuse != kPacked) item.lead = fuse == kFuseQuad ? box[1] & 7 : box[1] & 3; // a unit begins at a multiple of its width
+    item.units = item.window && fuse == kFuseQuad ? (item.lead + cw + 7) / 8 : (item.lead + cw + 3) / 4;
+    item.inv_units = inverse(item.units);
+    const int band = item.window ? item.window : shape_.band, bands = (out_h_ + band - 1) / band;
+    item.groups = groups(band);
+    if (bands > bands_) bands_ = bands;
+    return item;
 }
 
 template <typename OutT>
-static void launch_typed(const ResizeSource &src, int n, const int32_t *params, int n_params, const OpList &ops,
+static void launch_typed(const ResizeSource &src, int n, const int32_t *params, int n_params, const ResizeItem *items, const OpList &ops,
                          int resize, int out_h, int out_w, int planar, const ResizeShape &shape, int bands, const void *lut, void *out,
                          const int32_t *status, const SmallCopies &small, bool early, cudaStream_t stream) {
     auto kern = resize_augment_kernel<OutT>;
     if (shape.smem > 48 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shape.smem);
     dim3 grid(bands, n);
-    launch(early, grid, 256, shape.smem, stream, kern, src, params, n_params, ops, resize, out_h, out_w, shape, planar, (const OutT *)lut, (OutT *)out,
+    launch(early, grid, 256, shape.smem, stream, kern, src, params, n_params, items, ops, resize, out_h, out_w, shape, planar, (const OutT *)lut, (OutT *)out,
            status, small);
 }
 
-void launch_resize_augment(const ResizeSource &src, int n, const int32_t *params, int n_params,
+void launch_resize_augment(const ResizeSource &src, int n, const int32_t *params, int n_params, const ResizeItem *items,
                            const OpList &ops, int resize, int out_h, int out_w, int out_kind, int bands,
                            const void *lut, void *out, const int32_t *status, const SmallCopies &small, bool early, cudaStream_t stream) {
     if (n <= 0) return;
     const int planar = out_kind == kOutF16Nchw || out_kind == kOutF32Nchw;
     const ResizeShape shape = resize_shape(n, out_h, out_w, out_kind);
     if (out_kind == kOutU8)
-        launch_typed<uint8_t>(src, n, params, n_params, ops, resize, out_h, out_w, 0, shape, bands, nullptr, out, status, small, early, stream);
+        launch_typed<uint8_t>(src, n, params, n_params, items, ops, resize, out_h, out_w, 0, shape, bands, nullptr, out, status, small, early, stream);
     else if (out_kind == kOutF16Nhwc || out_kind == kOutF16Nchw)
-        launch_typed<uint16_t>(src, n, params, n_params, ops, resize, out_h, out_w, planar, shape, bands, lut, out, status, small, early, stream);
+        launch_typed<uint16_t>(src, n, params, n_params, items, ops, resize, out_h, out_w, planar, shape, bands, lut, out, status, small, early, stream);
     else
-        launch_typed<uint32_t>(src, n, params, n_params, ops, resize, out_h, out_w, planar, shape, bands, lut, out, status, small, early, stream);
+        launch_typed<uint32_t>(src, n, params, n_params, items, ops, resize, out_h, out_w, planar, shape, bands, lut, out, status, small, early, stream);
 }
 
 } // namespace ffcvb
