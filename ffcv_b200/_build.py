@@ -7,7 +7,7 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, 'csrc')
 LIB = os.path.join(HERE, 'libffcv_b200.so')
 SOURCES = ['context.cu', 'entropy.cu', 'idct.cu', 'gather.cu', 'resize.cu', 'pixel_ops.cu', 'static_decode.cu', 'jpeg_header.cpp']
-HEADERS = ['types.h', 'kernels.h', 'jpeg_header.h', 'huffman.h', 'color.h', 'decode_index.h', 'table_store.h', os.path.join('..', '..', 'include', 'ffcv_b200.h')]
+HEADERS = ['types.h', 'kernels.h', 'jpeg_header.h', 'huffman.h', 'color.h', 'two.h', 'decode_index.h', 'table_store.h', os.path.join('..', '..', 'include', 'ffcv_b200.h')]
 
 
 def _nvcc():
