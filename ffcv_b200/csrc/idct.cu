@@ -10,20 +10,16 @@
 #include "color.h"
 #include "huffman.h"
 #include "kernels.h"
+#include "two.h"
 
 namespace ffcvb {
 
-// Position in zig-zag order of the coefficient of row r, column c: zigzag_of(r * 8 + c).  Used with
-// compile-time indices only (fully unrolled loops), so the permutation costs nothing.
-__device__ __forceinline__ constexpr int zigzag_of(int n) {
-    constexpr int t[64] = {0, 1, 5, 6, 14, 15, 27, 28, 2, 4, 7, 13, 16, 26, 29, 42, 3, 8, 12, 17, 25, 30, 41, 43, 9, 11, 18, 24, 31, 40, 44, 53, 10, 19, 23, 32, 39, 45, 52, 54, 20, 22, 33, 38, 46, 51, 55, 60, 21, 34, 37, 47, 50, 56, 59, 61, 35, 36, 48, 49, 57, 58, 62, 63};
-    return t[n];
-}
+// Natural position (row-major) of the coefficient at a place in zig-zag order.
+__constant__ uint8_t c_natural[64] = {0, 1, 8, 16, 9, 2, 3, 10, 17, 24, 32, 25, 18, 11, 4, 5, 12, 19, 26, 33, 40, 48, 41, 34, 27, 20, 13, 6, 7, 14, 21, 28, 35, 42, 49, 56, 57, 50, 43, 36, 29, 22, 15, 23, 30, 37, 44, 51, 58, 59, 52, 45, 38, 31, 39, 46, 53, 60, 61, 54, 47, 55, 62, 63};
 
-// Coefficient of natural position n (row-major) out of a block in zig-zag order, two per register.
+// Coefficient of natural position n out of a block's words, two per register.
 __device__ __forceinline__ int coef_at(const int (&w)[32], int n) {
-    const int z = zigzag_of(n);
-    return (z & 1) ? (w[z >> 1] >> 16) : (int)(short)(w[z >> 1] & 0xffff);
+    return (n & 1) ? (w[n >> 1] >> 16) : (int)(short)(w[n >> 1] & 0xffff);
 }
 
 __device__ __forceinline__ int w16(int v) { return (int)(short)v; }
@@ -53,6 +49,84 @@ __device__ __forceinline__ void idct8(int &v0, int &v1, int &v2, int &v3, int &v
     v5 = w16(t2 - t5);
     v4 = w16(t3 + t4);
     v3 = w16(t3 - t4);
+}
+
+// The full-size transform of a block in floating point, two columns or two rows per instruction.  It gives the
+// wrapping 16-bit result because sums and differences may wrap anywhere as long as what is multiplied, and what is
+// shifted in the end, lies in 16 bits: integers below 2^24 are exact in a float, and a product rounded down onto
+// 1.5 * 2^23 is the shifted one.  `peak` gathers the largest of those values.  Up to kPeak the result is exact (the sum
+// of z10 and z12 is then below 2^15 as well); beyond it, which the streams of encoders do not reach, the integer
+// transform below has to be taken.  Kernel on 1024 photographs to 160x160, 256x256, 64 of 4:4:4 to 384x384: 110, 145 and
+// 596 us in integers, 98, 133 and 549 this way, 94, 124 and 500 with six CTAs per SM instead of five.
+constexpr float kPeak = 16383.f;
+constexpr float kOnes = 12582912.f; // 1.5 * 2^23: what is added to it leaves as an integer
+__device__ __forceinline__ Two both(float v) { return Two(v, v); }
+__device__ __forceinline__ void peak_of(Two v, float &peak) { peak = fmaxf(fmaxf(peak, fabsf(v.lo())), fabsf(v.hi())); }
+__device__ __forceinline__ void idct8(Two &v0, Two &v1, Two &v2, Two &v3, Two &v4, Two &v5, Two &v6, Two &v7, float &peak) {
+    const Two ones = both(kOnes);
+    const Two t10 = add_rn(v0, v4), t11 = sub_rn(v0, v4), t13 = add_rn(v2, v6), d26 = sub_rn(v2, v6);
+    const Two t12 = sub_rn(sub_rn(fma_rd(d26, both(362.f / 256), ones), ones), t13);
+    const Two t0 = add_rn(t10, t13), t3 = sub_rn(t10, t13), t1 = add_rn(t11, t12), t2 = sub_rn(t11, t12);
+    const Two z13 = add_rn(v5, v3), z10 = sub_rn(v5, v3), z11 = add_rn(v1, v7), z12 = sub_rn(v1, v7);
+    const Two t7 = add_rn(z11, z13), d = sub_rn(z11, z13);
+    const Two z5 = fma_rd(add_rn(z10, z12), both(473.f / 256), ones); // (on top of `ones`, as the two it is added to)
+    const Two t10b = sub_rn(fma_rd(z12, both(277.f / 256), ones), z5);
+    const Two t12b = add_rn(fma_rd(z10, both(-669.f / 256), both(-kOnes)), z5);
+    const Two t6 = sub_rn(t12b, t7);
+    const Two t5 = sub_rn(sub_rn(fma_rd(d, both(362.f / 256), ones), ones), t6);
+    const Two t4 = add_rn(t10b, t5);
+    peak_of(d26, peak);
+    peak_of(z10, peak);
+    peak_of(z12, peak);
+    peak_of(d, peak);
+    v0 = add_rn(t0, t7);
+    v7 = sub_rn(t0, t7);
+    v1 = add_rn(t1, t6);
+    v6 = sub_rn(t1, t6);
+    v2 = add_rn(t2, t5);
+    v5 = sub_rn(t2, t5);
+    v4 = add_rn(t3, t4);
+    v3 = sub_rn(t3, t4);
+}
+
+// Smaller of two pairs of 16-bit values and `most`, not below 0.
+__device__ __forceinline__ uint32_t clamp_halves(uint32_t v, uint32_t most) { return __vimin_s16x2_relu(v, most); }
+
+// Block out of 32 words of coefficients (one per kBlockTile words at `coef`), each value on top of 2^15.
+// Returns whether the result, which is stored in any case, is exact.
+__device__ __forceinline__ bool block_in_floats(const uint32_t *coef, uint8_t *__restrict__ dst, int pitch) {
+    float peak = 0.f;
+    Two a[8][4]; // [row][pair of columns]
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+#pragma unroll
+        for (int r = 0; r < 8; r++) {
+            const uint32_t w = coef[(4 * r + k) * kBlockTile]; // (each value becomes 2^23 + 2^15 + itself)
+            a[r][k] = sub_rn(Two(__uint_as_float(pick(w, 0x4B000000u, 0x7410u)), __uint_as_float(pick(w, 0x4B000000u, 0x7432u))), both(8388608.f + 32768.f));
+        }
+        idct8(a[0][k], a[1][k], a[2][k], a[3][k], a[4][k], a[5][k], a[6][k], a[7][k], peak);
+    }
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+        Two b[8]; // a column of two rows
+#pragma unroll
+        for (int c = 0; c < 8; c++) b[c] = Two(a[2 * q][c >> 1].half(c & 1), a[2 * q + 1][c >> 1].half(c & 1));
+        idct8(b[0], b[1], b[2], b[3], b[4], b[5], b[6], b[7], peak);
+#pragma unroll
+        for (int c = 0; c < 8; c++) {
+            peak_of(b[c], peak);
+            b[c] = fma_rd(b[c], both(1.f / 32), both(kOnes + 128.f)); // 16 bits of the sample, beyond its range as yet
+        }
+#pragma unroll
+        for (int r = 0; r < 2; r++) {
+            uint32_t w[4];
+#pragma unroll
+            for (int c = 0; c < 4; c++)
+                w[c] = clamp_halves(pick(__float_as_uint(b[2 * c].half(r)), __float_as_uint(b[2 * c + 1].half(r)), 0x5410u), 0x00ff00ffu);
+            *reinterpret_cast<uint2 *>(dst + (size_t)(2 * q + r) * pitch) = make_uint2(pick(w[0], w[1], 0x6420u), pick(w[2], w[3], 0x6420u));
+        }
+    }
+    return peak <= kPeak;
 }
 
 // Reduced-size inverse transforms for decoding at 1/2, 1/4, 1/8 scale (the scale_num / scale_denom
@@ -115,19 +189,22 @@ __device__ __forceinline__ void reduced_block(const int (&cw)[32], const uint16_
     }
 }
 
+constexpr uint32_t kCoefZero = 0x80008000u; // coefficients wait for the transform on top of 2^15
+
 // One thread per block: decodes the block's AC symbols from the place the entropy decoder recorded,
 // dequantising each value as it is stored (the block lies in shared memory, two coefficients per word,
 // one bank per lane), then transforms it in registers.  Only blocks inside the crop's reach run.
 // A warp takes blocks of one component that are neighbours in the plane: their symbol counts are
 // alike, their bits are near one another and their rows leave as one run.
-// Bound by instruction issue: about 30 per symbol and 1600 for the transform, per lane.
-__global__ void __launch_bounds__(kBlockTile)
+// Bound by instruction issue (61 % of the cycles) and the arithmetic pipe (53 %): about 30 instructions per symbol, of
+// which a warp's longest block has some 28.
+__global__ void __launch_bounds__(kBlockTile, 6)
 blocks_kernel(const ImageDesc *__restrict__ descs, const uint2 *__restrict__ tiles, const HuffTable *__restrict__ huff,
               const MultTable *__restrict__ mult, EntropyScratch scratch, uint8_t *__restrict__ planes) {
     constexpr int kLook = 1 << kHuffBits;
     __shared__ __align__(16) uint32_t s_coef[32][kBlockTile];
     __shared__ __align__(16) uint16_t s_look[2][kLook]; // AC tables of luma and of the first chroma component
-    __shared__ int16_t s_mult[3][64];
+    __shared__ uint32_t s_mult[3][64]; // by zig-zag position: multiplier, and where the value goes << 16
     next_may_begin();
     const uint2 tile = tiles[blockIdx.x];
     const ImageDesc &d = descs[tile.x];
@@ -142,8 +219,10 @@ blocks_kernel(const ImageDesc *__restrict__ descs, const uint2 *__restrict__ til
             const uint4 *src = reinterpret_cast<const uint4 *>(huff[d.tab_id[d.ac_tab[t]]].look);
             for (int k = tid; k < kLook / 8; k += kBlockTile) reinterpret_cast<uint4 *>(s_look[t])[k] = src[k];
         }
-        for (int k = tid; k < 64 * d.ncomp; k += kBlockTile)
-            s_mult[k >> 6][k & 63] = scaled && (k < 64 || d.bs_chroma != 8) ? (int16_t)1 : mult[d.q_tab[k >> 6]].m[k & 63];
+        for (int k = tid; k < 64 * d.ncomp; k += kBlockTile) {
+            const uint32_t m = scaled && (k < 64 || d.bs_chroma != 8) ? 1 : (uint16_t)mult[d.q_tab[k >> 6]].m[k & 63], n = c_natural[k & 63];
+            s_mult[k >> 6][k & 63] = m | ((n >> 1) * kBlockTile * 4 + (n & 1) * 2) << 16;
+        }
     }
     await_previous();
     __syncthreads();
@@ -175,10 +254,11 @@ blocks_kernel(const ImageDesc *__restrict__ descs, const uint2 *__restrict__ til
     const uint32_t p0 = scratch.pos[d.block_base + blk];
     int dc = scratch.dc[d.block_base + blk];
     if (d.seg_count > 1 && p0 != kNoBlock) dc += scratch.seg_dc[((size_t)d.seg_first + p0 / (d.seg_stride * 8)) * 4 + comp];
-    const int16_t *m = s_mult[comp];
+    const uint32_t *m = s_mult[comp];
+    unsigned char *coef = reinterpret_cast<unsigned char *>(&s_coef[0][tid]);
 #pragma unroll
-    for (int k = 0; k < 32; k++) s_coef[k][tid] = 0;
-    reinterpret_cast<int16_t *>(&s_coef[0][tid])[0] = (int16_t)((int16_t)dc * m[0]);
+    for (int k = 0; k < 32; k++) s_coef[k][tid] = kCoefZero;
+    *reinterpret_cast<uint16_t *>(coef) = (uint16_t)((uint32_t)dc * m[0] + 0x8000);
     if (p0 != kNoBlock) {
         const int t = comp == 0 ? 0 : 1, table = d.ac_tab[comp];
         const bool in_shared = comp < 2 || table == d.ac_tab[1]; // (a table of its own for Cr: read where it is)
@@ -202,13 +282,18 @@ blocks_kernel(const ImageDesc *__restrict__ descs, const uint2 *__restrict__ til
             edge += next ? 32 : 0;
             z += (int)(e >> 9);
             const int at = z - 1; // where the value goes
-            if (size != 0 && at < 64) reinterpret_cast<int16_t *>(&s_coef[at >> 1][tid])[at & 1] = (int16_t)(huff_value(w, n, size) * m[at]);
+            if (size != 0 && at < 64) { // (the low 16 bits of the product are the value's)
+                const uint32_t to = m[at];
+                *reinterpret_cast<uint16_t *>(coef + (to >> 16)) = (uint16_t)((uint32_t)huff_value(w, n, size) * to + 0x8000);
+            }
         } while (z < 64);
     }
+    uint8_t *dst = planes + d.plane_off[comp] + (size_t)(by * bs) * plane_w + bx * bs;
+    if (bs == 8 && block_in_floats(&s_coef[0][tid], dst, plane_w)) return;
+    asm volatile("" ::: "memory"); // (the words are read again: held since the first time they would cost 40 registers)
     int cw[32];
 #pragma unroll
-    for (int k = 0; k < 32; k++) cw[k] = (int)s_coef[k][tid];
-    uint8_t *dst = planes + d.plane_off[comp] + (size_t)(by * bs) * plane_w + bx * bs;
+    for (int k = 0; k < 32; k++) cw[k] = (int)(s_coef[k][tid] ^ kCoefZero);
     if (bs != 8) { // scaled decode: this block becomes bs x bs samples
         const MultTable &mt = mult[d.q_tab[comp]];
         if (bs == 4) {

@@ -215,3 +215,30 @@ def test_streams_that_each_bring_tables_of_their_own():
         assert imdecode(buf, out, 8, 8) == 0, k
         if k % 6000 == 0 or k > 60190:
             assert np.array_equal(out, O.jpeg_decode(buf)), k
+
+
+@pytest.mark.parametrize('sampling', [420, 444])
+@pytest.mark.parametrize('step', [1, 8, 40, 120, 255])
+def test_transform_where_16_bit_lanes_wrap(step, sampling):
+    """A stream whose quantiser steps were raised after encoding: coefficients beyond what images hold, up to
+    where the transform's 16-bit lanes overflow, which is where its two forms change over (block by block)."""
+    from ffcv_b200.libffcv import imdecode
+    rng = np.random.default_rng(step)
+    img = rng.integers(0, 256, (72, 104, 3)).astype(np.uint8) if step % 2 else _content(rng, 72, 104, 'smooth')
+    flags = [cv2.IMWRITE_JPEG_QUALITY, 95]
+    if sampling == 444:
+        flags += [cv2.IMWRITE_JPEG_SAMPLING_FACTOR, cv2.IMWRITE_JPEG_SAMPLING_FACTOR_444]
+    buf = cv2.imencode('.jpg', img, flags)[1].reshape(-1).copy()
+    at = 0
+    while True:
+        found = [k for k in range(at, buf.size - 1) if buf[k] == 0xFF and buf[k + 1] == 0xDB]
+        if not found:
+            break
+        first, size = found[0] + 4, 256 * int(buf[found[0] + 2]) + int(buf[found[0] + 3]) - 2
+        for k in range(size):
+            if k % 65:  # (the others are the tables' numbers)
+                buf[first + k] = min(255, int(buf[first + k]) * step)
+        at = first + size
+    out = np.zeros(img.shape, np.uint8)
+    assert imdecode(buf, out, *img.shape[:2]) == 0
+    assert np.array_equal(out, O.jpeg_decode(buf))
