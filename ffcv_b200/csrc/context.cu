@@ -269,13 +269,13 @@ struct DevBuf {
 struct Slot {
     uint8_t *host = nullptr; // pinned
     size_t host_cap = 0;
-    DevBuf blob, clean, segs, slot_tables, index, planes, rgb; // segs: per-segment scratch; index: per-block positions and DC values
+    DevBuf blob, clean, segs, records, slot_tables, index, planes, rgb; // segs: per-segment scratch; index: per-block positions and DC values
     BatchHeader hdr{};
     ffcvb_plan plan{};
     int n = 0, n_jpeg = 0;
     EntropyWork work{}; // (the lists' addresses are filled in when the batch runs)
     int n_quad = 0, n_444 = 0, n_other = 0, max_w = 0, max_h = 0;
-    uint64_t jpeg_list_off = 0, segs_off = 0, multi_off = 0, slot_images_off = 0, restart_off = 0, block_tiles_off = 0, quad_tiles_off = 0;
+    uint64_t jpeg_list_off = 0, segs_off = 0, parts_off = 0, slot_images_off = 0, restart_off = 0, block_tiles_off = 0, quad_tiles_off = 0;
     uint64_t status_off = 0; // status word and counter of finished segments of every sample
     uint64_t items_off = 0;  // ResizeItem of every sample
     int n_block_tiles = 0, n_quad_tiles = 0, bands = 1;
@@ -311,7 +311,8 @@ struct Slot {
     std::vector<JpegHeader> parsed;
     std::vector<std::array<uint64_t, 9>> hashes; // of a parsed header's (DC, AC, quantisation) tables x 3 components
     std::vector<ResizeItem> items;
-    std::vector<int32_t> jpeg_list, multi, slot_images, restart;
+    std::vector<int32_t> jpeg_list, slot_images, restart;
+    std::vector<uint4> parts, wholes;
     std::vector<uint2> slot_segs;  // those of slot_images, behind
     std::vector<uint2> seg_list;   // (sample, segment) of the entropy decoder's CTAs
     std::vector<uint2> blk_tiles;  // (sample, k) of the block decoder's CTAs
@@ -540,7 +541,7 @@ void ffcvb_destroy(ffcvb_ctx *ctx) {
     cudaDeviceSynchronize();
     for (auto &s : ctx->slots) {
         if (s.host) cudaFreeHost(s.host);
-        for (DevBuf *b : {&s.blob, &s.clean, &s.segs, &s.slot_tables, &s.index, &s.planes, &s.rgb})
+        for (DevBuf *b : {&s.blob, &s.clean, &s.segs, &s.records, &s.slot_tables, &s.index, &s.planes, &s.rgb})
             if (b->p) cudaFree(b->p);
         for (auto &e : s.ev)
             if (e) cudaEventDestroy(e);
@@ -716,6 +717,7 @@ int stage_impl(ffcvb_ctx *ctx, int slot, const Source &source, const uint64_t *p
             tail += sizeof(uint2) * (size_t)quad_tiles_x(widths[i]) * quad_tiles_y(heights[i]);
             tail += sizeof(uint2) * ((size_t)((heights[i] + 15) / 8) * ((widths[i] + 15) / 8) * 3 / kBlockTile + 4);
             tail += sizeof(uint2) * (size_t)(sizes[i] / (64 * kSegSubs / 8) + 2);
+            tail += sizeof(uint4) * (size_t)(sizes[i] / (64 * kSegSubs / 8 * kRepairPart) + 3);
         }
         int grc;
         if ((grc = grow_host(ctx, s.host, s.host_cap, fd_payload_end + tail))) return grc;
@@ -944,10 +946,11 @@ int stage_impl(ffcvb_ctx *ctx, int slot, const Source &source, const uint64_t *p
     };
     std::vector<BatchSet> batch_sets;
     int last_set = -1;
-    std::vector<int32_t> &jpeg_list = s.jpeg_list, &multi = s.multi, &slot_images = s.slot_images, &restart = s.restart;
+    std::vector<int32_t> &jpeg_list = s.jpeg_list, &slot_images = s.slot_images, &restart = s.restart;
     std::vector<uint2> &segs = s.seg_list, &blk_tiles = s.blk_tiles, &quad_tiles = s.quad_tiles;
     jpeg_list.clear();
-    multi.clear();
+    s.parts.clear();
+    s.wholes.clear();
     slot_images.clear();
     s.slot_segs.clear();
     restart.clear();
@@ -973,6 +976,7 @@ int stage_impl(ffcvb_ctx *ctx, int slot, const Source &source, const uint64_t *p
         few = bits <= kSlotModeBits && !ctx->tune_subseq_bits;
     }
     if (ctx->tune_subseq_bits) target_bits = (uint32_t)ctx->tune_subseq_bits;
+    work.local_repair = !ctx->index_pool.p && local_repair(target_bits, n);
     if (ctx->index_pool.p) {
         for (size_t k = 0; k < ctx->slots.size(); k++) { // whose writers have ended
             if (!ctx->index.unsettled((int)k)) continue;
@@ -1061,10 +1065,11 @@ int stage_impl(ffcvb_ctx *ctx, int slot, const Source &source, const uint64_t *p
             restart.push_back(i);
         } else {
             const bool slots = few && d.bpm > 3; // (a guess among three slots falls in step within 1.4 kbit)
-            const ScanLayout l = slots ? layout_scan_slots(d.scan_len) : layout_scan(d.scan_len, target_bits);
+            const ScanLayout l = slots ? layout_scan_slots(d.scan_len) : layout_scan(d.scan_len, target_bits, d.bpm, work.local_repair);
             d.subseq_bits = l.subseq_bits;
             d.seg_raw = l.seg_raw;
             d.seg_warm = l.seg_warm;
+            d.seg_run_up = l.seg_run_up;
             d.seg_stride = l.seg_stride;
             d.seg_count = l.seg_count;
             d.seg_first = seg_total;
@@ -1074,8 +1079,11 @@ int stage_impl(ffcvb_ctx *ctx, int slot, const Source &source, const uint64_t *p
                 d.slots = 1 + (uint32_t)s.slot_segs.size();
                 slot_images.push_back(i);
                 if ((int)l.seg_count > work.max_slot_segs) work.max_slot_segs = (int)l.seg_count;
-            } else if (l.seg_count > 1) {
-                multi.push_back(i);
+            } else {
+                const uint32_t parts = repair_parts(l.seg_count, work.local_repair);
+                for (uint32_t k = 0; k < parts; k++) s.parts.push_back(repair_part((uint32_t)i, l.seg_count, parts, k));
+                if (parts > 1) s.wholes.push_back(make_uint4((uint32_t)i, 0, l.seg_count, 0));
+                if (l.subseq_bits > work.max_subseq_bits) work.max_subseq_bits = l.subseq_bits;
             }
             for (uint32_t k = 0; k < l.seg_count; k++) (slots ? s.slot_segs : segs).push_back(make_uint2((uint32_t)i, k));
             const uint32_t raw = l.seg_stride - 64 - 16; // (at least run-up, own bytes and overlap)
@@ -1148,8 +1156,8 @@ int stage_impl(ffcvb_ctx *ctx, int slot, const Source &source, const uint64_t *p
     auto place_lists = [&] {
         s.jpeg_list_off = off;
         off = align_up(off + sizeof(int32_t) * jpeg_list.size(), 16);
-        s.multi_off = off;
-        off = align_up(off + sizeof(int32_t) * multi.size(), 16);
+        s.parts_off = off;
+        off = align_up(off + sizeof(uint4) * (s.parts.size() + s.wholes.size()), 16);
         s.slot_images_off = off;
         off = align_up(off + sizeof(int32_t) * slot_images.size(), 16);
         s.restart_off = off;
@@ -1245,7 +1253,8 @@ int stage_impl(ffcvb_ctx *ctx, int slot, const Source &source, const uint64_t *p
     if (rc) return rc;
     if ((rc = grow_dev(ctx, s.blob, off + 64))) return rc;
     if ((rc = grow_dev(ctx, s.clean, clean_bytes + 512))) return rc;
-    if ((rc = grow_dev(ctx, s.segs, seg_total * (sizeof(SegMeta) + 4 * kSegSubs + 16) + 64))) return rc;
+    if ((rc = grow_dev(ctx, s.segs, seg_total * kSegScratch + 64))) return rc;
+    if ((rc = grow_dev(ctx, s.records, segs.empty() ? 0 : (size_t)seg_total * kSegSubs * kRecords * sizeof(uint16_t)))) return rc;
     if (!s.slot_segs.empty() && (rc = grow_dev(ctx, s.slot_tables, s.slot_segs.size() * sizeof(SlotTables)))) return rc;
     if ((rc = grow_dev(ctx, s.index, (size_t)total_blocks * 6 + 64))) return rc;
     if ((rc = grow_dev(ctx, s.planes, plane_bytes + 64))) return rc;
@@ -1297,7 +1306,8 @@ int stage_impl(ffcvb_ctx *ctx, int slot, const Source &source, const uint64_t *p
         }
     }
     if (!jpeg_list.empty()) memcpy(s.host + s.jpeg_list_off, jpeg_list.data(), 4 * jpeg_list.size());
-    if (!multi.empty()) memcpy(s.host + s.multi_off, multi.data(), 4 * multi.size());
+    if (!s.parts.empty()) memcpy(s.host + s.parts_off, s.parts.data(), sizeof(uint4) * s.parts.size());
+    if (!s.wholes.empty()) memcpy(s.host + s.parts_off + sizeof(uint4) * s.parts.size(), s.wholes.data(), sizeof(uint4) * s.wholes.size());
     if (!slot_images.empty()) memcpy(s.host + s.slot_images_off, slot_images.data(), 4 * slot_images.size());
     if (!restart.empty()) memcpy(s.host + s.restart_off, restart.data(), 4 * restart.size());
     if (!segs.empty()) memcpy(s.host + s.segs_off, segs.data(), sizeof(uint2) * segs.size());
@@ -1308,7 +1318,8 @@ int stage_impl(ffcvb_ctx *ctx, int slot, const Source &source, const uint64_t *p
     s.n_block_tiles = (int)blk_tiles.size();
     work.n_guess = (int)segs.size();
     work.n_slots = (int)s.slot_segs.size();
-    work.n_multi = (int)multi.size();
+    work.n_parts = (int)s.parts.size();
+    work.n_whole = (int)s.wholes.size();
     work.n_slot_images = (int)slot_images.size();
     work.n_restart = (int)restart.size();
 
@@ -1534,14 +1545,16 @@ static int run_batch(ffcvb_ctx *ctx, Slot &s, cudaStream_t st, void *out_dev, bo
         scratch.clean = (uint8_t *)s.clean.p;
         EntropyWork work = s.work;
         work.segs = reinterpret_cast<const uint2 *>(blob + s.segs_off);
-        work.multi = reinterpret_cast<const int32_t *>(blob + s.multi_off);
+        work.parts = reinterpret_cast<const uint4 *>(blob + s.parts_off);
         work.slot_images = reinterpret_cast<const int32_t *>(blob + s.slot_images_off);
         work.restart = reinterpret_cast<const int32_t *>(blob + s.restart_off);
         const size_t n_segs = (size_t)work.n_guess + work.n_slots;
         scratch.seg_dc = (int32_t *)s.segs.p;
         scratch.sub_info = (uint32_t *)(scratch.seg_dc + 4 * n_segs);
-        scratch.meta = (SegMeta *)(scratch.sub_info + kSegSubs * n_segs);
+        scratch.sub_exit = (uint16_t *)(scratch.sub_info + kSegSubs * n_segs);
+        scratch.meta = (SegMeta *)(scratch.sub_exit + kSegSubs * n_segs); // (everything before it is a multiple of 16 bytes)
         scratch.slots = (SlotTables *)s.slot_tables.p;
+        scratch.records = (uint16_t *)s.records.p;
         scratch.done = (uint32_t *)(blob + s.status_off) + s.n;
         scratch.pos = (uint32_t *)s.index.p;
         scratch.dc = (int16_t *)(scratch.pos + s.total_blocks);
@@ -1783,8 +1796,8 @@ int ffcvb_batch_launches(const ffcvb_ctx *ctx, int slot) {
     if (!ctx || slot < 0 || slot >= (int)ctx->slots.size() || !ctx->slots[slot].staged) return -1;
     const Slot &s = ctx->slots[slot];
     int k = 1 + (s.direct && s.range_len == 0 ? 1 : 0); // fused resize/augment/normalise (+ payload gather)
-    k += (s.n_quad > 0) + (s.n_444 > 0) + (s.n_other > 0) + (s.n_block_tiles > 0) + (s.work.n_guess > 0) + (s.work.n_multi > 0) +
-         2 * (s.work.n_slots > 0) + (s.work.n_guess + s.work.n_slots > 0) + (s.work.n_restart > 0);
+    k += (s.n_quad > 0) + (s.n_444 > 0) + (s.n_other > 0) + (s.n_block_tiles > 0) + 2 * (s.work.n_guess > 0) + (s.work.n_whole > 0) +
+         2 * (s.work.n_slots > 0) + (s.work.n_guess > 0) + (s.work.n_slots > 0) + (s.work.n_restart > 0);
     return k;
 }
 

@@ -8,24 +8,25 @@
 // the inverse transform (idct.cu) decodes any block on its own, in parallel and only where the crop
 // needs it, and no coefficient ever travels through global memory.
 //
-//   scan_sync_kernel    one CTA per segment of a scan (about 128 subsequences): removes the byte
-//                       stuffing, decodes every subsequence from a guessed state and repairs the
-//                       guesses by re-decoding from the left neighbour's exit state until nothing
-//                       changes.  A decoder that starts mid-stream falls in step after 0.9 kbit on
-//                       average (4:2:0, quality 90; 99 % within 4 kbit), dominated by the block's
-//                       slot inside the MCU, so two passes and a few stragglers settle a segment.
-//                       Segments behind the first decode the last 8 kbit before them as a run-up.
-//   scan_stitch_kernel  scans of several segments: where a run-up was too short, walks
-//                       on from the exact state until it meets the recorded one.
+//   scan_guess_kernel   one thread per subsequence, up to 128 of them a segment, whose bytes lie in shared memory without
+//                       their stuffing: decodes a run-up before the subsequence from a guessed state, then the
+//                       subsequence itself, writing down where its blocks begin.  A decoder that starts
+//                       mid-stream falls in step after 0.9 kbit on average (4:2:0, quality 90), dominated by
+//                       the block's slot inside the MCU: after 1.9 kbit nine in ten have.
+//   scan_repair_kernel  decodes the others again, from the state the subsequence before them really ends in,
+//                       until every one begins where the one before it ends.
 //   scan_slots_kernel, scan_chain_kernel   instead of the two above while a batch's scans leave most of the
 //                       GPU idle: every subsequence from all block slots at once, see there.
-//   scan_index_kernel   every subsequence once more from its exact state: records the blocks; the
-//                       last CTA of an image integrates the DC differences.
+//   scan_index_kernel   positions and DC values of the blocks, out of what was written down (with
+//                       scan_slots_kernel: by decoding once more from the exact states); the last CTA of an
+//                       image integrates the DC differences.
 //
 // Integer work bound by instruction issue at large batches and by the chain look-up -> shift ->
 // look-up at small ones: about 25 instructions per symbol and lane, tables and stream in shared memory.
 #include "huffman.h"
 #include "kernels.h"
+
+#include <algorithm>
 
 namespace ffcvb {
 
@@ -35,12 +36,13 @@ constexpr int kThreads = kSegSubs;          // one thread per subsequence: a tea
 constexpr int kFastBytes = 2 * kHuffFast;   // a Huffman table in shared memory
 
 // The threads that work on one segment.  A CTA holds one team, or several that share the Huffman
-// tables in shared memory and meet at barriers of their own.
+// tables in shared memory and meet at barriers of their own.  Every team's first warp is another one of the
+// SM's quarters', because segments often need only the first two (130 us instead of 94 when they were the same ones').
 template <int TEAMS, int SIZE = kThreads>
 struct Team {
     static constexpr int size = SIZE;
     int index, tid;
-    __device__ __forceinline__ Team() : index(TEAMS == 1 ? 0 : threadIdx.x / SIZE), tid(TEAMS == 1 ? threadIdx.x : threadIdx.x % SIZE) {}
+    __device__ __forceinline__ Team() : index(TEAMS == 1 ? 0 : threadIdx.x / SIZE), tid(TEAMS == 1 ? threadIdx.x : (threadIdx.x + 32 * index) % SIZE) {}
     __device__ __forceinline__ void sync() const {
         if (TEAMS == 1)
             __syncthreads();
@@ -106,6 +108,7 @@ struct Tables {
     uint16_t fast[8];               // (the first vector of the tables)
 };
 constexpr size_t kTablesHead = offsetof(Tables, fast);
+static_assert(kSegSubs == 128, "SegMeta::doubt is read as four words");
 static_assert(kTablesHead % 16 == 0 && kFastBytes % 16 == 0 && offsetof(HuffTable, fast) % 16 == 0 && offsetof(HuffTable, pair) % 16 == 0,
               "tables are copied in vectors");
 __host__ __device__ constexpr size_t tables_bytes(int n_tables) { return kTablesHead + (size_t)n_tables * kFastBytes; }
@@ -143,17 +146,24 @@ struct Cursor {
 __device__ __forceinline__ uint32_t pack(const Cursor &s, uint32_t from) { return (s.p - from) | (uint32_t)s.c << 5 | (uint32_t)s.z << 8; }
 __device__ __forceinline__ Cursor unpack(uint32_t v, uint32_t from) { return Cursor{from + (v & 31), (int)((v >> 5) & 7), (int)((v >> 8) & 63)}; }
 
+// What a walk writes down: nothing, positions of blocks, or the records of a subsequence.
+enum { kNothing, kPositions, kRecord };
+
 // The walk below in plain code: for tables that are not fast_ok, and for the few walks on a stream in
 // global memory.  One symbol at a time, tables where they are.
-template <bool RECORD>
+template <int RECORD>
 __device__ __noinline__ uint32_t walk_plain(const uint32_t *words, Cursor &cur, uint32_t end, const ImageDesc &d,
-                                            const HuffTable *__restrict__ huff, uint32_t *pos, uint32_t blk, uint32_t limit) {
+                                            const HuffTable *__restrict__ huff, uint32_t *pos, uint32_t blk, uint32_t limit, uint16_t *rec) {
     const int luma = d.ncomp == 1 ? 1 : d.hs * d.vs;
-    uint32_t done = 0;
+    uint32_t done = 0, n = 0;
     while (cur.p < end) {
-        if (RECORD && cur.z == 0) {
+        if (RECORD == kPositions && cur.z == 0) {
             if (blk < limit) pos[blk] = cur.p;
             blk++;
+        }
+        if (RECORD == kRecord && cur.z == 0) {
+            if (n < kRecords - 1) rec[n] = (uint16_t)(cur.p + blk);
+            n++;
         }
         const uint32_t w = __funnelshift_l(words[(cur.p >> 5) + 1], words[cur.p >> 5], cur.p);
         const int comp = cur.c < luma ? 0 : cur.c - luma + 1;
@@ -172,71 +182,100 @@ __device__ __noinline__ uint32_t walk_plain(const uint32_t *words, Cursor &cur, 
 }
 
 // Decodes symbols from `cur` until its position reaches `end`; returns the number of blocks
-// completed.  `buf`: the segment's stream in shared memory (words most significant bit first).  With
-// RECORD every block that begins before `end` gets its position written to pos[blk], pos[blk + 1],
-// ... below pos[limit]; `blk` is the first of them.
+// completed.  `buf`: the segment's stream (words most significant bit first) in shared memory, or, with GLOBAL, in
+// global memory.  With kPositions every block that begins before `end` gets its position written to pos[blk], pos[blk + 1],
+// ... below pos[limit]; `blk` is the first of them.  With kRecord the low 16 bits of the positions, plus blk, go to
+// rec[0], rec[1], ... as far as rec[kRecords - 2]; what lies behind the last one may be overwritten.
 //
-// The 32 lanes of a warp walk unrelated places, so nothing in the loops branches: position (bits 0-17)
+// The 32 lanes of a warp walk unrelated places, so nothing in the loops branches: position (bits 0-23)
 // and zig-zag index (bits 24-30) share one word that an entry is simply added to; a 96-bit window over
 // the stream stays in registers (hi holds the word the position lies in, lo and nx the two behind it)
 // and is moved on by predicated instructions; so are the table switches and the slot at the end of a
 // block; codes too long for the first level are reached by the index's maximum.  As long as `end` is
 // more than kHuffBits away an entry may stand for two symbols (1.46 on average), so that the walk's
 // last position is the same whatever state it came from.
-constexpr uint32_t kPosMask = 0x3ffff;
-template <bool RECORD>
+constexpr uint32_t kPosMask = 0xffffff;
+constexpr int kLongest = 31; // bits of a symbol, at most
+template <int RECORD, bool GLOBAL = false>
 __device__ __forceinline__ uint32_t walk(const unsigned char *buf, Cursor &cur, uint32_t end, const Tables *s, const ImageDesc &d,
-                                         const HuffTable *__restrict__ huff, uint32_t *pos = nullptr, uint32_t blk = 0, uint32_t limit = 0) {
+                                         const HuffTable *__restrict__ huff, uint32_t *pos = nullptr, uint32_t blk = 0, uint32_t limit = 0,
+                                         uint16_t *rec = nullptr) {
     if (cur.p >= end) return 0;
-    if (!d.fast_tables) return walk_plain<RECORD>(reinterpret_cast<const uint32_t *>(buf), cur, end, d, huff, pos, blk, limit);
+    if (!d.fast_tables) return walk_plain<RECORD>(reinterpret_cast<const uint32_t *>(buf), cur, end, d, huff, pos, blk, limit, rec);
     const uint32_t pairs = s->pairs;
     uint32_t st = cur.p | (uint32_t)cur.z << 24, done = 0;
     const Slot here = s->slot[cur.c];
     uint32_t ac = here.tables >> 16, tab = cur.z ? ac : here.tables & 0xffff;
     uint32_t ahead = load_shared(here.next), after = load_shared(here.next + 4); // the slot that follows
-    uint32_t wa = shared_address(buf) + (cur.p >> 5) * 4;
-    uint32_t hi = load_shared(wa), lo = load_shared(wa + 4), nx = load_shared(wa + 8);
-    wa += 12;
-    if (RECORD && cur.z == 0) {
+    uint32_t wa = 0, hi, lo, nx;
+    const uint32_t *ga = reinterpret_cast<const uint32_t *>(buf) + (cur.p >> 5);
+    if (GLOBAL) {
+        for (uint32_t k = 0; k < (end - cur.p) / 8; k += 128) { // every line once, so that the words come from the cache below
+            uint32_t touched;
+            asm volatile("ld.global.u32 %0, [%1];" : "=r"(touched) : "l"(ga + k / 4));
+        }
+        hi = ga[0], lo = ga[1], nx = ga[2];
+        ga += 3;
+    } else {
+        wa = shared_address(buf) + (cur.p >> 5) * 4;
+        hi = load_shared(wa), lo = load_shared(wa + 4), nx = load_shared(wa + 8);
+        wa += 12;
+    }
+    if (RECORD == kPositions && cur.z == 0) {
         if (blk < limit) pos[blk] = cur.p;
         blk++;
     }
+    if (RECORD == kRecord && cur.z == 0) *rec++ = (uint16_t)(cur.p + blk);
     uint32_t p = cur.p;
-    auto symbol = [&](bool live, bool paired) { // (not live: nothing moves)
+    auto symbol = [&](bool paired) {
         const uint32_t w = __funnelshift_l(lo, hi, st);
         const uint32_t index = (uint32_t)__viaddmax_s32((int)(w >> 16), kHuffFast - 65536, (int)(w >> 22));
-        uint32_t e = 0;
+        uint32_t e;
         asm volatile("{\n\t"
-                     ".reg .pred q;\n\t"
-                     "setp.ne.u32 q, %2, 0;\n\t"
-                     "@q ld.shared.u16 %0, [%1];\n\t"
+                     ".reg .u16 h;\n\t"
+                     "ld.shared.u16 h, [%1];\n\t"
+                     "cvt.u32.u16 %0, h;\n\t"
                      "}"
-                     : "+r"(e)
-                     : "r"(tab + index * 2), "r"((uint32_t)live));
+                     : "=r"(e)
+                     : "r"(tab + index * 2));
         e = __byte_perm(e, 0, 0x1440); // bits consumed to bits 0-7, positions advanced to bits 24-31
         const uint32_t before = st;
         st += e;
-        asm volatile("{\n\t"
-                     ".reg .pred q;\n\t"
-                     ".reg .b32 t;\n\t"
-                     "xor.b32 t, %4, %5;\n\t"
-                     "and.b32 t, t, 32;\n\t"
-                     "setp.ne.u32 q, t, 0;\n\t"
-                     "@q mov.b32 %0, %1;\n\t"
-                     "@q mov.b32 %1, %2;\n\t"
-                     "@q ld.shared.u32 %2, [%3];\n\t"
-                     "@q add.u32 %3, %3, 4;\n\t"
-                     "}"
-                     : "+r"(hi), "+r"(lo), "+r"(nx), "+r"(wa)
-                     : "r"(before), "r"(st));
+        if (GLOBAL)
+            asm volatile("{\n\t"
+                         ".reg .pred q;\n\t"
+                         ".reg .b32 t;\n\t"
+                         "xor.b32 t, %4, %5;\n\t"
+                         "and.b32 t, t, 32;\n\t"
+                         "setp.ne.u32 q, t, 0;\n\t"
+                         "@q mov.b32 %0, %1;\n\t"
+                         "@q mov.b32 %1, %2;\n\t"
+                         "@q ld.global.u32 %2, [%3];\n\t"
+                         "@q add.u64 %3, %3, 4;\n\t"
+                         "}"
+                         : "+r"(hi), "+r"(lo), "+r"(nx), "+l"(ga)
+                         : "r"(before), "r"(st));
+        else
+            asm volatile("{\n\t"
+                         ".reg .pred q;\n\t"
+                         ".reg .b32 t;\n\t"
+                         "xor.b32 t, %4, %5;\n\t"
+                         "and.b32 t, t, 32;\n\t"
+                         "setp.ne.u32 q, t, 0;\n\t"
+                         "@q mov.b32 %0, %1;\n\t"
+                         "@q mov.b32 %1, %2;\n\t"
+                         "@q ld.shared.u32 %2, [%3];\n\t"
+                         "@q add.u32 %3, %3, 4;\n\t"
+                         "}"
+                         : "+r"(hi), "+r"(lo), "+r"(nx), "+r"(wa)
+                         : "r"(before), "r"(st));
         // (closer to the block's end a pair might reach beyond it with its first symbol)
-        const uint32_t to = ac + (paired && st < (uint32_t)(64 - kPairAdvance) << 24 ? pairs : 0);
-        tab = live ? to : tab;
+        tab = ac + (paired && st < (uint32_t)(64 - kPairAdvance) << 24 ? pairs : 0);
         const bool eob = st >= 0x40000000u;
         asm volatile("{\n\t"
                      ".reg .pred q;\n\t"
                      "setp.ge.u32 q, %0, 0x40000000;\n\t"
-                     "@q and.b32 %0, %0, 0x3ffff;\n\t"
+                     "@q and.b32 %0, %0, 0xffffff;\n\t"
                      "@q add.u32 %1, %1, 1;\n\t"
                      "@q and.b32 %2, %4, 0xffff;\n\t"
                      "@q shr.u32 %3, %4, 16;\n\t"
@@ -244,20 +283,22 @@ __device__ __forceinline__ uint32_t walk(const unsigned char *buf, Cursor &cur, 
                      "}"
                      : "+r"(st), "+r"(done), "+r"(tab), "+r"(ac), "+r"(ahead), "+r"(after));
         p = st & kPosMask;
-        if (RECORD) {
+        if (RECORD == kPositions) {
             if (eob && p < end && blk < limit) pos[blk] = p;
             blk += eob ? 1 : 0;
         }
+        if (RECORD == kRecord && eob && done < kRecords) rec[done - 1] = (uint16_t)(st + blk);
     };
     const int pairs_end = (int)end - kHuffBits; // the first symbol of a pair that begins up to here ends before `end`
     if ((int)p <= pairs_end) {
-        do {
-            symbol(true, true);
-            symbol((int)p <= pairs_end, true);
-        } while ((int)p <= pairs_end);
+        while ((int)p <= pairs_end - kLongest) { // (so does one behind it)
+            symbol(true);
+            symbol(true);
+        }
+        while ((int)p <= pairs_end) symbol(true);
         if (st >> 24) tab = ac; // (at 0 it is the DC table)
     }
-    while (p < end) symbol(true, false);
+    while (p < end) symbol(false);
     cur.p = p;
     cur.z = (int)(st >> 24);
     cur.c = (int)((cur.c + done) % s->bpm);
@@ -370,13 +411,11 @@ __device__ __forceinline__ uint32_t unstuff(const AnyTeam &team, unsigned char *
 
 // ---- kernels -------------------------------------------------------------------------------
 
-struct SyncShared {
-    uint16_t entry[kThreads + 2]; // state at the start of every subsequence, relative to it
-    uint16_t blocks[kThreads];    // blocks completed inside it
-    uint8_t list[2][kThreads];    // subsequences to decode (again)
-    int count[2];
+struct GuessShared {
+    uint16_t exit[kThreads];
     int warp[kThreads / 32];
     uint32_t mark[2];
+    alignas(16) uint32_t differ[2][kThreads / 32];
 };
 // Shared memory of a team's stream: the aligned vectors that hold max_raw bytes, and the zero bytes behind.
 __host__ __device__ constexpr size_t stream_bytes(uint32_t max_raw) { return ((size_t)max_raw + 16 + 64 + 31) / 16 * 16; }
@@ -386,24 +425,28 @@ __device__ __forceinline__ bool index_entry_valid(const DecodeIndexHeader *entry
     return h->magic == kDecodeIndexMagic && h->scan_len == d.scan_len && h->subseq_bits == d.subseq_bits && h->segments == d.seg_count;
 }
 
+// Every thread decodes one subsequence, beginning a run-up before it in a guessed state: a block, slot 0, begins there.  Most
+// have fallen in step with the real state where the subsequence begins; scan_repair_kernel sees to the others.  Nothing is
+// exchanged between the threads.
 template <int TEAMS>
-__global__ void __launch_bounds__(kThreads * TEAMS)
-scan_sync_kernel(const ImageDesc *__restrict__ descs, const uint2 *__restrict__ segs, int n_segs, const uint8_t *__restrict__ blob,
-                 const HuffTable *__restrict__ huff, EntropyScratch scratch, const uint8_t *__restrict__ index_pool,
-                 unsigned long long *__restrict__ index_stats, int table_slots, uint32_t buf_bytes) {
+__global__ void __launch_bounds__(kThreads * TEAMS, TEAMS == 4 ? 2 : 1)
+scan_guess_kernel(const ImageDesc *__restrict__ descs, const uint2 *__restrict__ segs, int n_segs, const uint8_t *__restrict__ blob,
+                  const HuffTable *__restrict__ huff, EntropyScratch scratch, const uint8_t *__restrict__ index_pool,
+                  unsigned long long *__restrict__ index_stats, int table_slots, uint32_t buf_bytes, bool local) {
+    const bool local_repair = TEAMS == 1 && local; // (segments that share tables never are)
     extern __shared__ __align__(16) unsigned char s_dyn[];
-    __shared__ SyncShared s_teams[TEAMS];
+    __shared__ GuessShared s_teams[TEAMS];
     next_may_begin();
     const Team<TEAMS> team;
     const int tid = team.tid;
-    SyncShared &sh = s_teams[team.index];
+    GuessShared &sh = s_teams[team.index];
     Tables *tables = reinterpret_cast<Tables *>(s_dyn);
     unsigned char *buf = s_dyn + tables_bytes(table_slots) + team.index * buf_bytes;
     const int mine = blockIdx.x * TEAMS + team.index;
     const uint2 which = segs[min(mine, n_segs - 1)];
     const uint32_t j = which.y;
     const ImageDesc &d = descs[which.x];
-    const uint32_t S = d.subseq_bits, R = d.seg_raw, warm = j == 0 ? 0 : d.seg_warm;
+    const uint32_t S = d.subseq_bits, R = d.seg_raw, run_up = d.seg_run_up, lead = TEAMS > 1 || j == 0 ? 0 : d.seg_warm;
     load_tables(tables, d, huff); // (the same whichever team's sample they are taken from)
     if (TEAMS > 1) {
         copies_wait();
@@ -413,7 +456,7 @@ scan_sync_kernel(const ImageDesc *__restrict__ descs, const uint2 *__restrict__ 
 
     // ---- the segment's raw bytes: run-up, own part, and what follows it to the end of a block
     const uint32_t scan_len = d.scan_len, own0 = j * R, own1 = min(own0 + R, scan_len);
-    const uint32_t raw0 = own0 - min(own0, warm * (S >> 3)), raw1 = min(own1 + kSegOverlap, scan_len);
+    const uint32_t raw0 = own0 - min(own0, (run_up + lead * S) >> 3), raw1 = min(own1 + kSegOverlap, scan_len);
     const uint32_t at[2] = {own0 - raw0, own1 - raw0};
     const uint32_t kept = unstuff(team, buf, blob + d.payload_off + d.scan_off + raw0, raw1 - raw0, raw0 == 0, at, sh.warp, sh.mark);
     const uint32_t own_bit = at[0] == 0 ? 0 : sh.mark[0] * 8, own_end = own1 == raw1 ? kept * 8 : sh.mark[1] * 8;
@@ -422,123 +465,190 @@ scan_sync_kernel(const ImageDesc *__restrict__ descs, const uint2 *__restrict__ 
         const uint4 *src = reinterpret_cast<const uint4 *>(buf);
         for (uint32_t k = tid; k < (kept + 64 + 15) / 16; k += kThreads) dst[k] = src[k];
     }
-    const size_t seg = (size_t)d.seg_first + j;
-    const int n_own = (int)((own_end - own_bit + S - 1) / S), n_subs = (int)warm + n_own;
+    // thread `lead` has the segment's first subsequence, those before it have some that lead up to it
+    const int t = tid - (int)lead, n_own = (int)((own_end - own_bit + S - 1) / S);
+    const size_t seg = (size_t)d.seg_first + j, sub = seg * kSegSubs + max(t, 0);
 
-    if (TEAMS == 1) copies_wait();
+    if (TEAMS == 1) {
+        copies_wait();
+        team.sync();
+    }
 
     // ---- decode index: the states an earlier decode of this very stream left behind (the answer is uniform: a
     // batch is only given an entry that no launch beside it writes)
+    const uint32_t *known = nullptr;
     if (index_pool != nullptr && d.index_use != 0) {
         const DecodeIndexHeader *h = reinterpret_cast<const DecodeIndexHeader *>(index_pool + d.index_off);
         if (index_entry_valid(h, d)) {
-            const uint32_t *src = reinterpret_cast<const uint32_t *>(h + 1) + (size_t)j * (kSegSubs + 2);
-            scratch.sub_info[seg * kSegSubs + tid] = __ldcg(src + tid);
-            if (tid == 0) {
-                scratch.meta[seg] = SegMeta{own_bit, own_end, kept, __ldcg(src + kSegSubs), __ldcg(src + kSegSubs + 1), 0};
-                if (j == 0 && index_stats) atomicAdd(index_stats, 1ull);
-            }
-            return;
+            known = reinterpret_cast<const uint32_t *>(h + 1) + (size_t)j * kSegSubs;
+            if (tid == 0 && j == 0 && index_stats) atomicAdd(index_stats, 1ull);
         }
     }
 
-    // ---- guess and repair.  Subsequences t < warm lie in the run-up.
-    auto start_of = [&](int t) -> int { return (int)own_bit + (t - (int)warm) * (int)S; };
-    sh.entry[tid] = 0; // guess: a block, slot 0, begins here (exact for the scan's first subsequence)
-    sh.blocks[tid] = 0;
-    if (tid == 0) {
-        sh.entry[kThreads] = 0;
-        sh.count[0] = sh.count[1] = 0;
+    const int begin = (int)own_bit + t * (int)S;
+    const bool live = t < n_own && (t >= 0 ? true : begin >= 0);
+    const uint32_t start = (uint32_t)max(begin, 0), end = min(start + S, own_end);
+    uint32_t done = 0, entry = 0;
+    if (live) {
+        Cursor cur{start - min(start, run_up), 0, 0}; // (the scan's first one begins in this state)
+        if (known)
+            cur = unpack(__ldcg(known + t) & 0xffff, start);
+        else
+            walk<kNothing>(buf, cur, start, tables, d, huff);
+        entry = pack(cur, start);
     }
-    team.sync();
-    int n_list = n_subs;
-    for (int round = 0; round <= n_subs && n_list > 0; round++) {
-        int t = -1;
-        uint32_t in = 0;
-        if (tid < n_list) {
-            t = round == 0 ? (start_of(tid) >= 0 ? tid : -1) : sh.list[round & 1][tid];
-            if (t >= 0) in = sh.entry[t];
-        }
-        team.sync(); // every entry state is read before any exit state is written
-        if (tid == 0) sh.count[round & 1] = 0; // filled again from the next round's second half on
-        bool changed = false;
-        if (t >= 0) {
-            const uint32_t start = (uint32_t)start_of(t), end = min(start + S, own_end);
-            Cursor cur = unpack(in, start);
-            sh.blocks[t] = (uint16_t)walk<false>(buf, cur, end, tables, d, huff);
-            const uint32_t out = pack(cur, end);
-            changed = sh.entry[t + 1] != out;
-            if (changed) sh.entry[t + 1] = (uint16_t)out; // only this thread writes entry t + 1 in this round
-            changed = changed && t + 1 < n_subs;
-        }
-        __syncwarp();
-        const uint32_t who = __ballot_sync(0xffffffffu, changed);
-        if (who != 0) { // one place in the next list per warp, then per lane
-            int base = 0;
-            if ((tid & 31) == 0) base = atomicAdd(&sh.count[(round + 1) & 1], __popc(who));
-            base = __shfl_sync(0xffffffffu, base, 0);
-            if (changed) sh.list[(round + 1) & 1][base + __popc(who & ((1u << (tid & 31)) - 1))] = (uint8_t)(t + 1);
+    // With local_repair subsequences are decoded again until each begins where the one before it ends.
+    const bool chained = live && tid > 0 && begin >= (int)S;
+    bool again = live;
+    uint32_t differ;
+    for (int round = 0;; round++) {
+        if (again) {
+            Cursor cur = unpack(entry, start);
+            done = scratch.records && t >= 0 ? walk<kRecord>(buf, cur, end, tables, d, huff, nullptr, 0, 0, scratch.records + sub * kRecords)
+                                             : walk<kNothing>(buf, cur, end, tables, d, huff);
+            sh.exit[tid] = (uint16_t)pack(cur, end);
         }
         team.sync();
-        n_list = sh.count[(round + 1) & 1];
+        const uint32_t before = chained ? sh.exit[tid - 1] : entry;
+        again = before != entry;
+        differ = __ballot_sync(0xffffffffu, again);
+        if ((tid & 31) == 0) sh.differ[round & 1][tid >> 5] = differ;
+        team.sync();
+        const uint4 all = *reinterpret_cast<const uint4 *>(sh.differ[round & 1]);
+        if (!local_repair || round >= kThreads || (all.x | all.y | all.z | all.w) == 0) break;
+        if (again) entry = before;
     }
-
-    // ---- own subsequences: entry state and completed blocks
-    const uint32_t done = tid < n_own ? sh.blocks[tid + warm] : 0;
-    if (tid < n_own) scratch.sub_info[seg * kSegSubs + tid] = sh.entry[tid + warm] | done << 16;
+    const bool own = live && t >= 0;
+    if (own) {
+        scratch.sub_info[sub] = entry | done << 16;
+        scratch.sub_exit[sub] = sh.exit[tid];
+    }
     int total;
-    team_scan(team, (int)done, sh.warp, total);
-    if (tid == 0) scratch.meta[seg] = SegMeta{own_bit, own_end, kept, sh.entry[n_subs], (uint32_t)total, 0};
+    team_scan(team, own ? (int)done : 0, sh.warp, total);
+    // (whether a segment's first one begins where the segment before ends is not known here)
+    if ((tid & 31) == 0) {
+        // (with local_repair none is left; otherwise lead is 0)
+        scratch.meta[seg].doubt[tid >> 5] = (local_repair ? 0 : differ) | (tid == 0 && j > 0 && n_own > 0 ? 1 : 0);
+    }
+    if (tid == 0) {
+        SegMeta &m = scratch.meta[seg];
+        m.own_bit = own_bit, m.own_end = own_end, m.bytes = kept, m.blocks = (uint32_t)total, m.entry = 0;
+    }
 }
 
-// Scans of several segments, one CTA each: the exit state of every segment has to be the entry state
-// the next one worked out from its run-up.  Where it is not, one thread walks on from the exact
-// state, subsequence by subsequence, until it meets the recorded ones; a walk that crosses a whole
-// segment makes the boundary behind it the next round's.
-__global__ void __launch_bounds__(kThreads)
-scan_stitch_kernel(const ImageDesc *__restrict__ descs, const int32_t *__restrict__ list, const HuffTable *__restrict__ huff,
-                   EntropyScratch scratch) {
+// Makes every subsequence begin in the state the one before it ends in, a CTA for `group` parts of scans (of the same
+// tables, unless it is one).  The first one of a part stays as it is, in doubt if anything is before it.  In a round all subsequences in doubt of which that is not so are decoded again from that state; the
+// ones behind them are in doubt in the next round.  A part's first such subsequence is right after the round, so the rounds
+// end.  The subsequences of all parts share the warps, because there are few of them: bound by the chain of look-ups, some
+// 350 a round in the longest ones.
+constexpr size_t kRepairStreams = 26 * 1024; // shared memory for streams (60 KB: 1 % faster alone, 2 % slower in flight)
+constexpr int kRepairThreads = 256, kRepairWarps = kRepairThreads / 32, kRepairList = 1024;
+__global__ void __launch_bounds__(kRepairThreads)
+scan_repair_kernel(const ImageDesc *__restrict__ descs, const uint4 *__restrict__ list, int n_parts, int group,
+                   const HuffTable *__restrict__ huff, EntropyScratch scratch, int table_slots, int stream_vectors, int at_once) {
+    extern __shared__ __align__(16) unsigned char s_dyn[];
+    __shared__ uint32_t s_item[kRepairList]; // subsequence of its scan | part of the group << 28
+    __shared__ uint16_t s_state[kRepairList];
+    __shared__ int s_warp[kRepairWarps], s_most;
     next_may_begin();
-    await_previous();
-    const ImageDesc &d = descs[list[blockIdx.x]];
-    const int tid = threadIdx.x, n_seg = (int)d.seg_count;
-    const uint32_t S = d.subseq_bits;
+    Tables *tables = reinterpret_cast<Tables *>(s_dyn);
+    unsigned char *streams = s_dyn + tables_bytes(table_slots);
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int first = blockIdx.x * group, here = min(group, n_parts - first);
+    bool loaded = false; // the tables
+    // the warps share the parts' segments out, a segment per lane
+    const int parts = kRepairWarps / group, part = warp / group, g = warp % group;
+    const uint4 mine = list[first + min(g, here - 1)];
+    const ImageDesc &d = descs[mine.x];
+    const int n_seg = g < here ? (int)mine.z : 0;
     SegMeta *meta = scratch.meta + d.seg_first;
-    uint32_t *info = scratch.sub_info + (size_t)d.seg_first * kSegSubs;
-    for (int round = 0; round < n_seg; round++) {
-        bool any = false;
-        for (int k0 = 1; k0 < n_seg; k0 += kThreads) { // (a round looks at all boundaries, kThreads at a time)
-            const int k = k0 + tid;
-            uint32_t exact = 0;
-            bool differs = false;
-            if (k < n_seg) {
-                exact = meta[k - 1].exit;
-                // an empty segment (its scan ended in stuffing) hands the state on
-                differs = meta[k].own_bit < meta[k].own_end ? exact != (info[(size_t)k * kSegSubs] & 0xffff) : exact != meta[k].exit;
+    const uint32_t *info = scratch.sub_info + (size_t)d.seg_first * kSegSubs;
+    const uint16_t *exits = scratch.sub_exit + (size_t)d.seg_first * kSegSubs;
+    if (tid == 0) s_most = 0;
+    await_previous();
+    __syncthreads();
+    if (lane == 0) atomicMax(&s_most, n_seg);
+    __syncthreads();
+    const int most = s_most;
+    auto own = [](const SegMeta &m, uint32_t S) -> uint32_t { return (m.own_end - m.own_bit + S - 1) / S; };
+    for (int round = 0; round <= most * group * kSegSubs; round++) {
+        int listed = 0;
+        for (int base = 0; base < most; base += parts * 32) {
+            const int in_part = base + part * 32 + lane, k = (int)mine.y + in_part;
+            uint32_t differ[4] = {0, 0, 0, 0}, kept = 0;
+            if (in_part < n_seg) { // (bits are set by atomic operations, hence not out of the first-level cache)
+                const uint4 doubt = __ldcg(reinterpret_cast<const uint4 *>(meta[k].doubt));
+                const uint32_t words[4] = {doubt.x, doubt.y, doubt.z, doubt.w};
+#pragma unroll
+                for (int q = 0; q < 4; q++)
+                    for (uint32_t left = words[q]; left; left &= left - 1) {
+                        const int bit = __ffs(left) - 1, i = k * kSegSubs + 32 * q + bit;
+                        if ((q | bit) == 0 || ((info[i] ^ exits[i - 1]) & 0xffff) != 0) differ[q] |= 1u << bit;
+                    }
             }
-            if (!__syncthreads_or(differs)) continue;
-            any = true;
-            if (differs) {
-                const SegMeta m = meta[k];
-                const uint32_t *words = reinterpret_cast<const uint32_t *>(scratch.clean + d.clean_off + (size_t)k * d.seg_stride);
-                uint32_t *mine = info + (size_t)k * kSegSubs;
-                const int n_own = (int)((m.own_end - m.own_bit + S - 1) / S);
-                uint32_t state = exact, blocks = m.blocks;
-                int t = 0;
-                for (; t < n_own && (mine[t] & 0xffff) != state; t++) {
-                    const uint32_t start = m.own_bit + (uint32_t)t * S, end = min(start + S, m.own_end);
-                    Cursor cur = unpack(state, start);
-                    const uint32_t done = walk_plain<false>(words, cur, end, d, huff, nullptr, 0, 0);
-                    blocks += done - (mine[t] >> 16);
-                    mine[t] = state | done << 16;
-                    state = pack(cur, end);
+            if (in_part == 0 && k > 0) kept = differ[0] & 1;
+            differ[0] &= ~kept;
+            // (a segment's first one: behind the last of the segment before, which is never empty: an empty one, out of a
+            // scan that ends in stuffing, has none behind it)
+            int before = 0;
+            if (differ[0] & 1) {
+                before = (k - 1) * kSegSubs + (int)own(meta[k - 1], d.subseq_bits) - 1;
+                if (((info[k * kSegSubs] ^ exits[before]) & 0xffff) == 0) differ[0] &= ~1u;
+            }
+            int total;
+            int at = listed + scan_exclusive(__popc(differ[0]) + __popc(differ[1]) + __popc(differ[2]) + __popc(differ[3]), tid, kRepairWarps, s_warp, total,
+                                             [] { __syncthreads(); });
+            // in the order of the segments, so that the first of some part is always among them
+#pragma unroll
+            for (int q = 0; q < 4; q++)
+                for (; differ[q] && at < kRepairList; differ[q] &= differ[q] - 1, at++) {
+                    const int bit = __ffs(differ[q]) - 1, i = k * kSegSubs + 32 * q + bit;
+                    s_item[at] = (uint32_t)i | (uint32_t)g << 28;
+                    s_state[at] = exits[(q | bit) == 0 ? before : i - 1];
                 }
-                meta[k].blocks = blocks;
-                if (t == n_own) meta[k].exit = state;
-            }
-            __syncthreads();
+            if (in_part < n_seg) // the others, for which the list has no room
+                *reinterpret_cast<uint4 *>(meta[k].doubt) = make_uint4(differ[0] | kept, differ[1], differ[2], differ[3]);
+            listed += total;
         }
-        if (!any) break;
+        if (listed == 0) break;
+        if (!loaded) load_tables(tables, descs[list[first].x], huff);
+        loaded = true;
+        const int count = min(listed, kRepairList);
+        for (int begin = 0; begin < count; begin += at_once) {
+            // their streams first: words that come from global memory one by one would keep a warp waiting
+            const int items = min(at_once, count - begin);
+            __syncthreads();
+            for (int v = tid; v < items * stream_vectors; v += kRepairThreads) {
+                const int n = v / stream_vectors;
+                const uint32_t item = s_item[begin + n], i = item & 0xfffffff, k = i / kSegSubs;
+                const ImageDesc &e = descs[list[first + (item >> 28)].x];
+                const uint32_t start = scratch.meta[e.seg_first + k].own_bit + (i - k * kSegSubs) * e.subseq_bits;
+                copy16_async(streams + (size_t)v * 16, reinterpret_cast<const uint4 *>(scratch.clean + e.clean_off + (size_t)k * e.seg_stride) + (start >> 7) + v - n * stream_vectors);
+            }
+            copies_wait();
+            __syncthreads();
+            if (tid < items) {
+                const uint32_t item = s_item[begin + tid], i = item & 0xfffffff, k = i / kSegSubs, t = i - k * kSegSubs, state = s_state[begin + tid];
+                const uint4 its = list[first + (item >> 28)];
+                const ImageDesc &e = descs[its.x];
+                const size_t seg = (size_t)e.seg_first + k, sub = (size_t)e.seg_first * kSegSubs + i;
+                const uint32_t S = e.subseq_bits, start = scratch.meta[seg].own_bit + t * S, end = min(start + S, scratch.meta[seg].own_end);
+                const uint32_t skip = start & ~127u; // position of the copied stream's bit 0
+                const unsigned char *stream = streams + (size_t)tid * stream_vectors * 16;
+                Cursor cur = unpack(state, start - skip);
+                const uint32_t done = scratch.records ? walk<kRecord>(stream, cur, end - skip, tables, e, huff, nullptr, skip, 0, scratch.records + sub * kRecords)
+                                                      : walk<kNothing>(stream, cur, end - skip, tables, e, huff);
+                const uint32_t was = scratch.sub_info[sub] >> 16;
+                scratch.sub_info[sub] = state | done << 16;
+                scratch.sub_exit[sub] = (uint16_t)pack(cur, end - skip);
+                if (done != was) atomicAdd(&scratch.meta[seg].blocks, done - was);
+                if (t + 1 < own(scratch.meta[seg], S))
+                    atomicOr(&scratch.meta[seg].doubt[(t + 1) >> 5], 1u << ((t + 1) & 31));
+                else if (k + 1 < its.y + its.z && scratch.meta[seg + 1].own_bit < scratch.meta[seg + 1].own_end)
+                    atomicOr(&scratch.meta[seg + 1].doubt[0], 1u);
+            }
+        }
+        __syncthreads();
     }
 }
 
@@ -620,7 +730,7 @@ scan_slots_kernel(const ImageDesc *__restrict__ descs, const uint2 *__restrict__
         // (the run-up lacks the bytes that its stuffing took: its first subsequence is shorter)
         const uint32_t start = (uint32_t)max(start_of(t), 0), end = (uint32_t)max(min(start_of(t + 1), (int)own_end), 0);
         Cursor cur = unpack(sh.state[t][i], start);
-        sh.blocks[t][i] = (uint16_t)walk<false>(buf, cur, end, tables, d, huff);
+        sh.blocks[t][i] = (uint16_t)walk<kNothing>(buf, cur, end, tables, d, huff);
         sh.exit[t][i] = (uint16_t)pack(cur, end);
     };
     int lo = 0; // states of this thread's subsequence that were decoded in the last round: [lo, hi)
@@ -711,7 +821,7 @@ scan_slots_kernel(const ImageDesc *__restrict__ descs, const uint2 *__restrict__
         out->info[t][i] = i < sh.count[t + warm] ? sh.state[t + warm][i] | (uint32_t)sh.blocks[t + warm][i] << 16 : kNoState;
         out->next[t][i] = sh.next[t + warm][i];
     }
-    if (tid == 0) scratch.meta[seg] = SegMeta{own_bit, own_end, kept, 0, 0, 0};
+    if (tid == 0) scratch.meta[seg] = SegMeta{own_bit, own_end, kept, 0, 0};
 }
 
 // One CTA per image: follows the real state from segment to segment through their maps.  Many segments are
@@ -748,7 +858,6 @@ scan_chain_kernel(const ImageDesc *__restrict__ descs, const int32_t *__restrict
             behind = __shfl_sync(0xffffffffu, m.to, src);
             if (lane == 0) {
                 meta[k].entry = src;
-                meta[k].exit = behind & 0xffff;
                 meta[k].blocks = behind >> 16;
             }
         } else {
@@ -771,7 +880,7 @@ scan_chain_kernel(const ImageDesc *__restrict__ descs, const int32_t *__restrict
                     uint32_t to = known && t + 1 < n_own ? tab.next[t][i] : kSlotMiss;
                     if (to == kSlotMiss) {
                         Cursor cur = unpack(at, start);
-                        const uint32_t done = walk_plain<false>(words, cur, end, d, huff, nullptr, 0, 0);
+                        const uint32_t done = walk_plain<kNothing>(words, cur, end, d, huff, nullptr, 0, 0, nullptr);
                         tab.info[t][i] = at | done << 16;
                         at = pack(cur, end);
                         blocks += done;
@@ -783,7 +892,6 @@ scan_chain_kernel(const ImageDesc *__restrict__ descs, const int32_t *__restrict
                     i = to;
                 }
                 if (n_own == 0) meta[k].entry = 0;
-                meta[k].exit = at;
                 meta[k].blocks = blocks;
                 behind = at;
             }
@@ -833,16 +941,24 @@ scan_chain_kernel(const ImageDesc *__restrict__ descs, const int32_t *__restrict
     }
 }
 
-template <int TEAMS>
-__global__ void __launch_bounds__(kThreads * TEAMS)
+// Where the blocks of a segment are, and their DC values.  SLOTS: of the samples decoded from every slot, by
+// walking every subsequence once more from its real state, its stream in shared memory.  Otherwise the records
+// say it already, unless a subsequence has more blocks than they hold (or there are none): the segments of
+// such a CTA are walked in global memory.
+template <bool SLOTS>
+constexpr int kIndexTeam = SLOTS ? kSlotSubs : kSegSubs;
+template <int TEAMS, bool SLOTS>
+__global__ void __launch_bounds__(kIndexTeam<SLOTS> * TEAMS, TEAMS == 4 ? 2 : 1)
 scan_index_kernel(const ImageDesc *__restrict__ descs, const uint2 *__restrict__ segs, int n_segs, const HuffTable *__restrict__ huff,
                   EntropyScratch scratch, int32_t *__restrict__ status, uint8_t *__restrict__ index_pool,
                   unsigned long long *__restrict__ index_stats, int table_slots, uint32_t buf_bytes) {
+    constexpr int kThreads = kIndexTeam<SLOTS>;
     extern __shared__ __align__(16) unsigned char s_dyn[];
     __shared__ int s_warps[TEAMS][kThreads / 32];
     __shared__ uint32_t s_lasts[TEAMS];
+    __shared__ __align__(16) uint16_t s_dc[kMaxComponents][1 << kHuffBits]; // first level of the DC tables
     next_may_begin();
-    const Team<TEAMS> team;
+    const Team<TEAMS, kThreads> team;
     const int tid = team.tid;
     int *s_warp = s_warps[team.index];
     uint32_t &s_last = s_lasts[team.index];
@@ -853,16 +969,29 @@ scan_index_kernel(const ImageDesc *__restrict__ descs, const uint2 *__restrict__
     const int img = (int)which.x;
     const uint32_t j = which.y;
     const ImageDesc &d = descs[img];
-    load_tables(tables, d, huff);
-    await_previous();
-    if (TEAMS > 1) {
-        copies_wait();
-        __syncthreads();
-        if (mine >= n_segs) return;
-    }
     const size_t seg = (size_t)d.seg_first + j;
+    if (SLOTS) load_tables(tables, d, huff);
+    for (int t = 0; t < d.n_dc_tab; t++) { // (the same whichever team's sample they are taken from)
+        const uint4 *src = reinterpret_cast<const uint4 *>(huff[d.tab_id[t]].look);
+        for (int k = threadIdx.x; k < (1 << kHuffBits) / 8; k += blockDim.x) reinterpret_cast<uint4 *>(s_dc[t])[k] = src[k];
+    }
+    await_previous();
     const SegMeta m = scratch.meta[seg];
     const uint32_t S = d.subseq_bits, nblocks = d.nblocks;
+    const int n_own = (int)((m.own_end - m.own_bit + S - 1) / S);
+    uint32_t info = 0, n_rec = 0;
+    bool walks = SLOTS;
+    if (!SLOTS) {
+        if (tid < n_own) {
+            info = scratch.sub_info[seg * kSegSubs + tid];
+            n_rec = (info >> 16) + (scratch.sub_exit[seg * kSegSubs + tid] >> 8 ? 1 : 0) - ((info >> 8 & 63) ? 1 : 0);
+        }
+        walks = __syncthreads_or(!scratch.records || n_rec >= kRecords) != 0;
+        if (walks) load_tables(tables, d, huff);
+    }
+    if (SLOTS || walks) copies_wait();
+    __syncthreads();
+    if (TEAMS > 1 && mine >= n_segs) return;
     uint32_t *pos = scratch.pos + d.block_base;
     int16_t *dc = scratch.dc + d.block_base;
 
@@ -873,11 +1002,7 @@ scan_index_kernel(const ImageDesc *__restrict__ descs, const uint2 *__restrict__
         team_scan(team, before, s_warp, all);
         base = (uint32_t)all;
     }
-    const int n_own = (int)((m.own_end - m.own_bit + S - 1) / S);
-    uint32_t info = 0;
-    if (d.slots == 0) {
-        if (tid < n_own) info = scratch.sub_info[seg * kSegSubs + tid];
-    } else { // one thread follows the real state from subsequence to subsequence
+    if (SLOTS) { // one thread follows the real state from subsequence to subsequence
         const SlotTables *t = scratch.slots + (d.slots - 1) + j;
         uint8_t *next = buf, *path = buf + sizeof(t->next); // (the buffer is free until the stream arrives)
         for (int k = tid; k < (int)(sizeof(t->next) / 16); k += kThreads) reinterpret_cast<uint4 *>(next)[k] = reinterpret_cast<const uint4 *>(t->next)[k];
@@ -893,52 +1018,82 @@ scan_index_kernel(const ImageDesc *__restrict__ descs, const uint2 *__restrict__
     }
     int sums[3] = {0, 0, 0};
     if (base < nblocks) { // (uniform) otherwise the crop needs nothing of this segment
-        const uint32_t skip = m.own_bit >> 7; // vectors of the run-up
-        const uint4 *src = reinterpret_cast<const uint4 *>(scratch.clean + d.clean_off + (size_t)j * d.seg_stride);
-        for (uint32_t k = skip + tid; k < (m.bytes + 64 + 15) / 16; k += kThreads) copy16_async(buf + (size_t)(k - skip) * 16, src + k);
-        copies_wait();
+        const unsigned char *stream = scratch.clean + d.clean_off + (size_t)j * d.seg_stride;
+        const uint32_t skip = SLOTS ? m.own_bit >> 7 : 0; // vectors of the run-up
+        if (SLOTS) {
+            for (uint32_t k = skip + tid; k < (m.bytes + 64 + 15) / 16; k += kThreads)
+                copy16_async(buf + (size_t)(k - skip) * 16, reinterpret_cast<const uint4 *>(stream) + k);
+            stream = buf;
+        }
+        if (SLOTS) copies_wait();
         int in_segment;
         const uint32_t first = base + (uint32_t)team_scan(team, (int)(info >> 16), s_warp, in_segment); // (and a barrier for the copies)
-        const uint32_t bias = j * d.seg_stride * 8 + skip * 128; // stream position of the buffer's bit 0
+        const uint32_t bias = j * d.seg_stride * 8 + skip * 128; // position of the walked stream's bit 0
         const uint32_t start = m.own_bit - skip * 128 + (uint32_t)tid * S;
         const uint32_t end = min(start + S, m.own_end - skip * 128);
         Cursor cur = unpack(info & 0xffff, start);
         const uint32_t b0 = first + (cur.z != 0 ? 1 : 0); // the block in progress belongs to the subsequence it began in
         uint32_t b1 = b0;
         int sum[3] = {0, 0, 0};
+        const uint32_t luma = d.ncomp == 1 ? 1 : d.hs * d.vs, bpm = d.bpm;
+        const uint32_t tab = d.dc_tab[0] | (uint32_t)d.dc_tab[1] << 8 | (uint32_t)d.dc_tab[2] << 16;
         if (tid < n_own && first < nblocks && cur.p < end) {
-            const uint32_t stream = shared_address(buf), luma = tables->luma, bpm = tables->bpm;
-            const uint32_t done = walk<true>(buf, cur, end, tables, d, huff, pos, b0, nblocks);
-            b1 = min(first + done + (cur.z != 0 ? 1 : 0), nblocks);
+            const uint16_t *rec = scratch.records + (seg * kSegSubs + tid) * kRecords;
+            if (walks) {
+                const uint32_t done = walk<kPositions, !SLOTS>(stream, cur, end, tables, d, huff, pos, b0, nblocks);
+                n_rec = done + (cur.z != 0 ? 1 : 0) - (b0 - first);
+            }
+            b1 = min(b0 + n_rec, nblocks);
             // the DC symbols of the blocks found: positions move on to the first AC symbol, values count
-            // from the thread's first block
-            uint32_t slot = b0 % bpm, next_pos = b0 < b1 ? pos[b0] : 0;
-            for (uint32_t b = b0; b < b1; b++) {
-                const uint32_t p = next_pos, wa = stream + (p >> 5) * 4;
-                if (b + 1 < b1) next_pos = pos[b + 1];
-                const uint32_t w = __funnelshift_l(load_shared(wa + 4), load_shared(wa), p);
-                const int comp = slot < luma ? 0 : (int)(slot - luma) + 1;
-                const HuffTable *table = huff + d.tab_id[d.dc_tab[comp]];
-                uint32_t e = table->look[w >> (32 - kHuffBits)];
-                if (e & kHuffLong) e = huff_long(table, e, w);
-                const uint32_t n = e & 31, size = (e >> 5) & 15;
-                const int v = size ? huff_value(w, n, size) : 0;
-                sum[0] += comp == 0 ? v : 0;
-                sum[1] += comp == 1 ? v : 0;
-                sum[2] += comp == 2 ? v : 0;
-                pos[b] = bias + p + n;
-                dc[b] = (int16_t)(comp == 0 ? sum[0] : (comp == 1 ? sum[1] : sum[2]));
-                slot = slot + 1 == bpm ? 0 : slot + 1;
+            // from the thread's first block.  Four blocks' words are fetched at a time.
+            uint32_t slot = b0 % bpm;
+            for (uint32_t b = b0; b < b1; b += 4) {
+                uint32_t p[4], w[4];
+                if (walks) {
+#pragma unroll
+                    for (int k = 0; k < 4; k++) p[k] = b + k < b1 ? pos[b + k] : start;
+                } else {
+                    const uint2 r = *reinterpret_cast<const uint2 *>(rec + (b - b0));
+                    const uint32_t low[4] = {r.x & 0xffff, r.x >> 16, r.y & 0xffff, r.y >> 16};
+#pragma unroll
+                    for (int k = 0; k < 4; k++) p[k] = b + k < b1 ? start + ((low[k] - start) & 0xffff) : start;
+                }
+#pragma unroll
+                for (int k = 0; k < 4; k++) {
+                    const uint32_t *at = reinterpret_cast<const uint32_t *>(stream) + (p[k] >> 5);
+                    w[k] = __funnelshift_l(at[1], at[0], p[k]);
+                }
+#pragma unroll
+                for (int k = 0; k < 4; k++) {
+                    if (b + k >= b1) break;
+                    const int comp = slot < luma ? 0 : (int)(slot - luma) + 1, t = tab >> 8 * comp & 255;
+                    uint32_t e = s_dc[t][w[k] >> (32 - kHuffBits)];
+                    if (e & kHuffLong) e = huff_long(huff + d.tab_id[t], e, w[k]);
+                    const uint32_t n = e & 31, size = (e >> 5) & 15;
+                    const int v = size ? huff_value(w[k], n, size) : 0;
+                    sum[0] += comp == 0 ? v : 0;
+                    sum[1] += comp == 1 ? v : 0;
+                    sum[2] += comp == 2 ? v : 0;
+                    pos[b + k] = bias + p[k] + n;
+                    dc[b + k] = (int16_t)(comp == 0 ? sum[0] : (comp == 1 ? sum[1] : sum[2]));
+                    slot = slot + 1 == bpm ? 0 : slot + 1;
+                }
             }
         }
         // what the segment holds before the thread's first block
         int before[3];
 #pragma unroll
         for (int c = 0; c < 3; c++) before[c] = c < d.ncomp ? team_scan(team, sum[c], s_warp, sums[c]) : 0;
-        uint32_t slot = b0 % tables->bpm;
-        for (uint32_t b = b0; b < b1; b++) {
-            dc[b] = (int16_t)(dc[b] + (slot < tables->luma ? before[0] : (slot == tables->luma ? before[1] : before[2])));
-            slot = slot + 1 == tables->bpm ? 0 : slot + 1;
+        uint32_t slot = b0 % bpm;
+        for (uint32_t b = b0; b < b1; b += 4) {
+            int v[4];
+#pragma unroll
+            for (int k = 0; k < 4; k++) v[k] = b + k < b1 ? dc[b + k] : 0;
+#pragma unroll
+            for (int k = 0; k < 4; k++) {
+                if (b + k < b1) dc[b + k] = (int16_t)(v[k] + (slot < luma ? before[0] : (slot == luma ? before[1] : before[2])));
+                slot = slot + 1 == bpm ? 0 : slot + 1;
+            }
         }
     }
     if (tid == 0) {
@@ -950,15 +1105,10 @@ scan_index_kernel(const ImageDesc *__restrict__ descs, const uint2 *__restrict__
     const bool record = index_pool != nullptr && (d.index_use & 2) != 0 && d.host_status == 0 &&
                         !index_entry_valid(reinterpret_cast<const DecodeIndexHeader *>(index_pool + d.index_off), d);
     if (record) {
-        uint32_t *dst = reinterpret_cast<uint32_t *>(index_pool + d.index_off + sizeof(DecodeIndexHeader)) + (size_t)j * (kSegSubs + 2);
+        uint32_t *dst = reinterpret_cast<uint32_t *>(index_pool + d.index_off + sizeof(DecodeIndexHeader)) + (size_t)j * kSegSubs;
         dst[tid] = info;
-        if (tid == 0) {
-            dst[kSegSubs] = m.exit;
-            dst[kSegSubs + 1] = m.blocks;
-        }
     }
     // ---- the CTA that finishes an image last turns the segments' DC sums into sums before them
-    if (TEAMS == 1) copies_wait(); // (nothing may be under way when the CTA ends)
     __threadfence();
     team.sync();
     if (tid == 0) s_last = atomicInc(&scratch.done[img], d.seg_count - 1) == d.seg_count - 1 ? 1 : 0; // wraps back to 0
@@ -1115,34 +1265,45 @@ scan_restart_kernel(const ImageDesc *__restrict__ descs, const int32_t *__restri
 
 } // namespace
 
+// Run-up before a subsequence, in bits.  Shorter ones leave more to repair: 1600 / 800 bits 244 us instead of 229 alone and
+// 370 instead of 368 as one of four in flight (1024 photographs), 1280 / 640 270 and 372.
+constexpr uint32_t kRunUp = 1920, kRunUpFewSlots = 960;
+
 uint32_t subseq_target(uint64_t total_bits) {
-    // A subsequence costs a re-synchronisation (0.9 kbit, 0.35 without subsampling) on top of its own length, so
-    // long ones are less work; short ones are a shorter chain, which decides while few bits leave the GPU
-    // mostly idle.  256 subsequences per SM are enough of them: batches of 80 Mbit, alone / four in flight, take
-    // 473 / 335 us at 512 bits, 424 / 274 at 1024, 388 / 255 at 1280; a 4:4:4 scan of 24 Mbit 554 us at 256 bits,
-    // 505 at 512, 499 at 768, 509 at 1024.
-    const uint64_t t = total_bits / (148 * 256);
+    // A subsequence costs a run-up on top of its own length, so long ones are less work; short ones are a shorter chain,
+    // which decides while few bits leave the GPU mostly idle.  Batches of 80 Mbit, alone / as one of four in flight, all
+    // kernels: 352 / 211 us with 200 subsequences per SM, 355 / 208 with 320, 390 / 226 with 480.
+    const uint64_t t = total_bits / (148 * 320);
     return (uint32_t)(t < 256 ? 256 : (t > kMaxSubseqBits ? kMaxSubseqBits : (t + 31) / 32 * 32));
 }
 
-ScanLayout layout_scan(uint32_t scan_len, uint32_t target_bits) {
+ScanLayout layout_scan(uint32_t scan_len, uint32_t target_bits, int bpm, bool local_repair) {
     ScanLayout l{};
-    const uint64_t bits = (uint64_t)scan_len * 8;
-    const uint32_t warm = (8192 + target_bits - 1) / target_bits; // all but one in 10^4 run-ups are long enough
-    if (bits <= (uint64_t)kSegSubs * target_bits || (target_bits > 512 && bits <= (uint64_t)kSegSubs * kMaxSubseqBits)) {
-        l.seg_count = 1;
-        l.subseq_bits = (uint32_t)((bits + kSegSubs - 1) / kSegSubs + 31) / 32 * 32;
-        if (l.subseq_bits < 128) l.subseq_bits = 128;
-        l.seg_raw = kSegSubs * l.subseq_bits / 8;
-    } else {
-        const uint64_t own = kSegSubs - warm;
-        l.seg_count = (uint32_t)((bits + own * target_bits - 1) / (own * target_bits));
-        l.subseq_bits = (uint32_t)((bits + own * l.seg_count - 1) / (own * l.seg_count) + 31) / 32 * 32;
-        l.seg_warm = warm;
-        l.seg_raw = (uint32_t)own * l.subseq_bits / 8;
-        l.seg_count = (scan_len + l.seg_raw - 1) / l.seg_raw;
+    const uint64_t bits = (uint64_t)scan_len * 8, target = target_bits;
+    auto up = [](uint64_t a, uint64_t b) { return (a + b - 1) / b; };
+    l.seg_run_up = bpm > 3 ? kRunUp : kRunUpFewSlots;
+    l.seg_count = 1;
+    uint64_t own = kSegSubs; // subsequences of a segment
+    if (local_repair) {
+        if (bits > own * target) {
+            // (8 kbit before a segment: all but one in 10^4 of its first subsequences begin in the real state then)
+            l.seg_warm = (uint32_t)up(8192 - l.seg_run_up, target);
+            own -= l.seg_warm;
+            l.seg_count = (uint32_t)up(bits, own * target);
+        }
+    } else { // two warps at most (128 of them share the SM's memory out worse: 64 images of 14 Mbit 696 us instead of 653)
+        own = 64;
+        l.seg_count = (uint32_t)up(bits, own * target);
+        if (l.seg_count < 1) l.seg_count = 1;
+        own = 32 * up(bits, 32 * target * l.seg_count);
+        if (own < 32) own = 32;
     }
-    l.seg_stride = (kSegSubs * l.subseq_bits / 8 + kSegOverlap + 64 + 31) / 16 * 16;
+    l.subseq_bits = (uint32_t)up(up(bits, own * l.seg_count), 32) * 32;
+    if (l.subseq_bits < 128) l.subseq_bits = 128;
+    l.seg_raw = (uint32_t)own * l.subseq_bits / 8;
+    l.seg_count = scan_len ? (scan_len + l.seg_raw - 1) / l.seg_raw : 1;
+    l.seg_stride = (((uint32_t)own + l.seg_warm) * l.subseq_bits + l.seg_run_up) / 8 + kSegOverlap + 64 + 31;
+    l.seg_stride = l.seg_stride / 16 * 16;
     return l;
 }
 
@@ -1173,16 +1334,28 @@ void launch_entropy_decode(const ImageDesc *descs, const EntropyWork &work, cons
         auto allow = [](auto kernel, size_t smem) { cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); };
         // With enough segments to fill every SM four teams share a set of tables: eight segments of up to
         // 22 KB fit an SM then, instead of five.
-        const int teams = work.alike && n_segs >= 148 * 5 ? 4 : 1;
+        const int teams = work.alike && !work.local_repair && n_segs >= 148 * 5 ? 4 : 1;
         const size_t smem = tables_bytes(tables) + (size_t)teams * buf;
         if (work.n_guess > 0) {
             const int grid = (work.n_guess + teams - 1) / teams;
             auto run = [&](auto kernel) {
                 allow(kernel, smem);
-                kernel<<<grid, kThreads * teams, smem, stream>>>(descs, work.segs, work.n_guess, blob, huff, scratch, index_pool, index_stats, tables, buf);
+                kernel<<<grid, kThreads * teams, smem, stream>>>(descs, work.segs, work.n_guess, blob, huff, scratch, index_pool, index_stats, tables, buf,
+                                                                 work.local_repair);
             };
-            if (teams == 4) run(scan_sync_kernel<4>); else run(scan_sync_kernel<1>);
-            if (work.n_multi > 0) launch(early, work.n_multi, kThreads, 0, stream, scan_stitch_kernel, descs, work.multi, huff, scratch);
+            if (teams == 4) run(scan_guess_kernel<4>); else run(scan_guess_kernel<1>);
+            int group = 1;
+            while (work.alike && group < kRepairWarps && work.n_parts >= 256 * group) group *= 2;
+            // (a subsequence may begin behind its first vector's start, and 64 bytes beyond)
+            const int vectors = (int)(work.max_subseq_bits / 128 + 5);
+            const int at_once = (int)std::min<size_t>(kRepairThreads, kRepairStreams / (16 * vectors));
+            const size_t repair = tables_bytes(tables) + (size_t)at_once * vectors * 16;
+            allow(scan_repair_kernel, repair);
+            launch(early, (work.n_parts + group - 1) / group, kRepairThreads, repair, stream, scan_repair_kernel, descs, work.parts, work.n_parts, group, huff,
+                   scratch, tables, vectors, at_once);
+            if (work.n_whole > 0)
+                launch(early, work.n_whole, kRepairThreads, repair, stream, scan_repair_kernel, descs, work.parts + work.n_parts, work.n_whole, 1, huff, scratch,
+                       tables, vectors, at_once);
         }
         if (work.n_slots > 0) {
             const size_t one = tables_bytes(tables) + buf;
@@ -1198,12 +1371,15 @@ void launch_entropy_decode(const ImageDesc *descs, const EntropyWork &work, cons
             allow(scan_chain_kernel, maps);
             launch(early, work.n_slot_images, warps * 32, maps, stream, scan_chain_kernel, descs, work.slot_images, huff, scratch, slots);
         }
-        auto run = [&](auto kernel) {
-            allow(kernel, smem);
-            launch(early, (n_segs + teams - 1) / teams, kThreads * teams, smem, stream, kernel, descs, work.segs, n_segs, huff, scratch, status, index_pool,
-                   index_stats, tables, buf);
+        auto index = [&](auto kernel, const uint2 *segs, int n, int team, size_t bytes) {
+            allow(kernel, bytes);
+            launch(early, (n + teams - 1) / teams, team * teams, bytes, stream, kernel, descs, segs, n, huff, scratch, status, index_pool, index_stats, tables,
+                   buf);
         };
-        if (teams == 4) run(scan_index_kernel<4>); else run(scan_index_kernel<1>);
+        if (work.n_guess > 0)
+            index(teams == 4 ? scan_index_kernel<4, false> : scan_index_kernel<1, false>, work.segs, work.n_guess, kIndexTeam<false>, tables_bytes(tables));
+        if (work.n_slots > 0)
+            index(teams == 4 ? scan_index_kernel<4, true> : scan_index_kernel<1, true>, work.segs + work.n_guess, work.n_slots, kIndexTeam<true>, smem);
     }
     if (work.n_restart > 0)
         scan_restart_kernel<<<work.n_restart, kRestartThreads, 0, stream>>>(descs, work.restart, blob, huff, scratch, status);

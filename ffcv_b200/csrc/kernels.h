@@ -48,10 +48,13 @@ void launch(bool early, dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
 
 // Scratch and results of the entropy decode of a batch (device memory, no initialisation needed
 // except `done`, which starts at zero once and is left at zero).
+constexpr size_t kSegScratch = sizeof(SegMeta) + (4 + 2) * kSegSubs + 16; // bytes per segment of meta, sub_info, sub_exit and seg_dc
 struct EntropyScratch {
     uint8_t *clean;      // unstuffed streams (ImageDesc::clean_off), 512 spare bytes behind them
     SegMeta *meta;       // per segment
     uint32_t *sub_info;  // per segment kSegSubs words: state at the start of a subsequence, blocks << 16
+    uint16_t *sub_exit;  // per segment kSegSubs: the state that leads to at its end
+    uint16_t *records;   // per segment kSegSubs x kRecords: where the blocks of a subsequence begin (16-byte aligned; nullptr: not kept)
     SlotTables *slots;   // per segment of the samples with ImageDesc::slots
     int32_t *seg_dc;     // per segment four words: DC value of each component before the segment
     uint32_t *done;      // per sample
@@ -63,12 +66,14 @@ struct EntropyScratch {
 struct EntropyWork {
     const uint2 *segs;     // (sample, segment) of every segment of the samples without restart markers:
     int n_guess, n_slots;  // first the n_guess of samples decoded from one guess per subsequence, then those with ImageDesc::slots
-    const int32_t *multi;  // samples of the first kind with more than one segment
-    int n_multi;
+    const uint4 *parts;    // (sample, first segment, segments) of the samples of the first kind in parts that are repaired
+    int n_parts, n_whole;  // on their own, see repair_parts; then those of the n_whole samples in several parts as a whole
     const int32_t *slot_images; // samples of the second kind
     int n_slot_images;
     const int32_t *restart; // samples with restart markers
     int n_restart;
+    uint32_t max_subseq_bits; // of the samples decoded from one guess
+    bool local_repair;     // see local_repair
     uint32_t max_raw;      // bounds a segment's raw bytes with run-up and overlap
     int max_tables;        // bounds the tables of a sample in shared memory (its distinct DC tables and twice its AC tables)
     int max_slot_segs;     // most segments of one of slot_images
@@ -84,11 +89,25 @@ void launch_entropy_decode(const ImageDesc *descs, const EntropyWork &work, cons
                            cudaStream_t stream);
 
 // How a scan of scan_len bytes is cut into subsequences and segments.  `target_bits`: wished length of
-// a subsequence, see subseq_target.
+// a subsequence, see subseq_target; bpm: blocks of an MCU.
 struct ScanLayout {
-    uint32_t subseq_bits, seg_raw, seg_warm, seg_stride, seg_count;
+    uint32_t subseq_bits, seg_raw, seg_warm, seg_run_up, seg_stride, seg_count;
 };
-ScanLayout layout_scan(uint32_t scan_len, uint32_t target_bits);
+ScanLayout layout_scan(uint32_t scan_len, uint32_t target_bits, int bpm, bool local_repair);
+// Where a batch leaves SMs idle, subsequences that began in the wrong state are decoded again at once, by the threads that have
+// their segment's bytes: a shorter way than scan_repair_kernel, but a segment keeps its shared memory until the last one
+// is right.  So too for a single image, beside which nothing runs.  One of 24 Mbit (4:4:4) / 33 Mbit (4:2:0), all kernels of
+// the entropy decode: 119 and 224 us with repairs behind, 91 and 182 this way.
+inline bool local_repair(uint32_t target_bits, int n_images) { return target_bits < kMaxSubseqBits / 2 || n_images == 1; }
+// Otherwise a scan of seg_count segments is repaired in parts: one, or, of long scans, of kRepairPart segments each, and what
+// they leave at their seams by one CTA afterwards.
+constexpr uint32_t kRepairPart = 32;
+inline uint32_t repair_parts(uint32_t seg_count, bool local) { return local || seg_count <= 2 * kRepairPart ? 1 : (seg_count + kRepairPart - 1) / kRepairPart; }
+inline uint4 repair_part(uint32_t sample, uint32_t seg_count, uint32_t parts, uint32_t k) {
+    if (parts == 1) return make_uint4(sample, 0, seg_count, 0);
+    const uint32_t first = k * kRepairPart, left = seg_count - first;
+    return make_uint4(sample, first, left < kRepairPart ? left : kRepairPart, 0);
+}
 // The same for a scan decoded from every slot at once, which is done while a batch's scans leave most of
 // the GPU idle otherwise: three times the work, but a chain of 4 x 512 bits instead of 6 to 10 kbit.  Kernels of a
 // batch of 4:2:0 photographs, alone / as one of four in flight, from every slot and from one guess: 0.2 Mbit 77 / 23

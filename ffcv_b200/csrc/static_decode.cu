@@ -34,9 +34,9 @@ constexpr size_t kMaxSegments = kMaxStreamBytes / ((kSegSubs / 2) * kSubseqTarge
 constexpr size_t kMaxBlocks = 3 * kMaxPaddedSamples / 64;
 constexpr size_t kMaxTiles = kMaxBlocks / kBlockTile + 4;
 constexpr size_t kMetaBytes = 96 * 1024;                             // descriptor, tables, lists, status
-// unstuffed bit stream: every segment with its run-up and overlap, at most half as much again
-constexpr size_t kCleanBytes = kMaxStreamBytes + kMaxStreamBytes / 2 + 4096;
-constexpr size_t kSegBytes = (kMaxSegments * (sizeof(SegMeta) + 4 * kSegSubs + 16) + 255) / 256 * 256;
+// unstuffed bit stream: every segment with its run-up and overlap, at most 1.58 times as much
+constexpr size_t kCleanBytes = kMaxStreamBytes + kMaxStreamBytes * 5 / 8 + 8192;
+constexpr size_t kSegBytes = (kMaxSegments * kSegScratch + 255) / 256 * 256;
 constexpr size_t kIndexBytes = (kMaxBlocks * 6 + 255) / 256 * 256;   // position and DC value of every block
 constexpr size_t kPlaneBytes = 3 * kMaxPaddedSamples + 1024;         // each plane rounded up to 256
 constexpr size_t kCleanOff = kMetaBytes;
@@ -57,6 +57,7 @@ struct Meta {
     ImageDesc desc;
     int32_t list[4];
     int32_t status[4]; // [0] the image's status, [1] its counter of finished segments
+    uint4 part;
     uint2 segs[kMaxSegments];
     uint2 tiles[kMaxTiles];
     alignas(16) HuffTable huff[6]; // read with 16-byte loads
@@ -150,16 +151,18 @@ extern "C" int ffcvb_imdecode_static(const uint8_t *jpeg_host, uint64_t jpeg_siz
 
     int n_segs = 0;
     if (!d.restart_interval) {
-        const ScanLayout l = layout_scan(d.scan_len, kSubseqTarget);
+        const ScanLayout l = layout_scan(d.scan_len, kSubseqTarget, d.bpm, true);
         d.subseq_bits = l.subseq_bits;
         d.seg_raw = l.seg_raw;
         d.seg_warm = l.seg_warm;
+        d.seg_run_up = l.seg_run_up;
         d.seg_stride = l.seg_stride;
         d.seg_count = l.seg_count;
         n_segs = (int)l.seg_count;
         if (l.seg_count > kMaxSegments || (size_t)l.seg_count * l.seg_stride + 512 > kCleanBytes)
             return reject(FFCVB_E_LIMIT, "JPEG stream too large for the static scratch");
         for (uint32_t k = 0; k < l.seg_count; k++) m.segs[k] = make_uint2(0, k);
+        m.part = repair_part(0, l.seg_count, 1, 0);
     }
     const uint32_t n_tiles = block_tiles(d);
     if (n_tiles > kMaxTiles || d.nblocks > kMaxBlocks) return reject(FFCVB_E_LIMIT, "image larger than FFCVB_STATIC_MAX_PADDED_PIXELS");
@@ -185,17 +188,21 @@ extern "C" int ffcvb_imdecode_static(const uint8_t *jpeg_host, uint64_t jpeg_siz
     es.clean = scratch + kCleanOff;
     es.seg_dc = reinterpret_cast<int32_t *>(scratch + kSegOff);
     es.sub_info = reinterpret_cast<uint32_t *>(es.seg_dc + 4 * kMaxSegments);
-    es.meta = reinterpret_cast<SegMeta *>(es.sub_info + kSegSubs * kMaxSegments);
+    es.sub_exit = reinterpret_cast<uint16_t *>(es.sub_info + kSegSubs * kMaxSegments);
+    es.meta = reinterpret_cast<SegMeta *>(es.sub_exit + kSegSubs * kMaxSegments);
     es.done = reinterpret_cast<uint32_t *>(&meta_dev->status[1]);
     es.pos = reinterpret_cast<uint32_t *>(scratch + kIndexOff);
     es.dc = reinterpret_cast<int16_t *>(es.pos + kMaxBlocks);
     EntropyWork work{};
     work.segs = meta_dev->segs;
     work.n_guess = n_segs;
-    work.multi = work.restart = list_dev;
-    work.n_multi = n_segs > 1 ? 1 : 0;
+    work.restart = list_dev;
+    work.parts = &meta_dev->part;
+    work.n_parts = n_segs > 0 ? 1 : 0;
+    work.max_subseq_bits = d.subseq_bits;
+    work.local_repair = true;
     work.n_restart = d.restart_interval ? 1 : 0;
-    work.max_raw = kSegSubs * d.subseq_bits / 8 + kSegOverlap;
+    work.max_raw = d.seg_stride; // (run-up, own bytes and overlap)
     work.max_tables = 3 * d.n_dc_tab;
     launch_entropy_decode(desc_dev, work, jpeg_dev, meta_dev->huff, es, meta_dev->status, nullptr, nullptr, st);
     launch_blocks(desc_dev, meta_dev->tiles, (int)n_tiles, meta_dev->huff, meta_dev->mult, es, scratch + kPlaneOff, work.early(), st);

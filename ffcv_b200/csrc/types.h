@@ -10,13 +10,13 @@ namespace ffcvb {
 constexpr int kMaxComponents = 3;
 constexpr int kPayloadAlign = 16;
 
-// A scan is entropy-decoded in segments of kSegSubs subsequences, one CTA each.  kSegOverlap raw
+// A scan is entropy-decoded in segments of up to kSegSubs subsequences, a thread each.  kSegOverlap raw
 // bytes behind a segment are unstuffed with it, so that a block that begins inside can be read to
 // its end (63 symbols of at most 26 bits = 205 bytes, twice that when every second byte is stuffing).
 constexpr int kSegSubs = 128;
 constexpr int kSegOverlap = 512;
-constexpr int kMaxSubseqBits = 1280; // longest subsequence: bounds a segment's shared memory
-static_assert(kSegSubs * kMaxSubseqBits + 8 * kSegOverlap < 1 << 18, "a position inside a segment has 18 bits");
+constexpr int kMaxSubseqBits = 2560; // longest subsequence: bounds a segment's shared memory
+static_assert(kSegSubs * kMaxSubseqBits + 8 * kSegOverlap + 4096 < 1 << 24, "a position inside a segment has 24 bits");
 // Few scans are decoded from every possible block slot at once (scan_slots_kernel): segments of up to
 // kSlotSubs subsequences of kSlotBits bits, each with up to kSlotStates entry states; the last place is kept
 // for a state that was not found in time.
@@ -70,9 +70,9 @@ struct ImageDesc {
     uint16_t dec_height, dec_width;
     // Entropy decode in segments (scans without restart markers): length in bits of the
     // subsequences (multiple of 32); raw bytes of a segment; subsequences of run-up before every
-    // segment but the first; bytes of a segment's place in the unstuffed stream; and which of the
+    // segment but the first; bits of run-up before every subsequence (a multiple of 32); bytes of a segment's place in the unstuffed stream; and which of the
     // batch's segments are this image's.
-    uint32_t subseq_bits, seg_raw, seg_warm, seg_stride, seg_first, seg_count;
+    uint32_t subseq_bits, seg_raw, seg_warm, seg_run_up, seg_stride, seg_first, seg_count;
     uint32_t slots;        // decoded from every slot at once: 1 + the first of the image's SlotTables (0: not)
     uint32_t index_use;    // place in the decode index: 0 none, bit 0 the entry may be read, bit 1 and is written
     uint64_t index_off;    // byte offset of the entry in the context's index pool
@@ -155,22 +155,27 @@ struct MultTable {
     uint16_t q[64];
 };
 
-// Segment of a scan as scan_sync_kernel leaves it.  Bits count from the start of the segment's
+// Segment of a scan as scan_guess_kernel leaves it.  Bits count from the start of the segment's
 // place in the unstuffed stream.
-struct SegMeta {
+struct alignas(16) SegMeta {
     uint32_t own_bit, own_end; // the segment's own bits (behind its run-up, before its overlap)
     uint32_t bytes;            // unstuffed bytes, overlap included
-    uint32_t exit;             // decoder state behind own_end (as in sub_info)
     uint32_t blocks;           // blocks completed in the segment
     uint32_t entry;            // SlotTables: which state of the first subsequence is the real one
+    uint32_t pad[3];
+    uint32_t doubt[kSegSubs / 32]; // a bit per subsequence that may not begin in the state the one before it ends in
 };
+
+// Positions of its blocks that the decode of a subsequence writes down as it goes (the last place is spare): 20 bits a
+// block in the longest ones.
+constexpr int kRecords = 128;
 
 constexpr uint32_t kNoBlock = 0xFFFFFFFFu; // position of a block that the scan does not hold
 
 // Decode index: what a finished decode of a stream knows and the next decode of the same stream can
 // start from -- the exact decoder state at the start of every subsequence and the number of blocks
 // completed in it.  With it no guess has to be repaired.  An entry lives in device memory:
-//   [DecodeIndexHeader][per segment: uint32 sub_info x kSegSubs, uint32 exit, uint32 blocks]
+//   [DecodeIndexHeader][per segment: uint32 sub_info x kSegSubs]
 // and is valid when `magic` is set (written last) and the other fields match.  Which batch writes it and which
 // may read it is settled on the host (DecodeIndex).
 struct DecodeIndexHeader {
@@ -178,7 +183,7 @@ struct DecodeIndexHeader {
 };
 constexpr uint32_t kDecodeIndexMagic = 0x58444947u;
 FFCVB_HD inline size_t decode_index_bytes(uint32_t segments) {
-    return (sizeof(DecodeIndexHeader) + (size_t)segments * (kSegSubs + 2) * 4 + 15) / 16 * 16;
+    return (sizeof(DecodeIndexHeader) + (size_t)segments * kSegSubs * 4 + 15) / 16 * 16;
 }
 
 struct BatchHeader {

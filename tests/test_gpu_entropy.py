@@ -178,3 +178,53 @@ def test_batches_whose_kernels_begin_early(n):
     for got, want in zip(outs, wants):
         assert np.array_equal(got.cpu().numpy(), want)
     ctx.close()
+
+
+def _stage_and_check(bufs, h, w):
+    """One batch of JPEG streams of one shape, decoded whole."""
+    from ffcv_b200 import libffcv as L
+    n = len(bufs)
+    sizes = np.array([b.size for b in bufs], np.uint64)
+    ctx = L.Context(0, 1, 4)
+    out = ch.zeros((n, h, w, 3), dtype=ch.uint8, device='cuda')
+    stream = ch.cuda.current_stream().cuda_stream
+    ctx.stage(0, np.concatenate(bufs), np.concatenate([[0], np.cumsum(sizes)[:-1]]).astype(np.uint64), sizes, np.zeros(n, np.uint8),
+              np.full(n, h, np.uint16), np.full(n, w, np.uint16), L.make_plan(h, w, 0, L.OUT_U8_NHWC),
+              np.tile(np.array([0, 0, h, w], np.int32), (n, 1)))
+    ctx.submit(0, stream, out.data_ptr())
+    assert (ctx.status(0, stream, n) == 0).all()
+    got = out.cpu().numpy()
+    for k, b in enumerate(bufs):
+        assert np.array_equal(got[k], O.jpeg_decode(b)), k
+    ctx.close()
+
+
+@pytest.mark.parametrize('subseq_bits', [128, 512, 2560])
+@pytest.mark.parametrize('sampling', [420, 444])
+def test_subsequences_of_very_many_blocks(subseq_bits, sampling, monkeypatch):
+    """Flat images: a subsequence holds up to 500 blocks, of which only 127 are written down; flat and busy parts in
+    one scan, so that segments of both kinds follow one another."""
+    monkeypatch.setenv('FFCV_B200_SUBSEQ_BITS', str(subseq_bits))
+    rng = np.random.default_rng(subseq_bits + sampling)
+    h, w = 640, 560
+    flat = np.full((h, w, 3), 117, np.uint8)
+    half = flat.copy()
+    half[200:330] = rng.integers(0, 256, (130, w, 3))
+    ramp = np.clip(np.arange(w)[None, :, None] // 9 + np.zeros((h, 1, 3)) + rng.integers(0, 2, (h, w, 3)), 0, 255).astype(np.uint8)
+    flags = [cv2.IMWRITE_JPEG_QUALITY, 85]
+    if sampling == 444:
+        flags += [cv2.IMWRITE_JPEG_SAMPLING_FACTOR, cv2.IMWRITE_JPEG_SAMPLING_FACTOR_444]
+    bufs = [cv2.imencode('.jpg', im, flags)[1].reshape(-1).copy() for im in (flat, half, ramp)]
+    _stage_and_check(bufs, h, w)
+
+
+@pytest.mark.parametrize('n', [255, 256, 517, 1030])
+def test_images_that_share_a_repair(n, monkeypatch):
+    """From 256, 512 and 1024 images of the same tables on, two, four and eight of them are repaired by one CTA;
+    noise, so that many subsequences have to be, and several rounds of them."""
+    monkeypatch.setenv('FFCV_B200_SUBSEQ_BITS', '128')
+    rng = np.random.default_rng(n)
+    h, w = 40, 56
+    few = [cv2.imencode('.jpg', rng.integers(0, 256, (h, w, 3), np.uint8), [cv2.IMWRITE_JPEG_QUALITY, int(rng.integers(70, 97))])[1].reshape(-1).copy()
+           for _ in range(40)]
+    _stage_and_check([few[int(rng.integers(0, 40))] for _ in range(n)], h, w)
