@@ -278,6 +278,8 @@ struct Slot {
     uint64_t jpeg_list_off = 0, segs_off = 0, parts_off = 0, slot_images_off = 0, restart_off = 0, block_tiles_off = 0, quad_tiles_off = 0;
     uint64_t status_off = 0; // status word and counter of finished segments of every sample
     uint64_t items_off = 0;  // ResizeItem of every sample
+    uint64_t gather_off = 0; // gather_ranges, for so many CTAs (0: nothing is gathered)
+    int gather_ctas = 0;
     int n_block_tiles = 0, n_quad_tiles = 0, bands = 1;
     uint32_t total_blocks = 0;
     size_t clean_bytes = 0, plane_bytes = 0, rgb_bytes = 0, scan_bytes = 0, raw_bytes = 0, jpeg_bytes = 0;
@@ -1168,6 +1170,9 @@ int stage_impl(ffcvb_ctx *ctx, int slot, const Source &source, const uint64_t *p
         off = align_up(off + sizeof(uint2) * blk_tiles.size(), 16);
         s.quad_tiles_off = off;
         off = align_up(off + sizeof(uint2) * quad_tiles.size(), 16);
+        s.gather_off = off;
+        s.gather_ctas = direct && s.range_len == 0 ? (ctx->gather_ctas < 1 ? kGatherCtas : ctx->gather_ctas) : 0;
+        if (s.gather_ctas) off = align_up(off + sizeof(uint2) * (s.gather_ctas + 1), 16);
     };
     if (!from_fd) place_tables();
     hd.params_off = off;
@@ -1314,6 +1319,7 @@ int stage_impl(ffcvb_ctx *ctx, int slot, const Source &source, const uint64_t *p
     if (!s.slot_segs.empty()) memcpy(s.host + s.segs_off + sizeof(uint2) * segs.size(), s.slot_segs.data(), sizeof(uint2) * s.slot_segs.size());
     if (!blk_tiles.empty()) memcpy(s.host + s.block_tiles_off, blk_tiles.data(), sizeof(uint2) * blk_tiles.size());
     if (!quad_tiles.empty()) memcpy(s.host + s.quad_tiles_off, quad_tiles.data(), sizeof(uint2) * quad_tiles.size());
+    if (s.gather_ctas) gather_ranges(descs.data(), n, s.gather_ctas, reinterpret_cast<uint2 *>(s.host + s.gather_off));
     s.n_quad_tiles = (int)quad_tiles.size();
     s.n_block_tiles = (int)blk_tiles.size();
     work.n_guess = (int)segs.size();
@@ -1513,7 +1519,7 @@ static int run_batch(ffcvb_ctx *ctx, Slot &s, cudaStream_t st, void *out_dev, bo
         s.gather_timed = s.range_len == 0;
         if (s.gather_timed) {
             CU(cudaEventRecord(s.ev_gather_start, ctx->copy_stream));
-            launch_gather_payloads(reinterpret_cast<ImageDesc *>(blob + hd.desc_off), s.n, blob, ctx->gather_ctas,
+            launch_gather_payloads(reinterpret_cast<ImageDesc *>(blob + hd.desc_off), reinterpret_cast<const uint2 *>(blob + s.gather_off), s.gather_ctas, blob,
                                    reinterpret_cast<int32_t *>(blob + s.status_off), ctx->gather_limit_ns, ctx->gather_failed, ctx->copy_stream);
         } else {
             CU(cudaMemcpyAsync(blob + hd.payload_off, s.range_src, s.range_len, cudaMemcpyHostToDevice, ctx->copy_stream));

@@ -86,10 +86,10 @@ __device__ __forceinline__ void send(Ring &r, uint8_t *buf, uint64_t *bars, uint
     }
 }
 
-// The CTAs take the samples in turn, each split into `parts` when there are few.  One that gives up marks all of its
+// CTA k fetches what lies between ranges[k] and ranges[k + 1] (see gather_ranges).  One that gives up marks all of its
 // samples as failed, for the kernels that follow and in `status`.
 __global__ void __launch_bounds__(32)
-gather_payloads_kernel(ImageDesc *descs, int n, int parts, uint8_t *__restrict__ blob, int32_t *status, uint64_t limit,
+gather_payloads_kernel(ImageDesc *descs, const uint2 *__restrict__ ranges, uint8_t *__restrict__ blob, int32_t *status, uint64_t limit,
                        int32_t *failed) {
     __shared__ __align__(128) uint8_t s_buf[kStages * kPiece];
     __shared__ __align__(8) uint64_t s_bars[kStages];
@@ -98,37 +98,37 @@ gather_payloads_kernel(ImageDesc *descs, int n, int parts, uint8_t *__restrict__
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     __syncwarp();
-    const int items = n * parts, step = gridDim.x;
+    const uint2 from = ranges[blockIdx.x], to = ranges[blockIdx.x + 1];
+    const uint32_t behind = to.x + (to.y != 0 ? 1 : 0); // samples [from.x, behind) have bytes for this CTA
     Ring ring{};
     ring.limit = limit;
-    for (int first = blockIdx.x; first < items; first += 32 * step) {
-        // the descriptors of this CTA's next 32 items, one per lane
-        const int item = first + lane * step;
+    for (uint32_t first = from.x; first < behind; first += 32) {
+        // the descriptors of this CTA's next 32 samples, one per lane: rows, or one run
+        const uint32_t item = first + lane;
         uint64_t src = 0, dst = 0;
         uint32_t run = 0, rows = 0, src_pitch = 0, dst_pitch = 0;
-        if (item < items) {
-            const ImageDesc &d = descs[item / parts];
-            const uint32_t part = item % parts;
+        if (item < behind) {
+            const ImageDesc &d = descs[item];
+            const uint32_t begin = item == from.x ? from.y : 0, end = item == to.x ? to.y : 0xFFFFFFFFu;
             if (d.src_addr != 0 && d.payload_size != 0) {
                 if (d.mode == 1 && d.raw_skew) { // a crop box: rows, each as the aligned 16-byte words that hold it
-                    const uint32_t per = ((uint32_t)d.rows + parts - 1) / parts, r0 = part * per, r1 = min(r0 + per, (uint32_t)d.rows);
+                    const uint32_t last = min((uint32_t)d.rows, end);
                     src_pitch = (uint32_t)d.width * 3;
                     dst_pitch = d.raw_pitch;
                     run = (uint32_t)d.cols * 3;
-                    rows = r1 > r0 ? r1 - r0 : 0;
-                    src = d.src_addr + (uint64_t)r0 * src_pitch;
-                    dst = d.payload_off + (uint64_t)r0 * dst_pitch;
-                } else { // one run; source and destination have the same alignment
-                    const uint32_t lead = (uint32_t)(d.src_addr & 15), all = lead + d.payload_size;
-                    const uint32_t per = ((all + parts - 1) / parts + 15) & ~15u, b0 = part * per, b1 = min(b0 + per, all);
-                    rows = b1 > b0 ? 1 : 0;
-                    run = b1 - b0;
-                    src = d.src_addr - lead + b0;
-                    dst = d.payload_off - lead + b0;
+                    rows = last > begin ? last - begin : 0;
+                    src = d.src_addr + (uint64_t)begin * src_pitch;
+                    dst = d.payload_off + (uint64_t)begin * dst_pitch;
+                } else { // source and destination have the same alignment
+                    const uint32_t lead = (uint32_t)(d.src_addr & 15), last = min(lead + d.payload_size, end);
+                    rows = last > begin ? 1 : 0;
+                    run = last - begin;
+                    src = d.src_addr - lead + begin;
+                    dst = d.payload_off - lead + begin;
                 }
             }
         }
-        for (int k = 0; k < 32 && first + k * step < items; k++) {
+        for (uint32_t k = 0; k < 32 && first + k < behind; k++) {
             const uint64_t s = __shfl_sync(0xffffffffu, src, k), t = __shfl_sync(0xffffffffu, dst, k);
             const uint32_t len = __shfl_sync(0xffffffffu, run, k), m = __shfl_sync(0xffffffffu, rows, k);
             const uint32_t sp = __shfl_sync(0xffffffffu, src_pitch, k), dp = __shfl_sync(0xffffffffu, dst_pitch, k);
@@ -136,9 +136,9 @@ gather_payloads_kernel(ImageDesc *descs, int n, int parts, uint8_t *__restrict__
                 for (uint32_t r = 0; r < m && !ring.failed; r++) {
                     // (a word that holds one byte of the run lies in the same page as that byte: the reads stay
                     // inside the pinned allocation)
-                    const uint64_t from = s + (uint64_t)r * sp;
-                    const uint32_t lead = (uint32_t)(from & 15);
-                    send(ring, s_buf, s_bars, blob, from - lead, t + (uint64_t)r * dp, (lead + len + 15) & ~15u);
+                    const uint64_t at = s + (uint64_t)r * sp;
+                    const uint32_t lead = (uint32_t)(at & 15);
+                    send(ring, s_buf, s_bars, blob, at - lead, t + (uint64_t)r * dp, (lead + len + 15) & ~15u);
                 }
             __syncwarp();
         }
@@ -147,11 +147,11 @@ gather_payloads_kernel(ImageDesc *descs, int n, int parts, uint8_t *__restrict__
         while (ring.stored != ring.issued && !ring.failed) store_oldest(ring, s_buf, s_bars, blob);
         asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
         if (ring.failed) {
-            for (int item = blockIdx.x; item < items; item += step) {
-                ImageDesc &d = descs[item / parts];
+            for (uint32_t item = from.x; item < behind; item++) {
+                ImageDesc &d = descs[item];
                 if (d.src_addr == 0 || d.payload_size == 0) continue;
                 d.host_status = (int16_t)kErrData;
-                status[item / parts] = kErrData;
+                status[item] = kErrData;
             }
             *failed = 1;
             const uint64_t drain = max(limit, (uint64_t)2000000000ull); // (shared memory must outlive the copies into it)
@@ -162,12 +162,36 @@ gather_payloads_kernel(ImageDesc *descs, int n, int parts, uint8_t *__restrict__
 
 } // namespace
 
-void launch_gather_payloads(ImageDesc *descs, int n, uint8_t *blob, int ctas, int32_t *status, uint64_t limit_ns, int32_t *failed,
+void gather_ranges(const ImageDesc *descs, int n, int ctas, uint2 *ranges) {
+    auto rowwise = [](const ImageDesc &d) { return d.mode == 1 && d.raw_skew != 0; };
+    // of a row; and of a run, without the lines that its ends share with nothing
+    auto row_lines = [](const ImageDesc &d) { return ((uint64_t)d.cols * 3 + kLine - 1) / kLine + 1; };
+    auto run_lines = [](const ImageDesc &d) { return ((d.src_addr & (kLine - 1)) + d.payload_size + kLine - 1) / kLine; };
+    auto lines = [&](const ImageDesc &d) -> uint64_t {
+        if (d.src_addr == 0 || d.payload_size == 0) return 0;
+        return rowwise(d) ? d.rows * row_lines(d) : run_lines(d);
+    };
+    uint64_t total = 0, before = 0; // before sample i
+    for (int i = 0; i < n; i++) total += lines(descs[i]);
+    int i = 0;
+    for (int k = 0; k <= ctas; k++) {
+        const uint64_t want = total * (uint64_t)k / (uint64_t)ctas;
+        while (i < n && before + lines(descs[i]) <= want) before += lines(descs[i++]);
+        if (k == 0 || k == ctas || i == n) {
+            ranges[k] = make_uint2((uint32_t)(k == 0 ? 0 : n), 0);
+            continue;
+        }
+        const ImageDesc &d = descs[i];
+        const uint64_t inside = want - before; // lines of it that come before (fewer than it has)
+        const uint64_t lead = d.src_addr & (kLine - 1), words = d.src_addr & 15; // a run begins with the word of its first byte
+        const uint64_t at = rowwise(d) ? inside / row_lines(d) : (inside == 0 ? 0 : inside * kLine - lead + words);
+        ranges[k] = make_uint2((uint32_t)i, (uint32_t)at);
+    }
+}
+
+void launch_gather_payloads(ImageDesc *descs, const uint2 *ranges, int ctas, uint8_t *blob, int32_t *status, uint64_t limit_ns, int32_t *failed,
                             cudaStream_t stream) {
-    if (n <= 0) return;
-    if (ctas < 1) ctas = kGatherCtas;
-    const int parts = n >= 4 * ctas ? 1 : (4 * ctas + n - 1) / n;
-    gather_payloads_kernel<<<ctas, 32, 0, stream>>>(descs, n, parts, blob, status, limit_ns, failed);
+    gather_payloads_kernel<<<ctas, 32, 0, stream>>>(descs, ranges, blob, status, limit_ns, failed);
 }
 
 } // namespace ffcvb

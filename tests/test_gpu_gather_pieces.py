@@ -57,3 +57,28 @@ def test_streams_of_every_alignment():
     modes = np.zeros(n, np.uint8)
     want, _ = O.run_batch(payloads, modes, hs, ws, params, True, out_size, out_size, [[] for _ in range(n)], None, L.OUT_U8_NHWC, 2)
     assert np.array_equal(gathered(payloads, modes, hs, ws, params, out_size, out_size), want)
+
+
+@pytest.mark.parametrize('ctas', [1, 7, 148, 1024])
+@pytest.mark.parametrize('n', [1, 3, 40])
+def test_samples_shared_out_to_any_number_of_ctas(ctas, n, monkeypatch):
+    """More CTAs than lines, one CTA for all, shares that begin and end inside rows' and streams' samples, samples of
+    less than a line among large ones."""
+    monkeypatch.setenv('FFCV_B200_GATHER_CTAS', str(ctas))
+    rng = np.random.default_rng(100 * ctas + n)
+    payloads, modes, hs, ws, params, wants = [], [], [], [], [], []
+    for k in range(n):
+        h, w = (2, 3) if k % 4 == 0 and n > 1 else (int(v) for v in rng.integers(20, 260, 2))
+        img = synth_content(rng, h, w)
+        raw = k % 3 != 1
+        payloads.append(img.reshape(-1) if raw else cv2.imencode('.jpg', img[..., ::-1], [cv2.IMWRITE_JPEG_QUALITY, 95])[1].reshape(-1).copy())
+        ch_, cw_ = int(rng.integers(1, h + 1)), int(rng.integers(1, w + 1))
+        r0, c0 = int(rng.integers(0, h - ch_ + 1)), int(rng.integers(0, w - cw_ + 1))
+        modes.append(int(raw))
+        hs.append(h)
+        ws.append(w)
+        params.append((r0, c0, ch_, cw_))
+        pixels = img if raw else O.jpeg_decode(payloads[-1])
+        wants.append(O.resize_area(pixels, r0, r0 + ch_, c0, c0 + cw_, 24, 24))
+    got = gathered(payloads, np.array(modes, np.uint8), np.array(hs, np.uint16), np.array(ws, np.uint16), np.array(params, np.int32), 24, 24)
+    assert np.array_equal(got, np.stack(wants))
