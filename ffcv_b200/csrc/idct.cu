@@ -57,7 +57,7 @@ __device__ __forceinline__ void idct8(int &v0, int &v1, int &v2, int &v3, int &v
 // 1.5 * 2^23 is the shifted one.  `peak` gathers the largest of those values.  Up to kPeak the result is exact (the sum
 // of z10 and z12 is then below 2^15 as well); beyond it, which the streams of encoders do not reach, the integer
 // transform below has to be taken.  Kernel on 1024 photographs to 160x160, 256x256, 64 of 4:4:4 to 384x384: 110, 145 and
-// 596 us in integers, 98, 133 and 549 this way, 94, 124 and 500 with six CTAs per SM instead of five.
+// 596 us in integers, 98, 133 and 549 this way.
 constexpr float kPeak = 16383.f;
 constexpr float kOnes = 12582912.f; // 1.5 * 2^23: what is added to it leaves as an integer
 __device__ __forceinline__ Two both(float v) { return Two(v, v); }
@@ -197,8 +197,11 @@ constexpr uint32_t kCoefZero = 0x80008000u; // coefficients wait for the transfo
 // A warp takes blocks of one component that are neighbours in the plane: their symbol counts are
 // alike, their bits are near one another and their rows leave as one run.
 // Bound by instruction issue (61 % of the cycles) and the arithmetic pipe (53 %): about 30 instructions per symbol, of
-// which a warp's longest block has some 28.
-__global__ void __launch_bounds__(kBlockTile, 6)
+// which a warp's longest block has some 28.  CTAS: as many per SM, by its registers.  Eight (64 registers, 40 words of the
+// transform in local memory) where there are tiles for them; 4:4:4 images 500 us with six, 473 with seven, 461 with eight,
+// 1024 photographs to 256x256 123, 119, 119.  Few tiles are done sooner without the detour.
+template <int CTAS>
+__global__ void __launch_bounds__(kBlockTile, CTAS)
 blocks_kernel(const ImageDesc *__restrict__ descs, const uint2 *__restrict__ tiles, const HuffTable *__restrict__ huff,
               const MultTable *__restrict__ mult, EntropyScratch scratch, uint8_t *__restrict__ planes) {
     constexpr int kLook = 1 << kHuffBits;
@@ -333,7 +336,9 @@ blocks_kernel(const ImageDesc *__restrict__ descs, const uint2 *__restrict__ til
 
 void launch_blocks(const ImageDesc *descs, const uint2 *tiles, int n_tiles, const HuffTable *huff, const MultTable *mult,
                    const EntropyScratch &scratch, uint8_t *planes, bool early, cudaStream_t stream) {
-    if (n_tiles > 0) launch(early, n_tiles, kBlockTile, 0, stream, blocks_kernel, descs, tiles, huff, mult, scratch, planes);
+    auto run = [&](auto kernel) { launch(early, n_tiles, kBlockTile, 0, stream, kernel, descs, tiles, huff, mult, scratch, planes); };
+    if (n_tiles >= 148 * 8) run(blocks_kernel<8>);
+    else if (n_tiles > 0) run(blocks_kernel<5>);
 }
 
 // ------------------------------------------------------------------------------------------

@@ -240,9 +240,12 @@ struct alignas(16) ResizeItem {
     int32_t groups;      // runs of rows that a band is dealt out in
 };
 // Makes them, and the CTAs per image of the kernel below: as many as the image with the most bands has, at most enough of
-// them for about eight waves of the GPU (148 SMs x 4 resident CTAs; fewer waves measured slower, more cost the set-up
-// its amortisation).  Worth a look at every box: a CTA without a band costs as much set-up as
-// one with (512 images of 32x32 pixels to 24x24: 21 us, 36 with a CTA for every four rows; 256 of 192x192 to 96x96: 39 and 60).
+// them for about four waves of the GPU (148 SMs x 4 resident CTAs) when all bands have windows, eight otherwise.  More waves cost
+// the set-up its amortisation, fewer leave the last one emptier.  1024 images to 160x160 / 256x256, 256 to 192x192, alone
+// (and all kernels as one of four in flight): 187 (369), 289 (506), 101 us (209) with eight, 183 (352), 281 (486), 103 (201)
+// with four, 187 (347), 281 (482), 109 (199) with three; 64 to 384x384 without windows 268 with eight, 285 with five.  Worth a
+// look at every box: a CTA without a band costs as much set-up as one with (512 images of 32x32 pixels to 24x24: 21 us,
+// 36 with a CTA for every four rows; 256 of 192x192 to 96x96: 39 and 60).
 class ResizeItems {
   public:
     ResizeItems(int n, int out_h, int out_w, int out_kind);
@@ -252,12 +255,14 @@ class ResizeItems {
     ResizeItem make(const int32_t *box, int img_h, int img_w, Fuse fuse);
     int bands() const { // (none made: without a window)
         const int bands = bands_ ? bands_ : (out_h_ + shape_.band - 1) / shape_.band;
-        return bands < most_ ? bands : most_;
+        const int most = windowed_ && bands_ ? most_windowed_ : most_;
+        return bands < most ? bands : most;
     }
 
   private:
     int groups(int band);
-    int out_h_, out_w_, bands_ = 0, most_;
+    int out_h_, out_w_, bands_ = 0, most_, most_windowed_;
+    bool windowed_ = true; // every band so far
     size_t tile_row_;
     ResizeShape shape_;
     std::vector<uint8_t> groups_; // by rows of a band, 0: not worked out

@@ -689,8 +689,10 @@ ResizeShape resize_shape(int n, int out_h, int out_w, int out_kind) {
     return s;
 }
 
+constexpr int kWaves = 8, kWindowedWaves = 4;
+
 ResizeItems::ResizeItems(int n, int out_h, int out_w, int out_kind)
-    : out_h_(out_h), out_w_(out_w), most_((8 * 148 * 4 + n - 1) / n), tile_row_((size_t)out_w * 3 * value_size(out_kind)),
+    : out_h_(out_h), out_w_(out_w), most_((kWaves * 148 * 4 + n - 1) / n), most_windowed_((kWindowedWaves * 148 * 4 + n - 1) / n), tile_row_((size_t)out_w * 3 * value_size(out_kind)),
       shape_(resize_shape(n, out_h, out_w, out_kind)), groups_((shape_.band > shape_.max_band ? shape_.band : shape_.max_band) + 1, 0) {}
 
 // The column paths deal a band's rows to this many runs per pair of columns, so that the (pair, run) items fill the
@@ -729,6 +731,7 @@ ResizeItem ResizeItems::make(const int32_t *box, int img_h, int img_w, Fuse fuse
     const int band = item.window ? item.window : shape_.band, bands = (out_h_ + band - 1) / band;
     item.groups = groups(band);
     if (bands > bands_) bands_ = bands;
+    windowed_ = windowed_ && item.window != 0;
     return item;
 }
 
