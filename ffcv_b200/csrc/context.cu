@@ -1298,12 +1298,14 @@ int stage_impl(ffcvb_ctx *ctx, int slot, const Source &source, const uint64_t *p
     if ((rc = grow_dev(ctx, s.rgb, rgb_bytes + 64))) return rc;
 
     memcpy(s.host, &hd, sizeof(hd));
-    memcpy(s.host + hd.desc_off, descs.data(), sizeof(ImageDesc) * (size_t)n);
+    // (past the caches: the lines were last read by a transfer, and the next one finds them in memory)
+    auto place = [&](uint64_t off, const void *src, size_t bytes) { stream_copy(s.host + off, static_cast<const uint8_t *>(src), bytes); };
+    place(hd.desc_off, descs.data(), sizeof(ImageDesc) * (size_t)n);
     for (size_t k = 0; k < huff_src.size(); k++)
         memcpy(s.host + hd.huff_off + k * sizeof(HuffTable), &ctx->tables.built(huff_src[k]), sizeof(HuffTable));
     for (size_t k = 0; k < mult_src.size(); k++)
         build_mult_table(ctx->tables.quant(mult_src[k]), reinterpret_cast<MultTable *>(s.host + hd.mult_off) + k);
-    memcpy(s.host + hd.params_off, params, sizeof(int32_t) * (size_t)n * n_params);
+    place(hd.params_off, params, sizeof(int32_t) * (size_t)n * n_params);
     {
         int32_t *st = reinterpret_cast<int32_t *>(s.host + s.status_off);
         for (int i = 0; i < n; i++) {
@@ -1317,7 +1319,7 @@ int stage_impl(ffcvb_ctx *ctx, int slot, const Source &source, const uint64_t *p
         if (descs[i].scale_shift == 0 || !plan->resize) continue;
         scaled_box(descs[i], reinterpret_cast<int32_t *>(s.host + hd.params_off) + (size_t)i * n_params);
     }
-    if (!s.items.empty()) memcpy(s.host + s.items_off, s.items.data(), sizeof(ResizeItem) * s.items.size());
+    if (!s.items.empty()) place(s.items_off, s.items.data(), sizeof(ResizeItem) * s.items.size());
     s.bands = items.bands();
     for (const auto &r : s.riders) {
         if (!r.inline_bytes.empty()) {
@@ -1343,14 +1345,14 @@ int stage_impl(ffcvb_ctx *ctx, int slot, const Source &source, const uint64_t *p
         }
     }
     if (!jpeg_list.empty()) memcpy(s.host + s.jpeg_list_off, jpeg_list.data(), 4 * jpeg_list.size());
-    if (!s.parts.empty()) memcpy(s.host + s.parts_off, s.parts.data(), sizeof(uint4) * s.parts.size());
+    if (!s.parts.empty()) place(s.parts_off, s.parts.data(), sizeof(uint4) * s.parts.size());
     if (!s.wholes.empty()) memcpy(s.host + s.parts_off + sizeof(uint4) * s.parts.size(), s.wholes.data(), sizeof(uint4) * s.wholes.size());
     if (!slot_images.empty()) memcpy(s.host + s.slot_images_off, slot_images.data(), 4 * slot_images.size());
     if (!restart.empty()) memcpy(s.host + s.restart_off, restart.data(), 4 * restart.size());
-    if (!segs.empty()) memcpy(s.host + s.segs_off, segs.data(), sizeof(uint2) * segs.size());
+    if (!segs.empty()) place(s.segs_off, segs.data(), sizeof(uint2) * segs.size());
     if (!s.slot_segs.empty()) memcpy(s.host + s.segs_off + sizeof(uint2) * segs.size(), s.slot_segs.data(), sizeof(uint2) * s.slot_segs.size());
-    if (!blk_tiles.empty()) memcpy(s.host + s.block_tiles_off, blk_tiles.data(), sizeof(uint2) * blk_tiles.size());
-    if (!quad_tiles.empty()) memcpy(s.host + s.quad_tiles_off, quad_tiles.data(), sizeof(uint2) * quad_tiles.size());
+    if (!blk_tiles.empty()) place(s.block_tiles_off, blk_tiles.data(), sizeof(uint2) * blk_tiles.size());
+    if (!quad_tiles.empty()) place(s.quad_tiles_off, quad_tiles.data(), sizeof(uint2) * quad_tiles.size());
     if (s.gather_ctas) gather_ranges(descs.data(), n, s.gather_ctas, reinterpret_cast<uint2 *>(s.host + s.gather_off));
     s.n_quad_tiles = (int)quad_tiles.size();
     s.n_block_tiles = (int)blk_tiles.size();
@@ -1360,6 +1362,7 @@ int stage_impl(ffcvb_ctx *ctx, int slot, const Source &source, const uint64_t *p
     work.n_whole = (int)s.wholes.size();
     work.n_slot_images = (int)slot_images.size();
     work.n_restart = (int)restart.size();
+    _mm_sfence();
 
     const auto t2 = std::chrono::steady_clock::now();
     // ---- parallel: gather the payload bytes into pinned memory

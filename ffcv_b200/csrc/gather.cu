@@ -171,12 +171,13 @@ void gather_ranges(const ImageDesc *descs, int n, int ctas, uint2 *ranges) {
         if (d.src_addr == 0 || d.payload_size == 0) return 0;
         return rowwise(d) ? d.rows * row_lines(d) : run_lines(d);
     };
+    std::vector<uint32_t> of(n);
     uint64_t total = 0, before = 0; // before sample i
-    for (int i = 0; i < n; i++) total += lines(descs[i]);
+    for (int i = 0; i < n; i++) total += of[i] = (uint32_t)lines(descs[i]);
     int i = 0;
     for (int k = 0; k <= ctas; k++) {
         const uint64_t want = total * (uint64_t)k / (uint64_t)ctas;
-        while (i < n && before + lines(descs[i]) <= want) before += lines(descs[i++]);
+        while (i < n && before + of[i] <= want) before += of[i++];
         if (k == 0 || k == ctas || i == n) {
             ranges[k] = make_uint2((uint32_t)(k == 0 ? 0 : n), 0);
             continue;

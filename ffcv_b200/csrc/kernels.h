@@ -3,6 +3,7 @@
 #include <float.h>
 #include <math.h>
 #include <cuda_runtime.h>
+#include <emmintrin.h>
 #include <stdint.h>
 
 #include <vector>
@@ -159,6 +160,13 @@ struct Scaling {
     int regime, isx, isy;
     double inv_x, inv_y, sc_x, sc_y;
 };
+FFCVB_HD inline int nearest(double v) { // (ties to even)
+#if defined(__CUDA_ARCH__)
+    return __double2int_rn(v);
+#else
+    return _mm_cvtsd_si32(_mm_set_sd(v)); // (rint is a call)
+#endif
+}
 FFCVB_HD inline Scaling scaling_of(int ch, int cw, int out_h, int out_w) {
     Scaling s{kCopy, 1, 1, 1, 1, 1, 1};
     if (ch != out_h || cw != out_w) {
@@ -167,8 +175,8 @@ FFCVB_HD inline Scaling scaling_of(int ch, int cw, int out_h, int out_w) {
         s.sc_x = 1.0 / s.inv_x;
         s.sc_y = 1.0 / s.inv_y;
         if (s.sc_x >= 1 && s.sc_y >= 1) {
-            s.isx = (int)rint(s.sc_x);
-            s.isy = (int)rint(s.sc_y);
+            s.isx = nearest(s.sc_x);
+            s.isy = nearest(s.sc_y);
             s.regime = (fabs(s.sc_x - s.isx) < DBL_EPSILON && fabs(s.sc_y - s.isy) < DBL_EPSILON) ? kInteger : kArea;
         } else {
             s.regime = kLinear;

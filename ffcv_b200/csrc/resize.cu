@@ -204,7 +204,7 @@ __device__ __forceinline__ uint32_t blended(float upper, float lower) { return (
 
 // a / n for a, n < 2^16, inv_n = ceil(2^32 / n)
 __device__ __forceinline__ int divided(uint32_t a, uint32_t inv_n, int n) { return n == 1 ? (int)a : (int)__umulhi(a, inv_n); }
-__host__ __device__ __forceinline__ uint32_t inverse(int n) { return (uint32_t)((0x100000000ull + n - 1) / n); }
+__host__ __device__ __forceinline__ uint32_t inverse(int n) { return 0xFFFFFFFFu / (uint32_t)n + 1u; }
 
 // One of SmallCopies, by a CTA of 256 threads: every thread has its words (at most kSmallCopyWords / 256) under way
 // at once.
