@@ -1291,7 +1291,8 @@ int stage_impl(ffcvb_ctx *ctx, int slot, const Source &source, const uint64_t *p
     if ((rc = grow_dev(ctx, s.blob, off + 64))) return rc;
     if ((rc = grow_dev(ctx, s.clean, clean_bytes + 512))) return rc;
     if ((rc = grow_dev(ctx, s.segs, seg_total * kSegScratch + 64))) return rc;
-    if ((rc = grow_dev(ctx, s.records, segs.empty() ? 0 : (size_t)seg_total * kSegSubs * kRecords * sizeof(uint16_t)))) return rc;
+    // (where there is no room for them the index kernel decodes once more)
+    if (grow_dev(ctx, s.records, segs.empty() ? 0 : (size_t)seg_total * kSegSubs * kRecords * sizeof(uint16_t)) != FFCVB_OK) cudaGetLastError();
     if (!s.slot_segs.empty() && (rc = grow_dev(ctx, s.slot_tables, s.slot_segs.size() * sizeof(SlotTables)))) return rc;
     if ((rc = grow_dev(ctx, s.index, (size_t)total_blocks * 6 + 64))) return rc;
     if ((rc = grow_dev(ctx, s.planes, plane_bytes + 64))) return rc;
