@@ -1099,13 +1099,14 @@ int stage_impl(ffcvb_ctx *ctx, int slot, const Source &source, const uint64_t *p
             restart.push_back(i);
         } else {
             const bool slots = few && d.bpm > 3; // (a guess among three slots falls in step within 1.4 kbit)
-            const ScanLayout l = slots ? layout_scan_slots(d.scan_len) : layout_scan(d.scan_len, target_bits, d.bpm, work.local_repair);
+            const ScanLayout l = slots ? layout_scan_slots(d.scan_len) : layout_scan(d.scan_len, target_bits, d.bpm, work.local_repair, ctx->index_pool.p != nullptr);
             d.subseq_bits = l.subseq_bits;
             d.seg_raw = l.seg_raw;
             d.seg_warm = l.seg_warm;
             d.seg_run_up = l.seg_run_up;
             d.seg_stride = l.seg_stride;
             d.seg_count = l.seg_count;
+            d.seg_lanes = l.seg_lanes;
             d.seg_first = seg_total;
             seg_total += l.seg_count;
             clean_bytes += (size_t)l.seg_count * l.seg_stride;
@@ -1123,7 +1124,7 @@ int stage_impl(ffcvb_ctx *ctx, int slot, const Source &source, const uint64_t *p
             const uint32_t raw = l.seg_stride - 64 - 16; // (at least run-up, own bytes and overlap)
             if (raw > work.max_raw) work.max_raw = raw;
             if (ctx->index_pool.p) {
-                const DecodeIndex::Place place = ctx->index.take(ptrs[i], l.seg_count, decode_index_bytes(l.seg_count), slot);
+                const DecodeIndex::Place place = ctx->index.take(ptrs[i], l.seg_count, decode_index_bytes(l.seg_count, l.seg_lanes), slot);
                 d.index_off = place.off;
                 d.index_use = place.use;
             }

@@ -480,7 +480,7 @@ scan_guess_kernel(const ImageDesc *__restrict__ descs, const uint2 *__restrict__
     if (index_pool != nullptr && d.index_use != 0) {
         const DecodeIndexHeader *h = reinterpret_cast<const DecodeIndexHeader *>(index_pool + d.index_off);
         if (index_entry_valid(h, d)) {
-            known = reinterpret_cast<const uint32_t *>(h + 1) + (size_t)j * kSegSubs;
+            known = reinterpret_cast<const uint32_t *>(h + 1) + (size_t)j * d.seg_lanes;
             if (tid == 0 && j == 0 && index_stats) atomicAdd(index_stats, 1ull);
         }
     }
@@ -525,10 +525,10 @@ scan_guess_kernel(const ImageDesc *__restrict__ descs, const uint2 *__restrict__
     }
     int total;
     team_scan(team, own ? (int)done : 0, sh.warp, total);
-    // (whether a segment's first one begins where the segment before ends is not known here)
+    // (whether a segment's first one begins where the segment before ends is not known here, unless its entry says so)
     if ((tid & 31) == 0) {
         // (with local_repair none is left; otherwise lead is 0)
-        scratch.meta[seg].doubt[tid >> 5] = (local_repair ? 0 : differ) | (tid == 0 && j > 0 && n_own > 0 ? 1 : 0);
+        scratch.meta[seg].doubt[tid >> 5] = (local_repair ? 0 : differ) | (tid == 0 && j > 0 && n_own > 0 && !known ? 1 : 0);
     }
     if (tid == 0) {
         SegMeta &m = scratch.meta[seg];
@@ -1105,8 +1105,8 @@ scan_index_kernel(const ImageDesc *__restrict__ descs, const uint2 *__restrict__
     const bool record = index_pool != nullptr && (d.index_use & 2) != 0 && d.host_status == 0 &&
                         !index_entry_valid(reinterpret_cast<const DecodeIndexHeader *>(index_pool + d.index_off), d);
     if (record) {
-        uint32_t *dst = reinterpret_cast<uint32_t *>(index_pool + d.index_off + sizeof(DecodeIndexHeader)) + (size_t)j * kSegSubs;
-        dst[tid] = info;
+        uint32_t *dst = reinterpret_cast<uint32_t *>(index_pool + d.index_off + sizeof(DecodeIndexHeader)) + (size_t)j * d.seg_lanes;
+        if (tid < (int)d.seg_lanes) dst[tid] = info;
     }
     // ---- the CTA that finishes an image last turns the segments' DC sums into sums before them
     __threadfence();
@@ -1277,7 +1277,7 @@ uint32_t subseq_target(uint64_t total_bits) {
     return (uint32_t)(t < 256 ? 256 : (t > kMaxSubseqBits ? kMaxSubseqBits : (t + 31) / 32 * 32));
 }
 
-ScanLayout layout_scan(uint32_t scan_len, uint32_t target_bits, int bpm, bool local_repair) {
+ScanLayout layout_scan(uint32_t scan_len, uint32_t target_bits, int bpm, bool local_repair, bool indexed) {
     ScanLayout l{};
     const uint64_t bits = (uint64_t)scan_len * 8, target = target_bits;
     auto up = [](uint64_t a, uint64_t b) { return (a + b - 1) / b; };
@@ -1292,7 +1292,7 @@ ScanLayout layout_scan(uint32_t scan_len, uint32_t target_bits, int bpm, bool lo
             l.seg_count = (uint32_t)up(bits, own * target);
         }
     } else { // two warps at most (128 of them share the SM's memory out worse: 64 images of 14 Mbit 696 us instead of 653)
-        own = 64;
+        own = indexed ? kSegSubs : 64;
         l.seg_count = (uint32_t)up(bits, own * target);
         if (l.seg_count < 1) l.seg_count = 1;
         own = 32 * up(bits, 32 * target * l.seg_count);
@@ -1301,6 +1301,7 @@ ScanLayout layout_scan(uint32_t scan_len, uint32_t target_bits, int bpm, bool lo
     l.subseq_bits = (uint32_t)up(up(bits, own * l.seg_count), 32) * 32;
     if (l.subseq_bits < 128) l.subseq_bits = 128;
     l.seg_raw = (uint32_t)own * l.subseq_bits / 8;
+    l.seg_lanes = (uint32_t)own;
     l.seg_count = scan_len ? (scan_len + l.seg_raw - 1) / l.seg_raw : 1;
     l.seg_stride = (((uint32_t)own + l.seg_warm) * l.subseq_bits + l.seg_run_up) / 8 + kSegOverlap + 64 + 31;
     l.seg_stride = l.seg_stride / 16 * 16;
@@ -1318,6 +1319,7 @@ ScanLayout layout_scan_slots(uint32_t scan_len) {
     if (l.subseq_bits < 384) l.subseq_bits = 384;
     l.seg_warm = kSlotRunUp;
     l.seg_raw = kSlotSubs * l.subseq_bits / 8;
+    l.seg_lanes = kSlotSubs;
     l.seg_count = scan_len ? (scan_len + l.seg_raw - 1) / l.seg_raw : 1;
     l.seg_stride = ((kSlotSubs + kSlotRunUp) * l.subseq_bits / 8 + kSegOverlap + 64 + 31) / 16 * 16;
     return l;

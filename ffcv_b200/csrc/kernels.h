@@ -95,11 +95,11 @@ void launch_entropy_decode(const ImageDesc *descs, const EntropyWork &work, cons
                            cudaStream_t stream);
 
 // How a scan of scan_len bytes is cut into subsequences and segments.  `target_bits`: wished length of
-// a subsequence, see subseq_target; bpm: blocks of an MCU.
+// a subsequence, see subseq_target; bpm: blocks of an MCU; indexed: with a decode index.
 struct ScanLayout {
-    uint32_t subseq_bits, seg_raw, seg_warm, seg_run_up, seg_stride, seg_count;
+    uint32_t subseq_bits, seg_raw, seg_warm, seg_run_up, seg_stride, seg_count, seg_lanes;
 };
-ScanLayout layout_scan(uint32_t scan_len, uint32_t target_bits, int bpm, bool local_repair);
+ScanLayout layout_scan(uint32_t scan_len, uint32_t target_bits, int bpm, bool local_repair, bool indexed);
 // Where a batch leaves SMs idle, subsequences that began in the wrong state are decoded again at once, by the threads that have
 // their segment's bytes: a shorter way than scan_repair_kernel, but a segment keeps its shared memory until the last one
 // is right.  So too for a single image, beside which nothing runs.  One of 24 Mbit (4:4:4) / 33 Mbit (4:2:0), all kernels of

@@ -151,13 +151,14 @@ extern "C" int ffcvb_imdecode_static(const uint8_t *jpeg_host, uint64_t jpeg_siz
 
     int n_segs = 0;
     if (!d.restart_interval) {
-        const ScanLayout l = layout_scan(d.scan_len, kSubseqTarget, d.bpm, true);
+        const ScanLayout l = layout_scan(d.scan_len, kSubseqTarget, d.bpm, true, false);
         d.subseq_bits = l.subseq_bits;
         d.seg_raw = l.seg_raw;
         d.seg_warm = l.seg_warm;
         d.seg_run_up = l.seg_run_up;
         d.seg_stride = l.seg_stride;
         d.seg_count = l.seg_count;
+        d.seg_lanes = l.seg_lanes;
         n_segs = (int)l.seg_count;
         if (l.seg_count > kMaxSegments || (size_t)l.seg_count * l.seg_stride + 512 > kCleanBytes)
             return reject(FFCVB_E_LIMIT, "JPEG stream too large for the static scratch");

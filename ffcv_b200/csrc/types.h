@@ -71,8 +71,8 @@ struct ImageDesc {
     // Entropy decode in segments (scans without restart markers): length in bits of the
     // subsequences (multiple of 32); raw bytes of a segment; subsequences of run-up before every
     // segment but the first; bits of run-up before every subsequence (a multiple of 32); bytes of a segment's place in the unstuffed stream; and which of the
-    // batch's segments are this image's.
-    uint32_t subseq_bits, seg_raw, seg_warm, seg_run_up, seg_stride, seg_first, seg_count;
+    // batch's segments are this image's; and how many subsequences of its own a segment has at most.
+    uint32_t subseq_bits, seg_raw, seg_warm, seg_run_up, seg_stride, seg_first, seg_count, seg_lanes;
     uint32_t slots;        // decoded from every slot at once: 1 + the first of the image's SlotTables (0: not)
     uint32_t index_use;    // place in the decode index: 0 none, bit 0 the entry may be read, bit 1 and is written
     uint64_t index_off;    // byte offset of the entry in the context's index pool
@@ -175,15 +175,15 @@ constexpr uint32_t kNoBlock = 0xFFFFFFFFu; // position of a block that the scan 
 // Decode index: what a finished decode of a stream knows and the next decode of the same stream can
 // start from -- the exact decoder state at the start of every subsequence and the number of blocks
 // completed in it.  With it no guess has to be repaired.  An entry lives in device memory:
-//   [DecodeIndexHeader][per segment: uint32 sub_info x kSegSubs]
+//   [DecodeIndexHeader][per segment: uint32 sub_info x ImageDesc::seg_lanes]
 // and is valid when `magic` is set (written last) and the other fields match.  Which batch writes it and which
 // may read it is settled on the host (DecodeIndex).
 struct DecodeIndexHeader {
     uint32_t magic, scan_len, subseq_bits, segments;
 };
 constexpr uint32_t kDecodeIndexMagic = 0x58444947u;
-FFCVB_HD inline size_t decode_index_bytes(uint32_t segments) {
-    return (sizeof(DecodeIndexHeader) + (size_t)segments * kSegSubs * 4 + 15) / 16 * 16;
+FFCVB_HD inline size_t decode_index_bytes(uint32_t segments, uint32_t lanes) {
+    return (sizeof(DecodeIndexHeader) + (size_t)segments * lanes * 4 + 15) / 16 * 16;
 }
 
 struct BatchHeader {

@@ -12,9 +12,9 @@ pytestmark = pytest.mark.gpu
 
 
 class _Job:
-    def __init__(self, n, h, w):
+    def __init__(self, n, h, w, bufs=None):
         rng = np.random.default_rng(n)
-        bufs = [cv2.imencode('.jpg', synth_content(rng, h, w), [cv2.IMWRITE_JPEG_QUALITY, 90])[1].reshape(-1) for _ in range(n)]
+        bufs = bufs or [cv2.imencode('.jpg', synth_content(rng, h, w), [cv2.IMWRITE_JPEG_QUALITY, 90])[1].reshape(-1) for _ in range(n)]
         self.want = np.stack([O.jpeg_decode(b) for b in bufs])
         sizes = np.array([b.size for b in bufs], np.uint64)
         self.args = (np.concatenate(bufs), np.concatenate([[0], np.cumsum(sizes)[:-1]]).astype(np.uint64), sizes, np.zeros(n, np.uint8),
@@ -80,4 +80,25 @@ def test_a_batch_staged_before_the_index_was_set_up_again_leaves_it_alone():
         ch.cuda.synchronize()
         assert np.array_equal(out.cpu().numpy(), job.want)
         assert ctx.decode_index_stats()['used'] == use
+    ctx.close()
+
+
+@pytest.mark.parametrize('subseq_bits', ['', '128', '2560'])
+def test_an_entry_takes_four_bytes_per_subsequence(subseq_bits, monkeypatch):
+    """Large streams, whose segments are full but for the last one: a word per subsequence of 1024 bits (or of as many
+    as are asked for), a header of 16 bytes and, at most, a segment of 128 words that is nearly empty."""
+    monkeypatch.setenv('FFCV_B200_SUBSEQ_BITS', subseq_bits)
+    rng = np.random.default_rng(0)
+    bufs = [cv2.imencode('.jpg', synth_content(rng, 700, 900), [cv2.IMWRITE_JPEG_QUALITY, q])[1].reshape(-1) for q in (60, 85, 97)]
+    bits, n = sum(8 * b.size for b in bufs), len(bufs)
+    job = _Job(n, 700, 900, bufs)
+    ctx, stream = L.Context(0, 1, 2), ch.cuda.Stream()
+    ctx.set_decode_index(1 << 24)
+    for _ in range(3):
+        out = job.queue(ctx, 0, stream)
+        stream.synchronize()
+        assert np.array_equal(out.cpu().numpy(), job.want)
+    stats = ctx.decode_index_stats()
+    assert (stats['used'], stats['recorded'], stats['entries']) == (2 * n, n, n)
+    assert stats['bytes'] <= 4 * bits / int(subseq_bits or 1024) * 33 / 32 + n * (16 + 4 * 128)  # (lengths are multiples of 32 bits)
     ctx.close()
