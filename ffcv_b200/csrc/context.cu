@@ -1001,6 +1001,7 @@ int stage_impl(ffcvb_ctx *ctx, int slot, const Source &source, const uint64_t *p
     // Subsequence length: by the batch's bits, or, with a decode index, a function of the stream alone
     // (1024 bits), so that the recorded states stay usable whatever batch the sample lands in.
     uint32_t target_bits = 1024, seg_total = 0;
+    uint64_t records = 0; // room for them, / 4
     bool few = false; // few enough bits to decode from every slot at once
     if (!ctx->index_pool.p) {
         uint64_t bits = 0;
@@ -1119,6 +1120,9 @@ int stage_impl(ffcvb_ctx *ctx, int slot, const Source &source, const uint64_t *p
                 for (uint32_t k = 0; k < parts; k++) s.parts.push_back(repair_part((uint32_t)i, l.seg_count, parts, k));
                 if (parts > 1) s.wholes.push_back(make_uint4((uint32_t)i, 0, l.seg_count, 0));
                 if (l.subseq_bits > work.max_subseq_bits) work.max_subseq_bits = l.subseq_bits;
+                d.rec_room = record_room(l.subseq_bits, d.scan_len, (uint32_t)d.bpm * d.mcus_x * d.mcus_y);
+                d.rec_first = (uint32_t)records;
+                records += (uint64_t)l.seg_count * l.seg_lanes * d.rec_room / 4;
             }
             for (uint32_t k = 0; k < l.seg_count; k++) (slots ? s.slot_segs : segs).push_back(make_uint2((uint32_t)i, k));
             const uint32_t raw = l.seg_stride - 64 - 16; // (at least run-up, own bytes and overlap)
@@ -1293,7 +1297,7 @@ int stage_impl(ffcvb_ctx *ctx, int slot, const Source &source, const uint64_t *p
     if ((rc = grow_dev(ctx, s.clean, clean_bytes + 512))) return rc;
     if ((rc = grow_dev(ctx, s.segs, seg_total * kSegScratch + 64))) return rc;
     // (where there is no room for them the index kernel decodes once more)
-    if (grow_dev(ctx, s.records, segs.empty() ? 0 : (size_t)seg_total * kSegSubs * kRecords * sizeof(uint16_t)) != FFCVB_OK) cudaGetLastError();
+    if (grow_dev(ctx, s.records, (size_t)records * 4 * sizeof(uint16_t)) != FFCVB_OK) cudaGetLastError();
     if (!s.slot_segs.empty() && (rc = grow_dev(ctx, s.slot_tables, s.slot_segs.size() * sizeof(SlotTables)))) return rc;
     if ((rc = grow_dev(ctx, s.index, (size_t)total_blocks * 6 + 64))) return rc;
     if ((rc = grow_dev(ctx, s.planes, plane_bytes + 64))) return rc;

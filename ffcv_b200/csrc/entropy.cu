@@ -162,7 +162,7 @@ __device__ __noinline__ uint32_t walk_plain(const uint32_t *words, Cursor &cur, 
             blk++;
         }
         if (RECORD == kRecord && cur.z == 0) {
-            if (n < kRecords - 1) rec[n] = (uint16_t)(cur.p + blk);
+            if (n < limit - 1) rec[n] = (uint16_t)(cur.p + blk);
             n++;
         }
         const uint32_t w = __funnelshift_l(words[(cur.p >> 5) + 1], words[cur.p >> 5], cur.p);
@@ -185,7 +185,7 @@ __device__ __noinline__ uint32_t walk_plain(const uint32_t *words, Cursor &cur, 
 // completed.  `buf`: the segment's stream (words most significant bit first) in shared memory, or, with GLOBAL, in
 // global memory.  With kPositions every block that begins before `end` gets its position written to pos[blk], pos[blk + 1],
 // ... below pos[limit]; `blk` is the first of them.  With kRecord the low 16 bits of the positions, plus blk, go to
-// rec[0], rec[1], ... as far as rec[kRecords - 2]; what lies behind the last one may be overwritten.
+// rec[0], rec[1], ... as far as rec[limit - 2]; what lies behind the last one, up to rec[limit - 1], may be overwritten.
 //
 // The 32 lanes of a warp walk unrelated places, so nothing in the loops branches: position (bits 0-23)
 // and zig-zag index (bits 24-30) share one word that an entry is simply added to; a 96-bit window over
@@ -287,7 +287,7 @@ __device__ __forceinline__ uint32_t walk(const unsigned char *buf, Cursor &cur, 
             if (eob && p < end && blk < limit) pos[blk] = p;
             blk += eob ? 1 : 0;
         }
-        if (RECORD == kRecord && eob && done < kRecords) rec[done - 1] = (uint16_t)(st + blk);
+        if (RECORD == kRecord && eob && done < limit) rec[done - 1] = (uint16_t)(st + blk);
     };
     const int pairs_end = (int)end - kHuffBits; // the first symbol of a pair that begins up to here ends before `end`
     if ((int)p <= pairs_end) {
@@ -425,6 +425,11 @@ __device__ __forceinline__ bool index_entry_valid(const DecodeIndexHeader *entry
     return h->magic == kDecodeIndexMagic && h->scan_len == d.scan_len && h->subseq_bits == d.subseq_bits && h->segments == d.seg_count;
 }
 
+// What subsequence t of segment j writes down.
+__device__ __forceinline__ uint16_t *records_of(const EntropyScratch &scratch, const ImageDesc &d, uint32_t j, uint32_t t) {
+    return scratch.records + 4 * (size_t)d.rec_first + ((size_t)j * d.seg_lanes + t) * d.rec_room;
+}
+
 // Every thread decodes one subsequence, beginning a run-up before it in a guessed state: a block, slot 0, begins there.  Most
 // have fallen in step with the real state where the subsequence begins; scan_repair_kernel sees to the others.  Nothing is
 // exchanged between the threads.
@@ -489,6 +494,7 @@ scan_guess_kernel(const ImageDesc *__restrict__ descs, const uint2 *__restrict__
     const bool live = t < n_own && (t >= 0 ? true : begin >= 0);
     const uint32_t start = (uint32_t)max(begin, 0), end = min(start + S, own_end);
     uint32_t done = 0, entry = 0;
+    uint16_t *rec = scratch.records && t >= 0 ? records_of(scratch, d, j, (uint32_t)t) : nullptr;
     if (live) {
         Cursor cur{start - min(start, run_up), 0, 0}; // (the scan's first one begins in this state)
         if (known)
@@ -504,8 +510,8 @@ scan_guess_kernel(const ImageDesc *__restrict__ descs, const uint2 *__restrict__
     for (int round = 0;; round++) {
         if (again) {
             Cursor cur = unpack(entry, start);
-            done = scratch.records && t >= 0 ? walk<kRecord>(buf, cur, end, tables, d, huff, nullptr, 0, 0, scratch.records + sub * kRecords)
-                                             : walk<kNothing>(buf, cur, end, tables, d, huff);
+            done = rec ? walk<kRecord>(buf, cur, end, tables, d, huff, nullptr, 0, d.rec_room, rec)
+                       : walk<kNothing>(buf, cur, end, tables, d, huff);
             sh.exit[tid] = (uint16_t)pack(cur, end);
         }
         team.sync();
@@ -636,7 +642,7 @@ scan_repair_kernel(const ImageDesc *__restrict__ descs, const uint4 *__restrict_
                 const uint32_t skip = start & ~127u; // position of the copied stream's bit 0
                 const unsigned char *stream = streams + (size_t)tid * stream_vectors * 16;
                 Cursor cur = unpack(state, start - skip);
-                const uint32_t done = scratch.records ? walk<kRecord>(stream, cur, end - skip, tables, e, huff, nullptr, skip, 0, scratch.records + sub * kRecords)
+                const uint32_t done = scratch.records ? walk<kRecord>(stream, cur, end - skip, tables, e, huff, nullptr, skip, e.rec_room, records_of(scratch, e, k, t))
                                                       : walk<kNothing>(stream, cur, end - skip, tables, e, huff);
                 const uint32_t was = scratch.sub_info[sub] >> 16;
                 scratch.sub_info[sub] = state | done << 16;
@@ -943,8 +949,8 @@ scan_chain_kernel(const ImageDesc *__restrict__ descs, const int32_t *__restrict
 
 // Where the blocks of a segment are, and their DC values.  SLOTS: of the samples decoded from every slot, by
 // walking every subsequence once more from its real state, its stream in shared memory.  Otherwise the records
-// say it already, unless a subsequence has more blocks than they hold (or there are none): the segments of
-// such a CTA are walked in global memory.
+// say it already, unless a subsequence has more blocks than they hold (or there are none): such a
+// one is walked in global memory.
 template <bool SLOTS>
 constexpr int kIndexTeam = SLOTS ? kSlotSubs : kSegSubs;
 template <int TEAMS, bool SLOTS>
@@ -986,10 +992,10 @@ scan_index_kernel(const ImageDesc *__restrict__ descs, const uint2 *__restrict__
             info = scratch.sub_info[seg * kSegSubs + tid];
             n_rec = (info >> 16) + (scratch.sub_exit[seg * kSegSubs + tid] >> 8 ? 1 : 0) - ((info >> 8 & 63) ? 1 : 0);
         }
-        walks = __syncthreads_or(!scratch.records || n_rec >= kRecords) != 0;
-        if (walks) load_tables(tables, d, huff);
+        walks = tid < n_own && (!scratch.records || n_rec >= d.rec_room);
+        if (__syncthreads_or(walks)) load_tables(tables, d, huff);
     }
-    if (SLOTS || walks) copies_wait();
+    copies_wait();
     __syncthreads();
     if (TEAMS > 1 && mine >= n_segs) return;
     uint32_t *pos = scratch.pos + d.block_base;
@@ -1038,7 +1044,7 @@ scan_index_kernel(const ImageDesc *__restrict__ descs, const uint2 *__restrict__
         const uint32_t luma = d.ncomp == 1 ? 1 : d.hs * d.vs, bpm = d.bpm;
         const uint32_t tab = d.dc_tab[0] | (uint32_t)d.dc_tab[1] << 8 | (uint32_t)d.dc_tab[2] << 16;
         if (tid < n_own && first < nblocks && cur.p < end) {
-            const uint16_t *rec = scratch.records + (seg * kSegSubs + tid) * kRecords;
+            const uint16_t *rec = SLOTS ? nullptr : records_of(scratch, d, j, (uint32_t)tid);
             if (walks) {
                 const uint32_t done = walk<kPositions, !SLOTS>(stream, cur, end, tables, d, huff, pos, b0, nblocks);
                 n_rec = done + (cur.z != 0 ? 1 : 0) - (b0 - first);

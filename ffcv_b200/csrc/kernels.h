@@ -60,7 +60,7 @@ struct EntropyScratch {
     SegMeta *meta;       // per segment
     uint32_t *sub_info;  // per segment kSegSubs words: state at the start of a subsequence, blocks << 16
     uint16_t *sub_exit;  // per segment kSegSubs: the state that leads to at its end
-    uint16_t *records;   // per segment kSegSubs x kRecords: where the blocks of a subsequence begin (16-byte aligned; nullptr: not kept)
+    uint16_t *records;   // of every image per segment seg_lanes x rec_room, from 4 * rec_first on: where the blocks of a subsequence begin (8-byte aligned; nullptr: not kept)
     SlotTables *slots;   // per segment of the samples with ImageDesc::slots
     int32_t *seg_dc;     // per segment four words: DC value of each component before the segment
     uint32_t *done;      // per sample

@@ -73,6 +73,7 @@ struct ImageDesc {
     // segment but the first; bits of run-up before every subsequence (a multiple of 32); bytes of a segment's place in the unstuffed stream; and which of the
     // batch's segments are this image's; and how many subsequences of its own a segment has at most.
     uint32_t subseq_bits, seg_raw, seg_warm, seg_run_up, seg_stride, seg_first, seg_count, seg_lanes;
+    uint32_t rec_first, rec_room; // room for what its subsequences write down, see record_room: the first one's place / 4, and of each
     uint32_t slots;        // decoded from every slot at once: 1 + the first of the image's SlotTables (0: not)
     uint32_t index_use;    // place in the decode index: 0 none, bit 0 the entry may be read, bit 1 and is written
     uint64_t index_off;    // byte offset of the entry in the context's index pool
@@ -166,9 +167,13 @@ struct alignas(16) SegMeta {
     uint32_t doubt[kSegSubs / 32]; // a bit per subsequence that may not begin in the state the one before it ends in
 };
 
-// Positions of its blocks that the decode of a subsequence writes down as it goes (the last place is spare): 20 bits a
-// block in the longest ones.
-constexpr int kRecords = 128;
+// Positions of its blocks that the decode of a subsequence writes down as it goes: room for so many, the last place
+// spare.  Twice as many as a subsequence has on average, and some, because short ones vary more; a quarter of its bits
+// are as many as the standard tables allow.  The few that have more are decoded once more.
+FFCVB_HD inline uint32_t record_room(uint32_t subseq_bits, uint32_t scan_len, uint32_t blocks) {
+    const uint64_t mean = scan_len ? (uint64_t)blocks * subseq_bits / (8 * (uint64_t)scan_len) : 0, most = subseq_bits / 4 + 2, room = 2 * mean + 8;
+    return (uint32_t)((room < most ? room : most) + 3) / 4 * 4;
+}
 
 constexpr uint32_t kNoBlock = 0xFFFFFFFFu; // position of a block that the scan does not hold
 
