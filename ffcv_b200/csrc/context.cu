@@ -283,6 +283,7 @@ struct Slot {
     int gather_ctas = 0;
     int n_block_tiles = 0, n_quad_tiles = 0, bands = 1;
     uint32_t total_blocks = 0;
+    bool keep_records = false; // `records` has room for the staged batch
     size_t clean_bytes = 0, plane_bytes = 0, rgb_bytes = 0, scan_bytes = 0, raw_bytes = 0, jpeg_bytes = 0;
     bool staged = false;
     bool packed = false; // single-image calls: the decoded rows are the result, without padding
@@ -375,6 +376,7 @@ struct ffcvb_ctx {
     // Tuning overrides, read from the environment once when the context is created (0 = none):
     // FFCV_B200_COPY_THREADS, FFCV_B200_SUBSEQ_BITS, FFCV_B200_GATHER_CTAS.
     int tune_copy_threads = 0, tune_subseq_bits = 0, gather_ctas = 0;
+    size_t records_limit = SIZE_MAX; // most device memory a slot asks for to write down blocks' places (FFCV_B200_RECORDS_MB)
     // Transfers of a page-locked source run on one stream of their own, in the order of the batches: two
     // batches that share the link would both arrive late, and the first one's kernels would have nothing
     // to overlap with.  High priority, so that a gather's few CTAs are placed ahead of the large grids
@@ -434,6 +436,40 @@ int grow_dev(ffcvb_ctx *ctx, DevBuf &b, size_t need) {
     CU(cudaMalloc(&b.p, cap));
     b.cap = cap;
     return 0;
+}
+
+// A buffer that a batch cannot do without.  What was written down of blocks' places it can: where memory runs out
+// that goes, of all slots.
+int grow_needed(ffcvb_ctx *ctx, DevBuf &b, size_t need) {
+    const std::string err = ctx->err;
+    int rc = grow_dev(ctx, b, need);
+    if (rc != FFCVB_E_NOMEM) return rc;
+    cudaGetLastError();
+    bool freed = false;
+    for (auto &s : ctx->slots) {
+        if (!s.records.p) continue;
+        if (!freed) CU(cudaDeviceSynchronize());
+        CU(cudaFree(s.records.p));
+        s.records = DevBuf{};
+        freed = true;
+    }
+    if (!freed) return rc;
+    ctx->records_limit = 0;
+    if ((rc = grow_dev(ctx, b, need)) == FFCVB_OK) ctx->err = err; // (no call has failed)
+    return rc;
+}
+
+// Room for what the slot's batch writes down of blocks' places (EntropyScratch::records); without it the index
+// kernel decodes once more.  A context that has run short of memory does not ask again.
+bool grow_records(ffcvb_ctx *ctx, Slot &s, size_t need) {
+    if (need <= s.records.cap) return true;
+    if (need > ctx->records_limit) return false;
+    const std::string err = ctx->err;
+    if (grow_dev(ctx, s.records, need) == FFCVB_OK) return true;
+    cudaGetLastError();
+    ctx->err = err; // (no call has failed)
+    ctx->records_limit = 0;
+    return false;
 }
 
 int grow_host(ffcvb_ctx *ctx, uint8_t *&p, size_t &cap_io, size_t need) {
@@ -533,6 +569,8 @@ int ffcvb_create(int device, int n_slots, int n_threads, ffcvb_ctx **out) {
     c->gather_ctas = env_int("FFCV_B200_GATHER_CTAS", 1, 1024);
     if (const char *e = getenv("FFCV_B200_GATHER_LIMIT_MS"))
         if (*e >= '0' && *e <= '9') c->gather_limit_ns = (uint64_t)env_int("FFCV_B200_GATHER_LIMIT_MS", 0, 600000) * 1000000;
+    if (const char *e = getenv("FFCV_B200_RECORDS_MB"))
+        if (*e >= '0' && *e <= '9') c->records_limit = (size_t)env_int("FFCV_B200_RECORDS_MB", 0, 1 << 20) << 20;
     *out = c;
     return FFCVB_OK;
 }
@@ -1293,15 +1331,14 @@ int stage_impl(ffcvb_ctx *ctx, int slot, const Source &source, const uint64_t *p
     else
         rc = grow_host(ctx, s.host, s.host_cap, host_need + 64);
     if (rc) return rc;
-    if ((rc = grow_dev(ctx, s.blob, off + 64))) return rc;
-    if ((rc = grow_dev(ctx, s.clean, clean_bytes + 512))) return rc;
-    if ((rc = grow_dev(ctx, s.segs, seg_total * kSegScratch + 64))) return rc;
-    // (where there is no room for them the index kernel decodes once more)
-    if (grow_dev(ctx, s.records, (size_t)records * 4 * sizeof(uint16_t)) != FFCVB_OK) cudaGetLastError();
-    if (!s.slot_segs.empty() && (rc = grow_dev(ctx, s.slot_tables, s.slot_segs.size() * sizeof(SlotTables)))) return rc;
-    if ((rc = grow_dev(ctx, s.index, (size_t)total_blocks * 6 + 64))) return rc;
-    if ((rc = grow_dev(ctx, s.planes, plane_bytes + 64))) return rc;
-    if ((rc = grow_dev(ctx, s.rgb, rgb_bytes + 64))) return rc;
+    if ((rc = grow_needed(ctx, s.blob, off + 64))) return rc;
+    if ((rc = grow_needed(ctx, s.clean, clean_bytes + 512))) return rc;
+    if ((rc = grow_needed(ctx, s.segs, seg_total * kSegScratch + 64))) return rc;
+    if (!s.slot_segs.empty() && (rc = grow_needed(ctx, s.slot_tables, s.slot_segs.size() * sizeof(SlotTables)))) return rc;
+    if ((rc = grow_needed(ctx, s.index, (size_t)total_blocks * 6 + 64))) return rc;
+    if ((rc = grow_needed(ctx, s.planes, plane_bytes + 64))) return rc;
+    if ((rc = grow_needed(ctx, s.rgb, rgb_bytes + 64))) return rc;
+    s.keep_records = grow_records(ctx, s, (size_t)records * 4 * sizeof(uint16_t)); // (last: the batch can do without)
 
     memcpy(s.host, &hd, sizeof(hd));
     // (past the caches: the lines were last read by a transfer, and the next one finds them in memory)
@@ -1603,7 +1640,7 @@ static int run_batch(ffcvb_ctx *ctx, Slot &s, cudaStream_t st, void *out_dev, bo
         scratch.sub_exit = (uint16_t *)(scratch.sub_info + kSegSubs * n_segs);
         scratch.meta = (SegMeta *)(scratch.sub_exit + kSegSubs * n_segs); // (everything before it is a multiple of 16 bytes)
         scratch.slots = (SlotTables *)s.slot_tables.p;
-        scratch.records = (uint16_t *)s.records.p;
+        scratch.records = s.keep_records ? (uint16_t *)s.records.p : nullptr;
         scratch.done = (uint32_t *)(blob + s.status_off) + s.n;
         scratch.pos = (uint32_t *)s.index.p;
         scratch.dc = (int16_t *)(scratch.pos + s.total_blocks);

@@ -36,15 +36,20 @@ def test_scans_around_the_segment_length(sampling):
 
 
 @pytest.mark.parametrize('n,mixed', [(739, False), (743, False), (743, True)], ids=['one_team', 'four_teams', 'tables_differ'])
-@pytest.mark.parametrize('subseq_bits', ['', '512'], ids=['from_every_slot', 'from_one_guess'])
+@pytest.mark.parametrize('subseq_bits', ['', '512', '1280', '2560'], ids=['from_every_slot', 'repaired_on_the_spot', 'repaired_behind', 'longest'])
 def test_batches_around_the_team_limit(n, mixed, subseq_bits, monkeypatch):
-    """740 segments are where four teams start to share a CTA (when all scans use the same tables): of the index
-    kernel, and, as these small batches only do when asked to, of the guess-and-repair kernel."""
+    """740 segments are where four teams start to share a CTA, when all scans use the same tables and, as these small
+    batches only do when asked to, leave the repairs to the kernel behind.  Images with flat parts among them, whose
+    subsequences have more blocks than is written down."""
     from ffcv_b200 import libffcv as L
     monkeypatch.setenv('FFCV_B200_SUBSEQ_BITS', subseq_bits)
     rng = np.random.default_rng(n + mixed)
     h, w = 40, 56
     bufs = [_jpeg(rng, h, w, int(rng.integers(60, 98)), 444 if mixed and k % 3 == 0 else 420) for k in range(n)]
+    for k in range(7, n, 29):
+        img = rng.integers(0, 256, (h, w, 3), np.uint8)
+        img[16:] = 99
+        bufs[k] = cv2.imencode('.jpg', img, [cv2.IMWRITE_JPEG_QUALITY, 95])[1].reshape(-1).copy()
     sizes = np.array([b.size for b in bufs], np.uint64)
     params = np.tile(np.array([0, 0, h, w], np.int32), (n, 1))
     ctx = L.Context(0, 1, 4)
@@ -180,10 +185,18 @@ def test_batches_whose_kernels_begin_early(n):
     ctx.close()
 
 
+def _grey_noise(rng, h, w, quality=90):
+    """A scan that decoders fall in step with slowly: of its subsequences of 600 to 2000 bits some 85 in a hundred are decoded
+    wrongly after the run-up, up to 30 in a row."""
+    img = np.repeat(rng.integers(0, 256, (h, w, 1), np.uint8), 3, 2)
+    return cv2.imencode('.jpg', img, [cv2.IMWRITE_JPEG_QUALITY, quality])[1].reshape(-1).copy()
+
+
 def _stage_and_check(bufs, h, w):
     """One batch of JPEG streams of one shape, decoded whole."""
     from ffcv_b200 import libffcv as L
     n = len(bufs)
+    want = {id(b): O.jpeg_decode(b) for b in {id(b): b for b in bufs}.values()}
     sizes = np.array([b.size for b in bufs], np.uint64)
     ctx = L.Context(0, 1, 4)
     out = ch.zeros((n, h, w, 3), dtype=ch.uint8, device='cuda')
@@ -195,16 +208,18 @@ def _stage_and_check(bufs, h, w):
     assert (ctx.status(0, stream, n) == 0).all()
     got = out.cpu().numpy()
     for k, b in enumerate(bufs):
-        assert np.array_equal(got[k], O.jpeg_decode(b)), k
+        assert np.array_equal(got[k], want[id(b)]), k
     ctx.close()
 
 
+@pytest.mark.parametrize('records', ['', '0'], ids=['written_down', 'nothing_written_down'])
 @pytest.mark.parametrize('subseq_bits', [128, 512, 2560])
 @pytest.mark.parametrize('sampling', [420, 444])
-def test_subsequences_of_very_many_blocks(subseq_bits, sampling, monkeypatch):
-    """Flat images: a subsequence holds up to 500 blocks, of which only 127 are written down; flat and busy parts in
-    one scan, so that segments of both kinds follow one another."""
+def test_subsequences_of_very_many_blocks(subseq_bits, sampling, records, monkeypatch):
+    """Flat images: a subsequence holds up to 500 blocks; flat and busy parts in one scan, whose flat subsequences have
+    more blocks than there is room to write down, beside others in one warp."""
     monkeypatch.setenv('FFCV_B200_SUBSEQ_BITS', str(subseq_bits))
+    monkeypatch.setenv('FFCV_B200_RECORDS_MB', records)
     rng = np.random.default_rng(subseq_bits + sampling)
     h, w = 640, 560
     flat = np.full((h, w, 3), 117, np.uint8)
@@ -218,13 +233,28 @@ def test_subsequences_of_very_many_blocks(subseq_bits, sampling, monkeypatch):
     _stage_and_check(bufs, h, w)
 
 
+@pytest.mark.parametrize('records', ['', '0'], ids=['written_down', 'nothing_written_down'])
 @pytest.mark.parametrize('n', [255, 256, 517, 1030])
-def test_images_that_share_a_repair(n, monkeypatch):
-    """From 256, 512 and 1024 images of the same tables on, two, four and eight of them are repaired by one CTA;
-    noise, so that many subsequences have to be, and several rounds of them."""
-    monkeypatch.setenv('FFCV_B200_SUBSEQ_BITS', '128')
+def test_images_that_share_a_repair(n, records, monkeypatch):
+    """From 256, 512 and 1024 images of the same tables on, two, four and eight of them are repaired by one CTA, here in
+    some 30 rounds; the lists of eight (160 subsequences in doubt each, in three segments) are longer than there is room for."""
+    monkeypatch.setenv('FFCV_B200_SUBSEQ_BITS', '1280')
+    monkeypatch.setenv('FFCV_B200_RECORDS_MB', records)
     rng = np.random.default_rng(n)
-    h, w = 40, 56
-    few = [cv2.imencode('.jpg', rng.integers(0, 256, (h, w, 3), np.uint8), [cv2.IMWRITE_JPEG_QUALITY, int(rng.integers(70, 97))])[1].reshape(-1).copy()
-           for _ in range(40)]
-    _stage_and_check([few[int(rng.integers(0, 40))] for _ in range(n)], h, w)
+    h, w = 192, 192
+    few = [_grey_noise(rng, h, w, int(rng.integers(84, 94))) for _ in range(24)]
+    few += [cv2.imencode('.jpg', rng.integers(0, 256, (h, w, 3), np.uint8))[1].reshape(-1).copy(), _jpeg(rng, h, w), _jpeg(rng, h, w, 20)]
+    _stage_and_check([few[int(rng.integers(0, len(few)))] for _ in range(n)], h, w)
+
+
+@pytest.mark.parametrize('subseq_bits', ['1280', '2560'])
+def test_long_scans_repaired_in_parts(subseq_bits, monkeypatch):
+    """Scans of more than 64 segments: parts of 32 of them side by side, each with some 1700 subsequences in doubt at
+    once, then their seams."""
+    monkeypatch.setenv('FFCV_B200_SUBSEQ_BITS', subseq_bits)
+    rng = np.random.default_rng(int(subseq_bits))
+    h, w = 1480, 1320
+    text = np.full((h, w, 3), 245, np.uint8)
+    for y in range(10, h - 12, 16):
+        text[y:y + 9, 12:900] = np.where(rng.random((9, 888, 1)) < 0.3, 30, 245)
+    _stage_and_check([_grey_noise(rng, h, w), cv2.imencode('.jpg', text, [cv2.IMWRITE_JPEG_QUALITY, 90])[1].reshape(-1).copy()], h, w)
