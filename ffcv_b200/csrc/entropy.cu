@@ -1299,10 +1299,12 @@ ScanLayout layout_scan(uint32_t scan_len, uint32_t target_bits, int bpm, bool lo
         }
     } else { // two warps at most (128 of them share the SM's memory out worse: 64 images of 14 Mbit 696 us instead of 653)
         own = indexed ? kSegSubs : 64;
-        l.seg_count = (uint32_t)up(bits, own * target);
+        // (with a decode index a scan that one segment of somewhat longer subsequences takes is not cut in two: 1024 photographs of
+        // 145 kbit from their entries 118 us in one segment each, 128 in two of 96 subsequences)
+        l.seg_count = indexed && bits <= own * std::min<uint64_t>(target + target / 4, kMaxSubseqBits) ? 1 : (uint32_t)up(bits, own * target);
         if (l.seg_count < 1) l.seg_count = 1;
-        own = 32 * up(bits, 32 * target * l.seg_count);
-        if (own < 32) own = 32;
+        const uint64_t lanes = 32 * up(bits, 32 * target * l.seg_count);
+        own = lanes < 32 ? 32 : (lanes > own ? own : lanes);
     }
     l.subseq_bits = (uint32_t)up(up(bits, own * l.seg_count), 32) * 32;
     if (l.subseq_bits < 128) l.subseq_bits = 128;
