@@ -1278,8 +1278,10 @@ constexpr uint32_t kRunUp = 1920, kRunUpFewSlots = 960;
 uint32_t subseq_target(uint64_t total_bits) {
     // A subsequence costs a run-up on top of its own length, so long ones are less work; short ones are a shorter chain,
     // which decides while few bits leave the GPU mostly idle.  Batches of 80 Mbit, alone / as one of four in flight, all
-    // kernels: 352 / 211 us with 200 subsequences per SM, 355 / 208 with 320, 390 / 226 with 480.
-    const uint64_t t = total_bits / (148 * 320);
+    // kernels: 352 / 211 us with 200 subsequences per SM, 355 / 208 with 320, 390 / 226 with 480.  Below some 32 Mbit, where the
+    // run-up is longer than they are, fewer do better: 18 Mbit 196 / 93 with 256 and 202 / 106 with 320, 27 Mbit 214 / 119 and
+    // 241 / 134, 30 Mbit 247 / 120 and 239 / 130, but 44 Mbit 280 / 189 and 278 / 190, 53 Mbit of 4:4:4 222 / 123 and 216 / 123.
+    const uint64_t t = total_bits / (148 * (total_bits <= (32u << 20) ? 256 : 320));
     return (uint32_t)(t < 256 ? 256 : (t > kMaxSubseqBits ? kMaxSubseqBits : (t + 31) / 32 * 32));
 }
 
