@@ -1041,10 +1041,10 @@ int stage_impl(ffcvb_ctx *ctx, int slot, const Source &source, const uint64_t *p
     uint32_t target_bits = 1024, seg_total = 0;
     uint64_t records = 0; // room for them, / 4
     bool few = false; // few enough bits to decode from every slot at once
+    uint64_t bits = 0;
+    for (int i = 0; i < n; i++)
+        if (descs[i].mode == FFCVB_MODE_JPG && descs[i].host_status == 0) bits += (uint64_t)descs[i].scan_len * 8;
     if (!ctx->index_pool.p) {
-        uint64_t bits = 0;
-        for (int i = 0; i < n; i++)
-            if (descs[i].mode == FFCVB_MODE_JPG && descs[i].host_status == 0) bits += (uint64_t)descs[i].scan_len * 8;
         target_bits = subseq_target(bits);
         few = bits <= kSlotModeBits && !ctx->tune_subseq_bits;
     }
@@ -1158,7 +1158,7 @@ int stage_impl(ffcvb_ctx *ctx, int slot, const Source &source, const uint64_t *p
                 for (uint32_t k = 0; k < parts; k++) s.parts.push_back(repair_part((uint32_t)i, l.seg_count, parts, k));
                 if (parts > 1) s.wholes.push_back(make_uint4((uint32_t)i, 0, l.seg_count, 0));
                 if (l.subseq_bits > work.max_subseq_bits) work.max_subseq_bits = l.subseq_bits;
-                d.rec_room = record_room(l.subseq_bits, d.scan_len, (uint32_t)d.bpm * d.mcus_x * d.mcus_y);
+                d.rec_room = record_room(l.subseq_bits, d.scan_len, (uint32_t)d.bpm * d.mcus_x * d.mcus_y, bits <= kAllRecordsBits);
                 d.rec_first = (uint32_t)records;
                 records += (uint64_t)l.seg_count * l.seg_lanes * d.rec_room / 4;
             }

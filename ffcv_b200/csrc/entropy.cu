@@ -494,7 +494,6 @@ scan_guess_kernel(const ImageDesc *__restrict__ descs, const uint2 *__restrict__
     const bool live = t < n_own && (t >= 0 ? true : begin >= 0);
     const uint32_t start = (uint32_t)max(begin, 0), end = min(start + S, own_end);
     uint32_t done = 0, entry = 0;
-    uint16_t *rec = scratch.records && t >= 0 ? records_of(scratch, d, j, (uint32_t)t) : nullptr;
     if (live) {
         Cursor cur{start - min(start, run_up), 0, 0}; // (the scan's first one begins in this state)
         if (known)
@@ -510,8 +509,8 @@ scan_guess_kernel(const ImageDesc *__restrict__ descs, const uint2 *__restrict__
     for (int round = 0;; round++) {
         if (again) {
             Cursor cur = unpack(entry, start);
-            done = rec ? walk<kRecord>(buf, cur, end, tables, d, huff, nullptr, 0, d.rec_room, rec)
-                       : walk<kNothing>(buf, cur, end, tables, d, huff);
+            done = scratch.records && t >= 0 ? walk<kRecord>(buf, cur, end, tables, d, huff, nullptr, 0, d.rec_room, records_of(scratch, d, j, (uint32_t)t))
+                                             : walk<kNothing>(buf, cur, end, tables, d, huff);
             sh.exit[tid] = (uint16_t)pack(cur, end);
         }
         team.sync();
@@ -949,8 +948,9 @@ scan_chain_kernel(const ImageDesc *__restrict__ descs, const int32_t *__restrict
 
 // Where the blocks of a segment are, and their DC values.  SLOTS: of the samples decoded from every slot, by
 // walking every subsequence once more from its real state, its stream in shared memory.  Otherwise the records
-// say it already, unless a subsequence has more blocks than they hold (or there are none): such a
-// one is walked in global memory.
+// say it already, unless a subsequence has more blocks than they hold (or there are none): the segments of
+// such a CTA are walked in global memory.  (Only the warps', or the subsequences themselves: the CTA takes no less time then, see
+// record_room.)
 template <bool SLOTS>
 constexpr int kIndexTeam = SLOTS ? kSlotSubs : kSegSubs;
 template <int TEAMS, bool SLOTS>
@@ -992,8 +992,8 @@ scan_index_kernel(const ImageDesc *__restrict__ descs, const uint2 *__restrict__
             info = scratch.sub_info[seg * kSegSubs + tid];
             n_rec = (info >> 16) + (scratch.sub_exit[seg * kSegSubs + tid] >> 8 ? 1 : 0) - ((info >> 8 & 63) ? 1 : 0);
         }
-        walks = tid < n_own && (!scratch.records || n_rec >= d.rec_room);
-        if (__syncthreads_or(walks)) load_tables(tables, d, huff);
+        walks = __syncthreads_or(tid < n_own && (!scratch.records || n_rec >= d.rec_room)) != 0;
+        if (walks) load_tables(tables, d, huff);
     }
     copies_wait();
     __syncthreads();
