@@ -13,6 +13,7 @@
 #include <stdio.h>
 #include <string.h>
 
+#include <algorithm>
 #include <mutex>
 
 #include "../../include/ffcv_b200.h"
@@ -38,12 +39,17 @@ constexpr size_t kMetaBytes = 96 * 1024;                             // descript
 constexpr size_t kCleanBytes = kMaxStreamBytes + kMaxStreamBytes * 5 / 8 + 8192;
 constexpr size_t kSegBytes = (kMaxSegments * kSegScratch + 255) / 256 * 256;
 constexpr size_t kIndexBytes = (kMaxBlocks * 6 + 255) / 256 * 256;   // position and DC value of every block
+// blocks' places that a decode writes down, see record_room (without room for them it decodes twice)
+constexpr size_t kMaxSubseqs = kMaxStreamBytes * 8 / kSubseqTarget + kSegSubs;
+constexpr size_t kRecords = 4 * kMaxBlocks + 12 * kMaxSubseqs;
+constexpr size_t kRecordBytes = (kRecords * sizeof(uint16_t) + 255) / 256 * 256;
 constexpr size_t kPlaneBytes = 3 * kMaxPaddedSamples + 1024;         // each plane rounded up to 256
 constexpr size_t kCleanOff = kMetaBytes;
 constexpr size_t kSegOff = kCleanOff + kCleanBytes;
 constexpr size_t kIndexOff = kSegOff + kSegBytes;
 constexpr size_t kPlaneOff = kIndexOff + kIndexBytes;
-constexpr size_t kScratchBytes = kPlaneOff + kPlaneBytes;
+constexpr size_t kRecordOff = kPlaneOff + (kPlaneBytes + 255) / 256 * 256;
+constexpr size_t kScratchBytes = kRecordOff + kRecordBytes;
 
 static __device__ __align__(256) unsigned char g_static_scratch[kScratchBytes];
 
@@ -164,6 +170,7 @@ extern "C" int ffcvb_imdecode_static(const uint8_t *jpeg_host, uint64_t jpeg_siz
             return reject(FFCVB_E_LIMIT, "JPEG stream too large for the static scratch");
         for (uint32_t k = 0; k < l.seg_count; k++) m.segs[k] = make_uint2(0, k);
         m.part = repair_part(0, l.seg_count, 1, 0);
+        d.rec_room = (uint32_t)std::min<size_t>(record_room(l.subseq_bits, d.scan_len, d.nblocks, true), kRecords / ((size_t)l.seg_count * l.seg_lanes) / 4 * 4);
     }
     const uint32_t n_tiles = block_tiles(d);
     if (n_tiles > kMaxTiles || d.nblocks > kMaxBlocks) return reject(FFCVB_E_LIMIT, "image larger than FFCVB_STATIC_MAX_PADDED_PIXELS");
@@ -194,6 +201,7 @@ extern "C" int ffcvb_imdecode_static(const uint8_t *jpeg_host, uint64_t jpeg_siz
     es.done = reinterpret_cast<uint32_t *>(&meta_dev->status[1]);
     es.pos = reinterpret_cast<uint32_t *>(scratch + kIndexOff);
     es.dc = reinterpret_cast<int16_t *>(es.pos + kMaxBlocks);
+    if (d.rec_room > 0) es.records = reinterpret_cast<uint16_t *>(scratch + kRecordOff);
     EntropyWork work{};
     work.segs = meta_dev->segs;
     work.n_guess = n_segs;

@@ -317,7 +317,7 @@ int ffcvb_poison(ffcvb_ctx *ctx, void *stream, uint8_t *images_dev, int n, int64
  *   rgb_dev   : DEVICE output buffer of the caller
  * The work is queued on `stream` and the call returns; a corrupt entropy segment is not reported.
  * All scratch (unstuffed bit stream, coefficients, component planes, tables) lives in a fixed
- * array inside the library image, about 3.4 MB that every GPU loading the library holds until
+ * array inside the library image, about 3.9 MB that every GPU loading the library holds until
  * exit, which bounds one call to FFCVB_STATIC_MAX_STREAM_BYTES of JPEG data and
  * FFCVB_STATIC_MAX_PADDED_PIXELS luma samples after padding both sides up to whole MCUs (multiples
  * of 8 or 16); larger inputs are refused with FFCVB_E_LIMIT and a message on stderr.  The call
