@@ -1,4 +1,4 @@
-"""Reads of few samples are shared out in pieces of 128 KB: samples on both sides of that size, anywhere in the file, on a
+"""Reads of few samples are shared out in pieces of 128 KB, except those with O_DIRECT from a disk: samples on both sides of that size, anywhere in the file, on a
 memory file system and on a disk's, with and without O_DIRECT, and a file that ends too early."""
 import os
 
