@@ -431,8 +431,10 @@ __device__ __forceinline__ uint16_t *records_of(const EntropyScratch &scratch, c
 }
 
 // Every thread decodes one subsequence, beginning a run-up before it in a guessed state: a block, slot 0, begins there.  Most
-// have fallen in step with the real state where the subsequence begins; scan_repair_kernel sees to the others.  Nothing is
-// exchanged between the threads.
+// have fallen in step with the real state where the subsequence begins.  Of the others each is noticed by its neighbour's
+// exit, once: SegMeta::doubt, for scan_repair_kernel.  With `local` the CTA repeats them itself, in rounds, until every
+// subsequence begins where the one before it ends, and only a segment's first one is left in doubt; only then have segments
+// subsequences that lead up to them (negative t, which a decode index, never used with `local`, has no words for).
 template <int TEAMS>
 __global__ void __launch_bounds__(kThreads * TEAMS, TEAMS == 4 ? 2 : 1)
 scan_guess_kernel(const ImageDesc *__restrict__ descs, const uint2 *__restrict__ segs, int n_segs, const uint8_t *__restrict__ blob,
