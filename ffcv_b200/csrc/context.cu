@@ -282,6 +282,7 @@ struct Slot {
     uint64_t gather_off = 0; // gather_ranges, for so many CTAs (0: nothing is gathered)
     int gather_ctas = 0;
     int n_block_tiles = 0, n_quad_tiles = 0, bands = 1;
+    bool plain = false; // see ResizeItems
     uint32_t total_blocks = 0;
     bool keep_records = false; // `records` has room for the staged batch
     size_t clean_bytes = 0, plane_bytes = 0, rgb_bytes = 0, scan_bytes = 0, raw_bytes = 0, jpeg_bytes = 0;
@@ -1367,6 +1368,7 @@ int stage_impl(ffcvb_ctx *ctx, int slot, const Source &source, const uint64_t *p
     }
     if (!s.items.empty()) place(s.items_off, s.items.data(), sizeof(ResizeItem) * s.items.size());
     s.bands = items.bands();
+    s.plain = items.plain();
     for (const auto &r : s.riders) {
         if (!r.inline_bytes.empty()) {
             memcpy(s.host + r.off, r.inline_bytes.data(), r.bytes);
@@ -1686,7 +1688,7 @@ static int run_batch(ffcvb_ctx *ctx, Slot &s, cudaStream_t st, void *out_dev, bo
         src.rgb = rgb;
         src.planes = (const uint8_t *)s.planes.p;
         launch_resize_augment(src, s.n, params, (int)hd.n_params, reinterpret_cast<const ResizeItem *>(blob + s.items_off), make_oplist(s.plan), s.plan.resize,
-                              s.plan.out_h, s.plan.out_w, s.plan.out_kind, s.bands, s.plan.lut_dev, out_dev, status, small,
+                              s.plan.out_h, s.plan.out_w, s.plan.out_kind, s.bands, s.plain, s.plan.lut_dev, out_dev, status, small,
                               early && !outputs_free, st);
         for (int k = 0; k < n_large; k++) // (behind the kernel, which may have been launched early)
             CU(cudaMemcpyAsync(large[k]->dst_dev, blob + large[k]->off, large[k]->bytes, cudaMemcpyDeviceToDevice, st));
@@ -1959,7 +1961,7 @@ int ffcvb_transform_device(ffcvb_ctx *ctx, void *stream, const uint8_t *src_dev,
     src.uniform_h = h;
     src.uniform_w = w;
     launch_resize_augment(src, n, (const int32_t *)((const uint8_t *)a.dev.p + items_off), n_params, (const ResizeItem *)a.dev.p, make_oplist(*plan), plan->resize,
-                          plan->out_h, plan->out_w, plan->out_kind, items.bands(), plan->lut_dev, out_dev, nullptr, SmallCopies{}, false, st);
+                          plan->out_h, plan->out_w, plan->out_kind, items.bands(), items.plain(), plan->lut_dev, out_dev, nullptr, SmallCopies{}, false, st);
     CU(cudaGetLastError());
     CU(cudaEventRecord(a.ev, st));
     a.used = true;
@@ -2262,7 +2264,7 @@ void resize(int64_t cresizer, int64_t source_p, int64_t sx, int64_t sy, int64_t 
     rs.uniform_w = cols;
     uint8_t *out = zero_copy ? ctx->one_host + kResultHead : (uint8_t *)ctx->one_dst.p;
     launch_resize_augment(rs, 1, (const int32_t *)ctx->one_src.p, 4, (const ResizeItem *)((const uint8_t *)ctx->one_src.p + 64), OpList{}, 1, (int)tx, (int)ty,
-                          FFCVB_OUT_U8_NHWC, items.bands(), nullptr, out, nullptr, SmallCopies{}, false, st);
+                          FFCVB_OUT_U8_NHWC, items.bands(), items.plain(), nullptr, out, nullptr, SmallCopies{}, false, st);
     if (cudaGetLastError() != cudaSuccess) return;
     if (zero_copy) {
         if (cudaStreamSynchronize(st) == cudaSuccess) memcpy((void *)(intptr_t)dest_p, out, dst_bytes);

@@ -103,7 +103,9 @@ ScanLayout layout_scan(uint32_t scan_len, uint32_t target_bits, int bpm, bool lo
 // Where a batch leaves SMs idle, subsequences that began in the wrong state are decoded again at once, by the threads that have
 // their segment's bytes: a shorter way than scan_repair_kernel, but a segment keeps its shared memory until the last one
 // is right.  So too for a single image, beside which nothing runs.  One of 24 Mbit (4:4:4) / 33 Mbit (4:2:0), all kernels of
-// the entropy decode: 119 and 224 us with repairs behind, 91 and 182 this way.
+// the entropy decode: 119 and 224 us with repairs behind, 91 and 182 this way.  Batches on both sides of the line (60 Mbit), all
+// kernels alone / as one of four in flight, at once and behind: 44 Mbit of 4:2:0 278 / 189 us and 284 / 174, 57 Mbit
+// 312 / 210 and 339 / 200, 65 Mbit 335 / 238 and 349 / 242, 53 Mbit of 4:4:4 212 / 121 and 243 / 130.
 inline bool local_repair(uint32_t target_bits, int n_images) { return target_bits < kMaxSubseqBits / 2 || n_images == 1; }
 // Otherwise a scan of seg_count segments is repaired in parts: one, or, of long scans, of kRepairPart segments each, and what
 // they leave at their seams by one CTA afterwards.
@@ -267,19 +269,23 @@ class ResizeItems {
         return bands < most ? bands : most;
     }
 
+    bool plain() const { return plain_; } // one of them is interpolated without a window
+
   private:
-    int groups(int band);
+    int groups(int band, bool window);
     int out_h_, out_w_, bands_ = 0, most_, most_windowed_;
     bool windowed_ = true; // every band so far
+    bool plain_ = false;
     size_t tile_row_;
     ResizeShape shape_;
     std::vector<uint8_t> groups_; // by rows of a band, 0: not worked out
+    uint8_t plain_groups_ = 0;    // of bands without a window
 };
 
 // Fused crop + INTER_AREA resize + flip/translate/cutout + lookup-table normalise.  items (device): one per image
 // (may be nullptr without `resize`).
 void launch_resize_augment(const ResizeSource &src, int n, const int32_t *params, int n_params, const ResizeItem *items,
-                           const OpList &ops, int resize, int out_h, int out_w, int out_kind, int bands,
+                           const OpList &ops, int resize, int out_h, int out_w, int out_kind, int bands, bool plain,
                            const void *lut, void *out, const int32_t *status, const SmallCopies &small, bool early, cudaStream_t stream);
 
 // Colour jitter kinds (ffcv/transforms/color_jitter.py).

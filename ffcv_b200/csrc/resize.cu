@@ -93,21 +93,12 @@ __device__ __forceinline__ float biased(uint32_t px) {
     return __uint_as_float(pick(px, kBias, 0x7440u | k));
 }
 
-// A pixel of a row: of the window's words, or of packed bytes, of which the first `width` pixels may be read.
-struct PackedRow {
-    const uint8_t *bytes;
-    int width;
-};
+// A pixel of a row: of the window's words, or of packed bytes.  (Those one by one: the aligned words that hold a pixel are
+// fewer requests, but took 276 us instead of 258 for 64 images of 1200x1400 pixels to 224x224.)
 __device__ __forceinline__ uint32_t pixel(const uint32_t *row, int x) { return row[x]; }
-// (The aligned words that hold it; what lies above its 24 bits is another's.  64 crops of some 1000x1200 pixels to
-// 384x384: 299 us byte by byte, 268 this way.)
-__device__ __forceinline__ uint32_t pixel(const PackedRow &row, int x) {
-    const uint8_t *p = row.bytes + 3 * min(x, row.width - 1);
-    const uint32_t phase = (uint32_t)(reinterpret_cast<uintptr_t>(p) & 3);
-    const uint32_t *w = reinterpret_cast<const uint32_t *>(p - phase);
-    uint32_t next = 0;
-    if (phase > 1) next = w[1];
-    return __funnelshift_r(w[0], next, 8 * phase);
+__device__ __forceinline__ uint32_t pixel(const uint8_t *row, int x) {
+    const uint8_t *p = row + 3 * x;
+    return (uint32_t)p[0] | (uint32_t)p[1] << 8 | (uint32_t)p[2] << 16;
 }
 
 // Taps of an output column or row, computed once per CTA (double-precision position arithmetic as
@@ -131,40 +122,42 @@ __device__ __forceinline__ uint4 make_linear_taps(int d, int ssize, double inv, 
 // converted value gives (2^23 * w is exact).  The columns share their instructions, one channel at a time.  A cell of
 // `scale` pixels has scale - 0.002 <= n < scale + 1.998 taps (area_taps), so the columns have equally many or one has
 // one more; the other's pixel there may be the one behind the crop's last, and its weight is zero, which changes no sum.
-struct AreaPair {
+// (V = One: a single column; b is a's.)
+template <class V>
+struct AreaColumns {
     int first[2], mids, taps; // tap `mids` + 1 is the first that is the last one of either column
-    Two w_first, w_mid, w_tail[2];
-    __device__ __forceinline__ AreaPair(uint4 a, uint4 b) {
+    V w_first, w_mid, w_tail[2];
+    __device__ __forceinline__ AreaColumns(uint4 a, uint4 b) {
         const int na = (int)(a.x >> 16), nb = (int)(b.x >> 16);
         first[0] = (int)(a.x & 0xffff);
         first[1] = (int)(b.x & 0xffff);
         taps = max(na, nb);
         mids = max(min(na, nb) - 2, 0);
-        w_first = Two(__uint_as_float(a.y), __uint_as_float(b.y));
-        w_mid = Two(__uint_as_float(a.z), __uint_as_float(b.z));
+        w_first = V(__uint_as_float(a.y), __uint_as_float(b.y));
+        w_mid = V(__uint_as_float(a.z), __uint_as_float(b.z));
 #pragma unroll
-        for (int k = 0; k < 2; k++) w_tail[k] = Two(weight(a, mids + 1 + k), weight(b, mids + 1 + k));
+        for (int k = 0; k < 2; k++) w_tail[k] = V(weight(a, mids + 1 + k), weight(b, mids + 1 + k));
     }
     // of tap k >= 1
     static __device__ __forceinline__ float weight(uint4 t, int k) {
         const int last = (int)(t.x >> 16) - 1;
         return k < last ? __uint_as_float(t.z) : (k == last ? __uint_as_float(t.w) : 0.f);
     }
-    static __device__ __forceinline__ void tap(uint32_t p, uint32_t q, Two w, Two (&v)[3]) {
-        const Two c = fma_rn(w, Two(-8388608.0f, -8388608.0f), Two(0.f, 0.f));
-        v[0] = fma_rn(Two(biased<0>(p), biased<0>(q)), w, c);
-        v[1] = fma_rn(Two(biased<1>(p), biased<1>(q)), w, c);
-        v[2] = fma_rn(Two(biased<2>(p), biased<2>(q)), w, c);
+    static __device__ __forceinline__ void tap(uint32_t p, uint32_t q, V w, V (&v)[3]) {
+        const V c = mul_rn(w, V(-8388608.0f, -8388608.0f));
+        v[0] = fma_rn(V(biased<0>(p), biased<0>(q)), w, c);
+        v[1] = fma_rn(V(biased<1>(p), biased<1>(q)), w, c);
+        v[2] = fma_rn(V(biased<2>(p), biased<2>(q)), w, c);
     }
     template <class Row>
-    __device__ __forceinline__ void more(Row row, int k, Two w, Two (&sum)[3]) const {
-        Two v[3];
+    __device__ __forceinline__ void more(Row row, int k, V w, V (&sum)[3]) const {
+        V v[3];
         tap(pixel(row, first[0] + k), pixel(row, first[1] + k), w, v);
 #pragma unroll
         for (int c = 0; c < 3; c++) sum[c] = add_rn(sum[c], v[c]);
     }
     template <class Row>
-    __device__ __forceinline__ void across(Row row, Two (&sum)[3]) const {
+    __device__ __forceinline__ void across(Row row, V (&sum)[3]) const {
         tap(pixel(row, first[0]), pixel(row, first[1]), w_first, sum);
         for (int k = 1; k <= mids; k++) more(row, k, w_mid, sum);
         if (taps > mids + 1) more(row, mids + 1, w_tail[0], sum);
@@ -176,23 +169,24 @@ struct AreaPair {
 // weighted sum (an exact integer below 2^20), 2^27 + S rounded down is 2^27 + 16 * (S >> 4), and
 // fma(b, that, 2^43 - 2^27 * b) rounded down is 2^43 + 2^20 * (b * (S >> 4) >> 16), the product of the integers
 // in the low bits of its mantissa.  Two neighbouring columns share their instructions.
-struct LinearPair {
+template <class V>
+struct LinearColumns {
     int x0[2], x1[2];
-    Two w0, w1, c0, c1;
-    __device__ __forceinline__ LinearPair(uint4 a, uint4 b) {
+    V w0, w1, c0, c1;
+    __device__ __forceinline__ LinearColumns(uint4 a, uint4 b) {
         x0[0] = (int)a.x, x1[0] = (int)a.y;
         x0[1] = (int)b.x, x1[1] = (int)b.y;
-        w0 = Two(__uint_as_float(a.z), __uint_as_float(b.z));
-        w1 = Two(__uint_as_float(a.w), __uint_as_float(b.w));
-        c0 = mul_rn(w0, Two(-8388608.0f, -8388608.0f));
-        c1 = mul_rn(w1, Two(-8388608.0f, -8388608.0f));
+        w0 = V(__uint_as_float(a.z), __uint_as_float(b.z));
+        w1 = V(__uint_as_float(a.w), __uint_as_float(b.w));
+        c0 = mul_rn(w0, V(-8388608.0f, -8388608.0f));
+        c1 = mul_rn(w1, V(-8388608.0f, -8388608.0f));
     }
     template <class Row>
-    __device__ __forceinline__ void across(Row row, Two (&h)[3]) const {
+    __device__ __forceinline__ void across(Row row, V (&h)[3]) const {
         const uint32_t p0 = pixel(row, x0[0]), q0 = pixel(row, x0[1]), p1 = pixel(row, x1[0]), q1 = pixel(row, x1[1]);
         auto one = [&](float a0, float b0, float a1, float b1) {
-            const Two s = add_rn(fma_rn(Two(a0, b0), w0, c0), fma_rn(Two(a1, b1), w1, c1));
-            return add_rd(s, Two(134217728.f, 134217728.f));
+            const V s = add_rn(fma_rn(V(a0, b0), w0, c0), fma_rn(V(a1, b1), w1, c1));
+            return add_rd(s, V(134217728.f, 134217728.f));
         };
         h[0] = one(biased<0>(p0), biased<0>(q0), biased<0>(p1), biased<0>(q1));
         h[1] = one(biased<1>(p0), biased<1>(q0), biased<1>(p1), biased<1>(q1));
@@ -233,7 +227,9 @@ __device__ __noinline__ void copy_small(const uint8_t *src, uint8_t *dst, uint32
         copy_words<uint8_t>(src, dst, bytes);
 }
 
-template <typename OutT>
+// kPlain: for batches with crops that are interpolated without a window.  Where there are none the kernel does without that way, which
+// costs the other one 3 % by being there (1024 images to 160x160 251 and 259 us).
+template <typename OutT, bool kPlain>
 __global__ void __launch_bounds__(256, 4)
 resize_augment_kernel(const __grid_constant__ ResizeSource src, const int32_t *__restrict__ params, int n_params,
                       const ResizeItem *__restrict__ items,
@@ -391,10 +387,10 @@ resize_augment_kernel(const __grid_constant__ ResizeSource src, const int32_t *_
         }
     };
     // The same for two neighbouring pixels of a row, the first of an even column; `bias` is on top of every value.
-    // They leave as whole words (bytes: half-words) where rows have an even number of pixels.
+    // They leave as whole words (bytes: half-words) where rows have an even number of pixels.  width 1: only the first.
     const bool even = (out_w & 1) == 0;
     const uint32_t lut_address = (uint32_t)__cvta_generic_to_shared(s_lut);
-    auto emit_pair = [&](OutT *o, const uint32_t (&v)[2][3], uint32_t bias, bool both) {
+    auto emit_pair = [&](OutT *o, const uint32_t (&v)[2][3], uint32_t bias, bool both, int width) {
         uint32_t e[2][3];
 #pragma unroll
         for (int p = 0; p < 2; p++)
@@ -409,7 +405,7 @@ resize_augment_kernel(const __grid_constant__ ResizeSource src, const int32_t *_
                 else
                     asm("ld.shared.u32 %0, [%1];" : "=r"(e[p][c]) : "r"(at + 256 * 4 * c));
             }
-        if (!even) {
+        if (width == 1 || !even) {
 #pragma unroll
             for (int p = 0; p < 2; p++) {
                 if (p == 1 && !both) break;
@@ -518,53 +514,59 @@ resize_augment_kernel(const __grid_constant__ ResizeSource src, const int32_t *_
         // whole run, what a source row contributes is computed once for neighbouring output rows that share
         // it, and the columns share instructions and the loop around them.
         // Same operations in the same order as the per-pixel form, so the same bits.
-        const int run = (rows + groups - 1) / groups, pairs = (out_w + 1) >> 1;
+        // Without a window a thread has one column: the taps come through the first-level cache, which four CTAs' shared memory leaves
+        // 28 KB of, and there 32 warps hold 600 bytes of a row each, at a scale of 6, but not 1200 (64 images of
+        // 1200x1400 pixels to 224x224 243 us, 304 with two columns; 400 of them 1271 and 1697; 64 of 1200x1500 to 384x384 269 and 310).
+        const int run = (rows + groups - 1) / groups;
         // row_of: a row of the crop, in the window or in global memory
-        auto columns = [&](auto row_of) {
-            for (int t = threadIdx.x; t < groups * pairs; t += blockDim.x) {
-                const int g = divided(t, inv_pairs, pairs), ox = 2 * (t - g * pairs);
-                const bool both = ox + 1 < out_w;
+        auto columns = [&](auto row_of, auto value) {
+            using V = decltype(value);
+            const int per_row = V::width == 2 ? (out_w + 1) >> 1 : out_w;
+            const uint32_t inv_per_row = V::width == 2 ? inv_pairs : inv_w;
+            for (int t = threadIdx.x; t < groups * per_row; t += blockDim.x) {
+                const int g = divided(t, inv_per_row, per_row), ox = V::width * (t - g * per_row);
+                const bool both = V::width == 2 && ox + 1 < out_w;
                 const int begin = max(y_lo, band0 + g * run + dy), end = min(y_hi, band0 + (g + 1) * run + dy);
                 auto taps_of = [&](int x) { return tx[min(max(step_x * x + dx, 0), out_w - 1)]; };
                 const uint4 taps = taps_of(ox), beside = taps_of(both ? ox + 1 : ox);
                 OutT *o = s_out + ((begin - dy - band0) * out_w + ox) * pix_step;
                 const int row_step = out_w * pix_step;
                 if (regime == kArea) {
-                    const AreaPair pair(taps, beside);
+                    const AreaColumns<V> pair(taps, beside);
                     int pj = -1; // source row whose horizontal sums are held
-                    Two row[3];
-                    row[0] = row[1] = row[2] = Two(0.f, 0.f);
+                    V row[3];
+                    row[0] = row[1] = row[2] = V(0.f, 0.f);
                     for (int y = begin; y < end; y++, o += row_step) {
                         const uint4 c = ty[y];
                         const int yf = (int)(c.x & 0xffff), ye = yf + (int)(c.x >> 16) - 1;
                         // only the first source row can be the one the previous output row ended with
                         if (yf != pj) pair.across(row_of(yf), row);
                         float beta = __uint_as_float(c.y);
-                        Two sum[3];
+                        V sum[3];
 #pragma unroll
-                        for (int k = 0; k < 3; k++) sum[k] = mul_rn(Two(beta, beta), row[k]);
+                        for (int k = 0; k < 3; k++) sum[k] = mul_rn(V(beta, beta), row[k]);
                         for (int j = yf + 1; j <= ye; j++) {
                             pair.across(row_of(j), row);
                             beta = __uint_as_float(j == ye ? c.w : c.z);
 #pragma unroll
-                            for (int k = 0; k < 3; k++) sum[k] = add_rn(sum[k], mul_rn(Two(beta, beta), row[k]));
+                            for (int k = 0; k < 3; k++) sum[k] = add_rn(sum[k], mul_rn(V(beta, beta), row[k]));
                         }
                         pj = ye;
                         // 2^23 + the rounded value.  (The weights of an axis sum up to 1 but for rounding, so 255 is not exceeded.)
                         uint32_t v[2][3];
 #pragma unroll
                         for (int k = 0; k < 3; k++) {
-                            const Two r = add_rn(sum[k], Two(8388608.f, 8388608.f));
+                            const V r = add_rn(sum[k], V(8388608.f, 8388608.f));
                             v[0][k] = __float_as_uint(r.lo());
                             v[1][k] = __float_as_uint(r.hi());
                         }
-                        emit_pair(o, v, kBias, both);
+                        emit_pair(o, v, kBias, both, V::width);
                     }
                 } else {
-                    const LinearPair pair(taps, beside);
+                    const LinearColumns<V> pair(taps, beside);
                     int ra = -1, rb = -1; // source rows whose interpolated values ha / hb hold
-                    Two ha[3], hb[3];
-                    ha[0] = ha[1] = ha[2] = hb[0] = hb[1] = hb[2] = Two(0.f, 0.f);
+                    V ha[3], hb[3];
+                    ha[0] = ha[1] = ha[2] = hb[0] = hb[1] = hb[2] = V(0.f, 0.f);
                     for (int y = begin; y < end; y++, o += row_step) {
                         const uint4 c = ty[y];
                         const int r0 = (int)c.x, r1 = (int)c.y;
@@ -582,25 +584,25 @@ resize_augment_kernel(const __grid_constant__ ResizeSource src, const int32_t *_
                             pair.across(row_of(r1), hb);
                             rb = r1;
                         }
-                        const Two b0(__uint_as_float(c.z), __uint_as_float(c.z)), b1(__uint_as_float(c.w), __uint_as_float(c.w));
-                        const Two k0 = fma_rn(b0, Two(-134217728.f, -134217728.f), Two(8796093022208.f, 8796093022208.f));
-                        const Two k1 = fma_rn(b1, Two(-134217728.f, -134217728.f), Two(8796093022208.f, 8796093022208.f));
+                        const V b0(__uint_as_float(c.z), __uint_as_float(c.z)), b1(__uint_as_float(c.w), __uint_as_float(c.w));
+                        const V k0 = fma_rn(b0, V(-134217728.f, -134217728.f), V(8796093022208.f, 8796093022208.f));
+                        const V k1 = fma_rn(b1, V(-134217728.f, -134217728.f), V(8796093022208.f, 8796093022208.f));
                         uint32_t v[2][3];
 #pragma unroll
                         for (int k = 0; k < 3; k++) {
-                            const Two upper = fma_rd(b0, ha[k], k0), lower = fma_rd(b1, hb[k], k1);
+                            const V upper = fma_rd(b0, ha[k], k0), lower = fma_rd(b1, hb[k], k1);
                             v[0][k] = blended(upper.lo(), lower.lo());
                             v[1][k] = blended(upper.hi(), lower.hi());
                         }
-                        emit_pair(o, v, 0, both);
+                        emit_pair(o, v, 0, both, V::width);
                     }
                 }
             }
         };
         if (window)
-            columns(window_row);
-        else
-            columns([&](int y) { return PackedRow{row_ptr(y), cw}; });
+            columns(window_row, Two());
+        else if constexpr (kPlain)
+            columns(row_ptr, One());
         if (!flips_only) { // what is filled, over it
             __syncthreads();
             for (int pix = threadIdx.x; pix < npix; pix += blockDim.x) {
@@ -671,8 +673,8 @@ ResizeShape resize_shape(int n, int out_h, int out_w, int out_kind) {
     const size_t elem = value_size(out_kind);
     ResizeShape s{};
     const size_t fixed = 768 * elem + sizeof(uint4) * ((size_t)out_w + out_h), row = (size_t)out_w * 3 * elem;
-    // without a window: about 3072 pixels per band
-    int band = (3072 + out_w - 1) / out_w;
+    // without a window: about 2048 pixels per band
+    int band = (2048 + out_w - 1) / out_w;
     if (band > out_h) band = out_h;
     while (band > 1 && fixed + band * row > 200 * 1024) band /= 2;
     s.band = band;
@@ -693,22 +695,23 @@ constexpr int kWaves = 8, kWindowedWaves = 4;
 
 ResizeItems::ResizeItems(int n, int out_h, int out_w, int out_kind)
     : out_h_(out_h), out_w_(out_w), most_((kWaves * 148 * 4 + n - 1) / n), most_windowed_((kWindowedWaves * 148 * 4 + n - 1) / n), tile_row_((size_t)out_w * 3 * value_size(out_kind)),
-      shape_(resize_shape(n, out_h, out_w, out_kind)), groups_((shape_.band > shape_.max_band ? shape_.band : shape_.max_band) + 1, 0) {}
+      shape_(resize_shape(n, out_h, out_w, out_kind)), groups_(shape_.max_band + 1, 0) {}
 
-// The column paths deal a band's rows to this many runs per pair of columns, so that the (pair, run) items fill the
-// CTA's 256 threads evenly, with runs of at least 2 rows.
-int ResizeItems::groups(int band) {
-    if (groups_[band]) return groups_[band];
-    const int pairs = (out_w_ + 1) / 2;
+// The column paths deal a band's rows to this many runs per pair of columns (without a window: per column), so that the
+// (pair, run) items fill the CTA's 256 threads evenly, with runs of at least 2 rows (3).
+int ResizeItems::groups(int band, bool window) {
+    uint8_t &known = window ? groups_[band] : plain_groups_;
+    if (known) return known;
+    const int width = window ? 2 : 1, per_row = (out_w_ + width - 1) / width;
     int groups = 1, best = 0;
-    for (int g = 1; g <= 8 && (band + g - 1) / g >= 2; g++) {
-        const int items = g * pairs, use = items * 256 / ((items + 255) / 256 * 256);
+    for (int g = 1; g <= 4 * width && (band + g - 1) / g >= 4 - width; g++) {
+        const int items = g * per_row, use = items * 256 / ((items + 255) / 256 * 256);
         if (use > best) {
             best = use;
             groups = g;
         }
     }
-    groups_[band] = (uint8_t)groups;
+    known = (uint8_t)groups;
     return groups;
 }
 
@@ -729,35 +732,41 @@ ResizeItem ResizeItems::make(const int32_t *box, int img_h, int img_w, Fuse fuse
     item.units = item.window && fuse == kFuseQuad ? (item.lead + cw + 7) / 8 : (item.lead + cw + 3) / 4;
     item.inv_units = inverse(item.units);
     const int band = item.window ? item.window : shape_.band, bands = (out_h_ + band - 1) / band;
-    item.groups = groups(band);
+    item.groups = groups(band, item.window != 0);
     if (bands > bands_) bands_ = bands;
     windowed_ = windowed_ && item.window != 0;
+    plain_ = plain_ || (item.window == 0 && (sc.regime == kArea || sc.regime == kLinear));
     return item;
 }
 
 template <typename OutT>
 static void launch_typed(const ResizeSource &src, int n, const int32_t *params, int n_params, const ResizeItem *items, const OpList &ops,
-                         int resize, int out_h, int out_w, int planar, const ResizeShape &shape, int bands, const void *lut, void *out,
+                         int resize, int out_h, int out_w, int planar, const ResizeShape &shape, int bands, bool plain, const void *lut, void *out,
                          const int32_t *status, const SmallCopies &small, bool early, cudaStream_t stream) {
-    auto kern = resize_augment_kernel<OutT>;
-    if (shape.smem > 48 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shape.smem);
-    dim3 grid(bands, n);
-    launch(early, grid, 256, shape.smem, stream, kern, src, params, n_params, items, ops, resize, out_h, out_w, shape, planar, (const OutT *)lut, (OutT *)out,
-           status, small);
+    auto run = [&](auto kern) {
+        if (shape.smem > 48 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shape.smem);
+        dim3 grid(bands, n);
+        launch(early, grid, 256, shape.smem, stream, kern, src, params, n_params, items, ops, resize, out_h, out_w, shape, planar, (const OutT *)lut, (OutT *)out,
+               status, small);
+    };
+    if (plain)
+        run(resize_augment_kernel<OutT, true>);
+    else
+        run(resize_augment_kernel<OutT, false>);
 }
 
 void launch_resize_augment(const ResizeSource &src, int n, const int32_t *params, int n_params, const ResizeItem *items,
-                           const OpList &ops, int resize, int out_h, int out_w, int out_kind, int bands,
+                           const OpList &ops, int resize, int out_h, int out_w, int out_kind, int bands, bool plain,
                            const void *lut, void *out, const int32_t *status, const SmallCopies &small, bool early, cudaStream_t stream) {
     if (n <= 0) return;
     const int planar = out_kind == kOutF16Nchw || out_kind == kOutF32Nchw;
     const ResizeShape shape = resize_shape(n, out_h, out_w, out_kind);
     if (out_kind == kOutU8)
-        launch_typed<uint8_t>(src, n, params, n_params, items, ops, resize, out_h, out_w, 0, shape, bands, nullptr, out, status, small, early, stream);
+        launch_typed<uint8_t>(src, n, params, n_params, items, ops, resize, out_h, out_w, 0, shape, bands, plain, nullptr, out, status, small, early, stream);
     else if (out_kind == kOutF16Nhwc || out_kind == kOutF16Nchw)
-        launch_typed<uint16_t>(src, n, params, n_params, items, ops, resize, out_h, out_w, planar, shape, bands, lut, out, status, small, early, stream);
+        launch_typed<uint16_t>(src, n, params, n_params, items, ops, resize, out_h, out_w, planar, shape, bands, plain, lut, out, status, small, early, stream);
     else
-        launch_typed<uint32_t>(src, n, params, n_params, items, ops, resize, out_h, out_w, planar, shape, bands, lut, out, status, small, early, stream);
+        launch_typed<uint32_t>(src, n, params, n_params, items, ops, resize, out_h, out_w, planar, shape, bands, plain, lut, out, status, small, early, stream);
 }
 
 } // namespace ffcvb

@@ -91,6 +91,19 @@ def test_windows_of_every_size(size, form):
         assert np.array_equal(got, want), out
 
 
+@pytest.mark.parametrize('ops', ['flip', 'flip_translate_cutout'])
+@pytest.mark.parametrize('kind', [L.OUT_U8_NHWC, L.OUT_F16_NCHW, L.OUT_F32_NHWC])
+def test_crops_too_wide_for_a_window(kind, ops):
+    """A column per thread: both ways to interpolate, odd and even outputs of one to very many columns, beside crops with
+    a window."""
+    rng = np.random.default_rng(kind)
+    images = [_image(rng, h, w, form) for form in ('420', '444', '422', 'raw') for h, w in ((90, 2600), (41, 3001), (70, 80))]
+    crops = [(k % 3, k, h - k % 3, w - k - 1) for k, (_, h, w, _) in enumerate(images)]
+    for out in ((23, 31), (20, 224), (131, 150), (12, 513), (16, 10)):
+        got, want = _run(rng, images, crops, *out, OPS[ops], kind)
+        assert np.array_equal(got, want), out
+
+
 @pytest.mark.parametrize('shape', [(340, 500), (341, 500), (400, 601), (511, 701), (1200, 1200)], ids=lambda s: f'{s[0]}x{s[1]}')
 def test_regions_copied_by_all_threads(shape):
     """The reference's resize call with regions around and above the size from which all staging threads copy: whole
