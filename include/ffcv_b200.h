@@ -97,7 +97,8 @@ typedef struct ffcvb_ctx ffcvb_ctx;
 /* Creates a context bound to CUDA device `device` with `n_slots` independent batch slots (the
  * ring of ffcv/loader/epoch_iterator.py:62-68) and `n_threads` host staging threads (<= 0: one
  * per available core, capped at 32).  Replaces the per-thread TurboJPEG handles of
- * libffcv/libffcv.cpp:21-31,63-76. */
+ * libffcv/libffcv.cpp:21-31,63-76.  FFCV_B200_RECORDS_MB in the environment bounds the device memory that a slot
+ * takes for what a decode writes down of blocks' places (0: none, the scans are then walked twice). */
 int ffcvb_create(int device, int n_slots, int n_threads, ffcvb_ctx **out);
 void ffcvb_destroy(ffcvb_ctx *ctx);
 const char *ffcvb_last_error(const ffcvb_ctx *ctx);
