@@ -159,12 +159,7 @@ struct AreaColumns {
     template <class Row>
     __device__ __forceinline__ void across(Row row, V (&sum)[3]) const {
         tap(pixel(row, first[0]), pixel(row, first[1]), w_first, sum);
-        if constexpr (V::width == 2) { // (4 at a time, as by itself, 1024 images to 160x160 take 260 us instead of 238)
-#pragma unroll 1
-            for (int k = 1; k <= mids; k++) more(row, k, w_mid, sum);
-        } else {
-            for (int k = 1; k <= mids; k++) more(row, k, w_mid, sum);
-        }
+        for (int k = 1; k <= mids; k++) more(row, k, w_mid, sum);
         if (taps > mids + 1) more(row, mids + 1, w_tail[0], sum);
         if (taps > mids + 2) more(row, mids + 2, w_tail[1], sum);
     }
@@ -233,7 +228,7 @@ __device__ __noinline__ void copy_small(const uint8_t *src, uint8_t *dst, uint32
 }
 
 // kPlain: for batches with crops that are interpolated without a window.  Where there are none the kernel does without that way, which
-// costs the other one 8 % by being there (1024 images to 160x160 238 and 258 us).
+// costs the other one 3 % by being there (1024 images to 160x160 251 and 259 us).
 template <typename OutT, bool kPlain>
 __global__ void __launch_bounds__(256, 4)
 resize_augment_kernel(const __grid_constant__ ResizeSource src, const int32_t *__restrict__ params, int n_params,
@@ -521,7 +516,7 @@ resize_augment_kernel(const __grid_constant__ ResizeSource src, const int32_t *_
         // Same operations in the same order as the per-pixel form, so the same bits.
         // Without a window a thread has one column: the taps come through the first-level cache, which four CTAs' shared memory leaves
         // 28 KB of, and there 32 warps hold 600 bytes of a row each, at a scale of 6, but not 1200 (64 images of
-        // 1200x1400 pixels to 224x224 240 us, 304 with two columns; 400 of them 1250 and 1697; 64 of 1200x1500 to 384x384 266 and 310).
+        // 1200x1400 pixels to 224x224 243 us, 304 with two columns; 400 of them 1271 and 1697; 64 of 1200x1500 to 384x384 269 and 310).
         const int run = (rows + groups - 1) / groups;
         // row_of: a row of the crop, in the window or in global memory
         auto columns = [&](auto row_of, auto value) {
