@@ -26,6 +26,8 @@
 #include "kernels.h"
 #include "two.h"
 
+#include <type_traits>
+
 namespace ffcvb {
 
 enum { kOpFlip = 1, kOpTranslate = 2, kOpCutout = 3 };
@@ -228,7 +230,7 @@ __device__ __noinline__ void copy_small(const uint8_t *src, uint8_t *dst, uint32
 }
 
 // kPlain: for batches with crops that are interpolated without a window.  Where there are none the kernel does without that way, which
-// costs the other one 3 % by being there (1024 images to 160x160 251 and 259 us).
+// costs the other one 3 % by being there (1024 images to 160x160 252 and 258 us).
 template <typename OutT, bool kPlain>
 __global__ void __launch_bounds__(256, 4)
 resize_augment_kernel(const __grid_constant__ ResizeSource src, const int32_t *__restrict__ params, int n_params,
@@ -516,11 +518,13 @@ resize_augment_kernel(const __grid_constant__ ResizeSource src, const int32_t *_
         // Same operations in the same order as the per-pixel form, so the same bits.
         // Without a window a thread has one column: the taps come through the first-level cache, which four CTAs' shared memory leaves
         // 28 KB of, and there 32 warps hold 600 bytes of a row each, at a scale of 6, but not 1200 (64 images of
-        // 1200x1400 pixels to 224x224 243 us, 304 with two columns; 400 of them 1271 and 1697; 64 of 1200x1500 to 384x384 269 and 310).
+        // 1200x1400 pixels to 224x224 240 us, 304 with two columns; 400 of them 1250 and 1697; 64 of 1200x1500 to 384x384 266 and 310).
         const int run = (rows + groups - 1) / groups;
-        // row_of: a row of the crop, in the window or in global memory
-        auto columns = [&](auto row_of, auto value) {
+        // row_of: a row of the crop, in the window or in global memory.  A loop for either way to interpolate: in one the
+        // linear way is 1 % slower (1024 images to 256x256 273 and 277 us).
+        auto columns = [&](auto row_of, auto value, auto way) {
             using V = decltype(value);
+            constexpr bool area = decltype(way)::value;
             const int per_row = V::width == 2 ? (out_w + 1) >> 1 : out_w;
             const uint32_t inv_per_row = V::width == 2 ? inv_pairs : inv_w;
             for (int t = threadIdx.x; t < groups * per_row; t += blockDim.x) {
@@ -531,7 +535,7 @@ resize_augment_kernel(const __grid_constant__ ResizeSource src, const int32_t *_
                 const uint4 taps = taps_of(ox), beside = taps_of(both ? ox + 1 : ox);
                 OutT *o = s_out + ((begin - dy - band0) * out_w + ox) * pix_step;
                 const int row_step = out_w * pix_step;
-                if (regime == kArea) {
+                if constexpr (area) {
                     const AreaColumns<V> pair(taps, beside);
                     int pj = -1; // source row whose horizontal sums are held
                     V row[3];
@@ -599,10 +603,16 @@ resize_augment_kernel(const __grid_constant__ ResizeSource src, const int32_t *_
                 }
             }
         };
+        auto both_ways = [&](auto row_of, auto value) {
+            if (regime == kArea)
+                columns(row_of, value, std::true_type{});
+            else
+                columns(row_of, value, std::false_type{});
+        };
         if (window)
-            columns(window_row, Two());
+            both_ways(window_row, Two());
         else if constexpr (kPlain)
-            columns(row_ptr, One());
+            both_ways(row_ptr, One());
         if (!flips_only) { // what is filled, over it
             __syncthreads();
             for (int pix = threadIdx.x; pix < npix; pix += blockDim.x) {
